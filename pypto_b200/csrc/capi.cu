@@ -139,7 +139,7 @@ size_t li_scores_bytes(int t, int max_blocks, int block_size) {
 
 int sfa_split(int t, int nq) {
   if (nq == 128) return pto::sfa_pair_split(t, 148);  // one cluster of two CTAs per (token, split)
-  const int n_hb = (nq + 63) / 64;
+  const int n_hb = nq / pto::sfa_slice_heads(nq);
   const long long ctas = static_cast<long long>(t) * n_hb;
   if (ctas >= 148) return 1;
   long long s = 148 / (ctas > 0 ? ctas : 1);
@@ -335,7 +335,7 @@ int run_sfa(const void* qn, const void* qr, const void* kn, const void* kr, cons
   p.n_rows = n_rows;
   p.scale_log2 = softmax_scale * 1.4426950408889634f;
   p.status = status;
-  PTO_CUDA(pto::launch_sfa(p, stream));
+  PTO_CUDA(pto::launch_sfa(p, di.num_sms, stream));
   return PTO_OK;
 }
 

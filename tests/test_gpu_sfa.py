@@ -92,6 +92,26 @@ def test_head_slice_of_16():
     _check(_run(d, nq=16), want)
 
 
+@pytest.mark.parametrize("packed", [False, True], ids=["split_arrays", "packed_rows"])
+@pytest.mark.parametrize("nq,lens,s1", [
+    (16, [1, 79, 80, 81, 160, 161, 2048, 2500], 1),    # edges of its 80-row tiles; one item per SM and split
+    (32, [63, 64, 65, 128, 2047, 130, 0, 3000], 2),    # edges of its 64-row tiles, tokens that see nothing
+    (48, [700, 2100], 2),                              # three blocks of 16 heads
+    (64, [300] * 90, 1),                               # more items than SMs: CTAs walk several, unsplit
+])
+def test_head_slices_at_tile_edges(nq, lens, s1, packed):
+    d = gen.make_inputs(lens, s1=s1, seed=37 + nq, with_indexer=False, with_topk=True, attn_heads=nq)
+    want = oracle.sparse_attention(d.query_nope, d.query_rope, d.key_nope_2d, d.key_rope_2d, d.k_nope_scales,
+                                   d.topk_indices, d.block_table, d.act_seq, d.s1, nq=nq)
+    got = _run(d, nq=nq, packed=packed)
+    for bi in range(d.b):
+        for i in range(d.s1):
+            if d.act_seq[bi] - d.s1 + 1 + i > 0:
+                _check(got[bi, i], want[bi, i])
+            else:
+                assert torch.all(got[bi, i] == 0)
+
+
 def test_order_of_indices_does_not_matter_beyond_rounding():
     d = gen.make_inputs([5000], s1=1, seed=2, with_indexer=False, with_topk=True)
     a = _run(d)
