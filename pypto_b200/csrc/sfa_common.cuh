@@ -137,6 +137,13 @@ __device__ __forceinline__ int ldg_pinned_i32(const void* p) {
   return v;
 }
 
+// Brings `bytes` (a multiple of 16, from a 16-byte boundary) into L2 with one instruction. Measured in the pair kernel, cold
+// L2, 64 tokens: packed rows, which straddle lines, 86.1 -> 79.3 us against one `prefetch.global.L2` per 128 bytes; rows
+// of separate arrays 69.5 -> 78.1 (three such copies per row instead of one).
+__device__ __forceinline__ void bulk_prefetch_l2(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
 // 16 bytes global -> shared without a register in between (L2 only); `src_bytes` 0 writes zeros
 __device__ __forceinline__ void cp_async_16(uint32_t dst_smem, const void* src, uint32_t src_bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst_smem), "l"(src), "r"(src_bytes) : "memory");

@@ -23,13 +23,13 @@
 //   warp 0          CTA 0: issues the q.K^T MMAs of a tile as soon as its keys are ready and a score buffer is free
 //   warp 2          CTA 0: issues the P.V MMAs of a tile as soon as P is written and the values are ready
 //                   (two issuing threads on two schedulers: neither queue waits behind the other's barrier)
-//   warp 1          CTA 1: forwards the "ready" events of its own CTA to CTA 0 (tcgen05.commit arrivals on CTA 0's barriers)
+//   warps 0, 1, 2   CTA 1: forward the "ready" events of their CTA to CTA 0 (tcgen05.commit arrivals on CTA 0's barriers)
 //   warps 4..11     softmax: four threads per head (two TMEM lanes x two column halves), P goes to shared memory
 //   warps 12..19    K producers: 16-byte gathers of the CTA's 64 rows, int8 -> bf16 in registers, swizzled stores
 //   warps 20..27    V producers: this CTA's half of the value columns of all 128 rows
 // Cache formats: int8 latent + bf16 rope + fp32 scales in three arrays, the same as packed 656-byte rows, or bf16
 // latent + rope arrays (the non-quantised cache): there the producers dequantise nothing, they copy the rows' bytes
-// from L2 to the same swizzled places with cp.async once a buffer half is free. The MMAs, the softmax and the
+// from L2 to the same swizzled places with cp.async once their part of the buffer is free. The MMAs, the softmax and the
 // output are the same code, so the bf16 cache of dequantised values gives the int8 cache's output bit for bit.
 // Roles are uniform within each group of four warps so that registers can be moved between them (setmaxnreg):
 // 72 per thread at launch (seven warps share one scheduler's file of 512 x 32), then 24 / 104 / 72 / 64:
@@ -69,21 +69,23 @@ constexpr uint32_t kPairColO = 0, kPairColS = 256;        // S buffer b at kPair
 constexpr float kPairRescale = 8.0f;
 
 struct PairCtl {
-  // The K chunks and the V regions are each handed over in two halves, so that a refill runs behind the MMAs that
-  // read the other half: K half 0 = chunks 0-3, half 1 = chunks 4-8 (with the rope chunk); V half h = keys 64h..+63.
-  uint64_t kfull[2];   // K producers filled half h of this CTA's K chunks of tile j     (8 warps)
+  // The K chunks are handed over in halves, the V regions in quarters, so that the refill of one runs behind the MMAs
+  // that read the others: K half h = chunks 4h .. 4h+3 (h = 1: and the rope chunk); V quarter q = keys 32q .. +31.
+  // The loop convert -> notice of the other CTA -> MMAs -> hand-back -> convert is a chain of latencies of about 3 k
+  // cycles beside the work itself; in halves a tile could not take less than that chain plus half its conversion.
+  uint64_t kfull[2];   // K producers filled half h of this CTA's K chunks of tile j     (4 warps)
   uint64_t kfree[2];   // the q.K^T MMAs that read half h are complete                   (tcgen05.commit, both CTAs)
-  uint64_t vfull[2];   // V producers filled this CTA's V region of key half h           (8 warps)
-  uint64_t vfree[2];   // the P.V MMAs that read key half h are complete                 (tcgen05.commit, both CTAs)
+  uint64_t vfull[4];   // V producers filled this CTA's V rows of key quarter q          (2 warps)
+  uint64_t vfree[4];   // the P.V MMAs that read key quarter q are complete              (tcgen05.commit, both CTAs)
   uint64_t sfull[2];   // q.K^T of a tile complete (score buffer b)                      (tcgen05.commit, both CTAs)
   uint64_t pvdone;     // P.V of a tile complete                                        (tcgen05.commit, both CTAs)
   uint64_t pfull;      // this CTA's P of tile j written                                (8 warps)
   uint64_t sread[2];   // this CTA's softmax warps have the scores in registers         (8 warps)
   // in CTA 0 only: the same events of CTA 1, forwarded (one arrival each)
-  uint64_t kpeer[2], vpeer[2], ppeer, speer[2];
+  uint64_t kpeer[2], vpeer[4], ppeer, speer[2];
   uint32_t tmem_base;
   int abort;
-  int go[3][2];        // outcome of a role's latest waits (softmax, K producers, V producers)
+  int go[2];           // outcome of the softmax role's latest waits
   float mt[2][4][64];  // [tile parity][key half * 2 + column half][head]: partial maxima; partial sums at the end
 };
 static_assert(kSmemCtl + sizeof(PairCtl) <= 232448, "exceeds the 227 KB of shared memory a CTA may use");
@@ -121,17 +123,14 @@ __device__ __forceinline__ void tc2_commit(uint32_t bar) {
                : "memory");
 }
 
-// Warp-wide bounded wait that sleeps between probes. A probe is a shared-memory access and a handful of
-// instructions; two dozen warps probing back to back take issue slots and shared-memory cycles from the warps
-// that have work.
-template <int kSleepNs>
+// Warp-wide bounded wait. try_wait parks the warp in hardware; probing with sleeps in between takes issue slots and
+// shared-memory cycles from the warps that have work.
 __device__ __forceinline__ bool pair_wait(uint32_t bar, uint32_t parity) {
   bool ok = true;
   if (!mbar_test_wait(bar, parity)) {
     const long long t0 = clock64();
     while (true) {
-      __nanosleep(kSleepNs);
-      if (mbar_test_wait(bar, parity)) break;
+      if (mbar_try_wait(bar, parity)) break;
       if (clock64() - t0 > kWaitBudgetCycles) {
         ok = false;
         break;
@@ -146,12 +145,12 @@ __device__ __forceinline__ bool pair_wait(uint32_t bar, uint32_t parity) {
 // in one of two slots (alternating: a thread is never more than one wait behind), every thread of the role reads
 // the same slot after the barrier, so the whole role takes the same branch; the barrier itself depends on no data
 // and every thread of the role reaches it on every path.
-template <int kSleepNs, int kBarId, int kThreads, int kRole>
+template <int kBarId, int kThreads>
 __device__ __forceinline__ bool pair_group_wait(PairCtl* ctl, uint32_t& nwait, uint32_t bar, uint32_t parity, bool first_warp) {
-  volatile int* go = &ctl->go[kRole][nwait & 1u];
+  volatile int* go = &ctl->go[nwait & 1u];
   ++nwait;
   if (first_warp) {
-    const bool ok = pair_wait<kSleepNs>(bar, parity);
+    const bool ok = pair_wait(bar, parity);
     if ((threadIdx.x & 31) == 0) *go = ok ? 1 : 0;
   }
   asm volatile("bar.sync %0, %1;" ::"n"(kBarId), "n"(kThreads) : "memory");
@@ -237,157 +236,161 @@ __device__ __forceinline__ uint32_t pair_setup_sync(PairCtl* ctl) {
 // per use. The order is kept by the chain itself: CTA 1's writers fence for the async proxy and arrive on their
 // own barrier, its forwarding thread observes that barrier before it sends the notice, and the MMA issued here
 // after the notice reads CTA 1's shared memory from CTA 1's side.)
-__device__ __forceinline__ bool pair_poll(uint32_t bar, uint32_t parity) {  // one thread, bounded
-  if (mbar_test_wait(bar, parity)) return true;
+// The issuing warps stay converged and one elected lane issues, with descriptors that are constants of the code (kBase:
+// the address where a kernel without static shared memory finds its dynamic part; kBase = 0 is the same code with the
+// address in a register). Under `if (lane == 0)` the descriptors are moved to uniform registers for every MMA: measured in
+// isolation, K = 16, 51-61 cycles per MMA whatever its shape, against the 39 / 48 / 64 / 128 the tensor core needs for N
+// = 16 / 64 / 128 / 256 (cta_group::1); beside two dozen busy warps an address in a register costs about as much.
+constexpr uint32_t kPairUsualBase = 1024;
+__device__ __forceinline__ bool pair_poll(uint32_t bar, uint32_t parity) {  // whole warp, bounded, uniform outcome
+  if (__all_sync(0xffffffffu, mbar_test_wait(bar, parity))) return true;
   const long long t0 = clock64();
   while (true) {
-    __nanosleep(20);
-    if (mbar_test_wait(bar, parity)) return true;
-    if (clock64() - t0 > kWaitBudgetCycles) return false;
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    if (__any_sync(0xffffffffu, clock64() - t0 > kWaitBudgetCycles)) return false;
   }
 }
 
+// half kH of the score product into score buffer `d`: four latent chunks, with the second half the rope chunk too
+template <int kH>
+__device__ __forceinline__ void pair_issue_qk_half(uint32_t d, uint64_t a_desc, uint64_t b_desc) {
+  constexpr uint32_t idesc_qk = umma_idesc(kCFmtF32, kABFmtBF16, kABFmtBF16, 0, 0, 128, kPT);
+#pragma unroll
+  for (int ch = 4 * kH; ch < (kH == 0 ? 4 : kQChunks); ++ch) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      mma2_f16_ss(d, a_desc + ch * (kChunk >> 4) + 2 * k, b_desc + ch * (kChunk >> 4) + 2 * k, idesc_qk, (ch | k) != 0 ? 1u : 0u);
+    }
+  }
+}
+
+template <uint32_t kBase>
 __device__ __forceinline__ void pair_role_issue_qk(const SfaParams& p, PairCtx c) {
+  if (kBase != 0) c.base = kBase;
   PairCtl* ctl = c.ctl;
   const int ntiles = c.ntiles;
-  c.tmem_base = pair_setup_sync(ctl);
-  if ((threadIdx.x & 31) == 0) {
-    const uint32_t idesc_qk = umma_idesc(kCFmtF32, kABFmtBF16, kABFmtBF16, 0, 0, 128, kPT);
-    const uint32_t q_base = c.base + kSmemQ, k_base = c.base + kSmemK;
-    auto issue_qk_chunks = [&](int j, int ch0, int ch1) {
-      const uint32_t d = c.tmem_base + kPairColS + 64 * (j & 1);
-#pragma unroll 1
-      for (int ch = ch0; ch < ch1; ++ch) {
-        const uint64_t a_desc = umma_desc_kmajor_sw128(q_base + ch * kChunk);
-        const uint64_t b_desc = umma_desc_kmajor_sw128(k_base + ch * kChunk);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) mma2_f16_ss(d, a_desc + 2 * k, b_desc + 2 * k, idesc_qk, (ch | k) != 0 ? 1u : 0u);
-      }
-    };
-    bool ok = true;
-    for (int j = 0; j < ntiles && ok; ++j) {
-      const uint32_t ph = j & 1;
-      ok = pair_poll(smem_u32(&ctl->kfull[0]), ph) && pair_poll(smem_u32(&ctl->kpeer[0]), ph);
-      if (ok && j >= 2) {  // the score buffer it overwrites has been read in both CTAs
-        const uint32_t sp = ((j - 2) >> 1) & 1;
-        ok = pair_poll(smem_u32(&ctl->sread[j & 1]), sp) && pair_poll(smem_u32(&ctl->speer[j & 1]), sp);
-      }
-      if (!ok) break;
-      tc_fence_after();
-      TLP(6, j);
-      issue_qk_chunks(j, 0, 4);
-      tc2_commit(smem_u32(&ctl->kfree[0]));
-      ok = pair_poll(smem_u32(&ctl->kfull[1]), ph) && pair_poll(smem_u32(&ctl->kpeer[1]), ph);
-      if (!ok) break;
-      tc_fence_after();
-      issue_qk_chunks(j, 4, kQChunks);
-      tc2_commit(smem_u32(&ctl->kfree[1]));
-      tc2_commit(smem_u32(&ctl->sfull[j & 1]));
-      TLP(7, j);
+  const uint32_t tmem_base = pair_setup_sync(ctl);
+  const uint64_t a_desc = umma_desc_kmajor_sw128(c.base + kSmemQ), b_desc = umma_desc_kmajor_sw128(c.base + kSmemK);
+  bool ok = true;
+  for (int j = 0; j < ntiles && ok; ++j) {
+    const uint32_t ph = j & 1;
+    if (j >= 2) {  // the score buffer it overwrites has been read in both CTAs
+      const uint32_t sp = ((j - 2) >> 1) & 1;
+      ok = pair_poll(smem_u32(&ctl->sread[j & 1]), sp) && pair_poll(smem_u32(&ctl->speer[j & 1]), sp);
     }
-    if (!ok) {
-      ctl->abort = 1;
-      set_status(p.status, PTO_ST_WAIT_EXPIRED, blockIdx.x, 50);
-    }
+    const uint32_t d = tmem_base + kPairColS + 64 * (j & 1);
+#define PAIR_QK_HALF(q)                                                                                      \
+  ok = ok && pair_poll(smem_u32(&ctl->kfull[q]), ph) && pair_poll(smem_u32(&ctl->kpeer[q]), ph);                \
+  if (!ok) break;                                                                                               \
+  tc_fence_after();                                                                                             \
+  if ((q) == 0 && (threadIdx.x & 31) == 0) TLP(6, j);                                                           \
+  if (elect_one()) {                                                                                            \
+    pair_issue_qk_half<q>(d, a_desc, b_desc);                                                                \
+    tc2_commit(smem_u32(&ctl->kfree[q]));                                                                       \
+    if ((q) == 1) tc2_commit(smem_u32(&ctl->sfull[j & 1]));                                                     \
+  }                                                                                                             \
+  __syncwarp();
+    PAIR_QK_HALF(0)
+    PAIR_QK_HALF(1)
+#undef PAIR_QK_HALF
+    if ((threadIdx.x & 31) == 0) TLP(7, j);
+  }
+  if (!ok && (threadIdx.x & 31) == 0) {
+    ctl->abort = 1;
+    set_status(p.status, PTO_ST_WAIT_EXPIRED, blockIdx.x, 50);
   }
   __syncwarp();
 }
 
+// keys 32 kQ .. +31 of a tile into both pairs of value columns
+template <int kQ>
+__device__ __forceinline__ void pair_issue_pv_quarter(uint32_t d, uint64_t a_desc, uint64_t b_desc, uint32_t accumulate) {
+  constexpr uint32_t idesc_pv = umma_idesc(kCFmtF32, kABFmtBF16, kABFmtBF16, 0, 1, 128, 256);
+#pragma unroll
+  for (int dp = 0; dp < 2; ++dp) {
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      constexpr int kh = kQ >> 1;
+      const int k = 2 * (kQ & 1) + e;
+      mma2_f16_ss(d + 128 * dp, a_desc + kh * (kChunk >> 4) + 2 * k,
+                  b_desc + ((kh * kVHalfBytes + dp * 2 * kChunk + k * 16 * 128) >> 4), idesc_pv,
+                  (kQ > 0 || e > 0) ? 1u : accumulate);
+    }
+  }
+}
+
+template <uint32_t kBase>
 __device__ __forceinline__ void pair_role_issue_pv(const SfaParams& p, PairCtx c) {
+  if (kBase != 0) c.base = kBase;
   PairCtl* ctl = c.ctl;
   const int ntiles = c.ntiles;
-  c.tmem_base = pair_setup_sync(ctl);
-  if ((threadIdx.x & 31) == 0) {
-    const uint32_t idesc_pv = umma_idesc(kCFmtF32, kABFmtBF16, kABFmtBF16, 0, 1, 128, 256);
-    const uint32_t v_base = c.base + kSmemV, p_base = c.base + kSmemP;
-    auto issue_pv_half = [&](int j, int kh) {  // keys 64 kh .. +63 into both pairs of value columns
-      const uint64_t a_desc = umma_desc_kmajor_sw128(p_base + kh * kChunk);
-#pragma unroll 1
-      for (int dp = 0; dp < 2; ++dp) {
-        const uint64_t b_desc = desc_mnmajor_sw128(v_base + kh * kVHalfBytes + dp * 2 * kChunk, kChunk, 1024);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          mma2_f16_ss(c.tmem_base + kPairColO + 128 * dp, a_desc + 2 * k, b_desc + k * ((16 * 128) >> 4), idesc_pv,
-                      (j > 0 || kh > 0 || k > 0) ? 1u : 0u);
-        }
-      }
-    };
-    bool ok = true;
-    for (int j = 0; j < ntiles && ok; ++j) {
-      const uint32_t ph = j & 1;
-      ok = pair_poll(smem_u32(&ctl->pfull), ph) && pair_poll(smem_u32(&ctl->ppeer), ph) &&
-           pair_poll(smem_u32(&ctl->vfull[0]), ph) && pair_poll(smem_u32(&ctl->vpeer[0]), ph);
-      if (!ok) break;
-      tc_fence_after();
-      TLP(8, j);
-      issue_pv_half(j, 0);
-      tc2_commit(smem_u32(&ctl->vfree[0]));
-      ok = pair_poll(smem_u32(&ctl->vfull[1]), ph) && pair_poll(smem_u32(&ctl->vpeer[1]), ph);
-      if (!ok) break;
-      tc_fence_after();
-      issue_pv_half(j, 1);
-      tc2_commit(smem_u32(&ctl->vfree[1]));
-      tc2_commit(smem_u32(&ctl->pvdone));
-      TLP(9, j);
-    }
-    if (!ok) {
-      ctl->abort = 1;
-      set_status(p.status, PTO_ST_WAIT_EXPIRED, blockIdx.x, 55);
-    }
+  const uint32_t tmem_base = pair_setup_sync(ctl);
+  const uint64_t a_desc = umma_desc_kmajor_sw128(c.base + kSmemP), b_desc = desc_mnmajor_sw128(c.base + kSmemV, kChunk, 1024);
+  bool ok = true;
+  for (int j = 0; j < ntiles && ok; ++j) {
+    const uint32_t ph = j & 1;
+    ok = pair_poll(smem_u32(&ctl->pfull), ph) && pair_poll(smem_u32(&ctl->ppeer), ph);
+#define PAIR_PV_QUARTER(q)                                                                                      \
+  ok = ok && pair_poll(smem_u32(&ctl->vfull[q]), ph) && pair_poll(smem_u32(&ctl->vpeer[q]), ph);                \
+  if (!ok) break;                                                                                               \
+  tc_fence_after();                                                                                             \
+  if ((q) == 0 && (threadIdx.x & 31) == 0) TLP(8, j);                                                           \
+  if (elect_one()) {                                                                                            \
+    pair_issue_pv_quarter<q>(tmem_base + kPairColO, a_desc, b_desc, j > 0 ? 1u : 0u);                           \
+    tc2_commit(smem_u32(&ctl->vfree[q]));                                                                       \
+    if ((q) == 3) tc2_commit(smem_u32(&ctl->pvdone));                                                           \
+  }                                                                                                             \
+  __syncwarp();
+    PAIR_PV_QUARTER(0)
+    PAIR_PV_QUARTER(1)
+    PAIR_PV_QUARTER(2)
+    PAIR_PV_QUARTER(3)
+#undef PAIR_PV_QUARTER
+    if ((threadIdx.x & 31) == 0) TLP(9, j);
+  }
+  if (!ok && (threadIdx.x & 31) == 0) {
+    ctl->abort = 1;
+    set_status(p.status, PTO_ST_WAIT_EXPIRED, blockIdx.x, 55);
   }
   __syncwarp();
 }
 
 // ================================ forwarding (CTA 1) ============================================
-// One thread: whenever one of this CTA's per-tile events completes, tell CTA 0.
+// Three warps, one per producer of events: when a per-tile event of this CTA completes, tell CTA 0. The events of a
+// role complete in order, so each warp waits for one at a time (a single warp that polled all of them in turn added
+// up to 1 k cycles to a notice).
+enum { kRelayK = 0, kRelayV = 1, kRelayP = 2 };
+template <int kWhat>
 __device__ __forceinline__ void pair_role_relay(const SfaParams& p, PairCtx c) {
   PairCtl* ctl = c.ctl;
   const int ntiles = c.ntiles;
   pair_setup_sync(ctl);
-  if ((threadIdx.x & 31) == 0) {
-    int k_i[2] = {0, 0}, v_i[2] = {0, 0}, p_i = 0, s_i = 0;  // s_i: scores of tile s_i read (only tiles that have a successor two on)
-    const int s_n = ntiles > 2 ? ntiles - 2 : 0;
-    long long t_last = clock64();
-    bool ok = true;
-    while (k_i[0] < ntiles || k_i[1] < ntiles || v_i[0] < ntiles || v_i[1] < ntiles || p_i < ntiles || s_i < s_n) {
-      bool progressed = false;
-      if (p_i < ntiles && mbar_test_wait(smem_u32(&ctl->pfull), p_i & 1)) {
-        pair_signal(smem_u32(&ctl->ppeer));
-        ++p_i;
-        progressed = true;
+  bool ok = true;
+  for (int j = 0; j < ntiles && ok; ++j) {
+    const uint32_t ph = j & 1;
+    if (kWhat == kRelayP) {
+      if (j < ntiles - 2) {  // scores of tile j read: only tiles that have a successor two on
+        ok = pair_poll(smem_u32(&ctl->sread[j & 1]), (j >> 1) & 1);
+        if (ok && elect_one()) pair_signal(smem_u32(&ctl->speer[j & 1]));
+        __syncwarp();
       }
+      ok = ok && pair_poll(smem_u32(&ctl->pfull), ph);
+      if (ok && elect_one()) pair_signal(smem_u32(&ctl->ppeer));
+      __syncwarp();
+    } else {
+      uint64_t* full = kWhat == kRelayK ? ctl->kfull : ctl->vfull;
+      uint64_t* peer = kWhat == kRelayK ? ctl->kpeer : ctl->vpeer;
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        if (k_i[h] < ntiles && mbar_test_wait(smem_u32(&ctl->kfull[h]), k_i[h] & 1)) {
-          pair_signal(smem_u32(&ctl->kpeer[h]));
-          ++k_i[h];
-          progressed = true;
-        }
-        if (v_i[h] < ntiles && mbar_test_wait(smem_u32(&ctl->vfull[h]), v_i[h] & 1)) {
-          pair_signal(smem_u32(&ctl->vpeer[h]));
-          ++v_i[h];
-          progressed = true;
-        }
-      }
-      if (s_i < s_n && mbar_test_wait(smem_u32(&ctl->sread[s_i & 1]), (s_i >> 1) & 1)) {
-        pair_signal(smem_u32(&ctl->speer[s_i & 1]));
-        ++s_i;
-        progressed = true;
-      }
-      if (progressed) {
-        t_last = clock64();
-      } else {
-        __nanosleep(20);
-        if (clock64() - t_last > kWaitBudgetCycles) {
-          ok = false;
-          break;
-        }
+      for (int q = 0; q < (kWhat == kRelayK ? 2 : 4); ++q) {
+        ok = ok && pair_poll(smem_u32(&full[q]), ph);
+        if (ok && elect_one()) pair_signal(smem_u32(&peer[q]));
+        __syncwarp();
       }
     }
-    if (!ok) {
-      ctl->abort = 1;
-      set_status(p.status, PTO_ST_WAIT_EXPIRED, blockIdx.x, 54);
-    }
+  }
+  if (!ok && (threadIdx.x & 31) == 0) {
+    ctl->abort = 1;
+    set_status(p.status, PTO_ST_WAIT_EXPIRED, blockIdx.x, 54);
   }
   __syncwarp();
 }
@@ -420,7 +423,7 @@ __device__ __forceinline__ void pair_role_softmax(const SfaParams& p, PairCtx c)
   };
   for (int j = 0; j < ntiles; ++j) {
     const int b = j & 1;
-    ok = pair_group_wait<20, 1, 256, 0>(ctl, nwait, smem_u32(&ctl->sfull[b]), (j >> 1) & 1, first_warp);
+    ok = pair_group_wait<1, 256>(ctl, nwait, smem_u32(&ctl->sfull[b]), (j >> 1) & 1, first_warp);
     if (!ok) break;
     if (tl) TLP(10, j);
     tc_fence_after();
@@ -475,7 +478,7 @@ __device__ __forceinline__ void pair_role_softmax(const SfaParams& p, PairCtx c)
     l_run = l_run * alpha + lsum * factor;
     // ---- the previous tile's P.V is complete: P may be overwritten, O is at rest ----------------------
     if (j > 0) {
-      ok = pair_group_wait<20, 1, 256, 0>(ctl, nwait, smem_u32(&ctl->pvdone), (j - 1) & 1, first_warp);
+      ok = pair_group_wait<1, 256>(ctl, nwait, smem_u32(&ctl->pvdone), (j - 1) & 1, first_warp);
       if (!ok) break;
       tc_fence_after();
     }
@@ -509,7 +512,7 @@ __device__ __forceinline__ void pair_role_softmax(const SfaParams& p, PairCtx c)
     if (tl) TLP(14, j);
   }
   // ---- output ---------------------------------------------------------------------------------------
-  if (ok) ok = pair_group_wait<20, 1, 256, 0>(ctl, nwait, smem_u32(&ctl->pvdone), (ntiles - 1) & 1, first_warp);
+  if (ok) ok = pair_group_wait<1, 256>(ctl, nwait, smem_u32(&ctl->pvdone), (ntiles - 1) & 1, first_warp);
   if (tl) TLP(5, 20);  // last P.V complete
   float l_tot = 0.f;
   if (ok) {
@@ -595,23 +598,25 @@ __device__ __forceinline__ void pair_role_softmax(const SfaParams& p, PairCtx c)
 }
 
 // ================================ K producers ===================================================
-// 256 threads; warp w owns rows 8w .. 8w+7 of this CTA's 64. A gather instruction reads half a row's latent bytes
-// (256 = two whole 128-byte lines) of TWO rows: lane l takes unit l % 16 of row 2m + l / 16, once for the first
-// half of the row (chunks 0-3) and once for the second (chunks 4-7), so a thread holds unit l % 16 and unit
-// 16 + l % 16 of four rows. (Four threads per row, each reading its own 16 bytes of eight different lines, cost
-// eight lines per instruction; with the V producers' gathers on top, the load/store unit's queue then delayed
-// the tensor core's operand reads: q.K^T took 5-6 k cycles instead of 2.5 k.)
-// Unit u (16 int8 -> 16 bf16 = two 16-byte stores) goes to chunk u / 4, store units 2 (u % 4) and 2 (u % 4) + 1 of
-// the row's 128 bytes; the lanes of an odd chunk store the second half first, so that the eight lanes of a
-// quarter-warp (two chunks, same row) hit eight different bank groups. The first-half units are stored when the
-// q.K^T of the previous tile has read chunks 0-3, the second-half units and the rope when it has read the rest.
-// Lane r % 8 also walks the look-ahead chain of row 8w + r % 8: the selected index four tiles ahead, its
-// block-table entry three tiles ahead, an L2 prefetch of the row two tiles ahead, the row itself (by all lanes)
-// one tile ahead.
+// Eight warps, four per half of the K chunks: warp (half, g) converts the half (256 bytes of latent: two lines of 128
+// dims, each with its scale) of the CTA's rows 16g .. 16g+15; the warps of half 1 also copy the rope part. Every warp
+// waits for its own half, so the load of a half, its conversion, the notice and the MMAs that read it overlap those of
+// the other, and each warp pays the hand-over (wait, fence, arrive) once per tile. (All eight warps walking through
+// quarters together paid it four times: 7.9 k cycles per tile instead of 6.5 k. Two warps per quarter, each one line of 32
+// rows: as fast with separate arrays, slower with packed rows, whose 128-byte pieces straddle lines.)
+// A gather instruction reads the line of FOUR rows, whole: lane l takes 16 bytes of row 4m + (l / 4) % 4. (Four threads
+// per row, each reading its own 16 bytes of eight different lines, cost eight lines per instruction; with the V
+// producers' gathers on top, the load/store unit's queue then delayed the tensor core's operand reads.)
+// Lane l holds unit l % 4 of chunk 2 line + l / 16 of the half (16 int8 -> 16 bf16 = the store units 2 (l % 4) and 2 (l % 4) + 1 of the
+// row's 128 bytes). The eight lanes of a quarter-warp are four units of two neighbouring rows, whose swizzle terms
+// differ in the lowest bit: eight different bank groups.
+// Lane r % 16 also walks the look-ahead chain of row 16g + r: the selected index four tiles ahead, its block-table entry three
+// tiles ahead, an L2 prefetch of the half row two tiles ahead, the half row itself (by all lanes) one tile ahead.
 // kFmt: 0 = int8 latent, bf16 rope and fp32 scales in three arrays, 1 = packed 656-byte rows, 2 = bf16 latent and
-// rope arrays (the non-quantised cache). With a bf16 cache nothing passes through registers: when a half of the
-// buffer is free every lane issues its 16-byte `cp.async` copies from L2 (the rows were prefetched there two tiles
-// ago) straight to the swizzled places the dequantised units would go, waits for them, fences and arrives.
+// rope arrays (the non-quantised cache). With a bf16 cache nothing passes through registers: when the half is free
+// every lane issues its 16-byte `cp.async` copies from L2 (the rows were prefetched there two tiles ago) straight to
+// the swizzled places the dequantised units would go, waits for them, fences and arrives.
+// A padding or rejected row reads row 0 with scale 0, which dequantises to zeros (its rope part is zero-filled).
 template <int kFmt>
 __device__ __forceinline__ void pair_role_kproducer(const SfaParams& p, const PairCtx c) {
   constexpr bool kPacked = kFmt == 1, kBf = kFmt == 2;
@@ -619,9 +624,10 @@ __device__ __forceinline__ void pair_role_kproducer(const SfaParams& p, const Pa
   const int ntiles = c.ntiles, bi = c.bi;
   const int lane = threadIdx.x & 31;
   const int ptid = threadIdx.x - kPairKWarp0 * 32;
-  const int w = ptid >> 5;
-  const int u = lane & 15, s2 = lane >> 4;
-  const int my_row = 64 * static_cast<int>(c.crank) + 8 * w + (lane & 7);  // key of the tile this lane looks ahead for
+  const int half = ptid >> 7, g = (ptid >> 5) & 3;
+  const int u = lane & 3, r4 = (lane >> 2) & 3, cp = lane >> 4;
+  const int line_off = cp * 64 + u * 16;  // this lane's 16 bytes of a line
+  const int my_row = 64 * static_cast<int>(c.crank) + 16 * g + (lane & 15);  // key of the tile this lane looks ahead for
   const int32_t* idx_ptr = c.idx_row + c.begin + my_row;
   const int n_mine = c.end - (c.begin + my_row);  // entry j * 128 of idx_ptr is valid iff j * 128 < n_mine
   constexpr int stride_n = kPacked ? 656 : (kBf ? 1024 : 512), stride_r = kPacked ? 656 : 128, stride_s = kPacked ? 656 : 16;
@@ -630,61 +636,42 @@ __device__ __forceinline__ void pair_role_kproducer(const SfaParams& p, const Pa
 #define PAIR_KN reinterpret_cast<const uint8_t*>(p.kn)
 #define PAIR_ROPE (kPacked ? PAIR_KN + 512 : reinterpret_cast<const uint8_t*>(p.kr))
 #define PAIR_SCL (kPacked ? PAIR_KN + 640 : reinterpret_cast<const uint8_t*>(p.kn_scales))
-  struct RowRegs {
-    uint4 d[2][4];  // [row half][m]: unit 16 half + u of row 8w + 2m + s2
-    uint4 r[2];     // rope unit lane % 8 of rows 8w + 4i + lane / 8
-    float sc;       // scale lane % 4 of row 8w + lane / 4
-  };
+  uint4 d[4][2];   // [m][line]: this lane's 16 bytes of the line of row 4m + r4
+  float sc = 0.f;  // scale lane / 16 (of the half's two) of row lane % 16
   auto load_idx = [&](int j) -> int { return (j < ntiles && j * kPT < n_mine) ? ldg_pinned_i32(idx_ptr + j * kPT) : -1; };
-  // `phys`: this lane's look-ahead row of the tile (-1: padding or rejected -> zeros with scale 0)
-  auto issue_loads = [&](RowRegs& r, int phys) {
+  // `phys`: this lane's look-ahead row of the tile
+  auto issue_loads = [&](int phys) {
     if (kBf) return;  // (copied from L2 when the buffer is free)
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
-      const int pm = __shfl_sync(0xffffffffu, phys, 2 * m + s2);
-      r.d[0][m] = make_uint4(0, 0, 0, 0);
-      r.d[1][m] = make_uint4(0, 0, 0, 0);
-      if (pm >= 0) {
-        const uint8_t* a = PAIR_KN + static_cast<int64_t>(pm) * stride_n + u * 16;
-        r.d[0][m] = ldg_pinned_v4(a);
-        r.d[1][m] = ldg_pinned_v4(a + 256);
-      }
+      const int pm = max(__shfl_sync(0xffffffffu, phys, 4 * m + r4), 0);
+      const uint8_t* src = PAIR_KN + static_cast<int64_t>(pm) * stride_n + half * 256 + line_off;
+      d[m][0] = ldg_pinned_v4(src);
+      d[m][1] = ldg_pinned_v4(src + 128);
     }
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int pr = __shfl_sync(0xffffffffu, phys, 4 * i + (lane >> 3));
-      r.r[i] = make_uint4(0, 0, 0, 0);
-      if (pr >= 0) r.r[i] = ldg_pinned_v4(PAIR_ROPE + static_cast<int64_t>(pr) * stride_r + (lane & 7) * 16);
-    }
-    const int ps = __shfl_sync(0xffffffffu, phys, lane >> 2);
-    r.sc = 0.f;
-    if (ps >= 0) asm volatile("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(r.sc) : "l"(PAIR_SCL + static_cast<int64_t>(ps) * stride_s + (lane & 3) * 4));
+    sc = 0.f;
+    if (phys >= 0) asm volatile("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(sc) : "l"(PAIR_SCL + static_cast<int64_t>(phys) * stride_s + half * 8 + (lane >> 4) * 4));
   };
-  auto prefetch_row = [&](int phys) {  // lanes r, r+8, r+16, r+24 share a row: one of its four latent lines each, two of them the rest
+  auto prefetch_row = [&](int phys) {  // lanes r and r + 16: a line each of the half row; half 1 also the rest of the row
     if (phys < 0) return;
-    if (kBf) {  // eight latent lines and the rope line of the row
-      const uint8_t* a = PAIR_KN + static_cast<int64_t>(phys) * 1024;
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(a + (lane >> 3) * 128));
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(a + 512 + (lane >> 3) * 128));
-      if (lane < 8) asm volatile("prefetch.global.L2 [%0];" ::"l"(PAIR_ROPE + static_cast<int64_t>(phys) * 128));
+    const int l = lane >> 4;
+    if (kBf) {
+      const uint8_t* a = PAIR_KN + static_cast<int64_t>(phys) * 1024 + half * 512 + l * 256;
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(a));
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(a + 128));
+      if (half == 1 && l == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(PAIR_ROPE + static_cast<int64_t>(phys) * 128));
     } else if (kPacked) {
-      const uint8_t* a = PAIR_KN + static_cast<int64_t>(phys) * 656;
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(a + (lane >> 3) * 128));
-      if (lane < 16) asm volatile("prefetch.global.L2 [%0];" ::"l"(a + 512 + (lane >> 3) * 128));
+      if (half == 0 && lane < 16) bulk_prefetch_l2(PAIR_KN + static_cast<int64_t>(phys) * 656, 656);
     } else {
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(PAIR_KN + static_cast<int64_t>(phys) * 512 + (lane >> 3) * 128));
-      if (lane < 8) asm volatile("prefetch.global.L2 [%0];" ::"l"(PAIR_ROPE + static_cast<int64_t>(phys) * 128));
-      else if (lane < 16) asm volatile("prefetch.global.L2 [%0];" ::"l"(PAIR_SCL + static_cast<int64_t>(phys) * 16));
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(PAIR_KN + static_cast<int64_t>(phys) * 512 + half * 256 + l * 128));
+      if (half == 1) asm volatile("prefetch.global.L2 [%0];" ::"l"(l == 0 ? PAIR_ROPE + static_cast<int64_t>(phys) * 128 : PAIR_SCL + static_cast<int64_t>(phys) * 16));
     }
   };
-  const uint32_t k_rows = c.base + kSmemK + (u >> 2) * kChunk + 8 * w * 128;  // row 8w of this lane's chunk of half 0
-  const bool odd = ((u >> 2) & 1) != 0;
+  const uint32_t k_rows = c.base + kSmemK + (4 * half + cp) * kChunk + (16 * g + r4) * 128;  // row r4 of this lane's chunk of line 0
   bool ok = true;
-  uint32_t nwait = 0;
-  RowRegs ra;
   pdl_wait();          // the selected indices come from the kernel before this one, which may still be running
   if (ptid == 0) TLP(3, 21);
-  int row_cur;         // this lane's row of tile j (bf16 cache: the copies are issued when the buffer is free)
+  int row_cur;         // this lane's row of tile j
   int row_n;           // this lane's row of tile j+1
   int idx_a, entry_a;  // tile j+2
   int idx_b;           // tile j+3
@@ -698,66 +685,60 @@ __device__ __forceinline__ void pair_role_kproducer(const SfaParams& p, const Pa
     entry_a = tc_table_entry(p, bi, idx_a);
     if (ptid == 0 && e0 + e1 + entry_a != -12345) TLP(5, 21);
     row_cur = pair_row(p, idx0, e0);
-    issue_loads(ra, row_cur);
+    issue_loads(row_cur);
     if (kBf) prefetch_row(row_cur);
     row_n = pair_row(p, idx1, e1);
     prefetch_row(row_n);
     if (ptid == 0) TLP(6, 21);
   }
-  if (!kBf && ptid == 0 && ra.d[0][0].x != 0x7fffffffu) TLP(7, 21);  // first rows arrived
+  if (!kBf && ptid == 0 && d[0][0].x != 0x7fffffffu) TLP(7, 21);  // first rows arrived
   pair_setup_sync(ctl);
-  for (int j = 0; j < ntiles && ok; ++j) {
+  for (int j = 0; j < ntiles; ++j) {
+    if (j > 0) {  // the q.K^T MMAs of the previous tile that read this half of the chunks are complete
+      ok = pair_wait(smem_u32(&ctl->kfree[half]), (j - 1) & 1);
+      if (!ok) break;
+    }
+    if (ptid == 0) TLP(0, j);
+    if (half == 1) {  // the rope part goes straight from L2 to shared memory behind the conversion below
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      if (j > 0) {  // the q.K^T MMAs of the previous tile that read this half of the chunks are complete
-        ok = pair_group_wait<32, 2, 256, 1>(ctl, nwait, smem_u32(&ctl->kfree[half]), (j - 1) & 1, ptid < 32);
-        if (!ok) break;
+      for (int m = 0; m < 4; ++m) {  // rows 4m + lane / 8 of the warp's 16
+        const int r = 4 * m + (lane >> 3);
+        const int pr = __shfl_sync(0xffffffffu, row_cur, r);
+        cp_async_16(c.base + kSmemK + 8 * kChunk + (16 * g + r) * 128 + (((lane & 7) ^ (r & 7)) << 4),
+                    PAIR_ROPE + (pr >= 0 ? static_cast<int64_t>(pr) * stride_r + (lane & 7) * 16 : 0), pr >= 0 ? 16u : 0u);
       }
-      if (ptid == 0 && half == 0) TLP(0, j);
+    }
 #pragma unroll
-      for (int m = 0; m < 4; ++m) {  // row 8w + 2m + s2 (its swizzle term is 2m + s2); scale 2 half + u / 8 of that row
-        const int x = 2 * m + s2;
-        const uint32_t row_addr = k_rows + half * 4 * kChunk + x * 128;
-        const uint32_t a = ((2 * (u & 3)) ^ x) << 4, b = ((2 * (u & 3) + 1) ^ x) << 4;
+    for (int m = 0; m < 4; ++m) {  // row 4m + r4: swizzle term 4 (m % 2) + r4
+      const int x = 4 * (m & 1) + r4;
+      const uint32_t a = ((2 * u) ^ x) << 4, b = ((2 * u + 1) ^ x) << 4;
+#pragma unroll
+      for (int l = 0; l < 2; ++l) {
+        const uint32_t row_addr = k_rows + 4 * m * 128 + l * 2 * kChunk;
         if (kBf) {  // the unit's 16 values are 32 bytes of the bf16 row: two copies
-          const int pm = __shfl_sync(0xffffffffu, row_cur, x);
-          const uint8_t* src = PAIR_KN + (pm >= 0 ? static_cast<int64_t>(pm) * 1024 + half * 512 + u * 32 : 0);
+          const int pm = __shfl_sync(0xffffffffu, row_cur, 4 * m + r4);
+          const uint8_t* src = PAIR_KN + (pm >= 0 ? static_cast<int64_t>(pm) * 1024 + half * 512 + l * 256 + 2 * line_off : 0);
           cp_async_16(row_addr + a, src, pm >= 0 ? 16u : 0u);
           cp_async_16(row_addr + b, src + (pm >= 0 ? 16 : 0), pm >= 0 ? 16u : 0u);
         } else {
-          const float scale = __shfl_sync(0xffffffffu, ra.sc, 4 * x + 2 * half + (u >> 3));
-          const uint4 v = ra.d[half][m];
-          // first half of the unit (bytes 0-7) belongs at `a`, second half at `b`; odd chunks store the second first
-          sts_v4u(row_addr + (odd ? b : a), pair_dequant8(odd ? v.z : v.x, odd ? v.w : v.y, scale));
-          sts_v4u(row_addr + (odd ? a : b), pair_dequant8(odd ? v.x : v.z, odd ? v.y : v.w, scale));
+          const float scale = __shfl_sync(0xffffffffu, sc, 16 * l + 4 * m + r4);
+          const uint4 v = d[m][l];
+          sts_v4u(row_addr + a, pair_dequant8(v.x, v.y, scale));
+          sts_v4u(row_addr + b, pair_dequant8(v.z, v.w, scale));
         }
       }
-      if (half == 1) {
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {  // rope of row 8w + 4i + lane / 8
-          const int r8 = 4 * i + (lane >> 3);
-          const uint32_t dst = c.base + kSmemK + 8 * kChunk + (8 * w + r8) * 128 + (((lane & 7) ^ r8) << 4);
-          if (kBf) {
-            const int pr = __shfl_sync(0xffffffffu, row_cur, r8);
-            cp_async_16(dst, PAIR_ROPE + (pr >= 0 ? static_cast<int64_t>(pr) * 128 + (lane & 7) * 16 : 0), pr >= 0 ? 16u : 0u);
-          } else {
-            sts_v4u(dst, ra.r[i]);
-          }
-        }
-      }
-      if (kBf) asm volatile("cp.async.wait_all;" ::: "memory");
-      fence_proxy_async();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&ctl->kfull[half]));
-      if (ptid == 0 && half == 1) TLP(1, j);
     }
-    if (!ok) break;
-    if (j + 1 < ntiles) issue_loads(ra, row_n);  // rows of tile j+1 (in L2: prefetched a tile ago)
+    if (kBf || half == 1) asm volatile("cp.async.wait_all;" ::: "memory");
+    fence_proxy_async();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(smem_u32(&ctl->kfull[half]));
+    if (ptid == 0) TLP(1, j);
+    if (j + 1 < ntiles) issue_loads(row_n);  // the half rows of tile j+1 (in L2: prefetched a tile ago)
     row_cur = row_n;
-    row_n = pair_row(p, idx_a, entry_a);         // tile j+2: into L2
+    row_n = pair_row(p, idx_a, entry_a);     // tile j+2: into L2
     prefetch_row(row_n);
     idx_a = idx_b;
-    entry_a = tc_table_entry(p, bi, idx_a);      // block-table entries of tile j+3
+    entry_a = tc_table_entry(p, bi, idx_a);  // block-table entries of tile j+3
     idx_b = load_idx(j + 4);
   }
   if (!ok && lane == 0) {
@@ -767,13 +748,10 @@ __device__ __forceinline__ void pair_role_kproducer(const SfaParams& p, const Pa
 }
 
 // ================================ V producers ===================================================
-// 256 threads; warp w owns rows 8w .. 8w+7 of EACH key half of the tile (keys 64 h + 8w ..). A gather instruction
-// reads this CTA's half of the value columns (256 of the 512 latent bytes) of TWO rows: lane l takes unit l % 16
-// of row 2m + l / 16, again whole 128-byte lines (the other CTA's K producers have fetched or are fetching the
-// same lines: L2 hits). Unit u goes to V chunk u / 4 of the row's key half, store units 2 (u % 4) and 2 (u % 4) + 1,
-// second half first in odd chunks as in the K producers. Key half 0 is stored when the P.V of the previous tile
-// has read keys 0-63, key half 1 when it has read the rest. Lane r % 16 walks the look-ahead chain of row
-// 64 (r / 8) + 8w + r % 8 (no L2 prefetch: the row's owner issues it).
+// Eight warps, two per key quarter: warp (q, h) converts this CTA's half of the value columns (256 of the 512 latent
+// bytes: two lines) of the 16 rows with keys 32q + 16h .. +15, lanes arranged as in the K producers (the other CTA's K
+// producers have fetched or are fetching the same lines: L2 hits). Lane r % 16 walks the look-ahead chain of row r (no
+// L2 prefetch: the row's owner issues it).
 template <int kFmt>
 __device__ __forceinline__ void pair_role_vproducer(const SfaParams& p, const PairCtx c) {
   constexpr bool kPacked = kFmt == 1, kBf = kFmt == 2;
@@ -781,90 +759,83 @@ __device__ __forceinline__ void pair_role_vproducer(const SfaParams& p, const Pa
   const int ntiles = c.ntiles;
   const int lane = threadIdx.x & 31;
   const int vtid = threadIdx.x - kPairVWarp0 * 32;
-  const int w = vtid >> 5;
-  const int u = lane & 15, s2 = lane >> 4;
-  const int my_row = 64 * ((lane >> 3) & 1) + 8 * w + (lane & 7);  // key of the tile this lane looks ahead for
+  const int q = vtid >> 6, h = (vtid >> 5) & 1;
+  const int u = lane & 3, r4 = (lane >> 2) & 3, cp = lane >> 4;
+  const int line_off = cp * 64 + u * 16;  // this lane's 16 bytes of a line
+  const int my_row = 32 * q + 16 * h + (lane & 15);  // key of the tile this lane looks ahead for
   const int32_t* idx_ptr = c.idx_row + c.begin + my_row;
   const int n_mine = c.end - (c.begin + my_row);
   const int col0 = 256 * static_cast<int>(c.crank);  // first latent byte of this CTA's value columns
   constexpr int stride_n = kPacked ? 656 : (kBf ? 1024 : 512), stride_s = kPacked ? 656 : 16;
-  struct RowRegs {
-    uint4 d[2][4];  // [key half][m]: unit u of row 64 half + 8w + 2m + s2
-    float sc;       // scale lane % 2 (of this CTA's two) of the row lane / 2 (chain order: half * 8 + r)
-  };
+  uint4 d[4][2];   // [m][line]: this lane's 16 bytes of the line of row 4m + r4
+  float sc = 0.f;  // scale lane / 16 (of this CTA's two) of row lane % 16
   auto load_idx = [&](int j) -> int { return (j < ntiles && j * kPT < n_mine) ? ldg_pinned_i32(idx_ptr + j * kPT) : -1; };
-  auto issue_loads = [&](RowRegs& r, int phys) {
+  auto issue_loads = [&](int phys) {
     if (kBf) return;
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-#pragma unroll
-      for (int m = 0; m < 4; ++m) {
-        const int pm = __shfl_sync(0xffffffffu, phys, 8 * half + 2 * m + s2);
-        r.d[half][m] = make_uint4(0, 0, 0, 0);
-        if (pm >= 0) r.d[half][m] = ldg_pinned_v4(PAIR_KN + static_cast<int64_t>(pm) * stride_n + col0 + u * 16);
-      }
+    for (int m = 0; m < 4; ++m) {
+      const int pm = max(__shfl_sync(0xffffffffu, phys, 4 * m + r4), 0);
+      const uint8_t* src = PAIR_KN + static_cast<int64_t>(pm) * stride_n + col0 + line_off;
+      d[m][0] = ldg_pinned_v4(src);
+      d[m][1] = ldg_pinned_v4(src + 128);
     }
-    const int ps = __shfl_sync(0xffffffffu, phys, lane >> 1);
-    r.sc = 0.f;
-    if (ps >= 0) asm volatile("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(r.sc) : "l"(PAIR_SCL + static_cast<int64_t>(ps) * stride_s + (col0 >> 5) + (lane & 1) * 4));
+    sc = 0.f;
+    if (phys >= 0) asm volatile("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(sc) : "l"(PAIR_SCL + static_cast<int64_t>(phys) * stride_s + (col0 >> 5) + (lane >> 4) * 4));
   };
-  // row 8w of chunk u / 4 in the V region of key half 0
-  const uint32_t v_rows = c.base + kSmemV + (u >> 2) * kChunk + 8 * w * 128;
-  const bool odd = ((u >> 2) & 1) != 0;
+  // row r4 of this warp's 16 in this lane's chunk of line 0; line 1 lies two chunks further
+  const uint32_t v_rows = c.base + kSmemV + (q >> 1) * kVHalfBytes + cp * kChunk + (32 * (q & 1) + 16 * h + r4) * 128;
   bool ok = true;
-  uint32_t nwait = 0;
-  RowRegs ra;
   pdl_wait();
-  int row_cur, row_n, idx_a, entry_a;  // this lane's row of tiles j and j+1; index and block-table entry of tile j+2
+  int row_cur, row_n, idx_a, entry_a, idx_b;  // this lane's row of tiles j, j+1; index and block-table entry of j+2; index of j+3
   {
     const int idx0 = load_idx(0), idx1 = load_idx(1);
     idx_a = load_idx(2);
+    idx_b = load_idx(3);
     const int e0 = tc_table_entry(p, c.bi, idx0);
     const int e1 = tc_table_entry(p, c.bi, idx1);
     entry_a = tc_table_entry(p, c.bi, idx_a);
     row_cur = pair_row(p, idx0, e0);
-    issue_loads(ra, row_cur);
+    issue_loads(row_cur);
     row_n = pair_row(p, idx1, e1);
   }
   pair_setup_sync(ctl);
-  for (int j = 0; j < ntiles && ok; ++j) {
+  for (int j = 0; j < ntiles; ++j) {
+    if (j > 0) {  // the P.V MMAs of the previous tile that read this key quarter are complete
+      ok = pair_wait(smem_u32(&ctl->vfree[q]), (j - 1) & 1);
+      if (!ok) break;
+    }
+    if (vtid == 0) TLP(4, j);
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      if (j > 0) {  // the P.V MMAs of the previous tile that read this key half are complete
-        ok = pair_group_wait<32, 3, 256, 2>(ctl, nwait, smem_u32(&ctl->vfree[half]), (j - 1) & 1, vtid < 32);
-        if (!ok) break;
-      }
-      if (vtid == 0 && half == 0) TLP(4, j);
+    for (int m = 0; m < 4; ++m) {  // row 4m + r4
+      const int x = 4 * (m & 1) + r4;
+      const uint32_t a = ((2 * u) ^ x) << 4, b = ((2 * u + 1) ^ x) << 4;
 #pragma unroll
-      for (int m = 0; m < 4; ++m) {  // row 64 half + 8w + 2m + s2: swizzle term 2m + s2, scale held by lane 2 (8 half + 2m + s2) + u / 8
-        const int x = 2 * m + s2;
-        const uint32_t row_addr = v_rows + half * kVHalfBytes + x * 128;
-        const uint32_t a = ((2 * (u & 3)) ^ x) << 4, b = ((2 * (u & 3) + 1) ^ x) << 4;
+      for (int l = 0; l < 2; ++l) {
+        const uint32_t row_addr = v_rows + 4 * m * 128 + l * 2 * kChunk;
         if (kBf) {
-          const int pm = __shfl_sync(0xffffffffu, row_cur, 8 * half + x);
-          const uint8_t* src = PAIR_KN + (pm >= 0 ? static_cast<int64_t>(pm) * 1024 + 2 * col0 + u * 32 : 0);
+          const int pm = __shfl_sync(0xffffffffu, row_cur, 4 * m + r4);
+          const uint8_t* src = PAIR_KN + (pm >= 0 ? static_cast<int64_t>(pm) * 1024 + 2 * (col0 + l * 128 + line_off) : 0);
           cp_async_16(row_addr + a, src, pm >= 0 ? 16u : 0u);
           cp_async_16(row_addr + b, src + (pm >= 0 ? 16 : 0), pm >= 0 ? 16u : 0u);
         } else {
-          const float scale = __shfl_sync(0xffffffffu, ra.sc, 2 * (8 * half + x) + (u >> 3));
-          const uint4 v = ra.d[half][m];
-          sts_v4u(row_addr + (odd ? b : a), pair_dequant8(odd ? v.z : v.x, odd ? v.w : v.y, scale));
-          sts_v4u(row_addr + (odd ? a : b), pair_dequant8(odd ? v.x : v.z, odd ? v.y : v.w, scale));
+          const float scale = __shfl_sync(0xffffffffu, sc, 16 * l + 4 * m + r4);
+          const uint4 v = d[m][l];
+          sts_v4u(row_addr + a, pair_dequant8(v.x, v.y, scale));
+          sts_v4u(row_addr + b, pair_dequant8(v.z, v.w, scale));
         }
       }
-      if (kBf) asm volatile("cp.async.wait_all;" ::: "memory");
-      fence_proxy_async();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&ctl->vfull[half]));
-      if (vtid == 0 && half == 1) TLP(5, j);
     }
-    if (!ok) break;
-    if (j + 1 < ntiles) issue_loads(ra, row_n);
+    if (kBf) asm volatile("cp.async.wait_all;" ::: "memory");
+    fence_proxy_async();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(smem_u32(&ctl->vfull[q]));
+    if (vtid == 0) TLP(5, j);
+    if (j + 1 < ntiles) issue_loads(row_n);
     row_cur = row_n;
     row_n = pair_row(p, idx_a, entry_a);
-    idx_a = load_idx(j + 3);
-    entry_a = tc_table_entry(p, c.bi, idx_a);  // (the index was requested this iteration: one trip to L2 here, after the
-                                               // tile's stores, a whole tile before the next wait)
+    idx_a = idx_b;
+    entry_a = tc_table_entry(p, c.bi, idx_a);
+    idx_b = load_idx(j + 4);
   }
   if (!ok && lane == 0) {
     ctl->abort = 1;
@@ -927,15 +898,17 @@ sfa_pair_kernel(const __grid_constant__ SfaParams p) {
     mbar_init(smem_u32(&ctl->pfull), kPairSoftmaxWarps);
     mbar_init(smem_u32(&ctl->ppeer), 1);
     for (int b = 0; b < 2; ++b) {
-      mbar_init(smem_u32(&ctl->kfull[b]), kPairKWarps);
-      mbar_init(smem_u32(&ctl->vfull[b]), kPairVWarps);
-      mbar_init(smem_u32(&ctl->kfree[b]), 1);
-      mbar_init(smem_u32(&ctl->vfree[b]), 1);
       mbar_init(smem_u32(&ctl->sfull[b]), 1);
       mbar_init(smem_u32(&ctl->sread[b]), kPairSoftmaxWarps);
-      mbar_init(smem_u32(&ctl->kpeer[b]), 1);
-      mbar_init(smem_u32(&ctl->vpeer[b]), 1);
       mbar_init(smem_u32(&ctl->speer[b]), 1);
+      mbar_init(smem_u32(&ctl->kfull[b]), kPairKWarps / 2);
+      mbar_init(smem_u32(&ctl->kfree[b]), 1);
+      mbar_init(smem_u32(&ctl->kpeer[b]), 1);
+    }
+    for (int q = 0; q < 4; ++q) {
+      mbar_init(smem_u32(&ctl->vfull[q]), kPairVWarps / 4);
+      mbar_init(smem_u32(&ctl->vfree[q]), 1);
+      mbar_init(smem_u32(&ctl->vpeer[q]), 1);
     }
     ctl->abort = 0;
     fence_mbar_init();
@@ -976,9 +949,14 @@ sfa_pair_kernel(const __grid_constant__ SfaParams p) {
 #define PAIR_SETREG(x) asm volatile(x)
   if (warp < kPairSoftmaxWarp0) {
     PAIR_SETREG("setmaxnreg.dec.sync.aligned.u32 24;");
-    if (warp == 0 && crank == 0) pair_role_issue_qk(p, c);
-    else if (warp == 2 && crank == 0) pair_role_issue_pv(p, c);
-    else if (warp == 1 && crank == 1) pair_role_relay(p, c);
+    const bool usual = base == kPairUsualBase;
+    if (warp == 0 && crank == 0 && usual) pair_role_issue_qk<kPairUsualBase>(p, c);
+    else if (warp == 0 && crank == 0) pair_role_issue_qk<0>(p, c);
+    else if (warp == 2 && crank == 0 && usual) pair_role_issue_pv<kPairUsualBase>(p, c);
+    else if (warp == 2 && crank == 0) pair_role_issue_pv<0>(p, c);
+    else if (warp == 0) pair_role_relay<kRelayK>(p, c);
+    else if (warp == 2) pair_role_relay<kRelayV>(p, c);
+    else if (warp == 1 && crank == 1) pair_role_relay<kRelayP>(p, c);
     else pair_setup_sync(ctl);
   } else if (warp < kPairKWarp0) {
     PAIR_SETREG("setmaxnreg.inc.sync.aligned.u32 104;");
