@@ -15,7 +15,7 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB = PKG / "libpypto_b200.so"
 SOURCES = ["capi.cu", "li_score.cu", "topk_select.cu", "sfa_decode.cu", "sfa_pair.cu", "sfa_slice.cu", "prolog.cu", "prolog_gemm.cu",
-           "prolog_sgemm.cu"]
+           "prolog_sgemm.cu", "prolog_wide.cu"]
 HEADERS = [CSRC / "common.cuh", CSRC / "sfa_common.cuh", PKG.parent / "include" / "pypto_b200.h"]
 
 

@@ -392,16 +392,29 @@ int prolog_side_stream(int* device) {
   return PTO_OK;
 }
 
-// One weight-streaming product (prolog_sgemm.cu): out = x[t, k] . W[k, n] per problem of the batch.
-// kind 0: bf16 -> fp32 partials, 1: bf16 -> bf16, 2: int8 -> int32. Row pitches in bytes.
+// Up to this many token rows the weights are the large operand of every product and its M dimension (prolog_sgemm.cu,
+// prolog_gemm.cu); with more the token rows are (prolog_wide.cu).
+constexpr int kNarrowRows = 64;
+inline bool prolog_is_wide(int t) { return t > kNarrowRows; }
+
+// One bf16 product: out = x[t, k] . W[k, n] per problem of the batch. kind 0: fp32 partials, 1: bf16. Row pitches in bytes.
 int run_sgemm(int kind, const void* x, size_t x_pitch, const void* w, size_t w_pitch, int64_t w_rows, void* out, int t,
               int n, int k, int batch, int w_batch_rows, int x_batch_bytes, long long out_batch, long long ld_out,
               int splits, long long split_stride, int num_sms, int32_t* status, cudaStream_t stream, bool pdl = false) {
+  // (up to 128 rows the projections have more items of 128 columns than of 128 rows x 256 columns: 70 tokens 66 us a call
+  // against 71)
+  const bool wide = prolog_is_wide(t) && (kind != 0 || t > 128);
   alignas(64) CUtensorMap map_w, map_x;
-  int rc = make_bytes_map(&map_w, w, w_pitch, static_cast<uint64_t>(w_rows), w_pitch, kind == 2 ? 128 : 64);
+  int rc = make_bytes_map(&map_w, w, w_pitch, static_cast<uint64_t>(w_rows), w_pitch, 64);
   if (rc != PTO_OK) return rc;
-  rc = make_bytes_map(&map_x, x, x_pitch, static_cast<uint64_t>(t), x_pitch, static_cast<uint32_t>(pto::prolog_sgemm_rows(t)));
+  rc = make_bytes_map(&map_x, x, x_pitch, static_cast<uint64_t>(t), x_pitch,
+                      wide ? 128u : static_cast<uint32_t>(pto::prolog_sgemm_rows(t)));
   if (rc != PTO_OK) return rc;
+  if (wide) {
+    PTO_CUDA(pto::launch_prolog_wide(kind, &map_w, &map_x, out, t, n, k, batch, w_batch_rows, x_batch_bytes, out_batch, ld_out,
+                                     splits, split_stride, num_sms, status, stream, pdl));
+    return PTO_OK;
+  }
   PTO_CUDA(pto::launch_prolog_sgemm(kind, &map_w, &map_x, out, t, n, k, batch, w_batch_rows, x_batch_bytes, out_batch,
                                     ld_out, splits, split_stride, num_sms, status, stream, pdl));
   return PTO_OK;
@@ -420,6 +433,9 @@ constexpr int kXProjExtra = 576 + 128 + 64;  // columns after the q_lora ones: l
 // Rows of the int8 activation buffer: the resident-activation kernel's tensor map covers whole 16-row groups.
 inline int prolog_int8_rows(int t) { return t < 64 ? 64 : t; }
 
+// The quantised prolog takes the wide path also where the resident-activation kernel cannot take the query's width.
+inline bool prolog_quant_is_wide(int t, int q_lora) { return prolog_is_wide(t) || !pto::prolog_i8_gemm_supported(t, q_lora); }
+
 PrologWs prolog_ws(int t, int hidden, int q_lora) {
   PrologWs w{};
   size_t off = 0;
@@ -435,9 +451,14 @@ PrologWs prolog_ws(int t, int hidden, int q_lora) {
   w.xproj = take(w.splits * tt * (q_lora + kXProjExtra) * 4);  // fp32 [splits, t, q_lora | 576 | 128 | 64]
   w.q_norm = take(tp * q_lora);
   w.q_norm_scale = take(tt * 4);
-  w.qb_i32 = take(tp * 128 * 192 * 4);
-  w.q_b = take(tt * 128 * 192 * 2);
-  w.qi_i32 = take(tp * 64 * 128 * 4);
+  if (prolog_quant_is_wide(t, q_lora)) {
+    w.q_b = take(tt * 128 * 128 * 2);      // bf16 nope parts [t, 128, 128]
+    w.qi_i32 = take(tt * 64 * 128 * 2);    // bf16 indexer rows [t, 64, 128]
+  } else {
+    w.qb_i32 = take(tp * 128 * 192 * 4);
+    w.q_b = take(tt * 128 * 192 * 2);
+    w.qi_i32 = take(tp * 64 * 128 * 4);
+  }
   w.total = off;
   return w;
 }
@@ -818,27 +839,43 @@ int pto_mla_indexer_prolog_quant(const void* token_x, const void* w_dq, const in
   // the one before it drains (it waits before it reads)
   PTO_CUDA(pto::launch_prolog_qnorm_quant(qa, ld, splits, split_stride, gamma_cq, t, q_lora, eps_cq, q_norm, q_norm_scale,
                                           stream, /*pdl=*/true));
-  // int8 up-projections of the normalised query: one launch for both with the activations resident in shared
-  // memory when the token rows fit (decode), else one streaming product per weight over blocks of 256 tokens
   const int tp = prolog_int8_rows(t);
-  if (pto::prolog_i8_gemm_supported(t, q_lora)) {
-    alignas(64) CUtensorMap map_w0, map_w1, map_x;
+  if (prolog_quant_is_wide(t, q_lora)) {
+    // many token rows: one launch for both up-projections, dequantisation and rope in its epilogue; the indexer's Hadamard
+    // rotation on the side stream beside the absorbed query
+    alignas(64) CUtensorMap map_w0, map_w1, map_x, map_had, map_rows;
     rc = make_bytes_map(&map_w0, w_uqqr, 128 * 192, q_lora, 128 * 192, 128);
     if (rc != PTO_OK) return rc;
     rc = make_bytes_map(&map_w1, w_idx_qb, 64 * 128, q_lora, 64 * 128, 128);
     if (rc != PTO_OK) return rc;
-    rc = make_bytes_map(&map_x, q_norm, q_lora, tp, q_lora, static_cast<uint32_t>((t + 15) / 16 * 16));
+    rc = make_bytes_map(&map_x, q_norm, q_lora, t, q_lora, 128);
     if (rc != PTO_OK) return rc;
-    PTO_CUDA(pto::launch_prolog_i8_gemm(&map_w0, &map_w1, &map_x, qb_i32, 128 * 192, qi_i32, 64 * 128, q_lora, t,
-                                        di.num_sms, status, stream, /*pdl=*/true));
-  } else {
-    rc = run_sgemm(2, q_norm, q_lora, w_uqqr, 128 * 192, q_lora, qb_i32, t, 128 * 192, q_lora, 1, 0, 0, 0, 128 * 192, 1, 0,
-                   di.num_sms, status, stream, /*pdl=*/true);
+    rc = make_bytes_map(&map_had, hadamard_q, 256, 128, 256, 64);
     if (rc != PTO_OK) return rc;
-    rc = run_sgemm(2, q_norm, q_lora, w_idx_qb, 64 * 128, q_lora, qi_i32, t, 64 * 128, q_lora, 1, 0, 0, 0, 64 * 128, 1, 0,
-                   di.num_sms, status, stream, /*pdl=*/true);
+    rc = make_bytes_map(&map_rows, qi_i32, 256, static_cast<uint64_t>(t) * 64, 256, 128);
     if (rc != PTO_OK) return rc;
+    PTO_CUDA(pto::launch_prolog_wide_up(&map_w0, &map_w1, &map_x, t, q_lora, q_norm_scale, w_qb_scale, w_idx_qb_scale, cos,
+                                        sin, q_b, query_rope_out, qi_i32, di.num_sms, status, stream, /*pdl=*/true));
+    PTO_CUDA(cudaEventRecord(ev[1], stream));
+    PTO_CUDA(cudaStreamWaitEvent(side, ev[1], 0));
+    PTO_CUDA(pto::launch_prolog_wide_hadamard(&map_had, &map_rows, t * 64, q_int8_out, q_scale_out, di.num_sms, status, side));
+    PTO_CUDA(cudaEventRecord(ev[2], side));
+    rc = run_sgemm(1, q_b, 128 * 128 * 2, w_uk, 512 * 2, 128 * 128, query_nope_out, t, 512, 128, 128, 128, 128 * 2, 512,
+                   128 * 512, 1, 0, di.num_sms, status, stream, /*pdl=*/true);
+    if (rc != PTO_OK) return rc;
+    PTO_CUDA(cudaStreamWaitEvent(stream, ev[2], 0));
+    return PTO_OK;
   }
+  // few: both int8 up-projections of the normalised query in one launch, the activations resident in shared memory
+  alignas(64) CUtensorMap map_w0, map_w1, map_x;
+  rc = make_bytes_map(&map_w0, w_uqqr, 128 * 192, q_lora, 128 * 192, 128);
+  if (rc != PTO_OK) return rc;
+  rc = make_bytes_map(&map_w1, w_idx_qb, 64 * 128, q_lora, 64 * 128, 128);
+  if (rc != PTO_OK) return rc;
+  rc = make_bytes_map(&map_x, q_norm, q_lora, tp, q_lora, static_cast<uint32_t>((t + 15) / 16 * 16));
+  if (rc != PTO_OK) return rc;
+  PTO_CUDA(pto::launch_prolog_i8_gemm(&map_w0, &map_w1, &map_x, qb_i32, 128 * 192, qi_i32, 64 * 128, q_lora, t, di.num_sms,
+                                      status, stream, /*pdl=*/true));
   // the indexer-query kernel joins the side stream; the attention query finishes on the caller's
   PTO_CUDA(cudaEventRecord(ev[1], stream));
   PTO_CUDA(cudaStreamWaitEvent(side, ev[1], 0));

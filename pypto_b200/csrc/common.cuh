@@ -397,6 +397,16 @@ cudaError_t launch_prolog_sgemm(int kind, const void* tmap_w, const void* tmap_x
                                 int batch, int w_batch_rows, int x_batch_bytes, long long out_batch, long long ld_out,
                                 int splits, long long split_stride, int num_sms, int32_t* status, cudaStream_t stream,
                                 bool pdl = false);
+// the same products for many token rows, with what follows them fused (prolog_wide.cu)
+cudaError_t launch_prolog_wide(int kind, const void* tmap_w, const void* tmap_x, void* out, int t, int n, int k, int batch,
+                               int w_batch_rows, int x_batch_bytes, long long out_batch, long long ld_out, int splits,
+                               long long split_stride, int num_sms, int32_t* status, cudaStream_t stream, bool pdl = false);
+cudaError_t launch_prolog_wide_up(const void* tmap_w, const void* tmap_w_idx, const void* tmap_x, int t, int k,
+                                  const float* row_scale, const float* col_scale, const float* col_scale_idx, const void* cos,
+                                  const void* sin, void* q_nope, void* q_rope, void* idx_rows, int num_sms, int32_t* status,
+                                  cudaStream_t stream, bool pdl = false);
+cudaError_t launch_prolog_wide_hadamard(const void* tmap_had, const void* tmap_rows, int n_rows, int8_t* q_int8,
+                                        void* q_scale, int num_sms, int32_t* status, cudaStream_t stream);
 cudaError_t launch_kv_pack_rows(const int8_t* kv, const void* kr, const float* sc, int64_t rows, int8_t* packed,
                                 int num_sms, cudaStream_t stream);
 cudaError_t launch_prolog_idxq(const int32_t* qi_i32, const float* q_norm_scale, const float* w_scale, const void* cos,

@@ -1,11 +1,10 @@
-// Weight-streaming products of the prolog on tcgen05, one kernel for its three shapes:
+// Weight-streaming bf16 products of the prologs on tcgen05 for few token rows (prolog_wide.cu takes many), two shapes:
 //
 //   * the projections of the hidden state, out[t, N] (fp32) = x[t, K] (bf16) . W[K, N] (bf16), K = 7168 split over
 //     CTAs (every split writes its own fp32 partial; the kernels that read the result add the partials in a fixed
 //     order, so the sum does not depend on which CTA finished first);
-//   * the absorbed query, per head h: out[t, h, 512] (bf16) = q_b[t, h, 0:128] (bf16) . w_uk[h] [128, 512] (bf16);
-//   * the int8 up-projections for more token rows than the resident-activation kernel takes,
-//     out[t, N] (int32) = x[t, K] (int8) . W[K, N] (int8).
+//   * the absorbed query, per head h: out[t, h, 512] (bf16) = q_b[t, h, 0:128] (bf16) . w_uk[h] [128, 512] (bf16), and the
+//     bf16 up-projections of the non-quantised prolog.
 //
 // (reference: examples/models/deepseek_v32_exp/mla_prolog_quant_impl.py:502-707,
 // lightning_indexer_prolog_quant_impl.py:325-504.)
@@ -13,8 +12,7 @@
 // The weights are the large operand, so the product is taken transposed, D[n, tok] = W^T[n, k] . x^T[k, tok]:
 // 128 weight columns are the M dimension of the MMA, up to 256 token rows its N dimension. W is row-major [K, N],
 // i.e. an MN-major A operand, which TMA delivers in the canonical 128-byte-swizzled layout (box of k-rows x 128
-// bytes of n). A ring stage holds one 16 KB weight tile (128 k x 128 n int8, or 64 k x 128 n bf16 as two 64-column
-// boxes) and the matching [token rows x 128 bytes] slice of x; rows and columns outside the tensors read as zeros.
+// bytes of n). A ring stage holds one 16 KB weight tile (64 k x 128 n as two 64-column boxes) and the matching [token rows x 128 bytes] slice of x; rows and columns outside the tensors read as zeros.
 // Work items (token block, problem of the batch, 128-column tile, K split) are dealt round-robin to persistent CTAs.
 // Roles: warp 0 TMA producer, warp 1 MMA issuer, warps 2-5 epilogue (TMEM lane quarter = warp & 3); two
 // accumulators in tensor memory. Every wait is bounded and reports PTO_ST_WAIT_EXPIRED.
@@ -33,7 +31,7 @@ constexpr int kSRingBytes = 192 * 1024;
 constexpr int kSThreads = 192;
 constexpr int kSMaxRows = 256;        // token rows per block (MMA N)
 
-enum { kOutF32 = 0, kOutBf16 = 1, kOutI32 = 2 };
+enum { kOutF32 = 0, kOutBf16 = 1 };
 
 struct SCtl {
   uint64_t full[kSMaxStages];
@@ -48,7 +46,7 @@ constexpr int kSSmemMax = kSRingBytes + sizeof(SCtl) + 1024;
 
 struct SGemmParams {
   int n_tiles;            // 128-column tiles per problem
-  int chunks;             // K chunks in all (64 bf16 / 128 int8 per chunk)
+  int chunks;             // K chunks of 64 in all
   int per_split;          // chunks per split
   int splits;
   int batch;              // problems (heads), >= 1
@@ -82,7 +80,7 @@ __device__ __forceinline__ SItem s_item(const SGemmParams& p, int item) {
   return it;
 }
 
-template <bool kI8, int kOut>
+template <int kOut>
 __global__ void __launch_bounds__(kSThreads, 1)
 prolog_sgemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                     const SGemmParams p) {
@@ -94,7 +92,7 @@ prolog_sgemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n_items = p.tok_blocks * p.batch * p.n_tiles * p.splits;
-  constexpr int kChunkK = kI8 ? 128 : 64;  // k rows per weight tile
+  constexpr int kChunkK = 64;  // k rows per weight tile
   const uint32_t x_bytes = static_cast<uint32_t>(p.t_pad) * 128u;
 
   if (tid == 0) {
@@ -147,12 +145,8 @@ prolog_sgemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
           const uint32_t dst = base + s * p.stage_bytes;
           const int krow = w.b * p.w_batch_rows + (k0 + c) * kChunkK;
           mbar_arrive_expect_tx(bar, kSWBytes + x_bytes);
-          if (kI8) {
-            tma_load_2d_hint(dst, &tmap_w, n0, krow, bar, w_policy);
-          } else {
-            tma_load_2d_hint(dst, &tmap_w, n0 * 2, krow, bar, w_policy);
-            tma_load_2d_hint(dst + kSWBytes / 2, &tmap_w, n0 * 2 + 128, krow, bar, w_policy);
-          }
+          tma_load_2d_hint(dst, &tmap_w, n0 * 2, krow, bar, w_policy);
+          tma_load_2d_hint(dst + kSWBytes / 2, &tmap_w, n0 * 2 + 128, krow, bar, w_policy);
           tma_load_2d(dst + kSWBytes, &tmap_x, w.b * p.x_batch_bytes + (k0 + c) * 128, w.tb * p.t_pad, bar);
         }
       }
@@ -164,8 +158,7 @@ prolog_sgemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     if (lane == 0) {
-      const uint32_t idesc = kI8 ? umma_idesc(kCFmtS32, kABFmtS8, kABFmtS8, 1, 0, kSTileN, static_cast<uint32_t>(p.t_pad))
-                                 : umma_idesc(kCFmtF32, kABFmtBF16, kABFmtBF16, 1, 0, kSTileN, static_cast<uint32_t>(p.t_pad));
+      const uint32_t idesc = umma_idesc(kCFmtF32, kABFmtBF16, kABFmtBF16, 1, 0, kSTileN, static_cast<uint32_t>(p.t_pad));
       bool ok = true;
       uint32_t it = 0, ti = 0;
       for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++ti) {
@@ -187,12 +180,8 @@ prolog_sgemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
           const uint64_t b_desc = umma_desc_kmajor_sw128(a + kSWBytes);
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            if (kI8) {  // K = 32 per instruction: 32 k-rows of A (4 KB), 32 bytes along x's rows
-              mma_i8_ss(d, desc_mnmajor_sw128(a + j * 4096, 16, 1024), b_desc + 2 * j, idesc, (c | j) != 0 ? 1u : 0u);
-            } else {    // K = 16: 16 k-rows of each 64-column half (2 KB), the halves 8 KB apart
-              mma_f16_ss(d, desc_mnmajor_sw128(a + j * 2048, kSWBytes / 2, 1024), b_desc + 2 * j, idesc,
-                         (c | j) != 0 ? 1u : 0u);
-            }
+            // K = 16: 16 k-rows of each 64-column half (2 KB), the halves 8 KB apart
+            mma_f16_ss(d, desc_mnmajor_sw128(a + j * 2048, kSWBytes / 2, 1024), b_desc + 2 * j, idesc, (c | j) != 0 ? 1u : 0u);
           }
           tc_commit(smem_u32(&ctl->empty[s]));
         }
@@ -231,7 +220,6 @@ prolog_sgemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             const long long at = static_cast<long long>(tok) * p.ld_out + col;
             if (kOut == kOutF32) reinterpret_cast<float*>(p.out)[at] = __uint_as_float(v[e]);
             if (kOut == kOutBf16) reinterpret_cast<__nv_bfloat16*>(p.out)[at] = __float2bfloat16_rn(__uint_as_float(v[e]));
-            if (kOut == kOutI32) reinterpret_cast<int32_t*>(p.out)[at] = static_cast<int32_t>(v[e]);
           }
         }
       }
@@ -258,10 +246,10 @@ prolog_sgemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
   }
 }
 
-template <bool kI8, int kOut>
+template <int kOut>
 cudaError_t launch_one(const void* tmap_w, const void* tmap_x, const SGemmParams& p, int grid, cudaStream_t stream,
                        bool pdl) {
-  auto kernel = prolog_sgemm_kernel<kI8, kOut>;
+  auto kernel = prolog_sgemm_kernel<kOut>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSSmemMax);
   if (e != cudaSuccess) return e;
   const size_t smem = static_cast<size_t>(p.n_stages) * p.stage_bytes + sizeof(SCtl) + 1024;
@@ -295,17 +283,15 @@ int prolog_sgemm_splits(int t, int n, int k, int num_sms) {
   }
 }
 
-// kind: 0 = bf16 x bf16 -> fp32 (with `splits` partials `split_stride` elements apart), 1 = bf16 x bf16 -> bf16,
-// 2 = int8 x int8 -> int32. The tensor maps are byte matrices: W with a [k rows x 128 B] box (64 rows for bf16, 128
-// for int8), x with a [prolog_sgemm_rows(t) x 128 B] box.
+// kind: 0 = bf16 x bf16 -> fp32 (with `splits` partials `split_stride` elements apart), 1 = bf16 x bf16 -> bf16. The
+// tensor maps are byte matrices: W with a [64 rows x 128 B] box, x with a [prolog_sgemm_rows(t) x 128 B] box.
 cudaError_t launch_prolog_sgemm(int kind, const void* tmap_w, const void* tmap_x, void* out, int t, int n, int k,
                                 int batch, int w_batch_rows, int x_batch_bytes, long long out_batch, long long ld_out,
                                 int splits, long long split_stride, int num_sms, int32_t* status, cudaStream_t stream,
                                 bool pdl) {
   SGemmParams p{};
-  const bool i8 = kind == kOutI32;
   p.n_tiles = (n + kSTileN - 1) / kSTileN;
-  p.chunks = i8 ? (k + 127) / 128 : (k + 63) / 64;
+  p.chunks = (k + 63) / 64;
   p.splits = splits < 1 ? 1 : splits;
   p.per_split = (p.chunks + p.splits - 1) / p.splits;
   if ((p.chunks + p.per_split - 1) / p.per_split != p.splits) return cudaErrorInvalidValue;  // a split without work
@@ -338,9 +324,8 @@ cudaError_t launch_prolog_sgemm(int kind, const void* tmap_w, const void* tmap_x
   uint32_t cols = 32;
   while (cols < accs * static_cast<uint32_t>(p.t_pad)) cols <<= 1;
   p.tmem_cols = cols;
-  if (kind == kOutF32) return launch_one<false, kOutF32>(tmap_w, tmap_x, p, grid, stream, pdl);
-  if (kind == kOutBf16) return launch_one<false, kOutBf16>(tmap_w, tmap_x, p, grid, stream, pdl);
-  return launch_one<true, kOutI32>(tmap_w, tmap_x, p, grid, stream, pdl);
+  if (kind == kOutF32) return launch_one<kOutF32>(tmap_w, tmap_x, p, grid, stream, pdl);
+  return launch_one<kOutBf16>(tmap_w, tmap_x, p, grid, stream, pdl);
 }
 
 }  // namespace pto

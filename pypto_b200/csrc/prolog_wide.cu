@@ -1,0 +1,541 @@
+// Products of the prologs for many token rows (prompt chunks): out[tok, n] = x[tok, k] . W[k, n] on tcgen05 with the token
+// rows as the M dimension, and what follows a product fused into its epilogue:
+//
+//   kWideF32    fp32 K-split partials (projections of the hidden state)
+//   kWideBf16   bf16 rows (absorbed query per head; up-projections of the non-quantised prolog)
+//   kWideUp     both int8 up-projections of the normalised query in one launch, int32 -> bf16 dequantisation. Attention: the
+//               128-wide nope part of a head goes to the scratch the absorbed product reads, the 64-wide tail is rotated
+//               and goes to the output. Indexer: a head's first 64 dims are rotated, the rows go to the Hadamard product
+//   kWideHad    indexer rows . Hadamard matrix, bf16 rounding, per-row int8 quantisation (rows = tokens x 64 heads)
+//
+// (reference: examples/models/deepseek_v32_exp/mla_prolog_quant_impl.py:502-707,
+// lightning_indexer_prolog_quant_impl.py:325-504; arithmetic and roundings as in prolog.cu.)
+//
+// Why tokens as M: a TMEM lane is a token row, so a thread of the epilogue holds neighbouring columns of one row. Row
+// scales are per-lane constants and a rope pair or a head's maximum lies inside a thread. A warp passes 128 bytes of each
+// of its 32 rows through shared memory and writes whole lines (32-byte stores straight from the lanes, each to a row of
+// its own, reached L2 as three times their sectors: 64 -> 41 us for the absorbed query of 1000 tokens). With the weight columns as lanes (prolog_sgemm.cu, made for few rows) every store instruction writes 64
+// bytes of one row and everything between the products needs a kernel of its own. 1000 tokens, one kernel each, before
+// -> after: dequantisation 33 us -> fused; indexer query 118 us (Hadamard on CUDA cores) -> product of 16 us.
+//
+// One CTA per SM, persistent. A ring stage is one 128-byte-wide K chunk: x tile [128 rows] (16 KB, K-major) and W tile
+// [chunk rows x kN columns] (32 KB at kN = 256, MN-major as it lies in memory), both 128-byte swizzled by TMA; rows and
+// columns outside the tensors read as zeros. Two accumulators of kN columns, one per epilogue group of four warps, so
+// that one tile is stored while the next is multiplied. Items run over token blocks first: the CTAs that are at work at
+// the same time read the same weight columns from L2.
+// Roles: warp 0 TMA, warp 1 MMA, warps 2-5 / 6-9 epilogue. All waits are bounded.
+#include <cuda.h>
+
+#include <initializer_list>
+
+#include "sfa_common.cuh"
+
+namespace pto {
+
+namespace {
+
+constexpr int kWRows = 128;                  // token rows per tile (MMA M)
+constexpr int kWXBytes = kWRows * 128;
+constexpr int kWStages = 4;
+constexpr int kWThreads = 320;
+constexpr int kWStaging = 8 * 4096;           // per epilogue warp: 128 bytes of 32 rows
+constexpr int kHeadQ = 192, kHeadNope = 128;  // widths of an attention head of the up-projection
+
+enum { kWideF32 = 0, kWideBf16 = 1, kWideUp = 2, kWideHad = 3 };
+
+struct WideCtl {
+  uint64_t full[kWStages];
+  uint64_t empty[kWStages];
+  uint64_t acc_full[2];
+  uint64_t acc_empty[2];
+  uint32_t tmem_base;
+  int abort;
+};
+
+struct WideParams {
+  int t;                  // rows of x
+  int n;                  // valid output columns per problem
+  int n_tiles;            // kN-column tiles per problem
+  int chunks, per_split, splits;
+  int batch;              // problems (heads)
+  int row_blocks;
+  int w_batch_rows;       // rows of W between problems
+  int x_batch_bytes;      // bytes along a row of x between problems
+  long long out_batch;    // output elements between problems
+  long long ld_out;       // output elements between rows
+  long long split_stride;
+  int idx_tiles;          // kWideUp: the first tiles are the indexer's (second tensor map of W), the others the attention's
+  void* out;              // kWideUp: nope scratch bf16 [t, 128, 128]; kWideHad: int8 rows
+  void* out2;             // kWideUp: query_rope [t, 128, 64]; kWideHad: fp16 scale per row
+  void* out_idx;          // kWideUp: indexer rows bf16 [t, 64, 128]
+  const float* row_scale; // kWideUp: per token
+  const float* col_scale; // per column of the attention's product
+  const float* col_scale_idx;
+  const __nv_bfloat16* cos;  // [t, 64]
+  const __nv_bfloat16* sin;
+  int aligned;            // everything the epilogue touches lies on 16-byte boundaries: wide accesses, else single elements
+  int32_t* status;
+};
+
+template <bool kI8, int kN>
+struct WideCfg {
+  static constexpr int kChunkK = kI8 ? 128 : 64;     // k per stage: 128 bytes of a row of x
+  static constexpr int kGroup = kI8 ? 128 : 64;      // columns per 128-byte box of W
+  static constexpr int kBoxBytes = kChunkK * 128;
+  static constexpr int kWBytes = kN / kGroup * kBoxBytes;
+  static constexpr int kStage = kWXBytes + kWBytes;
+  static constexpr int kSmem = kWStages * kStage + kWStaging + sizeof(WideCtl) + 1024;
+  static_assert(kSmem <= 232448, "exceeds the 227 KB of shared memory a CTA may use");
+  static constexpr uint32_t kTmemCols = 2 * kN;
+};
+
+struct WideItem {
+  int rb, b, tile, split;
+};
+__device__ __forceinline__ WideItem wide_item(const WideParams& p, int item) {
+  WideItem it;
+  it.rb = item % p.row_blocks;
+  int r = item / p.row_blocks;
+  it.split = r % p.splits;
+  r /= p.splits;
+  it.tile = r % p.n_tiles;
+  it.b = r / p.n_tiles;
+  return it;
+}
+
+__device__ __forceinline__ float wide_bf16_round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
+
+// This warp's rows: lane l holds 128 bytes of row l. They go to `dst` + l * `pitch` through the warp's staging area, four
+// whole lines per store instruction. `n_rows`: rows that exist; `n_bytes`: bytes that exist of each (a multiple of 16).
+__device__ __forceinline__ void store_rows(uint32_t stage, const uint32_t (&w)[32], uint8_t* dst, int64_t pitch, int n_rows,
+                                           int n_bytes, int aligned) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    sts_v4u(stage + lane * 128 + ((i ^ (lane & 7)) << 4), make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]));
+  }
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = 4 * i + (lane >> 3), u = lane & 7;
+    const uint4 v = lds_v4u(stage + r * 128 + ((u ^ (r & 7)) << 4));
+    if (r < n_rows && u * 16 < n_bytes) {
+      uint8_t* at = dst + r * pitch + u * 16;
+      if (aligned) {
+        *reinterpret_cast<uint4*>(at) = v;
+      } else {
+        const uint32_t x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int e = 0; e < 16; ++e) at[e] = static_cast<uint8_t>(x[e >> 2] >> (8 * (e & 3)));
+      }
+    }
+  }
+  __syncwarp();
+}
+__device__ __forceinline__ void pack_bf16_64(const float (&v)[64], uint32_t (&w)[32]) {
+#pragma unroll
+  for (int e = 0; e < 32; ++e) w[e] = pack_bf16x2(v[2 * e], v[2 * e + 1]);
+}
+
+// a token's 64 cosines or sines, eight at a time
+__device__ __forceinline__ void load_bf16_8(const __nv_bfloat16* p, float (&v)[8], int aligned) {
+  if (!aligned) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = __bfloat162float(p[e]);
+    return;
+  }
+  const uint4 w = __ldg(reinterpret_cast<const uint4*>(p));
+  const uint32_t x[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    v[2 * e] = __uint_as_float(x[e] << 16);
+    v[2 * e + 1] = __uint_as_float(x[e] & 0xffff0000u);
+  }
+}
+
+// int32 accumulators of 64 columns -> bf16-rounded products with the row and column scales
+__device__ __forceinline__ void wide_dequant_64(uint32_t taddr, float rs, const float* col_scale, float (&v)[64], int aligned) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    uint32_t r[32];
+    tmem_ld_32x32b_x32(taddr + 32 * h, r);
+    tc_wait_ld();
+#pragma unroll
+    for (int c = 0; c < 32; c += 4) {
+      const float* sp = col_scale + 32 * h + c;
+      const float4 ws = aligned ? __ldg(reinterpret_cast<const float4*>(sp)) : make_float4(sp[0], sp[1], sp[2], sp[3]);
+      v[32 * h + c] = wide_bf16_round(__fmul_rn(__fmul_rn(static_cast<float>(static_cast<int>(r[c])), rs), ws.x));
+      v[32 * h + c + 1] = wide_bf16_round(__fmul_rn(__fmul_rn(static_cast<float>(static_cast<int>(r[c + 1])), rs), ws.y));
+      v[32 * h + c + 2] = wide_bf16_round(__fmul_rn(__fmul_rn(static_cast<float>(static_cast<int>(r[c + 2])), rs), ws.z));
+      v[32 * h + c + 3] = wide_bf16_round(__fmul_rn(__fmul_rn(static_cast<float>(static_cast<int>(r[c + 3])), rs), ws.w));
+    }
+  }
+}
+
+// One tile's rows out of tensor memory: this warp's 32 rows start at `row0`, `taddr` is its lanes of the tile's accumulator.
+template <int kEpi, int kN>
+__device__ __forceinline__ void wide_epilogue(const WideParams& p, const WideItem& w, uint32_t taddr, int row0, uint32_t stage) {
+  const int n_rows = p.t - row0;                 // (may be more than 32, or none)
+  const int row = min(row0 + static_cast<int>(threadIdx.x & 31), p.t - 1);
+  const int n0 = w.tile * kN;
+  if (n_rows <= 0) return;
+  if constexpr (kEpi == kWideF32 || kEpi == kWideBf16) {
+    constexpr int kEl = kEpi == kWideF32 ? 4 : 2;
+    constexpr int kCols = 128 / kEl;
+    uint8_t* dst = reinterpret_cast<uint8_t*>(p.out) + (static_cast<long long>(row0) * p.ld_out + static_cast<long long>(w.b) * p.out_batch +
+                   n0 + static_cast<long long>(w.split) * p.split_stride) * kEl;
+#pragma unroll 1
+    for (int c = 0; c < kN; c += kCols) {
+      if (n0 + c >= p.n) break;  // (uniform)
+      uint32_t o[32];
+      if constexpr (kEpi == kWideF32) {
+        tmem_ld_32x32b_x32(taddr + c, o);
+        tc_wait_ld();
+      } else {
+        uint32_t r0[32], r1[32];
+        tmem_ld_32x32b_x32(taddr + c, r0);
+        tmem_ld_32x32b_x32(taddr + c + 32, r1);
+        tc_wait_ld();
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+          o[e] = pack_bf16x2(__uint_as_float(r0[2 * e]), __uint_as_float(r0[2 * e + 1]));
+          o[16 + e] = pack_bf16x2(__uint_as_float(r1[2 * e]), __uint_as_float(r1[2 * e + 1]));
+        }
+      }
+      // (n is a multiple of 16, so a cut-off piece ends on a 16-byte boundary)
+      store_rows(stage, o, dst + c * kEl, p.ld_out * kEl, n_rows, min(128, (p.n - n0 - c) * kEl), p.aligned);
+    }
+  } else if (kEpi == kWideUp && w.tile >= p.idx_tiles) {
+    const float rs = __ldg(p.row_scale + row);
+    const int n0 = (w.tile - p.idx_tiles) * kN;
+#pragma unroll 1
+    for (int c = 0; c < kN; c += 64) {  // a 64-column group is the low or high half of a head's nope part or its rope tail
+      const int col = n0 + c;
+      const int head = col / kHeadQ, part = (col % kHeadQ) >> 6;
+      float v[64];
+      uint32_t o[32];
+      wide_dequant_64(taddr + c, rs, p.col_scale + col, v, p.aligned);
+      if (part < 2) {
+        pack_bf16_64(v, o);
+        store_rows(stage, o, reinterpret_cast<uint8_t*>(p.out) + ((static_cast<int64_t>(row0) * 128 + head) * kHeadNope + 64 * part) * 2,
+                   128 * kHeadNope * 2, n_rows, 128, p.aligned);
+      } else {
+        // de-interleaved layout: outputs 0-31 from the even dims, 32-63 from the odd ones; rotate_half = (-second, first)
+#pragma unroll
+        for (int j0 = 0; j0 < 64; j0 += 8) {
+          float cs[8], sn[8], x[8];
+          load_bf16_8(p.cos + static_cast<int64_t>(row) * 64 + j0, cs, p.aligned);
+          load_bf16_8(p.sin + static_cast<int64_t>(row) * 64 + j0, sn, p.aligned);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const int j = (j0 + e) & 31;
+            const float even = v[2 * j], odd = v[2 * j + 1];
+            x[e] = __fadd_rn(__fmul_rn(j0 < 32 ? even : odd, cs[e]), __fmul_rn(j0 < 32 ? -odd : even, sn[e]));
+          }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) o[j0 / 2 + e] = pack_bf16x2(x[2 * e], x[2 * e + 1]);
+        }
+        store_rows(stage, o, reinterpret_cast<uint8_t*>(p.out2) + (static_cast<int64_t>(row0) * 128 + head) * 128, 128 * 128, n_rows,
+                   128, p.aligned);
+      }
+    }
+  } else if (kEpi == kWideUp) {
+    const float rs = __ldg(p.row_scale + row);
+#pragma unroll 1
+    for (int c = 0; c < kN; c += 64) {
+      const int col = n0 + c;
+      float v[64];
+      uint32_t o[32];
+      wide_dequant_64(taddr + c, rs, p.col_scale_idx + col, v, p.aligned);
+      if ((col & 64) != 0) {
+        pack_bf16_64(v, o);
+      } else {  // rope on the head's first 64 dims: halves, no de-interleave
+#pragma unroll
+        for (int j0 = 0; j0 < 64; j0 += 8) {
+          float cs[8], sn[8], x[8];
+          load_bf16_8(p.cos + static_cast<int64_t>(row) * 64 + j0, cs, p.aligned);
+          load_bf16_8(p.sin + static_cast<int64_t>(row) * 64 + j0, sn, p.aligned);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const int j = j0 + e;
+            const float rot = j < 32 ? -v[(j + 32) & 63] : v[(j - 32) & 63];
+            x[e] = __fadd_rn(__fmul_rn(v[j], cs[e]), __fmul_rn(rot, sn[e]));
+          }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) o[j0 / 2 + e] = pack_bf16x2(x[2 * e], x[2 * e + 1]);
+        }
+      }
+      store_rows(stage, o, reinterpret_cast<uint8_t*>(p.out_idx) + (static_cast<int64_t>(row0) * 64 * 128 + col) * 2, 64 * 128 * 2,
+                 n_rows, 128, p.aligned);
+    }
+  } else {  // kWideHad: two readings of the row's 128 accumulators, one for the maximum, one to quantise
+    static_assert(kEpi != kWideHad || kN == 128, "a Hadamard row is 128 wide");
+    float amax = 0.f;
+#pragma unroll 1
+    for (int c = 0; c < kN; c += 32) {
+      uint32_t r[32];
+      tmem_ld_32x32b_x32(taddr + c, r);
+      tc_wait_ld();
+#pragma unroll
+      for (int e = 0; e < 32; ++e) amax = fmaxf(amax, fabsf(wide_bf16_round(__uint_as_float(r[e]))));
+    }
+    const float sq = __fdiv_rn(127.0f, amax);
+    uint32_t o[32];
+#pragma unroll
+    for (int c = 0; c < kN; c += 32) {
+      uint32_t r[32];
+      tmem_ld_32x32b_x32(taddr + c, r);
+      tc_wait_ld();
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        uint32_t word = 0;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int q = static_cast<int8_t>(__float2int_rn(__fmul_rn(wide_bf16_round(__uint_as_float(r[4 * u + e])), sq)));
+          word |= (static_cast<uint32_t>(q) & 0xffu) << (8 * e);
+        }
+        o[c / 4 + u] = word;
+      }
+    }
+    store_rows(stage, o, reinterpret_cast<uint8_t*>(p.out) + static_cast<int64_t>(row0) * 128, 128, n_rows, 128, p.aligned);
+    if (static_cast<int>(threadIdx.x & 31) < n_rows) reinterpret_cast<__half*>(p.out2)[row] = __float2half_rn(__fdiv_rn(1.0f, sq));
+  }
+}
+
+template <bool kI8, int kEpi, int kN>
+__global__ void __launch_bounds__(kWThreads, 1)
+prolog_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_w_idx,
+                   const __grid_constant__ CUtensorMap tmap_x, const WideParams p) {
+  using Cfg = WideCfg<kI8, kN>;
+  extern __shared__ uint8_t wide_smem_raw[];
+  const uint32_t raw = smem_u32(wide_smem_raw);
+  const uint32_t base = (raw + 1023u) & ~1023u;
+  WideCtl* ctl = reinterpret_cast<WideCtl*>(wide_smem_raw + (base - raw) + kWStages * Cfg::kStage + kWStaging);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int n_items = p.row_blocks * p.batch * p.n_tiles * p.splits;
+
+  if (tid == 0) {
+    for (int i = 0; i < kWStages; ++i) {
+      mbar_init(smem_u32(&ctl->full[i]), 1);
+      mbar_init(smem_u32(&ctl->empty[i]), 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(smem_u32(&ctl->acc_full[i]), 1);
+      mbar_init(smem_u32(&ctl->acc_empty[i]), 4);
+    }
+    ctl->abort = 0;
+    fence_mbar_init();
+    fence_proxy_async();
+    tma_prefetch_desc(&tmap_w);
+    if (kEpi == kWideUp) tma_prefetch_desc(&tmap_w_idx);
+    tma_prefetch_desc(&tmap_x);
+  }
+  if (warp == 1) {
+    tmem_alloc(smem_u32(&ctl->tmem_base), Cfg::kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = ctl->tmem_base;
+  pdl_wait();  // the set-up above overlaps the tail of the kernel before this one
+  if (tid == 0) pdl_trigger();
+
+  if (warp == 0) {
+    // ---------------- producer ----------------
+    bool ok = true;
+    uint32_t it = 0;
+    for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+      const WideItem w = wide_item(p, item);
+      const int k0 = w.split * p.per_split;
+      const int kn = min(p.per_split, p.chunks - k0);
+      const bool idx = kEpi == kWideUp && w.tile < p.idx_tiles;
+      const CUtensorMap* tm = idx ? &tmap_w_idx : &tmap_w;
+      const int col = (kEpi == kWideUp && !idx ? w.tile - p.idx_tiles : w.tile) * kN * (kI8 ? 1 : 2);  // bytes
+      for (int c = 0; c < kn; ++c, ++it) {
+        const uint32_t s = it % kWStages;
+        if (it >= kWStages) ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->empty[s]), ((it / kWStages) - 1) & 1));
+        if (!ok) break;
+        if (elect_one()) {
+          const uint32_t bar = smem_u32(&ctl->full[s]);
+          const uint32_t dst = base + s * Cfg::kStage;
+          const int krow = w.b * p.w_batch_rows + (k0 + c) * Cfg::kChunkK;
+          mbar_arrive_expect_tx(bar, Cfg::kStage);
+          tma_load_2d(dst, &tmap_x, w.b * p.x_batch_bytes + (k0 + c) * 128, w.rb * kWRows, bar);
+#pragma unroll
+          for (int g = 0; g < kN / Cfg::kGroup; ++g) {
+            tma_load_2d(dst + kWXBytes + g * Cfg::kBoxBytes, tm, col + g * 128, krow, bar);
+          }
+        }
+        __syncwarp();
+      }
+    }
+    if (!ok && lane == 0) {
+      ctl->abort = 1;
+      set_status(p.status, PTO_ST_WAIT_EXPIRED, blockIdx.x, 80);
+    }
+  } else if (warp == 1) {
+    // ---------------- MMA issuer ----------------
+    constexpr uint32_t idesc = kI8 ? umma_idesc(kCFmtS32, kABFmtS8, kABFmtS8, 0, 1, kWRows, kN)
+                                   : umma_idesc(kCFmtF32, kABFmtBF16, kABFmtBF16, 0, 1, kWRows, kN);
+    bool ok = true;
+    uint32_t it = 0, ti = 0;
+    for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++ti) {
+      const WideItem w = wide_item(p, item);
+      const int kn = min(p.per_split, p.chunks - w.split * p.per_split);
+      const uint32_t acc = ti & 1;
+      if (ti >= 2) ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->acc_empty[acc]), ((ti >> 1) - 1) & 1));
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t d = tmem_base + acc * kN;
+      for (int c = 0; c < kn; ++c, ++it) {
+        const uint32_t s = it % kWStages;
+        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->full[s]), (it / kWStages) & 1));
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {
+          const uint32_t a = base + s * Cfg::kStage;
+          const uint64_t a_desc = umma_desc_kmajor_sw128(a);
+          const uint64_t b_desc = desc_mnmajor_sw128(a + kWXBytes, Cfg::kBoxBytes, 1024);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {  // 32 bytes along x's rows; 32 (int8) or 16 (bf16) rows of W
+            if (kI8) mma_i8_ss(d, a_desc + 2 * j, b_desc + j * (4096 >> 4), idesc, (c | j) != 0 ? 1u : 0u);
+            else mma_f16_ss(d, a_desc + 2 * j, b_desc + j * (2048 >> 4), idesc, (c | j) != 0 ? 1u : 0u);
+          }
+          tc_commit(smem_u32(&ctl->empty[s]));
+          if (c + 1 == kn) tc_commit(smem_u32(&ctl->acc_full[acc]));
+        }
+        __syncwarp();
+      }
+    }
+    if (!ok && lane == 0) {
+      ctl->abort = 1;
+      set_status(p.status, PTO_ST_WAIT_EXPIRED, blockIdx.x, 81);
+    }
+  } else {
+    // ---------------- epilogue: group g stores the tiles of accumulator g ----------------
+    const int q = warp & 3;  // TMEM lanes 32q .. 32q+31
+    const uint32_t g = static_cast<uint32_t>(warp - 2) >> 2;
+    bool ok = true;
+    uint32_t ti = 0;
+    for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++ti) {
+      if ((ti & 1) != g) continue;
+      ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->acc_full[g]), (ti >> 1) & 1));
+      if (!ok) break;
+      tc_fence_after();
+      const WideItem w = wide_item(p, item);
+      wide_epilogue<kEpi, kN>(p, w, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + g * kN, w.rb * kWRows + q * 32,
+                                base + kWStages * Cfg::kStage + static_cast<uint32_t>(warp - 2) * 4096u);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&ctl->acc_empty[g]));
+    }
+    if (!ok && lane == 0) {
+      ctl->abort = 1;
+      set_status(p.status, PTO_ST_WAIT_EXPIRED, blockIdx.x, 82);
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (ctl->abort) {
+    // give copies still in flight time to land before the CTA's shared memory is released
+    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+    __syncthreads();
+  }
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, Cfg::kTmemCols);
+  }
+}
+
+int wide_aligned(std::initializer_list<const void*> ptrs) {
+  for (const void* q : ptrs) {
+    if ((reinterpret_cast<uintptr_t>(q) & 15u) != 0) return 0;
+  }
+  return 1;
+}
+
+template <bool kI8, int kEpi, int kN>
+cudaError_t wide_launch(const void* tmap_w, const void* tmap_w_idx, const void* tmap_x, WideParams& p, int k, int num_sms, cudaStream_t stream, bool pdl) {
+  using Cfg = WideCfg<kI8, kN>;
+  p.n_tiles = (p.n + kN - 1) / kN;
+  p.chunks = (k + Cfg::kChunkK - 1) / Cfg::kChunkK;
+  p.per_split = (p.chunks + p.splits - 1) / p.splits;
+  if ((p.chunks + p.per_split - 1) / p.per_split != p.splits) return cudaErrorInvalidValue;  // a split without work
+  p.row_blocks = (p.t + kWRows - 1) / kWRows;
+  auto kernel = prolog_wide_kernel<kI8, kEpi, kN>;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem);
+  if (e != cudaSuccess) return e;
+  const long long items = static_cast<long long>(p.row_blocks) * p.batch * p.n_tiles * p.splits;
+  if (items > 0x7fffffffLL) return cudaErrorInvalidValue;
+  const int grid = static_cast<int>(items < num_sms ? items : num_sms);
+  count_launch();
+  return launch_maybe_pdl(kernel, dim3(grid), dim3(kWThreads), Cfg::kSmem, stream, pdl,
+                          *reinterpret_cast<const CUtensorMap*>(tmap_w), *reinterpret_cast<const CUtensorMap*>(tmap_w_idx),
+                          *reinterpret_cast<const CUtensorMap*>(tmap_x), p);
+}
+
+}  // namespace
+
+// The tensor maps are byte matrices: W with a [chunk rows x 128 B] box (64 rows for bf16, 128 for int8), x with a [128 x
+// 128 B] box. kind 0: bf16 -> fp32 partials, 1: bf16 -> bf16.
+cudaError_t launch_prolog_wide(int kind, const void* tmap_w, const void* tmap_x, void* out, int t, int n, int k, int batch,
+                               int w_batch_rows, int x_batch_bytes, long long out_batch, long long ld_out, int splits,
+                               long long split_stride, int num_sms, int32_t* status, cudaStream_t stream, bool pdl) {
+  WideParams p{};
+  p.t = t;
+  p.n = n;
+  p.splits = splits < 1 ? 1 : splits;
+  p.batch = batch < 1 ? 1 : batch;
+  p.w_batch_rows = w_batch_rows;
+  p.x_batch_bytes = x_batch_bytes;
+  p.out_batch = out_batch;
+  p.ld_out = ld_out;
+  p.split_stride = split_stride;
+  p.out = out;
+  p.aligned = wide_aligned({out});
+  p.status = status;
+  return kind == kWideF32 ? wide_launch<false, kWideF32, 256>(tmap_w, tmap_w, tmap_x, p, k, num_sms, stream, pdl)
+                          : wide_launch<false, kWideBf16, 256>(tmap_w, tmap_w, tmap_x, p, k, num_sms, stream, pdl);
+}
+
+// both up-projections: int8 [t, k] . int8 [k, 128 * 192] -> nope parts bf16 [t, 128, 128] and rotated tails [t, 128, 64];
+// int8 [t, k] . int8 [k, 64 * 128] -> rotated rows bf16 [t, 64, 128]
+cudaError_t launch_prolog_wide_up(const void* tmap_w, const void* tmap_w_idx, const void* tmap_x, int t, int k,
+                                  const float* row_scale, const float* col_scale, const float* col_scale_idx, const void* cos,
+                                  const void* sin, void* q_nope, void* q_rope, void* idx_rows, int num_sms, int32_t* status,
+                                  cudaStream_t stream, bool pdl) {
+  WideParams p{};
+  p.t = t;
+  p.n = 64 * 128 + 128 * kHeadQ;
+  p.idx_tiles = 64 * 128 / 256;
+  p.splits = p.batch = 1;
+  p.out = q_nope;
+  p.out2 = q_rope;
+  p.out_idx = idx_rows;
+  p.row_scale = row_scale;
+  p.col_scale = col_scale;
+  p.col_scale_idx = col_scale_idx;
+  p.cos = reinterpret_cast<const __nv_bfloat16*>(cos);
+  p.sin = reinterpret_cast<const __nv_bfloat16*>(sin);
+  p.aligned = wide_aligned({q_nope, q_rope, idx_rows, col_scale, col_scale_idx, cos, sin});
+  p.status = status;
+  return wide_launch<true, kWideUp, 256>(tmap_w, tmap_w_idx, tmap_x, p, k, num_sms, stream, pdl);
+}
+
+// rows bf16 [n_rows, 128] . Hadamard bf16 [128, 128] -> int8 rows and an fp16 scale per row
+cudaError_t launch_prolog_wide_hadamard(const void* tmap_had, const void* tmap_rows, int n_rows, int8_t* q_int8,
+                                        void* q_scale, int num_sms, int32_t* status, cudaStream_t stream) {
+  WideParams p{};
+  p.t = n_rows;
+  p.n = 128;
+  p.splits = p.batch = 1;
+  p.out = q_int8;
+  p.out2 = q_scale;
+  p.aligned = wide_aligned({q_int8});
+  p.status = status;
+  return wide_launch<false, kWideHad, 128>(tmap_had, tmap_had, tmap_rows, p, 128, num_sms, stream, false);
+}
+
+}  // namespace pto

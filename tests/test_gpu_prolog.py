@@ -36,7 +36,7 @@ def ref_compare(got, want, name, atol, rtol, ratio=0.005):
     assert bad <= round(ratio * want.numel()), (name, bad, want.numel(), float((got - want).abs().max()))
 
 
-def run_prolog(p, eps_cq=1e-5, eps_ckv=1e-5, prefill=False, separate_outputs=False):
+def run_prolog(p, eps_cq=1e-5, eps_ckv=1e-5, prefill=False, separate_outputs=False, odd_outputs=False):
     g = {k: (v.to(DEV) if isinstance(v, torch.Tensor) else v) for k, v in p.items()}
     t = g["token_x"].shape[0]
     out = dict(q_nope=torch.zeros(t, 128, 512, dtype=torch.bfloat16, device=DEV),
@@ -44,6 +44,10 @@ def run_prolog(p, eps_cq=1e-5, eps_ckv=1e-5, prefill=False, separate_outputs=Fal
                q_int8=torch.zeros(t, 64, 128, dtype=torch.int8, device=DEV),
                q_scale=torch.zeros(t, 64, 1, dtype=torch.float16, device=DEV),
                weights=torch.zeros(t, 64, dtype=torch.float16, device=DEV))
+    if odd_outputs:  # outputs (and the rope tables) that start one element behind a 16-byte boundary
+        shift = lambda v: torch.cat([v.new_zeros(1), v.reshape(-1)])[1:].reshape(v.shape)  # noqa: E731
+        out.update({k: shift(out[k]) for k in ("q_rope", "q_int8", "q_scale", "weights")})
+        g.update({k: shift(g[k]) for k in ("cos", "sin", "w_qb_scale", "w_idx_qb_scale")})
     caches = {}
     for k in ("kv_cache", "kr_cache", "kv_scale_cache", "idx_k_cache", "idx_k_scale_cache"):
         caches[k] = torch.zeros_like(g[k]) if separate_outputs else g[k]
@@ -175,6 +179,14 @@ def test_token_counts(act, s1):
     p = gen.make_prolog_inputs(act, s1=s1, seed=len(act))
     want = po.mla_indexer_prolog(p, eps_cq=1e-5, eps_ckv=1e-5)
     check_against(run_prolog(p), want, p["cache_index"])
+
+
+@pytest.mark.parametrize("t,odd", [(64, False), (65, False), (128, True), (129, False), (257, True)])
+def test_row_counts_at_tile_edges(t, odd):
+    """The last count of the weight-streaming kernels, the first ones with token rows as the M dimension (tiles of 128
+    rows; the projections change over at 129), with aligned and unaligned outputs."""
+    p = gen.make_prolog_inputs([130] * t, s1=1, seed=50 + t)
+    check_against(run_prolog(p, odd_outputs=odd), po.mla_indexer_prolog(p, eps_cq=1e-5, eps_ckv=1e-5), p["cache_index"])
 
 
 def test_bad_cache_index_is_reported_not_written():
