@@ -276,7 +276,7 @@ int pto_mla_indexer_prolog_quant(
     const void* w_idx_proj, const void* ln_gamma, const void* ln_beta, const void* hadamard_q,
     const void* hadamard_k, int8_t* idx_k_cache, void* idx_k_scale_cache, void* query_nope_out,
     void* query_rope_out, int8_t* q_int8_out, void* q_scale_out, void* weights_out,
-    const void* w_x_packed /* from pto_prolog_pack_weights, or NULL: four separate products */,
+    const void* w_x_packed /* from pto_prolog_pack_weights, or NULL: the four weights are read where they are */,
     int8_t* packed_kv_cache /* int8 [cache_rows, 656] or NULL: the token's row is also written there */,
     int t, int hidden, int q_lora, int64_t cache_rows, float eps_cq, float eps_ckv, float ln_eps,
     void* workspace, size_t workspace_bytes, pto_stream_t stream);
@@ -305,7 +305,7 @@ int pto_mla_indexer_prolog(
     void* kv_cache, void* kr_cache, const void* w_idx_qb, const void* w_idx_k, const void* w_idx_proj,
     const void* ln_gamma, const void* ln_beta, void* idx_k_cache, void* query_nope_out, void* query_rope_out,
     void* idx_query_out, void* weights_out, void* q_norm_out,
-    const void* w_x_packed /* from pto_prolog_pack_weights, or NULL */,
+    const void* w_x_packed /* from pto_prolog_pack_weights, or NULL: read where they are */,
     int t, int hidden, int q_lora, int64_t cache_rows, float eps_cq, float eps_ckv, float ln_eps,
     void* workspace, size_t workspace_bytes, pto_stream_t stream);
 

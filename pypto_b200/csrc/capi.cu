@@ -4,6 +4,7 @@
 #include <cuda.h>
 #include <dlfcn.h>
 
+#include <climits>
 #include <cstdarg>
 #include <cstdlib>
 #include <cstdio>
@@ -397,26 +398,81 @@ int prolog_side_stream(int* device) {
 constexpr int kNarrowRows = 64;
 inline bool prolog_is_wide(int t) { return t > kNarrowRows; }
 
-// One bf16 product: out = x[t, k] . W[k, n] per problem of the batch. kind 0: fp32 partials, 1: bf16. Row pitches in bytes.
-int run_sgemm(int kind, const void* x, size_t x_pitch, const void* w, size_t w_pitch, int64_t w_rows, void* out, int t,
-              int n, int k, int batch, int w_batch_rows, int x_batch_bytes, long long out_batch, long long ld_out,
+// A weight matrix of a product: row-major, `width` columns used of rows `pitch` bytes apart.
+struct WMatrix {
+  const void* base;
+  size_t pitch;
+  int width;
+};
+
+// One bf16 product: out = x[t, k] . W[k, n] per problem of the batch. W is `n_w` <= 4 matrices of `w_rows` rows side by
+// side, all widths but the last multiples of 64. kind 0: fp32 partials, 1: bf16. Row pitches in bytes.
+int run_sgemm(int kind, const void* x, size_t x_pitch, const WMatrix* ws, int n_w, int64_t w_rows, void* out, int t,
+              int k, int batch, int w_batch_rows, int x_batch_bytes, long long out_batch, long long ld_out,
               int splits, long long split_stride, int num_sms, int32_t* status, cudaStream_t stream, bool pdl = false) {
   // (up to 128 rows the projections have more items of 128 columns than of 128 rows x 256 columns: 70 tokens 66 us a call
   // against 71)
   const bool wide = prolog_is_wide(t) && (kind != 0 || t > 128);
-  alignas(64) CUtensorMap map_w, map_x;
-  int rc = make_bytes_map(&map_w, w, w_pitch, static_cast<uint64_t>(w_rows), w_pitch, 64);
-  if (rc != PTO_OK) return rc;
+  alignas(64) pto::PrologWMaps maps_w;
+  alignas(64) CUtensorMap map_x;
+  pto::PrologWBoxes boxes;
+  int n = 0, rc = PTO_OK;
+  for (int i = 0; i < 4; ++i) {
+    const WMatrix& w = ws[i < n_w ? i : n_w - 1];
+    if (i < n_w) {
+      rc = make_bytes_map(&maps_w.map[i], w.base, static_cast<size_t>(w.width) * 2, static_cast<uint64_t>(w_rows), w.pitch, 64);
+      if (rc != PTO_OK) return rc;
+      n += w.width;
+    } else {
+      maps_w.map[i] = maps_w.map[n_w - 1];
+    }
+    boxes.end[i] = i + 1 < n_w ? n / 64 : INT_MAX;
+  }
   rc = make_bytes_map(&map_x, x, x_pitch, static_cast<uint64_t>(t), x_pitch,
                       wide ? 128u : static_cast<uint32_t>(pto::prolog_sgemm_rows(t)));
   if (rc != PTO_OK) return rc;
   if (wide) {
-    PTO_CUDA(pto::launch_prolog_wide(kind, &map_w, &map_x, out, t, n, k, batch, w_batch_rows, x_batch_bytes, out_batch, ld_out,
-                                     splits, split_stride, num_sms, status, stream, pdl));
-    return PTO_OK;
+    PTO_CUDA(pto::launch_prolog_wide(kind, maps_w, boxes, &map_x, out, t, n, k, batch, w_batch_rows, x_batch_bytes, out_batch,
+                                     ld_out, splits, split_stride, num_sms, status, stream, pdl));
+  } else {
+    PTO_CUDA(pto::launch_prolog_sgemm(kind, maps_w, boxes, &map_x, out, t, n, k, batch, w_batch_rows, x_batch_bytes, out_batch,
+                                      ld_out, splits, split_stride, num_sms, status, stream, pdl));
   }
-  PTO_CUDA(pto::launch_prolog_sgemm(kind, &map_w, &map_x, out, t, n, k, batch, w_batch_rows, x_batch_bytes, out_batch,
-                                    ld_out, splits, split_stride, num_sms, status, stream, pdl));
+  return PTO_OK;
+}
+
+// The projections of the hidden state: x[t, hidden] . [w_dq | w_dkvkr | w_idx_k | w_idx_proj] -> fp32 partials
+// [splits][t, q_lora | 576 | 128 | 64]. The four weights are read where they lie, or out of the caller's packed copy.
+int run_projections(const void* x, const void* w_dq, const void* w_dkvkr, const void* w_idx_k, const void* w_idx_proj,
+                    const void* packed, float* out, int t, int hidden, int q_lora, int splits, int num_sms, int32_t* status,
+                    cudaStream_t stream) {
+  const int widths[4] = {q_lora, 576, 128, 64};
+  const void* bases[4] = {w_dq, w_dkvkr, w_idx_k, w_idx_proj};
+  const int ld = q_lora + 576 + 128 + 64;
+  const long long split_stride = static_cast<long long>(t) * ld;
+  const size_t x_pitch = static_cast<size_t>(hidden) * 2;
+  WMatrix m[4];
+  int off = 0;
+  for (int i = 0; i < 4; ++i) {
+    m[i].width = widths[i];
+    m[i].base = packed != nullptr ? static_cast<const uint8_t*>(packed) + static_cast<size_t>(off) * 2 : bases[i];
+    m[i].pitch = static_cast<size_t>(packed != nullptr ? ld : widths[i]) * 2;
+    off += widths[i];
+  }
+  if (packed != nullptr) {
+    m[0].width = ld;
+    return run_sgemm(0, x, x_pitch, m, 1, hidden, out, t, hidden, 1, 0, 0, 0, ld, splits, split_stride, num_sms, status, stream);
+  }
+  if (q_lora % 64 == 0) {
+    return run_sgemm(0, x, x_pitch, m, 4, hidden, out, t, hidden, 1, 0, 0, 0, ld, splits, split_stride, num_sms, status, stream);
+  }
+  off = 0;
+  for (int i = 0; i < 4; ++i) {  // boundaries inside a 64-column box: one product per weight
+    const int rc = run_sgemm(0, x, x_pitch, m + i, 1, hidden, out + off, t, hidden, 1, 0, 0, 0, ld, splits, split_stride, num_sms,
+                             status, stream);
+    if (rc != PTO_OK) return rc;
+    off += widths[i];
+  }
   return PTO_OK;
 }
 
@@ -805,30 +861,18 @@ int pto_mla_indexer_prolog_quant(const void* token_x, const void* w_dq, const in
   rc = prolog_side_stream(&dev);
   if (rc != PTO_OK) return rc;
   std::lock_guard<std::mutex> lock(prolog_side().dev_mu[dev]);
+  const WMatrix uk = {w_uk, 512 * 2, 512};
   cudaStream_t side = prolog_side().side[dev];
   cudaEvent_t* ev = prolog_side().ev[dev];
 
   // projections of the token: fp32 partials [splits][t, q_lora | 576 | 128 | 64] (K split over CTAs), added and
-  // rounded where the golden rounds by the kernels that read them. One product when the caller has packed the four
-  // weights side by side, else four.
+  // rounded where the golden rounds by the kernels that read them.
   const int splits = w.splits;
   const long long split_stride = static_cast<long long>(t) * ld;
-  const size_t x_pitch = static_cast<size_t>(hidden) * 2;
-  if (w_x_packed != nullptr) {
-    PTO_REQUIRE(aligned16(w_x_packed), "w_x_packed must be 16-byte aligned");
-    rc = run_sgemm(0, token_x, x_pitch, w_x_packed, static_cast<size_t>(ld) * 2, hidden, qa, t, ld, hidden, 1, 0, 0, 0, ld,
-                   splits, split_stride, di.num_sms, status, stream);
-    if (rc != PTO_OK) return rc;
-  } else {
-    const void* ws[4] = {w_dq, w_dkvkr, w_idx_k, w_idx_proj};
-    float* outs[4] = {qa, kv, ki, wp};
-    const int ns[4] = {q_lora, 576, 128, 64};
-    for (int i = 0; i < 4; ++i) {
-      rc = run_sgemm(0, token_x, x_pitch, ws[i], static_cast<size_t>(ns[i]) * 2, hidden, outs[i], t, ns[i], hidden, 1, 0, 0,
-                     0, ld, splits, split_stride, di.num_sms, status, stream);
-      if (rc != PTO_OK) return rc;
-    }
-  }
+  PTO_REQUIRE(aligned16(w_x_packed), "w_x_packed must be 16-byte aligned");
+  rc = run_projections(token_x, w_dq, w_dkvkr, w_idx_k, w_idx_proj, w_x_packed, qa, t, hidden, q_lora, splits, di.num_sms,
+                       status, stream);
+  if (rc != PTO_OK) return rc;
   // fork: the per-token kernel (caches, indexer key, weights) needs only the projections
   PTO_CUDA(cudaEventRecord(ev[0], stream));
   PTO_CUDA(cudaStreamWaitEvent(side, ev[0], 0));
@@ -860,8 +904,7 @@ int pto_mla_indexer_prolog_quant(const void* token_x, const void* w_dq, const in
     PTO_CUDA(cudaStreamWaitEvent(side, ev[1], 0));
     PTO_CUDA(pto::launch_prolog_wide_hadamard(&map_had, &map_rows, t * 64, q_int8_out, q_scale_out, di.num_sms, status, side));
     PTO_CUDA(cudaEventRecord(ev[2], side));
-    rc = run_sgemm(1, q_b, 128 * 128 * 2, w_uk, 512 * 2, 128 * 128, query_nope_out, t, 512, 128, 128, 128, 128 * 2, 512,
-                   128 * 512, 1, 0, di.num_sms, status, stream, /*pdl=*/true);
+    rc = run_sgemm(1, q_b, 128 * 128 * 2, &uk, 1, 128 * 128, query_nope_out, t, 128, 128, 128, 128 * 2, 512, 128 * 512, 1, 0, di.num_sms, status, stream, /*pdl=*/true);
     if (rc != PTO_OK) return rc;
     PTO_CUDA(cudaStreamWaitEvent(stream, ev[2], 0));
     return PTO_OK;
@@ -885,8 +928,7 @@ int pto_mla_indexer_prolog_quant(const void* token_x, const void* w_dq, const in
   PTO_CUDA(pto::launch_prolog_qb_dequant_rope(qb_i32, q_norm_scale, w_qb_scale, cos, sin, t, q_b, query_rope_out, stream,
                                               /*pdl=*/true));
   // absorbed nope part: per head [t, 128] (row pitch 128*192, head pitch 192 elements) @ w_uk[head] [128, 512] -> bf16
-  rc = run_sgemm(1, q_b, 128 * 192 * 2, w_uk, 512 * 2, 128 * 128, query_nope_out, t, 512, 128, 128, 128, 192 * 2, 512,
-                 128 * 512, 1, 0, di.num_sms, status, stream, /*pdl=*/true);
+  rc = run_sgemm(1, q_b, 128 * 192 * 2, &uk, 1, 128 * 128, query_nope_out, t, 128, 128, 128, 192 * 2, 512, 128 * 512, 1, 0, di.num_sms, status, stream, /*pdl=*/true);
   if (rc != PTO_OK) return rc;
   PTO_CUDA(cudaStreamWaitEvent(stream, ev[2], 0));  // join: everything is ordered before what the caller enqueues next
   return PTO_OK;
@@ -940,28 +982,17 @@ int pto_mla_indexer_prolog(const void* token_x, const void* w_dq, const void* w_
   rc = prolog_side_stream(&dev);
   if (rc != PTO_OK) return rc;
   std::lock_guard<std::mutex> lock(prolog_side().dev_mu[dev]);
+  const WMatrix uk = {w_uk, 512 * 2, 512};
   cudaStream_t side = prolog_side().side[dev];
   cudaEvent_t* ev = prolog_side().ev[dev];
 
   // projections of the token, as in the quantised prolog: fp32 K-split partials [splits][t, q_lora | 576 | 128 | 64]
   const int splits = w.splits;
   const long long split_stride = static_cast<long long>(t) * ld;
-  const size_t x_pitch = static_cast<size_t>(hidden) * 2;
-  if (w_x_packed != nullptr) {
-    PTO_REQUIRE(aligned16(w_x_packed), "w_x_packed must be 16-byte aligned");
-    rc = run_sgemm(0, token_x, x_pitch, w_x_packed, static_cast<size_t>(ld) * 2, hidden, qa, t, ld, hidden, 1, 0, 0, 0, ld,
-                   splits, split_stride, di.num_sms, status, stream);
-    if (rc != PTO_OK) return rc;
-  } else {
-    const void* ws[4] = {w_dq, w_dkvkr, w_idx_k, w_idx_proj};
-    float* outs[4] = {qa, kv, ki, wp};
-    const int ns[4] = {q_lora, 576, 128, 64};
-    for (int i = 0; i < 4; ++i) {
-      rc = run_sgemm(0, token_x, x_pitch, ws[i], static_cast<size_t>(ns[i]) * 2, hidden, outs[i], t, ns[i], hidden, 1, 0, 0,
-                     0, ld, splits, split_stride, di.num_sms, status, stream);
-      if (rc != PTO_OK) return rc;
-    }
-  }
+  PTO_REQUIRE(aligned16(w_x_packed), "w_x_packed must be 16-byte aligned");
+  rc = run_projections(token_x, w_dq, w_dkvkr, w_idx_k, w_idx_proj, w_x_packed, qa, t, hidden, q_lora, splits, di.num_sms,
+                       status, stream);
+  if (rc != PTO_OK) return rc;
   // fork: caches, indexer key and weights need only the projections
   PTO_CUDA(cudaEventRecord(ev[0], stream));
   PTO_CUDA(cudaStreamWaitEvent(side, ev[0], 0));
@@ -975,18 +1006,18 @@ int pto_mla_indexer_prolog(const void* token_x, const void* w_dq, const void* w_
                                          /*pdl=*/true));
   PTO_CUDA(cudaEventRecord(ev[1], stream));
   const size_t qn_pitch = static_cast<size_t>(q_lora) * 2;
-  rc = run_sgemm(1, q_norm, qn_pitch, w_uqqr, 128 * 192 * 2, q_lora, q_b, t, 128 * 192, q_lora, 1, 0, 0, 0, 128 * 192, 1, 0,
-                 di.num_sms, status, stream);
+  const WMatrix uqqr = {w_uqqr, 128 * 192 * 2, 128 * 192}, idx_qb = {w_idx_qb, 64 * 128 * 2, 64 * 128};
+  rc = run_sgemm(1, q_norm, qn_pitch, &uqqr, 1, q_lora, q_b, t, q_lora, 1, 0, 0, 0, 128 * 192, 1, 0, di.num_sms, status,
+                 stream);
   if (rc != PTO_OK) return rc;
   PTO_CUDA(cudaStreamWaitEvent(side, ev[1], 0));
-  rc = run_sgemm(1, q_norm, qn_pitch, w_idx_qb, 64 * 128 * 2, q_lora, idx_query_out, t, 64 * 128, q_lora, 1, 0, 0, 0,
-                 64 * 128, 1, 0, di.num_sms, status, side);
+  rc = run_sgemm(1, q_norm, qn_pitch, &idx_qb, 1, q_lora, idx_query_out, t, q_lora, 1, 0, 0, 0, 64 * 128, 1, 0, di.num_sms,
+                 status, side);
   if (rc != PTO_OK) return rc;
   PTO_CUDA(cudaEventRecord(ev[2], side));
   PTO_CUDA(cudaStreamWaitEvent(stream, ev[2], 0));  // the rope kernel reads both products
   PTO_CUDA(pto::launch_prolog_rope_bf16(q_b, cos, sin, t, query_rope_out, idx_query_out, stream));
-  rc = run_sgemm(1, q_b, 128 * 192 * 2, w_uk, 512 * 2, 128 * 128, query_nope_out, t, 512, 128, 128, 128, 192 * 2, 512,
-                 128 * 512, 1, 0, di.num_sms, status, stream, /*pdl=*/true);
+  rc = run_sgemm(1, q_b, 128 * 192 * 2, &uk, 1, 128 * 128, query_nope_out, t, 128, 128, 128, 192 * 2, 512, 128 * 512, 1, 0, di.num_sms, status, stream, /*pdl=*/true);
   if (rc != PTO_OK) return rc;
   return PTO_OK;  // (the side stream was joined in front of the rope kernel)
 }

@@ -2,6 +2,7 @@
 // parameter blocks passed from the C ABI to the kernels. sm_100a only.
 #pragma once
 
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -390,15 +391,36 @@ bool prolog_i8_gemm_supported(int t, int k);
 cudaError_t launch_prolog_i8_gemm(const void* tmap_w0, const void* tmap_w1, const void* tmap_x, int32_t* out0, int n0,
                                   int32_t* out1, int n1, int k, int t, int num_sms, int32_t* status, cudaStream_t stream,
                                   bool pdl = false);
+// The weight of a product as up to four matrices that lie side by side: 64-column box g of the product is a box of the
+// matrix whose range it falls into. (The hidden state is multiplied by four weights of a layer at once; they are read where
+// they are, nothing is packed.) Box boundaries only: every width but the last is a multiple of 64.
+struct PrologWMaps {
+  CUtensorMap map[4];
+};
+struct PrologWBoxes {
+  int end[4];  // first box behind each matrix (the last one takes the rest)
+};
+__device__ __forceinline__ const CUtensorMap* prolog_w_box(const PrologWMaps& m, const PrologWBoxes& b, int box, int* col_bytes) {
+  int i = 0, begin = 0;
+#pragma unroll
+  for (int e = 0; e < 3; ++e) {
+    if (box >= b.end[e]) {
+      i = e + 1;
+      begin = b.end[e];
+    }
+  }
+  *col_bytes = (box - begin) * 128;
+  return &m.map[i];
+}
 // the weight-streaming products of the prolog (prolog_sgemm.cu)
 int prolog_sgemm_rows(int t);
 int prolog_sgemm_splits(int t, int n, int k, int num_sms);
-cudaError_t launch_prolog_sgemm(int kind, const void* tmap_w, const void* tmap_x, void* out, int t, int n, int k,
+cudaError_t launch_prolog_sgemm(int kind, const PrologWMaps& maps_w, const PrologWBoxes& boxes, const void* tmap_x, void* out, int t, int n, int k,
                                 int batch, int w_batch_rows, int x_batch_bytes, long long out_batch, long long ld_out,
                                 int splits, long long split_stride, int num_sms, int32_t* status, cudaStream_t stream,
                                 bool pdl = false);
 // the same products for many token rows, with what follows them fused (prolog_wide.cu)
-cudaError_t launch_prolog_wide(int kind, const void* tmap_w, const void* tmap_x, void* out, int t, int n, int k, int batch,
+cudaError_t launch_prolog_wide(int kind, const PrologWMaps& maps_w, const PrologWBoxes& boxes, const void* tmap_x, void* out, int t, int n, int k, int batch,
                                int w_batch_rows, int x_batch_bytes, long long out_batch, long long ld_out, int splits,
                                long long split_stride, int num_sms, int32_t* status, cudaStream_t stream, bool pdl = false);
 cudaError_t launch_prolog_wide_up(const void* tmap_w, const void* tmap_w_idx, const void* tmap_x, int t, int k,

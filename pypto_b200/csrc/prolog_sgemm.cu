@@ -63,6 +63,7 @@ struct SGemmParams {
   int n_stages;
   uint32_t stage_bytes;   // kSWBytes + t_pad * 128
   uint32_t tmem_cols;
+  PrologWBoxes boxes;
   int32_t* status;
 };
 
@@ -82,7 +83,7 @@ __device__ __forceinline__ SItem s_item(const SGemmParams& p, int item) {
 
 template <int kOut>
 __global__ void __launch_bounds__(kSThreads, 1)
-prolog_sgemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
+prolog_sgemm_kernel(const __grid_constant__ PrologWMaps maps_w, const __grid_constant__ CUtensorMap tmap_x,
                     const SGemmParams p) {
   extern __shared__ uint8_t sgemm_smem_raw[];
   const uint32_t raw = smem_u32(sgemm_smem_raw);
@@ -107,7 +108,7 @@ prolog_sgemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     ctl->abort = 0;
     fence_mbar_init();
     fence_proxy_async();
-    tma_prefetch_desc(&tmap_w);
+    for (int i = 0; i < (kOut == kOutF32 ? 4 : 1); ++i) tma_prefetch_desc(&maps_w.map[i]);
     tma_prefetch_desc(&tmap_x);
   }
   if (warp == 1) {
@@ -134,7 +135,9 @@ prolog_sgemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         const SItem w = s_item(p, item);
         const int k0 = w.split * p.per_split;
         const int kn = min(p.per_split, p.chunks - k0);
-        const int n0 = w.tile * kSTileN;
+        int col0, col1;  // the tile's two 64-column boxes
+        const CUtensorMap* m0 = prolog_w_box(maps_w, p.boxes, 2 * w.tile, &col0);
+        const CUtensorMap* m1 = prolog_w_box(maps_w, p.boxes, 2 * w.tile + 1, &col1);
         for (int c = 0; c < kn; ++c, ++it) {
           const uint32_t s = it % p.n_stages;
           if (it >= static_cast<uint32_t>(p.n_stages)) {
@@ -145,8 +148,8 @@ prolog_sgemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
           const uint32_t dst = base + s * p.stage_bytes;
           const int krow = w.b * p.w_batch_rows + (k0 + c) * kChunkK;
           mbar_arrive_expect_tx(bar, kSWBytes + x_bytes);
-          tma_load_2d_hint(dst, &tmap_w, n0 * 2, krow, bar, w_policy);
-          tma_load_2d_hint(dst + kSWBytes / 2, &tmap_w, n0 * 2 + 128, krow, bar, w_policy);
+          tma_load_2d_hint(dst, m0, col0, krow, bar, w_policy);
+          tma_load_2d_hint(dst + kSWBytes / 2, m1, col1, krow, bar, w_policy);
           tma_load_2d(dst + kSWBytes, &tmap_x, w.b * p.x_batch_bytes + (k0 + c) * 128, w.tb * p.t_pad, bar);
         }
       }
@@ -247,7 +250,7 @@ prolog_sgemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
 }
 
 template <int kOut>
-cudaError_t launch_one(const void* tmap_w, const void* tmap_x, const SGemmParams& p, int grid, cudaStream_t stream,
+cudaError_t launch_one(const PrologWMaps& maps_w, const void* tmap_x, const SGemmParams& p, int grid, cudaStream_t stream,
                        bool pdl) {
   auto kernel = prolog_sgemm_kernel<kOut>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSSmemMax);
@@ -255,7 +258,8 @@ cudaError_t launch_one(const void* tmap_w, const void* tmap_x, const SGemmParams
   const size_t smem = static_cast<size_t>(p.n_stages) * p.stage_bytes + sizeof(SCtl) + 1024;
   count_launch();
   return launch_maybe_pdl(kernel, dim3(grid), dim3(kSThreads), smem, stream, pdl,
-                          *reinterpret_cast<const CUtensorMap*>(tmap_w), *reinterpret_cast<const CUtensorMap*>(tmap_x), p);
+                          maps_w,
+                          *reinterpret_cast<const CUtensorMap*>(tmap_x), p);
 }
 
 }  // namespace
@@ -285,7 +289,7 @@ int prolog_sgemm_splits(int t, int n, int k, int num_sms) {
 
 // kind: 0 = bf16 x bf16 -> fp32 (with `splits` partials `split_stride` elements apart), 1 = bf16 x bf16 -> bf16. The
 // tensor maps are byte matrices: W with a [64 rows x 128 B] box, x with a [prolog_sgemm_rows(t) x 128 B] box.
-cudaError_t launch_prolog_sgemm(int kind, const void* tmap_w, const void* tmap_x, void* out, int t, int n, int k,
+cudaError_t launch_prolog_sgemm(int kind, const PrologWMaps& maps_w, const PrologWBoxes& boxes, const void* tmap_x, void* out, int t, int n, int k,
                                 int batch, int w_batch_rows, int x_batch_bytes, long long out_batch, long long ld_out,
                                 int splits, long long split_stride, int num_sms, int32_t* status, cudaStream_t stream,
                                 bool pdl) {
@@ -296,6 +300,7 @@ cudaError_t launch_prolog_sgemm(int kind, const void* tmap_w, const void* tmap_x
   p.per_split = (p.chunks + p.splits - 1) / p.splits;
   if ((p.chunks + p.per_split - 1) / p.per_split != p.splits) return cudaErrorInvalidValue;  // a split without work
   p.batch = batch < 1 ? 1 : batch;
+  p.boxes = boxes;
   p.t = t;
   p.t_pad = prolog_sgemm_rows(t);
   p.tok_blocks = (t + p.t_pad - 1) / p.t_pad;
@@ -324,8 +329,8 @@ cudaError_t launch_prolog_sgemm(int kind, const void* tmap_w, const void* tmap_x
   uint32_t cols = 32;
   while (cols < accs * static_cast<uint32_t>(p.t_pad)) cols <<= 1;
   p.tmem_cols = cols;
-  if (kind == kOutF32) return launch_one<kOutF32>(tmap_w, tmap_x, p, grid, stream, pdl);
-  return launch_one<kOutBf16>(tmap_w, tmap_x, p, grid, stream, pdl);
+  if (kind == kOutF32) return launch_one<kOutF32>(maps_w, tmap_x, p, grid, stream, pdl);
+  return launch_one<kOutBf16>(maps_w, tmap_x, p, grid, stream, pdl);
 }
 
 }  // namespace pto

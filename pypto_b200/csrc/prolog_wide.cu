@@ -73,6 +73,7 @@ struct WideParams {
   const float* col_scale_idx;
   const __nv_bfloat16* cos;  // [t, 64]
   const __nv_bfloat16* sin;
+  PrologWBoxes boxes;     // bf16 products: 64-column boxes of the matrices of W
   int aligned;            // everything the epilogue touches lies on 16-byte boundaries: wide accesses, else single elements
   int32_t* status;
 };
@@ -304,7 +305,7 @@ __device__ __forceinline__ void wide_epilogue(const WideParams& p, const WideIte
 
 template <bool kI8, int kEpi, int kN>
 __global__ void __launch_bounds__(kWThreads, 1)
-prolog_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_w_idx,
+prolog_wide_kernel(const __grid_constant__ PrologWMaps maps_w,  // int8: map 0 attention, map 1 indexer
                    const __grid_constant__ CUtensorMap tmap_x, const WideParams p) {
   using Cfg = WideCfg<kI8, kN>;
   extern __shared__ uint8_t wide_smem_raw[];
@@ -326,8 +327,7 @@ prolog_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     ctl->abort = 0;
     fence_mbar_init();
     fence_proxy_async();
-    tma_prefetch_desc(&tmap_w);
-    if (kEpi == kWideUp) tma_prefetch_desc(&tmap_w_idx);
+    for (int i = 0; i < (kEpi == kWideF32 ? 4 : (kEpi == kWideUp ? 2 : 1)); ++i) tma_prefetch_desc(&maps_w.map[i]);
     tma_prefetch_desc(&tmap_x);
   }
   if (warp == 1) {
@@ -350,8 +350,18 @@ prolog_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       const int k0 = w.split * p.per_split;
       const int kn = min(p.per_split, p.chunks - k0);
       const bool idx = kEpi == kWideUp && w.tile < p.idx_tiles;
-      const CUtensorMap* tm = idx ? &tmap_w_idx : &tmap_w;
-      const int col = (kEpi == kWideUp && !idx ? w.tile - p.idx_tiles : w.tile) * kN * (kI8 ? 1 : 2);  // bytes
+      constexpr int kBoxes = kN / Cfg::kGroup;
+      const CUtensorMap* tm[kBoxes];
+      int col[kBoxes];  // bytes
+#pragma unroll
+      for (int g = 0; g < kBoxes; ++g) {
+        if (kI8) {
+          tm[g] = &maps_w.map[idx ? 1 : 0];
+          col[g] = (idx ? w.tile : w.tile - p.idx_tiles) * kN + g * 128;
+        } else {
+          tm[g] = prolog_w_box(maps_w, p.boxes, w.tile * kBoxes + g, &col[g]);
+        }
+      }
       for (int c = 0; c < kn; ++c, ++it) {
         const uint32_t s = it % kWStages;
         if (it >= kWStages) ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->empty[s]), ((it / kWStages) - 1) & 1));
@@ -363,8 +373,8 @@ prolog_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
           mbar_arrive_expect_tx(bar, Cfg::kStage);
           tma_load_2d(dst, &tmap_x, w.b * p.x_batch_bytes + (k0 + c) * 128, w.rb * kWRows, bar);
 #pragma unroll
-          for (int g = 0; g < kN / Cfg::kGroup; ++g) {
-            tma_load_2d(dst + kWXBytes + g * Cfg::kBoxBytes, tm, col + g * 128, krow, bar);
+          for (int g = 0; g < kBoxes; ++g) {
+            tma_load_2d(dst + kWXBytes + g * Cfg::kBoxBytes, tm[g], col[g], krow, bar);
           }
         }
         __syncwarp();
@@ -457,7 +467,7 @@ int wide_aligned(std::initializer_list<const void*> ptrs) {
 }
 
 template <bool kI8, int kEpi, int kN>
-cudaError_t wide_launch(const void* tmap_w, const void* tmap_w_idx, const void* tmap_x, WideParams& p, int k, int num_sms, cudaStream_t stream, bool pdl) {
+cudaError_t wide_launch(const PrologWMaps& maps_w, const void* tmap_x, WideParams& p, int k, int num_sms, cudaStream_t stream, bool pdl) {
   using Cfg = WideCfg<kI8, kN>;
   p.n_tiles = (p.n + kN - 1) / kN;
   p.chunks = (k + Cfg::kChunkK - 1) / Cfg::kChunkK;
@@ -472,18 +482,18 @@ cudaError_t wide_launch(const void* tmap_w, const void* tmap_w_idx, const void* 
   const int grid = static_cast<int>(items < num_sms ? items : num_sms);
   count_launch();
   return launch_maybe_pdl(kernel, dim3(grid), dim3(kWThreads), Cfg::kSmem, stream, pdl,
-                          *reinterpret_cast<const CUtensorMap*>(tmap_w), *reinterpret_cast<const CUtensorMap*>(tmap_w_idx),
-                          *reinterpret_cast<const CUtensorMap*>(tmap_x), p);
+                          maps_w, *reinterpret_cast<const CUtensorMap*>(tmap_x), p);
 }
 
 }  // namespace
 
 // The tensor maps are byte matrices: W with a [chunk rows x 128 B] box (64 rows for bf16, 128 for int8), x with a [128 x
 // 128 B] box. kind 0: bf16 -> fp32 partials, 1: bf16 -> bf16.
-cudaError_t launch_prolog_wide(int kind, const void* tmap_w, const void* tmap_x, void* out, int t, int n, int k, int batch,
+cudaError_t launch_prolog_wide(int kind, const PrologWMaps& maps_w, const PrologWBoxes& boxes, const void* tmap_x, void* out, int t, int n, int k, int batch,
                                int w_batch_rows, int x_batch_bytes, long long out_batch, long long ld_out, int splits,
                                long long split_stride, int num_sms, int32_t* status, cudaStream_t stream, bool pdl) {
   WideParams p{};
+  p.boxes = boxes;
   p.t = t;
   p.n = n;
   p.splits = splits < 1 ? 1 : splits;
@@ -496,8 +506,8 @@ cudaError_t launch_prolog_wide(int kind, const void* tmap_w, const void* tmap_x,
   p.out = out;
   p.aligned = wide_aligned({out});
   p.status = status;
-  return kind == kWideF32 ? wide_launch<false, kWideF32, 256>(tmap_w, tmap_w, tmap_x, p, k, num_sms, stream, pdl)
-                          : wide_launch<false, kWideBf16, 256>(tmap_w, tmap_w, tmap_x, p, k, num_sms, stream, pdl);
+  return kind == kWideF32 ? wide_launch<false, kWideF32, 256>(maps_w, tmap_x, p, k, num_sms, stream, pdl)
+                          : wide_launch<false, kWideBf16, 256>(maps_w, tmap_x, p, k, num_sms, stream, pdl);
 }
 
 // both up-projections: int8 [t, k] . int8 [k, 128 * 192] -> nope parts bf16 [t, 128, 128] and rotated tails [t, 128, 64];
@@ -521,7 +531,10 @@ cudaError_t launch_prolog_wide_up(const void* tmap_w, const void* tmap_w_idx, co
   p.sin = reinterpret_cast<const __nv_bfloat16*>(sin);
   p.aligned = wide_aligned({q_nope, q_rope, idx_rows, col_scale, col_scale_idx, cos, sin});
   p.status = status;
-  return wide_launch<true, kWideUp, 256>(tmap_w, tmap_w_idx, tmap_x, p, k, num_sms, stream, pdl);
+  PrologWMaps maps;
+  maps.map[0] = maps.map[2] = maps.map[3] = *reinterpret_cast<const CUtensorMap*>(tmap_w);
+  maps.map[1] = *reinterpret_cast<const CUtensorMap*>(tmap_w_idx);
+  return wide_launch<true, kWideUp, 256>(maps, tmap_x, p, k, num_sms, stream, pdl);
 }
 
 // rows bf16 [n_rows, 128] . Hadamard bf16 [128, 128] -> int8 rows and an fp16 scale per row
@@ -535,7 +548,10 @@ cudaError_t launch_prolog_wide_hadamard(const void* tmap_had, const void* tmap_r
   p.out2 = q_scale;
   p.aligned = wide_aligned({q_int8});
   p.status = status;
-  return wide_launch<false, kWideHad, 128>(tmap_had, tmap_had, tmap_rows, p, 128, num_sms, stream, false);
+  PrologWMaps maps;
+  for (int i = 0; i < 4; ++i) maps.map[i] = *reinterpret_cast<const CUtensorMap*>(tmap_had);
+  p.boxes = PrologWBoxes{{2, 2, 2, 2}};
+  return wide_launch<false, kWideHad, 128>(maps, tmap_rows, p, 128, num_sms, stream, false);
 }
 
 }  // namespace pto
