@@ -1,4 +1,5 @@
-"""In-tree build of the CUDA library: nvcc -> pypto_b200/libpypto_b200.so (sm_100a only).
+"""In-tree build of the CUDA library: nvcc -> pypto_b200/libpypto_b200.so (sm_100a only), and of the native host path of
+the operators in front of it: g++ -> pypto_b200/_native.so (a CPython module over torch's C++ headers).
 
 The shared object links the CUDA runtime statically and resolves the one driver symbol it needs
 (cuTensorMapEncodeTiled) at run time, so it loads on a machine without a GPU driver.
@@ -9,6 +10,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
@@ -17,6 +19,10 @@ LIB = PKG / "libpypto_b200.so"
 SOURCES = ["capi.cu", "li_score.cu", "topk_select.cu", "sfa_decode.cu", "sfa_pair.cu", "sfa_slice.cu", "prolog.cu", "prolog_gemm.cu",
            "prolog_sgemm.cu", "prolog_wide.cu"]
 HEADERS = [CSRC / "common.cuh", CSRC / "sfa_common.cuh", PKG.parent / "include" / "pypto_b200.h"]
+
+
+NATIVE = PKG / "_native.so"
+NATIVE_SOURCE = CSRC / "native.cpp"
 
 
 def nvcc_path() -> str:
@@ -34,7 +40,31 @@ def needs_build() -> bool:
     return any(d.stat().st_mtime > t for d in deps)
 
 
+def build_native(force: bool = False) -> Path:
+    """The module links the CUDA library next to it and torch's own libraries (loaded by `import torch` before it)."""
+    deps = (NATIVE_SOURCE, LIB, PKG.parent / "include" / "pypto_b200.h")
+    if not force and NATIVE.exists() and all(d.stat().st_mtime <= NATIVE.stat().st_mtime for d in deps):
+        return NATIVE
+    import torch
+
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(nvcc_path()).resolve().parent.parent
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-isystem", str(root / "include"),
+           "-isystem", str(root / "include" / "torch" / "csrc" / "api" / "include"), "-isystem", str(cuda / "include"),
+           "-isystem", sysconfig.get_paths()["include"], str(NATIVE_SOURCE), "-o", str(NATIVE), str(LIB),
+           "-Wl,-rpath,$ORIGIN", "-L", str(root / "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    subprocess.run(cmd, check=True)
+    return NATIVE
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
+    _build_library(force, verbose)
+    build_native(force)
+    return LIB
+
+
+def _build_library(force: bool, verbose: bool) -> Path:
     if not force and not needs_build():
         return LIB
     objs = []
@@ -56,7 +86,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         failed |= pr.returncode != 0
     if failed:
         raise RuntimeError("nvcc failed")
-    link = [nvcc_path(), "-shared", "-cudart", "static", "-gencode", "arch=compute_100a,code=sm_100a", "-o", str(LIB)] + objs + ["-ldl"]
+    link = [nvcc_path(), "-shared", "-Xlinker", "-soname=libpypto_b200.so", "-cudart", "static", "-gencode", "arch=compute_100a,code=sm_100a", "-o", str(LIB)] + objs + ["-ldl"]
     subprocess.run(link, check=True)
     return LIB
 

@@ -22,9 +22,18 @@ from typing import Dict, Tuple
 import torch
 
 from . import _lib
+from .compat import Tensor as _Handle
 from .compat import unwrap
 
 _workspaces: Dict[Tuple[int, int], torch.Tensor] = {}
+
+try:
+    # the same checks and the same call in native code for an ordinary call; a function of it that returns False has done
+    # nothing, and the code below it here raises the operator's error, allocates the workspace or makes the call
+    from . import _native
+    _native.setup(_Handle, _workspaces, _lib.check)
+except ImportError:  # built for another torch, or not built: everything runs through the checks of this module
+    _native = None
 
 
 def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:
@@ -142,6 +151,10 @@ def lightning_indexer_topk_nonquant(idx_query, idx_key_cache, idx_weight, act_se
     198-203, body :23-147 with isQuant = false): score = sum_h w_h * relu(q_h . k) over bf16 tensors in fp32, top-
     `selected_count` per query token. `scores_out` (float32 [t, max_blocks*128], optional) receives the score rows
     instead of the top-k running (the reference's `tmpOut` hook)."""
+    if _native is not None and scores_out is None and _native.li_decode_bf16(
+            idx_query, idx_key_cache, idx_weight, act_seq_key, block_table, topk_res, selected_count,
+            0 if sort else _lib.PTO_LI_UNSORTED):
+        return None
     (q, kc, w, act, bt), m = _li_args_bf16(idx_query, idx_key_cache, idx_weight, act_seq_key, block_table)
     lib = _lib.load()
     common = (m["b"], m["s1"], 64, 128, 128, m["block_num"], m["max_blocks"])
@@ -180,6 +193,12 @@ def lightning_indexer_decode(idx_query, idx_query_scale, idx_key_cache, idx_key_
     A bfloat16 `idx_query` selects the non-quantised formulation (`lightning_indexer_topk_nonquant`; the two scale
     arguments must then be None). `histogram=True` (s1 <= 2): the score kernel leaves a histogram of every row for
     the selection to start from (same results; measured slightly slower, hence off by default)."""
+    flags = (0 if sort else _lib.PTO_LI_UNSORTED) | (_lib.PTO_LI_SCORE_SIMT if _simt_scores else 0)
+    flags |= _lib.PTO_LI_FP16_CHAIN if fp16_chain else 0
+    flags |= _lib.PTO_LI_EPILOGUE_HIST if histogram else 0
+    if _native is not None and _native.li_decode(idx_query, idx_query_scale, idx_key_cache, idx_key_scale, idx_weight,
+                                                 act_seq_key, block_table, topk_res, selected_count, flags):
+        return None
     if unwrap(idx_query, "idx_query").dtype == torch.bfloat16:
         _need(idx_query_scale is None and idx_key_scale is None, "bfloat16 idx_query: the scale tensors must be None")
         _need(not (_simt_scores or fp16_chain), "bfloat16 idx_query: one formulation, tensor cores only")
@@ -194,9 +213,6 @@ def lightning_indexer_decode(idx_query, idx_query_scale, idx_key_cache, idx_key_
     dev = _same_device([q, qs, kc, ks, w, act, bt, out])
     lib = _lib.load()
     nbytes = lib.pto_li_workspace_bytes(m["t"], m["max_blocks"], m["block_size"])
-    flags = (0 if sort else _lib.PTO_LI_UNSORTED) | (_lib.PTO_LI_SCORE_SIMT if _simt_scores else 0)
-    flags |= _lib.PTO_LI_FP16_CHAIN if fp16_chain else 0
-    flags |= _lib.PTO_LI_EPILOGUE_HIST if histogram else 0
     with torch.cuda.device(dev):
         ws = _workspace(dev, nbytes)
         _lib.check(lib.pto_li_decode(q.data_ptr(), qs.data_ptr(), kc.data_ptr(), ks.data_ptr(), w.data_ptr(),
@@ -286,6 +302,10 @@ def _sfa_common(query_nope, query_rope, topk_indices, block_table, kv_act_seqs, 
 def _sparse_flash_attention_quant(query_nope, query_rope, key_nope_2d, key_rope_2d, k_nope_scales, topk_indices,
                                   block_table, kv_act_seqs, attention_out, nq, n_kv, softmax_scale, topk, block_size,
                                   max_blocknum_perbatch, tile_config=None, head_begin=0, nq_total=None):
+    if _native is not None and _native.sfa(query_nope, query_rope, key_nope_2d, key_rope_2d, k_nope_scales, topk_indices,
+                                           block_table, kv_act_seqs, attention_out, nq, n_kv, softmax_scale, topk,
+                                           block_size, max_blocknum_perbatch, head_begin, nq_total):
+        return None
     qn, qr, ti, bt, act, out, t, b = _sfa_common(query_nope, query_rope, topk_indices, block_table, kv_act_seqs,
                                                  attention_out, nq, n_kv, topk, nq_total, head_begin)
     kn = unwrap(key_nope_2d, "key_nope_2d")
@@ -349,6 +369,9 @@ def sparse_flash_attention_quant_p(query_nope, query_rope, key_nope_2d, key_rope
 def _sparse_attention_antiquant(query_nope, query_rope, nope_cache, topk_indices, block_table, kv_act_seqs,
                                 attention_out, nq, n_kv, softmax_scale, topk, block_size, max_blocknum_perbatch,
                                 tile_config=None):
+    if _native is not None and _native.sfa_packed(query_nope, query_rope, nope_cache, topk_indices, block_table,
+                                                  kv_act_seqs, attention_out, nq, n_kv, softmax_scale, topk, block_size):
+        return None
     qn, qr, ti, bt, act, out, t, b = _sfa_common(query_nope, query_rope, topk_indices, block_table, kv_act_seqs,
                                                  attention_out, nq, n_kv, topk)
     cache = unwrap(nope_cache, "nope_cache")
@@ -403,6 +426,15 @@ def _mla_indexer_prolog_quant(token_x, mla_w_dq, mla_w_uq_qr, mla_dequant_scale,
                               ip_q_int8_out, ip_q_scale_out, ip_k_int8_out, ip_k_scale_out, ip_weights_out,
                               mla_epsilon_cq, mla_epsilon_ckv, mla_cache_mode="PA_BSND", mla_tile_config=None,
                               ip_attrs=None, ip_configs=None, rope_cfg=None, *, packed_kv_cache=None):
+    ln_eps = float(getattr(ip_attrs, "eps", 1e-6)) if ip_attrs is not None else 1e-6
+    if _native is not None and mla_cache_mode == "PA_BSND" and _native.prolog_quant(
+            token_x, mla_w_dq, mla_w_uq_qr, mla_dequant_scale, mla_w_uk, mla_w_dkv_kr, mla_gamma_cq, mla_gamma_ckv, cos,
+            sin, cache_index, mla_kv_cache, mla_kr_cache, mla_k_scale_cache, ip_w_qb_in, ip_w_qb_scale_in, ip_wk_in,
+            ip_w_proj_in, ip_ln_gamma_k_in, ip_ln_beta_k_in, ip_hadamard_q_in, ip_hadamard_k_in, ip_k_cache,
+            ip_k_cache_scale, mla_query_nope_out, mla_query_rope_out, mla_kv_cache_out, mla_kr_cache_out,
+            mla_k_scale_cache_out, ip_q_int8_out, ip_q_scale_out, ip_k_int8_out, ip_k_scale_out, ip_weights_out,
+            packed_kv_cache, mla_epsilon_cq, mla_epsilon_ckv, ln_eps):
+        return None
     bf, i8, f32, f16 = torch.bfloat16, torch.int8, torch.float32, torch.float16
     x = unwrap(token_x, "token_x")
     _need(x.dtype == bf and x.dim() == 2, "token_x: bfloat16 [t, h]")
@@ -450,7 +482,6 @@ def _mla_indexer_prolog_quant(token_x, mla_w_dq, mla_w_uq_qr, mla_dequant_scale,
     q_i8 = want(ip_q_int8_out, "ip_q_int8_out", i8, t * 64 * 128, "int8 [t, 64, 128]")
     q_sc = want(ip_q_scale_out, "ip_q_scale_out", f16, t * 64, "float16 [t, 64, 1]")
     w_out = want(ip_weights_out, "ip_weights_out", f16, t * 64, "float16 [t, 64]")
-    ln_eps = float(getattr(ip_attrs, "eps", 1e-6)) if ip_attrs is not None else 1e-6
     tensors = [x, w_dq, w_uqqr, w_qb_scale, w_uk, w_dkvkr, g_cq, g_ckv, cos_t, sin_t, ci, kv, kr, ks, w_idx_qb,
                w_idx_qb_scale, w_idx_k, w_idx_proj, ln_g, ln_b, had_q, had_k, ik, iks, q_nope, q_rope, q_i8, q_sc,
                w_out]
@@ -509,6 +540,13 @@ def decode_indexer_attention_quant(idx_query, idx_query_scale, idx_key_cache, id
                                    sort=False, fp16_chain=False, histogram=False):
     """Fused chain: indexer score -> top-k -> sparse attention with the kernel's own indices.
     Both caches share `block_table` / `act_seq`. Writes `topk_res` and `attention_out`."""
+    flags = (0 if sort else _lib.PTO_LI_UNSORTED) | (_lib.PTO_LI_FP16_CHAIN if fp16_chain else 0)
+    flags |= _lib.PTO_LI_EPILOGUE_HIST if histogram else 0
+    if _native is not None and _native.fused(idx_query, idx_query_scale, idx_key_cache, idx_key_scale, idx_weight,
+                                             query_nope, query_rope, key_nope_2d, key_rope_2d, k_nope_scales, act_seq,
+                                             block_table, topk_res, attention_out, nq, softmax_scale, selected_count,
+                                             flags):
+        return None
     dev, (q, qs, kc, ks, w, act, bt), m = _li_args(idx_query, idx_query_scale, idx_key_cache, idx_key_scale,
                                                     idx_weight, act_seq, block_table)
     out_idx = unwrap(topk_res, "topk_res")
@@ -526,8 +564,6 @@ def decode_indexer_attention_quant(idx_query, idx_query_scale, idx_key_cache, id
     dev = _same_device([q, qs, kc, ks, w, act, bt, qn, qr, kn, kr, sc, out_idx, out])
     lib = _lib.load()
     nbytes = lib.pto_decode_workspace_bytes(t, m["max_blocks"], 128, int(nq))
-    flags = (0 if sort else _lib.PTO_LI_UNSORTED) | (_lib.PTO_LI_FP16_CHAIN if fp16_chain else 0)
-    flags |= _lib.PTO_LI_EPILOGUE_HIST if histogram else 0
     with torch.cuda.device(dev):
         ws = _workspace(dev, nbytes)
         _lib.check(lib.pto_decode_fused(q.data_ptr(), qs.data_ptr(), kc.data_ptr(), ks.data_ptr(), w.data_ptr(),
@@ -546,6 +582,11 @@ def decode_indexer_attention(idx_query, idx_key_cache, idx_weight, query_nope, q
     (framework/src/operator/models/deepseek_v3.2_exp/decode_indexer_attention.cpp:108-129): bf16 indexer -> top-k
     -> sparse attention over the bf16 latent cache with the kernel's own indices. Writes `topk_res` and
     `attention_out`."""
+    if _native is not None and _native.fused_bf16(idx_query, idx_key_cache, idx_weight, query_nope, query_rope,
+                                                  key_nope_2d, key_rope_2d, act_seq, block_table, topk_res,
+                                                  attention_out, nq, softmax_scale, selected_count,
+                                                  0 if sort else _lib.PTO_LI_UNSORTED):
+        return None
     (q, kc, w, act, bt), m = _li_args_bf16(idx_query, idx_key_cache, idx_weight, act_seq, block_table)
     out_idx = unwrap(topk_res, "topk_res")
     qn, qr, ti, bt2, act2, out, t, b = _sfa_common(query_nope, query_rope, out_idx, bt, act, attention_out, nq, 1,
@@ -586,6 +627,11 @@ def mla_indexer_prolog(token_x, w_dq, w_uq_qr, w_uk, w_dkv_kr, gamma_cq, gamma_c
     [.., 64], idx_k_cache bf16 [.., 128]. Written: query_nope_out [t, 128, 512], query_rope_out [t, 128, 64],
     idx_query_out [t, 64, 128], idx_weights_out [t, 64] (all bf16), and `q_norm_out` [t, q_lora] (the reference's
     `rmsRes`) when given."""
+    if _native is not None and cache_mode == "PA_BSND" and _native.prolog(
+            token_x, w_dq, w_uq_qr, w_uk, w_dkv_kr, gamma_cq, gamma_ckv, cos, sin, cache_index, kv_cache, kr_cache,
+            idx_w_qb, idx_wk, idx_w_proj, idx_ln_gamma, idx_ln_beta, idx_k_cache, query_nope_out, query_rope_out,
+            idx_query_out, idx_weights_out, q_norm_out, epsilon_cq, epsilon_ckv, ln_eps):
+        return None
     bf = torch.bfloat16
     x = unwrap(token_x, "token_x")
     _need(x.dtype == bf and x.dim() == 2, "token_x: bfloat16 [t, h]")
