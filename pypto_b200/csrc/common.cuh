@@ -299,7 +299,7 @@ struct LiParams {
   int bf16;        // non-quantised formulation: q, k_cache and weight are bf16, the scales are not read
   int s1_total;    // query tokens per sequence in memory (>= s1)
   int tok_offset;  // first token of each sequence handled by this launch
-  int groups;      // token groups of s1 tokens taken by one launch (grid y; tensor-core kernel), >= 1
+  int groups;      // token groups of s1 tokens taken by one launch (tensor-core kernel), >= 1
   // optional, tensor-core kernel with s1 <= 2 per launch: per query token a histogram [t, kLiHistBins] (zeroed by the
   // caller) of the scores at positions below the token's causal end, binned by the top 12 bits of the
   // order-preserving image of the float; the top-k kernel starts from it instead of scanning the row for one

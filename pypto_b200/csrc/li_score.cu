@@ -8,22 +8,27 @@
 // deepseekv32_lightning_indexer_quant.py:205-241).
 //
 // Tensor-core kernel: persistent CTAs, each owning a contiguous range of the flattened
-// (sequence, page) list. Per page: one TMA load of the 16 KB key page (128 keys x 128 B,
-// 128-byte swizzle) -> four tcgen05.mma kind::i8 (M = 128 keys, N = 64*s1 heads, K = 32) into a
-// TMEM accumulator -> epilogue warps read their key's row (one TMEM lane = one key), apply
-// ReLU/2^-11/fp16 rounding and the weighted head sum, and write the fp32 score.
-// Warp roles: warp 0 TMA producer, warps 1..2 MMA issuers (alternate pages; warp 1 owns TMEM),
-// warps 3..18 epilogue (four groups of four warps that take pages round-robin; a single warp is
+// (token group, sequence, page) list. Per page: one TMA load of the 16 KB key page (128 keys x 128 B,
+// 128-byte swizzle) and its key scales; per page and pair of query tokens (an item): four tcgen05.mma kind::i8
+// (M = 128 keys, N = 64 or 128 heads, K = 32) into a TMEM accumulator -> epilogue warps read their key's
+// row (one TMEM lane = one key), apply ReLU/2^-11/fp16 rounding and the weighted head sum, and write the fp32 score.
+// Warp roles: warp 0 TMA producer, warps 1..2 MMA issuers (alternate items; warp 1 owns TMEM),
+// warps 3..18 epilogue (four groups of four warps that take items round-robin; a single warp is
 // latency-bound on the conversion chain, so thread-level parallelism has to come from many warps).
-// A ring of 8 slots pairs one shared-memory stage with one TMEM accumulator. All waits are bounded.
+// Two rings: key pages in shared memory (8), freed by the MMAs that read them, and accumulators in TMEM (8 of 64
+// columns, 4 of 128), freed by the epilogue. With one ring for both, a page's load was requested only when the epilogue
+// had let go of an accumulator, and every slot paid load latency + product + epilogue in turn: 1117 cycles per page with
+// two query tokens, where the page's bytes take 750 at the memory's rate. Items of at most two tokens keep all four
+// epilogue groups at work when a pass takes three or four tokens of a sequence (with 256 columns per item two of
+// them had no accumulator to serve). All waits are bounded.
 //
 // Non-quantised formulation (bf16 queries, keys and weights; reference LightningIndexerTopkImpl with isQuant =
 // false, framework/src/operator/models/deepseek_v3.2_exp/lightning_indexer.cpp:113-147, golden
 // indexer_topk_compute(is_quant=False), framework/tests/st/operator/src/test_deepseek_v3.2_exp/
 // gen_lightning_indexer.py:189-279):   score[pos] = sum_h fp32(w_h) * relu( fp32( q[h, :] . k[pos, :] ) ).
-// Same kernel and ring, mode kLiBf16: a key page is 32 KB (two 128-byte-swizzled halves of the 128 dims), the
-// product is tcgen05.mma kind::f16 (bf16 x bf16 -> fp32, eight MMAs of K = 16 per page), four ring slots, at
-// most two query tokens of a sequence per launch, and the epilogue is max/fma on the fp32 accumulators.
+// Same kernel and rings, mode kLiBf16: a key page is 32 KB (two 128-byte-swizzled halves of the 128 dims), the
+// product is tcgen05.mma kind::f16 (bf16 x bf16 -> fp32, eight MMAs of K = 16 per page), four pages, at
+// most two query tokens of a sequence per pass, and the epilogue is max/fma on the fp32 accumulators.
 #include <cuda.h>
 
 #include "common.cuh"
@@ -32,14 +37,16 @@ namespace pto {
 
 namespace {
 
-constexpr int kLiSlots = 8;            // ring of (smem stage, TMEM accumulator) pairs
+constexpr int kLiStages = 8;           // ring of key pages in shared memory
+constexpr int kLiAccs = 8;             // accumulators of 64 columns (4 of 128)
+constexpr int kLiScaleRing = 16;       // key scales of the pages in flight, see the producer
 constexpr int kPageKeys = 128;
 constexpr int kPageBytes = kPageKeys * 128;
-constexpr int kStageBytes = kPageBytes + 1024;  // key page + the page's 128 key scales (<= 512 B), 1024-aligned
+constexpr int kScaleBytes = 512;                // the page's 128 key scales
 constexpr int kHeads = 64;
 constexpr int kQBytesPerToken = kHeads * 128;
 constexpr int kLiMmaWarps = 2;         // warps 1..2: issuer for pages n with n % 2 == warp - 1
-constexpr int kLiEpilogueGroups = 4;   // groups of four warps; a slot is always served by the same group (below)
+constexpr int kLiEpilogueGroups = 4;   // groups of four warps; an accumulator is always served by the same group (below)
 constexpr int kLiEpilogueWarp0 = 1 + kLiMmaWarps;
 constexpr int kLiThreads = 32 * (kLiEpilogueWarp0 + 4 * kLiEpilogueGroups);
 constexpr int kMaxS1 = 4;
@@ -48,15 +55,17 @@ constexpr int kTmemCols = 512;
 // score formulations the tensor-core kernel is instantiated for
 enum { kLiQuant = 0, kLiChain = 1, kLiBf16 = 2 };
 constexpr int kBf16PageBytes = kPageKeys * 256;  // one stage of the bf16 ring: the page's two 16 KB halves
-constexpr int kBf16Slots = 4;                    // 4 x 32 KB fit where the int8 ring keeps 8 x 17 KB
+constexpr int kBf16Stages = 4;                   // 4 x 32 KB where the int8 ring keeps 8 x 16 KB
 constexpr int kBf16MaxS1 = 2;                    // 2 tokens x 64 heads x 256 B of queries fit the int8 Q area
-static_assert(kBf16Slots * kBf16PageBytes <= kLiSlots * kStageBytes, "bf16 ring exceeds the stage area");
+static_assert(kBf16Stages * kBf16PageBytes <= kLiStages * kPageBytes, "bf16 ring exceeds the stage area");
+static_assert(kLiScaleRing >= kLiStages + kLiAccs, "a page's scales are read until its items' accumulators are free again");
 static_assert(kBf16MaxS1 * kHeads * 256 <= kMaxS1 * kQBytesPerToken, "bf16 queries exceed the Q area");
 
 struct LiCtl {
-  uint64_t full[kLiSlots];     // TMA bytes of the slot's page landed
-  uint64_t accfull[kLiSlots];  // the slot's MMAs completed (tcgen05.commit)
-  uint64_t empty[kLiSlots];    // the slot's epilogue warps finished reading TMEM and the scales
+  uint64_t full[kLiStages];    // TMA bytes of the page (and its scales) landed
+  uint64_t kempty[kLiStages];  // all MMAs that read the page completed (tcgen05.commit, one per item of the page)
+  uint64_t accfull[kLiAccs];   // the item's MMAs completed (tcgen05.commit)
+  uint64_t accempty[kLiAccs];  // the item's epilogue warps have read the accumulator
   uint64_t qfull;
   uint32_t tmem_base;
   int abort;
@@ -65,7 +74,10 @@ struct LiCtl {
 };
 
 constexpr size_t kLiHistSmemBytes = static_cast<size_t>(kLiHistMaxS1) * kLiHistBins * sizeof(unsigned int) + 16;  // 32 KB (+ alignment of its start)
-constexpr size_t kLiSmemBytes = 1024 /*alignment slack*/ + kLiSlots * kStageBytes + kMaxS1 * kQBytesPerToken + sizeof(LiCtl);
+constexpr int kLiSmemScales = kLiStages * kPageBytes, kLiSmemQ = kLiSmemScales + kLiScaleRing * kScaleBytes;
+constexpr int kLiSmemCtl = kLiSmemQ + kMaxS1 * kQBytesPerToken;
+static_assert(kLiSmemQ % 1024 == 0, "swizzled query tile");
+constexpr size_t kLiSmemBytes = 1024 /*alignment slack*/ + kLiSmemCtl + sizeof(LiCtl);
 static_assert(kLiSmemBytes + kLiHistSmemBytes <= 227 * 1024, "score kernel shared memory");
 
 __device__ __forceinline__ float load_scale(const void* base, int dtype, int64_t i) {
@@ -149,16 +161,16 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* smem = smem_raw + (base - raw);
   const uint32_t stage_base = base;
-  const uint32_t q_base = base + kLiSlots * kStageBytes;
-  LiCtl* ctl = reinterpret_cast<LiCtl*>(smem + kLiSlots * kStageBytes + kMaxS1 * kQBytesPerToken);
+  const uint32_t q_base = base + kLiSmemQ;
+  LiCtl* ctl = reinterpret_cast<LiCtl*>(smem + kLiSmemCtl);
   // per-CTA histogram of the current sequence's scores (present only when the launch asked for it)
-  unsigned int* hist_sm = reinterpret_cast<unsigned int*>(smem + kLiSlots * kStageBytes + kMaxS1 * kQBytesPerToken +
-                                                          ((sizeof(LiCtl) + 15) & ~size_t(15)));
+  unsigned int* hist_sm = reinterpret_cast<unsigned int*>(smem + kLiSmemCtl + ((sizeof(LiCtl) + 15) & ~size_t(15)));
   const bool with_hist = p.hist != nullptr;
 
   constexpr bool kChain = kMode == kLiChain;
   constexpr bool kBf16 = kMode == kLiBf16;
-  constexpr uint32_t kStage = kBf16 ? kBf16PageBytes : kStageBytes;
+  constexpr uint32_t kStage = kBf16 ? kBf16PageBytes : kPageBytes;
+  constexpr uint32_t kStages = kBf16 ? kBf16Stages : kLiStages;
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
   const int lane = tid & 31;
@@ -166,14 +178,18 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
   // may be scheduled as soon as SMs drain and waits there for this grid to complete
   if (tid == 0) pdl_trigger();
   const int s1 = p.s1;
-  const int n_cols = kHeads * s1;                                // accumulator columns per page
-  const uint32_t n_slots = min(kBf16 ? kBf16Slots : kLiSlots, kTmemCols / n_cols);   // int8: 8, 4, 2, 2 for s1 = 1..4
-
+  const int items_per_page = s1 > 2 ? 2 : 1;                     // an item: one or two query tokens of a page
+  const uint32_t unit_cols = s1 > 1 ? 2 * kHeads : kHeads;       // columns of an accumulator
+  const uint32_t n_accs = kTmemCols / unit_cols;                 // 8 or 4
+  const uint32_t acc_shift = s1 > 1 ? 2 : 3;                     // log2 of it
   if (tid == 0) {
-    for (int i = 0; i < kLiSlots; ++i) {
+    for (int i = 0; i < kLiStages; ++i) {
       mbar_init(smem_u32(&ctl->full[i]), 1);
+      mbar_init(smem_u32(&ctl->kempty[i]), static_cast<uint32_t>(items_per_page));
+    }
+    for (int i = 0; i < kLiAccs; ++i) {
       mbar_init(smem_u32(&ctl->accfull[i]), 1);
-      mbar_init(smem_u32(&ctl->empty[i]), 4);
+      mbar_init(smem_u32(&ctl->accempty[i]), 4);
     }
     mbar_init(smem_u32(&ctl->qfull), 1);
     ctl->abort = 0;
@@ -215,25 +231,31 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
   tc_fence_after();
   const uint32_t tmem_base = ctl->tmem_base;
 
+  // pages of all sequences, once per token group
   const int total = ctl->prefix[p.b];
-  const int it0 = static_cast<int>(static_cast<long long>(total) * blockIdx.x / gridDim.x);
-  const int it1 = static_cast<int>(static_cast<long long>(total) * (blockIdx.x + 1) / gridDim.x);
+  const long long all = static_cast<long long>(total) * p.groups;
+  const long long it0 = all * blockIdx.x / gridDim.x, it1 = all * (blockIdx.x + 1) / gridDim.x;
 
-  const uint32_t idesc = kBf16 ? umma_idesc(kCFmtF32, kABFmtBF16, kABFmtBF16, 0, 0, 128, n_cols)
-                               : umma_idesc(kCFmtS32, kABFmtS8, kABFmtS8, 0, 0, 128, n_cols);
+  const uint32_t idesc1 = kBf16 ? umma_idesc(kCFmtF32, kABFmtBF16, kABFmtBF16, 0, 0, 128, kHeads)
+                                : umma_idesc(kCFmtS32, kABFmtS8, kABFmtS8, 0, 0, 128, kHeads);
+  const uint32_t idesc2 = kBf16 ? umma_idesc(kCFmtF32, kABFmtBF16, kABFmtBF16, 0, 0, 128, 2 * kHeads)
+                                : umma_idesc(kCFmtS32, kABFmtS8, kABFmtS8, 0, 0, 128, 2 * kHeads);
   const uint32_t scale_bytes = kBf16 ? 0u : kPageKeys * (p.scale_dtype == PTO_DT_F16 ? 2u : 4u);
-  const uint32_t q_half_bytes = static_cast<uint32_t>(n_cols) * 128u;  // bf16: one 64-dim half of the query tile
+  const uint32_t q_half_bytes = static_cast<uint32_t>(s1 * kHeads) * 128u;  // bf16: one 64-dim half of the query tile
 
-  int cur = it0;
-  int bi = 0;
+  long long cur = it0;
+  int bi = 0, group = 0;
   if (cur < it1) {
-    int lo = 0, hi = p.b;  // largest bi with prefix[bi] <= cur
+    group = static_cast<int>(cur / total);
+    const int lc = static_cast<int>(cur - static_cast<long long>(group) * total);
+    int lo = 0, hi = p.b;  // largest bi with prefix[bi] <= lc
     while (hi - lo > 1) {
       int mid = (lo + hi) >> 1;
-      if (ctl->prefix[mid] <= cur) lo = mid; else hi = mid;
+      if (ctl->prefix[mid] <= lc) lo = mid; else hi = mid;
     }
     bi = lo;
   }
+  uint32_t n_page = 0;  // pages and items of the segments before
   uint32_t n_item = 0;
   uint32_t seg = 0;
   int64_t prev_tok0 = 0;
@@ -250,13 +272,18 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
   };
 
   while (cur < it1) {
-    while (ctl->prefix[bi + 1] <= cur) ++bi;
-    const int seg_end = min(it1, ctl->prefix[bi + 1]);
-    const int page0 = cur - ctl->prefix[bi];
-    const int npages = seg_end - cur;
+    int lc = static_cast<int>(cur - static_cast<long long>(group) * total);
+    if (lc >= total) {  // next token group, from the first sequence
+      ++group;
+      bi = 0;
+      lc = 0;
+    }
+    while (ctl->prefix[bi + 1] <= lc) ++bi;
+    const int page0 = lc - ctl->prefix[bi];
+    const int npages = static_cast<int>(min(it1 - cur, static_cast<long long>(ctl->prefix[bi + 1] - lc)));
     const int seq_len = p.act_seq[bi];
-    // (grid y: further groups of s1 tokens of the same sequences, prefill chunks)
-    const int64_t tok0 = static_cast<int64_t>(bi) * p.s1_total + p.tok_offset + static_cast<int>(blockIdx.y) * p.s1;
+    const int tok_first = p.tok_offset + group * s1;  // first query token of the segment within its sequence
+    const int64_t tok0 = static_cast<int64_t>(bi) * p.s1_total + tok_first;
 
     // The producer warp takes no part in the two barriers of a segment: the ring's own barriers order its loads, so
     // the next segment's first pages are on their way while this one drains and the scale products are fetched.
@@ -297,8 +324,10 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
       if (warp == 0) {
         // ---------------- TMA producer ----------------
         const int32_t* bt = p.block_table + static_cast<int64_t>(bi) * p.max_blocks + page0;
-        // key pages are read once: first to leave L2, so that the score rows written for the selection stay there
+        // key pages that are read once are the first to leave L2, so that the score rows written for the selection stay
+        // there (a prompt chunk reads them once per token group)
         const uint64_t stream_policy = l2_policy_evict_first();
+        const bool once = p.groups == 1;
         bool ok = true;
         for (int j0 = 0; j0 < npages && ok; j0 += 32) {
           const int mine = (j0 + lane < npages) ? bt[j0 + lane] : 0;
@@ -306,10 +335,10 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
           for (int jj = 0; jj < cnt; ++jj) {
             int phys = __shfl_sync(0xffffffffu, mine, jj);
             if (lane == 0) {
-              const uint32_t n = n_item + j0 + jj;
-              const uint32_t slot = n % n_slots;
-              const uint32_t ph = (n / n_slots) & 1u;
-              if (!mbar_wait(smem_u32(&ctl->empty[slot]), ph ^ 1u)) {
+              const uint32_t n = n_page + j0 + jj;
+              const uint32_t slot = n % kStages;
+              const uint32_t ph = (n / kStages) & 1u;
+              if (!mbar_wait(smem_u32(&ctl->kempty[slot]), ph ^ 1u)) {
                 ok = false;
                 ctl->abort = 1;
                 set_status(p.status, PTO_ST_WAIT_EXPIRED, static_cast<int>(n), 1);
@@ -324,12 +353,21 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
                 const uint32_t dst = stage_base + slot * kStage;
                 if (kBf16) {
                   mbar_arrive_expect_tx(bar, kBf16PageBytes);
-                  tma_load_2d_hint(dst, &tmap_k, 0, phys * kPageKeys, bar, stream_policy);
-                  tma_load_2d_hint(dst + kPageBytes, &tmap_k, 128, phys * kPageKeys, bar, stream_policy);
+                  if (once) {
+                    tma_load_2d_hint(dst, &tmap_k, 0, phys * kPageKeys, bar, stream_policy);
+                    tma_load_2d_hint(dst + kPageBytes, &tmap_k, 128, phys * kPageKeys, bar, stream_policy);
+                  } else {
+                    tma_load_2d(dst, &tmap_k, 0, phys * kPageKeys, bar);
+                    tma_load_2d(dst + kPageBytes, &tmap_k, 128, phys * kPageKeys, bar);
+                  }
                 } else {
                   mbar_arrive_expect_tx(bar, kPageBytes + scale_bytes);
-                  tma_load_2d_hint(dst, &tmap_k, 0, phys * kPageKeys, bar, stream_policy);
-                  bulk_load_1d(dst + kPageBytes,
+                  if (once) tma_load_2d_hint(dst, &tmap_k, 0, phys * kPageKeys, bar, stream_policy);
+                  else tma_load_2d(dst, &tmap_k, 0, phys * kPageKeys, bar);
+                  // The place of these scales was last used by page n - 16. Its epilogue has read them: the MMAs of every
+                  // page up to n - 8 are complete (the waits above), so the accumulators that they overwrote, those of the
+                  // items up to 8 before each, have been read.
+                  bulk_load_1d(base + kLiSmemScales + (n % kLiScaleRing) * kScaleBytes,
                                reinterpret_cast<const uint8_t*>(p.k_scale) + static_cast<int64_t>(scale_page) * scale_bytes,
                                scale_bytes, bar);
                 }
@@ -340,25 +378,31 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
           }
         }
       } else if (warp < kLiEpilogueWarp0) {
-        // ---------------- MMA issuers: warp w takes pages n with n % 2 == w - 1 ----------------
-        if (lane == 0) {
-          bool ok = mbar_wait(smem_u32(&ctl->qfull), seg & 1u);
-          if (!ok) set_status(p.status, PTO_ST_WAIT_EXPIRED, static_cast<int>(seg), 2);
-          const uint64_t b_desc = umma_desc_kmajor_sw128(q_base);
-          const uint64_t a_desc0 = umma_desc_kmajor_sw128(stage_base);
-          for (int j = 0; j < npages && ok; ++j) {
-            const uint32_t n = n_item + j;
-            if (static_cast<int>(n % kLiMmaWarps) != warp - 1) continue;
-            const uint32_t slot = n % n_slots;
-            const uint32_t ph = (n / n_slots) & 1u;
-            if (!mbar_wait(smem_u32(&ctl->full[slot]), ph)) {
-              ok = false;
-              set_status(p.status, PTO_ST_WAIT_EXPIRED, static_cast<int>(n), 3);
-              break;
-            }
-            tc_fence_after();
-            const uint64_t a_desc = a_desc0 + ((slot * kStage) >> 4);
-            const uint32_t d = tmem_base + slot * n_cols;
+        // ---------------- MMA issuers: warp w takes items n with n % 2 == w - 1 ----------------
+        // (the warp stays converged and an elected lane issues: the descriptors stay in uniform registers)
+        bool ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->qfull), seg & 1u));
+        if (!ok && lane == 0) set_status(p.status, PTO_ST_WAIT_EXPIRED, static_cast<int>(seg), 2);
+        const uint64_t b_desc0 = umma_desc_kmajor_sw128(q_base);
+        const uint64_t a_desc0 = umma_desc_kmajor_sw128(stage_base);
+        const int n_items = npages * items_per_page;
+        for (int j = static_cast<int>((n_item + static_cast<uint32_t>(warp - 1)) & 1u); j < n_items && ok; j += kLiMmaWarps) {
+          const uint32_t n = n_item + j;
+          const int half = items_per_page == 2 ? j & 1 : 0;
+          const uint32_t np = n_page + static_cast<uint32_t>(items_per_page == 2 ? j >> 1 : j);
+          const uint32_t stage = np % kStages, acc = n & (n_accs - 1u);
+          ok = mbar_wait(smem_u32(&ctl->accempty[acc]), ((n >> acc_shift) & 1u) ^ 1u) &&
+               mbar_wait(smem_u32(&ctl->full[stage]), (np / kStages) & 1u);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) {
+            if (lane == 0) set_status(p.status, PTO_ST_WAIT_EXPIRED, static_cast<int>(n), 3);
+            break;
+          }
+          tc_fence_after();
+          const uint64_t a_desc = a_desc0 + ((stage * kStage) >> 4);
+          const uint64_t b_desc = b_desc0 + (static_cast<uint32_t>(half * 2 * kQBytesPerToken) >> 4);  // (int8; bf16 has one item)
+          const uint32_t idesc = s1 - 2 * half >= 2 ? idesc2 : idesc1;
+          const uint32_t d = tmem_base + acc * unit_cols;
+          if (elect_one()) {
             if (kBf16) {
               // K = 16 bf16 (32 bytes) per instruction: four steps inside each 64-dim half
 #pragma unroll
@@ -371,74 +415,80 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
 #pragma unroll
               for (int k = 0; k < 4; ++k) mma_i8_ss(d, a_desc + 2 * k, b_desc + 2 * k, idesc, k > 0 ? 1u : 0u);
             }
-            tc_commit(smem_u32(&ctl->accfull[slot]));
+            tc_commit(smem_u32(&ctl->accfull[acc]));
+            tc_commit(smem_u32(&ctl->kempty[stage]));
           }
-          if (!ok) ctl->abort = 1;
+          __syncwarp();
         }
+        if (!ok && lane == 0) ctl->abort = 1;
         __syncwarp();
       } else {
         // ---------------- epilogue ----------------
         const int grp = (warp - kLiEpilogueWarp0) >> 2;
         const int quarter = warp & 3;  // TMEM lane quarter this warp may read
         const int row = quarter * 32 + lane;
-        // A slot belongs to one group, so that the group sees every use of the slot and consecutive waits on its
-        // barriers alternate in parity. (Taking pages n % 4 == grp is the same thing for 8 and 4 slots, but with
-        // the two slots of s1 = 3, 4 a group met only every second use of a slot: two waits in a row on the same
-        // parity, of which the second returned at once, before the page's products were there.) The ring has 8, 4
-        // or 2 slots, so group g owns the pages n with n % min(slots, 4) == g and walks them directly: stepping
-        // through every page and skipping three of four cost a tenth of the kernel's instructions.
-        const int gstride = static_cast<int>(n_slots < 4u ? n_slots : 4u);
-        const uint32_t slot_shift = 31u - static_cast<uint32_t>(__clz(static_cast<int>(n_slots)));
-        for (int j = (grp - static_cast<int>(n_item % static_cast<uint32_t>(gstride)) + gstride) % gstride;
-             grp < gstride && j < npages; j += gstride) {
+        // Group g takes the items n with n % 4 == g: there are 4 or 8 accumulators, so an accumulator belongs to one group,
+        // which sees every use of it, and consecutive waits on its barriers alternate in parity. (A group that met only
+        // every second use of an accumulator would wait twice in a row on the same parity, and the second wait would
+        // return at once, before the products are there.)
+        const int n_items = npages * items_per_page;
+        for (int j = (grp - static_cast<int>(n_item % kLiEpilogueGroups) + kLiEpilogueGroups) % kLiEpilogueGroups; j < n_items;
+             j += kLiEpilogueGroups) {
           const uint32_t n = n_item + j;
-          const uint32_t slot = n & (n_slots - 1u);
-          const uint32_t ph = (n >> slot_shift) & 1u;
-          if (!mbar_wait(smem_u32(&ctl->accfull[slot]), ph)) {
+          const uint32_t acc = n & (n_accs - 1u);
+          const int half = items_per_page == 2 ? j & 1 : 0;
+          const int page = items_per_page == 2 ? j >> 1 : j;
+          const uint32_t np = n_page + static_cast<uint32_t>(page);
+          const int cnt = min(2, s1 - 2 * half);  // query tokens of the item
+          if (!mbar_wait(smem_u32(&ctl->accfull[acc]), (n >> acc_shift) & 1u)) {
             ctl->abort = 1;
             set_status(p.status, PTO_ST_WAIT_EXPIRED, static_cast<int>(n), 4);
             break;
           }
           tc_fence_after();
-          // the page's scales came in with the page; its `full` phase has completed (the MMA issuer
-          // waited on it); observing it here orders this thread after the bulk copy
-          if (!kBf16) mbar_wait(smem_u32(&ctl->full[slot]), ph);
-          const uint8_t* sc_smem = smem + slot * kStage + kPageBytes;
+          // the page's scales came in with the page; its `full` phase has completed (the MMA issuer waited on it). Observing
+          // it here orders this thread after the bulk copy, unless the stage has been loaded again since: then the
+          // wait is for another page, which a bounded probe must not sit out, and the chain issuer -> accumulator orders
+          // the copy
+          if (!kBf16) mbar_test_wait(smem_u32(&ctl->full[np % kStages]), (np / kStages) & 1u);
+          const uint8_t* sc_smem = smem + kLiSmemScales + (np % kLiScaleRing) * kScaleBytes;
           float ks = 1.f;
           if (!kBf16) {
             ks = (p.scale_dtype == PTO_DT_F16) ? __half2float(reinterpret_cast<const __half*>(sc_smem)[row])
                                                : reinterpret_cast<const float*>(sc_smem)[row];
           }
-          const int pos = (page0 + j) * kPageKeys + row;
-          const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + slot * n_cols;
-          float res[kMaxS1];
+          __half2 ks2 = __float2half2_rn(0.f);
+          if (kChain) ks2 = __half2half2(reinterpret_cast<const __half*>(sc_smem)[row]);
+          const int pos = (page0 + page) * kPageKeys + row;
+          const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * unit_cols;
+          const float* ws = ctl->ws + half * 2 * kHeads;
+          float res[2];
 #pragma unroll
-          for (int i = 0; i < kMaxS1; ++i) {
-            if (i < s1) {
+          for (int i = 0; i < 2; ++i) {
+            if (i < cnt) {
               uint32_t v0[32], v1[32];
               tmem_ld_32x32b_x32(taddr + i * kHeads, v0);
               tmem_ld_32x32b_x32(taddr + i * kHeads + 32, v1);
               tc_wait_ld();
-              if (i == s1 - 1) {
-                // TMEM and the scale row are read: hand the slot back before the arithmetic
+              if (i == cnt - 1) {
+                // TMEM and the scale row are read: hand the accumulator back before the arithmetic
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&ctl->empty[slot]));
+                if (lane == 0) mbar_arrive(smem_u32(&ctl->accempty[acc]));
               }
               if (kBf16) {
-                res[i] = weighted_relu_sum_32(v0, ctl->ws + i * kHeads) + weighted_relu_sum_32(v1, ctl->ws + i * kHeads + 32);
+                res[i] = weighted_relu_sum_32(v0, ws + i * kHeads) + weighted_relu_sum_32(v1, ws + i * kHeads + 32);
               } else if (kChain) {
-                const __half2 ks2 = __half2half2(reinterpret_cast<const __half*>(sc_smem)[row]);
-                res[i] = __fadd_rn(chain_sum_32(v0, ctl->ws + i * kHeads, ks2), chain_sum_32(v1, ctl->ws + i * kHeads + 32, ks2));
+                res[i] = __fadd_rn(chain_sum_32(v0, ws + i * kHeads, ks2), chain_sum_32(v1, ws + i * kHeads + 32, ks2));
               } else {
-                res[i] = (weighted_sum_32(v0, ctl->ws + i * kHeads) + weighted_sum_32(v1, ctl->ws + i * kHeads + 32)) * ks;
+                res[i] = (weighted_sum_32(v0, ws + i * kHeads) + weighted_sum_32(v1, ws + i * kHeads + 32)) * ks;
               }
             }
           }
           if (pos < seq_len) {
 #pragma unroll
-            for (int i = 0; i < kMaxS1; ++i) {
-              if (i < s1) p.scores[(tok0 + i) * p.row_stride + pos] = res[i];
+            for (int i = 0; i < 2; ++i) {
+              if (i < cnt) p.scores[(tok0 + 2 * half + i) * p.row_stride + pos] = res[i];
             }
           }
           if (with_hist) {
@@ -446,7 +496,7 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
 #pragma unroll
             for (int i = 0; i < kLiHistMaxS1; ++i) {
               if (i < s1) {
-                const int eff = seq_len - (p.s1_total - 1 - (p.tok_offset + static_cast<int>(blockIdx.y) * p.s1 + i));
+                const int eff = seq_len - (p.s1_total - 1 - (tok_first + i));
                 if (pos < eff) atomicAdd(&hist_sm[i * kLiHistBins + (li_float_order(res[i]) >> kLiHistShift)], 1u);
               }
             }
@@ -454,8 +504,9 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
         }
       }
     }
-    n_item += npages;
-    cur = seg_end;
+    n_page += npages;
+    n_item += npages * items_per_page;
+    cur += npages;
     ++seg;
   }
 
@@ -565,14 +616,10 @@ cudaError_t launch_li_score_tc(const LiParams& p, const void* tmap_k, const void
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(kLiSmemBytes + kLiHistSmemBytes));
   if (e != cudaSuccess) return e;
-  // a launch that takes several token groups gives each group its share of the SMs: every CTA then walks more
-  // pages and the fixed cost of a launch (about 8 us) is paid once for all of them
-  const int groups = p.groups < 1 ? 1 : p.groups;
-  long long max_items = static_cast<long long>(p.b) * p.max_blocks;
-  const int per_group = num_sms / groups < 1 ? 1 : num_sms / groups;
-  int gx = static_cast<int>(max_items < per_group ? max_items : per_group);
+  const long long max_items = static_cast<long long>(p.b) * p.max_blocks * p.groups;
+  int gx = static_cast<int>(max_items < num_sms ? max_items : num_sms);
   if (gx < 1) gx = 1;
-  const dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(groups), 1);
+  const dim3 grid(static_cast<unsigned>(gx), 1, 1);
   count_launch();
   kernel<<<grid, kLiThreads, smem_bytes, stream>>>(*reinterpret_cast<const CUtensorMap*>(tmap_k),
                                                                  *reinterpret_cast<const CUtensorMap*>(tmap_q), p);
