@@ -12,6 +12,15 @@
 // 128-byte swizzle) and its key scales; per page and pair of query tokens (an item): four tcgen05.mma kind::i8
 // (M = 128 keys, N = 64 or 128 heads, K = 32) into a TMEM accumulator -> epilogue warps read their key's
 // row (one TMEM lane = one key), apply ReLU/2^-11/fp16 rounding and the weighted head sum, and write the fp32 score.
+// With two and more query tokens per pass the head sum is a second product (kLiQuantTc): the epilogue writes the fp16
+// values back over the accumulator, tcgen05.mma kind::f16 takes them as its A operand from TMEM (K = 64 heads), B is the
+// weights, and what comes back is the key's score. The weights of a token are fp32: B holds them as three fp16 limbs (33 bits below the token's largest weight, scaled to
+// 2^13 by a power of two). The tensor core truncates where it adds, so a column of the product takes sixteen heads of one
+// limb (one step of K; zeros elsewhere) and its twelve columns are added here. On
+// CUDA cores the head sum was the kernel's bound: unpacking the fp16 values and the multiply-adds were 1.5 of its 3.5
+// instructions per (key, head) and kept the half-rate FP16 / packed-FP32 pipe 70 % busy (16 x 65536 keys, two query
+// tokens 39.6 -> 37.4 us, four 66.0 -> 59.0; 256 tokens over 65536 keys 230 -> 192 us). With one query token the key
+// pages bound the kernel and the second product only adds to an item's latency (64 x 32768 keys 50.4 -> 51.9 us).
 // Warp roles: warp 0 TMA producer, warps 1..2 MMA issuers (alternate items; warp 1 owns TMEM),
 // warps 3..18 epilogue (four groups of four warps that take items round-robin; a single warp is
 // latency-bound on the conversion chain, so thread-level parallelism has to come from many warps).
@@ -31,7 +40,7 @@
 // most two query tokens of a sequence per pass, and the epilogue is max/fma on the fp32 accumulators.
 #include <cuda.h>
 
-#include "common.cuh"
+#include "sfa_common.cuh"
 
 namespace pto {
 
@@ -53,7 +62,7 @@ constexpr int kMaxS1 = 4;
 constexpr int kMaxSeqPerLaunch = 2048;
 constexpr int kTmemCols = 512;
 // score formulations the tensor-core kernel is instantiated for
-enum { kLiQuant = 0, kLiChain = 1, kLiBf16 = 2 };
+enum { kLiQuant = 0, kLiChain = 1, kLiBf16 = 2, kLiQuantTc = 3 };  // kLiQuantTc: the head sum on the tensor cores
 constexpr int kBf16PageBytes = kPageKeys * 256;  // one stage of the bf16 ring: the page's two 16 KB halves
 constexpr int kBf16Stages = 4;                   // 4 x 32 KB where the int8 ring keeps 8 x 16 KB
 constexpr int kBf16MaxS1 = 2;                    // 2 tokens x 64 heads x 256 B of queries fit the int8 Q area
@@ -66,15 +75,20 @@ struct LiCtl {
   uint64_t kempty[kLiStages];  // all MMAs that read the page completed (tcgen05.commit, one per item of the page)
   uint64_t accfull[kLiAccs];   // the item's MMAs completed (tcgen05.commit)
   uint64_t accempty[kLiAccs];  // the item's epilogue warps have read the accumulator
+  uint64_t sumfull[kLiAccs];   // the item's head sums completed (tcgen05.commit; int8 formulation)
   uint64_t qfull;
   uint32_t tmem_base;
   int abort;
   int prefix[kMaxSeqPerLaunch + 1];
   __align__(16) float ws[kMaxS1 * kHeads];
+  unsigned int wmax[kMaxS1][2];  // bit patterns of the largest |ws| of each half of a token's heads
+  float winv[kMaxS1];            // power of two that undoes the scaling of the limbs
 };
 
 constexpr size_t kLiHistSmemBytes = static_cast<size_t>(kLiHistMaxS1) * kLiHistBins * sizeof(unsigned int) + 16;  // 32 KB (+ alignment of its start)
-constexpr int kLiSmemScales = kLiStages * kPageBytes, kLiSmemQ = kLiSmemScales + kLiScaleRing * kScaleBytes;
+constexpr int kLimbBytes = 16 * 128;  // B operand of the head sum per token: 16 rows (limb x sixteen heads, four of zeros) of 64 heads
+constexpr int kLiSmemScales = kLiStages * kPageBytes, kLiSmemLimbs = kLiSmemScales + kLiScaleRing * kScaleBytes;
+constexpr int kLiSmemQ = kLiSmemLimbs + kMaxS1 * kLimbBytes;
 constexpr int kLiSmemCtl = kLiSmemQ + kMaxS1 * kQBytesPerToken;
 static_assert(kLiSmemQ % 1024 == 0, "swizzled query tile");
 constexpr size_t kLiSmemBytes = 1024 /*alignment slack*/ + kLiSmemCtl + sizeof(LiCtl);
@@ -96,13 +110,51 @@ __device__ __forceinline__ float load_ws(const void* qs, const void* w, int dtyp
 
 // relu(d) * 2^-11 rounded to fp16, for two dots at once; exact for |d| < 2^21:
 // adding d to the bit pattern of 6144.0f (ulp 2^-11) and subtracting 6144 gives d * 2^-11.
-__device__ __forceinline__ float2 relu_scale_round(int d0, int d1) {
+__device__ __forceinline__ uint32_t relu_scale_half2(int d0, int d1) {
   // the two subtractions as one packed fp32 instruction (each half is an ordinary IEEE subtraction)
   const float2 f = __fadd2_rn(make_float2(__int_as_float(0x45C00000 + d0), __int_as_float(0x45C00000 + d1)),
                               make_float2(-6144.0f, -6144.0f));
   uint32_t packed;  // round to fp16 and clamp negatives to zero in one conversion (f.x in the low half)
   asm("cvt.rn.relu.f16x2.f32 %0, %1, %2;" : "=r"(packed) : "f"(f.y), "f"(f.x));
-  return __half22float2(*reinterpret_cast<const __half2*>(&packed));
+  return packed;
+}
+
+// The same values weighted and summed on CUDA cores, 32 heads of one key.
+__device__ __forceinline__ float weighted_sum_32(const uint32_t (&v)[32], const float* ws) {
+  // four running sums as two packed pairs: one packed FMA per two heads (the same four chains of ordinary FMAs)
+  float2 a01 = make_float2(0.f, 0.f), a23 = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int c = 0; c < 32; c += 4) {
+    const float4 w = *reinterpret_cast<const float4*>(ws + c);
+    const uint32_t hx = relu_scale_half2(static_cast<int>(v[c]), static_cast<int>(v[c + 1]));
+    const uint32_t hy = relu_scale_half2(static_cast<int>(v[c + 2]), static_cast<int>(v[c + 3]));
+    a01 = __ffma2_rn(make_float2(w.x, w.y), __half22float2(*reinterpret_cast<const __half2*>(&hx)), a01);
+    a23 = __ffma2_rn(make_float2(w.z, w.w), __half22float2(*reinterpret_cast<const __half2*>(&hy)), a23);
+  }
+  return (a01.x + a01.y) + (a23.x + a23.y);
+}
+
+// named barrier of kThreads threads that returns the OR of their predicates: the same answer in every thread, so whoever
+// meets at later barriers stays together
+template <int kThreads>
+__device__ __forceinline__ bool li_vote(int id, bool pred) {
+  uint32_t any;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %2, 0;\n\tbarrier.cta.red.or.pred q, %1, %3, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(any)
+      : "r"(id), "r"(pred ? 1u : 0u), "n"(kThreads)
+      : "memory");
+  return any != 0;
+}
+
+// the twelve columns of a head sum (limb l of heads 16 s .. 16 s + 15 at 4 l + s) -> the sum in units of the largest limb
+__device__ __forceinline__ float limb_sum(const uint32_t (&r)[16]) {
+  float v[3];
+#pragma unroll
+  for (int l = 0; l < 3; ++l) {
+    v[l] = (__uint_as_float(r[4 * l]) + __uint_as_float(r[4 * l + 1])) + (__uint_as_float(r[4 * l + 2]) + __uint_as_float(r[4 * l + 3]));
+  }
+  return fmaf(fmaf(v[2], 1.0f / 2048.0f, v[1]), 1.0f / 2048.0f, v[0]);
 }
 
 // The older formulation for 32 heads of one key: table entries come in pairs, (q_scale_2p, q_scale_2p+1) and
@@ -123,20 +175,6 @@ __device__ __forceinline__ float chain_sum_32(const uint32_t (&v)[32], const flo
     acc = __fadd_rn(__fadd_rn(acc, m.x), m.y);
   }
   return acc;
-}
-
-__device__ __forceinline__ float weighted_sum_32(const uint32_t (&v)[32], const float* ws) {
-  // four running sums as two packed pairs: one packed FMA per two heads (the same four chains of ordinary FMAs)
-  float2 a01 = make_float2(0.f, 0.f), a23 = make_float2(0.f, 0.f);
-#pragma unroll
-  for (int c = 0; c < 32; c += 4) {
-    const float4 w = *reinterpret_cast<const float4*>(ws + c);
-    const float2 x = relu_scale_round(static_cast<int>(v[c]), static_cast<int>(v[c + 1]));
-    const float2 y = relu_scale_round(static_cast<int>(v[c + 2]), static_cast<int>(v[c + 3]));
-    a01 = __ffma2_rn(make_float2(w.x, w.y), x, a01);
-    a23 = __ffma2_rn(make_float2(w.z, w.w), y, a23);
-  }
-  return (a01.x + a01.y) + (a23.x + a23.y);
 }
 
 // Non-quantised formulation, 32 heads of one key: the accumulators are fp32 dots.
@@ -190,6 +228,7 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
     for (int i = 0; i < kLiAccs; ++i) {
       mbar_init(smem_u32(&ctl->accfull[i]), 1);
       mbar_init(smem_u32(&ctl->accempty[i]), 4);
+      mbar_init(smem_u32(&ctl->sumfull[i]), 1);
     }
     mbar_init(smem_u32(&ctl->qfull), 1);
     ctl->abort = 0;
@@ -200,6 +239,11 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
   }
   if (with_hist) {
     for (int j = tid; j < s1 * kLiHistBins; j += kLiThreads) hist_sm[j] = 0u;
+  }
+  if (kMode == kLiQuantTc) {  // (what is not written below stays zero)
+    for (int j = tid; j < kMaxS1 * kLimbBytes / 16; j += kLiThreads) {
+      *reinterpret_cast<uint4*>(smem + kLiSmemLimbs + j * 16) = make_uint4(0, 0, 0, 0);
+    }
   }
   if (warp == 1) {
     tmem_alloc(smem_u32(&ctl->tmem_base), kTmemCols);
@@ -288,10 +332,10 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
     // The producer warp takes no part in the two barriers of a segment: the ring's own barriers order its loads, so
     // the next segment's first pages are on their way while this one drains and the scale products are fetched.
     // previous segment fully drained: Q tile and ws may be overwritten
-    if (warp != 0) asm volatile("bar.sync 1, %0;" ::"n"(kLiThreads - 32) : "memory");
+    bool aborted = ctl->abort != 0;
+    if (warp != 0) aborted = li_vote<kLiThreads - 32>(1, aborted);
     if (with_hist && seg > 0) flush_hist(prev_tok0);  // (the barrier below orders it before the next segment's counts)
     prev_tok0 = tok0;
-    const bool aborted = ctl->abort != 0;
     if (!aborted) {
       if (warp == 1 && lane == 0) {
         if (kBf16) {
@@ -313,8 +357,31 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
           const __half2 two = __halves2half2(src[0], src[1]);
           reinterpret_cast<uint32_t*>(ctl->ws)[e] = *reinterpret_cast<const uint32_t*>(&two);
         } else {
-          ctl->ws[e] = load_ws(p.q_scale, p.weight, p.scale_dtype, tok0 * kHeads + e);
+          const float w = load_ws(p.q_scale, p.weight, p.scale_dtype, tok0 * kHeads + e);
+          ctl->ws[e] = w;
+          const unsigned int m = __reduce_max_sync(0xffffffffu, __float_as_uint(w) & 0x7fffffffu);  // (whole warps: 64 heads)
+          if (lane == 0) ctl->wmax[e >> 6][(e >> 5) & 1] = m;
         }
+      }
+    }
+    if (kMode == kLiQuantTc) {
+      if (warp != 0) asm volatile("bar.sync 1, %0;" ::"n"(kLiThreads - 32) : "memory");
+      const int e = tid - 32 * kLiEpilogueWarp0;
+      if (!aborted && e >= 0 && e < s1 * kHeads) {
+        const int i = e >> 6, h = e & 63;
+        const unsigned int m = max(ctl->wmax[i][0], ctl->wmax[i][1]);
+        const int ex = max(-100, min(127, static_cast<int>(m >> 23) - 127));  // 2^ex <= largest weight < 2^(ex + 1)
+        float r = ctl->ws[e] * __int_as_float((127 + 13 - ex) << 23);
+#pragma unroll
+        for (int l = 0; l < 3; ++l) {  // exact splitting: what a limb leaves over, scaled up by 2^11, goes to the next
+          const __half w = __float2half_rn(r);
+          // row (limb, sixteen heads) of 128 bytes (64 heads), 128-byte swizzle
+          const int rw = l * 4 + (h >> 4);
+          *reinterpret_cast<__half*>(smem + kLiSmemLimbs + i * kLimbBytes + rw * 128 + (((h >> 3) ^ (rw & 7)) << 4) + (h & 7) * 2) = w;
+          r = (r - __half2float(w)) * 2048.0f;
+        }
+        if (h == 0) ctl->winv[i] = __int_as_float((127 + ex - 13) << 23);
+        fence_proxy_async();
       }
     }
     // the scale products are visible to the MMA and epilogue warps
@@ -432,6 +499,7 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
         // every second use of an accumulator would wait twice in a row on the same parity, and the second wait would
         // return at once, before the products are there.)
         const int n_items = npages * items_per_page;
+        bool ok = true;
         for (int j = (grp - static_cast<int>(n_item % kLiEpilogueGroups) + kLiEpilogueGroups) % kLiEpilogueGroups; j < n_items;
              j += kLiEpilogueGroups) {
           const uint32_t n = n_item + j;
@@ -440,10 +508,11 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
           const int page = items_per_page == 2 ? j >> 1 : j;
           const uint32_t np = n_page + static_cast<uint32_t>(page);
           const int cnt = min(2, s1 - 2 * half);  // query tokens of the item
-          if (!mbar_wait(smem_u32(&ctl->accfull[acc]), (n >> acc_shift) & 1u)) {
+          ok = ok && mbar_wait(smem_u32(&ctl->accfull[acc]), (n >> acc_shift) & 1u);
+          if (!ok) {
             ctl->abort = 1;
             set_status(p.status, PTO_ST_WAIT_EXPIRED, static_cast<int>(n), 4);
-            break;
+            if (kMode != kLiQuantTc) break;
           }
           tc_fence_after();
           // the page's scales came in with the page; its `full` phase has completed (the MMA issuer waited on it). Observing
@@ -463,6 +532,61 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
           const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * unit_cols;
           const float* ws = ctl->ws + half * 2 * kHeads;
           float res[2];
+          if constexpr (kMode == kLiQuantTc) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              if (i < cnt) {
+                uint32_t h[32];  // the key's 64 values: K elements 2c, 2c + 1 of column c
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                  uint32_t v[32];
+                  tmem_ld_32x32b_x32(taddr + i * kHeads + 32 * u, v);
+                  tc_wait_ld();
+#pragma unroll
+                  for (int c = 0; c < 16; ++c) h[16 * u + c] = relu_scale_half2(static_cast<int>(v[2 * c]), static_cast<int>(v[2 * c + 1]));
+                }
+                tmem_st_32x32b_x32(taddr + i * kHeads, h);
+              }
+            }
+            tc_wait_st();
+            tc_fence_before();
+            // the group's four warps have written theirs; a wait that expired in one of them ends the loop for all four
+            if (li_vote<128>(2 + grp, !ok)) break;
+            if (((warp - kLiEpilogueWarp0) & 3) == 0) {
+              tc_fence_after();
+              constexpr uint32_t idesc_sum = umma_idesc(kCFmtF32, 0, 0, 0, 0, 128, 16);  // fp16 x fp16
+              const uint64_t w_desc = umma_desc_kmajor_sw128(base + kLiSmemLimbs) + ((half * 2 * kLimbBytes) >> 4);
+              const uint32_t unit = tmem_base + acc * unit_cols;
+              if (elect_one()) {
+                for (int i = 0; i < cnt; ++i) {
+#pragma unroll
+                  for (int k = 0; k < 4; ++k) {  // K = 16 heads: eight columns of A, 32 bytes of B's rows
+                    mma_f16_ts(unit + i * kHeads + 32, unit + i * kHeads + 8 * k, w_desc + i * (kLimbBytes >> 4) + 2 * k, idesc_sum,
+                               k > 0 ? 1u : 0u);
+                  }
+                }
+                tc_commit(smem_u32(&ctl->sumfull[acc]));
+              }
+              __syncwarp();
+            }
+            ok = mbar_wait(smem_u32(&ctl->sumfull[acc]), (n >> acc_shift) & 1u);
+            if (!ok) {  // the group leaves together, at its next barrier
+              ctl->abort = 1;
+              set_status(p.status, PTO_ST_WAIT_EXPIRED, static_cast<int>(n), 6);
+            }
+            tc_fence_after();
+            uint32_t r[2][16];
+            tmem_ld_32x32b_x16(taddr + 32, r[0]);
+            if (cnt > 1) tmem_ld_32x32b_x16(taddr + kHeads + 32, r[1]);
+            tc_wait_ld();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&ctl->accempty[acc]));
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              if (i < cnt) res[i] = limb_sum(r[i]) * ctl->winv[half * 2 + i] * ks;
+            }
+          } else {
 #pragma unroll
           for (int i = 0; i < 2; ++i) {
             if (i < cnt) {
@@ -478,12 +602,13 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
               }
               if (kBf16) {
                 res[i] = weighted_relu_sum_32(v0, ws + i * kHeads) + weighted_relu_sum_32(v1, ws + i * kHeads + 32);
-              } else if (kChain) {
-                res[i] = __fadd_rn(chain_sum_32(v0, ws + i * kHeads, ks2), chain_sum_32(v1, ws + i * kHeads + 32, ks2));
-              } else {
+              } else if (kMode == kLiQuant) {
                 res[i] = (weighted_sum_32(v0, ws + i * kHeads) + weighted_sum_32(v1, ws + i * kHeads + 32)) * ks;
+              } else {
+                res[i] = __fadd_rn(chain_sum_32(v0, ws + i * kHeads, ks2), chain_sum_32(v1, ws + i * kHeads + 32, ks2));
               }
             }
+          }
           }
           if (pos < seq_len) {
 #pragma unroll
@@ -610,7 +735,7 @@ li_score_simt_kernel(LiParams p) {
 cudaError_t launch_li_score_tc(const LiParams& p, const void* tmap_k, const void* tmap_q, int num_sms,
                                cudaStream_t stream) {
   auto kernel = p.bf16 ? li_score_tc_kernel<kLiBf16>
-                       : (p.fp16_chain ? li_score_tc_kernel<kLiChain> : li_score_tc_kernel<kLiQuant>);
+                       : (p.fp16_chain ? li_score_tc_kernel<kLiChain> : (p.s1 > 1 ? li_score_tc_kernel<kLiQuantTc> : li_score_tc_kernel<kLiQuant>));
   if (p.hist != nullptr && p.s1 > kLiHistMaxS1) return cudaErrorInvalidValue;
   const size_t smem_bytes = kLiSmemBytes + (p.hist != nullptr ? kLiHistSmemBytes : 0);
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -215,6 +215,21 @@ def test_fp16_chain_needs_fp16_scales():
                                      g.act_seq_key, g.block_table, sc, None, fp16_chain=True)
 
 
+@pytest.mark.parametrize("s1", [1, 2, 3, 4])
+@pytest.mark.parametrize("spread", [0, 12, 30])
+def test_head_weights_of_very_different_size(s1, spread):
+    """The head sum takes fp32 weights as limbs of a common scale (two and more query tokens): weights that span 2^spread,
+    a token whose weights are all zero, and the CUDA-core kernel's fp32 sums as the reference."""
+    d = gen.make_inputs([700, 130], s1=s1, seed=60 + s1)
+    g = torch.Generator().manual_seed(spread)
+    d.idx_weight = d.idx_weight * torch.pow(2.0, -torch.randint(0, spread + 1, d.idx_weight.shape, generator=g).float())
+    d.idx_weight[-1] = 0
+    got, want = _scores(d, False)[0], _scores(d, True)[0]
+    for ti in range(d.t):
+        n = d.act_seq[ti // s1]
+        torch.testing.assert_close(got[ti, :n], want[ti, :n], rtol=3e-6, atol=float(want[ti, :n].abs().max()) * 1e-6)
+
+
 @pytest.mark.parametrize("s1", [3, 4])
 def test_three_and_four_query_tokens_with_many_pages_per_cta(s1):
     """s1 = 3, 4 leave room for two accumulator slots only; with more than four pages per CTA every slot is
