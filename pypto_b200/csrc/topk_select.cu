@@ -6,25 +6,26 @@
 // are valid and the rest is -1; eff <= 0 gives all -1. Ties are broken toward the smaller position,
 // which makes the result deterministic (torch.topk leaves tie order unspecified).
 //
-// One cluster of 1, 2, 4 or 8 CTAs per row (as many as keep the grid within one wave of SMs). The
-// scanning passes (1-3) are split over the CTAs of the cluster by position range; what they must agree
-// on travels through distributed shared memory: the range's min/max, the histogram (added into rank
-// every other rank's with remote atomics), the per-rank counts. In the unordered mode every rank writes
-// the positions it selected straight to the output at its offset and pushes only its candidates of
-// the threshold bucket into rank 0's list; in the ordered mode the selected keys are pushed too.
-// Every element is mapped to a unique 64-bit key (order-preserving image of the
-// float in the high word, ~position in the low word), so "the k largest keys" is well defined.
-//   1. min/max of the row                    2. 2048-bin histogram over a monotone linear bucket map
-//   3. bucket above the threshold bucket -> selected; threshold bucket -> candidate buffer (shared)
-//   4. candidates sorted (bitonic) and the best `need` appended; if the threshold bucket does not
-//      fit the buffer (massive ties), an MSB-first radix select over the 64-bit keys runs on the row
-//   5. the k selected keys are sorted (bitonic) and the positions written.
+// Every element is mapped to a unique 64-bit key (order-preserving image of the float in the high word, ~position in the
+// low word), so "the k largest keys" is well defined.
+//   1. Lower bound. A sample of the row (4096 values or more, groups of four spread over it) gives a value that about k +
+//      4.5 standard deviations elements exceed. Rows of at most 6144 positions skip this: all of them are the list.
+//   2. One scan of the row, which bulk copies bring into shared memory meanwhile, collects the keys at or above the bound
+//      into a list of up to 6144. It is split over a cluster of 1, 2, 4 or 8 CTAs (as many as keep the grid within one
+//      wave of SMs), each of which finds the bound for itself; the lists travel to rank 0 through distributed shared
+//      memory.
+//   3. Rank 0 distributes the list over 2048 bins that divide its value range, a prefix sum over the bins gives every bin
+//      its place in the order, and a key's place within its bin is the number of larger keys there (a bin holds a
+//      few keys). The first k places are the result; a caller that asked for no order gets the whole bins as they are.
+// A list that is too long or too short, or a bin of more than 512 keys (massive ties, infinite values), sends the row to
+// an MSB-first radix select over the 64-bit keys on rank 0.
+// What bounds it: one trip of the row from L2 (the first version scanned it three times, for its extremes, a histogram
+// and the collection, with a cluster barrier behind each, and ordered its result with a bitonic sort) and about a dozen
+// block barriers. Before -> after, alone: one row of 4096 12.4 -> 6.3 us (in order 18.5 -> 8.3), 8 x 32768 in order
+// 26.7 -> 12.4, 64 x 65536 16.5 -> 14.4, 256 x 131072 86 -> 54, 1024 x 131072 295 -> 181 us.
 // When the score kernel has left a histogram of the row (4096 bins over the top 12 bits of the order-preserving
-// image of the float, counted over the positions below the row's causal end), passes 1 and 2 are skipped: the
-// threshold bin comes from that histogram and pass 3 is the only scan of the row. The histogram is used only if
-// its total equals the row's length and its threshold bin fits the candidate buffer; otherwise passes 1-2 run.
-#include <cstdlib>
-
+// image of the float, counted over the positions below the row's causal end), the bound comes from it instead of the sample,
+// if its total equals the row's length and the list it leads to is not too long.
 #include "common.cuh"
 
 namespace pto {
@@ -40,33 +41,40 @@ __device__ long long g_topk_tl[16];
 #define TKT(i) do { } while (0)
 #endif
 
-constexpr int kTopkThreads = 1024;
+constexpr int kTopkThreads = 512;  // (1024 threads wait longer at each of the dozen barriers than they save between them)
+constexpr int kTopkWarps = kTopkThreads / 32;
 constexpr int kBins = 2048;
-constexpr int kHistSlots = kLiHistBins > kBins ? kLiHistBins : kBins;
 constexpr int kMaxK = 2048;
-constexpr int kCandCap = 4096;
-constexpr int kRowCap = 32768;  // positions of a rank's share that stay in shared memory between the scans
+constexpr int kListCap = 6144;
+constexpr int kChunk = 16 * kTopkThreads;  // positions per bulk copy
+constexpr int kRing = 3;                   // copies in flight (96 KB)
+constexpr int kWarpCap = kListCap / kTopkWarps;  // keys a warp collects before they go to the list
+constexpr int kBinCap = 512;               // keys of a bin that are still ranked by counting
+static_assert(kMaxK <= kListCap, "a row of at most k positions is handled as a list");
 
 struct TopkSmem {
-  unsigned long long sel[kMaxK];
-  unsigned long long cand[kCandCap];
-  unsigned int hist[kHistSlots];
+  union {
+    float ring[kRing][kChunk];             // the row on its way through (until the list is complete)
+    struct {
+      unsigned long long sorted[kMaxK + kBinCap];
+      unsigned int base[kBins];            // place of a bin's first key
+    };
+  };
+  unsigned long long list[kListCap];       // rank 0: the candidates of the row
+  unsigned long long mine[kTopkWarps][kWarpCap];  // the keys each warp of this CTA collected
+  unsigned int hist[kLiHistBins > kBins ? kLiHistBins : kBins];
   unsigned int warp_tot[32];
+  unsigned int warp_n[32];
+  unsigned int red_min[32], red_max[32];   // order-preserving images
+  uint64_t full[kRing];                    // bytes of a chunk landed
+  uint64_t empty[kRing];                   // every warp has read it
+  unsigned int n_list;                     // rank 0: keys in `list` (more than kListCap: some are missing)
+  unsigned int offset;                     // of this CTA's keys in the list
   unsigned int hist_total;
-  float red_min[32];
-  float red_max[32];
   unsigned int n_sel;
-  unsigned int n_cand;
-  unsigned int n_sel2, n_cand2;  // second radix step over the candidates of a coarse bin
-  // values every rank of the cluster publishes into every other rank's copy (remote stores, made visible
-  // by the next cluster barrier), so that nobody waits for a chain of remote loads
-  float all_min[8], all_max[8];
-  unsigned int all_sel[8], all_cand[8];
   int thr_bin;
   unsigned int thr_above;
   unsigned int thr_count;
-  // this rank's share of the row, kept from the first scan for the other two (when it fits)
-  __align__(16) float row[kRowCap];
 };
 
 __device__ __forceinline__ unsigned int cluster_rank() {
@@ -79,10 +87,8 @@ __device__ __forceinline__ unsigned int cluster_size() {
   asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
   return r;
 }
-// all threads of all CTAs of the cluster; orders shared-memory accesses across the cluster
-__device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ uint32_t peer_addr(const void* local, unsigned int rank) {
   uint32_t r;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(local)), "r"(rank));
@@ -94,8 +100,10 @@ __device__ __forceinline__ void st_peer_u64(uint32_t a, unsigned long long v) {
 __device__ __forceinline__ void st_peer_u32(uint32_t a, unsigned int v) {
   asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
-__device__ __forceinline__ void red_peer_add_u32(uint32_t a, unsigned int v) {
-  asm volatile("red.relaxed.cluster.shared::cluster.add.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+__device__ __forceinline__ unsigned int atom_peer_add_u32(uint32_t a, unsigned int v) {
+  unsigned int old;
+  asm volatile("atom.relaxed.cluster.shared::cluster.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(a), "r"(v) : "memory");
+  return old;
 }
 
 __device__ __forceinline__ unsigned int float_order(float f) {
@@ -108,6 +116,11 @@ __device__ __forceinline__ unsigned long long make_key(float f, int pos) {
 __device__ __forceinline__ int key_pos(unsigned long long key) {
   return static_cast<int>(~static_cast<unsigned int>(key & 0xffffffffull));
 }
+
+__device__ __forceinline__ float order_float(unsigned int o) {  // inverse of float_order
+  return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
+}
+__device__ __forceinline__ float key_value(unsigned long long key) { return order_float(static_cast<unsigned int>(key >> 32)); }
 
 // Descending bitonic sort of n (power of two) keys in shared memory; all threads of the CTA call it.
 // Shared-memory version: pair t of a stage is handled by thread t (and t + blockDim, ...), so for strides
@@ -196,9 +209,10 @@ __device__ void bitonic_sort_desc(unsigned long long* buf, int n) {
   __syncthreads();
 }
 
-// Finds, scanning the histogram of kPer * 1024 bins from the top bin down, the bin where the running count reaches
+// Finds, scanning the histogram of kPer * kTopkThreads bins from the top bin down, the bin where the running count reaches
 // `need`. Results in sm->thr_bin (bin), thr_above (count in bins above it), thr_count (its count), hist_total.
-template <int kPer>
+// kBase: every bin's count of the bins above it goes to sm->base.
+template <int kPer, bool kBase = false>
 __device__ void find_threshold_bin(TopkSmem* sm, unsigned int need) {
   constexpr int kN = kPer * kTopkThreads;
   const int tid = threadIdx.x;
@@ -220,7 +234,7 @@ __device__ void find_threshold_bin(TopkSmem* sm, unsigned int need) {
   if (lane == 31) sm->warp_tot[warp] = incl;
   __syncthreads();
   if (warp == 0) {
-    unsigned int w = sm->warp_tot[lane];
+    unsigned int w = lane < kTopkWarps ? sm->warp_tot[lane] : 0u;
     unsigned int wi = w;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -239,38 +253,99 @@ __device__ void find_threshold_bin(TopkSmem* sm, unsigned int need) {
       sm->thr_above = run;
       sm->thr_count = c[e];
     }
+    if constexpr (kBase) sm->base[kN - 1 - kPer * tid - e] = run;
     run += c[e];
   }
   __syncthreads();
 }
 
-// Applies f(value, position) to every element of row[0, eff). Loads go through the read-only path
-// and are issued four 16-byte loads at a time before the bodies run, so the latency of one batch is
-// paid once (the bodies contain shared-memory atomics the compiler will not move loads across).
-template <bool kGlobal, typename F>
-__device__ __forceinline__ void for_each_element(const float* row, int begin, int end, F&& f) {
+// Monotone map of a value range to the bins. Values that are not finite, or a range that is not, end up in bin 0.
+struct BinMap {
+  float lo, inv;
+  __device__ __forceinline__ void set(float vmin, float vmax) {
+    lo = vmin;
+    inv = 0.f;
+    const float range = vmax - vmin;
+    if (range > 0.f && range < INFINITY) inv = static_cast<float>(kBins - 1) / range;
+    if (!(inv < INFINITY)) inv = 0.f;
+  }
+  __device__ __forceinline__ int bin(float v) const { return max(0, min(kBins - 1, static_cast<int>((v - lo) * inv))); }
+};
+
+// block-wide minimum and maximum, returned to every thread (one barrier)
+__device__ __forceinline__ void block_range(TopkSmem* sm, float& vmin, float& vmax) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned int lo = __reduce_min_sync(0xffffffffu, float_order(vmin)), hi = __reduce_max_sync(0xffffffffu, float_order(vmax));
+  if (lane == 0) {
+    sm->red_min[warp] = lo;
+    sm->red_max[warp] = hi;
+  }
+  __syncthreads();
+  vmin = order_float(__reduce_min_sync(0xffffffffu, sm->red_min[lane & (kTopkWarps - 1)]));
+  vmax = order_float(__reduce_max_sync(0xffffffffu, sm->red_max[lane & (kTopkWarps - 1)]));
+}
+
+// Lower bound of the k largest of row[0, eff) from a sample: 1024 groups of four (or a multiple of that), evenly spread. About
+// k + 4.5 standard deviations elements exceed the value returned. -inf: no useful bound.
+__device__ float sample_bound(TopkSmem* sm, const float* row, int eff, int k) {
   const int tid = threadIdx.x;
-  const int n4 = begin + ((end - begin) & ~3);  // begin is a multiple of 4
-  constexpr int kStep = kTopkThreads * 4;
-  for (int j0 = begin + tid * 4; j0 < n4; j0 += 4 * kStep) {
-    float4 v[4];
+  const int groups = eff >> 2;
+  // groups per thread: long rows need a larger sample for a list of the same length
+  constexpr int kMaxPer = 4096 / kTopkThreads;
+  const int per = (eff <= (1 << 16) ? 1024 : (eff <= (1 << 18) ? 2048 : 4096)) / kTopkThreads;
+  float4 v[kMaxPer];
+  float vmin = INFINITY, vmax = -INFINITY;
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int j = j0 + u * kStep;
-      if (j < n4) v[u] = kGlobal ? __ldg(reinterpret_cast<const float4*>(row + j)) : *reinterpret_cast<const float4*>(row + j);
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int j = j0 + u * kStep;
-      if (j < n4) {
-        f(v[u].x, j);
-        f(v[u].y, j + 1);
-        f(v[u].z, j + 2);
-        f(v[u].w, j + 3);
-      }
+  for (int u = 0; u < kMaxPer; ++u) {
+    if (u < per) {
+      const int g = static_cast<int>(static_cast<long long>(tid + u * kTopkThreads) * groups / (kTopkThreads * per));
+      v[u] = __ldg(reinterpret_cast<const float4*>(row) + g);
     }
   }
-  for (int j = n4 + tid; j < end; j += kTopkThreads) f(kGlobal ? __ldg(row + j) : row[j], j);
+#pragma unroll
+  for (int u = 0; u < kMaxPer; ++u) {
+    if (u < per) {
+      vmin = fminf(vmin, fminf(fminf(v[u].x, v[u].y), fminf(v[u].z, v[u].w)));
+      vmax = fmaxf(vmax, fmaxf(fmaxf(v[u].x, v[u].y), fmaxf(v[u].z, v[u].w)));
+    }
+  }
+  for (int j = tid; j < kBins; j += kTopkThreads) sm->hist[j] = 0;
+  block_range(sm, vmin, vmax);
+  BinMap map;
+  map.set(vmin, vmax);
+#pragma unroll
+  for (int u = 0; u < kMaxPer; ++u) {
+    if (u < per) {
+      atomicAdd(&sm->hist[map.bin(v[u].x)], 1u);
+      atomicAdd(&sm->hist[map.bin(v[u].y)], 1u);
+      atomicAdd(&sm->hist[map.bin(v[u].z)], 1u);
+      atomicAdd(&sm->hist[map.bin(v[u].w)], 1u);
+    }
+  }
+  __syncthreads();
+  const float mean = static_cast<float>(k) * static_cast<float>(4 * kTopkThreads * per) / static_cast<float>(eff);
+  find_threshold_bin<kBins / kTopkThreads>(sm, static_cast<unsigned int>(mean + 4.5f * sqrtf(mean) + 4.0f));
+  const int b = sm->thr_bin;
+  if (map.inv == 0.f || b == 0) return -INFINITY;
+  return map.lo + static_cast<float>(b) / map.inv;
+}
+
+// Applies f(value, position) to every element of row[0, eff). Loads are issued four at a time before the bodies run, so the
+// latency of one batch is paid once (the bodies contain shared-memory atomics the compiler will not move loads across).
+template <typename F>
+__device__ __forceinline__ void for_each_element(const float* row, int eff, F&& f) {
+  const int tid = threadIdx.x;
+  for (int j0 = tid; j0 < eff; j0 += 4 * kTopkThreads) {
+    float v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (j0 + u * kTopkThreads < eff) v[u] = __ldg(row + j0 + u * kTopkThreads);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (j0 + u * kTopkThreads < eff) f(v[u], j0 + u * kTopkThreads);
+    }
+  }
 }
 
 __global__ void __launch_bounds__(kTopkThreads, 1)
@@ -286,395 +361,320 @@ li_topk_kernel(TopkParams p) {
   const int row_id = blockIdx.x / csize;
   const int bi = row_id / p.s1;
   const int i = row_id % p.s1;
-  const int k = p.k;
-  int32_t* out = p.out + static_cast<int64_t>(row_id) * k;
+  int32_t* out = p.out + static_cast<int64_t>(row_id) * p.k;
   const float* row = p.scores + static_cast<int64_t>(row_id) * p.row_stride;
   // the row's length is an input of the call, not a result of the score kernel: its trip to memory runs while
   // this grid still waits for that kernel
   int eff = p.act_seq[bi] - (p.s1 - 1 - i);
   if (eff > p.row_stride) eff = static_cast<int>(p.row_stride);
-  const bool unsorted = (p.flags & PTO_LI_UNSORTED) != 0;
+  const int k = min(p.k, eff);  // entries of the result
+  if (tid == 0) {
+    for (int c = 0; c < kRing; ++c) {
+      mbar_init(smem_u32(&sm->full[c]), 1);
+      mbar_init(smem_u32(&sm->empty[c]), kTopkWarps);
+    }
+    fence_mbar_init();
+    fence_proxy_async();
+    sm->n_list = 0;
+    sm->n_sel = 0;
+    sm->thr_bin = 0;
+  }
+  const bool whole = eff <= kListCap;         // the list is the row: rank 0 alone, no cluster barrier on this path
+  if (!whole && csize > 1) cluster_arrive();  // (rank 0's counter is set before anyone adds to it)
   pdl_wait();
   pdl_trigger();
   TKT(1);
-
-  // short rows: rank 0 alone, no cluster barrier on this path (every CTA of the cluster takes it)
-  if (eff <= k) {
-    if (rank != 0) return;
-    if (eff <= 0) {
-      for (int j = tid; j < k; j += kTopkThreads) out[j] = -1;
-      return;
-    }
-    int kpow2 = 1;
-    while (kpow2 < k) kpow2 <<= 1;
-    for (int j = tid; j < kpow2; j += kTopkThreads) sm->sel[j] = (j < eff) ? make_key(row[j], j) : 0ull;
-    if (!unsorted) bitonic_sort_desc(sm->sel, kpow2); else __syncthreads();
-    for (int j = tid; j < k; j += kTopkThreads) out[j] = (j < eff) ? key_pos(sm->sel[j]) : -1;
+  if (rank == 0) {
+    for (int j = max(k, 0) + tid; j < p.k; j += kTopkThreads) out[j] = -1;
+  }
+  if (eff <= 0 || (whole && rank != 0)) return;
+  if (eff <= p.k && (p.flags & PTO_LI_UNSORTED) != 0) {  // everything is selected and the order is free
+    for (int j = tid; j < eff; j += kTopkThreads) out[j] = j;  // (k <= kListCap: `whole`, so this is rank 0)
     return;
   }
-  int kpow2 = 1;
-  while (kpow2 < k) kpow2 <<= 1;
 
-  // this rank's share of the positions (a multiple of 4 so that 16-byte loads stay aligned)
-  const int chunk = (((eff + static_cast<int>(csize) - 1) / static_cast<int>(csize)) + 3) & ~3;
-  const int begin = min(eff, static_cast<int>(rank) * chunk);
-  const int end = min(eff, begin + chunk);
-
-  // ---- 0. the score kernel's histogram of the row, when there is one ------------------------------
-  bool coarse = false;
-  float vmin = 0.f, inv = 0.f;
-  if (p.hist != nullptr) {
-    const uint4* h4 = reinterpret_cast<const uint4*>(p.hist + static_cast<int64_t>(row_id) * kLiHistBins);
-    static_assert(kLiHistBins == 4 * kTopkThreads, "one 16-byte load per thread");
-    reinterpret_cast<uint4*>(sm->hist)[tid] = __ldg(h4 + tid);
-    if (tid == 0) {
-      sm->n_sel = 0;
-      sm->n_cand = 0;
-    }
+  float lmin = INFINITY, lmax = -INFINITY;  // range of the list
+  unsigned int n_list, n_front = kListCap;  // the first n_front keys at the front, the others from the end backwards
+  auto key_at = [&](unsigned int j) { return sm->list[j < n_front ? j : kListCap - 1 - (j - n_front)]; };
+  if (whole) {
     __syncthreads();
-    find_threshold_bin<kLiHistBins / kTopkThreads>(sm, static_cast<unsigned int>(k));
-    // usable if it counted exactly this row's positions and its threshold bin fits the candidate buffer; the
-    // same answer in every rank of the cluster (all read the same histogram)
-    coarse = sm->hist_total == static_cast<unsigned int>(eff) && sm->thr_count <= static_cast<unsigned int>(kCandCap);
-    __syncthreads();  // every thread has read the outcome before the histogram area is reused
-  }
-  auto bucket = [&](float v) -> int {
-    if (coarse) return static_cast<int>(float_order(v) >> kLiHistShift);
-    const float x = (v - vmin) * inv;
-    int bkt = static_cast<int>(x);
-    bkt = max(0, min(kBins - 1, bkt));
-    return bkt;
-  };
-  // the share stays in shared memory between the scans when it fits (not when the first scan is skipped)
-  const bool resident = !coarse && (end - begin) <= kRowCap;
-  TKT(2);
-  if (!coarse) {
-    // ---- 1. row min / max -------------------------------------------------------------------
-    vmin = INFINITY;
-    float vmax = -INFINITY;
-    {
-      // the one scan that reads the row from global memory (L2): this rank's share also goes into shared memory,
-      // where the other two scans read it (three trips to L2 were three of the latencies this kernel consists of)
-      const int n4 = begin + ((end - begin) & ~3);
-      constexpr int kStep = kTopkThreads * 4;
-      for (int j0 = begin + tid * 4; j0 < n4; j0 += 4 * kStep) {
-        float4 v[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int j = j0 + u * kStep;
-          if (j < n4) v[u] = __ldg(reinterpret_cast<const float4*>(row + j));
-        }
+    for (int u = 0; u < (kListCap / 4 + kTopkThreads - 1) / kTopkThreads; ++u) {
+      const int j = 4 * (tid + u * kTopkThreads);
+      if (j < eff) {
+        const float4 v = __ldg(reinterpret_cast<const float4*>(row + j));  // (rows are a multiple of 4 long)
+        const float x[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int j = j0 + u * kStep;
-          if (j < n4) {
-            vmin = fminf(fminf(vmin, fminf(v[u].x, v[u].y)), fminf(v[u].z, v[u].w));
-            vmax = fmaxf(fmaxf(vmax, fmaxf(v[u].x, v[u].y)), fmaxf(v[u].z, v[u].w));
-            if (resident) *reinterpret_cast<float4*>(sm->row + (j - begin)) = v[u];
+        for (int e = 0; e < 4; ++e) {
+          if (j + e < eff) {
+            sm->list[j + e] = make_key(x[e], j + e);
+            lmin = fminf(lmin, x[e]);
+            lmax = fmaxf(lmax, x[e]);
           }
         }
       }
-      for (int j = n4 + tid; j < end; j += kTopkThreads) {
-        const float v = __ldg(row + j);
-        vmin = fminf(vmin, v);
-        vmax = fmaxf(vmax, v);
-        if (resident) sm->row[j - begin] = v;
-      }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      vmin = fminf(vmin, __shfl_xor_sync(0xffffffffu, vmin, o));
-      vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
-    }
-    if (lane == 0) {
-      sm->red_min[warp] = vmin;
-      sm->red_max[warp] = vmax;
-    }
-    for (int j = tid; j < kBins; j += kTopkThreads) sm->hist[j] = 0;
-    if (tid == 0) {
-      sm->n_sel = 0;
-      sm->n_cand = 0;
-    }
-    __syncthreads();
-    vmin = sm->red_min[lane];
-    vmax = sm->red_max[lane];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      vmin = fminf(vmin, __shfl_xor_sync(0xffffffffu, vmin, o));
-      vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
-    }
-    if (csize > 1) {
-      if (tid < csize) {  // thread r tells rank r
-        st_peer_u32(peer_addr(&sm->all_min[rank], tid), __float_as_uint(vmin));
-        st_peer_u32(peer_addr(&sm->all_max[rank], tid), __float_as_uint(vmax));
-      }
-      cluster_barrier();
-      for (unsigned int r = 0; r < csize; ++r) {  // every rank arrives at the same pair
-        vmin = fminf(vmin, sm->all_min[r]);
-        vmax = fmaxf(vmax, sm->all_max[r]);
-      }
-    }
-    // monotone bucket map: floor((v - vmin) * inv), clamped. Non-finite range -> everything in bin 0
-    // and the radix fallback resolves it.
-    {
-      const float range = vmax - vmin;
-      if (range > 0.f && range < INFINITY) inv = static_cast<float>(kBins - 1) / range;
-      if (!(inv < INFINITY)) inv = 0.f;
-    }
-
-    TKT(3);
-    // ---- 2. histogram -----------------------------------------------------------------------
-    {
-      auto count = [&](float v, int) { atomicAdd(&sm->hist[bucket(v)], 1u); };
-      if (resident) for_each_element<false>(sm->row - begin, begin, end, count);
-      else for_each_element<true>(row, begin, end, count);
-    }
-    __syncthreads();
-    if (csize == 2) {
-      // two ranks: each stores its counts into the free upper half of the other's histogram area (plain remote
-      // stores, all bins), one cluster barrier, and adds what it received to its own
-      static_assert(kHistSlots >= 2 * kBins, "no room for the peer's counts");
-#pragma unroll
-      for (int u = 0; u < kBins / kTopkThreads; ++u) {
-        const int bin = tid + u * kTopkThreads;
-        st_peer_u32(peer_addr(&sm->hist[kBins + bin], rank ^ 1u), sm->hist[bin]);
-      }
-      cluster_barrier();
-#pragma unroll
-      for (int u = 0; u < kBins / kTopkThreads; ++u) {
-        const int bin = tid + u * kTopkThreads;
-        sm->hist[bin] += sm->hist[kBins + bin];
-      }
-      __syncthreads();
-    } else if (csize > 1) {
-      // every rank adds its counts into every other rank's histogram; a rank must not receive additions
-      // before its own pass is over (they would be indistinguishable from its own counts only after it)
-      unsigned int mine[kBins / kTopkThreads];
-#pragma unroll
-      for (int u = 0; u < kBins / kTopkThreads; ++u) mine[u] = sm->hist[tid + u * kTopkThreads];
-      cluster_barrier();  // all local histograms complete and read into registers
-#pragma unroll
-      for (int u = 0; u < kBins / kTopkThreads; ++u) {
-        if (mine[u] != 0) {
-          for (unsigned int r = 0; r < csize; ++r) {
-            if (r != rank) red_peer_add_u32(peer_addr(&sm->hist[tid + u * kTopkThreads], r), mine[u]);
-          }
-        }
-      }
-      cluster_barrier();  // every rank holds the row's histogram
-    }
-    TKT(4);
-    find_threshold_bin<kBins / kTopkThreads>(sm, static_cast<unsigned int>(k));  // the same answer in every rank
-  }
-  TKT(5);
-  const int thr_bin = sm->thr_bin;
-  const unsigned int above = sm->thr_above;
-  const unsigned int thr_count = sm->thr_count;
-  const unsigned int need = static_cast<unsigned int>(k) - above;  // to take from the threshold bucket
-
-  if (thr_count <= static_cast<unsigned int>(kCandCap)) {
-    // ---- 3. collect (this rank's positions) ---------------------------------------------------
-    {
-      auto collect = [&](float v, int pos) {
-        const int bkt = bucket(v);
-        if (bkt > thr_bin) {
-          sm->sel[atomicAdd(&sm->n_sel, 1u)] = make_key(v, pos);
-        } else if (bkt == thr_bin) {
-          sm->cand[atomicAdd(&sm->n_cand, 1u)] = make_key(v, pos);
-        }
-      };
-      if (resident) for_each_element<false>(sm->row - begin, begin, end, collect);
-      else for_each_element<true>(row, begin, end, collect);
-    }
-    __syncthreads();
-    TKT(6);
-    unsigned int direct_base = above;  // first output slot of the keys chosen among the candidates (direct mode)
-    if (csize == 2 && unsorted) {
-      // Two ranks, unordered output: ONE cluster barrier. Rank 1 writes its selected positions from the END of
-      // the output row and pushes its candidates to the END of rank 0's candidate buffer (neither needs rank 0's
-      // counts), with its count; after the barrier rank 0 moves them behind its own and fills the slots between
-      // its selected positions and rank 1's with the chosen candidates.
-      const unsigned int my_sel = sm->n_sel, my_cand = sm->n_cand;
-      if (rank == 1) {
-        for (unsigned int j = tid; j < my_sel; j += kTopkThreads) out[k - 1 - static_cast<int>(j)] = key_pos(sm->sel[j]);
-        for (unsigned int j = tid; j < my_cand; j += kTopkThreads) st_peer_u64(peer_addr(&sm->cand[kCandCap - 1 - j], 0), sm->cand[j]);
-        if (tid == 0) st_peer_u32(peer_addr(&sm->all_cand[1], 0), my_cand);
-      } else {
-        for (unsigned int j = tid; j < my_sel; j += kTopkThreads) out[j] = key_pos(sm->sel[j]);
-      }
-      cluster_barrier();  // rank 0 holds every candidate and rank 1's count
-      if (rank != 0) return;
-      const unsigned int c1 = sm->all_cand[1];
-      // (thr_count = my_cand + c1 <= kCandCap, so the two segments cannot overlap)
-      // (the two regions can overlap when there are many candidates: all reads, a barrier, then the writes)
-      unsigned long long moved[kCandCap / kTopkThreads];
-#pragma unroll
-      for (int u = 0; u < kCandCap / kTopkThreads; ++u) {
-        const unsigned int j = tid + u * kTopkThreads;
-        moved[u] = j < c1 ? sm->cand[kCandCap - 1 - j] : 0ull;
-      }
-      __syncthreads();
-#pragma unroll
-      for (int u = 0; u < kCandCap / kTopkThreads; ++u) {
-        const unsigned int j = tid + u * kTopkThreads;
-        if (j < c1) sm->cand[my_cand + j] = moved[u];
-      }
-      direct_base = my_sel;
-      __syncthreads();
-    } else if (csize > 1) {
-      if (tid < csize) {
-        st_peer_u32(peer_addr(&sm->all_sel[rank], tid), sm->n_sel);
-        st_peer_u32(peer_addr(&sm->all_cand[rank], tid), sm->n_cand);
-      }
-      cluster_barrier();  // every rank's lists are complete and all counts are known everywhere
-      // offsets of this rank's lists in the row's lists
-      unsigned int sel_off = 0, cand_off = 0;
-      for (unsigned int r = 0; r < rank; ++r) {
-        sel_off += sm->all_sel[r];
-        cand_off += sm->all_cand[r];
-      }
-      // the candidates (and, for ordered output, the selected keys) of ranks 1.. are pushed into rank 0's
-      // lists at their offsets: remote stores from all ranks at once, completed by the barrier below
-      if (rank != 0) {
-        const unsigned int my_cand = sm->n_cand;
-        for (unsigned int j = tid; j < my_cand; j += kTopkThreads) st_peer_u64(peer_addr(&sm->cand[cand_off + j], 0), sm->cand[j]);
-      }
-      const unsigned int my_sel = sm->n_sel;
-      if (unsorted) {
-        // the selected positions go straight to the output
-        for (unsigned int j = tid; j < my_sel; j += kTopkThreads) out[sel_off + j] = key_pos(sm->sel[j]);
-      } else if (rank != 0) {
-        for (unsigned int j = tid; j < my_sel; j += kTopkThreads) st_peer_u64(peer_addr(&sm->sel[sel_off + j], 0), sm->sel[j]);
-      }
-      cluster_barrier();  // rank 0's lists are complete; the other ranks are done
-      if (rank != 0) return;
-      __syncthreads();
-    }
-    TKT(7);
-    // ---- 4. best `need` of the candidates (rank 0) --------------------------------------------
-    // a chosen key goes to its place among the selected ones: straight to the output when every rank wrote its own
-    // part there (unordered, cluster), else behind the `above` keys already in `sel`
-    const bool direct = unsorted && csize > 1;
-    auto emit = [&](unsigned int j, unsigned long long key) {
-      if (direct) out[direct_base + j] = key_pos(key); else sm->sel[above + j] = key;
-    };
-    bool refined = false;
-    if (coarse && need != thr_count && thr_count > 256u) {
-      // The candidates of a coarse bin share the top 12 bits of their value word and are many (the bin is wide):
-      // one more radix step inside shared memory instead of sorting them all. Digit: the next 11 bits of the value.
-      constexpr int kFineShift = 32 + kLiHistShift - 11;
-      for (int j = tid; j < kBins; j += kTopkThreads) sm->hist[j] = 0;
-      if (tid == 0) {
-        sm->n_sel2 = 0;
-        sm->n_cand2 = 0;
-      }
-      __syncthreads();
-      for (unsigned int j = tid; j < thr_count; j += kTopkThreads) {
-        atomicAdd(&sm->hist[static_cast<unsigned int>(sm->cand[j] >> kFineShift) & (kBins - 1)], 1u);
-      }
-      __syncthreads();
-      find_threshold_bin<kBins / kTopkThreads>(sm, need);
-      const unsigned int fine_bin = static_cast<unsigned int>(sm->thr_bin), fine_above = sm->thr_above, fine_count = sm->thr_count;
-      __syncthreads();  // the histogram area becomes the list of the keys in the fine threshold bin
-      unsigned long long* tmp = reinterpret_cast<unsigned long long*>(sm->hist);
-      constexpr unsigned int kTmpCap = kHistSlots * sizeof(unsigned int) / sizeof(unsigned long long);
-      if (fine_count <= kTmpCap) {
-        for (unsigned int j = tid; j < thr_count; j += kTopkThreads) {
-          const unsigned long long key = sm->cand[j];
-          const unsigned int f = static_cast<unsigned int>(key >> kFineShift) & (kBins - 1);
-          if (f > fine_bin) emit(atomicAdd(&sm->n_sel2, 1u), key);
-          else if (f == fine_bin) tmp[atomicAdd(&sm->n_cand2, 1u)] = key;
-        }
-        __syncthreads();
-        const unsigned int need2 = need - fine_above;
-        if (need2 != fine_count) {
-          int cpow2 = 2;
-          while (cpow2 < static_cast<int>(fine_count)) cpow2 <<= 1;
-          for (int j = fine_count + tid; j < cpow2; j += kTopkThreads) tmp[j] = 0ull;
-          bitonic_sort_desc(tmp, cpow2);
-        }
-        for (unsigned int j = tid; j < need2; j += kTopkThreads) emit(fine_above + j, tmp[j]);
-        refined = true;
-      }
-    }
-    if (!refined) {
-      if (need != thr_count && thr_count <= 512u) {
-        // few candidates (the usual case: a fine bucket holds a few dozen): every candidate counts the candidates
-        // above it (keys are unique, so the counts are the ranks) and the first `need` ranks go out. All threads
-        // read the same candidate at a time (a broadcast); no barrier inside, where a bitonic sort of 1024 threads
-        // spends its time.
-        __syncthreads();
-        if (static_cast<unsigned int>(tid) < thr_count) {
-          const unsigned long long mine = sm->cand[tid];
-          unsigned int rank_of = 0;
-          for (unsigned int j = 0; j < thr_count; ++j) rank_of += sm->cand[j] > mine ? 1u : 0u;
-          if (rank_of < need) emit(rank_of, mine);
-        }
-      } else {
-        if (need != thr_count) {
-          int cpow2 = 1;
-          while (cpow2 < static_cast<int>(thr_count)) cpow2 <<= 1;
-          for (int j = thr_count + tid; j < cpow2; j += kTopkThreads) sm->cand[j] = 0ull;
-          bitonic_sort_desc(sm->cand, cpow2);
-        }
-        for (unsigned int j = tid; j < need; j += kTopkThreads) emit(j, sm->cand[j]);
-      }
-    }
-    TKT(8);
-    if (direct) return;
-    __syncthreads();
+    n_list = static_cast<unsigned int>(eff);
   } else {
-    // ---- 4'. massive ties: MSB-first radix select on the 64-bit keys of the threshold bucket ----
-    // (rank 0 alone, over the whole row; the decision above is the same in every rank)
-    if (rank != 0) return;
-    if (tid == 0) sm->n_sel = 0;
+    // this rank's share of the row: the first chunks are on their way while the bound is found
+    const int share = (((eff + static_cast<int>(csize) - 1) / static_cast<int>(csize)) + 3) & ~3;
+    const int begin = min(eff, static_cast<int>(rank) * share);
+    const int end = min(eff, begin + share);
+    const int chunks = (end - begin + kChunk - 1) / kChunk;
+    auto fetch = [&](int c) {  // one thread
+      const uint32_t bytes = static_cast<uint32_t>((min(kChunk, end - begin - c * kChunk) + 3) & ~3) * 4u;
+      const uint32_t bar = smem_u32(&sm->full[c % kRing]);
+      mbar_arrive_expect_tx(bar, bytes);
+      bulk_load_1d(smem_u32(sm->ring[c % kRing]), row + begin + c * kChunk, bytes, bar);
+    };
+    if (tid == 0) {
+      for (int c = 0; c < min(chunks, kRing); ++c) fetch(c);
+    }
+    // ---- 1. lower bound -------------------------------------------------------------------------
+    float bound = -INFINITY;
+    bool known = false;
+    if (p.hist != nullptr) {
+      const uint4* h4 = reinterpret_cast<const uint4*>(p.hist + static_cast<int64_t>(row_id) * kLiHistBins);
+      for (int j = tid; j < kLiHistBins / 4; j += kTopkThreads) reinterpret_cast<uint4*>(sm->hist)[j] = __ldg(h4 + j);
+      __syncthreads();
+      find_threshold_bin<kLiHistBins / kTopkThreads>(sm, static_cast<unsigned int>(k));
+      known = sm->hist_total == static_cast<unsigned int>(eff) && sm->thr_above + sm->thr_count <= static_cast<unsigned int>(kListCap);
+      bound = order_float(static_cast<unsigned int>(sm->thr_bin) << kLiHistShift);
+      __syncthreads();  // every thread has read the outcome before the histogram area is reused
+    }
+    if (!known) bound = sample_bound(sm, row, eff, k);
+    TKT(2);
+    // ---- 2. this rank's keys at or above the bound ------------------------------------------------
+    unsigned int n = 0;
+    bool ok = true;
+    for (int c = 0; c < chunks; ++c) {
+      const uint32_t ph = (c / kRing) & 1;
+      if (tid == 0 && c > 0 && c - 1 + kRing < chunks) {  // the chunk before this one is read: refill its place
+        if (mbar_wait_spin(smem_u32(&sm->empty[(c - 1) % kRing]), ((c - 1) / kRing) & 1)) fetch(c - 1 + kRing);
+      }
+      __syncwarp();
+      ok = mbar_wait_warp(smem_u32(&sm->full[c % kRing]), ph) && ok;
+      const float* chunk = sm->ring[c % kRing];
+      const int p0 = begin + c * kChunk;
+      // Few elements pass. Sixteen comparisons a thread give a mask; its count behind the counts of the lanes below is the
+      // thread's place in the warp's list (a ballot per element needs two population counts each, which run at an eighth
+      // of the rate); the few set bits are walked and their values read again. A warp takes 512 neighbouring positions.
+      auto offset = [&](int e) { return warp * 512 + (e >> 2) * 128 + lane * 4 + (e & 3); };
+      unsigned int mask = 0u;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float4 v = *reinterpret_cast<const float4*>(chunk + offset(4 * u));
+        mask |= (v.x >= bound ? 1u << (4 * u) : 0u) | (v.y >= bound ? 2u << (4 * u) : 0u) | (v.z >= bound ? 4u << (4 * u) : 0u) |
+                (v.w >= bound ? 8u << (4 * u) : 0u);
+      }
+      if (p0 + kChunk > end) {  // the last chunk: what lies behind the end is not part of the row
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+          if (p0 + offset(e) >= end) mask &= ~(1u << e);
+        }
+      }
+      const unsigned int cnt = __popc(mask);
+      unsigned int incl = cnt;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned int up = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += up;
+      }
+      unsigned int at = n + incl - cnt;
+      n += __shfl_sync(0xffffffffu, incl, 31);
+      if (n <= static_cast<unsigned int>(kWarpCap)) {  // (else the list is spoilt, its length says so below)
+        while (mask != 0u) {
+          const int e = __ffs(mask) - 1;
+          mask &= mask - 1u;
+          const int off = offset(e);
+          sm->mine[warp][at++] = make_key(chunk[off], p0 + off);
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&sm->empty[c % kRing]));
+    }
+    if (!ok) {
+      if (lane == 0) set_status(p.status, PTO_ST_WAIT_EXPIRED, row_id, 30);
+      n = kListCap + 1;
+    }
+    TKT(3);
+    if (lane == 0) sm->warp_n[warp] = n;
     __syncthreads();
-    // digits: 11/11/10 bits of the value word, then 11/11/10 bits of the inverted position.
-    // invariant: keys in the bucket with (key >> shift) > prefix are selected; `remaining` more are
-    // needed among those with (key >> shift) == prefix.
-    unsigned long long prefix = 0ull;
-    int shift = 64;
-    unsigned int remaining = need;
-    const int widths[6] = {11, 11, 10, 11, 11, 10};
-    bool exact = false;
-    for (int pass = 0; pass < 6 && !exact; ++pass) {
-      const int w = widths[pass];
-      const int new_shift = shift - w;
-      for (int j = tid; j < kBins; j += kTopkThreads) sm->hist[j] = 0;
+    // ---- the lists of all warps and ranks, one behind the other, into rank 0's ----------------------
+    const unsigned int mine_n = lane < kTopkWarps ? sm->warp_n[lane] : 0u;
+    unsigned int incl = mine_n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned int x = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += x;
+    }
+    // a warp that found more than it could keep spoils the list: its length says so
+    unsigned int total = __shfl_sync(0xffffffffu, incl, 31);
+    if (__any_sync(0xffffffffu, mine_n > static_cast<unsigned int>(kWarpCap))) total = kListCap + 1;
+    const unsigned int warp_off = __shfl_sync(0xffffffffu, incl - mine_n, warp);
+    if (csize == 2) {
+      // two ranks: rank 0's keys from the front of the list, rank 1's from its end, with their number: nobody waits for a count
+      cluster_wait();
+      if (total <= static_cast<unsigned int>(kListCap)) {
+        for (unsigned int j = lane; j < n; j += 32) {
+          if (rank == 0) sm->list[warp_off + j] = sm->mine[warp][j];
+          else st_peer_u64(peer_addr(&sm->list[kListCap - 1 - (warp_off + j)], 0), sm->mine[warp][j]);
+        }
+      }
+      if (rank == 1 && tid == 0) st_peer_u32(peer_addr(&sm->n_list, 0), total);
+      cluster_arrive();
+      cluster_wait();
+      if (rank != 0) return;
+      n_front = total;
+      n_list = total + sm->n_list;  // (where the two would overlap the list is too long and not read)
+    } else if (csize > 1) {
+      cluster_wait();
+      if (tid == 0) sm->offset = atom_peer_add_u32(peer_addr(&sm->n_list, 0), total);
       __syncthreads();
-      for_each_element<true>(row, 0, eff, [&](float v, int pos) {
-        if (bucket(v) != thr_bin) return;
-        const unsigned long long key = make_key(v, pos);
-        if (shift < 64 && (key >> shift) != prefix) return;
-        atomicAdd(&sm->hist[static_cast<unsigned int>(key >> new_shift) & ((1u << w) - 1u)], 1u);
-      });
-      __syncthreads();
-      find_threshold_bin<kBins / kTopkThreads>(sm, remaining);
-      remaining -= sm->thr_above;
-      exact = (sm->thr_count == remaining);
-      prefix = (prefix << w) | static_cast<unsigned long long>(sm->thr_bin);
-      shift = new_shift;
+      const unsigned int off = sm->offset;
+      if (total <= static_cast<unsigned int>(kListCap)) {
+        for (unsigned int j = lane; j < n; j += 32) {
+          const unsigned int at = off + warp_off + j;
+          if (at < static_cast<unsigned int>(kListCap)) st_peer_u64(peer_addr(&sm->list[at], 0), sm->mine[warp][j]);
+        }
+      }
+      cluster_arrive();
+      cluster_wait();
+      if (rank != 0) return;
+      n_list = sm->n_list;
+    } else {
+      if (total <= static_cast<unsigned int>(kListCap)) {
+        for (unsigned int j = lane; j < n; j += 32) sm->list[warp_off + j] = sm->mine[warp][j];
+      }
+      n_list = total;
       __syncthreads();
     }
-    // every key with (key >> shift) >= prefix inside the bucket, plus all higher buckets
-    for_each_element<true>(row, 0, eff, [&](float v, int pos) {
-      const int bkt = bucket(v);
-      if (bkt < thr_bin) return;
-      const unsigned long long key = make_key(v, pos);
-      if (bkt > thr_bin || (key >> shift) >= prefix) {
-        const unsigned int slot = atomicAdd(&sm->n_sel, 1u);
-        if (slot < static_cast<unsigned int>(kMaxK)) sm->sel[slot] = key;
+    if (n_list <= static_cast<unsigned int>(kListCap)) {
+      for (unsigned int j = tid; j < n_list; j += kTopkThreads) {
+        const float x = key_value(key_at(j));
+        lmin = fminf(lmin, x);
+        lmax = fmaxf(lmax, x);
       }
+    }
+  }
+  TKT(4);
+
+  // ---- 3. order ------------------------------------------------------------------------------------
+  bool good = n_list <= static_cast<unsigned int>(kListCap) && n_list >= static_cast<unsigned int>(k);  // (uniform)
+  if (good) {
+    for (int j = tid; j < kBins; j += kTopkThreads) sm->hist[j] = 0;
+    block_range(sm, lmin, lmax);
+    BinMap map;
+    map.set(lmin, lmax);
+    constexpr int kPer = kListCap / kTopkThreads;
+    unsigned int where[kPer];  // bin, and which of its keys
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const unsigned int j = tid + u * kTopkThreads;
+      if (j < n_list) {
+        const unsigned int b = static_cast<unsigned int>(map.bin(key_value(key_at(j))));
+        where[u] = (b << 16) | atomicAdd(&sm->hist[b], 1u);
+      }
+    }
+    __syncthreads();
+    TKT(5);
+    find_threshold_bin<kBins / kTopkThreads, true>(sm, static_cast<unsigned int>(k));
+    // Bins that lie in the result whole need no order when the caller asked for none: only the keys of the others go to their
+    // bin's place in `sorted`, to be ranked there.
+    const bool unsorted = (p.flags & PTO_LI_UNSORTED) != 0;
+    const unsigned int uk = static_cast<unsigned int>(k);
+    bool crowded = false;
+    unsigned int chosen[kPer], n_chosen = 0;  // per run of 32 keys of the list: which go out as they are (unordered)
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const unsigned int j = tid + u * kTopkThreads;
+      bool go = false;
+      if (j < n_list) {
+        const unsigned int b = where[u] >> 16, first = sm->base[b], slot = where[u] & 0xffffu;
+        if (first < uk) {
+          if (unsorted && first + sm->hist[b] <= uk) go = true;
+          else if (slot < static_cast<unsigned int>(kBinCap)) sm->sorted[first + slot] = key_at(j);
+          else crowded = true;
+        }
+      }
+      chosen[u] = __ballot_sync(0xffffffffu, go);
+      n_chosen += __popc(chosen[u]);
+    }
+    if (unsorted) {
+      // In runs as they lie in the list, i.e. of neighbouring positions: the attention kernel gathers the selected rows in this
+      // order, and in the order of the bins (a random walk over the cache) its gathers cost 64 sequences 3 us more than the
+      // selection had gained.
+      unsigned int at = 0;
+      if (lane == 0) at = atomicAdd(&sm->n_sel, n_chosen);
+      at = __shfl_sync(0xffffffffu, at, 0);
+#pragma unroll
+      for (int u = 0; u < kPer; ++u) {
+        if ((chosen[u] >> lane) & 1u) out[at + __popc(chosen[u] & ((1u << lane) - 1u))] = key_pos(key_at(tid + u * kTopkThreads));
+        at += __popc(chosen[u]);
+      }
+    }
+    good = __syncthreads_or(crowded ? 1 : 0) == 0;
+    TKT(6);
+    if (good) {
+      // keys of the bins that reach into the result; without order, of the one bin that lies across its end
+      const unsigned int n_sorted = sm->thr_above + sm->thr_count;
+      if (!(unsorted && n_sorted == uk)) {
+        for (unsigned int j = (unsorted ? sm->thr_above : 0u) + tid; j < n_sorted; j += kTopkThreads) {
+          const unsigned long long key = sm->sorted[j];
+          const int b = map.bin(key_value(key));
+          const unsigned int first = sm->base[b], last = first + sm->hist[b];
+          unsigned int at = first;
+          for (unsigned int x = first; x < last; ++x) at += sm->sorted[x] > key ? 1u : 0u;
+          if (at < uk) out[at] = key_pos(key);
+        }
+      }
+      TKT(7);
+      return;
+    }
+  }
+
+  // ---- 3'. MSB-first radix select on the 64-bit keys of the whole row (rank 0) ----------------------------
+  if (tid == 0) sm->n_sel = 0;
+  // digits: 11/11/10 bits of the value word, then 11/11/10 bits of the inverted position.
+  // invariant: keys with (key >> shift) > prefix are selected; `remaining` more are needed among those with
+  // (key >> shift) == prefix.
+  __syncthreads();
+  unsigned long long prefix = 0ull;
+  int shift = 64;
+  unsigned int remaining = static_cast<unsigned int>(k);
+  const int widths[6] = {11, 11, 10, 11, 11, 10};
+  bool exact = false;
+  for (int pass = 0; pass < 6 && !exact; ++pass) {
+    const int w = widths[pass];
+    const int new_shift = shift - w;
+    for (int j = tid; j < kBins; j += kTopkThreads) sm->hist[j] = 0;
+    __syncthreads();
+    for_each_element(row, eff, [&](float v, int pos) {
+      const unsigned long long key = make_key(v, pos);
+      if (shift < 64 && (key >> shift) != prefix) return;
+      atomicAdd(&sm->hist[static_cast<unsigned int>(key >> new_shift) & ((1u << w) - 1u)], 1u);
     });
     __syncthreads();
+    find_threshold_bin<kBins / kTopkThreads>(sm, remaining);
+    remaining -= sm->thr_above;
+    exact = (sm->thr_count == remaining);
+    prefix = (prefix << w) | static_cast<unsigned long long>(sm->thr_bin);
+    shift = new_shift;
+    __syncthreads();
   }
-
-  // ---- 5. order and write -------------------------------------------------------------------
-  if (!unsorted) {
-    for (int j = k + tid; j < kpow2; j += kTopkThreads) sm->sel[j] = 0ull;
-    bitonic_sort_desc(sm->sel, kpow2);
-  }
-  for (int j = tid; j < k; j += kTopkThreads) out[j] = key_pos(sm->sel[j]);
+  for_each_element(row, eff, [&](float v, int pos) {
+    const unsigned long long key = make_key(v, pos);
+    if ((key >> shift) >= prefix) {
+      const unsigned int slot = atomicAdd(&sm->n_sel, 1u);
+      if (slot < static_cast<unsigned int>(kMaxK)) sm->sorted[slot] = key;
+    }
+  });
+  __syncthreads();
+  int kpow2 = 2;
+  while (kpow2 < k) kpow2 <<= 1;
+  for (int j = k + tid; j < kpow2; j += kTopkThreads) sm->sorted[j] = 0ull;
+  bitonic_sort_desc(sm->sorted, kpow2);
+  for (int j = tid; j < k; j += kTopkThreads) out[j] = key_pos(sm->sorted[j]);
 }
 
 }  // namespace
@@ -683,19 +683,11 @@ cudaError_t launch_li_topk(const TopkParams& p, int num_sms, cudaStream_t stream
   cudaError_t e = cudaFuncSetAttribute(li_topk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(sizeof(TopkSmem)));
   if (e != cudaSuccess) return e;
-  // as many CTAs per row as keep the grid within one wave (portable cluster sizes: up to 8)
+  // as many CTAs per row as keep the grid within one wave, each with 8192 positions or more to scan (a row
+  // that fits the list is one CTA's work)
   const int rows = p.b * p.s1;
   int csize = 1;
-  while (csize < 8 && rows * csize * 2 <= num_sms) csize *= 2;
-  // ordered output ends in a 2048-key sort on rank 0 that dwarfs the scans of short rows: measured, a
-  // cluster only pays there for rows beyond ~40 K positions
-  if ((p.flags & PTO_LI_UNSORTED) == 0 && p.row_stride <= 40960) csize = 1;
-  static const int forced = [] {  // PTO_TOPK_CLUSTER=1|2|4|8 in the environment: CTAs per row (A/B timing aid)
-    const char* v = getenv("PTO_TOPK_CLUSTER");
-    const int want = v != nullptr ? atoi(v) : 0;
-    return (want == 1 || want == 2 || want == 4 || want == 8) ? want : 0;
-  }();
-  if (forced != 0) csize = forced;
+  while (csize < 8 && rows * csize * 2 <= num_sms && p.row_stride > static_cast<int64_t>(csize) * 8192) csize *= 2;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(rows * csize), 1, 1);
   cfg.blockDim = dim3(kTopkThreads, 1, 1);

@@ -307,3 +307,41 @@ def test_two_ctas_per_row_with_thousands_of_tied_candidates():
         want = set(torch.topk(key, 2048).indices.tolist())
         got = out[r, 0].tolist()
         assert len(set(got)) == 2048 and set(got) == want, f"row {r}"
+
+
+@pytest.mark.parametrize("sort", [True, False], ids=["ordered", "unordered"])
+@pytest.mark.parametrize("rows,n,k", [
+    (3, 2047, 2048), (3, 2049, 2048), (2, 6144, 2048), (2, 6145, 2048),   # rows that are the list, and the first that are not
+    (5, 8192, 7), (2, 8193, 1), (40, 20000, 2048), (9, 32769, 2048),      # clusters of one to eight CTAs, chunk edges
+    (2, 70000, 2048), (1, 300001, 1000), (160, 9000, 300),                # larger samples; more rows than SMs
+])
+@pytest.mark.parametrize("kind", ["normal", "clustered", "ties", "constant", "infinite"])
+def test_topk_stage_over_row_lengths_and_distributions(rows, n, k, kind, sort):
+    """Selection alone: the sampled bound, its failures (one value, values that are not finite, ties across the end of the
+    selection) and the positions at which the row, the list and the chunks end. Ties go to the smaller position."""
+    g = torch.Generator().manual_seed(n + k)
+    stride = (n + 127) // 128 * 128
+    sc = torch.randn(rows, stride, generator=g)
+    if kind == "clustered":  # everything that is selected lies side by side
+        sc[:, n // 3:n // 3 + 2 * k + 5] += 9.0
+    elif kind == "ties":
+        sc = (sc * 3).round() / 3 + 0.0
+    elif kind == "constant":
+        sc.fill_(0.25)
+    elif kind == "infinite":
+        sc[:, ::11] = float("-inf")
+        sc[:, 5::997] = float("inf")
+    sc[:, n:] = float("nan")  # never read as part of the row
+    act = torch.full((rows,), n, dtype=torch.int32, device=DEV)
+    out = torch.full((rows, 1, k), -7, dtype=torch.int32, device=DEV)
+    pto.lightning_indexer_topk(sc.to(DEV), act, out, 1, k, sort=sort)
+    torch.cuda.synchronize()
+    assert pto.workspace_status()[0] == 0
+    got = out.cpu()[:, 0].long()
+    want = sc[:, :n].sort(dim=1, descending=True, stable=True).indices[:, :k]
+    m = min(n, k)
+    assert torch.all(got[:, m:] == -1)
+    got = got[:, :m]
+    if not sort:
+        got, want = got.sort(dim=1).values, want.sort(dim=1).values
+    assert torch.equal(got, want)
