@@ -94,8 +94,8 @@ def test_head_slice_of_16():
 
 @pytest.mark.parametrize("packed", [False, True], ids=["split_arrays", "packed_rows"])
 @pytest.mark.parametrize("nq,lens,s1", [
-    (16, [1, 79, 80, 81, 160, 161, 2048, 2500], 1),    # edges of its 80-row tiles; one item per SM and split
-    (32, [63, 64, 65, 128, 2047, 130, 0, 3000], 2),    # edges of its 64-row tiles, tokens that see nothing
+    (16, [1, 127, 128, 129, 256, 257, 2048, 2500], 1),  # edges of its 128-row tiles; one item per SM and split
+    (32, [63, 64, 65, 128, 2047, 130, 0, 3000], 2),    # two blocks of 16 heads, tokens that see nothing
     (48, [700, 2100], 2),                              # three blocks of 16 heads
     (64, [300] * 90, 1),                               # more items than SMs: CTAs walk several, unsplit
 ])
