@@ -409,7 +409,8 @@ struct WMatrix {
 // side, all widths but the last multiples of 64. kind 0: fp32 partials, 1: bf16. Row pitches in bytes.
 int run_sgemm(int kind, const void* x, size_t x_pitch, const WMatrix* ws, int n_w, int64_t w_rows, void* out, int t,
               int k, int batch, int w_batch_rows, int x_batch_bytes, long long out_batch, long long ld_out,
-              int splits, long long split_stride, int num_sms, int32_t* status, cudaStream_t stream, bool pdl = false) {
+              int splits, long long split_stride, int num_sms, int32_t* status, cudaStream_t stream, bool pdl = false,
+              const pto::PrologOut2* out2 = nullptr) {  // (out2: few token rows only)
   // (up to 128 rows the projections have more items of 128 columns than of 128 rows x 256 columns: 70 tokens 66 us a call
   // against 71)
   const bool wide = prolog_is_wide(t) && (kind != 0 || t > 128);
@@ -436,7 +437,7 @@ int run_sgemm(int kind, const void* x, size_t x_pitch, const WMatrix* ws, int n_
                                      ld_out, splits, split_stride, num_sms, status, stream, pdl));
   } else {
     PTO_CUDA(pto::launch_prolog_sgemm(kind, maps_w, boxes, &map_x, out, t, n, k, batch, w_batch_rows, x_batch_bytes, out_batch,
-                                      ld_out, splits, split_stride, num_sms, status, stream, pdl));
+                                      ld_out, splits, split_stride, num_sms, status, stream, pdl, out2));
   }
   return PTO_OK;
 }
@@ -878,7 +879,8 @@ int pto_mla_indexer_prolog_quant(const void* token_x, const void* w_dq, const in
   PTO_CUDA(cudaStreamWaitEvent(side, ev[0], 0));
   PTO_CUDA(pto::launch_prolog_kv(kv, ki, wp, ld, splits, split_stride, gamma_ckv, cos, sin, ln_gamma, ln_beta, hadamard_k,
                                  cache_index, cache_rows, t, eps_ckv, ln_eps, kv_cache, kr_cache, kv_scale_cache,
-                                 idx_k_cache, idx_k_scale_cache, weights_out, packed_kv_cache, status, side));
+                                 idx_k_cache, idx_k_scale_cache, weights_out, packed_kv_cache, hadamard_q, w_idx_qb_scale, status,
+                                 side));
   // from here on every kernel of the caller's stream follows a kernel of this call: each may be scheduled while
   // the one before it drains (it waits before it reads)
   PTO_CUDA(pto::launch_prolog_qnorm_quant(qa, ld, splits, split_stride, gamma_cq, t, q_lora, eps_cq, q_norm, q_norm_scale,
@@ -900,13 +902,13 @@ int pto_mla_indexer_prolog_quant(const void* token_x, const void* w_dq, const in
     if (rc != PTO_OK) return rc;
     PTO_CUDA(pto::launch_prolog_wide_up(&map_w0, &map_w1, &map_x, t, q_lora, q_norm_scale, w_qb_scale, w_idx_qb_scale, cos,
                                         sin, q_b, query_rope_out, qi_i32, di.num_sms, status, stream, /*pdl=*/true));
-    PTO_CUDA(cudaEventRecord(ev[1], stream));
-    PTO_CUDA(cudaStreamWaitEvent(side, ev[1], 0));
+    PTO_CUDA(cudaEventRecord(ev[2], stream));
+    PTO_CUDA(cudaStreamWaitEvent(side, ev[2], 0));
     PTO_CUDA(pto::launch_prolog_wide_hadamard(&map_had, &map_rows, t * 64, q_int8_out, q_scale_out, di.num_sms, status, side));
-    PTO_CUDA(cudaEventRecord(ev[2], side));
+    PTO_CUDA(cudaEventRecord(ev[1], side));
     rc = run_sgemm(1, q_b, 128 * 128 * 2, &uk, 1, 128 * 128, query_nope_out, t, 128, 128, 128, 128 * 2, 512, 128 * 512, 1, 0, di.num_sms, status, stream, /*pdl=*/true);
     if (rc != PTO_OK) return rc;
-    PTO_CUDA(cudaStreamWaitEvent(stream, ev[2], 0));
+    PTO_CUDA(cudaStreamWaitEvent(stream, ev[1], 0));
     return PTO_OK;
   }
   // few: both int8 up-projections of the normalised query in one launch, the activations resident in shared memory
@@ -920,17 +922,17 @@ int pto_mla_indexer_prolog_quant(const void* token_x, const void* w_dq, const in
   PTO_CUDA(pto::launch_prolog_i8_gemm(&map_w0, &map_w1, &map_x, qb_i32, 128 * 192, qi_i32, 64 * 128, q_lora, t, di.num_sms,
                                       status, stream, /*pdl=*/true));
   // the indexer-query kernel joins the side stream; the attention query finishes on the caller's
-  PTO_CUDA(cudaEventRecord(ev[1], stream));
-  PTO_CUDA(cudaStreamWaitEvent(side, ev[1], 0));
+  PTO_CUDA(cudaEventRecord(ev[2], stream));
+  PTO_CUDA(cudaStreamWaitEvent(side, ev[2], 0));
   PTO_CUDA(pto::launch_prolog_idxq(qi_i32, q_norm_scale, w_idx_qb_scale, cos, sin, hadamard_q, t, q_int8_out, q_scale_out,
                                    side));
-  PTO_CUDA(cudaEventRecord(ev[2], side));
+  PTO_CUDA(cudaEventRecord(ev[1], side));
   PTO_CUDA(pto::launch_prolog_qb_dequant_rope(qb_i32, q_norm_scale, w_qb_scale, cos, sin, t, q_b, query_rope_out, stream,
                                               /*pdl=*/true));
   // absorbed nope part: per head [t, 128] (row pitch 128*192, head pitch 192 elements) @ w_uk[head] [128, 512] -> bf16
   rc = run_sgemm(1, q_b, 128 * 192 * 2, &uk, 1, 128 * 128, query_nope_out, t, 128, 128, 128, 192 * 2, 512, 128 * 512, 1, 0, di.num_sms, status, stream, /*pdl=*/true);
   if (rc != PTO_OK) return rc;
-  PTO_CUDA(cudaStreamWaitEvent(stream, ev[2], 0));  // join: everything is ordered before what the caller enqueues next
+  PTO_CUDA(cudaStreamWaitEvent(stream, ev[1], 0));  // join: everything is ordered before what the caller enqueues next
   return PTO_OK;
 }
 
@@ -999,27 +1001,36 @@ int pto_mla_indexer_prolog(const void* token_x, const void* w_dq, const void* w_
   PTO_CUDA(pto::launch_prolog_kv_bf16(kv, ki, wp, ld, splits, split_stride, gamma_ckv, cos, sin, ln_gamma, ln_beta,
                                       cache_index, cache_rows, t, eps_ckv, ln_eps, kv_cache, kr_cache, idx_k_cache,
                                       weights_out, status, side));
-  // caller's stream: normalised query -> attention up-projection (bf16 in, bf16 out) -> ropes -> absorbed nope part.
-  // The indexer's up-projection (64 column tiles) runs on the side stream beside the attention one (192 tiles on
-  // 148 CTAs: its second wave leaves two thirds of the SMs free), behind the per-token kernel.
+  PTO_CUDA(cudaEventRecord(ev[1], side));
+  // caller's stream: normalised query -> both up-projections (bf16 in, bf16 out) -> ropes -> absorbed nope part
   PTO_CUDA(pto::launch_prolog_qnorm_bf16(qa, ld, splits, split_stride, gamma_cq, t, q_lora, eps_cq, q_norm, stream,
                                          /*pdl=*/true));
-  PTO_CUDA(cudaEventRecord(ev[1], stream));
   const size_t qn_pitch = static_cast<size_t>(q_lora) * 2;
-  const WMatrix uqqr = {w_uqqr, 128 * 192 * 2, 128 * 192}, idx_qb = {w_idx_qb, 64 * 128 * 2, 64 * 128};
-  rc = run_sgemm(1, q_norm, qn_pitch, &uqqr, 1, q_lora, q_b, t, q_lora, 1, 0, 0, 0, 128 * 192, 1, 0, di.num_sms, status,
-                 stream);
-  if (rc != PTO_OK) return rc;
-  PTO_CUDA(cudaStreamWaitEvent(side, ev[1], 0));
-  rc = run_sgemm(1, q_norm, qn_pitch, &idx_qb, 1, q_lora, idx_query_out, t, q_lora, 1, 0, 0, 0, 64 * 128, 1, 0, di.num_sms,
-                 status, side);
-  if (rc != PTO_OK) return rc;
-  PTO_CUDA(cudaEventRecord(ev[2], side));
-  PTO_CUDA(cudaStreamWaitEvent(stream, ev[2], 0));  // the rope kernel reads both products
-  PTO_CUDA(pto::launch_prolog_rope_bf16(q_b, cos, sin, t, query_rope_out, idx_query_out, stream));
+  const WMatrix up[2] = {{w_uqqr, 128 * 192 * 2, 128 * 192}, {w_idx_qb, 64 * 128 * 2, 64 * 128}};
+  if (!prolog_is_wide(t)) {
+    // few: one launch, 256 column tiles. As two launches on two streams the second one's CTAs waited for the first one's to
+    // end (16 tokens: 31 us for both).
+    const pto::PrologOut2 idx = {idx_query_out, 128 * 192, 64 * 128};
+    rc = run_sgemm(1, q_norm, qn_pitch, up, 2, q_lora, q_b, t, q_lora, 1, 0, 0, 0, 128 * 192, 1, 0, di.num_sms, status,
+                   stream, /*pdl=*/true, &idx);
+    if (rc != PTO_OK) return rc;
+  } else {
+    // many: the indexer's (a third of the work) beside the attention's, on the side stream behind the per-token kernel
+    PTO_CUDA(cudaEventRecord(ev[2], stream));
+    rc = run_sgemm(1, q_norm, qn_pitch, up, 1, q_lora, q_b, t, q_lora, 1, 0, 0, 0, 128 * 192, 1, 0, di.num_sms, status, stream);
+    if (rc != PTO_OK) return rc;
+    PTO_CUDA(cudaStreamWaitEvent(side, ev[2], 0));
+    rc = run_sgemm(1, q_norm, qn_pitch, up + 1, 1, q_lora, idx_query_out, t, q_lora, 1, 0, 0, 0, 64 * 128, 1, 0, di.num_sms,
+                   status, side);
+    if (rc != PTO_OK) return rc;
+    PTO_CUDA(cudaEventRecord(ev[1], side));
+    PTO_CUDA(cudaStreamWaitEvent(stream, ev[1], 0));  // the rope kernel reads both products
+  }
+  PTO_CUDA(pto::launch_prolog_rope_bf16(q_b, cos, sin, t, query_rope_out, idx_query_out, stream, /*pdl=*/!prolog_is_wide(t)));
   rc = run_sgemm(1, q_b, 128 * 192 * 2, &uk, 1, 128 * 128, query_nope_out, t, 128, 128, 128, 192 * 2, 512, 128 * 512, 1, 0, di.num_sms, status, stream, /*pdl=*/true);
   if (rc != PTO_OK) return rc;
-  return PTO_OK;  // (the side stream was joined in front of the rope kernel)
+  PTO_CUDA(cudaStreamWaitEvent(stream, ev[1], 0));  // join: everything is ordered before what the caller enqueues next
+  return PTO_OK;
 }
 
 size_t pto_decode_workspace_bytes(int t, int max_blocks, int block_size, int nq) {

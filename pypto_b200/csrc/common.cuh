@@ -384,8 +384,8 @@ cudaError_t launch_prolog_kv(const float* kv, const float* ki, const float* wp, 
                              long long split_stride, const void* gamma_ckv, const void* cos, const void* sin, const void* ln_gamma, const void* ln_beta, const void* hadamard_k,
                              const int64_t* cache_index, int64_t cache_rows, int t, float eps_ckv, float ln_eps,
                              int8_t* kv_cache, void* kr_cache, float* kv_scale_cache, int8_t* idx_k_cache,
-                             void* idx_k_scale_cache, void* weights, int8_t* packed_cache, int32_t* status,
-                             cudaStream_t stream);
+                             void* idx_k_scale_cache, void* weights, int8_t* packed_cache, const void* next_hadamard,
+                             const void* next_scale, int32_t* status, cudaStream_t stream);
 // both int8 up-projections of the prolog in one tcgen05 launch (prolog_gemm.cu); t <= 64 token rows
 bool prolog_i8_gemm_supported(int t, int k);
 cudaError_t launch_prolog_i8_gemm(const void* tmap_w0, const void* tmap_w1, const void* tmap_x, int32_t* out0, int n0,
@@ -412,13 +412,19 @@ __device__ __forceinline__ const CUtensorMap* prolog_w_box(const PrologWMaps& m,
   *col_bytes = (box - begin) * 128;
   return &m.map[i];
 }
+// A product whose last columns go to a tensor of their own: from column `first` (a multiple of 128) on, rows `ld` elements apart.
+struct PrologOut2 {
+  void* out;
+  int first;
+  long long ld;
+};
 // the weight-streaming products of the prolog (prolog_sgemm.cu)
 int prolog_sgemm_rows(int t);
 int prolog_sgemm_splits(int t, int n, int k, int num_sms);
 cudaError_t launch_prolog_sgemm(int kind, const PrologWMaps& maps_w, const PrologWBoxes& boxes, const void* tmap_x, void* out, int t, int n, int k,
                                 int batch, int w_batch_rows, int x_batch_bytes, long long out_batch, long long ld_out,
                                 int splits, long long split_stride, int num_sms, int32_t* status, cudaStream_t stream,
-                                bool pdl = false);
+                                bool pdl = false, const PrologOut2* out2 = nullptr);
 // the same products for many token rows, with what follows them fused (prolog_wide.cu)
 cudaError_t launch_prolog_wide(int kind, const PrologWMaps& maps_w, const PrologWBoxes& boxes, const void* tmap_x, void* out, int t, int n, int k, int batch,
                                int w_batch_rows, int x_batch_bytes, long long out_batch, long long ld_out, int splits,

@@ -66,13 +66,17 @@ __device__ __forceinline__ int8_t quant_one(float v, float scale_q) {
 // grid = tokens, 512 threads, dynamic shared memory = q_lora floats (16-byte aligned rows: ld and q_lora multiples of 4)
 template <bool kQuant>
 __global__ void __launch_bounds__(512)
-prolog_qnorm_kernel(const float* __restrict__ qa, int ld, int n_split, long long split_stride,
+prolog_qnorm_kernel(const float* qa, int ld, int n_split, long long split_stride,
                     const __nv_bfloat16* __restrict__ gamma, int q_lora, float eps, int8_t* __restrict__ q_norm,
                     float* __restrict__ q_norm_scale, __nv_bfloat16* __restrict__ q_norm_bf16) {
   extern __shared__ __align__(16) float row[];
   __shared__ float red[32];
-  pdl_wait();  // the projection before it may still be running when this grid is scheduled
+  // First the trigger: the product behind this kernel fills its rings with weights meanwhile. What is no kernel's result is
+  // requested before the wait too: while weights stream, a read that misses L2 takes some microseconds. (Here and below.)
   if (threadIdx.x == 0) pdl_trigger();
+  uint2 gm0 = make_uint2(0u, 0u);  // four bf16
+  if (threadIdx.x < (q_lora >> 2)) gm0 = __ldg(reinterpret_cast<const uint2*>(gamma) + threadIdx.x);
+  pdl_wait();  // the projection before it may still be running when this grid is scheduled
   const int ti = blockIdx.x;
   const float4* src = reinterpret_cast<const float4*>(qa + static_cast<int64_t>(ti) * ld);
   float4* row4 = reinterpret_cast<float4*>(row);
@@ -83,7 +87,7 @@ prolog_qnorm_kernel(const float* __restrict__ qa, int ld, int n_split, long long
     float4 part[8];  // K-split partials of the projection (n_split <= 8): requested together, added in split order
 #pragma unroll
     for (int sp = 0; sp < 8; ++sp) {
-      part[sp] = sp < n_split ? __ldg(src + g + sp * (split_stride >> 2)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      part[sp] = sp < n_split ? src[g + sp * (split_stride >> 2)] : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     float4 v = part[0];
 #pragma unroll
@@ -109,7 +113,7 @@ prolog_qnorm_kernel(const float* __restrict__ qa, int ld, int n_split, long long
   float amax = 0.f;
   for (int g = threadIdx.x; g < groups; g += blockDim.x) {
     float4 v = row4[g];
-    const uint2 gm = __ldg(reinterpret_cast<const uint2*>(gamma) + g);  // four bf16
+    const uint2 gm = g == threadIdx.x ? gm0 : __ldg(reinterpret_cast<const uint2*>(gamma) + g);
     v.x = bf16_round(__fmul_rn(__fdiv_rn(v.x, rms), __uint_as_float(gm.x << 16)));
     v.y = bf16_round(__fmul_rn(__fdiv_rn(v.y, rms), __uint_as_float(gm.x & 0xffff0000u)));
     v.z = bf16_round(__fmul_rn(__fdiv_rn(v.z, rms), __uint_as_float(gm.y << 16)));
@@ -140,43 +144,183 @@ prolog_qnorm_kernel(const float* __restrict__ qa, int ld, int n_split, long long
   if (threadIdx.x == 0) q_norm_scale[ti] = __fdiv_rn(1.0f, scale_q);
 }
 
+// Hadamard rotation of 16 rows (bf16, row pitch kIdxPitch, shared memory) by the warps' own matrix instruction (m16n8k16):
+// 64 columns from col0, 16 * kSteps values of the contraction from k0. For few tokens only: the 128-row tile of the
+// tensor-memory path would be mostly empty and its set-up costs as much as the kernels here take. The instruction wants two
+// neighbours along k in one register where the matrix has two columns: a lane reads eight columns of four rows, 16 bytes each
+// (a warp: whole lines), and exchanges halves in registers; column g of tile n is column 8 g + n of the 64.
+// acc[n]: of row lane / 4 (first two) and lane / 4 + 8: columns 16 (lane % 4) + n and 16 (lane % 4) + 8 + n.
+constexpr int kIdxPitch = kIdxDim + 8;  // the eight rows of a fragment fall into different banks
+template <int kSteps>
+__device__ __forceinline__ void hadamard_rows(const __nv_bfloat16* __restrict__ h, int k0, int col0, const __nv_bfloat16* rows,
+                                              int lane, float (&acc)[8][4]) {
+  const int g = lane >> 2, l4 = lane & 3;
+#pragma unroll
+  for (int n = 0; n < 8; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+#pragma unroll
+  for (int ks = 0; ks < kSteps; ++ks) {
+    const int k = k0 + ks * 16;
+    uint32_t b[2][8];
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const __nv_bfloat16* src = h + (k + half * 8 + 2 * l4) * kIdxDim + col0 + 8 * g;
+      const uint4 even = __ldg(reinterpret_cast<const uint4*>(src));
+      const uint4 odd = __ldg(reinterpret_cast<const uint4*>(src + kIdxDim));
+      const uint32_t e[4] = {even.x, even.y, even.z, even.w}, o[4] = {odd.x, odd.y, odd.z, odd.w};
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        b[half][2 * c] = __byte_perm(e[c], o[c], 0x5410);
+        b[half][2 * c + 1] = __byte_perm(e[c], o[c], 0x7632);
+      }
+    }
+    uint32_t a[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      a[i] = *reinterpret_cast<const uint32_t*>(rows + (g + 8 * (i & 1)) * kIdxPitch + k + 8 * (i >> 1) + 2 * l4);
+    }
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+      asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+          : "+f"(acc[n][0]), "+f"(acc[n][1]), "+f"(acc[n][2]), "+f"(acc[n][3])
+          : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0][n]), "r"(b[1][n]));
+    }
+  }
+}
+// `bytes` (a multiple of 128) at `p` into L2, by `n` threads of which this one is number `i`
+__device__ __forceinline__ void prefetch_l2(const void* p, int bytes, int i, int n) {
+  for (int at = i * 128; at < bytes; at += n * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint8_t*>(p) + at));
+}
+
 // ---- query up-projection: int32 -> bf16, rope of the 64-wide tail ----------------------------------------
 // grid = (16 head groups, tokens), block = 256: eight heads (1536 values) per block
 constexpr int kQbHeadsPerBlock = 8;
 __global__ void __launch_bounds__(256)
-prolog_qb_dequant_rope_kernel(const int32_t* __restrict__ qb_i32, const float* __restrict__ q_norm_scale,
-                              const float* __restrict__ w_scale, const __nv_bfloat16* __restrict__ cos,
-                              const __nv_bfloat16* __restrict__ sin, __nv_bfloat16* __restrict__ q_b,
-                              __nv_bfloat16* __restrict__ q_rope) {
+prolog_qb_dequant_rope_kernel(const int32_t* qb_i32, const float* q_norm_scale, const float* __restrict__ w_scale,
+                              const __nv_bfloat16* __restrict__ cos, const __nv_bfloat16* __restrict__ sin,
+                              __nv_bfloat16* __restrict__ q_b, __nv_bfloat16* __restrict__ q_rope) {
+  // (the results of the kernels before this one are not __restrict__: loads of what nothing may write could be moved in
+  // front of pdl_wait())
   __shared__ float pe[kQbHeadsPerBlock][kRope];
-  pdl_wait();
-  if (threadIdx.x == 0) pdl_trigger();
-  const int hg = blockIdx.x, ti = blockIdx.y;
-  const float rs = q_norm_scale[ti];
+  const int ti = blockIdx.y, tid = threadIdx.x;
+  const int hg = blockIdx.x;
   const int64_t col0 = static_cast<int64_t>(hg) * kQbHeadsPerBlock * kQHead;
   const int64_t row0 = static_cast<int64_t>(ti) * kHeads * kQHead;
+  float ws[kQbHeadsPerBlock * kQHead / 256];
+#pragma unroll
+  for (int u = 0; u < kQbHeadsPerBlock * kQHead / 256; ++u) ws[u] = __ldg(w_scale + col0 + u * 256 + tid);
+  static_assert(256 % kRope == 0, "a thread rotates one dim of several heads");
+  const int c = tid % kRope;
+  const float cs = ld_bf16(cos + ti * kRope + c), sn = ld_bf16(sin + ti * kRope + c);
+  pdl_wait();
+  // not before: CTAs of the product behind this kernel would take the room that the per-token kernel's blocks need
+  if (tid == 0) pdl_trigger();
+  const float rs = q_norm_scale[ti];
+  int32_t product[kQbHeadsPerBlock * kQHead / 256];
+#pragma unroll
+  for (int u = 0; u < kQbHeadsPerBlock * kQHead / 256; ++u) product[u] = qb_i32[row0 + col0 + u * 256 + tid];
 #pragma unroll
   for (int u = 0; u < kQbHeadsPerBlock * kQHead / 256; ++u) {
-    const int e = u * 256 + threadIdx.x;  // element of the block's 8 x 192 slice
+    const int e = u * 256 + tid;  // element of the block's 8 x 192 slice
     const int64_t col = col0 + e;
-    const float v = bf16_round(__fmul_rn(__fmul_rn(static_cast<float>(qb_i32[row0 + col]), rs), w_scale[col]));
+    const float v = bf16_round(__fmul_rn(__fmul_rn(static_cast<float>(product[u]), rs), ws[u]));
     q_b[row0 + col] = __float2bfloat16_rn(v);
-    const int hh = e / kQHead, c = e % kQHead;
-    if (c >= kNope) pe[hh][c - kNope] = v;
+    const int hh = e / kQHead, d = e % kQHead;
+    if (d >= kNope) pe[hh][d - kNope] = v;
   }
   __syncthreads();
 #pragma unroll
   for (int u = 0; u < kQbHeadsPerBlock * kRope / 256; ++u) {
-    const int e = u * 256 + threadIdx.x;
-    const int hh = e / kRope, c = e % kRope;
+    const int hh = (u * 256 + tid) / kRope;
     // de-interleaved layout: first half = even dims, second half = odd dims; rotate_half = (-second, first)
     const int j = c & 31;
     const float even = pe[hh][2 * j], odd = pe[hh][2 * j + 1];
-    const float cs = ld_bf16(cos + ti * kRope + c), sn = ld_bf16(sin + ti * kRope + c);
     const float x = c < 32 ? even : odd;
     const float rot = c < 32 ? -odd : even;
     q_rope[(static_cast<int64_t>(ti) * kHeads + hg * kQbHeadsPerBlock + hh) * kRope + c] =
         __float2bfloat16_rn(__fadd_rn(__fmul_rn(x, cs), __fmul_rn(rot, sn)));
+  }
+}
+
+// ---- indexer query of few tokens: int32 -> bf16, rope, Hadamard rotation, per-head int8 -------------------------
+// grid = tokens, block = 256: all 64 heads; a warp rotates 16 heads x 64 columns. On a second stream beside the absorbed
+// query, with little shared memory, so that its blocks find room beside that product's CTAs. On CUDA cores with the matrix in
+// shared memory (41 KB, eight heads a block) it waited for those CTAs and took 12.6 us at 64 tokens (7.9 at 3): it ended the call.
+__global__ void __launch_bounds__(256)
+prolog_idxq_kernel(const int32_t* __restrict__ qi_i32, const float* __restrict__ q_norm_scale,
+                   const float* __restrict__ w_scale, const __nv_bfloat16* __restrict__ cos,
+                   const __nv_bfloat16* __restrict__ sin, const __nv_bfloat16* __restrict__ hadamard_q,
+                   int8_t* __restrict__ q_int8, __half* __restrict__ q_scale) {
+  __shared__ __align__(16) __nv_bfloat16 q[kIdxHeads][kIdxPitch];
+  __shared__ float half_amax[2][kIdxHeads];
+  const int ti = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, l4 = lane & 3;
+  {
+    const int l = tid & 15;  // dims l, l + 16, ... of a head: a dim and its partner of the rotation are in one thread
+    const float rs = q_norm_scale[ti];
+    float cs[4], sn[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      cs[j] = ld_bf16(cos + ti * kRope + l + 16 * j);
+      sn[j] = ld_bf16(sin + ti * kRope + l + 16 * j);
+    }
+#pragma unroll
+    for (int u = 0; u < kIdxHeads / 16; ++u) {
+      const int hh = u * 16 + (tid >> 4);
+      const int32_t* src = qi_i32 + (static_cast<int64_t>(ti) * kIdxHeads + hh) * kIdxDim + l;
+      float v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        v[j] = bf16_round(__fmul_rn(__fmul_rn(static_cast<float>(src[16 * j]), rs), __ldg(w_scale + hh * kIdxDim + l + 16 * j)));
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        float o = v[j];
+        if (j < 4) {
+          const float rot = j < 2 ? -v[j + 2] : v[j - 2];
+          o = __fadd_rn(__fmul_rn(v[j], cs[j]), __fmul_rn(rot, sn[j]));
+        }
+        q[hh][l + 16 * j] = __float2bfloat16_rn(o);
+      }
+    }
+  }
+  __syncthreads();
+  const int head0 = (warp >> 1) * 16, half = warp & 1;
+  float acc[8][4];
+  hadamard_rows<8>(hadamard_q, 0, half * 64, &q[head0][0], lane, acc);
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    float m = 0.f;
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        acc[n][2 * r + e] = bf16_round(acc[n][2 * r + e]);
+        m = fmaxf(m, fabsf(acc[n][2 * r + e]));
+      }
+    }
+    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+    if (l4 == 0) half_amax[half][head0 + g + 8 * r] = m;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const int hh = head0 + g + 8 * r;
+    const float sq = __fdiv_rn(127.0f, fmaxf(half_amax[0][hh], half_amax[1][hh]));
+    const int64_t head = static_cast<int64_t>(ti) * kIdxHeads + hh;
+    __align__(16) int8_t out[16];
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+      out[n] = quant_one(acc[n][2 * r], sq);
+      out[8 + n] = quant_one(acc[n][2 * r + 1], sq);
+    }
+    int8_t* dst = q_int8 + head * kIdxDim + half * 64 + 16 * l4;
+    if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+      *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(out);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 16; ++e) dst[e] = out[e];
+    }
+    if (half == 0 && l4 == 0) q_scale[head] = __float2half_rn(__fdiv_rn(1.0f, sq));
   }
 }
 
@@ -190,19 +334,23 @@ prolog_kv_kernel(const float* __restrict__ kv, const float* __restrict__ ki, con
                  const int64_t* __restrict__ cache_index, int64_t cache_rows, float eps_ckv, float ln_eps,
                  int8_t* __restrict__ kv_cache, __nv_bfloat16* __restrict__ kr_cache, float* __restrict__ kv_scale_cache,
                  int8_t* __restrict__ idx_k_cache, __half* __restrict__ idx_k_scale_cache, __half* __restrict__ weights,
-                 int8_t* __restrict__ packed_cache, int32_t* status) {
+                 int8_t* __restrict__ packed_cache, const void* next_hadamard, const void* next_scale, int32_t* status) {
   __shared__ float red[32];
   __shared__ float pe[kRope];
   __shared__ float kvec[kIdxDim];
-  __shared__ __align__(16) __nv_bfloat16 had[kIdxDim * kIdxDim];  // 32 KB, fetched while the norms are computed
+  __shared__ __align__(16) __nv_bfloat16 krow[16][kIdxPitch];  // the rotation's operand: row 0; what the others give is not read
+  __shared__ float kpart[2][kIdxDim];
   const int ti = blockIdx.x, i = threadIdx.x, lane = i & 31, warp = i >> 5;
-  {
-    const uint4* hsrc = reinterpret_cast<const uint4*>(hadamard_k);
-    uint4* hdst = reinterpret_cast<uint4*>(had);
-#pragma unroll 4
-    for (int u = i; u < kIdxDim * kIdxDim / 8; u += 128) hdst[u] = __ldg(hsrc + u);
-  }
+  prefetch_l2(hadamard_k, 2 * kIdxDim * kIdxDim, i, 128);
+  // for the indexer query's kernel, which would miss L2 while weights stream (some microseconds); each block a share
+  prefetch_l2(next_hadamard, 2 * kIdxDim * kIdxDim, ti * 128 + i, gridDim.x * 128);
+  prefetch_l2(next_scale, 4 * kIdxHeads * kIdxDim, ti * 128 + i, gridDim.x * 128);
   const int64_t row = cache_index[ti];
+  float gm[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) gm[e] = ld_bf16(gamma_ckv + 4 * i + e);
+  const float cs = ld_bf16(cos + ti * kRope + i % kRope), sn = ld_bf16(sin + ti * kRope + i % kRope);
+  const float lg = ld_bf16(ln_gamma + i), lb = ld_bf16(ln_beta + i);
   const bool row_ok = row >= 0 && row < cache_rows;
   if (!row_ok && i == 0) set_status(status, PTO_ST_BAD_PAGE, static_cast<int>(row), 60);
 
@@ -218,20 +366,24 @@ prolog_kv_kernel(const float* __restrict__ kv, const float* __restrict__ ki, con
     }
     return a;
   };
-  // latent part: bf16 rounding, RMSNorm, int8 per 128-wide tile
+  // latent part: bf16 rounding, RMSNorm, int8 per 128-wide tile. Everything that the thread reads of the projections is
+  // requested here, before the first sum over the block.
   const float* src = kv + static_cast<int64_t>(ti) * ld;
+  const float x = proj(ki + static_cast<int64_t>(ti) * ld + i);
+  const float tail = i < kRope ? proj(src + kLora + i) : proj(wp + static_cast<int64_t>(ti) * ld + (i - kRope));
   float v[4];
   float ss = 0.f;
 #pragma unroll
+  for (int e = 0; e < 4; ++e) v[e] = bf16_round(proj(src + 4 * i + e));
+#pragma unroll
   for (int e = 0; e < 4; ++e) {
-    v[e] = bf16_round(proj(src + 4 * i + e));
     ss = __fadd_rn(ss, __fmul_rn(__fmul_rn(v[e], v[e]), 1.0f / kLora));
   }
   const float rms = sqrtf(block_sum(ss, red) + eps_ckv);
   float amax = 0.f;
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
-    v[e] = bf16_round(__fmul_rn(__fdiv_rn(v[e], rms), ld_bf16(gamma_ckv + 4 * i + e)));
+    v[e] = bf16_round(__fmul_rn(__fdiv_rn(v[e], rms), gm[e]));
     amax = fmaxf(amax, fabsf(v[e]));
   }
   amax = warp_max(amax);
@@ -252,12 +404,11 @@ prolog_kv_kernel(const float* __restrict__ kv, const float* __restrict__ ki, con
   }
 
   // rope key: the 64 values after the latent part, de-interleaved rope
-  if (i < kRope) pe[i] = bf16_round(proj(src + kLora + i));
+  if (i < kRope) pe[i] = bf16_round(tail);
   __syncthreads();
   if (i < kRope && row_ok) {
     const int j = i & 31;
     const float even = pe[2 * j], odd = pe[2 * j + 1];
-    const float cs = ld_bf16(cos + ti * kRope + i), sn = ld_bf16(sin + ti * kRope + i);
     const float x = i < 32 ? even : odd;
     const float rot = i < 32 ? -odd : even;
     const __nv_bfloat16 kr = __float2bfloat16_rn(__fadd_rn(__fmul_rn(x, cs), __fmul_rn(rot, sn)));
@@ -266,26 +417,35 @@ prolog_kv_kernel(const float* __restrict__ kv, const float* __restrict__ ki, con
   }
 
   // indexer key: LayerNorm in fp32 -> bf16, rope on the first 64 dims (halves, no de-interleave), Hadamard, int8
-  const float x = proj(ki + static_cast<int64_t>(ti) * ld + i);
   const float mean = block_sum(x, red) * (1.0f / kIdxDim);
   const float dx = x - mean;
   const float var = block_sum(__fmul_rn(dx, dx), red) * (1.0f / kIdxDim);
   const float y = __fdiv_rn(dx, sqrtf(var + ln_eps));
-  kvec[i] = bf16_round(__fadd_rn(__fmul_rn(y, ld_bf16(ln_gamma + i)), ld_bf16(ln_beta + i)));
+  kvec[i] = bf16_round(__fadd_rn(__fmul_rn(y, lg), lb));
   __syncthreads();
   float k = kvec[i];
   if (i < kRope) {
-    const float cs = ld_bf16(cos + ti * kRope + i), sn = ld_bf16(sin + ti * kRope + i);
     const float rot = i < 32 ? -kvec[i + 32] : kvec[i - 32];
     k = bf16_round(__fadd_rn(__fmul_rn(k, cs), __fmul_rn(rot, sn)));
   }
+  krow[0][i] = __float2bfloat16_rn(k);
+#pragma unroll
+  for (int r = 1; r < 16; ++r) krow[r][i] = __float2bfloat16_rn(0.f);
+  __syncthreads();  // (and kvec has been read)
+  {
+    float acc[8][4];
+    const int half = warp & 1, part = warp >> 1;  // warp: 64 columns, half of the contraction
+    hadamard_rows<4>(hadamard_k, part * 64, half * 64, &krow[0][0], lane, acc);
+    if (lane < 4) {
+#pragma unroll
+      for (int n = 0; n < 8; ++n) {
+        kpart[part][half * 64 + 16 * lane + n] = acc[n][0];
+        kpart[part][half * 64 + 16 * lane + 8 + n] = acc[n][1];
+      }
+    }
+  }
   __syncthreads();
-  kvec[i] = k;
-  __syncthreads();
-  float acc = 0.f;
-#pragma unroll 8
-  for (int r = 0; r < kIdxDim; ++r) acc = fmaf(kvec[r], __bfloat162float(had[r * kIdxDim + i]), acc);
-  const float hk = bf16_round(acc);
+  const float hk = bf16_round(__fadd_rn(kpart[0][i], kpart[1][i]));
   const float kmax = block_max(fabsf(hk), red);
   const float ksq = __fdiv_rn(127.0f, kmax);
   if (row_ok) {
@@ -294,89 +454,10 @@ prolog_kv_kernel(const float* __restrict__ kv, const float* __restrict__ ki, con
   }
 
   // indexer weights: bf16 rounding, then heads^-1/2 and dim^-1/2 in fp32, fp16 out
-  if (i < kIdxHeads) {
-    const float w = bf16_round(proj(wp + static_cast<int64_t>(ti) * ld + i));
-    weights[static_cast<int64_t>(ti) * kIdxHeads + i] =
+  if (i >= kRope) {
+    const float w = bf16_round(tail);
+    weights[static_cast<int64_t>(ti) * kIdxHeads + i - kRope] =
         __float2half_rn(__fmul_rn(__fmul_rn(w, 0.125f), 0.08838834764831845f));
-  }
-}
-
-// ---- indexer query: int32 -> bf16, rope, Hadamard, per-head int8 ------------------------------------------
-// grid = (8 head groups, tokens), block = 128: eight heads per block share the Hadamard matrix, staged in
-// shared memory while the products are dequantised
-constexpr int kHeadsPerBlock = 8;
-__global__ void __launch_bounds__(128)
-prolog_idxq_kernel(const int32_t* __restrict__ qi_i32, const float* __restrict__ q_norm_scale,
-                   const float* __restrict__ w_scale, const __nv_bfloat16* __restrict__ cos,
-                   const __nv_bfloat16* __restrict__ sin, const __nv_bfloat16* __restrict__ hadamard_q,
-                   int8_t* __restrict__ q_int8, __half* __restrict__ q_scale) {
-  __shared__ float red8[4][kHeadsPerBlock];
-  __shared__ float qv[kHeadsPerBlock][kIdxDim];
-  __shared__ __align__(16) float qt[kIdxDim][kHeadsPerBlock];  // the roped rows, dim-major: 8 heads of a dim in 32 B
-  __shared__ __align__(16) __nv_bfloat16 had[kIdxDim * kIdxDim];
-  const int hg = blockIdx.x, ti = blockIdx.y, i = threadIdx.x;
-  {
-    const uint4* hsrc = reinterpret_cast<const uint4*>(hadamard_q);
-    uint4* hdst = reinterpret_cast<uint4*>(had);
-#pragma unroll 4
-    for (int u = i; u < kIdxDim * kIdxDim / 8; u += 128) hdst[u] = __ldg(hsrc + u);
-  }
-  const float rs = q_norm_scale[ti];
-  const float cs = i < kRope ? ld_bf16(cos + ti * kRope + i) : 0.f;
-  const float sn = i < kRope ? ld_bf16(sin + ti * kRope + i) : 0.f;
-#pragma unroll
-  for (int hh = 0; hh < kHeadsPerBlock; ++hh) {
-    const int64_t col = static_cast<int64_t>(hg * kHeadsPerBlock + hh) * kIdxDim + i;
-    const float v = __fmul_rn(__fmul_rn(static_cast<float>(qi_i32[static_cast<int64_t>(ti) * kIdxHeads * kIdxDim + col]), rs),
-                              w_scale[col]);
-    qv[hh][i] = bf16_round(v);
-  }
-  __syncthreads();
-  float q[kHeadsPerBlock];
-#pragma unroll
-  for (int hh = 0; hh < kHeadsPerBlock; ++hh) {
-    q[hh] = qv[hh][i];
-    if (i < kRope) {
-      const float rot = i < 32 ? -qv[hh][i + 32] : qv[hh][i - 32];
-      q[hh] = bf16_round(__fadd_rn(__fmul_rn(q[hh], cs), __fmul_rn(rot, sn)));
-    }
-  }
-#pragma unroll
-  for (int hh = 0; hh < kHeadsPerBlock; ++hh) qt[i][hh] = q[hh];
-  __syncthreads();
-  float acc[kHeadsPerBlock];
-#pragma unroll
-  for (int hh = 0; hh < kHeadsPerBlock; ++hh) acc[hh] = 0.f;
-#pragma unroll 4
-  for (int r = 0; r < kIdxDim; ++r) {  // per dim: one Hadamard element and two broadcast 16-byte reads of the 8 heads
-    const float hv = __bfloat162float(had[r * kIdxDim + i]);
-    const float4 a = *reinterpret_cast<const float4*>(&qt[r][0]);
-    const float4 b = *reinterpret_cast<const float4*>(&qt[r][4]);
-    acc[0] = fmaf(a.x, hv, acc[0]);
-    acc[1] = fmaf(a.y, hv, acc[1]);
-    acc[2] = fmaf(a.z, hv, acc[2]);
-    acc[3] = fmaf(a.w, hv, acc[3]);
-    acc[4] = fmaf(b.x, hv, acc[4]);
-    acc[5] = fmaf(b.y, hv, acc[5]);
-    acc[6] = fmaf(b.z, hv, acc[6]);
-    acc[7] = fmaf(b.w, hv, acc[7]);
-  }
-  // the eight row maxima with one hand-over through shared memory
-  float hq[kHeadsPerBlock];
-#pragma unroll
-  for (int hh = 0; hh < kHeadsPerBlock; ++hh) {
-    hq[hh] = bf16_round(acc[hh]);
-    const float m = warp_max(fabsf(hq[hh]));
-    if ((i & 31) == 0) red8[i >> 5][hh] = m;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int hh = 0; hh < kHeadsPerBlock; ++hh) {
-    const float amax = fmaxf(fmaxf(red8[0][hh], red8[1][hh]), fmaxf(red8[2][hh], red8[3][hh]));
-    const float sq = __fdiv_rn(127.0f, amax);
-    const int64_t head = static_cast<int64_t>(ti) * kIdxHeads + hg * kHeadsPerBlock + hh;
-    q_int8[head * kIdxDim + i] = quant_one(hq[hh], sq);
-    if (i == 0) q_scale[head] = __float2half_rn(__fdiv_rn(1.0f, sq));
   }
 }
 
@@ -472,12 +553,14 @@ prolog_kv_bf16_kernel(const float* __restrict__ kv, const float* __restrict__ ki
 // each (q_b[t, head, 128:192] -> q_rope[t, head, :]), groups 16..23 eight indexer heads each
 // (idx_query[t, head, 0:64] rotated in place; the other 64 dims of a head stay as the product wrote them)
 __global__ void __launch_bounds__(256)
-prolog_rope_bf16_kernel(const __nv_bfloat16* __restrict__ q_b, const __nv_bfloat16* __restrict__ cos,
-                        const __nv_bfloat16* __restrict__ sin, __nv_bfloat16* __restrict__ q_rope,
-                        __nv_bfloat16* __restrict__ idx_query) {
+prolog_rope_bf16_kernel(const __nv_bfloat16* q_b, const __nv_bfloat16* __restrict__ cos,
+                        const __nv_bfloat16* __restrict__ sin, __nv_bfloat16* __restrict__ q_rope, __nv_bfloat16* idx_query) {
+  // (q_b not __restrict__, as above)
   __shared__ float pe[8][kRope];
-  pdl_wait();
   if (threadIdx.x == 0) pdl_trigger();
+  const int rc = threadIdx.x % kRope;  // a thread rotates one dim of several heads
+  const float cs = ld_bf16(cos + blockIdx.y * kRope + rc), sn = ld_bf16(sin + blockIdx.y * kRope + rc);
+  pdl_wait();
   const int g = blockIdx.x, ti = blockIdx.y;
   const bool att = g < kHeads / 8;
   const int head0 = att ? g * 8 : (g - kHeads / 8) * 8;
@@ -494,7 +577,6 @@ prolog_rope_bf16_kernel(const __nv_bfloat16* __restrict__ q_b, const __nv_bfloat
   for (int u = 0; u < 2; ++u) {
     const int e = u * 256 + threadIdx.x;
     const int hh = e >> 6, c = e & 63;
-    const float cs = ld_bf16(cos + ti * kRope + c), sn = ld_bf16(sin + ti * kRope + c);
     const __nv_bfloat16 o = __float2bfloat16_rn(rope_deinterleaved(pe[hh], c, cs, sn));
     if (att) {
       q_rope[(static_cast<int64_t>(ti) * kHeads + head0 + hh) * kRope + c] = o;
@@ -574,8 +656,8 @@ cudaError_t launch_prolog_kv(const float* kv, const float* ki, const float* wp, 
                              const void* sin, const void* ln_gamma, const void* ln_beta, const void* hadamard_k,
                              const int64_t* cache_index, int64_t cache_rows, int t, float eps_ckv, float ln_eps,
                              int8_t* kv_cache, void* kr_cache, float* kv_scale_cache, int8_t* idx_k_cache,
-                             void* idx_k_scale_cache, void* weights, int8_t* packed_cache, int32_t* status,
-                             cudaStream_t stream) {
+                             void* idx_k_scale_cache, void* weights, int8_t* packed_cache, const void* next_hadamard,
+                             const void* next_scale, int32_t* status, cudaStream_t stream) {
   count_launch();
   prolog_kv_kernel<<<t, 128, 0, stream>>>(
       kv, ki, wp, ld, n_split, split_stride, reinterpret_cast<const __nv_bfloat16*>(gamma_ckv),
@@ -583,7 +665,8 @@ cudaError_t launch_prolog_kv(const float* kv, const float* ki, const float* wp, 
       reinterpret_cast<const __nv_bfloat16*>(sin), reinterpret_cast<const __nv_bfloat16*>(ln_gamma),
       reinterpret_cast<const __nv_bfloat16*>(ln_beta), reinterpret_cast<const __nv_bfloat16*>(hadamard_k), cache_index,
       cache_rows, eps_ckv, ln_eps, kv_cache, reinterpret_cast<__nv_bfloat16*>(kr_cache), kv_scale_cache, idx_k_cache,
-      reinterpret_cast<__half*>(idx_k_scale_cache), reinterpret_cast<__half*>(weights), packed_cache, status);
+      reinterpret_cast<__half*>(idx_k_scale_cache), reinterpret_cast<__half*>(weights), packed_cache,
+      next_hadamard, next_scale, status);
   return cudaGetLastError();
 }
 
@@ -615,7 +698,7 @@ cudaError_t launch_prolog_idxq(const int32_t* qi_i32, const float* q_norm_scale,
                                const void* sin, const void* hadamard_q, int t, int8_t* q_int8, void* q_scale,
                                cudaStream_t stream) {
   count_launch();
-  prolog_idxq_kernel<<<dim3(kIdxHeads / kHeadsPerBlock, t), 128, 0, stream>>>(
+  prolog_idxq_kernel<<<t, 256, 0, stream>>>(
       qi_i32, q_norm_scale, w_scale, reinterpret_cast<const __nv_bfloat16*>(cos),
       reinterpret_cast<const __nv_bfloat16*>(sin), reinterpret_cast<const __nv_bfloat16*>(hadamard_q), q_int8,
       reinterpret_cast<__half*>(q_scale));

@@ -23,15 +23,12 @@ namespace {
 constexpr int kGTileN = 128;              // weight columns per tile (MMA M)
 constexpr int kGTileK = 128;              // k rows per stage
 constexpr int kGStageBytes = kGTileN * kGTileK;  // 16 KB
-constexpr int kGMaxStages = 10;           // ring stages: as many as fit beside the activations, see kGDataBudget
+constexpr int kGMaxStages = 10;           // ring stages: as many as fit beside the activations, see kGDataMax
 constexpr int kGXBytesMax = 96 * 1024;    // resident activations: (K / 128) * t_pad * 128 bytes
-// Ring + activations: at most kGDataMax. With more than 32 token rows they stay within kGDataBudget, so that a
-// block of the prolog's per-token kernel (33 KB of shared memory, launched on a second stream just before this
-// kernel) fits on the same SM: with all of shared memory taken here, those blocks (one per token) kept their SMs to
-// themselves and this kernel's CTAs there started 5 us late (64 tokens: 63.3 -> 60.5 us per prolog call; with 8 or
-// 32 tokens sharing costs about 1 us more than it returns, so fewer tokens keep the larger ring).
-constexpr int kGDataBudget = 176 * 1024;
-constexpr int kGDataMax = 192 * 1024;
+// Ring + activations: a block of the prolog's per-token kernel (34 KB of shared memory, on a second stream beside this
+// kernel) has to fit on the same SM. Where it did not, it either waited for this kernel's first CTAs to end (26 us into a
+// call of 3 tokens, where its input is there at 14) or, scheduled first, kept a CTA of this kernel waiting.
+constexpr int kGDataMax = 190 * 1024;
 constexpr int kGThreads = 192;
 
 struct GemmCtl {
@@ -45,7 +42,7 @@ struct GemmCtl {
 };
 
 constexpr int kGSmemBytes = kGDataMax + sizeof(GemmCtl) + 1024;
-static_assert(kGXBytesMax + 2 * kGStageBytes <= kGDataBudget, "no room for a ring beside the activations");
+static_assert(kGXBytesMax + 2 * kGStageBytes <= kGDataMax, "no room for a ring beside the activations");
 
 struct GemmParams {
   int32_t* out[2];   // [t, ld] row-major
@@ -101,16 +98,21 @@ prolog_i8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = ctl->tmem_base;
-  // the set-up above overlaps the tail of the kernel before it; its results are read from here on
-  pdl_wait();
+  // The set-up above overlaps the tail of the kernel before it; its results are read behind pdl_wait(). The weights are
+  // nobody's result: the producer fills the ring with them first.
   if (tid == 0) pdl_trigger();
+  if (warp != 0) pdl_wait();
 
   if (warp == 0) {
     // ---------------- producer ----------------
     if (lane == 0) {
-      bool ok = true;
-      mbar_arrive_expect_tx(smem_u32(&ctl->x_full), static_cast<uint32_t>(chunks) * x_slab);
-      for (int c = 0; c < chunks; ++c) tma_load_2d(x_base + c * x_slab, &tmap_x, c * kGTileK, 0, smem_u32(&ctl->x_full));
+      bool ok = true, waited = false;
+      auto load_x = [&]() {
+        pdl_wait();
+        waited = true;
+        mbar_arrive_expect_tx(smem_u32(&ctl->x_full), static_cast<uint32_t>(chunks) * x_slab);
+        for (int c = 0; c < chunks; ++c) tma_load_2d(x_base + c * x_slab, &tmap_x, c * kGTileK, 0, smem_u32(&ctl->x_full));
+      };
       uint32_t it = 0;
       const uint64_t w_policy = l2_policy_evict_first();  // weights are read once per call
       for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
@@ -120,6 +122,7 @@ prolog_i8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_
         for (int c = 0; c < chunks; ++c, ++it) {
           const uint32_t s = it % n_stages;
           if (it >= n_stages) {
+            if (!waited) load_x();
             ok = mbar_wait(smem_u32(&ctl->empty[s]), ((it / n_stages) - 1) & 1);
             if (!ok) break;
           }
@@ -127,6 +130,7 @@ prolog_i8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_
           tma_load_2d_hint(a_base + s * kGStageBytes, tm, n0, c * kGTileK, smem_u32(&ctl->full[s]), w_policy);
         }
       }
+      if (!waited) load_x();
       if (!ok) {
         ctl->abort = 1;
         set_status(p.status, PTO_ST_WAIT_EXPIRED, blockIdx.x, 70);
@@ -228,6 +232,9 @@ cudaError_t launch_prolog_i8_gemm(const void* tmap_w0, const void* tmap_w1, cons
                                   bool pdl) {
   cudaError_t e = cudaFuncSetAttribute(prolog_i8_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGSmemBytes);
   if (e != cudaSuccess) return e;
+  // all of the SM's shared memory, not just what a CTA of this kernel takes: kernels beside it need some as well
+  e = cudaFuncSetAttribute(prolog_i8_gemm_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+  if (e != cudaSuccess) return e;
   GemmParams p{};
   p.out[0] = out0;
   p.out[1] = out1;
@@ -239,9 +246,9 @@ cudaError_t launch_prolog_i8_gemm(const void* tmap_w0, const void* tmap_w1, cons
   p.t = t;
   p.t_pad = (t + 15) / 16 * 16;
   const int x_bytes = (k / kGTileK) * p.t_pad * 128;
-  p.data_bytes = p.t_pad > 32 ? kGDataBudget : kGDataMax;
-  p.n_stages = (p.data_bytes - x_bytes) / kGStageBytes;
+  p.n_stages = (kGDataMax - x_bytes) / kGStageBytes;
   if (p.n_stages > kGMaxStages) p.n_stages = kGMaxStages;
+  p.data_bytes = p.n_stages * kGStageBytes + x_bytes;
   const int smem_bytes = p.data_bytes + static_cast<int>(sizeof(GemmCtl)) + 1024;
   p.status = status;
   const int n_tiles = p.tiles[0] + p.tiles[1];

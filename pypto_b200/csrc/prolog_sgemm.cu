@@ -18,6 +18,8 @@
 // accumulators in tensor memory. Every wait is bounded and reports PTO_ST_WAIT_EXPIRED.
 #include <cuda.h>
 
+#include <climits>
+
 #include "sfa_common.cuh"
 
 namespace pto {
@@ -26,7 +28,7 @@ namespace {
 
 constexpr int kSTileN = 128;          // weight columns per tile (MMA M)
 constexpr int kSWBytes = 16384;       // weight tile bytes per stage
-constexpr int kSMaxStages = 8;
+constexpr int kSMaxStages = 10;
 constexpr int kSRingBytes = 192 * 1024;
 constexpr int kSThreads = 192;
 constexpr int kSMaxRows = 256;        // token rows per block (MMA N)
@@ -60,6 +62,7 @@ struct SGemmParams {
   long long ld_out;       // output elements between token rows
   long long split_stride; // output elements between the partials of two splits
   void* out;
+  PrologOut2 out2;        // `first` is INT_MAX without one
   int n_stages;
   uint32_t stage_bytes;   // kSWBytes + t_pad * 128
   uint32_t tmem_cols;
@@ -108,7 +111,7 @@ prolog_sgemm_kernel(const __grid_constant__ PrologWMaps maps_w, const __grid_con
     ctl->abort = 0;
     fence_mbar_init();
     fence_proxy_async();
-    for (int i = 0; i < (kOut == kOutF32 ? 4 : 1); ++i) tma_prefetch_desc(&maps_w.map[i]);
+    for (int i = 0; i < (kOut == kOutF32 ? 4 : 2); ++i) tma_prefetch_desc(&maps_w.map[i]);
     tma_prefetch_desc(&tmap_x);
   }
   if (warp == 1) {
@@ -119,38 +122,46 @@ prolog_sgemm_kernel(const __grid_constant__ PrologWMaps maps_w, const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = ctl->tmem_base;
-  // the set-up above overlaps the tail of the kernel before it; its results are read (and buffers it may still
-  // read are overwritten) from here on
-  pdl_wait();
+  // The set-up above overlaps the tail of the kernel before it; its results are read (and buffers it may still read are
+  // overwritten) behind pdl_wait(). The weights are nobody's result: the producer fills the ring with them first.
   if (tid == 0) pdl_trigger();
+  if (warp != 0) pdl_wait();
 
   if (warp == 0) {
     // ---------------- producer ----------------
     if (lane == 0) {
       bool ok = true;
-      uint32_t it = 0;
       // weights are read once per call: first to leave L2, so that activations and partial sums stay there
       const uint64_t w_policy = l2_policy_evict_first();
-      for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-        const SItem w = s_item(p, item);
-        const int k0 = w.split * p.per_split;
-        const int kn = min(p.per_split, p.chunks - k0);
-        int col0, col1;  // the tile's two 64-column boxes
-        const CUtensorMap* m0 = prolog_w_box(maps_w, p.boxes, 2 * w.tile, &col0);
-        const CUtensorMap* m1 = prolog_w_box(maps_w, p.boxes, 2 * w.tile + 1, &col1);
-        for (int c = 0; c < kn; ++c, ++it) {
-          const uint32_t s = it % p.n_stages;
-          if (it >= static_cast<uint32_t>(p.n_stages)) {
-            ok = mbar_wait(smem_u32(&ctl->empty[s]), ((it / p.n_stages) - 1) & 1);
-            if (!ok) break;
+      const uint32_t n_stages = static_cast<uint32_t>(p.n_stages);
+#pragma unroll 1
+      for (int pass = 0; pass < 2 && ok; ++pass) {  // 0: weights of the first n_stages chunks; 1: their rows of x, and the rest
+        uint32_t it = 0;
+        if (pass == 1) pdl_wait();
+        for (int item = blockIdx.x; item < n_items && ok && (pass == 1 || it < n_stages); item += gridDim.x) {
+          const SItem w = s_item(p, item);
+          const int k0 = w.split * p.per_split;
+          const int kn = min(p.per_split, p.chunks - k0);
+          int col0, col1;  // the tile's two 64-column boxes
+          const CUtensorMap* m0 = prolog_w_box(maps_w, p.boxes, 2 * w.tile, &col0);
+          const CUtensorMap* m1 = prolog_w_box(maps_w, p.boxes, 2 * w.tile + 1, &col1);
+          for (int c = 0; c < kn; ++c, ++it) {
+            if (pass == 0 && it >= n_stages) break;
+            const uint32_t s = it % n_stages;
+            const uint32_t bar = smem_u32(&ctl->full[s]);
+            const uint32_t dst = base + s * p.stage_bytes;
+            if (it >= n_stages) {
+              ok = mbar_wait(smem_u32(&ctl->empty[s]), ((it / n_stages) - 1) & 1);
+              if (!ok) break;
+            }
+            if (pass == 0 || it >= n_stages) {
+              const int krow = w.b * p.w_batch_rows + (k0 + c) * kChunkK;
+              mbar_arrive_expect_tx(bar, kSWBytes + x_bytes);
+              tma_load_2d_hint(dst, m0, col0, krow, bar, w_policy);
+              tma_load_2d_hint(dst + kSWBytes / 2, m1, col1, krow, bar, w_policy);
+            }
+            if (pass == 1) tma_load_2d(dst + kSWBytes, &tmap_x, w.b * p.x_batch_bytes + (k0 + c) * 128, w.tb * p.t_pad, bar);
           }
-          const uint32_t bar = smem_u32(&ctl->full[s]);
-          const uint32_t dst = base + s * p.stage_bytes;
-          const int krow = w.b * p.w_batch_rows + (k0 + c) * kChunkK;
-          mbar_arrive_expect_tx(bar, kSWBytes + x_bytes);
-          tma_load_2d_hint(dst, m0, col0, krow, bar, w_policy);
-          tma_load_2d_hint(dst + kSWBytes / 2, m1, col1, krow, bar, w_policy);
-          tma_load_2d(dst + kSWBytes, &tmap_x, w.b * p.x_batch_bytes + (k0 + c) * 128, w.tb * p.t_pad, bar);
         }
       }
       if (!ok) {
@@ -209,7 +220,11 @@ prolog_sgemm_kernel(const __grid_constant__ PrologWMaps maps_w, const __grid_con
       tc_fence_after();
       const int n = w.tile * kSTileN + q * 32 + lane;
       const bool col_ok = n < p.n;
-      const long long col = static_cast<long long>(w.b) * p.out_batch + n + static_cast<long long>(w.split) * p.split_stride;
+      const bool second = w.tile * kSTileN >= p.out2.first;
+      void* out = second ? p.out2.out : p.out;
+      const long long ld_out = second ? p.out2.ld : p.ld_out;
+      const long long col = static_cast<long long>(w.b) * p.out_batch + (second ? n - p.out2.first : n) +
+                            static_cast<long long>(w.split) * p.split_stride;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * static_cast<uint32_t>(p.t_pad);
       const int tok0 = w.tb * p.t_pad;
       for (int c0 = 0; c0 < p.t_pad && tok0 + c0 < p.t; c0 += 16) {
@@ -220,9 +235,9 @@ prolog_sgemm_kernel(const __grid_constant__ PrologWMaps maps_w, const __grid_con
         for (int e = 0; e < 16; ++e) {
           const int tok = tok0 + c0 + e;
           if (tok < p.t && col_ok) {  // 32 lanes: consecutive columns of one token row
-            const long long at = static_cast<long long>(tok) * p.ld_out + col;
-            if (kOut == kOutF32) reinterpret_cast<float*>(p.out)[at] = __uint_as_float(v[e]);
-            if (kOut == kOutBf16) reinterpret_cast<__nv_bfloat16*>(p.out)[at] = __float2bfloat16_rn(__uint_as_float(v[e]));
+            const long long at = static_cast<long long>(tok) * ld_out + col;
+            if (kOut == kOutF32) reinterpret_cast<float*>(out)[at] = __uint_as_float(v[e]);
+            if (kOut == kOutBf16) reinterpret_cast<__nv_bfloat16*>(out)[at] = __float2bfloat16_rn(__uint_as_float(v[e]));
           }
         }
       }
@@ -254,6 +269,9 @@ cudaError_t launch_one(const PrologWMaps& maps_w, const void* tmap_x, const SGem
                        bool pdl) {
   auto kernel = prolog_sgemm_kernel<kOut>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSSmemMax);
+  if (e != cudaSuccess) return e;
+  // all of the SM's shared memory, not just what a CTA of this kernel takes: kernels beside it need some as well
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return e;
   const size_t smem = static_cast<size_t>(p.n_stages) * p.stage_bytes + sizeof(SCtl) + 1024;
   count_launch();
@@ -292,8 +310,10 @@ int prolog_sgemm_splits(int t, int n, int k, int num_sms) {
 cudaError_t launch_prolog_sgemm(int kind, const PrologWMaps& maps_w, const PrologWBoxes& boxes, const void* tmap_x, void* out, int t, int n, int k,
                                 int batch, int w_batch_rows, int x_batch_bytes, long long out_batch, long long ld_out,
                                 int splits, long long split_stride, int num_sms, int32_t* status, cudaStream_t stream,
-                                bool pdl) {
+                                bool pdl, const PrologOut2* out2) {
   SGemmParams p{};
+  p.out2.first = INT_MAX;
+  if (out2 != nullptr) p.out2 = *out2;
   p.n_tiles = (n + kSTileN - 1) / kSTileN;
   p.chunks = (k + 63) / 64;
   p.splits = splits < 1 ? 1 : splits;
