@@ -112,6 +112,14 @@ def test_head_slices_at_tile_edges(nq, lens, s1, packed):
                 assert torch.all(got[bi, i] == 0)
 
 
+@pytest.mark.parametrize("tokens", [1, 14, 15, 24, 37], ids=lambda t: f"{t}_tokens")  # 16, 5, 4, 3 and 2 splits
+def test_merge_of_splits(tokens):
+    d = gen.make_inputs([(1, 130, 300, 700)[i % 4] for i in range(tokens)], s1=1, seed=tokens, with_indexer=False, with_topk=True)
+    want = oracle.sparse_attention(d.query_nope, d.query_rope, d.key_nope_2d, d.key_rope_2d, d.k_nope_scales,
+                                   d.topk_indices, d.block_table, d.act_seq, d.s1)
+    _check(_run(d), want)
+
+
 def test_order_of_indices_does_not_matter_beyond_rounding():
     d = gen.make_inputs([5000], s1=1, seed=2, with_indexer=False, with_topk=True)
     a = _run(d)
