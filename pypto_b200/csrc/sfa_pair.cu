@@ -865,6 +865,23 @@ sfa_pair_kernel(const __grid_constant__ SfaParams p) {
   c.ti = bid / p.n_split;
   c.bi = c.ti / p.s1;
   const int si = c.ti % p.s1;
+  c.q_row0 = static_cast<int64_t>(c.ti) * p.nq_total + p.head_begin;
+
+  // This CTA's 64 query rows for shared memory, nine swizzled chunks of 64 dims (A operand of q.K^T): 64 x 72 16-byte
+  // units, twelve per thread of the twelve warps that are not producers. Requested before the sequence length is there (it
+  // takes as long as they do), stored below.
+  constexpr int kLoaders = 32 * kPairKWarp0;
+  uint4 w[12];
+  if (warp < kPairKWarp0) {
+    const int64_t row0 = c.q_row0 + 64 * crank;
+#pragma unroll
+    for (int i = 0; i < 12; ++i) {
+      const int e = tid + i * kLoaders;
+      const int r = e / 72, u = e % 72;
+      w[i] = (u < 64) ? ldg_pinned_v4(reinterpret_cast<const uint8_t*>(p.q_nope + (row0 + r) * 512) + 16 * u)
+                      : ldg_pinned_v4(reinterpret_cast<const uint8_t*>(p.q_rope + (row0 + r) * 64) + 16 * (u - 64));
+    }
+  }
 
   int n = p.act_seq[c.bi] - p.s1 + 1 + si;
   n = max(0, min(n, p.topk_k));
@@ -874,7 +891,6 @@ sfa_pair_kernel(const __grid_constant__ SfaParams p) {
   c.end = min(n, (c.sp + 1) * tiles_per_split * kPT);
   c.ntiles = (c.end - c.begin + kPT - 1) / kPT;
   c.idx_row = p.topk + static_cast<int64_t>(c.ti) * p.topk_k;
-  c.q_row0 = static_cast<int64_t>(c.ti) * p.nq_total + p.head_begin;
 
   if (c.ntiles == 0) {  // same decision in both CTAs of the pair
     if (p.n_split == 1) {
@@ -921,20 +937,8 @@ sfa_pair_kernel(const __grid_constant__ SfaParams p) {
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     if (tid == 0) TLP(1, 21);
   }
-  // this CTA's 64 query rows into shared memory, nine swizzled chunks of 64 dims (A operand of q.K^T): 64 x 72
-  // 16-byte units, twelve per thread of the twelve warps that are not producers, all loads in flight before the
-  // first store. The producers go straight to their first rows.
+  // (the producers go straight to their first rows)
   if (warp < kPairKWarp0) {
-    constexpr int kLoaders = 32 * kPairKWarp0;
-    const int64_t row0 = c.q_row0 + 64 * crank;
-    uint4 w[12];
-#pragma unroll
-    for (int i = 0; i < 12; ++i) {
-      const int e = tid + i * kLoaders;
-      const int r = e / 72, u = e % 72;
-      w[i] = (u < 64) ? __ldg(reinterpret_cast<const uint4*>(p.q_nope + (row0 + r) * 512) + u)
-                      : __ldg(reinterpret_cast<const uint4*>(p.q_rope + (row0 + r) * 64) + (u - 64));
-    }
 #pragma unroll
     for (int i = 0; i < 12; ++i) {
       const int e = tid + i * kLoaders;
