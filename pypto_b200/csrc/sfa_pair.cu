@@ -204,15 +204,25 @@ struct PairCtx {
   int ntiles, begin, end, ti, sp, bi;
 };
 
-// The one meeting of all threads of the pair before the tile loop: barriers initialised, tensor memory allocated,
-// both Q halves in shared memory. Every role calls it exactly once; the producers call it after they have
-// requested their first rows, so that the index -> block table -> row chain of the first tile (three dependent
-// trips to memory) runs beside the set-up instead of after it.
+// The one meeting of all threads of the pair before the tile loop (barriers initialised, tensor memory allocated, both Q
+// halves in shared memory), in two parts. The producers have nothing to show the others and arrive first thing; they wait
+// when tile 0 is converted, whose place nobody has used before, so that the index -> block table -> row chain and the
+// conversion of the first tile run beside the set-up and the meeting's own latency (1.5-2 k cycles) instead of after them.
+// The other twelve warps meet among themselves, then arrive for what they wrote, and wait.
+__device__ __forceinline__ void pair_setup_arrive() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void pair_setup_wait() {
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  tc_fence_after();
+}
 __device__ __forceinline__ uint32_t pair_setup_sync(PairCtl* ctl) {
   tc_fence_before();
-  __syncthreads();
-  pair_cluster_sync();
-  tc_fence_after();
+  asm volatile("bar.sync 2, %0;" ::"n"(32 * kPairKWarp0) : "memory");
+  pair_setup_arrive();
+  pair_setup_wait();
   // the kernel behind this one (the merge of the split partials) may be scheduled from here on; it waits for
   // this grid to complete before it reads anything
   if (threadIdx.x == 0) pdl_trigger();
@@ -669,6 +679,7 @@ __device__ __forceinline__ void pair_role_kproducer(const SfaParams& p, const Pa
   };
   const uint32_t k_rows = c.base + kSmemK + (4 * half + cp) * kChunk + (16 * g + r4) * 128;  // row r4 of this lane's chunk of line 0
   bool ok = true;
+  pair_setup_arrive();
   pdl_wait();          // the selected indices come from the kernel before this one, which may still be running
   if (ptid == 0) TLP(3, 21);
   int row_cur;         // this lane's row of tile j
@@ -692,7 +703,6 @@ __device__ __forceinline__ void pair_role_kproducer(const SfaParams& p, const Pa
     if (ptid == 0) TLP(6, 21);
   }
   if (!kBf && ptid == 0 && d[0][0].x != 0x7fffffffu) TLP(7, 21);  // first rows arrived
-  pair_setup_sync(ctl);
   for (int j = 0; j < ntiles; ++j) {
     if (j > 0) {  // the q.K^T MMAs of the previous tile that read this half of the chunks are complete
       ok = pair_wait(smem_u32(&ctl->kfree[half]), (j - 1) & 1);
@@ -730,6 +740,7 @@ __device__ __forceinline__ void pair_role_kproducer(const SfaParams& p, const Pa
     }
     if (kBf || half == 1) asm volatile("cp.async.wait_all;" ::: "memory");
     fence_proxy_async();
+    if (j == 0) pair_setup_wait();
     __syncwarp();
     if (lane == 0) mbar_arrive(smem_u32(&ctl->kfull[half]));
     if (ptid == 0) TLP(1, j);
@@ -785,6 +796,7 @@ __device__ __forceinline__ void pair_role_vproducer(const SfaParams& p, const Pa
   // row r4 of this warp's 16 in this lane's chunk of line 0; line 1 lies two chunks further
   const uint32_t v_rows = c.base + kSmemV + (q >> 1) * kVHalfBytes + cp * kChunk + (32 * (q & 1) + 16 * h + r4) * 128;
   bool ok = true;
+  pair_setup_arrive();
   pdl_wait();
   int row_cur, row_n, idx_a, entry_a, idx_b;  // this lane's row of tiles j, j+1; index and block-table entry of j+2; index of j+3
   {
@@ -798,7 +810,6 @@ __device__ __forceinline__ void pair_role_vproducer(const SfaParams& p, const Pa
     issue_loads(row_cur);
     row_n = pair_row(p, idx1, e1);
   }
-  pair_setup_sync(ctl);
   for (int j = 0; j < ntiles; ++j) {
     if (j > 0) {  // the P.V MMAs of the previous tile that read this key quarter are complete
       ok = pair_wait(smem_u32(&ctl->vfree[q]), (j - 1) & 1);
@@ -827,6 +838,7 @@ __device__ __forceinline__ void pair_role_vproducer(const SfaParams& p, const Pa
     }
     if (kBf) asm volatile("cp.async.wait_all;" ::: "memory");
     fence_proxy_async();
+    if (j == 0) pair_setup_wait();
     __syncwarp();
     if (lane == 0) mbar_arrive(smem_u32(&ctl->vfull[q]));
     if (vtid == 0) TLP(5, j);
