@@ -64,6 +64,7 @@ struct SGemmParams {
   void* out;
   PrologOut2 out2;        // `first` is INT_MAX without one
   int n_stages;
+  int ahead;              // launched behind a kernel that may still run: weights first, see the producer
   uint32_t stage_bytes;   // kSWBytes + t_pad * 128
   uint32_t tmem_cols;
   PrologWBoxes boxes;
@@ -134,11 +135,14 @@ prolog_sgemm_kernel(const __grid_constant__ PrologWMaps maps_w, const __grid_con
       // weights are read once per call: first to leave L2, so that activations and partial sums stay there
       const uint64_t w_policy = l2_policy_evict_first();
       const uint32_t n_stages = static_cast<uint32_t>(p.n_stages);
+      // pass 0: weights of the first n_stages chunks; 1: their rows of x, and the rest. With nothing to wait for, pass 1 alone:
+      // behind a ring full of weights the first rows of x arrive last, 8 k cycles later, and no chunk is complete before.
+      const uint32_t ahead = p.ahead != 0 ? n_stages : 0u;
 #pragma unroll 1
-      for (int pass = 0; pass < 2 && ok; ++pass) {  // 0: weights of the first n_stages chunks; 1: their rows of x, and the rest
+      for (int pass = p.ahead != 0 ? 0 : 1; pass < 2 && ok; ++pass) {
         uint32_t it = 0;
         if (pass == 1) pdl_wait();
-        for (int item = blockIdx.x; item < n_items && ok && (pass == 1 || it < n_stages); item += gridDim.x) {
+        for (int item = blockIdx.x; item < n_items && ok && (pass == 1 || it < ahead); item += gridDim.x) {
           const SItem w = s_item(p, item);
           const int k0 = w.split * p.per_split;
           const int kn = min(p.per_split, p.chunks - k0);
@@ -146,7 +150,7 @@ prolog_sgemm_kernel(const __grid_constant__ PrologWMaps maps_w, const __grid_con
           const CUtensorMap* m0 = prolog_w_box(maps_w, p.boxes, 2 * w.tile, &col0);
           const CUtensorMap* m1 = prolog_w_box(maps_w, p.boxes, 2 * w.tile + 1, &col1);
           for (int c = 0; c < kn; ++c, ++it) {
-            if (pass == 0 && it >= n_stages) break;
+            if (pass == 0 && it >= ahead) break;
             const uint32_t s = it % n_stages;
             const uint32_t bar = smem_u32(&ctl->full[s]);
             const uint32_t dst = base + s * p.stage_bytes;
@@ -154,7 +158,7 @@ prolog_sgemm_kernel(const __grid_constant__ PrologWMaps maps_w, const __grid_con
               ok = mbar_wait(smem_u32(&ctl->empty[s]), ((it / n_stages) - 1) & 1);
               if (!ok) break;
             }
-            if (pass == 0 || it >= n_stages) {
+            if (pass == 0 || it >= ahead) {
               const int krow = w.b * p.w_batch_rows + (k0 + c) * kChunkK;
               mbar_arrive_expect_tx(bar, kSWBytes + x_bytes);
               tma_load_2d_hint(dst, m0, col0, krow, bar, w_policy);
@@ -335,6 +339,7 @@ cudaError_t launch_prolog_sgemm(int kind, const PrologWMaps& maps_w, const Prolo
   p.n_stages = kSRingBytes / static_cast<int>(p.stage_bytes);
   if (p.n_stages > kSMaxStages) p.n_stages = kSMaxStages;
   p.status = status;
+  p.ahead = pdl ? 1 : 0;
   const long long items = static_cast<long long>(p.tok_blocks) * p.batch * p.n_tiles * p.splits;
   int grid = static_cast<int>(items < num_sms ? items : num_sms);
   uint32_t accs = 2;
