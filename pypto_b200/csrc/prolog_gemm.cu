@@ -138,38 +138,42 @@ prolog_i8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      const uint32_t idesc = umma_idesc(kCFmtS32, kABFmtS8, kABFmtS8, 1, 0, kGTileN, static_cast<uint32_t>(p.t_pad));
-      bool ok = mbar_wait(smem_u32(&ctl->x_full), 0);
-      uint32_t it = 0, ti = 0;
-      for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, ++ti) {
-        const uint32_t acc = ti & 1;
-        if (ti >= 2) {
-          ok = mbar_wait(smem_u32(&ctl->acc_empty[acc]), ((ti >> 1) - 1) & 1);
-          if (!ok) break;
-        }
+    // The warp stays converged and one elected lane issues; waits probe without blocking. (From a lone lane, with blocking
+    // waits and a division per chunk for the ring's place, a chunk of four MMAs took 760 cycles: as long as its weights take
+    // to stream, but the weights of the first tile are already there.)
+    const uint32_t idesc = umma_idesc(kCFmtS32, kABFmtS8, kABFmtS8, 1, 0, kGTileN, static_cast<uint32_t>(p.t_pad));
+    bool ok = mbar_wait_warp(smem_u32(&ctl->x_full), 0);
+    uint32_t s = 0, phase = 0, ti = 0;
+    const uint64_t a_base_desc = desc_mnmajor_sw128(a_base, 16, 1024), b_base_desc = umma_desc_kmajor_sw128(x_base);
+    for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, ++ti) {
+      const uint32_t acc = ti & 1;
+      if (ti >= 2) ok = mbar_wait_warp(smem_u32(&ctl->acc_empty[acc]), ((ti >> 1) - 1) & 1);
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t d = tmem_base + acc * 64u;
+      for (int c = 0; c < chunks; ++c) {
+        ok = mbar_wait_warp(smem_u32(&ctl->full[s]), phase);
+        if (!ok) break;
         tc_fence_after();
-        const uint32_t d = tmem_base + acc * 64u;
-        for (int c = 0; c < chunks; ++c, ++it) {
-          const uint32_t s = it % n_stages;
-          ok = mbar_wait(smem_u32(&ctl->full[s]), (it / n_stages) & 1);
-          if (!ok) break;
-          tc_fence_after();
-          const uint64_t b_desc = umma_desc_kmajor_sw128(x_base + c * x_slab);
+        if (elect_one()) {
+          const uint64_t a_desc = a_base_desc + s * (kGStageBytes >> 4), b_desc = b_base_desc + c * (x_slab >> 4);
 #pragma unroll
           for (int j = 0; j < 4; ++j) {  // K = 32 per instruction: 32 k-rows of A (4 KB), 32 bytes along B's rows
-            const uint64_t a_desc = desc_mnmajor_sw128(a_base + s * kGStageBytes + j * 4096, 16, 1024);
-            mma_i8_ss(d, a_desc, b_desc + 2 * j, idesc, (c | j) != 0 ? 1u : 0u);
+            mma_i8_ss(d, a_desc + j * (4096 >> 4), b_desc + 2 * j, idesc, (c | j) != 0 ? 1u : 0u);
           }
           tc_commit(smem_u32(&ctl->empty[s]));
+          if (c + 1 == chunks) tc_commit(smem_u32(&ctl->acc_full[acc]));
         }
-        if (!ok) break;
-        tc_commit(smem_u32(&ctl->acc_full[acc]));
+        __syncwarp();
+        if (++s == n_stages) {
+          s = 0;
+          phase ^= 1;
+        }
       }
-      if (!ok) {
-        ctl->abort = 1;
-        set_status(p.status, PTO_ST_WAIT_EXPIRED, blockIdx.x, 71);
-      }
+    }
+    if (!ok && lane == 0) {
+      ctl->abort = 1;
+      set_status(p.status, PTO_ST_WAIT_EXPIRED, blockIdx.x, 71);
     }
   } else {
     // ---------------- epilogue: accumulator -> int32 rows ----------------

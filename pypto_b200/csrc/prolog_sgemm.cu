@@ -175,41 +175,42 @@ prolog_sgemm_kernel(const __grid_constant__ PrologWMaps maps_w, const __grid_con
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      const uint32_t idesc = umma_idesc(kCFmtF32, kABFmtBF16, kABFmtBF16, 1, 0, kSTileN, static_cast<uint32_t>(p.t_pad));
-      bool ok = true;
-      uint32_t it = 0, ti = 0;
-      for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++ti) {
-        const SItem w = s_item(p, item);
-        const int kn = min(p.per_split, p.chunks - w.split * p.per_split);
-        const uint32_t acc = ti & 1;
-        if (ti >= 2) {
-          ok = mbar_wait(smem_u32(&ctl->acc_empty[acc]), ((ti >> 1) - 1) & 1);
-          if (!ok) break;
-        }
+    // (converged warp, elected lane, waits that probe without blocking, no division per chunk: see prolog_gemm.cu)
+    const uint32_t idesc = umma_idesc(kCFmtF32, kABFmtBF16, kABFmtBF16, 1, 0, kSTileN, static_cast<uint32_t>(p.t_pad));
+    bool ok = true;
+    uint32_t s = 0, phase = 0, ti = 0;
+    const uint64_t a_base_desc = desc_mnmajor_sw128(base, kSWBytes / 2, 1024), b_base_desc = umma_desc_kmajor_sw128(base + kSWBytes);
+    for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++ti) {
+      const SItem w = s_item(p, item);
+      const int kn = min(p.per_split, p.chunks - w.split * p.per_split);
+      const uint32_t acc = ti & 1;
+      if (ti >= 2) ok = mbar_wait_warp(smem_u32(&ctl->acc_empty[acc]), ((ti >> 1) - 1) & 1);
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t d = tmem_base + acc * static_cast<uint32_t>(p.t_pad);
+      for (int c = 0; c < kn; ++c) {
+        ok = mbar_wait_warp(smem_u32(&ctl->full[s]), phase);
+        if (!ok) break;
         tc_fence_after();
-        const uint32_t d = tmem_base + acc * static_cast<uint32_t>(p.t_pad);
-        for (int c = 0; c < kn; ++c, ++it) {
-          const uint32_t s = it % p.n_stages;
-          ok = mbar_wait(smem_u32(&ctl->full[s]), (it / p.n_stages) & 1);
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t a = base + s * p.stage_bytes;
-          const uint64_t b_desc = umma_desc_kmajor_sw128(a + kSWBytes);
+        if (elect_one()) {
+          const uint64_t at = s * (p.stage_bytes >> 4);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            // K = 16: 16 k-rows of each 64-column half (2 KB), the halves 8 KB apart
-            mma_f16_ss(d, desc_mnmajor_sw128(a + j * 2048, kSWBytes / 2, 1024), b_desc + 2 * j, idesc, (c | j) != 0 ? 1u : 0u);
+          for (int j = 0; j < 4; ++j) {  // K = 16: 16 k-rows of each 64-column half (2 KB), the halves 8 KB apart
+            mma_f16_ss(d, a_base_desc + at + j * (2048 >> 4), b_base_desc + at + 2 * j, idesc, (c | j) != 0 ? 1u : 0u);
           }
           tc_commit(smem_u32(&ctl->empty[s]));
+          if (c + 1 == kn) tc_commit(smem_u32(&ctl->acc_full[acc]));
         }
-        if (!ok) break;
-        tc_commit(smem_u32(&ctl->acc_full[acc]));
+        __syncwarp();
+        if (++s == static_cast<uint32_t>(p.n_stages)) {
+          s = 0;
+          phase ^= 1;
+        }
       }
-      if (!ok) {
-        ctl->abort = 1;
-        set_status(p.status, PTO_ST_WAIT_EXPIRED, blockIdx.x, 74);
-      }
+    }
+    if (!ok && lane == 0) {
+      ctl->abort = 1;
+      set_status(p.status, PTO_ST_WAIT_EXPIRED, blockIdx.x, 74);
     }
   } else {
     // ---------------- epilogue: accumulator rows (one weight column per lane) -> output ----------------
