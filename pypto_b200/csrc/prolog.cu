@@ -148,11 +148,13 @@ prolog_qnorm_kernel(const float* qa, int ld, int n_split, long long split_stride
 // 64 columns from col0, 16 * kSteps values of the contraction from k0. For few tokens only: the 128-row tile of the
 // tensor-memory path would be mostly empty and its set-up costs as much as the kernels here take. The instruction wants two
 // neighbours along k in one register where the matrix has two columns: a lane reads eight columns of four rows, 16 bytes each
-// (a warp: whole lines), and exchanges halves in registers; column g of tile n is column 8 g + n of the 64.
+// and exchanges halves in registers; column g of tile n is column 8 g + n of the 64. `h`: the matrix, rows
+// kPitch apart: in global memory, or where the call waits for it in shared memory (pitch kIdxPitch, conflict-free for these
+// reads), requested at once by hadamard_fetch: from L2 step by step each trip takes over a microsecond while weights stream.
 // acc[n]: of row lane / 4 (first two) and lane / 4 + 8: columns 16 (lane % 4) + n and 16 (lane % 4) + 8 + n.
 constexpr int kIdxPitch = kIdxDim + 8;  // the eight rows of a fragment fall into different banks
-template <int kSteps>
-__device__ __forceinline__ void hadamard_rows(const __nv_bfloat16* __restrict__ h, int k0, int col0, const __nv_bfloat16* rows,
+template <int kSteps, int kPitch>
+__device__ __forceinline__ void hadamard_rows(const __nv_bfloat16* h, int k0, int col0, const __nv_bfloat16* rows,
                                               int lane, float (&acc)[8][4]) {
   const int g = lane >> 2, l4 = lane & 3;
 #pragma unroll
@@ -163,9 +165,9 @@ __device__ __forceinline__ void hadamard_rows(const __nv_bfloat16* __restrict__ 
     uint32_t b[2][8];
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
-      const __nv_bfloat16* src = h + (k + half * 8 + 2 * l4) * kIdxDim + col0 + 8 * g;
-      const uint4 even = __ldg(reinterpret_cast<const uint4*>(src));
-      const uint4 odd = __ldg(reinterpret_cast<const uint4*>(src + kIdxDim));
+      const __nv_bfloat16* src = h + (k + half * 8 + 2 * l4) * kPitch + col0 + 8 * g;
+      const uint4 even = *reinterpret_cast<const uint4*>(src);
+      const uint4 odd = *reinterpret_cast<const uint4*>(src + kPitch);
       const uint32_t e[4] = {even.x, even.y, even.z, even.w}, o[4] = {odd.x, odd.y, odd.z, odd.w};
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
@@ -184,6 +186,12 @@ __device__ __forceinline__ void hadamard_rows(const __nv_bfloat16* __restrict__ 
           : "+f"(acc[n][0]), "+f"(acc[n][1]), "+f"(acc[n][2]), "+f"(acc[n][3])
           : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0][n]), "r"(b[1][n]));
     }
+  }
+}
+constexpr int kHadBytes = kIdxDim * kIdxPitch * 2;  // 34 KB
+__device__ __forceinline__ void hadamard_fetch(const __nv_bfloat16* __restrict__ src, __nv_bfloat16* dst, int i, int n) {
+  for (int u = i; u < kIdxDim * kIdxDim / 8; u += n) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst + (u >> 4) * kIdxPitch + (u & 15) * 8)), "l"(src + u * 8) : "memory");
   }
 }
 // `bytes` (a multiple of 128) at `p` into L2, by `n` threads of which this one is number `i`
@@ -243,20 +251,34 @@ prolog_qb_dequant_rope_kernel(const int32_t* qb_i32, const float* q_norm_scale, 
 
 // ---- indexer query of few tokens: int32 -> bf16, rope, Hadamard rotation, per-head int8 -------------------------
 // grid = tokens, block = 256: all 64 heads; a warp rotates 16 heads x 64 columns. On a second stream beside the absorbed
-// query, with little shared memory, so that its blocks find room beside that product's CTAs. On CUDA cores with the matrix in
+// query; its blocks (53 KB) find room on the SMs that hold three of that product's 512 CTAs instead of four. On CUDA cores with the matrix in
 // shared memory (41 KB, eight heads a block) it waited for those CTAs and took 12.6 us at 64 tokens (7.9 at 3): it ended the call.
 __global__ void __launch_bounds__(256)
 prolog_idxq_kernel(const int32_t* __restrict__ qi_i32, const float* __restrict__ q_norm_scale,
                    const float* __restrict__ w_scale, const __nv_bfloat16* __restrict__ cos,
                    const __nv_bfloat16* __restrict__ sin, const __nv_bfloat16* __restrict__ hadamard_q,
                    int8_t* __restrict__ q_int8, __half* __restrict__ q_scale) {
+  extern __shared__ __align__(16) __nv_bfloat16 had[];
   __shared__ __align__(16) __nv_bfloat16 q[kIdxHeads][kIdxPitch];
   __shared__ float half_amax[2][kIdxHeads];
   const int ti = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, l4 = lane & 3;
+  hadamard_fetch(hadamard_q, had, tid, 256);
   {
     const int l = tid & 15;  // dims l, l + 16, ... of a head: a dim and its partner of the rotation are in one thread
     const float rs = q_norm_scale[ti];
-    float cs[4], sn[4];
+    float cs[4], sn[4], scale[kIdxHeads / 16][8];
+    int32_t product[kIdxHeads / 16][8];  // all requested before the first is used
+#pragma unroll
+    for (int u = 0; u < kIdxHeads / 16; ++u) {
+      const int hh = u * 16 + (tid >> 4);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const void* a = qi_i32 + (static_cast<int64_t>(ti) * kIdxHeads + hh) * kIdxDim + l + 16 * j;
+        const void* b = w_scale + hh * kIdxDim + l + 16 * j;
+        asm volatile("ld.global.b32 %0, [%1];" : "=r"(product[u][j]) : "l"(a));
+        asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(scale[u][j]) : "l"(b));
+      }
+    }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       cs[j] = ld_bf16(cos + ti * kRope + l + 16 * j);
@@ -265,12 +287,9 @@ prolog_idxq_kernel(const int32_t* __restrict__ qi_i32, const float* __restrict__
 #pragma unroll
     for (int u = 0; u < kIdxHeads / 16; ++u) {
       const int hh = u * 16 + (tid >> 4);
-      const int32_t* src = qi_i32 + (static_cast<int64_t>(ti) * kIdxHeads + hh) * kIdxDim + l;
       float v[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        v[j] = bf16_round(__fmul_rn(__fmul_rn(static_cast<float>(src[16 * j]), rs), __ldg(w_scale + hh * kIdxDim + l + 16 * j)));
-      }
+      for (int j = 0; j < 8; ++j) v[j] = bf16_round(__fmul_rn(__fmul_rn(static_cast<float>(product[u][j]), rs), scale[u][j]));
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         float o = v[j];
@@ -282,10 +301,11 @@ prolog_idxq_kernel(const int32_t* __restrict__ qi_i32, const float* __restrict__
       }
     }
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
   const int head0 = (warp >> 1) * 16, half = warp & 1;
   float acc[8][4];
-  hadamard_rows<8>(hadamard_q, 0, half * 64, &q[head0][0], lane, acc);
+  hadamard_rows<8, kIdxPitch>(had, 0, half * 64, &q[head0][0], lane, acc);
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
     float m = 0.f;
@@ -435,7 +455,7 @@ prolog_kv_kernel(const float* __restrict__ kv, const float* __restrict__ ki, con
   {
     float acc[8][4];
     const int half = warp & 1, part = warp >> 1;  // warp: 64 columns, half of the contraction
-    hadamard_rows<4>(hadamard_k, part * 64, half * 64, &krow[0][0], lane, acc);
+    hadamard_rows<4, kIdxDim>(hadamard_k, part * 64, half * 64, &krow[0][0], lane, acc);
     if (lane < 4) {
 #pragma unroll
       for (int n = 0; n < 8; ++n) {
@@ -698,7 +718,9 @@ cudaError_t launch_prolog_idxq(const int32_t* qi_i32, const float* q_norm_scale,
                                const void* sin, const void* hadamard_q, int t, int8_t* q_int8, void* q_scale,
                                cudaStream_t stream) {
   count_launch();
-  prolog_idxq_kernel<<<t, 256, 0, stream>>>(
+  cudaError_t e = cudaFuncSetAttribute(prolog_idxq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kHadBytes);
+  if (e != cudaSuccess) return e;
+  prolog_idxq_kernel<<<t, 256, kHadBytes, stream>>>(
       qi_i32, q_norm_scale, w_scale, reinterpret_cast<const __nv_bfloat16*>(cos),
       reinterpret_cast<const __nv_bfloat16*>(sin), reinterpret_cast<const __nv_bfloat16*>(hadamard_q), q_int8,
       reinterpret_cast<__half*>(q_scale));
