@@ -908,7 +908,7 @@ def main():
             roof_li.update({"bound": "tensor", "achieved": li_tops, "peak": 2 * tf_peak, "unit": "TOP/s (int8)",
                             "frac": li_tops / (2 * tf_peak),
                             "peak_source": "2 x " + tf_src + " bf16 burst peak (stated, not measured for int8)"})
-        sfa_kernel = "sfa_pair_kernel" if nq == 128 else "sfa_mma_kernel"
+        sfa_kernel = "sfa_pair_kernel" if nq == 128 else "sfa_slice_kernel"
         tensor_bound = fl_sfa / (tf_peak * 1e12) >= by_sfa / (peak * 1e9)
         roof_sfa = {"bound": "tensor" if tensor_bound else "hbm", "kernel": sfa_kernel,
                     "achieved": sfa_tfs if tensor_bound else sfa_gbs, "peak": tf_peak if tensor_bound else peak,
