@@ -386,7 +386,10 @@ int prolog_side_stream(int* device) {
   PTO_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return fail(PTO_ERR_UNSUPPORTED, "device ordinal %d out of range", dev);
   if (b.side[dev] == nullptr) {
-    PTO_CUDA(cudaStreamCreateWithFlags(&b.side[dev], cudaStreamNonBlocking));
+    int least = 0, greatest = 0;
+    PTO_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    // first in line: else its small blocks wait until every CTA of a product on the caller's stream has found room
+    PTO_CUDA(cudaStreamCreateWithPriority(&b.side[dev], cudaStreamNonBlocking, greatest));
     for (int i = 0; i < 3; ++i) PTO_CUDA(cudaEventCreateWithFlags(&b.ev[dev][i], cudaEventDisableTiming));
   }
   *device = dev;

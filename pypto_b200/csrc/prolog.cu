@@ -145,7 +145,7 @@ prolog_qnorm_kernel(const float* qa, int ld, int n_split, long long split_stride
 }
 
 // Hadamard rotation of 16 rows (bf16, row pitch kIdxPitch, shared memory) by the warps' own matrix instruction (m16n8k16):
-// 64 columns from col0, 16 * kSteps values of the contraction from k0. For few tokens only: the 128-row tile of the
+// 64 columns from col0, 16 * kSteps values of the contraction from k0; with kOneRow only row 0 is there. For few tokens only: the 128-row tile of the
 // tensor-memory path would be mostly empty and its set-up costs as much as the kernels here take. The instruction wants two
 // neighbours along k in one register where the matrix has two columns: a lane reads eight columns of four rows, 16 bytes each
 // and exchanges halves in registers; column g of tile n is column 8 g + n of the 64. `h`: the matrix, rows
@@ -153,7 +153,7 @@ prolog_qnorm_kernel(const float* qa, int ld, int n_split, long long split_stride
 // reads), requested at once by hadamard_fetch: from L2 step by step each trip takes over a microsecond while weights stream.
 // acc[n]: of row lane / 4 (first two) and lane / 4 + 8: columns 16 (lane % 4) + n and 16 (lane % 4) + 8 + n.
 constexpr int kIdxPitch = kIdxDim + 8;  // the eight rows of a fragment fall into different banks
-template <int kSteps, int kPitch>
+template <int kSteps, int kPitch, bool kOneRow>
 __device__ __forceinline__ void hadamard_rows(const __nv_bfloat16* h, int k0, int col0, const __nv_bfloat16* rows,
                                               int lane, float (&acc)[8][4]) {
   const int g = lane >> 2, l4 = lane & 3;
@@ -178,7 +178,8 @@ __device__ __forceinline__ void hadamard_rows(const __nv_bfloat16* h, int k0, in
     uint32_t a[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      a[i] = *reinterpret_cast<const uint32_t*>(rows + (g + 8 * (i & 1)) * kIdxPitch + k + 8 * (i >> 1) + 2 * l4);
+      const uint32_t* row = reinterpret_cast<const uint32_t*>(rows + (kOneRow ? 0 : (g + 8 * (i & 1)) * kIdxPitch) + k + 8 * (i >> 1) + 2 * l4);
+      a[i] = !kOneRow || (g == 0 && (i & 1) == 0) ? *row : 0u;
     }
 #pragma unroll
     for (int n = 0; n < 8; ++n) {
@@ -210,6 +211,9 @@ prolog_qb_dequant_rope_kernel(const int32_t* qb_i32, const float* q_norm_scale, 
   // front of pdl_wait())
   __shared__ float pe[kQbHeadsPerBlock][kRope];
   const int ti = blockIdx.y, tid = threadIdx.x;
+  // (CTAs of the product behind this kernel fill their rings while the up-projections end; the other stream's kernels are
+  // first in line for what room there is)
+  if (tid == 0) pdl_trigger();
   const int hg = blockIdx.x;
   const int64_t col0 = static_cast<int64_t>(hg) * kQbHeadsPerBlock * kQHead;
   const int64_t row0 = static_cast<int64_t>(ti) * kHeads * kQHead;
@@ -220,8 +224,6 @@ prolog_qb_dequant_rope_kernel(const int32_t* qb_i32, const float* q_norm_scale, 
   const int c = tid % kRope;
   const float cs = ld_bf16(cos + ti * kRope + c), sn = ld_bf16(sin + ti * kRope + c);
   pdl_wait();
-  // not before: CTAs of the product behind this kernel would take the room that the per-token kernel's blocks need
-  if (tid == 0) pdl_trigger();
   const float rs = q_norm_scale[ti];
   int32_t product[kQbHeadsPerBlock * kQHead / 256];
 #pragma unroll
@@ -305,7 +307,7 @@ prolog_idxq_kernel(const int32_t* __restrict__ qi_i32, const float* __restrict__
   __syncthreads();
   const int head0 = (warp >> 1) * 16, half = warp & 1;
   float acc[8][4];
-  hadamard_rows<8, kIdxPitch>(had, 0, half * 64, &q[head0][0], lane, acc);
+  hadamard_rows<8, kIdxPitch, false>(had, 0, half * 64, &q[head0][0], lane, acc);
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
     float m = 0.f;
@@ -358,7 +360,7 @@ prolog_kv_kernel(const float* __restrict__ kv, const float* __restrict__ ki, con
   __shared__ float red[32];
   __shared__ float pe[kRope];
   __shared__ float kvec[kIdxDim];
-  __shared__ __align__(16) __nv_bfloat16 krow[16][kIdxPitch];  // the rotation's operand: row 0; what the others give is not read
+  __shared__ __align__(16) __nv_bfloat16 krow[kIdxDim];  // the rotation's operand
   __shared__ float kpart[2][kIdxDim];
   const int ti = blockIdx.x, i = threadIdx.x, lane = i & 31, warp = i >> 5;
   prefetch_l2(hadamard_k, 2 * kIdxDim * kIdxDim, i, 128);
@@ -448,14 +450,12 @@ prolog_kv_kernel(const float* __restrict__ kv, const float* __restrict__ ki, con
     const float rot = i < 32 ? -kvec[i + 32] : kvec[i - 32];
     k = bf16_round(__fadd_rn(__fmul_rn(k, cs), __fmul_rn(rot, sn)));
   }
-  krow[0][i] = __float2bfloat16_rn(k);
-#pragma unroll
-  for (int r = 1; r < 16; ++r) krow[r][i] = __float2bfloat16_rn(0.f);
+  krow[i] = __float2bfloat16_rn(k);
   __syncthreads();  // (and kvec has been read)
   {
     float acc[8][4];
     const int half = warp & 1, part = warp >> 1;  // warp: 64 columns, half of the contraction
-    hadamard_rows<4, kIdxDim>(hadamard_k, part * 64, half * 64, &krow[0][0], lane, acc);
+    hadamard_rows<4, kIdxDim, true>(hadamard_k, part * 64, half * 64, krow, lane, acc);
     if (lane < 4) {
 #pragma unroll
       for (int n = 0; n < 8; ++n) {
