@@ -140,11 +140,11 @@ size_t li_scores_bytes(int t, int max_blocks, int block_size) {
 
 int sfa_split(int t, int nq) {
   if (nq == 128) return pto::sfa_pair_split(t, 148);  // one cluster of two CTAs per (token, split)
-  const int n_hb = nq / pto::sfa_slice_heads();
+  const int n_hb = nq / pto::sfa_slice_heads(nq);
   const long long ctas = static_cast<long long>(t) * n_hb;
   if (ctas >= 148) return 1;
   long long s = 148 / (ctas > 0 ? ctas : 1);
-  if (s > 16) s = 16;  // (2048 selected rows are 16 tiles)
+  if (s > 32) s = 32;
   if (s < 1) s = 1;
   return static_cast<int>(s);
 }

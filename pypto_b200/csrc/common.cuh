@@ -351,7 +351,7 @@ cudaError_t launch_sfa(const SfaParams& p, int num_sms, cudaStream_t stream);
 cudaError_t launch_sfa_pair(const SfaParams& p, cudaStream_t stream);     // nq == 128, any cache format: 2-SM MMAs, heads split over the pair
 int sfa_pair_split(int t, int num_sms);
 cudaError_t launch_sfa_slice(const SfaParams& p, int num_sms, cudaStream_t stream);  // other head counts, int8 caches
-int sfa_slice_heads();  // heads per work item of that kernel
+int sfa_slice_heads(int nq);  // heads per work item of that kernel
 
 // Launch with the programmatic-serialization attribute when `pdl`: the grid may be scheduled while the kernel
 // before it in the stream drains, and must execute pdl_wait() before it touches global memory that kernel wrote.

@@ -95,7 +95,7 @@ sfa_combine_kernel(SfaParams p, int rows) {
 cudaError_t launch_sfa(const SfaParams& p, int num_sms, cudaStream_t stream) {
   const int t = p.b * p.s1;
   // all 128 heads of a token: a pair of SMs that shares every MMA (sfa_pair.cu; int8, packed and bf16 caches); other
-  // head counts: one SM per token and block of 16 heads, the rows as the M dimension (sfa_slice.cu)
+  // head counts: one SM per token and block of 16 or 32 heads, the rows as the M dimension (sfa_slice.cu)
   cudaError_t e = p.nq == 128 ? launch_sfa_pair(p, stream) : launch_sfa_slice(p, num_sms, stream);
   if (e != cudaSuccess) return e;
   if (p.n_split > 1) {

@@ -1,34 +1,32 @@
 // Sparse MLA attention for a slice of a token's heads (16 .. 112, a device's share of a head-sharded call), on
-// tcgen05 with the operands swapped and the latent rows left as they are: int8.
+// tcgen05 with the operands swapped: the selected rows are the M dimension of both products, the heads their N.
 //
 // Arithmetic as in sfa_pair.cu (reference: examples/models/deepseek_v32_exp/sparse_flash_attention_quant_impl.py:45-207;
 // golden deepseekv32_sparse_flash_attention_quant.py:169-254; packed rows sparse_attention_antiquant_impl.py:45-243):
-//   S^T[key, head] = K . q^T      M = 128 keys,                N = 16 heads, K = 576
-//   O^T[dim, head] = V^T . P^T    four blocks of M = 128 dims, N = 16 heads, K = 128 keys
-// With few heads a product with the heads as M would pad 16 rows to 128. Swapped, nothing is padded, and the same tile
-// [key][128-byte chunk], 128-byte swizzled, is a K-major A operand for S^T and an MN-major A operand for O^T.
+//   S^T[key, head] = K . q^T      M = 128 lanes (kTK keys used), N = kHB heads, K = 576
+//   O^T[dim, head] = V^T . P^T    four blocks of M = 128 dims,   N = kHB heads, K = kTK keys
+// With few heads a product with the heads as M would pad 16 rows to 128 (the mma.sync kernel this one replaced padded
+// them to 64 and took 6.53 ms for 4096 tokens x 2048 rows x 16 heads). Swapped, nothing is padded but the lanes above
+// kTK of the score product, and a row is converted ONCE: the bf16 tile [key][64-dim chunk of 128 bytes], 128-byte
+// swizzled, is a K-major A operand for S^T and, the same bytes, an MN-major A operand for O^T.
 //
-// The latent part is multiplied as int8 (kind::i8, exact): the gathered bytes go straight from L2 to the operand tile, no
-// conversion stands between. A chunk is one 128-dim tile with its scale, so the scale of a (row, tile) is applied where
-// there are few values: to the four partial scores of the row, and, for O^T, to the probabilities of block c.
-//   q          per head a fixed-point number of 14 bits and sign below the head's largest |q| (a power of two), as two int8
-//              limbs: columns 0-15 and 16-31 of the product, combined in int32. bf16 values down to 2^-6 of the largest are
-//              exact, smaller ones are off by at most 2^-14 of it; the bf16 rounding of the dequantised keys (2^-9 of every
-//              term) that other forms of this product carry is not there.
-//   p scale_c  per tile and chunk a fixed-point number below twice the tile's largest |scale_c|, again as two limbs (the
-//              reference maximum of a head follows its scores within a factor of two): 2^-14 of the largest, against 2^-9
-//              of each value when the scaled probabilities are bf16.
-//   rope part  bf16 x bf16 -> fp32 as before.
-// The int32 results of a tile's O^T are added to fp32 accumulators in registers with the tile's factor.
+// The latent bytes are converted without their scale: an int8 is exact in bf16. The scale of a (row, 128-dim tile) is
+// applied where there are few values: to the four partial scores of the row's tiles (one accumulator per tile, the rope
+// part a fifth), and, for O^T, whose four M blocks are those same tiles, to the probabilities: block c multiplies
+// bf16(p * scale_c). One rounding per (row, tile, head) instead of one per value and one per probability.
 //
-// Persistent CTAs, one per SM, walk (token, block of 16 heads, split) items; tiles of 128 rows alternate between two
-// buffers and run on across items; the query tile is double-buffered too.
+// Persistent CTAs, one per SM, walk (token, head block, split) items; tiles of kTK rows alternate between two buffers
+// and run on across items, so that only the query tile and the output are handed over at an item's end.
 //   warp 0          issues the score MMAs of a tile        warp 1   issues the value MMAs of a tile
-//   warps 2..3      query tile of the next item            warps 4..11  softmax (TMEM lane = key, eight heads per warp)
-//   warps 12..15    output (TMEM lane = dim)               warps 16..23 producers, 16 rows of a tile each (cp.async)
-// What bounds it: the issue of 36 MMAs of 39 cycles per 128 rows (N = 32: any smaller shape costs as much) and the softmax
-// warps' instruction stream beside it. History at 4096 tokens x 2048 rows x 16 heads: mma.sync with 64-row tiles 6.53
-// ms; swapped, rows converted to bf16 by the producers (5.6 k cycles per 80 rows) 2.10 ms.
+//   warps 2..3      query tile of the next item (cp.async) warps 4..7  softmax and output (TMEM lane = key / dim)
+//   warps 8..       producers, four rows of a tile each: gather, int8 -> bf16, swizzled stores
+// What bounds it: the producers. 4096 tokens x 2048 rows x 16 heads take 2.1 ms, i.e. 5.6 k cycles per tile of 80 rows, of
+// which the MMAs are 2184: one with N = 16 takes 39 cycles (4.5 KB of operands at 128 bytes per cycle; measured in
+// isolation), and there are 36 + 4 kTK/16 of them.
+// Why bf16: a form that multiplied the rows as int8, queries and probabilities as fixed-point limbs, took 1.24 ms, but a
+// fixed-point probability has an absolute error: beside a row with 0.96 of the weight the others rounded to zero (rel-L2
+// against 64 bits 0.22, 16 heads; this form 0.0020, the mma.sync kernel before it 0.0024).
+// kTK: as many rows as leave room for two tile buffers (80 with 16 heads, 64 with 32).
 // All waits are bounded.
 #include "common.cuh"
 #include "sfa_common.cuh"
@@ -37,76 +35,70 @@ namespace pto {
 
 namespace {
 
-constexpr int kSHeads = 16;                  // heads per work item
-constexpr int kSRows = 128;                  // selected rows per tile
-constexpr int kSChunk = kSRows * 128;        // 128 rows x 128 bytes: one dim tile of int8, or the bf16 rope part
-constexpr int kSTile = 5 * kSChunk;          // chunks 0-3 latent, chunk 4 rope
-constexpr int kSQChunk = 2 * kSHeads * 128;  // two limbs of 16 heads x 128 dims
-constexpr int kSQRope = kSHeads * 128;
-constexpr int kSQ = 4 * kSQChunk + kSQRope;
-constexpr int kSPBlock = kSRows * 2 * kSHeads;  // P^T of one dim tile: per key 16 high and 16 low limbs
-constexpr int kSSmemTile = 0;
-constexpr int kSSmemQ = 2 * kSTile;
-constexpr int kSSmemP = kSSmemQ + 2 * kSQ;
-constexpr int kSSmemCtl = kSSmemP + 4 * kSPBlock;
-constexpr int kSSoftWarp0 = 4, kSSoftWarps = 8, kSOutWarp0 = 12, kSProdWarp0 = 16, kSProdWarps = 8;
-constexpr int kSThreads = 32 * (kSProdWarp0 + kSProdWarps);
-constexpr uint32_t kSTmemCols = 512;
-constexpr uint32_t kSColS = 0, kSSBuf = 4 * 2 * kSHeads + kSHeads;  // S buffer b: four blocks of two limbs, then the rope part
-constexpr uint32_t kSColO = 2 * kSSBuf;                             // O block c at kSColO + 32 c
-static_assert(kSColO + 4 * 2 * kSHeads <= kSTmemCols, "tensor memory");
-// registers per thread: at launch, and after the split (six groups of four warps)
-constexpr int kSRegIssue = 56, kSRegSoft = 96, kSRegOut = 120, kSRegProd = 56, kSRegLaunch = 80;
-static_assert(kSRegIssue + 2 * kSRegSoft + kSRegOut + 2 * kSRegProd <= 6 * kSRegLaunch, "register split");
-constexpr float kSRescale = 1.0f;   // log2 units a score may exceed its head's reference: p <= 2
-constexpr float kSPUnit = 8191.0f;  // fixed-point units of p = 1: 2 * 8191 fits 7 + 7 bits
+constexpr int kSliceChunks = 9;  // 8 latent chunks of 64 dims + the rope chunk
 
+template <int kHB, int kTK>
+struct SliceCfg {
+  static constexpr int kChunk = kTK * 128;                  // kTK rows x 64 bf16
+  static constexpr int kTile = kSliceChunks * kChunk;
+  static constexpr int kQChunk = kHB * 128;
+  static constexpr int kPBytes = kTK * kHB * 2;             // one scaled copy of P^T
+  static constexpr int kSmemTile = 0;
+  static constexpr int kSmemQ = 2 * kTile;
+  static constexpr int kSmemP = kSmemQ + kSliceChunks * kQChunk;  // [buffer][tile c]
+  static constexpr int kSmemCtl = kSmemP + 2 * 4 * kPBytes;
+  static constexpr int kProdWarps = kTK / 4;
+  static constexpr int kThreads = 32 * (8 + kProdWarps);
+  static constexpr uint32_t kColS = 0;                      // S buffer b, accumulator c at (b * 5 + c) * kHB
+  static constexpr uint32_t kColO = 2 * 5 * kHB;            // O block c at kColO + c * kHB
+  static constexpr uint32_t kTmemCols = kHB == 16 ? 256 : 512;
+  static_assert(kColO + 4 * kHB <= kTmemCols, "tensor memory");
+  // registers per thread: at launch, issuers / loaders, softmax, producers
+  static constexpr int kRegLaunch = kHB == 16 ? 72 : 80;
+  static constexpr int kRegIssue = 40, kRegSoftmax = kHB == 16 ? 128 : 152, kRegProd = 64;
+  static_assert(128 * kRegIssue + 128 * kRegSoftmax + 32 * kProdWarps * kRegProd <= kThreads * kRegLaunch, "register split");
+};
+
+template <int kHB, int kTK>
 struct SliceCtl {
-  __align__(16) float scales[2][kSRows][4];  // the tile's row scales
-  float live[2][kSRows];                     // 1: a row to attend to, 0: padding or rejected
-  __align__(16) float smax[2][4][4];         // [tile parity][lane quarter][c]: largest |scale_c|
-  __align__(16) float fac[2][4];             // [tile parity][c]: value of a unit of the tile's O^T
-  __align__(16) float alpha[2][kSHeads];     // [tile parity]: factor for what was summed before
-  int rescale[2];
-  __align__(16) float mref[kSHeads];         // reference maximum of a head (log2 units)
-  __align__(16) float red[4][kSHeads];
-  __align__(16) float linv[2][kSHeads];      // [item parity]
-  __align__(16) float qunit[4][kSHeads];     // [item % 4]: value of a unit of the head's query limbs
-  uint64_t full[2];   // rows of the tile landed                     (8 producer warps)
-  uint64_t done[2];   // O^T of the tile complete: tile buffer and P free (commit)
+  __align__(16) float scales[2][kTK][4];  // the tile's row scales
+  float live[2][kTK];                     // 1: a row to attend to, 0: padding or rejected
+  __align__(16) float mref[kHB];          // reference maximum of a head (log2 units)
+  __align__(16) float alpha[kHB];
+  float red[4][kHB];
+  uint64_t full[2];   // producers filled the tile buffer            (producer warps)
+  uint64_t done[2];   // P.V of the tile complete: tile buffer and P buffer free, O at rest (commit)
   uint64_t sfull[2];  // scores of the tile complete                 (commit)
-  uint64_t sfree[2];  // scores read                                 (8 softmax warps)
-  uint64_t pfull;     // P^T of the tile written                     (8 softmax warps)
-  uint64_t ofree;     // O^T of the tile read                        (4 output warps)
-  uint64_t qfull[2];  // query tile of the item written              (2 query warps)
-  uint64_t qfree[2];  // last score product of the item complete     (commit)
-  uint64_t lfull[2];  // row sums of the item known                  (8 softmax warps)
+  uint64_t sfree[2];  // scores read                                 (4 softmax warps)
+  uint64_t pfull[2];  // P^T of the tile written                     (4 softmax warps)
+  uint64_t qfull;     // query tile of the item loaded               (2 loader warps)
+  uint64_t qfree;     // last score product of the item complete     (commit)
+  uint64_t ofree;     // output of the item read from tensor memory  (4 softmax warps)
   uint32_t tmem_base;
   int abort;
 };
-static_assert(kSSmemCtl + sizeof(SliceCtl) <= 232448, "exceeds the 227 KB of shared memory a CTA may use");
-constexpr size_t kSSmemBytes = kSSmemCtl + sizeof(SliceCtl);
 
 // what a role needs to know of a work item
 struct SliceItem {
   int ti, bi, sp, head0, begin, end, ntiles;
 };
 
-__device__ __forceinline__ SliceItem slice_item(const SfaParams& p, int item) {
+template <int kTK>
+__device__ __forceinline__ SliceItem slice_item(const SfaParams& p, int hb_heads, int item) {
   SliceItem it;
-  const int n_hb = p.nq / kSHeads;
+  const int n_hb = (p.nq + hb_heads - 1) / hb_heads;
   it.sp = item % p.n_split;
   item /= p.n_split;
-  it.head0 = (item % n_hb) * kSHeads;
+  it.head0 = (item % n_hb) * hb_heads;
   it.ti = item / n_hb;
   it.bi = it.ti / p.s1;
   int n = __ldg(p.act_seq + it.bi) - p.s1 + 1 + it.ti % p.s1;
   n = max(0, min(n, p.topk_k));
-  const int tiles_total = (n + kSRows - 1) / kSRows;
+  const int tiles_total = (n + kTK - 1) / kTK;
   const int tiles_per_split = (tiles_total + p.n_split - 1) / p.n_split;
-  it.begin = min(n, it.sp * tiles_per_split * kSRows);
-  it.end = min(n, (it.sp + 1) * tiles_per_split * kSRows);
-  it.ntiles = (it.end - it.begin + kSRows - 1) / kSRows;
+  it.begin = min(n, it.sp * tiles_per_split * kTK);
+  it.end = min(n, (it.sp + 1) * tiles_per_split * kTK);
+  it.ntiles = (it.end - it.begin + kTK - 1) / kTK;
   return it;
 }
 
@@ -119,49 +111,57 @@ __device__ __forceinline__ bool slice_wait(uint32_t bar, uint32_t parity) {  // 
   }
 }
 
-// MN-major B operand of 32 int8 columns: keys of 32 bytes, 32-byte swizzle, eight keys per atom
+// MN-major B operand of kHB = 16 / 32 heads: rows (keys) of 32 / 64 bytes, 32- / 64-byte swizzle, eight rows per atom
+template <int kHB>
 __device__ __forceinline__ uint64_t slice_desc_p(uint32_t smem_addr) {
+  constexpr uint32_t row = kHB * 2;
   uint64_t d = 0;
   d |= static_cast<uint64_t>((smem_addr & 0x3FFFFu) >> 4);
-  d |= static_cast<uint64_t>(1) << 16;           // one group along the columns
-  d |= static_cast<uint64_t>(256 >> 4) << 32;    // eight keys
+  d |= static_cast<uint64_t>(1) << 16;                 // one group along the heads
+  d |= static_cast<uint64_t>((8 * row) >> 4) << 32;    // eight keys
   d |= static_cast<uint64_t>(1) << 46;
-  d |= static_cast<uint64_t>(6) << 61;           // SWIZZLE_32B
+  d |= static_cast<uint64_t>(kHB == 16 ? 6 : 4) << 61;  // SWIZZLE_32B / SWIZZLE_64B
   return d;
 }
 
-__device__ __forceinline__ void tmem_ld_32x32b_x8(uint32_t taddr, uint32_t (&r)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "r"(taddr)
-               : "memory");
+// four int8 -> two bf16 pairs, exact. With the byte b in the low half of a bf16 0x43bb, bits 0-6 are the integers 128 + (b &
+// 127) (exponent 2^7, one unit per mantissa step) and bit 7 alone is 128 or 256; their difference is the signed byte.
+__device__ __forceinline__ uint2 slice_cvt4(uint32_t w) {
+  uint2 o;
+  const uint32_t a = __byte_perm(w, 0x43434343u, 0x4140), b = __byte_perm(w, 0x43434343u, 0x4342);
+  asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(o.x) : "r"(a & 0xff7fff7fu), "r"(a & 0xff80ff80u));
+  asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(o.y) : "r"(b & 0xff7fff7fu), "r"(b & 0xff80ff80u));
+  return o;
 }
 
 // ================================ producers =====================================================
-// Warp w owns rows 16w .. 16w+15 of every tile. Nothing passes through registers: an instruction copies one row's 512 latent
-// bytes (or four rows' rope parts) from L2 to their swizzled places. The copies of a tile are issued when its buffer
-// is free and waited for at the next tile, before that tile's buffer is. Lane r % 16 walks the look-ahead chain of row
-// 16w + r: selected index three tiles ahead of the copies, block-table entry two, L2 prefetch one.
-template <bool kPacked>
-__device__ __forceinline__ void slice_role_producer(const SfaParams& p, SliceCtl* ctl, uint32_t base, int n_items) {
-  const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) - kSProdWarp0;
-  const int r = lane & 15;
+// Warp w owns rows 4w .. 4w+3 of every tile. A gather instruction reads half the latent bytes of two rows (four whole
+// 128-byte lines); the eight lanes of a quarter-warp hold four 16-byte units of two neighbouring rows, whose swizzle
+// terms differ in the lowest bit, so their stores hit eight different bank groups. Lane r % 4 walks the look-ahead chain
+// of row 4w + r: selected index three tiles ahead, block-table entry two, L2 prefetch of the row two, the row itself
+// one tile ahead (into registers, as soon as the tile before it is converted). The chain runs on across items.
+template <int kHB, int kTK, bool kPacked>
+__device__ __forceinline__ void slice_role_producer(const SfaParams& p, SliceCtl<kHB, kTK>* ctl, uint32_t base, int n_items) {
+  using Cfg = SliceCfg<kHB, kTK>;
+  const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) - 8;
+  const int r = lane & 3, rsel = (lane >> 2) & 1;
+  const int src_off = (((lane & 3) | ((lane >> 3) << 2)) << 4);  // this lane's 16 bytes of a half row
   const uint8_t* const kn = reinterpret_cast<const uint8_t*>(p.kn);
   const uint8_t* const kr = kPacked ? kn + 512 : reinterpret_cast<const uint8_t*>(p.kr);
   const uint8_t* const ks = kPacked ? kn + 640 : reinterpret_cast<const uint8_t*>(p.kn_scales);
   constexpr int stride_n = kPacked ? 656 : 512, stride_r = kPacked ? 656 : 128, stride_s = kPacked ? 656 : 16;
 
   int cur_item = blockIdx.x, cur_j = 0;
-  SliceItem it = slice_item(p, cur_item);
+  SliceItem it = slice_item<kTK>(p, kHB, cur_item);
   // index of this lane's row in the next tile of this CTA (false: no further tile; the same answer in every lane)
   auto fetch = [&](int& idx, int& bi) -> bool {
     while (cur_j >= it.ntiles) {
       cur_item += gridDim.x;
       if (cur_item >= n_items) return false;
-      it = slice_item(p, cur_item);
+      it = slice_item<kTK>(p, kHB, cur_item);
       cur_j = 0;
     }
-    const int pos = it.begin + cur_j * kSRows + 16 * w + r;
+    const int pos = it.begin + cur_j * kTK + 4 * w + r;
     idx = pos < it.end ? ldg_pinned_i32(p.topk + static_cast<int64_t>(it.ti) * p.topk_k + pos) : -1;
     bi = it.bi;
     ++cur_j;
@@ -170,84 +170,100 @@ __device__ __forceinline__ void slice_role_producer(const SfaParams& p, SliceCtl
   auto row_of = [&](int idx, int entry) -> int {  // 32 bits: the host side refuses caches of 2^31 rows or more
     return static_cast<int>(tc_row_from_entry(p, idx, entry));
   };
-  auto prefetch_row = [&](int phys) {  // two lanes per row
+  uint4 d[2][2];  // [row pair][half]: this lane's 16 bytes of row 2 pair + rsel
+  uint4 rope;     // unit lane % 8 of row lane / 8
+  float4 sc;      // the four scales of row r
+  int row_loaded = -1;
+  // a padding or rejected row reads row 0; it is masked out of the softmax (`live`), its rope part is zeroed
+  auto issue_loads = [&](int phys) {
+    row_loaded = phys;
+#pragma unroll
+    for (int pr = 0; pr < 2; ++pr) {
+      const int pm = max(__shfl_sync(0xffffffffu, phys, 2 * pr + rsel), 0);
+      const uint8_t* src = kn + static_cast<int64_t>(pm) * stride_n + src_off;
+      d[pr][0] = ldg_pinned_v4(src);
+      d[pr][1] = ldg_pinned_v4(src + 256);
+    }
+    const int px = __shfl_sync(0xffffffffu, phys, lane >> 3);
+    rope = make_uint4(0, 0, 0, 0);
+    if (px >= 0) rope = ldg_pinned_v4(kr + static_cast<int64_t>(px) * stride_r + (lane & 7) * 16);
+    uint4 s4 = make_uint4(0, 0, 0, 0);
+    if (phys >= 0) s4 = ldg_pinned_v4(ks + static_cast<int64_t>(phys) * stride_s);
+    sc = make_float4(__uint_as_float(s4.x), __uint_as_float(s4.y), __uint_as_float(s4.z), __uint_as_float(s4.w));
+  };
+  auto prefetch_row = [&](int phys) {  // lanes r, r+4, ...: one line of the row each
     if (phys < 0) return;
+    const int l = lane >> 2;
     if (kPacked) {
-      if (lane < 16) bulk_prefetch_l2(kn + static_cast<int64_t>(phys) * 656, 656);
+      if (l < 6) asm volatile("prefetch.global.L2 [%0];" ::"l"(kn + static_cast<int64_t>(phys) * 656 + min(l * 128, 640)));
     } else {
-      const uint8_t* a = kn + static_cast<int64_t>(phys) * 512 + (lane >> 4) * 256;
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(a));
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(a + 128));
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(lane < 16 ? kr + static_cast<int64_t>(phys) * 128 : ks + static_cast<int64_t>(phys) * 16));
+      if (l < 4) asm volatile("prefetch.global.L2 [%0];" ::"l"(kn + static_cast<int64_t>(phys) * 512 + l * 128));
+      else if (l == 4) asm volatile("prefetch.global.L2 [%0];" ::"l"(kr + static_cast<int64_t>(phys) * 128));
+      else if (l == 5) asm volatile("prefetch.global.L2 [%0];" ::"l"(ks + static_cast<int64_t>(phys) * 16));
     }
   };
 
-  int idx_n = -1, bi_n = 0, idx_a = -1, bi_a = 0, entry_n = kTableSkip, row = -1;
-  bool has, has_n = false, has_a = false;
+  int idx_n = -1, bi_n = 0, idx_a = -1, bi_a = 0, entry_a = kTableSkip, row_n = -1;
+  bool has = false, has_n = false, has_a = false;
   {
     int idx0 = -1, bi0 = 0;
     has = fetch(idx0, bi0);
     has_n = has && fetch(idx_n, bi_n);
     has_a = has_n && fetch(idx_a, bi_a);
     const int e0 = has ? tc_table_entry(p, bi0, idx0) : kTableSkip;
-    if (has_n) entry_n = tc_table_entry(p, bi_n, idx_n);
-    if (has) row = row_of(idx0, e0);
-  }
-  bool ok = true;
-  uint32_t t = 0;
-  for (; has; ++t) {
-    const uint32_t b = t & 1;
-    int idx_b = -1, bi_b = 0;
-    const bool has_b = has_a && fetch(idx_b, bi_b);
-    // the tile after this one: into L2
-    int row_n = -1;
+    const int e1 = has_n ? tc_table_entry(p, bi_n, idx_n) : kTableSkip;
+    if (has_a) entry_a = tc_table_entry(p, bi_a, idx_a);
+    if (has) issue_loads(row_of(idx0, e0));
     if (has_n) {
-      row_n = row_of(idx_n, entry_n);
+      row_n = row_of(idx_n, e1);
       prefetch_row(row_n);
     }
-    if (t >= 1) {  // the tile before this one has had a whole step to arrive
-      asm volatile("cp.async.wait_all;" ::: "memory");
-      fence_proxy_async();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&ctl->full[b ^ 1]));
-    }
+  }
+  bool ok = true;
+  for (uint32_t t = 0; has; ++t) {
+    const uint32_t b = t & 1;
+    // the tile after the next: index (requested now, used at the end of this step) and block-table entry
+    int idx_b = -1, bi_b = 0;
+    const bool has_b = has_a && fetch(idx_b, bi_b);
     if (t >= 2) {
       ok = slice_wait(smem_u32(&ctl->done[b]), ((t >> 1) - 1) & 1);
       if (!ok) break;
     }
-    const uint32_t tile = base + kSSmemTile + b * kSTile;
+    const uint32_t tile = base + Cfg::kSmemTile + b * Cfg::kTile;
 #pragma unroll
-    for (int m = 0; m < 16; ++m) {  // row 16w + m: 32 units, eight per chunk (a padding or rejected row reads as zeros)
-      const int pm = __shfl_sync(0xffffffffu, row, m);
-      cp_async_16(tile + (lane >> 3) * kSChunk + (16 * w + m) * 128 + (((lane & 7) ^ (m & 7)) << 4),
-                  kn + (pm >= 0 ? static_cast<int64_t>(pm) * stride_n + lane * 16 : 0), pm >= 0 ? 16u : 0u);
-    }
+    for (int pr = 0; pr < 2; ++pr) {
+      const int row = 4 * w + 2 * pr + rsel, x = row & 7;
+      const uint32_t dst = tile + (lane >> 3) * Cfg::kChunk + row * 128;
+      const uint32_t a = ((2 * (lane & 3)) ^ x) << 4, c = ((2 * (lane & 3) + 1) ^ x) << 4;
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      const int x = 4 * m + (lane >> 3);
-      const int pm = __shfl_sync(0xffffffffu, row, x);
-      cp_async_16(tile + 4 * kSChunk + (16 * w + x) * 128 + (((lane & 7) ^ (x & 7)) << 4),
-                  kr + (pm >= 0 ? static_cast<int64_t>(pm) * stride_r + (lane & 7) * 16 : 0), pm >= 0 ? 16u : 0u);
+      for (int hf = 0; hf < 2; ++hf) {
+        const uint4 v = d[pr][hf];
+        const uint2 v0 = slice_cvt4(v.x), v1 = slice_cvt4(v.y), v2 = slice_cvt4(v.z), v3 = slice_cvt4(v.w);
+        sts_v4u(dst + hf * 4 * Cfg::kChunk + a, make_uint4(v0.x, v0.y, v1.x, v1.y));
+        sts_v4u(dst + hf * 4 * Cfg::kChunk + c, make_uint4(v2.x, v2.y, v3.x, v3.y));
+      }
     }
-    if (lane < 16) {
-      cp_async_16(smem_u32(&ctl->scales[b][16 * w + lane][0]), ks + (row >= 0 ? static_cast<int64_t>(row) * stride_s : 0),
-                  row >= 0 ? 16u : 0u);
-      ctl->live[b][16 * w + lane] = row >= 0 ? 1.f : 0.f;
+    {
+      const int row = 4 * w + (lane >> 3);
+      sts_v4u(tile + 8 * Cfg::kChunk + row * 128 + (((lane & 7) ^ (row & 7)) << 4), rope);
+      if (lane < 4) {
+        *reinterpret_cast<float4*>(&ctl->scales[b][4 * w + lane][0]) = sc;
+        ctl->live[b][4 * w + lane] = row_loaded >= 0 ? 1.f : 0.f;
+      }
     }
-    row = row_n;
-    has = has_n;
-    has_n = has_a;
-    idx_n = idx_a;
-    if (has_a) entry_n = tc_table_entry(p, bi_a, idx_a);
-    has_a = has_b;
-    idx_a = idx_b;
-    bi_a = bi_b;
-  }
-  asm volatile("cp.async.wait_all;" ::: "memory");
-  if (ok && t > 0) {
     fence_proxy_async();
     __syncwarp();
-    if (lane == 0) mbar_arrive(smem_u32(&ctl->full[(t - 1) & 1]));
+    if (lane == 0) mbar_arrive(smem_u32(&ctl->full[b]));
+    if (has_n) issue_loads(row_n);
+    has = has_n;
+    has_n = has_a;
+    if (has_a) {
+      row_n = row_of(idx_a, entry_a);
+      prefetch_row(row_n);
+    }
+    has_a = has_b;
+    idx_a = idx_b;
+    if (has_b) entry_a = tc_table_entry(p, bi_b, idx_b);
   }
   if (!ok && lane == 0) {
     ctl->abort = 1;
@@ -258,48 +274,49 @@ __device__ __forceinline__ void slice_role_producer(const SfaParams& p, SliceCtl
 // ================================ MMA issuers ====================================================
 // What an MMA of this size costs is its issue: measured in isolation, 51-61 cycles whatever the shape when one lane
 // issues under `if (lane == 0)`, where the descriptors are moved to uniform registers for every MMA, against 39 (N = 16)
-// when the warp stays converged and an elected lane issues. Beside two dozen busy warps, the descriptors have to be
+// when the warp stays converged and an elected lane issues. Here, beside 26 busy warps, the descriptors have to be
 // constants of the code for that (kBase, the address where a kernel without static shared memory finds its dynamic
-// part; kBase = 0 is the same code with the address in a register).
+// part; kBase = 0 is the same code with the address in a register): 2.25 -> 2.05 ms for 4096 tokens of 16 heads.
 constexpr uint32_t kSliceUsualBase = 1024;
+template <int kHB, int kTK>
 __device__ __forceinline__ void slice_issue_scores(uint32_t d, uint64_t a_desc, uint64_t b_desc) {
-  constexpr uint32_t idesc_i8 = umma_idesc(kCFmtS32, kABFmtS8, kABFmtS8, 0, 0, 128, 2 * kSHeads);
-  constexpr uint32_t idesc_bf = umma_idesc(kCFmtF32, kABFmtBF16, kABFmtBF16, 0, 0, 128, kSHeads);
+  using Cfg = SliceCfg<kHB, kTK>;
+  constexpr uint32_t idesc = umma_idesc(kCFmtF32, kABFmtBF16, kABFmtBF16, 0, 0, 128, kHB);
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
+  for (int ch = 0; ch < kSliceChunks; ++ch) {  // accumulator ch / 2: one per scale tile, the rope part the fifth
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      mma_i8_ss(d + c * 2 * kSHeads, a_desc + c * (kSChunk >> 4) + 2 * k, b_desc + c * (kSQChunk >> 4) + 2 * k, idesc_i8, k != 0 ? 1u : 0u);
+      mma_f16_ss(d + (ch >> 1) * kHB, a_desc + ch * (Cfg::kChunk >> 4) + 2 * k, b_desc + ch * (Cfg::kQChunk >> 4) + 2 * k,
+                 idesc, ((ch & 1) | k) != 0 ? 1u : 0u);
     }
   }
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    mma_f16_ss(d + 4 * 2 * kSHeads, a_desc + 4 * (kSChunk >> 4) + 2 * k, b_desc + 4 * (kSQChunk >> 4) + 2 * k, idesc_bf, k != 0 ? 1u : 0u);
-  }
 }
-__device__ __forceinline__ void slice_issue_values(uint32_t d, uint64_t a_desc, uint64_t b_desc) {
-  constexpr uint32_t idesc = umma_idesc(kCFmtS32, kABFmtS8, kABFmtS8, 1, 1, 128, 2 * kSHeads);
+template <int kHB, int kTK>
+__device__ __forceinline__ void slice_issue_values(uint32_t d, uint64_t a_desc, uint64_t b_desc, uint32_t accumulate) {
+  using Cfg = SliceCfg<kHB, kTK>;
+  constexpr uint32_t idesc = umma_idesc(kCFmtF32, kABFmtBF16, kABFmtBF16, 1, 1, 128, kHB);
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {  // 32 keys per step: 4 KB of a chunk, 1 KB of the block's P^T
-      mma_i8_ss(d + c * 2 * kSHeads, a_desc + c * (kSChunk >> 4) + k * (4096 >> 4), b_desc + c * (kSPBlock >> 4) + k * (1024 >> 4),
-                idesc, k != 0 ? 1u : 0u);
+    for (int k = 0; k < kTK / 16; ++k) {  // 16 rows per step: 2 KB of a chunk, 16 rows of the tile's copy of P^T
+      mma_f16_ss(d + c * kHB, a_desc + c * (2 * Cfg::kChunk >> 4) + k * (2048 >> 4),
+                 b_desc + c * (Cfg::kPBytes >> 4) + k * ((16 * kHB * 2) >> 4), idesc, k > 0 ? 1u : accumulate);
     }
   }
 }
 
-template <uint32_t kBase>
-__device__ __forceinline__ void slice_role_scores(const SfaParams& p, SliceCtl* ctl, uint32_t base, uint32_t tmem, int n_items) {
+template <int kHB, int kTK, uint32_t kBase>
+__device__ __forceinline__ void slice_role_scores(const SfaParams& p, SliceCtl<kHB, kTK>* ctl, uint32_t base, uint32_t tmem,
+                                                  int n_items) {
+  using Cfg = SliceCfg<kHB, kTK>;
   if (kBase != 0) base = kBase;
-  const uint64_t a_desc = umma_desc_kmajor_sw128(base + kSSmemTile), b_desc = umma_desc_kmajor_sw128(base + kSSmemQ);
+  const uint64_t a_desc = umma_desc_kmajor_sw128(base + Cfg::kSmemTile), b_desc = umma_desc_kmajor_sw128(base + Cfg::kSmemQ);
   bool ok = true;
   uint32_t t = 0, n = 0;
   for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-    const int ntiles = slice_item(p, item).ntiles;
+    const int ntiles = slice_item<kTK>(p, kHB, item).ntiles;
     if (ntiles == 0) continue;
-    const uint32_t qb = n & 1;
-    ok = slice_wait(smem_u32(&ctl->qfull[qb]), (n >> 1) & 1);
+    ok = slice_wait(smem_u32(&ctl->qfull), n & 1);
     for (int j = 0; j < ntiles && ok; ++j, ++t) {
       const uint32_t b = t & 1;
       if (t >= 2) ok = slice_wait(smem_u32(&ctl->sfree[b]), ((t >> 1) - 1) & 1);
@@ -307,9 +324,9 @@ __device__ __forceinline__ void slice_role_scores(const SfaParams& p, SliceCtl* 
       if (!ok) break;
       tc_fence_after();
       if (elect_one()) {
-        slice_issue_scores(tmem + kSColS + b * kSSBuf, a_desc + b * (kSTile >> 4), b_desc + qb * (kSQ >> 4));
+        slice_issue_scores<kHB, kTK>(tmem + Cfg::kColS + b * 5 * kHB, a_desc + b * (Cfg::kTile >> 4), b_desc);
         tc_commit(smem_u32(&ctl->sfull[b]));
-        if (j + 1 == ntiles) tc_commit(smem_u32(&ctl->qfree[qb]));
+        if (j + 1 == ntiles) tc_commit(smem_u32(&ctl->qfree));
       }
       __syncwarp();
     }
@@ -322,27 +339,32 @@ __device__ __forceinline__ void slice_role_scores(const SfaParams& p, SliceCtl* 
   __syncwarp();
 }
 
-template <uint32_t kBase>
-__device__ __forceinline__ void slice_role_values(const SfaParams& p, SliceCtl* ctl, uint32_t base, uint32_t tmem, int n_items) {
+template <int kHB, int kTK, uint32_t kBase>
+__device__ __forceinline__ void slice_role_values(const SfaParams& p, SliceCtl<kHB, kTK>* ctl, uint32_t base, uint32_t tmem,
+                                                  int n_items) {
+  using Cfg = SliceCfg<kHB, kTK>;
   if (kBase != 0) base = kBase;
-  const uint64_t a_desc = desc_mnmajor_sw128(base + kSSmemTile, 16, 1024);
-  const uint64_t b_desc = slice_desc_p(base + kSSmemP);
+  const uint64_t a_desc = desc_mnmajor_sw128(base + Cfg::kSmemTile, Cfg::kChunk, 1024);
+  const uint64_t b_desc = slice_desc_p<kHB>(base + Cfg::kSmemP);
   bool ok = true;
-  uint32_t t = 0;
+  uint32_t t = 0, n = 0;
   for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-    const int ntiles = slice_item(p, item).ntiles;
+    const int ntiles = slice_item<kTK>(p, kHB, item).ntiles;
+    if (ntiles == 0) continue;
+    if (n > 0) ok = slice_wait(smem_u32(&ctl->ofree), (n - 1) & 1);
     for (int j = 0; j < ntiles && ok; ++j, ++t) {
       const uint32_t b = t & 1;
-      ok = slice_wait(smem_u32(&ctl->pfull), t & 1);
-      if (ok && t >= 1) ok = slice_wait(smem_u32(&ctl->ofree), (t - 1) & 1);
+      ok = slice_wait(smem_u32(&ctl->pfull[b]), (t >> 1) & 1) && slice_wait(smem_u32(&ctl->full[b]), (t >> 1) & 1);
       if (!ok) break;
       tc_fence_after();
       if (elect_one()) {
-        slice_issue_values(tmem + kSColO, a_desc + b * (kSTile >> 4), b_desc);
+        slice_issue_values<kHB, kTK>(tmem + Cfg::kColO, a_desc + b * (Cfg::kTile >> 4), b_desc + b * (4 * Cfg::kPBytes >> 4),
+                                     j > 0 ? 1u : 0u);
         tc_commit(smem_u32(&ctl->done[b]));
       }
       __syncwarp();
     }
+    ++n;
   }
   if (!ok && (threadIdx.x & 31) == 0) {
     ctl->abort = 1;
@@ -352,256 +374,247 @@ __device__ __forceinline__ void slice_role_values(const SfaParams& p, SliceCtl* 
 }
 
 // ================================ query tile =====================================================
-// Two warps, eight heads each: a head's 512 latent values as fixed-point limbs (lane l holds dims 16l .. 16l+15), its rope part
-// as it is.
-__device__ __forceinline__ void slice_role_query(const SfaParams& p, SliceCtl* ctl, uint32_t base, int n_items) {
-  const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) - 2;
+template <int kHB, int kTK>
+__device__ __forceinline__ void slice_role_query(const SfaParams& p, SliceCtl<kHB, kTK>* ctl, uint32_t base, int n_items) {
+  using Cfg = SliceCfg<kHB, kTK>;
+  const int tid = threadIdx.x - 64;  // 0..63
   bool ok = true;
   uint32_t n = 0;
   for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-    const SliceItem it = slice_item(p, item);
+    const SliceItem it = slice_item<kTK>(p, kHB, item);
     if (it.ntiles == 0) continue;
-    const uint32_t qb = n & 1;
-    const int64_t row0 = static_cast<int64_t>(it.ti) * p.nq_total + p.head_begin + it.head0 + 8 * w;
-    if (n >= 2) {
-      ok = slice_wait(smem_u32(&ctl->qfree[qb]), ((n >> 1) - 1) & 1);
+    const int64_t row0 = static_cast<int64_t>(it.ti) * p.nq_total + p.head_begin + it.head0;
+    if (n > 0) {
+      // the rows are wanted in L2 by the time the previous item's last score product lets go of the buffer
+      for (int e = tid; e < kHB * 8; e += 64) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.q_nope + row0 * 512 + e * 64));
+      for (int e = tid; e < kHB; e += 64) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.q_rope + row0 * 64 + e * 64));
+      ok = slice_wait(smem_u32(&ctl->qfree), (n - 1) & 1);
       if (!ok) break;
     }
-    const uint32_t q = base + kSSmemQ + qb * kSQ;
-#pragma unroll 2
-    for (int m = 0; m < 8; ++m) {
-      const int head = 8 * w + m;
-      const uint4* src = reinterpret_cast<const uint4*>(p.q_nope + (row0 + m) * 512) + 2 * lane;
-      const uint4 v0 = __ldg(src), v1 = __ldg(src + 1);
-      const uint32_t v[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-      uint32_t mx = 0;
-#pragma unroll
-      for (int e = 0; e < 8; ++e) mx = max(mx, max((v[e] << 16) & 0x7fffffffu, v[e] & 0x7fff0000u));
-      mx = __reduce_max_sync(0xffffffffu, mx);  // bit pattern of the head's largest |q|
-      const int ex = max(-100, static_cast<int>(mx >> 23) - 127);  // 2^ex <= largest < 2^(ex + 1)
-      const float up = __int_as_float((127 + 13 - ex) << 23);
-      uint32_t hi[4], lo[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        uint32_t y[4];  // low 22 bits: the integer (two's complement)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const uint32_t word = v[2 * u + (e >> 1)];
-          const float x = __uint_as_float((e & 1) ? (word & 0xffff0000u) : (word << 16));
-          y[e] = __float_as_uint(fmaf(x, up, 12582912.0f));
-        }
-        lo[u] = __byte_perm(__byte_perm(y[0], y[1], 0x0040), __byte_perm(y[2], y[3], 0x0040), 0x5410) & 0x7f7f7f7fu;
-        hi[u] = __byte_perm(__byte_perm(y[0] << 1, y[1] << 1, 0x0051), __byte_perm(y[2] << 1, y[3] << 1, 0x0051), 0x5410);
-      }
-      // dims 16 lane ..: chunk lane / 8, unit lane % 8 of rows `head` (high limbs) and 16 + `head`
-      const uint32_t at = q + (lane >> 3) * kSQChunk + head * 128 + (((lane & 7) ^ (head & 7)) << 4);
-      sts_v4u(at, make_uint4(hi[0], hi[1], hi[2], hi[3]));
-      sts_v4u(at + kSHeads * 128, make_uint4(lo[0], lo[1], lo[2], lo[3]));
-      if (lane < 8) {
-        sts_v4u(q + 4 * kSQChunk + head * 128 + ((lane ^ (head & 7)) << 4),
-                __ldg(reinterpret_cast<const uint4*>(p.q_rope + (row0 + m) * 64) + lane));
-      }
-      // (a query that is not finite makes the head's scores, and with them its output, NaN)
-      if (lane == 0) ctl->qunit[n & 3][head] = mx >= 0x7f800000u ? __int_as_float(0x7fffffff) : __int_as_float((127 + ex - 13) << 23);
+    for (int e = tid; e < kHB * 72; e += 64) {
+      const int r = e / 72, u = e % 72;
+      cp_async_16(base + Cfg::kSmemQ + (u >> 3) * Cfg::kQChunk + r * 128 + (((u & 7) ^ (r & 7)) << 4),
+                  u < 64 ? p.q_nope + (row0 + r) * 512 + u * 8 : p.q_rope + (row0 + r) * 64 + (u - 64) * 8, 16u);
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     fence_proxy_async();
     __syncwarp();
-    if (lane == 0) mbar_arrive(smem_u32(&ctl->qfull[qb]));
+    if ((threadIdx.x & 31) == 0) mbar_arrive(smem_u32(&ctl->qfull));
     ++n;
   }
-  if (!ok && lane == 0) {
+  if (!ok && (threadIdx.x & 31) == 0) {
     ctl->abort = 1;
     set_status(p.status, PTO_ST_WAIT_EXPIRED, blockIdx.x, 93);
   }
 }
 
-// ================================ softmax ========================================================
-// Eight warps, TMEM lane = key of the tile (warp quarter q holds keys 32q .. +31); warps 4-7 take heads 0-7, warps 8-11 heads
-// 8-15. The reference maximum of a head moves only when a score exceeds it by more than a factor of two (first tile:
-// always), which one vote over the eight warps finds out; so the reduction over keys, here across lanes, is rare, and
-// the row sums stay per-thread partials until the item ends.
-__device__ __forceinline__ bool slice_vote(bool pred) {  // OR over the softmax warps; also their barrier
+// ================================ softmax and output =============================================
+// Four warps, TMEM lane = key of the tile (warp q holds keys 32q .. +31; lanes above kTK take part in the barriers only).
+// A thread has one key's scores for all kHB heads. The reference maximum of a head moves only when a score exceeds it by
+// more than 2^8 (first tile: always), which one vote over the four warps finds out; so the reduction over keys, here
+// across lanes, is rare, and the row sums stay per-thread partials until the item ends.
+constexpr float kSliceRescale = 8.0f;
+
+template <int kHB>
+__device__ __forceinline__ void slice_ld(uint32_t taddr, float (&v)[kHB]) {
+  uint32_t r[kHB];
+  if constexpr (kHB == 16) tmem_ld_32x32b_x16(taddr, r);
+  else tmem_ld_32x32b_x32(taddr, r);
+  tc_wait_ld();
+#pragma unroll
+  for (int h = 0; h < kHB; ++h) v[h] = __uint_as_float(r[h]);
+}
+
+__device__ __forceinline__ bool slice_vote(bool pred) {  // OR over the four softmax warps; also their barrier
   uint32_t any;
   asm volatile(
-      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.cta.red.or.pred q, 1, 256, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.cta.red.or.pred q, 1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
       : "=r"(any)
       : "r"(pred ? 1u : 0u)
       : "memory");
   return any != 0;
 }
-__device__ __forceinline__ void slice_meet() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+__device__ __forceinline__ void slice_meet() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
-__device__ __forceinline__ void slice_role_softmax(const SfaParams& p, SliceCtl* ctl, uint32_t base, uint32_t tmem, int n_items) {
-  const int lane = threadIdx.x & 31, quarter = (threadIdx.x >> 5) & 3, g = ((threadIdx.x >> 5) - kSSoftWarp0) >> 2;
-  const int tid = threadIdx.x - 32 * kSSoftWarp0;
-  const int key = 32 * quarter + lane, h0 = 8 * g;
+template <int kHB, int kTK>
+__device__ __forceinline__ void slice_role_softmax(const SfaParams& p, SliceCtl<kHB, kTK>* ctl, uint32_t base, uint32_t tmem,
+                                                   int n_items) {
+  using Cfg = SliceCfg<kHB, kTK>;
+  const int lane = threadIdx.x & 31, quarter = (threadIdx.x >> 5) & 3, tid = threadIdx.x - 128;
+  const int key = 32 * quarter + lane;
   const uint32_t lane_addr = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
-  // this key's 32 bytes of a block of P^T; 32-byte swizzle: unit ^= (key / 4) % 2. High limbs at unit 0, low at unit 1
-  const uint32_t p_row = base + kSSmemP + key * 32 + 8 * g;
-  const uint32_t u_hi = ((key >> 2) & 1) << 4, u_lo = u_hi ^ 16u;
   bool ok = true;
-  uint32_t t = 0, n = 0;
+  uint32_t t = 0;
   for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-    const SliceItem it = slice_item(p, item);
-    if (it.ntiles == 0) continue;
-    float l[8], qunit[8];
+    const SliceItem it = slice_item<kTK>(p, kHB, item);
+    const int64_t orow0 = static_cast<int64_t>(it.ti) * p.nq_total + p.head_begin + it.head0;
+    const int64_t prow0 = (static_cast<int64_t>(it.ti) * p.n_split + it.sp) * p.nq + it.head0;
+    if (it.ntiles == 0) {
+      if (p.n_split == 1) {
+        for (int e = tid; e < kHB * 64; e += 128) *reinterpret_cast<uint4*>(p.out + orow0 * 512 + e * 8) = make_uint4(0, 0, 0, 0);
+      } else if (tid < kHB) {
+        p.part_ml[(prow0 + tid) * 2] = -INFINITY;
+        p.part_ml[(prow0 + tid) * 2 + 1] = 0.f;
+      }
+      continue;
+    }
+    float l[kHB];
 #pragma unroll
-    for (int h = 0; h < 8; ++h) l[h] = qunit[h] = 0.f;
+    for (int h = 0; h < kHB; ++h) l[h] = 0.f;
     for (int j = 0; j < it.ntiles; ++j, ++t) {
       const uint32_t b = t & 1;
+      // (a wait that expired is voted on below, so that the four warps leave together: one that left alone would leave the
+      // others at a barrier)
       ok = ok && slice_wait(smem_u32(&ctl->sfull[b]), (t >> 1) & 1) && slice_wait(smem_u32(&ctl->full[b]), (t >> 1) & 1);
-      // (a wait that expired is voted on below, so that the eight warps leave together)
       tc_fence_after();
-      const float4 sc = *reinterpret_cast<const float4*>(&ctl->scales[b][key][0]);
-      const float scv[4] = {sc.x, sc.y, sc.z, sc.w};
-      const bool valid = ctl->live[b][key] != 0.f && it.begin + j * kSRows + key < it.end;
-      if (j == 0) {  // (before the scores are handed back: the slot is written again four items on, behind two more products)
-#pragma unroll
-        for (int h = 0; h < 8; ++h) qunit[h] = ctl->qunit[n & 3][h0 + h];
-      }
-      const uint32_t col = lane_addr + kSColS + b * kSSBuf + h0;
-      float s[8], rope[8];
-#pragma unroll
-      for (int h = 0; h < 8; ++h) s[h] = 0.f;
-#pragma unroll
-      for (int cc = 0; cc < 2; ++cc) {
-        uint32_t hi[2][8], lo[2][8], rp[8];
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          tmem_ld_32x32b_x8(col + (2 * cc + e) * 2 * kSHeads, hi[e]);
-          tmem_ld_32x32b_x8(col + (2 * cc + e) * 2 * kSHeads + kSHeads, lo[e]);
+      float s[kHB];
+      float4 sc = make_float4(0.f, 0.f, 0.f, 0.f);
+      bool valid = false;
+      if (32 * quarter < kTK) {
+        const uint32_t col = lane_addr + Cfg::kColS + b * 5 * kHB;
+        if (key < kTK) {
+          sc = *reinterpret_cast<const float4*>(&ctl->scales[b][key][0]);
+          valid = ctl->live[b][key] != 0.f && it.begin + j * kTK + key < it.end;
         }
-        if (cc == 1) tmem_ld_32x32b_x8(col + 4 * 2 * kSHeads, rp);
-        tc_wait_ld();
-        if (cc == 1) {
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(smem_u32(&ctl->sfree[b]));
+        slice_ld<kHB>(col + 4 * kHB, s);  // rope part
+        const float scv[4] = {sc.x, sc.y, sc.z, sc.w};
 #pragma unroll
-          for (int h = 0; h < 8; ++h) rope[h] = __uint_as_float(rp[h]);
-        }
+        for (int c = 0; c < 4; ++c) {
+          float x[kHB];
+          slice_ld<kHB>(col + c * kHB, x);
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-#pragma unroll
-          for (int h = 0; h < 8; ++h) {
-            const int d = static_cast<int>(hi[e][h]) * 128 + static_cast<int>(lo[e][h]);
-            s[h] = fmaf(static_cast<float>(d), scv[2 * cc + e], s[h]);
-          }
+          for (int h = 0; h < kHB; ++h) s[h] = fmaf(x[h], scv[c], s[h]);
         }
       }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&ctl->sfree[b]));
       float over = -INFINITY;
 #pragma unroll
-      for (int h = 0; h < 8; ++h) {
-        s[h] = valid ? fmaf(s[h], qunit[h], rope[h]) * p.scale_log2 : -INFINITY;
-        over = fmaxf(over, s[h] - (j > 0 ? ctl->mref[h0 + h] : 0.f));
+      for (int h = 0; h < kHB; ++h) {
+        s[h] = valid ? s[h] * p.scale_log2 : -INFINITY;
+        over = fmaxf(over, s[h] - (j > 0 ? ctl->mref[h] : 0.f));
       }
-      if (g == 0) {  // largest |scale| of the quarter's rows (zero in rows that are not there)
-        float m4[4];
+      if (slice_vote(j == 0 || over > kSliceRescale || !ok)) {
+        // ---- new reference maxima --------------------------------------------------------------------
 #pragma unroll
-        for (int c = 0; c < 4; ++c) m4[c] = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(scv[c]) & 0x7fffffffu));
-        if (lane == 0) *reinterpret_cast<float4*>(&ctl->smax[b][quarter][0]) = make_float4(m4[0], m4[1], m4[2], m4[3]);
-      }
-      const bool fresh = slice_vote(j == 0 || over > kSRescale || !ok);
-      if (fresh) {
-        // ---- new reference maxima (uniform branch) ----------------------------------------------------
+        for (int h = 0; h < kHB; ++h) {
+          float m = s[h];
 #pragma unroll
-        for (int h = 0; h < 8; ++h) {
-          const float m = s[h];
-          const uint32_t o = li_float_order(m);
-          const uint32_t mx = __reduce_max_sync(0xffffffffu, o);
-          if (lane == 0) ctl->red[quarter][h0 + h] = __uint_as_float((mx & 0x80000000u) ? (mx & 0x7fffffffu) : ~mx);
+          for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+          if (lane == 0) ctl->red[quarter][h] = m;
         }
         if (slice_vote(!ok)) {
           ok = false;
           break;
         }
-        if (tid < kSHeads) {
+        if (tid < kHB) {
           const float old = j > 0 ? ctl->mref[tid] : -INFINITY;
           const float m = fmaxf(fmaxf(ctl->red[0][tid], ctl->red[1][tid]), fmaxf(ctl->red[2][tid], ctl->red[3][tid]));
-          ctl->mref[tid] = fmaxf(old, m);
-          ctl->red[0][tid] = old == -INFINITY ? 0.f : ex2f(old - fmaxf(old, m));
+          const float mn = fmaxf(old, m);
+          ctl->alpha[tid] = old == -INFINITY ? 0.f : ex2f(old - mn);
+          ctl->mref[tid] = mn;
         }
         slice_meet();
         if (j > 0) {
+          ok = slice_wait(smem_u32(&ctl->done[b ^ 1]), ((t - 1) >> 1) & 1);  // the output so far is at rest
+          if (ok) tc_fence_after();
 #pragma unroll
-          for (int h = 0; h < 8; ++h) l[h] *= ctl->red[0][h0 + h];
+          for (int h = 0; h < kHB; ++h) l[h] *= ctl->alpha[h];
+          if (ok) {
+#pragma unroll 1
+            for (int c = 0; c < 4 * kHB; c += 16) {
+              uint32_t o[16];
+              tmem_ld_32x32b_x16(lane_addr + Cfg::kColO + c, o);
+              tc_wait_ld();
+#pragma unroll
+              for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * ctl->alpha[(c + e) & (kHB - 1)]);
+              tmem_st_32x32b_x16(lane_addr + Cfg::kColO + c, o);
+            }
+            tc_wait_st();
+          }
+          if (slice_vote(!ok)) {  // (alpha is read; a later tile may write it)
+            ok = false;
+            break;
+          }
         }
       }
 #pragma unroll
-      for (int h = 0; h < 8; ++h) {
-        const float m = ctl->mref[h0 + h];
+      for (int h = 0; h < kHB; ++h) {
+        const float m = ctl->mref[h];
         s[h] = ex2f(s[h] - (m == -INFINITY ? 0.f : m));
         l[h] += s[h];
       }
-      if (t >= 1) {  // the products that read the P^T of the tile before are complete, its O^T has a reader
-        ok = slice_wait(smem_u32(&ctl->done[b ^ 1]), ((t - 1) >> 1) & 1) && ok;
+      if (t >= 2) {  // the products that read this P buffer are complete
+        ok = slice_wait(smem_u32(&ctl->done[b]), ((t >> 1) - 1) & 1) && ok;
       }
-      float unit[4];
+      if (ok && key < kTK) {
+        const float scv[4] = {sc.x, sc.y, sc.z, sc.w};
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        unit[c] = fmaxf(fmaxf(ctl->smax[b][0][c], ctl->smax[b][1][c]), fmaxf(ctl->smax[b][2][c], ctl->smax[b][3][c]));
-      }
-      if (tid < kSHeads) {
-        if (tid == 0) {
-          ctl->rescale[b] = fresh && j > 0 ? 1 : 0;
-          *reinterpret_cast<float4*>(&ctl->fac[b][0]) =
-              make_float4(unit[0] * (1.0f / kSPUnit), unit[1] * (1.0f / kSPUnit), unit[2] * (1.0f / kSPUnit), unit[3] * (1.0f / kSPUnit));
+        for (int c = 0; c < 4; ++c) {
+          const uint32_t row = base + Cfg::kSmemP + (b * 4 + c) * Cfg::kPBytes + key * kHB * 2;
+#pragma unroll
+          for (int u = 0; u < kHB / 8; ++u) {
+            uint4 w;
+            w.x = pack_bf16x2(s[8 * u] * scv[c], s[8 * u + 1] * scv[c]);
+            w.y = pack_bf16x2(s[8 * u + 2] * scv[c], s[8 * u + 3] * scv[c]);
+            w.z = pack_bf16x2(s[8 * u + 4] * scv[c], s[8 * u + 5] * scv[c]);
+            w.w = pack_bf16x2(s[8 * u + 6] * scv[c], s[8 * u + 7] * scv[c]);
+            // swizzle: 32-byte rows, unit ^= (row / 4) % 2; 64-byte rows, unit ^= (row / 2) % 4
+            const int x = kHB == 16 ? (key >> 2) & 1 : (key >> 1) & 3;
+            sts_v4u(row + ((u ^ x) << 4), w);
+          }
         }
-        ctl->alpha[b][tid] = fresh && j > 0 ? ctl->red[0][tid] : 1.f;
-      }
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const float f = unit[c] > 0.f ? __fdividef(scv[c], unit[c]) * kSPUnit : 0.f;
-        uint32_t hi[2], lo[2];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          uint32_t y[4];  // low 22 bits: round(p * scale in units), two's complement; 7 low bits and the rest are the limbs
-#pragma unroll
-          for (int e = 0; e < 4; ++e) y[e] = __float_as_uint(fmaf(s[4 * u + e], f, 12582912.0f));
-          lo[u] = __byte_perm(__byte_perm(y[0], y[1], 0x0040), __byte_perm(y[2], y[3], 0x0040), 0x5410) & 0x7f7f7f7fu;
-          hi[u] = __byte_perm(__byte_perm(y[0] << 1, y[1] << 1, 0x0051), __byte_perm(y[2] << 1, y[3] << 1, 0x0051), 0x5410);
-        }
-        const uint32_t at = p_row + c * kSPBlock;
-        asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(at + u_hi), "r"(hi[0]), "r"(hi[1]) : "memory");
-        asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(at + u_lo), "r"(lo[0]), "r"(lo[1]) : "memory");
       }
       fence_proxy_async();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&ctl->pfull));
-      // (a `done` that expired is voted on at the next tile, or here at the last one)
-      if (j + 1 == it.ntiles) {
-        if (slice_vote(!ok)) {
-          ok = false;
-          break;
-        }
-      }
+      if (lane == 0) mbar_arrive(smem_u32(&ctl->pfull[b]));
     }
-    if (!ok) break;
-    // ---- row sums ------------------------------------------------------------------------------------
+    // (a `done` that expired at the last tile; the break above comes with the same answer in all four)
+    if (slice_vote(!ok)) {
+      ok = false;
+      break;
+    }
+    // ---- output --------------------------------------------------------------------------------------
 #pragma unroll
-    for (int h = 0; h < 8; ++h) {
+    for (int h = 0; h < kHB; ++h) {
       float v = l[h];
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if (lane == 0) ctl->red[quarter][h0 + h] = v;
+      if (lane == 0) ctl->red[quarter][h] = v;
     }
     slice_meet();
-    if (tid < kSHeads) {
+    if (tid < kHB) {
       const float tot = (ctl->red[0][tid] + ctl->red[1][tid]) + (ctl->red[2][tid] + ctl->red[3][tid]);
       if (p.n_split == 1) {
-        ctl->linv[n & 1][tid] = tot != 0.f ? 1.f / tot : 0.f;
+        ctl->alpha[tid] = tot > 0.f ? 1.f / tot : 0.f;
       } else {
-        ctl->linv[n & 1][tid] = 1.f;
-        const int64_t prow = (static_cast<int64_t>(it.ti) * p.n_split + it.sp) * p.nq + it.head0 + tid;
-        p.part_ml[prow * 2] = ctl->mref[tid];
-        p.part_ml[prow * 2 + 1] = tot;
+        ctl->alpha[tid] = 1.f;
+        p.part_ml[(prow0 + tid) * 2] = ctl->mref[tid];
+        p.part_ml[(prow0 + tid) * 2 + 1] = tot;
       }
     }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(smem_u32(&ctl->lfull[n & 1]));
-    slice_meet();  // (red and mref are read; the next item may write them)
-    ++n;
+    slice_meet();
+    ok = slice_wait(smem_u32(&ctl->done[(t - 1) & 1]), ((t - 1) >> 1) & 1);
+    tc_fence_after();
+#pragma unroll
+    for (int c = 0; c < 4 && ok; ++c) {  // dim 128 c + key of every head: 32 lanes write consecutive dims of a head's row
+      float o[kHB];
+      slice_ld<kHB>(lane_addr + Cfg::kColO + c * kHB, o);
+      if (c == 3) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&ctl->ofree));
+      }
+#pragma unroll
+      for (int h = 0; h < kHB; ++h) {
+        const float v = o[h] * ctl->alpha[h];
+        if (p.n_split == 1) p.out[(orow0 + h) * 512 + 128 * c + key] = __float2bfloat16_rn(v);
+        else p.part_o[(prow0 + h) * 512 + 128 * c + key] = v;
+      }
+    }
+    if (slice_vote(!ok)) ok = false;  // (alpha and mref are read; the next item may write them)
   }
   if (!ok && lane == 0) {
     ctl->abort = 1;
@@ -609,118 +622,34 @@ __device__ __forceinline__ void slice_role_softmax(const SfaParams& p, SliceCtl*
   }
 }
 
-// ================================ output =========================================================
-// Four warps, TMEM lane = dim of the block: fp32 sums of four blocks x 16 heads in registers.
-__device__ __forceinline__ void slice_role_output(const SfaParams& p, SliceCtl* ctl, uint32_t tmem, int n_items) {
-  const int lane = threadIdx.x & 31, quarter = (threadIdx.x >> 5) & 3;
-  const int dim = 32 * quarter + lane;
-  const uint32_t lane_addr = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + kSColO;
-  bool ok = true;
-  uint32_t t = 0, n = 0;
-  for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-    const SliceItem it = slice_item(p, item);
-    const int64_t orow0 = static_cast<int64_t>(it.ti) * p.nq_total + p.head_begin + it.head0;
-    const int64_t prow0 = (static_cast<int64_t>(it.ti) * p.n_split + it.sp) * p.nq + it.head0;
-    if (it.ntiles == 0) {
-      const int tid = threadIdx.x - 32 * kSOutWarp0;
-      if (p.n_split == 1) {
-        for (int e = tid; e < kSHeads * 64; e += 128) *reinterpret_cast<uint4*>(p.out + orow0 * 512 + e * 8) = make_uint4(0, 0, 0, 0);
-      } else if (tid < kSHeads) {
-        p.part_ml[(prow0 + tid) * 2] = -INFINITY;
-        p.part_ml[(prow0 + tid) * 2 + 1] = 0.f;
-      }
-      continue;
-    }
-    float o[4][kSHeads];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-#pragma unroll
-      for (int h = 0; h < kSHeads; ++h) o[c][h] = 0.f;
-    }
-    for (int j = 0; j < it.ntiles; ++j, ++t) {
-      const uint32_t b = t & 1;
-      ok = slice_wait(smem_u32(&ctl->done[b]), (t >> 1) & 1);
-      if (!ok) break;
-      tc_fence_after();
-      if (ctl->rescale[b] != 0) {
-#pragma unroll
-        for (int h = 0; h < kSHeads; ++h) {
-          const float a = ctl->alpha[b][h];
-#pragma unroll
-          for (int c = 0; c < 4; ++c) o[c][h] *= a;
-        }
-      }
-      const float4 f4 = *reinterpret_cast<const float4*>(&ctl->fac[b][0]);
-      const float f[4] = {f4.x, f4.y, f4.z, f4.w};
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t v[32];
-        tmem_ld_32x32b_x32(lane_addr + c * 2 * kSHeads, v);
-        tc_wait_ld();
-#pragma unroll
-        for (int h = 0; h < kSHeads; ++h) {
-          o[c][h] = fmaf(static_cast<float>(static_cast<int>(v[h]) * 128 + static_cast<int>(v[kSHeads + h])), f[c], o[c][h]);
-        }
-      }
-      // the item's row sums are read before its last tile lets go, so that they can be written again two items on
-      if (j + 1 == it.ntiles) {
-        ok = slice_wait(smem_u32(&ctl->lfull[n & 1]), (n >> 1) & 1);
-        if (!ok) break;
-#pragma unroll
-        for (int h = 0; h < kSHeads; ++h) {
-          const float a = ctl->linv[n & 1][h];
-#pragma unroll
-          for (int c = 0; c < 4; ++c) o[c][h] *= a;
-        }
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&ctl->ofree));
-    }
-    if (!ok) break;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {  // 32 lanes write consecutive dims of a head's row
-#pragma unroll
-      for (int h = 0; h < kSHeads; ++h) {
-        if (p.n_split == 1) p.out[(orow0 + h) * 512 + 128 * c + dim] = __float2bfloat16_rn(o[c][h]);
-        else p.part_o[(prow0 + h) * 512 + 128 * c + dim] = o[c][h];
-      }
-    }
-    ++n;
-  }
-  if (!ok && lane == 0) {
-    ctl->abort = 1;
-    set_status(p.status, PTO_ST_WAIT_EXPIRED, blockIdx.x, 96);
-  }
-}
-
-__global__ void __launch_bounds__(kSThreads, 1)
+template <int kHB, int kTK>
+__global__ void __launch_bounds__(SliceCfg<kHB, kTK>::kThreads, 1)
 sfa_slice_kernel(const __grid_constant__ SfaParams p, int n_items) {
+  using Cfg = SliceCfg<kHB, kTK>;
   extern __shared__ __align__(1024) uint8_t sfa_slice_smem[];
   const uint32_t base = smem_u32(sfa_slice_smem);
   if ((base & 1023u) != 0) {  // the swizzled operand tiles need a 1024-byte aligned base
     if (threadIdx.x == 0) set_status(p.status, PTO_ST_WAIT_EXPIRED, static_cast<int>(base), 95);
     return;
   }
-  SliceCtl* ctl = reinterpret_cast<SliceCtl*>(sfa_slice_smem + kSSmemCtl);
+  auto* ctl = reinterpret_cast<SliceCtl<kHB, kTK>*>(sfa_slice_smem + Cfg::kSmemCtl);
   const int tid = threadIdx.x, warp = tid >> 5;
   if (tid == 0) {
     for (int b = 0; b < 2; ++b) {
-      mbar_init(smem_u32(&ctl->full[b]), kSProdWarps);
+      mbar_init(smem_u32(&ctl->full[b]), Cfg::kProdWarps);
       mbar_init(smem_u32(&ctl->done[b]), 1);
       mbar_init(smem_u32(&ctl->sfull[b]), 1);
-      mbar_init(smem_u32(&ctl->sfree[b]), kSSoftWarps);
-      mbar_init(smem_u32(&ctl->qfull[b]), 2);
-      mbar_init(smem_u32(&ctl->qfree[b]), 1);
-      mbar_init(smem_u32(&ctl->lfull[b]), kSSoftWarps);
+      mbar_init(smem_u32(&ctl->sfree[b]), 4);
+      mbar_init(smem_u32(&ctl->pfull[b]), 4);
     }
-    mbar_init(smem_u32(&ctl->pfull), kSSoftWarps);
+    mbar_init(smem_u32(&ctl->qfull), 2);
+    mbar_init(smem_u32(&ctl->qfree), 1);
     mbar_init(smem_u32(&ctl->ofree), 4);
     ctl->abort = 0;
     fence_mbar_init();
   }
   if (warp == 0) {
-    tmem_alloc(smem_u32(&ctl->tmem_base), kSTmemCols);
+    tmem_alloc(smem_u32(&ctl->tmem_base), Cfg::kTmemCols);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -729,45 +658,51 @@ sfa_slice_kernel(const __grid_constant__ SfaParams p, int n_items) {
   const uint32_t tmem = ctl->tmem_base;
   pdl_wait();  // the set-up above overlaps the tail of the kernel before this one
   if (tid == 0) pdl_trigger();
-  if (warp < kSSoftWarp0) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kSRegIssue));
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::kRegIssue));
     if (warp < 2 && base == kSliceUsualBase) {
-      if (warp == 0) slice_role_scores<kSliceUsualBase>(p, ctl, base, tmem, n_items);
-      else slice_role_values<kSliceUsualBase>(p, ctl, base, tmem, n_items);
-    } else if (warp == 0) slice_role_scores<0>(p, ctl, base, tmem, n_items);
-    else if (warp == 1) slice_role_values<0>(p, ctl, base, tmem, n_items);
-    else slice_role_query(p, ctl, base, n_items);
-  } else if (warp < kSOutWarp0) {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSRegSoft));
-    slice_role_softmax(p, ctl, base, tmem, n_items);
-  } else if (warp < kSProdWarp0) {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSRegOut));
-    slice_role_output(p, ctl, tmem, n_items);
+      if (warp == 0) slice_role_scores<kHB, kTK, kSliceUsualBase>(p, ctl, base, tmem, n_items);
+      else slice_role_values<kHB, kTK, kSliceUsualBase>(p, ctl, base, tmem, n_items);
+    } else if (warp == 0) slice_role_scores<kHB, kTK, 0>(p, ctl, base, tmem, n_items);
+    else if (warp == 1) slice_role_values<kHB, kTK, 0>(p, ctl, base, tmem, n_items);
+    else slice_role_query<kHB, kTK>(p, ctl, base, n_items);
+  } else if (warp < 8) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Cfg::kRegSoftmax));
+    slice_role_softmax<kHB, kTK>(p, ctl, base, tmem, n_items);
   } else {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kSRegProd));
-    if (p.packed) slice_role_producer<true>(p, ctl, base, n_items);
-    else slice_role_producer<false>(p, ctl, base, n_items);
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::kRegProd));
+    if (p.packed) slice_role_producer<kHB, kTK, true>(p, ctl, base, n_items);
+    else slice_role_producer<kHB, kTK, false>(p, ctl, base, n_items);
   }
   tc_fence_before();
   __syncthreads();
   if (warp == 0) {
     tc_fence_after();
-    tmem_dealloc(tmem, kSTmemCols);
+    tmem_dealloc(tmem, Cfg::kTmemCols);
   }
+}
+
+template <int kHB, int kTK>
+cudaError_t launch_one(const SfaParams& p, int num_sms, cudaStream_t stream) {
+  using Cfg = SliceCfg<kHB, kTK>;
+  constexpr size_t smem = Cfg::kSmemCtl + sizeof(SliceCtl<kHB, kTK>);
+  static_assert(smem <= 232448, "exceeds the 227 KB of shared memory a CTA may use");
+  auto kernel = sfa_slice_kernel<kHB, kTK>;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  if (e != cudaSuccess) return e;
+  const long long items = static_cast<long long>(p.b) * p.s1 * (p.nq / kHB) * p.n_split;
+  if (items > 0x7fffffffLL) return cudaErrorInvalidValue;
+  const int grid = static_cast<int>(items < num_sms ? items : num_sms);
+  count_launch();
+  return launch_maybe_pdl(kernel, dim3(grid), dim3(Cfg::kThreads), smem, stream, p.pdl != 0, p, static_cast<int>(items));
 }
 
 }  // namespace
 
-int sfa_slice_heads() { return kSHeads; }
+int sfa_slice_heads(int nq) { return nq % 32 == 0 ? 32 : 16; }
 
 cudaError_t launch_sfa_slice(const SfaParams& p, int num_sms, cudaStream_t stream) {
-  const cudaError_t e = cudaFuncSetAttribute(sfa_slice_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSSmemBytes));
-  if (e != cudaSuccess) return e;
-  const long long items = static_cast<long long>(p.b) * p.s1 * (p.nq / kSHeads) * p.n_split;
-  if (items > 0x7fffffffLL) return cudaErrorInvalidValue;
-  const int grid = static_cast<int>(items < num_sms ? items : num_sms);
-  count_launch();
-  return launch_maybe_pdl(sfa_slice_kernel, dim3(grid), dim3(kSThreads), kSSmemBytes, stream, p.pdl != 0, p, static_cast<int>(items));
+  return sfa_slice_heads(p.nq) == 32 ? launch_one<32, 64>(p, num_sms, stream) : launch_one<16, 80>(p, num_sms, stream);
 }
 
 }  // namespace pto

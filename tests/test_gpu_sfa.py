@@ -94,8 +94,9 @@ def test_head_slice_of_16():
 
 @pytest.mark.parametrize("packed", [False, True], ids=["split_arrays", "packed_rows"])
 @pytest.mark.parametrize("nq,lens,s1", [
-    (16, [1, 127, 128, 129, 256, 257, 2048, 2500], 1),  # edges of its 128-row tiles; one item per SM and split
-    (32, [63, 64, 65, 128, 2047, 130, 0, 3000], 2),    # two blocks of 16 heads, tokens that see nothing
+    (16, [1, 127, 128, 129, 256, 257, 2048, 2500], 1),
+    (16, [1, 79, 80, 81, 160, 161, 2048, 2500], 1),    # edges of its 80-row tiles; one item per SM and split
+    (32, [63, 64, 65, 128, 2047, 130, 0, 3000], 2),    # edges of its 64-row tiles, tokens that see nothing
     (48, [700, 2100], 2),                              # three blocks of 16 heads
     (64, [300] * 90, 1),                               # more items than SMs: CTAs walk several, unsplit
 ])
@@ -110,6 +111,58 @@ def test_head_slices_at_tile_edges(nq, lens, s1, packed):
                 _check(got[bi, i], want[bi, i])
             else:
                 assert torch.all(got[bi, i] == 0)
+
+
+def _uneven_inputs(kind, nq, act, s1):
+    """Attention inputs whose terms differ much in size; the rest of a token's rows share an offset of their latent values,
+    so that weight that is lost shows in the output."""
+    d = gen.make_inputs(act, s1=s1, seed=71, with_indexer=False, with_topk=True, attn_heads=nq)
+    g = torch.Generator().manual_seed(nq)
+    offset = torch.randint(-60, 61, (1, 512), generator=g)
+    d.key_nope_2d = (offset + torch.randint(-40, 41, d.key_nope_2d.shape, generator=g)).to(torch.int8)
+    d.query_rope[:, :2] = 8.0
+    d.key_rope_2d[:, :2] = 0.0
+    for bi in range(d.b):
+        table = d.block_table[bi].long()
+        if kind.startswith("sink"):  # the sequence's first row, `nats` above the others; a token selects it first of all
+            row = table[0] * 128
+            nats = float(kind[4:])
+            d.key_rope_2d[row, 0] = nats * 24.0 / 8.0
+            d.key_nope_2d[row] = torch.randint(-3, 4, (512,), generator=g).to(torch.int8)
+            for ti in range(bi * s1, (bi + 1) * s1):
+                sel = d.topk_indices[ti]
+                sel[(sel == 0).nonzero()] = sel[0].clone()
+                sel[0] = 0
+        elif kind == "scale":  # a row in 128 with a scale 300 times its neighbours', little weight and few values
+            rows = table[torch.arange(act[bi] // 128)] * 128 + torch.randint(0, 128, (act[bi] // 128,), generator=g)
+            d.k_nope_scales[rows] = 1.5
+            d.key_rope_2d[rows, 1] = -9.0
+            d.key_nope_2d[rows] = (torch.rand((rows.numel(), 512), generator=g) < 0.02).to(torch.int8)
+    if kind == "query":  # one dim of every query a hundred times the others
+        d.query_nope[:, 5] *= 100.0
+    return d
+
+
+@pytest.mark.parametrize("nq", [16, 64, 128])
+@pytest.mark.parametrize("act,s1", [([2300, 700], 2), ([2400], 148)], ids=["split", "unsplit"])
+@pytest.mark.parametrize("kind", ["sink7", "sink9", "sink11", "scale", "query"])
+def test_terms_of_very_different_size(kind, act, s1, nq):
+    """Against 64 bits, per token and head, since a norm over the whole output hides single heads. The bound: probabilities (or
+    probability times row scale), row values and outputs are rounded to bf16 once each, 2^-9 of a term at most. The dominant
+    term may meet the worst of the first two; the other terms' and the output's roundings are independent (0.0011 rms):
+    2 * 2^-9 + 0.0011 = REL_L2. (The oracle rounds its probabilities to bf16 as well: up to another 2^-9 apart.)"""
+    s1 = s1 if nq == 16 or s1 == 2 else 80
+    d = _uneven_inputs(kind, nq, act, s1)
+    got = _run(d, nq=nq).double()
+    for ti in range(d.t):
+        bi, i = divmod(ti, s1)
+        sel = d.topk_indices[ti, :min(act[bi] - s1 + 1 + i, 2048)].long()
+        rows = d.block_table[bi].long()[sel // 128] * 128 + sel % 128
+        v = (d.key_nope_2d[rows].double().reshape(-1, 4, 128) * d.k_nope_scales[rows].double()[:, :, None]).reshape(-1, 512)
+        qn, qr = (q.reshape(d.t, nq, -1)[ti].double() for q in (d.query_nope, d.query_rope))
+        want = torch.softmax((qn @ v.T + qr @ d.key_rope_2d[rows].double().T) * SCALE, dim=-1) @ v
+        err = (got[bi, i] - want).norm(dim=-1) / want.norm(dim=-1)
+        assert float(err.max()) <= REL_L2, (ti, float(err.max()), float(err.mean()))
 
 
 @pytest.mark.parametrize("tokens", [1, 14, 15, 24, 37], ids=lambda t: f"{t}_tokens")  # 16, 5, 4, 3 and 2 splits
