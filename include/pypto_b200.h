@@ -69,6 +69,9 @@ typedef struct CUstream_st* pto_stream_t; /* cudaStream_t */
 #define PTO_STATUS_WORDS 8
 #define PTO_ST_BAD_PAGE 0x1    /* a block-table entry or top-k index outside its range was skipped */
 #define PTO_ST_WAIT_EXPIRED 0x2 /* a bounded mbarrier wait gave up; results are incomplete */
+/* word 3 counts the rows whose selection fell back to the radix select (massive ties, values that are not
+ * finite): right, but several scans of the row by one SM. Not an error. */
+#define PTO_STATUS_RADIX_ROWS 3
 
 int pto_abi_version(void);
 const char* pto_strerror(int code);

@@ -15,6 +15,7 @@ PTO_LI_SCORE_SIMT, PTO_LI_UNSORTED, PTO_LI_FP16_CHAIN, PTO_LI_EPILOGUE_HIST = 0x
 PTO_STATUS_WORDS = 8
 PTO_LI_STATIC_SCRATCH_BYTES = (8 << 20) + 256
 PTO_ST_BAD_PAGE, PTO_ST_WAIT_EXPIRED = 0x1, 0x2
+PTO_STATUS_RADIX_ROWS = 3  # status word: rows whose selection fell back to the radix select
 
 _vp, _i, _sz, _i64, _f = C.c_void_p, C.c_int, C.c_size_t, C.c_int64, C.c_float
 

@@ -48,7 +48,6 @@ constexpr int kMaxK = 2048;
 constexpr int kListCap = 6144;
 constexpr int kChunk = 16 * kTopkThreads;  // positions per bulk copy
 constexpr int kRing = 3;                   // copies in flight (96 KB)
-constexpr int kWarpCap = kListCap / kTopkWarps;  // keys a warp collects before they go to the list
 constexpr int kBinCap = 512;               // keys of a bin that are still ranked by counting
 static_assert(kMaxK <= kListCap, "a row of at most k positions is handled as a list");
 
@@ -61,13 +60,13 @@ struct TopkSmem {
     };
   };
   unsigned long long list[kListCap];       // rank 0: the candidates of the row
-  unsigned long long mine[kTopkWarps][kWarpCap];  // the keys each warp of this CTA collected
+  unsigned long long mine[kListCap];       // the keys this CTA collected, where they have to go elsewhere
   unsigned int hist[kLiHistBins > kBins ? kLiHistBins : kBins];
   unsigned int warp_tot[32];
-  unsigned int warp_n[32];
   unsigned int red_min[32], red_max[32];   // order-preserving images
   uint64_t full[kRing];                    // bytes of a chunk landed
   uint64_t empty[kRing];                   // every warp has read it
+  unsigned int n_mine;                     // keys this CTA collected (more than kListCap: some are missing)
   unsigned int n_list;                     // rank 0: keys in `list` (more than kListCap: some are missing)
   unsigned int offset;                     // of this CTA's keys in the list
   unsigned int hist_total;
@@ -375,6 +374,7 @@ li_topk_kernel(TopkParams p) {
     }
     fence_mbar_init();
     fence_proxy_async();
+    sm->n_mine = 0;
     sm->n_list = 0;
     sm->n_sel = 0;
     sm->thr_bin = 0;
@@ -445,7 +445,12 @@ li_topk_kernel(TopkParams p) {
     if (!known) bound = sample_bound(sm, row, eff, k);
     TKT(2);
     // ---- 2. this rank's keys at or above the bound ------------------------------------------------
-    unsigned int n = 0;
+    // One list for the CTA, in which a warp reserves its places chunk by chunk: however the selected positions lie in the row,
+    // nothing but their number limits it. (With a list of its own for each warp, 384 places, a run of 385 neighbouring
+    // selected positions could fill one, and sent the row to the radix select: 64 rows of 65536 whose last 2048 positions are
+    // selected 62 -> 27 us, scattered selections 26 either way.) It is the row's list at once where this rank's
+    // keys are the first in that: where it is the only rank, and rank 0 of two.
+    unsigned long long* const mine = rank == 0 && csize <= 2 ? sm->list : sm->mine;
     bool ok = true;
     for (int c = 0; c < chunks; ++c) {
       const uint32_t ph = (c / kRing) & 1;
@@ -457,8 +462,8 @@ li_topk_kernel(TopkParams p) {
       const float* chunk = sm->ring[c % kRing];
       const int p0 = begin + c * kChunk;
       // Few elements pass. Sixteen comparisons a thread give a mask; its count behind the counts of the lanes below is the
-      // thread's place in the warp's list (a ballot per element needs two population counts each, which run at an eighth
-      // of the rate); the few set bits are walked and their values read again. A warp takes 512 neighbouring positions.
+      // thread's place in the warp's part of the list (a ballot per element needs two population counts each, which run at an
+      // eighth of the rate); the few set bits are walked and their values read again. A warp takes 512 neighbouring positions.
       auto offset = [&](int e) { return warp * 512 + (e >> 2) * 128 + lane * 4 + (e & 3); };
       unsigned int mask = 0u;
 #pragma unroll
@@ -474,54 +479,47 @@ li_topk_kernel(TopkParams p) {
         }
       }
       const unsigned int cnt = __popc(mask);
-      unsigned int incl = cnt;
+      const unsigned int n = __reduce_add_sync(0xffffffffu, cnt);
+      if (n != 0u) {  // (uniform)
+        unsigned int at = 0;
+        if (lane == 0) at = atomicAdd(&sm->n_mine, n);
+        unsigned int incl = cnt;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const unsigned int up = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += up;
-      }
-      unsigned int at = n + incl - cnt;
-      n += __shfl_sync(0xffffffffu, incl, 31);
-      if (n <= static_cast<unsigned int>(kWarpCap)) {  // (else the list is spoilt, its length says so below)
-        while (mask != 0u) {
-          const int e = __ffs(mask) - 1;
-          mask &= mask - 1u;
-          const int off = offset(e);
-          sm->mine[warp][at++] = make_key(chunk[off], p0 + off);
+        for (int o = 1; o < 32; o <<= 1) {
+          const unsigned int up = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += up;
+        }
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (at + n <= static_cast<unsigned int>(kListCap)) {  // (else the list is spoilt, its length says so below)
+          at += incl - cnt;
+          while (mask != 0u) {
+            const int e = __ffs(mask) - 1;
+            mask &= mask - 1u;
+            const int off = offset(e);
+            mine[at++] = make_key(chunk[off], p0 + off);
+          }
         }
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&sm->empty[c % kRing]));
     }
-    if (!ok) {
-      if (lane == 0) set_status(p.status, PTO_ST_WAIT_EXPIRED, row_id, 30);
-      n = kListCap + 1;
+    if (!ok && lane == 0) {
+      set_status(p.status, PTO_ST_WAIT_EXPIRED, row_id, 30);
+      atomicAdd(&sm->n_mine, static_cast<unsigned int>(kListCap + 1));
     }
     TKT(3);
-    if (lane == 0) sm->warp_n[warp] = n;
     __syncthreads();
-    // ---- the lists of all warps and ranks, one behind the other, into rank 0's ----------------------
-    const unsigned int mine_n = lane < kTopkWarps ? sm->warp_n[lane] : 0u;
-    unsigned int incl = mine_n;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned int x = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += x;
-    }
-    // a warp that found more than it could keep spoils the list: its length says so
-    unsigned int total = __shfl_sync(0xffffffffu, incl, 31);
-    if (__any_sync(0xffffffffu, mine_n > static_cast<unsigned int>(kWarpCap))) total = kListCap + 1;
-    const unsigned int warp_off = __shfl_sync(0xffffffffu, incl - mine_n, warp);
+    // ---- the lists of all ranks, one behind the other, into rank 0's --------------------------------
+    const unsigned int total = min(sm->n_mine, static_cast<unsigned int>(kListCap + 1));  // (what is spoilt stays spoilt)
     if (csize == 2) {
       // two ranks: rank 0's keys from the front of the list, rank 1's from its end, with their number: nobody waits for a count
       cluster_wait();
-      if (total <= static_cast<unsigned int>(kListCap)) {
-        for (unsigned int j = lane; j < n; j += 32) {
-          if (rank == 0) sm->list[warp_off + j] = sm->mine[warp][j];
-          else st_peer_u64(peer_addr(&sm->list[kListCap - 1 - (warp_off + j)], 0), sm->mine[warp][j]);
+      if (rank == 1) {
+        if (total <= static_cast<unsigned int>(kListCap)) {
+          for (unsigned int j = tid; j < total; j += kTopkThreads) st_peer_u64(peer_addr(&sm->list[kListCap - 1 - j], 0), sm->mine[j]);
         }
+        if (tid == 0) st_peer_u32(peer_addr(&sm->n_list, 0), total);
       }
-      if (rank == 1 && tid == 0) st_peer_u32(peer_addr(&sm->n_list, 0), total);
       cluster_arrive();
       cluster_wait();
       if (rank != 0) return;
@@ -533,9 +531,8 @@ li_topk_kernel(TopkParams p) {
       __syncthreads();
       const unsigned int off = sm->offset;
       if (total <= static_cast<unsigned int>(kListCap)) {
-        for (unsigned int j = lane; j < n; j += 32) {
-          const unsigned int at = off + warp_off + j;
-          if (at < static_cast<unsigned int>(kListCap)) st_peer_u64(peer_addr(&sm->list[at], 0), sm->mine[warp][j]);
+        for (unsigned int j = tid; j < total; j += kTopkThreads) {
+          if (off + j < static_cast<unsigned int>(kListCap)) st_peer_u64(peer_addr(&sm->list[off + j], 0), sm->mine[j]);
         }
       }
       cluster_arrive();
@@ -543,11 +540,7 @@ li_topk_kernel(TopkParams p) {
       if (rank != 0) return;
       n_list = sm->n_list;
     } else {
-      if (total <= static_cast<unsigned int>(kListCap)) {
-        for (unsigned int j = lane; j < n; j += 32) sm->list[warp_off + j] = sm->mine[warp][j];
-      }
       n_list = total;
-      __syncthreads();
     }
     if (n_list <= static_cast<unsigned int>(kListCap)) {
       for (unsigned int j = tid; j < n_list; j += kTopkThreads) {
@@ -634,7 +627,10 @@ li_topk_kernel(TopkParams p) {
   }
 
   // ---- 3'. MSB-first radix select on the 64-bit keys of the whole row (rank 0) ----------------------------
-  if (tid == 0) sm->n_sel = 0;
+  if (tid == 0) {
+    sm->n_sel = 0;
+    if (p.status != nullptr) atomicAdd(p.status + PTO_STATUS_RADIX_ROWS, 1);
+  }
   // digits: 11/11/10 bits of the value word, then 11/11/10 bits of the inverted position.
   // invariant: keys with (key >> shift) > prefix are selected; `remaining` more are needed among those with
   // (key >> shift) == prefix.

@@ -5,6 +5,7 @@ import torch
 
 import oracle
 import pypto_b200 as pto
+from pypto_b200 import _lib
 from pypto_b200 import inputs as gen
 from golden_util import LI_CASES, load_case
 
@@ -342,6 +343,30 @@ def test_topk_stage_over_row_lengths_and_distributions(rows, n, k, kind, sort):
     m = min(n, k)
     assert torch.all(got[:, m:] == -1)
     got = got[:, :m]
+    if not sort:
+        got, want = got.sort(dim=1).values, want.sort(dim=1).values
+    assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("sort", [True, False], ids=["ordered", "unordered"])
+@pytest.mark.parametrize("rows,n", [(8, 32768), (40, 65536), (160, 20000), (3, 131072)])  # clusters of 4, 2, 1 and 8 CTAs
+@pytest.mark.parametrize("where", ["last", "runs", "aligned", "scattered"])
+def test_neighbouring_positions_need_no_radix_select(where, rows, n, sort):
+    """A selection of neighbouring positions (recency makes that the normal case) goes the same way as a scattered one."""
+    k = 2048
+    g = torch.Generator().manual_seed(n)
+    sc = torch.randn(rows, n, generator=g)
+    starts, run = {"last": ([n - k], k), "runs": ([n // 5 + 1, n // 3 + 7, n // 2 + 3, n - 700], 512),
+                   "aligned": ([0, 4096, 8192, 16384], 512), "scattered": ([], 0)}[where]
+    for at in starts:
+        sc[:, at:at + run] += 20.0
+    act = torch.full((rows,), n, dtype=torch.int32, device=DEV)
+    out = torch.zeros((rows, 1, k), dtype=torch.int32, device=DEV)
+    pto.reset_workspace_status()
+    pto.lightning_indexer_topk(sc.to(DEV), act, out, 1, k, sort=sort)
+    status = pto.workspace_status()
+    assert status[0] == 0 and status[_lib.PTO_STATUS_RADIX_ROWS] == 0
+    got, want = out.cpu()[:, 0].long(), sc.sort(dim=1, descending=True, stable=True).indices[:, :k]
     if not sort:
         got, want = got.sort(dim=1).values, want.sort(dim=1).values
     assert torch.equal(got, want)
