@@ -289,40 +289,48 @@ __device__ __forceinline__ void block_range(TopkSmem* sm, float& vmin, float& vm
 __device__ float sample_bound(TopkSmem* sm, const float* row, int eff, int k) {
   const int tid = threadIdx.x;
   const int groups = eff >> 2;
-  // groups per thread: long rows need a larger sample for a list of the same length
+  // groups per thread: long rows need a larger sample for a list of the same length (beyond 2^20 positions one that meets 32 or
+  // more of 2048 selected ones)
   constexpr int kMaxPer = 4096 / kTopkThreads;
-  const int per = (eff <= (1 << 16) ? 1024 : (eff <= (1 << 18) ? 2048 : 4096)) / kTopkThreads;
-  float4 v[kMaxPer];
+  const int per = eff <= (1 << 20) ? (eff <= (1 << 16) ? 1024 : (eff <= (1 << 18) ? 2048 : 4096)) / kTopkThreads : (eff + (1 << 17) - 1) >> 17;
+  const float samples = static_cast<float>(4 * kTopkThreads) * static_cast<float>(per);
+  float4 v[kMaxPer];  // the sample, or the part of a larger one at hand
+  auto load = [&](int u0) {
+#pragma unroll
+    for (int u = 0; u < kMaxPer; ++u) {
+      if (u0 + u < per) {
+        const int g = static_cast<int>(static_cast<long long>(tid + (u0 + u) * kTopkThreads) * groups / (static_cast<long long>(kTopkThreads) * per));
+        v[u] = __ldg(reinterpret_cast<const float4*>(row) + g);
+      }
+    }
+  };
+  auto each = [&](auto&& f) {
+    for (int u0 = 0; u0 < per; u0 += kMaxPer) {
+      if (per > kMaxPer) load(u0);
+#pragma unroll
+      for (int u = 0; u < kMaxPer; ++u) {
+        if (u0 + u < per) {
+          f(v[u].x);
+          f(v[u].y);
+          f(v[u].z);
+          f(v[u].w);
+        }
+      }
+    }
+  };
+  if (per <= kMaxPer) load(0);
   float vmin = INFINITY, vmax = -INFINITY;
-#pragma unroll
-  for (int u = 0; u < kMaxPer; ++u) {
-    if (u < per) {
-      const int g = static_cast<int>(static_cast<long long>(tid + u * kTopkThreads) * groups / (kTopkThreads * per));
-      v[u] = __ldg(reinterpret_cast<const float4*>(row) + g);
-    }
-  }
-#pragma unroll
-  for (int u = 0; u < kMaxPer; ++u) {
-    if (u < per) {
-      vmin = fminf(vmin, fminf(fminf(v[u].x, v[u].y), fminf(v[u].z, v[u].w)));
-      vmax = fmaxf(vmax, fmaxf(fmaxf(v[u].x, v[u].y), fmaxf(v[u].z, v[u].w)));
-    }
-  }
+  each([&](float x) {
+    vmin = fminf(vmin, x);
+    vmax = fmaxf(vmax, x);
+  });
   for (int j = tid; j < kBins; j += kTopkThreads) sm->hist[j] = 0;
   block_range(sm, vmin, vmax);
   BinMap map;
   map.set(vmin, vmax);
-#pragma unroll
-  for (int u = 0; u < kMaxPer; ++u) {
-    if (u < per) {
-      atomicAdd(&sm->hist[map.bin(v[u].x)], 1u);
-      atomicAdd(&sm->hist[map.bin(v[u].y)], 1u);
-      atomicAdd(&sm->hist[map.bin(v[u].z)], 1u);
-      atomicAdd(&sm->hist[map.bin(v[u].w)], 1u);
-    }
-  }
+  each([&](float x) { atomicAdd(&sm->hist[map.bin(x)], 1u); });
   __syncthreads();
-  const float mean = static_cast<float>(k) * static_cast<float>(4 * kTopkThreads * per) / static_cast<float>(eff);
+  const float mean = static_cast<float>(k) * samples / static_cast<float>(eff);
   find_threshold_bin<kBins / kTopkThreads>(sm, static_cast<unsigned int>(mean + 4.5f * sqrtf(mean) + 4.0f));
   const int b = sm->thr_bin;
   if (map.inv == 0.f || b == 0) return -INFINITY;

@@ -349,7 +349,8 @@ def test_topk_stage_over_row_lengths_and_distributions(rows, n, k, kind, sort):
 
 
 @pytest.mark.parametrize("sort", [True, False], ids=["ordered", "unordered"])
-@pytest.mark.parametrize("rows,n", [(8, 32768), (40, 65536), (160, 20000), (3, 131072)])  # clusters of 4, 2, 1 and 8 CTAs
+@pytest.mark.parametrize("rows,n", [(8, 32768), (40, 65536), (160, 20000), (3, 131072),  # clusters of 4, 2, 1 and 8 CTAs
+                                    (1, 5000000)])  # a sample of its own size
 @pytest.mark.parametrize("where", ["last", "runs", "aligned", "scattered"])
 def test_neighbouring_positions_need_no_radix_select(where, rows, n, sort):
     """A selection of neighbouring positions (recency makes that the normal case) goes the same way as a scattered one."""
