@@ -371,3 +371,43 @@ def test_neighbouring_positions_need_no_radix_select(where, rows, n, sort):
     if not sort:
         got, want = got.sort(dim=1).values, want.sort(dim=1).values
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("sort", [True, False], ids=["ordered", "unordered"])
+@pytest.mark.parametrize("rows,n", [(3, 5000), (8, 32768), (40, 65536), (160, 20000), (2, 1200000)])
+@pytest.mark.parametrize("kind", ["outlier", "far_outliers", "tail", "masked", "infinite", "offset", "small"])
+def test_uneven_scores_need_no_radix_select(kind, rows, n, sort):
+    """Values far from the others must not send the others to one bin."""
+    k = 2048
+    g = torch.Generator().manual_seed(n)
+    sc = torch.randn(rows, n, generator=g)
+    if kind == "outlier":
+        sc[:, 5] = 300.0
+    elif kind == "far_outliers":
+        sc[:, 5], sc[:, 7], sc[:, 4000] = 3e38, -3e38, 1e9
+    elif kind == "tail":
+        sc = (2.5 * sc).exp()
+    elif kind == "masked":
+        sc[:, ::7] = -1e4
+        sc[:, 1::7] = torch.finfo(torch.float32).min
+    elif kind == "infinite":
+        sc[:, ::7] = float("-inf")
+        sc[:, 1::997] = float("inf")
+    elif kind == "offset":
+        sc = sc + 1000.0
+    elif kind == "small":
+        sc = sc * 1e-20 - 1e-20
+    act = torch.full((rows,), n, dtype=torch.int32, device=DEV)
+    out = torch.zeros((rows, 1, k), dtype=torch.int32, device=DEV)
+    pto.reset_workspace_status()
+    pto.lightning_indexer_topk(sc.to(DEV), act, out, 1, k, sort=sort)
+    status = pto.workspace_status()
+    assert status[0] == 0
+    # (of 1.2 million values 1204 are +inf, more than a bin holds; beside 3e38, 127 powers of two away, a bin is a 16th of one and
+    # holds a thousand of those at the end of the selection)
+    if n < 1000000 or kind not in ("infinite", "far_outliers"):
+        assert status[_lib.PTO_STATUS_RADIX_ROWS] == 0
+    got, want = out.cpu()[:, 0].long(), sc.sort(dim=1, descending=True, stable=True).indices[:, :k]
+    if not sort:
+        got, want = got.sort(dim=1).values, want.sort(dim=1).values
+    assert torch.equal(got, want)
