@@ -309,9 +309,11 @@ struct LiParams {
 constexpr int kLiHistBins = 4096;
 constexpr int kLiHistShift = 20;  // bin = order(score) >> 20: sign, exponent, three mantissa bits
 constexpr int kLiHistMaxS1 = 2;   // tokens per launch the score kernel keeps a shared-memory histogram for
+// Order-preserving image of a float. (The sign bit set by `|` is compiled to a floating negation, which turns every NaN into
+// 0x7fffffff, an image between the negative numbers and the positive ones.)
 __device__ __forceinline__ unsigned int li_float_order(float f) {
   const unsigned int u = __float_as_uint(f);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+  return u ^ (static_cast<unsigned int>(static_cast<int>(u) >> 31) | 0x80000000u);
 }
 
 struct TopkParams {

@@ -454,7 +454,7 @@ li_topk_kernel(TopkParams p) {
         for (int e = 0; e < 4; ++e) {
           if (j + e < eff) {
             sm->list[j + e] = make_key(x[e], j + e);
-            if (x[e] == x[e]) {
+            if (x[e] == x[e] || eff <= p.k) {  // (see OrderMap's use below: NaN)
               omin = min(omin, float_order(x[e]));
               omax = max(omax, float_order(x[e]));
             }
@@ -611,7 +611,7 @@ li_topk_kernel(TopkParams p) {
     even.set(order_float(omin), order_float(omax));
     OrderMap map;
     map.set(omin, omax);
-    map.top = 0xff800000u;  // (NaN: bin 0)
+    if (eff > p.k) map.top = 0xff800000u;  // (NaN is not selected before numbers, but in a row that is selected whole it comes first)
     auto order = [&](auto&& bin) {  // true: the result is written
       constexpr int kPer = kListCap / kTopkThreads;
       unsigned int where[kPer];  // bin, and which of its keys

@@ -411,3 +411,14 @@ def test_uneven_scores_need_no_radix_select(kind, rows, n, sort):
     if not sort:
         got, want = got.sort(dim=1).values, want.sort(dim=1).values
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("n", [1, 700, 1999, 2048])
+def test_nan_comes_first_in_a_row_that_is_selected_whole(n):
+    g = torch.Generator().manual_seed(n)
+    sc = torch.randn(2, 2048, generator=g)
+    sc[0, n // 2], sc[1, n - 1] = float("nan"), float("inf")
+    out = torch.zeros((2, 1, 2048), dtype=torch.int32, device=DEV)
+    pto.lightning_indexer_topk(sc.to(DEV), torch.full((2,), n, dtype=torch.int32, device=DEV), out, 1, 2048)
+    want = sc[:, :n].sort(dim=1, descending=True, stable=True).indices
+    assert torch.equal(out.cpu()[:, 0, :n].long(), want) and torch.all(out[:, 0, n:] == -1)
