@@ -14,9 +14,12 @@
 // row (one TMEM lane = one key), apply ReLU/2^-11/fp16 rounding and the weighted head sum, and write the fp32 score.
 // With two and more query tokens per pass the head sum is a second product (kLiQuantTc): the epilogue writes the fp16
 // values back over the accumulator, tcgen05.mma kind::f16 takes them as its A operand from TMEM (K = 64 heads), B is the
-// weights, and what comes back is the key's score. The weights of a token are fp32: B holds them as three fp16 limbs (33 bits below the token's largest weight, scaled to
-// 2^13 by a power of two). The tensor core truncates where it adds, so a column of the product takes sixteen heads of one
-// limb (one step of K; zeros elsewhere) and its twelve columns are added here. On
+// weights, and what comes back is the key's score. The weights of a token are fp32, scaled to 2^13 by a power of two: B holds
+// them as three fp16 limbs. The tensor core truncates where it adds, so a column of the product takes sixteen heads of one limb
+// (one step of K; zeros elsewhere), its twelve columns are added here, and the first limb has six bits, multiples of 2^8 for
+// all heads: its products, which are the large ones, share a grid that the sum has room for. (With 11 bits, each limb as many of
+// a weight as it could hold, the scores were a third further from 64 bits than the fp32 sum on CUDA cores, and too small: relative error 6.7e-8 rms with a mean of -2.0e-8,
+// now 3.8e-8 without one, the fp32 sum 5.1e-8. Of a weight below 2^-7 of the token's largest the limbs hold 22 bits.) On
 // CUDA cores the head sum was the kernel's bound: unpacking the fp16 values and the multiply-adds were 1.5 of its 3.5
 // instructions per (key, head) and kept the half-rate FP16 / packed-FP32 pipe 70 % busy (16 x 65536 keys, two query
 // tokens 39.6 -> 37.4 us, four 66.0 -> 59.0; 256 tokens over 65536 keys 230 -> 192 us). With one query token the key
@@ -154,7 +157,7 @@ __device__ __forceinline__ float limb_sum(const uint32_t (&r)[16]) {
   for (int l = 0; l < 3; ++l) {
     v[l] = (__uint_as_float(r[4 * l]) + __uint_as_float(r[4 * l + 1])) + (__uint_as_float(r[4 * l + 2]) + __uint_as_float(r[4 * l + 3]));
   }
-  return fmaf(fmaf(v[2], 1.0f / 2048.0f, v[1]), 1.0f / 2048.0f, v[0]);
+  return fmaf(fmaf(v[2], 1.0f / 2048.0f, v[1]), 1.0f / 128.0f, v[0]);
 }
 
 // The older formulation for 32 heads of one key: table entries come in pairs, (q_scale_2p, q_scale_2p+1) and
@@ -373,12 +376,13 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
         const int ex = max(-100, min(127, static_cast<int>(m >> 23) - 127));  // 2^ex <= largest weight < 2^(ex + 1)
         float r = ctl->ws[e] * __int_as_float((127 + 13 - ex) << 23);
 #pragma unroll
-        for (int l = 0; l < 3; ++l) {  // exact splitting: what a limb leaves over, scaled up by 2^11, goes to the next
-          const __half w = __float2half_rn(r);
+        for (int l = 0; l < 3; ++l) {  // exact splitting: what a limb leaves over, scaled up by 2^7 or 2^11, goes to the next
+          // (the first: multiples of 2^8)
+          const __half w = __float2half_rn(l == 0 ? __fsub_rn(__fadd_rn(r, 3221225472.0f), 3221225472.0f) : r);
           // row (limb, sixteen heads) of 128 bytes (64 heads), 128-byte swizzle
           const int rw = l * 4 + (h >> 4);
           *reinterpret_cast<__half*>(smem + kLiSmemLimbs + i * kLimbBytes + rw * 128 + (((h >> 3) ^ (rw & 7)) << 4) + (h & 7) * 2) = w;
-          r = (r - __half2float(w)) * 2048.0f;
+          r = (r - __half2float(w)) * (l == 0 ? 128.0f : 2048.0f);
         }
         if (h == 0) ctl->winv[i] = __int_as_float((127 + ex - 13) << 23);
         fence_proxy_async();

@@ -231,6 +231,38 @@ def test_head_weights_of_very_different_size(s1, spread):
         torch.testing.assert_close(got[ti, :n], want[ti, :n], rtol=3e-6, atol=float(want[ti, :n].abs().max()) * 1e-6)
 
 
+@pytest.mark.parametrize("s1", [2, 4])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("spread", [0, 6, 12])
+def test_head_sum_is_no_further_from_64_bits_than_an_fp32_sum(s1, dtype, spread):
+    """The head sum on the tensor cores (two and more query tokens) against the fp32 sum on CUDA cores (one), over the same rows:
+    root mean square error and mean error, relative to the sum of the terms' sizes."""
+    d = gen.make_inputs([6000, 900], s1=s1, seed=80 + spread, with_attention=False, scale_dtype=dtype).to(DEV)
+    g = torch.Generator(device=DEV).manual_seed(spread)
+    small = torch.pow(2.0, -torch.randint(0, spread + 1, d.idx_weight.shape, generator=g, device=DEV).float())
+    d.idx_weight = (d.idx_weight.float().abs() * small).to(dtype)
+
+    def scores(act, table):
+        sc = torch.zeros((d.t, d.max_blocks * 128), device=DEV)
+        pto.lightning_indexer_scores(d.idx_query, d.idx_query_scale, d.idx_key_cache, d.idx_key_scale, d.idx_weight, act, table, sc)
+        return sc.double()
+
+    tc = scores(d.act_seq_key, d.block_table)
+    fp32 = scores(d.act_seq_key.repeat_interleave(s1), d.block_table.repeat_interleave(s1, 0).contiguous())
+    err = {"tc": [], "fp32": []}
+    for ti in range(d.t):
+        pos = torch.arange(d.act_seq[ti // s1], device=DEV)
+        rows = d.block_table[ti // s1].long()[pos // 128] * 128 + pos % 128
+        dots = torch.relu(d.idx_key_cache.reshape(-1, 128)[rows].double() @ d.idx_query[ti].double().T)
+        h = (dots / 2048).to(torch.float16).double()
+        want = (h @ (d.idx_query_scale[ti] * d.idx_weight[ti]).double()) * d.idx_key_scale.reshape(-1)[rows].double()
+        for name, got in (("tc", tc), ("fp32", fp32)):
+            err[name].append((got[ti, :pos.numel()] - want) / want.clamp(min=1e-30))
+    tc_err, fp32_err = torch.cat(err["tc"]), torch.cat(err["fp32"])
+    assert float(tc_err.square().mean().sqrt()) <= float(fp32_err.square().mean().sqrt())
+    assert abs(float(tc_err.mean())) <= 2.0 ** -28  # no truncation towards zero (rounding alone: 2^-25 over the root of 13800)
+
+
 @pytest.mark.parametrize("s1", [3, 4])
 def test_three_and_four_query_tokens_with_many_pages_per_cta(s1):
     """s1 = 3, 4 leave room for two accumulator slots only; with more than four pages per CTA every slot is
