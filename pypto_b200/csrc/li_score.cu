@@ -382,7 +382,8 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
           // row (limb, sixteen heads) of 128 bytes (64 heads), 128-byte swizzle
           const int rw = l * 4 + (h >> 4);
           *reinterpret_cast<__half*>(smem + kLiSmemLimbs + i * kLimbBytes + rw * 128 + (((h >> 3) ^ (rw & 7)) << 4) + (h & 7) * 2) = w;
-          r = (r - __half2float(w)) * (l == 0 ? 128.0f : 2048.0f);
+          // (nothing is left over of an infinite weight: its product decides alone, as in a sum of fp32 products)
+          r = __hisinf(w) != 0 ? 0.f : (r - __half2float(w)) * (l == 0 ? 128.0f : 2048.0f);
         }
         if (h == 0) ctl->winv[i] = __int_as_float((127 + ex - 13) << 23);
         fence_proxy_async();

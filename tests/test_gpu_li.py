@@ -263,6 +263,19 @@ def test_head_sum_is_no_further_from_64_bits_than_an_fp32_sum(s1, dtype, spread)
     assert abs(float(tc_err.mean())) <= 2.0 ** -28  # no truncation towards zero (rounding alone: 2^-25 over the root of 13800)
 
 
+@pytest.mark.parametrize("s1", [1, 2, 4])
+def test_infinite_head_weights(s1):
+    """A weight that overflowed decides the scores of the keys that its head sees, and only those, as in the CUDA-core sum."""
+    d = gen.make_inputs([700, 600], s1=s1, seed=66, with_attention=False)
+    d.idx_weight[0, 3] = float("inf")
+    d.idx_weight[-1, 40] = float("-inf")
+    got, want = _scores(d, False)[0], _scores(d, True)[0]
+    for ti in range(d.t):
+        a, b = (v[ti, :d.act_seq[ti // s1]] for v in (got, want))
+        torch.testing.assert_close(a, b, rtol=3e-6, atol=float(b.nan_to_num(0, 0, 0).abs().max()) * 1e-6, equal_nan=True)
+        assert bool(torch.isinf(a).any()) == (ti in (0, d.t - 1))
+
+
 @pytest.mark.parametrize("s1", [3, 4])
 def test_three_and_four_query_tokens_with_many_pages_per_cta(s1):
     """s1 = 3, 4 leave room for two accumulator slots only; with more than four pages per CTA every slot is
