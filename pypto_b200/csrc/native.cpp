@@ -76,8 +76,10 @@ class Call {
   int dev_ = -1;
 };
 
-// The current stream's workspace if it exists and is large enough.
-bool find_workspace(const Call& c, size_t bytes, void** ws, size_t* have, cudaStream_t* stream) {
+// The current stream's workspace if it exists and is large enough. `*ws` is a reference of the caller's own: another thread on
+// the same stream that needs a larger workspace replaces the entry as soon as the interpreter lock is let go, and with the
+// entry goes the last other reference.
+bool find_workspace(const Call& c, size_t bytes, at::Tensor* ws, cudaStream_t* stream) {
   const cudaStream_t s = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(c.device())).stream();
   PyObject* key = Py_BuildValue("(iK)", c.device(), static_cast<unsigned long long>(reinterpret_cast<uintptr_t>(s)));
   if (key == nullptr) {
@@ -92,8 +94,7 @@ bool find_workspace(const Call& c, size_t bytes, void** ws, size_t* have, cudaSt
   }
   const at::Tensor& w = THPVariable_Unpack(t);
   if (static_cast<size_t>(w.numel()) < bytes) return false;
-  *ws = w.data_ptr();
-  *have = static_cast<size_t>(w.numel());
+  *ws = w;
   *stream = s;
   return true;
 }
@@ -101,16 +102,17 @@ bool find_workspace(const Call& c, size_t bytes, void** ws, size_t* have, cudaSt
 // Runs `f(workspace, bytes, stream)` on the call's device without the interpreter lock.
 template <typename F>
 PyObject* launch(const Call& c, size_t bytes, F&& f) {
-  void* ws = nullptr;
-  size_t have = 0;
+  at::Tensor ws;  // (let go with the lock held, after the last use)
   cudaStream_t stream = nullptr;
-  if (!c.ok() || c.device() < 0 || !find_workspace(c, bytes, &ws, &have, &stream)) Py_RETURN_FALSE;
+  if (!c.ok() || c.device() < 0 || !find_workspace(c, bytes, &ws, &stream)) Py_RETURN_FALSE;
+  void* const base = ws.data_ptr();
+  const size_t have = static_cast<size_t>(ws.numel());
   int rc = 0;
   Py_BEGIN_ALLOW_THREADS;
   const auto before = c10::cuda::current_device();
   const bool other = before != c.device();
   if (other) c10::cuda::set_device(static_cast<c10::DeviceIndex>(c.device()));
-  rc = f(ws, have, reinterpret_cast<pto_stream_t>(stream));
+  rc = f(base, have, reinterpret_cast<pto_stream_t>(stream));
   if (other) c10::cuda::set_device(before);
   Py_END_ALLOW_THREADS;
   if (rc != 0) {
