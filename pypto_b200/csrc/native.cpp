@@ -10,7 +10,7 @@
 #include <Python.h>
 
 #include <ATen/core/Tensor.h>
-#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -99,7 +99,20 @@ bool find_workspace(const Call& c, size_t bytes, at::Tensor* ws, cudaStream_t* s
   return true;
 }
 
-// Runs `f(workspace, bytes, stream)` on the call's device without the interpreter lock.
+// Lets go of the interpreter lock for a scope; an exception takes it again on its way out.
+class WithoutLock {
+ public:
+  WithoutLock() : state_(PyEval_SaveThread()) {}
+  ~WithoutLock() { PyEval_RestoreThread(state_); }
+  WithoutLock(const WithoutLock&) = delete;
+  WithoutLock& operator=(const WithoutLock&) = delete;
+
+ private:
+  PyThreadState* state_;
+};
+
+// Runs `f(workspace, bytes, stream)` on the call's device without the interpreter lock. Throws, if at all, before `f`: what has
+// been enqueued is not enqueued again by the caller's other path.
 template <typename F>
 PyObject* launch(const Call& c, size_t bytes, F&& f) {
   at::Tensor ws;  // (let go with the lock held, after the last use)
@@ -108,13 +121,11 @@ PyObject* launch(const Call& c, size_t bytes, F&& f) {
   void* const base = ws.data_ptr();
   const size_t have = static_cast<size_t>(ws.numel());
   int rc = 0;
-  Py_BEGIN_ALLOW_THREADS;
-  const auto before = c10::cuda::current_device();
-  const bool other = before != c.device();
-  if (other) c10::cuda::set_device(static_cast<c10::DeviceIndex>(c.device()));
-  rc = f(base, have, reinterpret_cast<pto_stream_t>(stream));
-  if (other) c10::cuda::set_device(before);
-  Py_END_ALLOW_THREADS;
+  {
+    const WithoutLock without_lock;
+    const c10::cuda::CUDAGuard device(static_cast<c10::DeviceIndex>(c.device()));  // (its destructor does not throw)
+    rc = f(base, have, reinterpret_cast<pto_stream_t>(stream));
+  }
   if (rc != 0) {
     PyObject* r = PyObject_CallFunction(g_check, "i", rc);  // raises
     Py_XDECREF(r);
