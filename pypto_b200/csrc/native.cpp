@@ -14,6 +14,8 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <cuda_runtime_api.h>
+
 #include <exception>
 
 // (the C declarations take a cudaStream_t through pto_stream_t)
@@ -81,6 +83,8 @@ class Call {
 // entry goes the last other reference.
 bool find_workspace(const Call& c, size_t bytes, at::Tensor* ws, cudaStream_t* stream) {
   const cudaStream_t s = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(c.device())).stream();
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;  // (a workspace that a capture records is kept: `ops._workspace`)
+  if (cudaStreamIsCapturing(s, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return false;
   PyObject* key = Py_BuildValue("(iK)", c.device(), static_cast<unsigned long long>(reinterpret_cast<uintptr_t>(s)));
   if (key == nullptr) {
     PyErr_Clear();

@@ -37,19 +37,36 @@ class CapturedCall:
         self.device = dev
         self._keep = (args, kwargs)  # the graph reads and writes these buffers: keep them alive
         self._stream = torch.cuda.Stream(dev)
-        self._stream.wait_stream(torch.cuda.current_stream(dev))
-        with torch.cuda.stream(self._stream):
-            op(*args, **kwargs)  # warm-up: creates the workspace of this stream, outside the capture
-        torch.cuda.current_stream(dev).wait_stream(self._stream)
-        torch.cuda.synchronize(dev)
-        self.graph = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(self.graph, stream=self._stream):
-            op(*args, **kwargs)
+        # The graph holds the address of its workspace, so the workspace is this object's own: stream handles come from a small
+        # pool, and the table's entry for this one belongs to whoever else calls operators on it, or records another call.
+        key = (dev.index, self._stream.cuda_stream)
+        others = ops._workspaces.pop(key, None)
+        self._workspace = None
+        try:
+            self._stream.wait_stream(torch.cuda.current_stream(dev))
+            with torch.cuda.stream(self._stream):
+                op(*args, **kwargs)  # warm-up: creates the workspace, outside the capture
+            torch.cuda.current_stream(dev).wait_stream(self._stream)
+            torch.cuda.synchronize(dev)
+            self.graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(self.graph, stream=self._stream):
+                op(*args, **kwargs)
+        finally:
+            self._workspace = ops._workspaces.pop(key, None)
+            if self._workspace is not None:
+                ops._recorded.pop(self._workspace.data_ptr(), None)
+            if others is not None:
+                ops._workspaces[key] = others
+        self._replayed_on = set()
 
     def replay(self):
+        stream = torch.cuda.current_stream(self.device)
+        if self._workspace is not None and stream.cuda_stream not in self._replayed_on:
+            self._replayed_on.add(stream.cuda_stream)
+            self._workspace.record_stream(stream)  # its memory is not reused before the replays there, whenever it is freed
         self.graph.replay()
 
     def workspace_status(self):
-        """Device status words of the captured call's workspace (synchronises the capture stream)."""
-        with torch.cuda.stream(self._stream):
-            return ops.workspace_status(self.device)
+        """Device status words of the captured call's workspace (synchronises the device's current stream)."""
+        with torch.cuda.device(self.device):
+            return ops.workspace_status(self.device, self._workspace)

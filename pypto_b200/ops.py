@@ -26,6 +26,8 @@ from .compat import Tensor as _Handle
 from .compat import unwrap
 
 _workspaces: Dict[Tuple[int, int], torch.Tensor] = {}
+# workspaces whose address a stream capture has recorded, by address: they stay when a larger one takes their place above
+_recorded: Dict[int, torch.Tensor] = {}
 
 try:
     # the same checks and the same call in native code for an ordinary call; a function of it that returns False has done
@@ -43,14 +45,16 @@ def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     if ws is None or ws.numel() < nbytes:
         ws = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
         _workspaces[key] = ws
+    if torch.cuda.is_current_stream_capturing():
+        _recorded[ws.data_ptr()] = ws
     return ws
 
 
-def workspace_status(device=None):
-    """Status words of the current stream's workspace (synchronises the stream).
+def workspace_status(device=None, workspace=None):
+    """Status words of the current stream's workspace, or of `workspace` (synchronises the stream).
     Word 0 is an OR of PTO_ST_BAD_PAGE / PTO_ST_WAIT_EXPIRED."""
     device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
-    ws = _workspace(device, 256)
+    ws = _workspace(device, 256) if workspace is None else workspace
     out = (C.c_int32 * _lib.PTO_STATUS_WORDS)()
     _lib.check(_lib.load().pto_workspace_status(ws.data_ptr(), out, torch.cuda.current_stream(device).cuda_stream))
     return list(out)

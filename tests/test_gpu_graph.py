@@ -4,6 +4,7 @@ import pytest
 import torch
 
 import pypto_b200 as pto
+from pypto_b200 import ops
 from pypto_b200 import inputs as gen
 
 pytestmark = pytest.mark.gpu
@@ -110,3 +111,64 @@ def test_captured_prolog_then_decode_layer():
     torch.cuda.synchronize()
     assert not torch.equal(q_nope, want[0])
     assert torch.cuda.memory_allocated() == base
+
+
+def _decode(lens, seed):
+    d = gen.make_inputs(lens, s1=1, seed=seed).to(DEV)
+    idx = torch.zeros((d.t, 1, 2048), dtype=torch.int32, device=DEV)
+    return d, idx, torch.zeros((d.b, d.s1, 128, 512), dtype=torch.bfloat16, device=DEV)
+
+
+def test_recorded_call_owns_its_workspace():
+    """Stream handles come from a pool of 32: two recorded calls and an eager one may share a handle, never a workspace. The
+    first call's replays are not disturbed by a larger call on its stream and by what is allocated then."""
+    small, idx, out = _decode([300] * 40, 31)
+    steps = [pto.CapturedCall(pto.decode_indexer_attention_quant, *_args(small, idx, out), sort=True) for _ in range(34)]
+    handles = [s._stream.cuda_stream for s in steps]
+    assert len(set(handles)) < len(handles)
+    assert len({s._workspace.data_ptr() for s in steps}) == len(steps)
+    step = steps[0]
+    idx.fill_(-7)
+    step.replay()
+    torch.cuda.synchronize()
+    want = idx.clone(), out.clone()
+    large, idx_l, out_l = _decode([20000] * 40, 32)
+    with torch.cuda.stream(step._stream):
+        pto.decode_indexer_attention_quant(*_args(large, idx_l, out_l), sort=True)
+        other = [torch.full((n,), 0x5A, dtype=torch.uint8, device=DEV) for n in (1 << 20, 1 << 21, 1 << 22, 1 << 23)]
+    torch.cuda.synchronize()
+    idx.fill_(-7)
+    out.fill_(3.0)
+    step.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(idx, want[0]) and torch.equal(out, want[1])
+    assert all(bool((o == 0x5A).all()) for o in other)
+    assert step.workspace_status()[0] == 0
+
+
+def test_workspace_recorded_by_a_plain_capture_is_kept():
+    """The same for a capture that the caller makes without `CapturedCall`: a larger call on the stream takes another workspace,
+    and the recorded one stays allocated."""
+    small, idx, out = _decode([300] * 40, 33)
+    side = torch.cuda.Stream()
+    key = (torch.cuda.current_device(), side.cuda_stream)
+    ops._workspaces.pop(key, None)  # (the handle may have been someone else's)
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        pto.decode_indexer_attention_quant(*_args(small, idx, out), sort=True)
+    torch.cuda.synchronize()
+    want = idx.clone(), out.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        pto.decode_indexer_attention_quant(*_args(small, idx, out), sort=True)
+    recorded = ops._workspaces[key].data_ptr()
+    large, idx_l, out_l = _decode([20000] * 40, 34)
+    with torch.cuda.stream(side):
+        pto.decode_indexer_attention_quant(*_args(large, idx_l, out_l), sort=True)
+    assert ops._workspaces[key].data_ptr() != recorded
+    assert recorded in ops._recorded
+    torch.cuda.synchronize()
+    idx.fill_(-7)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(idx, want[0]) and torch.equal(out, want[1])
