@@ -293,6 +293,7 @@ int run_sfa(const void* qn, const void* qr, const void* kn, const void* kr, cons
   PTO_REQUIRE(nq_total >= nq && head_begin >= 0 && head_begin + nq <= nq_total, "head slice [%d, %d) of %d", head_begin,
               head_begin + nq, nq_total);
   PTO_REQUIRE(topk >= 1 && block_size >= 1 && max_blocks >= 1 && n_rows >= 1, "topk/block_size/max_blocks/n_rows");
+  PTO_REQUIRE(n_rows <= INT_MAX, "n_rows %lld: the kernels hold a row's number in 32 bits", static_cast<long long>(n_rows));
   PTO_REQUIRE(softmax_scale > 0.f, "softmax_scale %f", softmax_scale);
   PTO_REQUIRE(aligned16(qn) && aligned16(qr) && aligned16(kn) && aligned16(out) &&
                   (packed || (aligned16(kr) && (bf16 || aligned16(sc)))),

@@ -4,6 +4,7 @@ import pytest
 import torch
 
 import pypto_b200 as pto
+from pypto_b200 import _lib
 from pypto_b200 import inputs as gen
 
 
@@ -159,3 +160,19 @@ def test_nonquant_prolog_rejects_bad_arguments_before_any_launch():
         call(cache_index=p["cache_index"].to(torch.int32))
     with pytest.raises(ValueError, match="PA_BSND"):
         call(1e-5, 1e-5, "BSND")
+
+
+PTO_ERR_INVALID = -1
+
+
+def _refusal(entry, *args):
+    """Return code and message of a C entry point that refuses its arguments before it touches a device (pointers are never read)."""
+    lib = _lib.load()
+    return getattr(lib, entry)(*args), lib.pto_last_error().decode()
+
+
+@pytest.mark.parametrize("entry,pointers", [("pto_sfa_quant", 9), ("pto_sfa_bf16", 8), ("pto_sfa_packed", 7)])
+def test_caches_of_more_rows_than_a_row_number_holds_are_refused(entry, pointers):
+    args = [0x10000] * pointers + [1, 1, 128, 1, 0.04, 2048, 128, 2 ** 31, 4, 128, 0, 0x10000, 1 << 30, None]
+    rc, message = _refusal(entry, *args)
+    assert rc == PTO_ERR_INVALID and "n_rows" in message
