@@ -176,3 +176,13 @@ def test_caches_of_more_rows_than_a_row_number_holds_are_refused(entry, pointers
     args = [0x10000] * pointers + [1, 1, 128, 1, 0.04, 2048, 128, 2 ** 31, 4, 128, 0, 0x10000, 1 << 30, None]
     rc, message = _refusal(entry, *args)
     assert rc == PTO_ERR_INVALID and "n_rows" in message
+
+
+@pytest.mark.parametrize("which", ["hadamard_q", "hadamard_k"])
+def test_unaligned_hadamard_matrices_are_refused(which):
+    """Both are read sixteen bytes at a time."""
+    pointers = [0x10000] * 31
+    pointers[{"hadamard_q": 20, "hadamard_k": 21}[which]] += 2
+    pointers[29] = None  # w_x_packed
+    rc, message = _refusal("pto_mla_indexer_prolog_quant", *pointers, 4, 7168, 1536, 128, 1e-5, 1e-5, 1e-6, 0x10000, 1 << 30, None)
+    assert rc == PTO_ERR_INVALID and "aligned" in message
