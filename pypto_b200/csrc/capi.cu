@@ -256,7 +256,7 @@ bool li_hist_usable(int s1, int flags) {
 }
 
 int run_li_topk(const float* scores, int64_t row_stride, const int32_t* act, int32_t* out, int b, int s1, int k,
-                int flags, int32_t* status, cudaStream_t stream, const unsigned int* hist = nullptr) {
+                int flags, int32_t* status, cudaStream_t stream, const unsigned int* hist = nullptr, bool behind_scores = true) {
   PTO_REQUIRE(k >= 1 && k <= pto::topk_max_k(), "selected_count %d outside [1, %d]", k, pto::topk_max_k());
   PTO_REQUIRE(row_stride % 4 == 0 && aligned16(scores), "score rows must be 16-byte aligned");
   pto::TopkParams p{};
@@ -273,7 +273,7 @@ int run_li_topk(const float* scores, int64_t row_stride, const int32_t* act, int
   DeviceInfo di;
   const int rc = get_device_info(&di);
   if (rc != PTO_OK) return rc;
-  PTO_CUDA(pto::launch_li_topk(p, di.num_sms, stream));
+  PTO_CUDA(pto::launch_li_topk(p, di.num_sms, stream, behind_scores));
   return PTO_OK;
 }
 
@@ -617,7 +617,7 @@ int pto_li_topk(const float* scores, int64_t row_stride, const int32_t* act_seq_
   int rc = check_workspace(workspace, workspace_bytes, kStatusBytes);
   if (rc != PTO_OK) return rc;
   return run_li_topk(scores, row_stride, act_seq_key, topk_res, b, s1, selected_count, flags,
-                     reinterpret_cast<int32_t*>(workspace), stream);
+                     reinterpret_cast<int32_t*>(workspace), stream, nullptr, /*behind_scores=*/false);
 }
 
 int pto_li_decode(const int8_t* idx_query, const void* idx_query_scale, const int8_t* idx_key_cache,

@@ -348,7 +348,7 @@ struct SfaParams {
 cudaError_t launch_li_score_tc(const LiParams& p, const void* tmap_k, const void* tmap_q, int num_sms,
                                cudaStream_t stream);
 cudaError_t launch_li_score_simt(const LiParams& p, cudaStream_t stream);
-cudaError_t launch_li_topk(const TopkParams& p, int num_sms, cudaStream_t stream);
+cudaError_t launch_li_topk(const TopkParams& p, int num_sms, cudaStream_t stream, bool pdl);  // pdl: behind its score kernel
 cudaError_t launch_sfa(const SfaParams& p, int num_sms, cudaStream_t stream);
 cudaError_t launch_sfa_pair(const SfaParams& p, cudaStream_t stream);     // nq == 128, any cache format: 2-SM MMAs, heads split over the pair
 int sfa_pair_split(int t, int num_sms);

@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(kTopkThreads, 1)
 li_topk_kernel(TopkParams p) {
   extern __shared__ __align__(16) uint8_t topk_smem_raw[];
   TopkSmem* sm = reinterpret_cast<TopkSmem*>(topk_smem_raw);
-  // launched with programmatic serialization: the score kernel before it may still be running
+  // with programmatic serialization the score kernel before it may still be running
   TKT(0);
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
@@ -735,7 +735,7 @@ li_topk_kernel(TopkParams p) {
 
 }  // namespace
 
-cudaError_t launch_li_topk(const TopkParams& p, int num_sms, cudaStream_t stream) {
+cudaError_t launch_li_topk(const TopkParams& p, int num_sms, cudaStream_t stream, bool pdl) {
   cudaError_t e = cudaFuncSetAttribute(li_topk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(sizeof(TopkSmem)));
   if (e != cudaSuccess) return e;
@@ -754,11 +754,12 @@ cudaError_t launch_li_topk(const TopkParams& p, int num_sms, cudaStream_t stream
   attr[0].val.clusterDim.x = static_cast<unsigned>(csize);
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
-  // may be scheduled while the kernel before it drains; it waits (first instruction) before it reads anything
+  // behind the score kernel of the same call: may be scheduled while that drains, and reads only the row's length, which is no
+  // result of it, before it waits. Behind a kernel of somebody else's, which may have written the lengths: the ordinary way
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 2;
+  cfg.numAttrs = pdl ? 2 : 1;
   count_launch();
   return cudaLaunchKernelEx(&cfg, li_topk_kernel, p);
 }
