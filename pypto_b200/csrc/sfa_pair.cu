@@ -42,14 +42,6 @@ namespace pto {
 
 namespace {
 
-// Developer aid: -DPTO_PAIR_TIMELINE records clock64() at 16 points of the first 24 tiles of cluster 0.
-#ifdef PTO_PAIR_TIMELINE
-__device__ long long g_pair_tl[2 * 24 * 16];
-#define TLP(slot, j) do { if (blockIdx.x < 2 && (j) >= 0 && (j) < 24) g_pair_tl[((blockIdx.x & 1) * 24 + (j)) * 16 + (slot)] = clock64(); } while (0)
-#else
-#define TLP(slot, j) do { } while (0)
-#endif
-
 constexpr int kPT = 128;                 // selected rows per tile (64 per CTA)
 constexpr int kPRows = 64;               // rows a CTA gathers in full width per tile; also heads per CTA
 constexpr int kChunk = kPRows * 128;     // 64 rows x 64 bf16 (128-byte rows, 128-byte swizzle): 8 KB
@@ -226,7 +218,6 @@ __device__ __forceinline__ uint32_t pair_setup_sync(PairCtl* ctl) {
   // the kernel behind this one (the merge of the split partials) may be scheduled from here on; it waits for
   // this grid to complete before it reads anything
   if (threadIdx.x == 0) pdl_trigger();
-  if (threadIdx.x == 0) TLP(1, 20);  // roles start
   return ctl->tmem_base;
 }
 
@@ -293,7 +284,6 @@ __device__ __forceinline__ void pair_role_issue_qk(const SfaParams& p, PairCtx c
   ok = ok && pair_poll(smem_u32(&ctl->kfull[q]), ph) && pair_poll(smem_u32(&ctl->kpeer[q]), ph);                \
   if (!ok) break;                                                                                               \
   tc_fence_after();                                                                                             \
-  if ((q) == 0 && (threadIdx.x & 31) == 0) TLP(6, j);                                                           \
   if (elect_one()) {                                                                                            \
     pair_issue_qk_half<q>(d, a_desc, b_desc);                                                                \
     tc2_commit(smem_u32(&ctl->kfree[q]));                                                                       \
@@ -303,7 +293,6 @@ __device__ __forceinline__ void pair_role_issue_qk(const SfaParams& p, PairCtx c
     PAIR_QK_HALF(0)
     PAIR_QK_HALF(1)
 #undef PAIR_QK_HALF
-    if ((threadIdx.x & 31) == 0) TLP(7, j);
   }
   if (!ok && (threadIdx.x & 31) == 0) {
     ctl->abort = 1;
@@ -344,7 +333,6 @@ __device__ __forceinline__ void pair_role_issue_pv(const SfaParams& p, PairCtx c
   ok = ok && pair_poll(smem_u32(&ctl->vfull[q]), ph) && pair_poll(smem_u32(&ctl->vpeer[q]), ph);                \
   if (!ok) break;                                                                                               \
   tc_fence_after();                                                                                             \
-  if ((q) == 0 && (threadIdx.x & 31) == 0) TLP(8, j);                                                           \
   if (elect_one()) {                                                                                            \
     pair_issue_pv_quarter<q>(tmem_base + kPairColO, a_desc, b_desc, j > 0 ? 1u : 0u);                           \
     tc2_commit(smem_u32(&ctl->vfree[q]));                                                                       \
@@ -356,7 +344,6 @@ __device__ __forceinline__ void pair_role_issue_pv(const SfaParams& p, PairCtx c
     PAIR_PV_QUARTER(2)
     PAIR_PV_QUARTER(3)
 #undef PAIR_PV_QUARTER
-    if ((threadIdx.x & 31) == 0) TLP(9, j);
   }
   if (!ok && (threadIdx.x & 31) == 0) {
     ctl->abort = 1;
@@ -421,7 +408,6 @@ __device__ __forceinline__ void pair_role_softmax(const SfaParams& p, PairCtx c)
   const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(sub * 32) << 16);
   const uint32_t p_row = c.base + kSmemP + kh * kChunk + head * 128;
   const int psw = head & 7;
-  const bool tl = threadIdx.x == 32 * kPairSoftmaxWarp0;
   float m_seen = -INFINITY;  // the head's reference max (identical in its four threads)
   float l_run = 0.f;         // this thread's share of the row sum
   bool ok = true;
@@ -435,7 +421,6 @@ __device__ __forceinline__ void pair_role_softmax(const SfaParams& p, PairCtx c)
     const int b = j & 1;
     ok = pair_group_wait<1, 256>(ctl, nwait, smem_u32(&ctl->sfull[b]), (j >> 1) & 1, first_warp);
     if (!ok) break;
-    if (tl) TLP(10, j);
     tc_fence_after();
     float s[32];
     {
@@ -472,9 +457,7 @@ __device__ __forceinline__ void pair_role_softmax(const SfaParams& p, PairCtx c)
       ls2[i & 1] += s[i];
     }
     const float lsum = ls2[0] + ls2[1];
-    if (tl) TLP(11, j);
     meet();
-    if (tl) TLP(12, j);
     const float mt = fmaxf(fmaxf(ctl->mt[b][0][head], ctl->mt[b][1][head]), fmaxf(ctl->mt[b][2][head], ctl->mt[b][3][head]));
     const float m_new = fmaxf(m_seen, mt);
     const bool need = (m_new > m_seen + kPairRescale) || (m_seen == -INFINITY && m_new > -INFINITY);
@@ -492,7 +475,6 @@ __device__ __forceinline__ void pair_role_softmax(const SfaParams& p, PairCtx c)
       if (!ok) break;
       tc_fence_after();
     }
-    if (tl) TLP(13, j);
     if (j > 0 && __any_sync(0xffffffffu, need)) {  // rare: rescale this thread's 128 output columns
 #pragma unroll 1
       for (int cc = 0; cc < 8; ++cc) {
@@ -519,11 +501,9 @@ __device__ __forceinline__ void pair_role_softmax(const SfaParams& p, PairCtx c)
     tc_fence_before();
     __syncwarp();
     if (lane == 0) mbar_arrive(smem_u32(&ctl->pfull));
-    if (tl) TLP(14, j);
   }
   // ---- output ---------------------------------------------------------------------------------------
   if (ok) ok = pair_group_wait<1, 256>(ctl, nwait, smem_u32(&ctl->pvdone), (ntiles - 1) & 1, first_warp);
-  if (tl) TLP(5, 20);  // last P.V complete
   float l_tot = 0.f;
   if (ok) {
     ctl->mt[ntiles & 1][slot][head] = l_run;
@@ -681,7 +661,6 @@ __device__ __forceinline__ void pair_role_kproducer(const SfaParams& p, const Pa
   bool ok = true;
   pair_setup_arrive();
   pdl_wait();          // the selected indices come from the kernel before this one, which may still be running
-  if (ptid == 0) TLP(3, 21);
   int row_cur;         // this lane's row of tile j
   int row_n;           // this lane's row of tile j+1
   int idx_a, entry_a;  // tile j+2
@@ -690,25 +669,20 @@ __device__ __forceinline__ void pair_role_kproducer(const SfaParams& p, const Pa
     const int idx0 = load_idx(0), idx1 = load_idx(1);
     idx_a = load_idx(2);
     idx_b = load_idx(3);
-    if (ptid == 0 && idx0 + idx1 + idx_a + idx_b != -12345) TLP(4, 21);
     const int e0 = tc_table_entry(p, bi, idx0);
     const int e1 = tc_table_entry(p, bi, idx1);
     entry_a = tc_table_entry(p, bi, idx_a);
-    if (ptid == 0 && e0 + e1 + entry_a != -12345) TLP(5, 21);
     row_cur = pair_row(p, idx0, e0);
     issue_loads(row_cur);
     if (kBf) prefetch_row(row_cur);
     row_n = pair_row(p, idx1, e1);
     prefetch_row(row_n);
-    if (ptid == 0) TLP(6, 21);
   }
-  if (!kBf && ptid == 0 && d[0][0].x != 0x7fffffffu) TLP(7, 21);  // first rows arrived
   for (int j = 0; j < ntiles; ++j) {
     if (j > 0) {  // the q.K^T MMAs of the previous tile that read this half of the chunks are complete
       ok = pair_wait(smem_u32(&ctl->kfree[half]), (j - 1) & 1);
       if (!ok) break;
     }
-    if (ptid == 0) TLP(0, j);
     if (half == 1) {  // the rope part goes straight from L2 to shared memory behind the conversion below
 #pragma unroll
       for (int m = 0; m < 4; ++m) {  // rows 4m + lane / 8 of the warp's 16
@@ -743,7 +717,6 @@ __device__ __forceinline__ void pair_role_kproducer(const SfaParams& p, const Pa
     if (j == 0) pair_setup_wait();
     __syncwarp();
     if (lane == 0) mbar_arrive(smem_u32(&ctl->kfull[half]));
-    if (ptid == 0) TLP(1, j);
     if (j + 1 < ntiles) issue_loads(row_n);  // the half rows of tile j+1 (in L2: prefetched a tile ago)
     row_cur = row_n;
     row_n = pair_row(p, idx_a, entry_a);     // tile j+2: into L2
@@ -815,7 +788,6 @@ __device__ __forceinline__ void pair_role_vproducer(const SfaParams& p, const Pa
       ok = pair_wait(smem_u32(&ctl->vfree[q]), (j - 1) & 1);
       if (!ok) break;
     }
-    if (vtid == 0) TLP(4, j);
 #pragma unroll
     for (int m = 0; m < 4; ++m) {  // row 4m + r4
       const int x = 4 * (m & 1) + r4;
@@ -841,7 +813,6 @@ __device__ __forceinline__ void pair_role_vproducer(const SfaParams& p, const Pa
     if (j == 0) pair_setup_wait();
     __syncwarp();
     if (lane == 0) mbar_arrive(smem_u32(&ctl->vfull[q]));
-    if (vtid == 0) TLP(5, j);
     if (j + 1 < ntiles) issue_loads(row_n);
     row_cur = row_n;
     row_n = pair_row(p, idx_a, entry_a);
@@ -863,7 +834,6 @@ sfa_pair_kernel(const __grid_constant__ SfaParams p) {
     if (threadIdx.x == 0) set_status(p.status, PTO_ST_WAIT_EXPIRED, static_cast<int>(base), 55);
     return;
   }
-  if (threadIdx.x == 0) TLP(0, 20);  // kernel entry
   PairCtx c;
   c.base = base;
   c.ctl = reinterpret_cast<PairCtl*>(sfa_pair_smem + kSmemCtl);
@@ -940,14 +910,12 @@ sfa_pair_kernel(const __grid_constant__ SfaParams p) {
     }
     ctl->abort = 0;
     fence_mbar_init();
-    TLP(0, 21);
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctl->tmem_base)),
                  "r"(kPairTmemCols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-    if (tid == 0) TLP(1, 21);
   }
   // (the producers go straight to their first rows)
   if (warp < kPairKWarp0) {
@@ -958,7 +926,6 @@ sfa_pair_kernel(const __grid_constant__ SfaParams p) {
       sts_v4u(base + kSmemQ + (u >> 3) * kChunk + r * 128 + (((u & 7) ^ (r & 7)) << 4), w[i]);
     }
     fence_proxy_async();
-    if (tid == 0) TLP(2, 21);
   }
   static_assert(12 * 32 * kPairKWarp0 == 64 * 72, "Q units per loader thread");
 
@@ -991,26 +958,17 @@ sfa_pair_kernel(const __grid_constant__ SfaParams p) {
 
   // ---- teardown: neither CTA may leave while the peer's MMAs can still read its shared memory --------
   // (nothing is kept in registers across the roles: what the teardown needs is read again)
-  if (threadIdx.x == 32 * kPairSoftmaxWarp0) TLP(2, 20);  // first softmax warp done with its output
   tc_fence_before();
   __syncthreads();
-  if (threadIdx.x == 0) TLP(3, 20);
   pair_cluster_sync();
   if ((threadIdx.x >> 5) == 0) {
     tc_fence_after();
     const uint32_t tmem = reinterpret_cast<const PairCtl*>(sfa_pair_smem + kSmemCtl)->tmem_base;
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kPairTmemCols) : "memory");
   }
-  if (threadIdx.x == 0) TLP(4, 20);  // exit
 }
 
 }  // namespace
-
-#ifdef PTO_PAIR_TIMELINE
-extern "C" int pto_debug_pair_timeline(long long* host, int n) {
-  return static_cast<int>(cudaMemcpyFromSymbol(host, g_pair_tl, sizeof(long long) * n));
-}
-#endif
 
 // split of a token's selected rows over clusters so that the grid fills the SM pairs once
 int sfa_pair_split(int t, int num_sms) {

@@ -32,15 +32,6 @@ namespace pto {
 
 namespace {
 
-// -DPTO_TOPK_TIMELINE: clock64 stamps of thread 0 of CTA 0 at the phase boundaries (development aid, read back
-// through pto_debug_topk_timeline; not part of the ABI)
-#ifdef PTO_TOPK_TIMELINE
-__device__ long long g_topk_tl[16];
-#define TKT(i) do { if (blockIdx.x == 0 && threadIdx.x == 0) g_topk_tl[i] = clock64(); } while (0)
-#else
-#define TKT(i) do { } while (0)
-#endif
-
 constexpr int kTopkThreads = 512;  // (1024 threads wait longer at each of the dozen barriers than they save between them)
 constexpr int kTopkWarps = kTopkThreads / 32;
 constexpr int kBins = 2048;
@@ -398,7 +389,6 @@ li_topk_kernel(TopkParams p) {
   extern __shared__ __align__(16) uint8_t topk_smem_raw[];
   TopkSmem* sm = reinterpret_cast<TopkSmem*>(topk_smem_raw);
   // with programmatic serialization the score kernel before it may still be running
-  TKT(0);
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
   const unsigned int csize = cluster_size();
@@ -429,7 +419,6 @@ li_topk_kernel(TopkParams p) {
   if (!whole && csize > 1) cluster_arrive();  // (rank 0's counter is set before anyone adds to it)
   pdl_wait();
   pdl_trigger();
-  TKT(1);
   if (rank == 0) {
     for (int j = max(k, 0) + tid; j < p.k; j += kTopkThreads) out[j] = -1;
   }
@@ -491,7 +480,6 @@ li_topk_kernel(TopkParams p) {
       __syncthreads();  // every thread has read the outcome before the histogram area is reused
     }
     if (!known) bound = sample_bound(sm, row, eff, k);
-    TKT(2);
     // ---- 2. this rank's keys at or above the bound ------------------------------------------------
     // One list for the CTA, in which a warp reserves its places chunk by chunk: however the selected positions lie in the row,
     // nothing but their number limits it. (With a list of its own for each warp, 384 places, a run of 385 neighbouring
@@ -555,7 +543,6 @@ li_topk_kernel(TopkParams p) {
       set_status(p.status, PTO_ST_WAIT_EXPIRED, row_id, 30);
       atomicAdd(&sm->n_mine, static_cast<unsigned int>(kListCap + 1));
     }
-    TKT(3);
     __syncthreads();
     // ---- the lists of all ranks, one behind the other, into rank 0's --------------------------------
     const unsigned int total = min(sm->n_mine, static_cast<unsigned int>(kListCap + 1));  // (what is spoilt stays spoilt)
@@ -598,7 +585,6 @@ li_topk_kernel(TopkParams p) {
       }
     }
   }
-  TKT(4);
 
   // ---- 3. order ------------------------------------------------------------------------------------
   const bool good = n_list <= static_cast<unsigned int>(kListCap) && n_list >= static_cast<unsigned int>(k);  // (uniform)
@@ -624,7 +610,6 @@ li_topk_kernel(TopkParams p) {
         }
       }
       __syncthreads();
-      TKT(5);
       find_threshold_bin<kBins / kTopkThreads, true>(sm, static_cast<unsigned int>(k));
       // Bins that lie in the result whole need no order when the caller asked for none: only the keys of the others go to their
       // bin's place in `sorted`, to be ranked there.
@@ -661,7 +646,6 @@ li_topk_kernel(TopkParams p) {
         }
       }
       if (__syncthreads_or(crowded ? 1 : 0) != 0) return false;
-      TKT(6);
       // keys of the bins that reach into the result; without order, of the one bin that lies across its end
       const unsigned int n_sorted = sm->thr_above + sm->thr_count;
       if (!(unsorted && n_sorted == uk)) {
@@ -674,7 +658,6 @@ li_topk_kernel(TopkParams p) {
           if (at < uk) out[at] = key_pos(key);
         }
       }
-      TKT(7);
       return true;
     };
     if (whole && even.inv != 0.f) {
@@ -765,11 +748,5 @@ cudaError_t launch_li_topk(const TopkParams& p, int num_sms, cudaStream_t stream
 }
 
 int topk_max_k() { return kMaxK; }
-
-#ifdef PTO_TOPK_TIMELINE
-extern "C" int pto_debug_topk_timeline(long long* host, int n) {
-  return static_cast<int>(cudaMemcpyFromSymbol(host, g_topk_tl, sizeof(long long) * n));
-}
-#endif
 
 }  // namespace pto
