@@ -14,10 +14,11 @@
 //      into a list of up to 6144. It is split over a cluster of 1, 2, 4 or 8 CTAs (as many as keep the grid within one
 //      wave of SMs), each of which finds the bound for itself; the lists travel to rank 0 through distributed shared
 //      memory.
-//   3. Rank 0 distributes the list over 2048 bins that divide the range of its values' images, a prefix sum over the bins gives every bin
+//   3. Rank 0 distributes the list over 2048 bins that divide its value range, a prefix sum over the bins gives every bin
 //      its place in the order, and a key's place within its bin is the number of larger keys there (a bin holds a
 //      few keys). The first k places are the result; a caller that asked for no order gets the whole bins as they are.
-// A list that is too long or too short, or a bin of more than 512 keys (massive ties), sends the row to
+// Where one of either histogram's bins holds too much, the values are distributed once more, by their images (see OrderMap). A
+// list that is too long or too short all the same, or a bin of more than 512 keys then (massive ties), sends the row to
 // an MSB-first radix select over the 64-bit keys on rank 0.
 // What bounds it: one trip of the row from L2 (the first version scanned it three times, for its extremes, a histogram
 // and the collection, with a cluster barrier behind each, and ordered its result with a bitonic sort) and about a dozen
@@ -263,7 +264,7 @@ struct BinMap {
 // The same over the order-preserving images: equal widths within a power of two, and as many bins for each power of two of the
 // range. A few values far from the others (an outlier, a long tail, masked positions) leave the others spread over many bins,
 // where equal widths put all of them into one: 256 rows of 131072 with one value at 300 standard deviations 293 us, all of them
-// in the radix select, against 72 without it. What lies outside goes to the ends; images above `top` (NaN) to bin 0.
+// in the radix select, now 70. What lies outside goes to the ends; images above `top` (NaN) to bin 0.
 struct OrderMap {
   unsigned int lo, top;
   float scale;
@@ -291,69 +292,48 @@ __device__ __forceinline__ void block_range(TopkSmem* sm, unsigned int& omin, un
   omax = __reduce_max_sync(0xffffffffu, sm->red_max[lane & (kTopkWarps - 1)]);
 }
 
-// Lower bound of the k largest of row[0, eff) from a sample: 1024 groups of four (or a multiple of that), evenly spread. About
-// k + 4.5 standard deviations elements exceed the value returned. -inf: no useful bound.
-__device__ float sample_bound(TopkSmem* sm, const float* row, int eff, int k) {
-  const int tid = threadIdx.x;
-  const int groups = eff >> 2;
-  // groups per thread: long rows need a larger sample for a list of the same length (beyond 2^20 positions one that meets 32 or
-  // more of 2048 selected ones)
-  constexpr int kMaxPer = 4096 / kTopkThreads;
-  const int per = eff <= (1 << 20) ? (eff <= (1 << 16) ? 1024 : (eff <= (1 << 18) ? 2048 : 4096)) / kTopkThreads : (eff + (1 << 17) - 1) >> 17;
+// The sample of a row: groups of four, evenly spread, `per` of them for every thread.
+__device__ __forceinline__ float4 sample_group(const float* row, int eff, int per, int u) {
+  const int g = static_cast<int>(static_cast<long long>(threadIdx.x + u * kTopkThreads) * (eff >> 2) / (static_cast<long long>(kTopkThreads) * per));
+  return __ldg(reinterpret_cast<const float4*>(row) + g);
+}
+// How many samples are to lie above the bound: about k + 4.5 standard deviations elements of the row exceed it. At most `most` of
+// them let expect a list of three quarters of its capacity.
+__device__ __forceinline__ unsigned int sample_need(int eff, int k, int per, float* most) {
   const float samples = static_cast<float>(4 * kTopkThreads) * static_cast<float>(per);
-  float4 v[kMaxPer];  // the sample, or the part of a larger one at hand
-  auto load = [&](int u0) {
-#pragma unroll
-    for (int u = 0; u < kMaxPer; ++u) {
-      if (u0 + u < per) {
-        const int g = static_cast<int>(static_cast<long long>(tid + (u0 + u) * kTopkThreads) * groups / (static_cast<long long>(kTopkThreads) * per));
-        v[u] = __ldg(reinterpret_cast<const float4*>(row) + g);
-      }
-    }
-  };
-  auto each = [&](auto&& f) {
-    for (int u0 = 0; u0 < per; u0 += kMaxPer) {
-      if (per > kMaxPer) load(u0);
-#pragma unroll
-      for (int u = 0; u < kMaxPer; ++u) {
-        if (u0 + u < per) {
-          f(v[u].x);
-          f(v[u].y);
-          f(v[u].z);
-          f(v[u].w);
-        }
-      }
-    }
-  };
-  if (per <= kMaxPer) load(0);
-  float vmin = INFINITY, vmax = -INFINITY;
-  each([&](float x) {
-    vmin = fminf(vmin, x);
-    vmax = fmaxf(vmax, x);
-  });
-  for (int j = tid; j < kBins; j += kTopkThreads) sm->hist[j] = 0;
-  unsigned int zlo = float_order(vmin), zhi = float_order(vmax);
-  block_range(sm, zlo, zhi);
-  BinMap map;
-  map.set(order_float(zlo), order_float(zhi));
   const float mean = static_cast<float>(k) * samples / static_cast<float>(eff);
-  const unsigned int need = static_cast<unsigned int>(mean + 4.5f * sqrtf(mean) + 4.0f);
-  // samples above the bound that let expect a list of three quarters of its capacity
-  const float most = 0.75f * static_cast<float>(kListCap) * samples / static_cast<float>(eff);
-  if (map.inv != 0.f) {
-    each([&](float x) { atomicAdd(&sm->hist[map.bin(x)], 1u); });
-    __syncthreads();
-    find_threshold_bin<kBins / kTopkThreads>(sm, need);
-    const int b = sm->thr_bin;
-    if (static_cast<float>(sm->thr_above + sm->thr_count) <= most) return map.lo + static_cast<float>(b) / map.inv;
-    if (b + 1 < kBins) zhi = float_order(map.lo + static_cast<float>(b + 1) / map.inv);
-    zlo = float_order(map.lo + static_cast<float>(b) / map.inv);
+  *most = 0.75f * static_cast<float>(kListCap) * samples / static_cast<float>(eff);
+  return static_cast<unsigned int>(mean + 4.5f * sqrtf(mean) + 4.0f);
+}
+
+// The bound where the first histogram does not give it: the bin that holds the threshold over again, by the images of its values
+// [zlo, zhi], until it is fine enough. zlo > zhi: all of the row. The sample is read again for every pass.
+__device__ __noinline__ float sample_bound_fine(TopkSmem* sm, const float* row, int eff, int k, int per, unsigned int zlo, unsigned int zhi) {
+  float most;
+  const unsigned int need = sample_need(eff, k, per, &most);
+  auto each = [&](auto&& f) {
+    for (int u = 0; u < per; ++u) {
+      const float4 v = sample_group(row, eff, per, u);
+      f(v.x);
+      f(v.y);
+      f(v.z);
+      f(v.w);
+    }
+  };
+  if (zlo > zhi) {
+    float vmin = INFINITY, vmax = -INFINITY;
+    each([&](float x) {
+      vmin = fminf(vmin, x);
+      vmax = fmaxf(vmax, x);
+    });
+    zlo = float_order(vmin);
+    zhi = float_order(vmax);
+    block_range(sm, zlo, zhi);
   }
-  // Too many values in the bin of the threshold: that bin over again, by the images of its values, until it is fine enough
-  for (int pass = 0; pass < 2 && zhi > zlo; ++pass) {
+  for (int pass = 0; pass < 3 && zhi > zlo; ++pass) {
     OrderMap zoom;
     zoom.set(zlo, zhi);
-    for (int j = tid; j < kBins; j += kTopkThreads) sm->hist[j] = 0;
+    for (int j = threadIdx.x; j < kBins; j += kTopkThreads) sm->hist[j] = 0;
     __syncthreads();
     each([&](float x) { atomicAdd(&sm->hist[zoom.bin(float_order(x))], 1u); });
     __syncthreads();
@@ -364,6 +344,54 @@ __device__ float sample_bound(TopkSmem* sm, const float* row, int eff, int k) {
     if (static_cast<float>(sm->thr_above + sm->thr_count) <= most) return order_float(zlo);
   }
   return -INFINITY;
+}
+
+// Lower bound of the k largest of row[0, eff) from a sample: 1024 groups of four, or a multiple of that: long rows need a larger
+// sample for a list of the same length (beyond 2^20 positions one that meets 32 or more of 2048 selected ones). -inf: no useful bound.
+__device__ float sample_bound(TopkSmem* sm, const float* row, int eff, int k) {
+  const int tid = threadIdx.x;
+  if (eff > (1 << 20)) return sample_bound_fine(sm, row, eff, k, (eff + (1 << 17) - 1) >> 17, 1u, 0u);
+  constexpr int kMaxPer = 4096 / kTopkThreads;
+  const int per = (eff <= (1 << 16) ? 1024 : (eff <= (1 << 18) ? 2048 : 4096)) / kTopkThreads;
+  float4 v[kMaxPer];
+  float vmin = INFINITY, vmax = -INFINITY;
+#pragma unroll
+  for (int u = 0; u < kMaxPer; ++u) {
+    if (u < per) v[u] = sample_group(row, eff, per, u);
+  }
+#pragma unroll
+  for (int u = 0; u < kMaxPer; ++u) {
+    if (u < per) {
+      vmin = fminf(vmin, fminf(fminf(v[u].x, v[u].y), fminf(v[u].z, v[u].w)));
+      vmax = fmaxf(vmax, fmaxf(fmaxf(v[u].x, v[u].y), fmaxf(v[u].z, v[u].w)));
+    }
+  }
+  for (int j = tid; j < kBins; j += kTopkThreads) sm->hist[j] = 0;
+  unsigned int olo = float_order(vmin), ohi = float_order(vmax);
+  block_range(sm, olo, ohi);
+  BinMap map;
+  map.set(order_float(olo), order_float(ohi));
+#pragma unroll
+  for (int u = 0; u < kMaxPer; ++u) {
+    if (u < per) {
+      atomicAdd(&sm->hist[map.bin(v[u].x)], 1u);
+      atomicAdd(&sm->hist[map.bin(v[u].y)], 1u);
+      atomicAdd(&sm->hist[map.bin(v[u].z)], 1u);
+      atomicAdd(&sm->hist[map.bin(v[u].w)], 1u);
+    }
+  }
+  __syncthreads();
+  float most;
+  const unsigned int need = sample_need(eff, k, per, &most);
+  find_threshold_bin<kBins / kTopkThreads>(sm, need);
+  const int b = sm->thr_bin;
+  const float bound = map.lo + static_cast<float>(b) / map.inv;
+  if (map.inv != 0.f) {
+    if (static_cast<float>(sm->thr_above + sm->thr_count) <= most) return bound;
+    olo = float_order(bound);
+    if (b + 1 < kBins) ohi = float_order(map.lo + static_cast<float>(b + 1) / map.inv);
+  }
+  return sample_bound_fine(sm, row, eff, k, per, olo, ohi);
 }
 
 // Applies f(value, position) to every element of row[0, eff). Loads are issued four at a time before the bodies run, so the
@@ -591,14 +619,7 @@ li_topk_kernel(TopkParams p) {
   if (good) {
     for (int j = tid; j < kBins; j += kTopkThreads) sm->hist[j] = 0;
     block_range(sm, omin, omax);
-    // Equal widths first in a row that is the list: around zero the images have many powers of two for few values (8 x 4096 in
-    // order 18 us against 22).
-    BinMap even;
-    even.set(order_float(omin), order_float(omax));
-    OrderMap map;
-    map.set(omin, omax);
-    if (eff > p.k) map.top = 0xff800000u;  // (NaN is not selected before numbers, but in a row that is selected whole it comes first)
-    auto order = [&](auto&& bin) {  // true: the result is written
+    auto order = [&](auto&& bin, unsigned int cap) {  // true: the result is written. cap: keys of a bin that are ranked by counting
       constexpr int kPer = kListCap / kTopkThreads;
       unsigned int where[kPer];  // bin, and which of its keys
 #pragma unroll
@@ -625,7 +646,7 @@ li_topk_kernel(TopkParams p) {
           const unsigned int b = where[u] >> 16, first = sm->base[b], slot = where[u] & 0xffffu;
           if (first < uk) {
             if (unsorted && first + sm->hist[b] <= uk) go = true;
-            else if (slot < static_cast<unsigned int>(kBinCap)) sm->sorted[first + slot] = key_at(j);
+            else if (slot < cap) sm->sorted[first + slot] = key_at(j);
             else crowded = true;
           }
         }
@@ -660,13 +681,20 @@ li_topk_kernel(TopkParams p) {
       }
       return true;
     };
-    if (whole && even.inv != 0.f) {
-      if (order([&](unsigned long long key) { return static_cast<unsigned int>(even.bin(order_float(key_order(key)))); })) return;
+    BinMap even;
+    even.set(order_float(omin), order_float(omax));
+    // Equal widths first: the images give the values near zero many bins and the others few, and their conversion costs more (64 x
+    // 65536 in a whole step 139.1 us, with the images at once 141.3).
+    if (even.inv != 0.f) {
+      if (order([&](unsigned long long key) { return static_cast<unsigned int>(even.bin(order_float(key_order(key)))); }, kBinCap / 4)) return;
       for (int j = tid; j < kBins; j += kTopkThreads) sm->hist[j] = 0;
       if (tid == 0) sm->n_sel = 0;
       __syncthreads();
     }
-    if (order([&](unsigned long long key) { return static_cast<unsigned int>(map.bin(key_order(key))); })) return;
+    OrderMap map;
+    map.set(omin, omax);
+    if (eff > p.k) map.top = 0xff800000u;  // (NaN is not selected before numbers, but in a row that is selected whole it comes first)
+    if (order([&](unsigned long long key) { return static_cast<unsigned int>(map.bin(key_order(key))); }, kBinCap)) return;
   }
 
   // ---- 3'. MSB-first radix select on the 64-bit keys of the whole row (rank 0) ----------------------------
