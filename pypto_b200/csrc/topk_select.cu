@@ -264,7 +264,7 @@ struct BinMap {
 // The same over the order-preserving images: equal widths within a power of two, and as many bins for each power of two of the
 // range. A few values far from the others (an outlier, a long tail, masked positions) leave the others spread over many bins,
 // where equal widths put all of them into one: 256 rows of 131072 with one value at 300 standard deviations 293 us, all of them
-// in the radix select, now 70. What lies outside goes to the ends; images above `top` (NaN) to bin 0.
+// in the radix select, now 75. What lies outside goes to the ends; images above `top` (NaN) to bin 0.
 struct OrderMap {
   unsigned int lo, top;
   float scale;
