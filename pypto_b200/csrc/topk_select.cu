@@ -394,20 +394,26 @@ __device__ float sample_bound(TopkSmem* sm, const float* row, int eff, int k) {
   return sample_bound_fine(sm, row, eff, k, per, olo, ohi);
 }
 
-// Applies f(value, position) to every element of row[0, eff). Loads are issued four at a time before the bodies run, so the
-// latency of one batch is paid once (the bodies contain shared-memory atomics the compiler will not move loads across).
+// Applies f(value, position) to every element of row[0, eff). Sixteen values are requested before the first body runs, so the
+// latency of one batch is paid once (the bodies contain shared-memory atomics the compiler will not move loads across). A row is
+// a multiple of four long in memory.
 template <typename F>
 __device__ __forceinline__ void for_each_element(const float* row, int eff, F&& f) {
-  const int tid = threadIdx.x;
-  for (int j0 = tid; j0 < eff; j0 += 4 * kTopkThreads) {
-    float v[4];
+  constexpr int kStep = 4 * kTopkThreads;
+  for (int j0 = 4 * threadIdx.x; j0 < eff; j0 += 4 * kStep) {
+    float4 v[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      if (j0 + u * kTopkThreads < eff) v[u] = __ldg(row + j0 + u * kTopkThreads);
+      if (j0 + u * kStep < eff) v[u] = __ldg(reinterpret_cast<const float4*>(row + j0 + u * kStep));
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      if (j0 + u * kTopkThreads < eff) f(v[u], j0 + u * kTopkThreads);
+      const float x[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int pos = j0 + u * kStep + e;
+        if (pos < eff) f(x[e], pos);
+      }
     }
   }
 }
@@ -457,6 +463,7 @@ li_topk_kernel(TopkParams p) {
   }
 
   unsigned int omin = 0xffffffffu, omax = 0u;  // range of the list, as order-preserving images
+  float bound = -INFINITY;                     // no smaller value is among the k largest, if the list has k keys or more
   unsigned int n_list, n_front = kListCap;  // the first n_front keys at the front, the others from the end backwards
   auto key_at = [&](unsigned int j) { return sm->list[j < n_front ? j : kListCap - 1 - (j - n_front)]; };
   if (whole) {
@@ -496,7 +503,6 @@ li_topk_kernel(TopkParams p) {
       for (int c = 0; c < min(chunks, kRing); ++c) fetch(c);
     }
     // ---- 1. lower bound -------------------------------------------------------------------------
-    float bound = -INFINITY;
     bool known = false;
     if (p.hist != nullptr) {
       const uint4* h4 = reinterpret_cast<const uint4*>(p.hist + static_cast<int64_t>(row_id) * kLiHistBins);
@@ -702,6 +708,8 @@ li_topk_kernel(TopkParams p) {
     sm->n_sel = 0;
     if (p.status != nullptr) atomicAdd(p.status + PTO_STATUS_RADIX_ROWS, 1);
   }
+  // (of a list that is too long, i.e. of many equal values, at least the bound is good: what lies below it needs no counting)
+  const float floor = n_list >= static_cast<unsigned int>(k) ? bound : -INFINITY;
   // digits: 11/11/10 bits of the value word, then 11/11/10 bits of the inverted position.
   // invariant: keys with (key >> shift) > prefix are selected; `remaining` more are needed among those with
   // (key >> shift) == prefix.
@@ -717,6 +725,7 @@ li_topk_kernel(TopkParams p) {
     for (int j = tid; j < kBins; j += kTopkThreads) sm->hist[j] = 0;
     __syncthreads();
     for_each_element(row, eff, [&](float v, int pos) {
+      if (v < floor) return;
       const unsigned long long key = make_key(v, pos);
       if (shift < 64 && (key >> shift) != prefix) return;
       atomicAdd(&sm->hist[static_cast<unsigned int>(key >> new_shift) & ((1u << w) - 1u)], 1u);
@@ -730,6 +739,7 @@ li_topk_kernel(TopkParams p) {
     __syncthreads();
   }
   for_each_element(row, eff, [&](float v, int pos) {
+    if (v < floor) return;
     const unsigned long long key = make_key(v, pos);
     if ((key >> shift) >= prefix) {
       const unsigned int slot = atomicAdd(&sm->n_sel, 1u);
