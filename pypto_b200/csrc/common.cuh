@@ -77,9 +77,10 @@ __device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
 // Programmatic dependent launch. A kernel launched with the programmatic-serialization attribute may start
 // while its predecessor in the stream still runs; `pdl_wait` blocks until that predecessor has completed and
 // its writes are visible (a no-op in a kernel launched the ordinary way). `pdl_trigger` lets the successor
-// start early. Rule kept throughout: a kernel triggers only after its own wait, and the first kernel of a
-// chain is launched the ordinary way, so a successor that is running implies that everything before the
-// chain has completed.
+// start early. Rule kept throughout: the first kernel of a chain is launched the ordinary way, and a kernel starts only when
+// every block of the one before it has begun (has triggered), so a kernel of a chain that is running implies that everything
+// before the chain has completed: inputs of the call may be read before the wait, results of the chain only behind it. A kernel's
+// completion implies its own wait, so the waits carry over, whether it triggers before its wait (prologs) or behind it.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

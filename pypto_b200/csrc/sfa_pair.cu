@@ -8,7 +8,7 @@
 // Why a pair: the fp32 output of 128 heads x 512 values is 256 KB, all of one SM's tensor memory. With the
 // heads split, CTA c keeps O for its 64 heads (256 columns) and two score buffers (2 x 64 columns), and the
 // whole 576-wide contraction is local to the pair's MMA: no score ever crosses between the CTAs, and nothing
-// else does either except four "ready" notices per tile. A 2-SM MMA reads half of its B operand from
+// else does either except the "ready" notices of a tile (two for K, four for V, P, scores read). A 2-SM MMA reads half of its B operand from
 // each CTA's shared memory:
 //   q.K^T  (M = 128 heads, N = 128 keys of a tile, K = 576): A = this CTA's 64 query rows, B = the tile's keys,
 //          of which CTA c gathers and dequantises keys [64c, 64c+64) in full width (9 chunks of 64 dims).
@@ -225,12 +225,10 @@ __device__ __forceinline__ uint32_t pair_setup_sync(PairCtl* ctl) {
 // Two threads on two different schedulers: warp 0 issues the score products, warp 2 the value products.
 //   q.K^T first half  (chunks 0-3: 16 MMAs)  needs K half 0 of the tile and the score buffer it overwrites read
 //   q.K^T second half (chunks 4-8: 20 MMAs)  needs K half 1; completes the tile's scores
-//   P.V first half    (keys 0-63:   8 MMAs)  needs P of the tile and V key half 0
-//   P.V second half   (keys 64-127: 8 MMAs)  needs V key half 1; completes the tile's P.V
-// After each action a commit hands the half it read back to its producers, so that the refill for the next tile
-// runs behind the MMAs that read the other half. One thread issuing everything (an event loop over the four
-// actions) was what a tile waited for: 36 + 16 MMAs kept it busy for 8.7 k cycles per tile; side by side the two
-// threads take 3.2-4.0 k and 1.5-2.7 k (80.1 -> 77.7 us on 64 tokens x 2048 rows). The products of the two threads
+//   P.V quarter q     (keys 32q .. +31: 4 MMAs)  needs P of the tile and V key quarter q; the last completes the tile's P.V
+// After each action a commit hands the part it read back to its producers, so that the refill for the next tile
+// runs behind the MMAs that read the others. One thread issuing everything was what a tile waited for: 36 + 16 MMAs kept it
+// busy for 8.7 k cycles per tile (two threads: 80.1 -> 77.7 us on 64 tokens x 2048 rows). The products of the two threads
 // are independent (different accumulators), every dependency between them goes through the mbarriers, and a
 // commit covers the MMAs of the thread that executes it.
 // (No cluster-scope fence before the MMAs: measured, `fence.acq_rel.cluster` holds a thread for 2000-3700 cycles

@@ -20,9 +20,10 @@
 //   warp 0          issues the score MMAs of a tile        warp 1   issues the value MMAs of a tile
 //   warps 2..3      query tile of the next item (cp.async) warps 4..7  softmax and output (TMEM lane = key / dim)
 //   warps 8..       producers, four rows of a tile each: gather, int8 -> bf16, swizzled stores
-// What bounds it: the producers. 4096 tokens x 2048 rows x 16 heads take 2.1 ms, i.e. 5.6 k cycles per tile of 80 rows, of
-// which the MMAs are 2184: one with N = 16 takes 39 cycles (4.5 KB of operands at 128 bytes per cycle; measured in
-// isolation), and there are 36 + 4 kTK/16 of them.
+// What bounds it: the chain gather -> conversion -> scores -> softmax -> products over two tile buffers. 4096 tokens x 2048 rows
+// x 16 heads take 2.1 ms, i.e. 5.6 k cycles per tile of 80 rows, of which the MMAs' issue is 2184 (one with N = 16 takes 39
+// cycles, measured in isolation, and there are 36 + 4 kTK/16 of them); the counters show no unit more than half busy (issue slots
+// 46 %, tensor pipe 7 %, L2 16 %).
 // Why bf16: a form that multiplied the rows as int8, queries and probabilities as fixed-point limbs, took 1.24 ms, but a
 // fixed-point probability has an absolute error: beside a row with 0.96 of the weight the others rounded to zero (rel-L2
 // against 64 bits 0.22, 16 heads; this form 0.0020, the mma.sync kernel before it 0.0024).
