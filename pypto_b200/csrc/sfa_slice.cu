@@ -18,10 +18,11 @@
 // Persistent CTAs, one per SM, walk (token, head block, split) items; tiles of kTK rows alternate between two buffers
 // and run on across items, so that only the query tile and the output are handed over at an item's end.
 //   warp 0          issues the score MMAs of a tile        warp 1   issues the value MMAs of a tile
-//   warps 2..3      query tile of the next item (cp.async) warps 4..7  softmax and output (TMEM lane = key / dim)
-//   warps 8..       producers, four rows of a tile each: gather, int8 -> bf16, swizzled stores
+//   warps 2..3      query tile of the next item (cp.async) warps 4..11 softmax and output (TMEM lane = key / dim), in two
+//                   groups of four warps, half of the heads each
+//   warps 12..      producers, four rows of a tile each: gather, int8 -> bf16, swizzled stores
 // What bounds it: the chain gather -> conversion -> scores -> softmax -> products over two tile buffers. 4096 tokens x 2048 rows
-// x 16 heads take 2.1 ms, i.e. 5.6 k cycles per tile of 80 rows, of which the MMAs' issue is 2184 (one with N = 16 takes 39
+// x 16 heads take 2.00 ms, i.e. 5.3 k cycles per tile of 80 rows (2.11 ms with all heads in four softmax warps), of which the MMAs' issue is 2184 (one with N = 16 takes 39
 // cycles, measured in isolation, and there are 36 + 4 kTK/16 of them); the counters show no unit more than half busy (issue slots
 // 46 %, tensor pipe 7 %, L2 16 %).
 // Why bf16: a form that multiplied the rows as int8, queries and probabilities as fixed-point limbs, took 1.24 ms, but a
@@ -49,15 +50,16 @@ struct SliceCfg {
   static constexpr int kSmemP = kSmemQ + kSliceChunks * kQChunk;  // [buffer][tile c]
   static constexpr int kSmemCtl = kSmemP + 2 * 4 * kPBytes;
   static constexpr int kProdWarps = kTK / 4;
-  static constexpr int kThreads = 32 * (8 + kProdWarps);
+  static constexpr int kH = kHB / 2;                        // heads of a softmax group
+  static constexpr int kThreads = 32 * (12 + kProdWarps);
   static constexpr uint32_t kColS = 0;                      // S buffer b, accumulator c at (b * 5 + c) * kHB
   static constexpr uint32_t kColO = 2 * 5 * kHB;            // O block c at kColO + c * kHB
   static constexpr uint32_t kTmemCols = kHB == 16 ? 256 : 512;
   static_assert(kColO + 4 * kHB <= kTmemCols, "tensor memory");
   // registers per thread: at launch, issuers / loaders, softmax, producers
-  static constexpr int kRegLaunch = kHB == 16 ? 72 : 80;
-  static constexpr int kRegIssue = 40, kRegSoftmax = kHB == 16 ? 128 : 152, kRegProd = 64;
-  static_assert(128 * kRegIssue + 128 * kRegSoftmax + 32 * kProdWarps * kRegProd <= kThreads * kRegLaunch, "register split");
+  static constexpr int kRegLaunch = kHB == 16 ? 64 : 72;
+  static constexpr int kRegIssue = 40, kRegSoftmax = kHB == 16 ? 72 : 104, kRegProd = 64;
+  static_assert(128 * kRegIssue + 256 * kRegSoftmax + 32 * kProdWarps * kRegProd <= kThreads * kRegLaunch, "register split");
 };
 
 template <int kHB, int kTK>
@@ -70,11 +72,11 @@ struct SliceCtl {
   uint64_t full[2];   // producers filled the tile buffer            (producer warps)
   uint64_t done[2];   // P.V of the tile complete: tile buffer and P buffer free, O at rest (commit)
   uint64_t sfull[2];  // scores of the tile complete                 (commit)
-  uint64_t sfree[2];  // scores read                                 (4 softmax warps)
-  uint64_t pfull[2];  // P^T of the tile written                     (4 softmax warps)
+  uint64_t sfree[2];  // scores read                                 (8 softmax warps)
+  uint64_t pfull[2];  // P^T of the tile written                     (8 softmax warps)
   uint64_t qfull;     // query tile of the item loaded               (2 loader warps)
   uint64_t qfree;     // last score product of the item complete     (commit)
-  uint64_t ofree;     // output of the item read from tensor memory  (4 softmax warps)
+  uint64_t ofree;     // output of the item read from tensor memory  (8 softmax warps)
   uint32_t tmem_base;
   int abort;
 };
@@ -144,7 +146,7 @@ __device__ __forceinline__ uint2 slice_cvt4(uint32_t w) {
 template <int kHB, int kTK, bool kPacked>
 __device__ __forceinline__ void slice_role_producer(const SfaParams& p, SliceCtl<kHB, kTK>* ctl, uint32_t base, int n_items) {
   using Cfg = SliceCfg<kHB, kTK>;
-  const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) - 8;
+  const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) - 12;
   const int r = lane & 3, rsel = (lane >> 2) & 1;
   const int src_off = (((lane & 3) | ((lane >> 3) << 2)) << 4);  // this lane's 16 bytes of a half row
   const uint8_t* const kn = reinterpret_cast<const uint8_t*>(p.kn);
@@ -410,81 +412,88 @@ __device__ __forceinline__ void slice_role_query(const SfaParams& p, SliceCtl<kH
 }
 
 // ================================ softmax and output =============================================
-// Four warps, TMEM lane = key of the tile (warp q holds keys 32q .. +31; lanes above kTK take part in the barriers only).
-// A thread has one key's scores for all kHB heads. The reference maximum of a head moves only when a score exceeds it by
-// more than 2^8 (first tile: always), which one vote over the four warps finds out; so the reduction over keys, here
-// across lanes, is rare, and the row sums stay per-thread partials until the item ends.
+// Two groups of four warps, each with half of the heads; TMEM lane = key of the tile (warp q of a group holds keys 32q .. +31;
+// lanes above kTK take part in the barriers only). A thread has one key's scores for its group's kH heads: the scores ->
+// probabilities chain of a tile sits between its two products, and half as many heads are half as long a chain.
+// The reference maximum of a head moves only when a score exceeds it by more than 2^8 (first tile: always), which one vote over the
+// group finds out; so the reduction over keys, here across lanes, is rare, and the row sums stay per-thread partials until the
+// item ends.
 constexpr float kSliceRescale = 8.0f;
 
-template <int kHB>
-__device__ __forceinline__ void slice_ld(uint32_t taddr, float (&v)[kHB]) {
-  uint32_t r[kHB];
-  if constexpr (kHB == 16) tmem_ld_32x32b_x16(taddr, r);
-  else tmem_ld_32x32b_x32(taddr, r);
+template <int kH>
+__device__ __forceinline__ void slice_ld(uint32_t taddr, float (&v)[kH]) {
+  uint32_t r[kH];
+  if constexpr (kH == 8) tmem_ld_32x32b_x8(taddr, r);
+  else tmem_ld_32x32b_x16(taddr, r);
   tc_wait_ld();
 #pragma unroll
-  for (int h = 0; h < kHB; ++h) v[h] = __uint_as_float(r[h]);
+  for (int h = 0; h < kH; ++h) v[h] = __uint_as_float(r[h]);
 }
 
-__device__ __forceinline__ bool slice_vote(bool pred) {  // OR over the four softmax warps; also their barrier
+__device__ __forceinline__ bool slice_vote(int group, bool pred) {  // OR over the group's four warps; also their barrier
   uint32_t any;
   asm volatile(
-      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.cta.red.or.pred q, 1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %2, 0;\n\tbarrier.cta.red.or.pred q, %1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
       : "=r"(any)
-      : "r"(pred ? 1u : 0u)
+      : "r"(1 + group), "r"(pred ? 1u : 0u)
       : "memory");
   return any != 0;
 }
-__device__ __forceinline__ void slice_meet() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+__device__ __forceinline__ void slice_meet(int group) { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); }
 
 template <int kHB, int kTK>
 __device__ __forceinline__ void slice_role_softmax(const SfaParams& p, SliceCtl<kHB, kTK>* ctl, uint32_t base, uint32_t tmem,
                                                    int n_items) {
   using Cfg = SliceCfg<kHB, kTK>;
-  const int lane = threadIdx.x & 31, quarter = (threadIdx.x >> 5) & 3, tid = threadIdx.x - 128;
+  constexpr int kH = Cfg::kH;
+  const int lane = threadIdx.x & 31, quarter = (threadIdx.x >> 5) & 3;
+  const int group = (threadIdx.x >> 7) - 1, tid = threadIdx.x & 127;  // heads kH group .. + kH - 1 of the block; thread of the group
+  const int h0 = kH * group;
+  float* const mref = ctl->mref + h0;
+  float* const alpha = ctl->alpha + h0;
   const int key = 32 * quarter + lane;
   const uint32_t lane_addr = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
   bool ok = true;
   uint32_t t = 0;
   for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
     const SliceItem it = slice_item<kTK>(p, kHB, item);
-    const int64_t orow0 = static_cast<int64_t>(it.ti) * p.nq_total + p.head_begin + it.head0;
-    const int64_t prow0 = (static_cast<int64_t>(it.ti) * p.n_split + it.sp) * p.nq + it.head0;
+    const int64_t orow0 = static_cast<int64_t>(it.ti) * p.nq_total + p.head_begin + it.head0 + h0;
+    const int64_t prow0 = (static_cast<int64_t>(it.ti) * p.n_split + it.sp) * p.nq + it.head0 + h0;
     if (it.ntiles == 0) {
       if (p.n_split == 1) {
-        for (int e = tid; e < kHB * 64; e += 128) *reinterpret_cast<uint4*>(p.out + orow0 * 512 + e * 8) = make_uint4(0, 0, 0, 0);
-      } else if (tid < kHB) {
+        for (int e = tid; e < kH * 64; e += 128) *reinterpret_cast<uint4*>(p.out + orow0 * 512 + e * 8) = make_uint4(0, 0, 0, 0);
+      } else if (tid < kH) {
         p.part_ml[(prow0 + tid) * 2] = -INFINITY;
         p.part_ml[(prow0 + tid) * 2 + 1] = 0.f;
       }
       continue;
     }
-    float l[kHB];
+    float l[kH];
 #pragma unroll
-    for (int h = 0; h < kHB; ++h) l[h] = 0.f;
+    for (int h = 0; h < kH; ++h) l[h] = 0.f;
     for (int j = 0; j < it.ntiles; ++j, ++t) {
       const uint32_t b = t & 1;
-      // (a wait that expired is voted on below, so that the four warps leave together: one that left alone would leave the
+      // (a wait that expired is voted on below, so that the group's four warps leave together: one that left alone would leave the
       // others at a barrier)
       ok = ok && slice_wait(smem_u32(&ctl->sfull[b]), (t >> 1) & 1) && slice_wait(smem_u32(&ctl->full[b]), (t >> 1) & 1);
       tc_fence_after();
-      float s[kHB];
+      float s[kH];
       float4 sc = make_float4(0.f, 0.f, 0.f, 0.f);
       bool valid = false;
       if (32 * quarter < kTK) {
-        const uint32_t col = lane_addr + Cfg::kColS + b * 5 * kHB;
+        const uint32_t col = lane_addr + Cfg::kColS + b * 5 * kHB + h0;
         if (key < kTK) {
           sc = *reinterpret_cast<const float4*>(&ctl->scales[b][key][0]);
           valid = ctl->live[b][key] != 0.f && it.begin + j * kTK + key < it.end;
         }
-        slice_ld<kHB>(col + 4 * kHB, s);  // rope part
+        slice_ld<kH>(col + 4 * kHB, s);  // rope part
         const float scv[4] = {sc.x, sc.y, sc.z, sc.w};
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          float x[kHB];
-          slice_ld<kHB>(col + c * kHB, x);
+          float x[kH];
+          slice_ld<kH>(col + c * kHB, x);
 #pragma unroll
-          for (int h = 0; h < kHB; ++h) s[h] = fmaf(x[h], scv[c], s[h]);
+          for (int h = 0; h < kH; ++h) s[h] = fmaf(x[h], scv[c], s[h]);
         }
       }
       tc_fence_before();
@@ -492,57 +501,60 @@ __device__ __forceinline__ void slice_role_softmax(const SfaParams& p, SliceCtl<
       if (lane == 0) mbar_arrive(smem_u32(&ctl->sfree[b]));
       float over = -INFINITY;
 #pragma unroll
-      for (int h = 0; h < kHB; ++h) {
+      for (int h = 0; h < kH; ++h) {
         s[h] = valid ? s[h] * p.scale_log2 : -INFINITY;
-        over = fmaxf(over, s[h] - (j > 0 ? ctl->mref[h] : 0.f));
+        over = fmaxf(over, s[h] - (j > 0 ? mref[h] : 0.f));
       }
-      if (slice_vote(j == 0 || over > kSliceRescale || !ok)) {
+      if (slice_vote(group, j == 0 || over > kSliceRescale || !ok)) {
         // ---- new reference maxima --------------------------------------------------------------------
 #pragma unroll
-        for (int h = 0; h < kHB; ++h) {
+        for (int h = 0; h < kH; ++h) {
           float m = s[h];
 #pragma unroll
           for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-          if (lane == 0) ctl->red[quarter][h] = m;
+          if (lane == 0) ctl->red[quarter][h0 + h] = m;
         }
-        if (slice_vote(!ok)) {
+        if (slice_vote(group, !ok)) {
           ok = false;
           break;
         }
-        if (tid < kHB) {
-          const float old = j > 0 ? ctl->mref[tid] : -INFINITY;
-          const float m = fmaxf(fmaxf(ctl->red[0][tid], ctl->red[1][tid]), fmaxf(ctl->red[2][tid], ctl->red[3][tid]));
+        if (tid < kH) {
+          const float old = j > 0 ? mref[tid] : -INFINITY;
+          const float m = fmaxf(fmaxf(ctl->red[0][h0 + tid], ctl->red[1][h0 + tid]), fmaxf(ctl->red[2][h0 + tid], ctl->red[3][h0 + tid]));
           const float mn = fmaxf(old, m);
-          ctl->alpha[tid] = old == -INFINITY ? 0.f : ex2f(old - mn);
-          ctl->mref[tid] = mn;
+          alpha[tid] = old == -INFINITY ? 0.f : ex2f(old - mn);
+          mref[tid] = mn;
         }
-        slice_meet();
+        slice_meet(group);
         if (j > 0) {
           ok = slice_wait(smem_u32(&ctl->done[b ^ 1]), ((t - 1) >> 1) & 1);  // the output so far is at rest
           if (ok) tc_fence_after();
 #pragma unroll
-          for (int h = 0; h < kHB; ++h) l[h] *= ctl->alpha[h];
+          for (int h = 0; h < kH; ++h) l[h] *= alpha[h];
           if (ok) {
 #pragma unroll 1
-            for (int c = 0; c < 4 * kHB; c += 16) {
-              uint32_t o[16];
-              tmem_ld_32x32b_x16(lane_addr + Cfg::kColO + c, o);
+            for (int c = 0; c < 4; ++c) {
+              uint32_t o[kH];
+              const uint32_t taddr = lane_addr + Cfg::kColO + c * kHB + h0;
+              if constexpr (kH == 8) tmem_ld_32x32b_x8(taddr, o);
+              else tmem_ld_32x32b_x16(taddr, o);
               tc_wait_ld();
 #pragma unroll
-              for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * ctl->alpha[(c + e) & (kHB - 1)]);
-              tmem_st_32x32b_x16(lane_addr + Cfg::kColO + c, o);
+              for (int e = 0; e < kH; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha[e]);
+              if constexpr (kH == 8) tmem_st_32x32b_x8(taddr, o);
+              else tmem_st_32x32b_x16(taddr, o);
             }
             tc_wait_st();
           }
-          if (slice_vote(!ok)) {  // (alpha is read; a later tile may write it)
+          if (slice_vote(group, !ok)) {  // (alpha is read; a later tile may write it)
             ok = false;
             break;
           }
         }
       }
 #pragma unroll
-      for (int h = 0; h < kHB; ++h) {
-        const float m = ctl->mref[h];
+      for (int h = 0; h < kH; ++h) {
+        const float m = mref[h];
         s[h] = ex2f(s[h] - (m == -INFINITY ? 0.f : m));
         l[h] += s[h];
       }
@@ -555,7 +567,7 @@ __device__ __forceinline__ void slice_role_softmax(const SfaParams& p, SliceCtl<
         for (int c = 0; c < 4; ++c) {
           const uint32_t row = base + Cfg::kSmemP + (b * 4 + c) * Cfg::kPBytes + key * kHB * 2;
 #pragma unroll
-          for (int u = 0; u < kHB / 8; ++u) {
+          for (int u = 0; u < kH / 8; ++u) {
             uint4 w;
             w.x = pack_bf16x2(s[8 * u] * scv[c], s[8 * u + 1] * scv[c]);
             w.y = pack_bf16x2(s[8 * u + 2] * scv[c], s[8 * u + 3] * scv[c]);
@@ -563,7 +575,7 @@ __device__ __forceinline__ void slice_role_softmax(const SfaParams& p, SliceCtl<
             w.w = pack_bf16x2(s[8 * u + 6] * scv[c], s[8 * u + 7] * scv[c]);
             // swizzle: 32-byte rows, unit ^= (row / 4) % 2; 64-byte rows, unit ^= (row / 2) % 4
             const int x = kHB == 16 ? (key >> 2) & 1 : (key >> 1) & 3;
-            sts_v4u(row + ((u ^ x) << 4), w);
+            sts_v4u(row + (((h0 / 8 + u) ^ x) << 4), w);
           }
         }
       }
@@ -572,50 +584,50 @@ __device__ __forceinline__ void slice_role_softmax(const SfaParams& p, SliceCtl<
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&ctl->pfull[b]));
     }
-    // (a `done` that expired at the last tile; the break above comes with the same answer in all four)
-    if (slice_vote(!ok)) {
+    // (a `done` that expired at the last tile; the break above comes with the same answer in the whole group)
+    if (slice_vote(group, !ok)) {
       ok = false;
       break;
     }
     // ---- output --------------------------------------------------------------------------------------
 #pragma unroll
-    for (int h = 0; h < kHB; ++h) {
+    for (int h = 0; h < kH; ++h) {
       float v = l[h];
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if (lane == 0) ctl->red[quarter][h] = v;
+      if (lane == 0) ctl->red[quarter][h0 + h] = v;
     }
-    slice_meet();
-    if (tid < kHB) {
-      const float tot = (ctl->red[0][tid] + ctl->red[1][tid]) + (ctl->red[2][tid] + ctl->red[3][tid]);
+    slice_meet(group);
+    if (tid < kH) {
+      const float tot = (ctl->red[0][h0 + tid] + ctl->red[1][h0 + tid]) + (ctl->red[2][h0 + tid] + ctl->red[3][h0 + tid]);
       if (p.n_split == 1) {
-        ctl->alpha[tid] = tot > 0.f ? 1.f / tot : 0.f;
+        alpha[tid] = tot > 0.f ? 1.f / tot : 0.f;
       } else {
-        ctl->alpha[tid] = 1.f;
-        p.part_ml[(prow0 + tid) * 2] = ctl->mref[tid];
+        alpha[tid] = 1.f;
+        p.part_ml[(prow0 + tid) * 2] = mref[tid];
         p.part_ml[(prow0 + tid) * 2 + 1] = tot;
       }
     }
-    slice_meet();
+    slice_meet(group);
     ok = slice_wait(smem_u32(&ctl->done[(t - 1) & 1]), ((t - 1) >> 1) & 1);
     tc_fence_after();
 #pragma unroll
     for (int c = 0; c < 4 && ok; ++c) {  // dim 128 c + key of every head: 32 lanes write consecutive dims of a head's row
-      float o[kHB];
-      slice_ld<kHB>(lane_addr + Cfg::kColO + c * kHB, o);
+      float o[kH];
+      slice_ld<kH>(lane_addr + Cfg::kColO + c * kHB + h0, o);
       if (c == 3) {
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&ctl->ofree));
       }
 #pragma unroll
-      for (int h = 0; h < kHB; ++h) {
-        const float v = o[h] * ctl->alpha[h];
+      for (int h = 0; h < kH; ++h) {
+        const float v = o[h] * alpha[h];
         if (p.n_split == 1) p.out[(orow0 + h) * 512 + 128 * c + key] = __float2bfloat16_rn(v);
         else p.part_o[(prow0 + h) * 512 + 128 * c + key] = v;
       }
     }
-    if (slice_vote(!ok)) ok = false;  // (alpha and mref are read; the next item may write them)
+    if (slice_vote(group, !ok)) ok = false;  // (alpha and mref are read; the next item may write them)
   }
   if (!ok && lane == 0) {
     ctl->abort = 1;
@@ -640,12 +652,12 @@ sfa_slice_kernel(const __grid_constant__ SfaParams p, int n_items) {
       mbar_init(smem_u32(&ctl->full[b]), Cfg::kProdWarps);
       mbar_init(smem_u32(&ctl->done[b]), 1);
       mbar_init(smem_u32(&ctl->sfull[b]), 1);
-      mbar_init(smem_u32(&ctl->sfree[b]), 4);
-      mbar_init(smem_u32(&ctl->pfull[b]), 4);
+      mbar_init(smem_u32(&ctl->sfree[b]), 8);
+      mbar_init(smem_u32(&ctl->pfull[b]), 8);
     }
     mbar_init(smem_u32(&ctl->qfull), 2);
     mbar_init(smem_u32(&ctl->qfree), 1);
-    mbar_init(smem_u32(&ctl->ofree), 4);
+    mbar_init(smem_u32(&ctl->ofree), 8);
     ctl->abort = 0;
     fence_mbar_init();
   }
@@ -667,7 +679,7 @@ sfa_slice_kernel(const __grid_constant__ SfaParams p, int n_items) {
     } else if (warp == 0) slice_role_scores<kHB, kTK, 0>(p, ctl, base, tmem, n_items);
     else if (warp == 1) slice_role_values<kHB, kTK, 0>(p, ctl, base, tmem, n_items);
     else slice_role_query<kHB, kTK>(p, ctl, base, n_items);
-  } else if (warp < 8) {
+  } else if (warp < 12) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Cfg::kRegSoftmax));
     slice_role_softmax<kHB, kTK>(p, ctl, base, tmem, n_items);
   } else {
