@@ -329,6 +329,10 @@ int run_sfa(const void* qn, const void* qr, const void* kn, const void* kr, cons
   p.head_begin = head_begin;
   p.topk_k = topk;
   p.block_size = block_size;
+  int l = 0;
+  while ((1ll << l) < block_size) ++l;
+  p.page_shift = 31 + l;
+  p.page_mul = static_cast<uint32_t>((1ull << p.page_shift) / static_cast<uint32_t>(block_size) + 1);
   p.max_blocks = max_blocks;
   p.n_split = ns;
   p.packed = packed ? 1 : 0;

@@ -340,6 +340,8 @@ struct SfaParams {
   float* part_o;                // [t, n_split, nq, 512]
   float* part_ml;               // [t, n_split, nq, 2]
   int b, s1, nq, nq_total, head_begin, topk_k, block_size, max_blocks, n_split, packed, kn_bf16;
+  uint32_t page_mul;  // position / block_size = position * page_mul >> page_shift, for every position below 2^31: a division by an
+  int page_shift;     // integer that the kernel does not know is about 35 instructions (Granlund and Montgomery 1994)
   int pdl;  // launched behind the top-k kernel with programmatic serialization: setup overlaps the selection
   int64_t n_rows;
   float scale_log2;  // softmax_scale * log2(e)

@@ -75,22 +75,6 @@ __device__ __forceinline__ void dequant16(const uint4 v, const float scale, uint
   o1 = make_uint4(o[4], o[5], o[6], o[7]);
 }
 
-__device__ __forceinline__ long long tc_physical_row(const SfaParams& p, int bi, int idx) {
-  if (idx < 0) return -1;
-  const int blk = idx / p.block_size;
-  if (blk >= p.max_blocks) {
-    set_status(p.status, PTO_ST_BAD_PAGE, idx, 20);
-    return -1;
-  }
-  const int phys = p.block_table[static_cast<int64_t>(bi) * p.max_blocks + blk];
-  const long long r = static_cast<long long>(phys) * p.block_size + idx % p.block_size;
-  if (phys < 0 || r >= p.n_rows) {
-    set_status(p.status, PTO_ST_BAD_PAGE, phys, 21);
-    return -1;
-  }
-  return r;
-}
-
 // tcgen05.mma with the A operand in tensor memory (row m of A = TMEM lane m, 32-bit column c holds the
 // K elements 2c and 2c+1 of a 16-bit type), B in shared memory.
 __device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
@@ -161,26 +145,30 @@ __device__ __forceinline__ void cp_async_16(uint32_t dst_smem, const void* src, 
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst_smem), "l"(src), "r"(src_bytes) : "memory");
 }
 
-// The same lookup in two steps, so that a caller can fetch the block-table entry a tile ahead and
+// Paged row of a selected position, in two steps, so that a caller can fetch the block-table entry a tile ahead and
 // only branch on it once it has arrived.
 constexpr int kTableSkip = INT_MIN;  // nothing to fetch: padding index, or an index already reported
+__device__ __forceinline__ int tc_block_of(const SfaParams& p, int idx) {
+  return static_cast<int>((static_cast<unsigned long long>(static_cast<uint32_t>(idx)) * p.page_mul) >> p.page_shift);
+}
 __device__ __forceinline__ int tc_table_entry(const SfaParams& p, int bi, int idx) {
   if (idx < 0) return kTableSkip;
-  const int blk = idx / p.block_size;
+  const int blk = tc_block_of(p, idx);
   if (blk >= p.max_blocks) {
     set_status(p.status, PTO_ST_BAD_PAGE, idx, 20);
     return kTableSkip;
   }
   return ldg_pinned_i32(p.block_table + static_cast<int64_t>(bi) * p.max_blocks + blk);
 }
-__device__ __forceinline__ long long tc_row_from_entry(const SfaParams& p, int idx, int entry) {
+// 32 bits: the host side refuses caches of 2^31 rows or more. -1: a padding index, or a rejected one
+__device__ __forceinline__ int tc_row_from_entry(const SfaParams& p, int idx, int entry) {
   if (entry == kTableSkip) return -1;
-  const long long r = static_cast<long long>(entry) * p.block_size + idx % p.block_size;
+  const long long r = static_cast<long long>(entry) * p.block_size + (idx - tc_block_of(p, idx) * p.block_size);
   if (entry < 0 || r >= p.n_rows) {
     set_status(p.status, PTO_ST_BAD_PAGE, entry, 21);
     return -1;
   }
-  return r;
+  return static_cast<int>(r);
 }
 
 }  // namespace pto

@@ -176,18 +176,6 @@ __device__ __forceinline__ uint4 pair_dequant8(const uint32_t w0, const uint32_t
   return o;
 }
 
-// Paged row of a selected position, in 32 bits (the host side refuses caches of 2^31 rows or more): -1 for a
-// padding index or a rejected one (reported once through the status words).
-__device__ __forceinline__ int pair_row(const SfaParams& p, int idx, int entry) {
-  if (entry == kTableSkip) return -1;
-  const long long r = static_cast<long long>(entry) * p.block_size + idx % p.block_size;
-  if (entry < 0 || r >= p.n_rows) {
-    set_status(p.status, PTO_ST_BAD_PAGE, entry, 21);
-    return -1;
-  }
-  return static_cast<int>(r);
-}
-
 struct PairCtx {
   PairCtl* ctl;
   const int32_t* idx_row;  // this token's selected positions
@@ -670,10 +658,10 @@ __device__ __forceinline__ void pair_role_kproducer(const SfaParams& p, const Pa
     const int e0 = tc_table_entry(p, bi, idx0);
     const int e1 = tc_table_entry(p, bi, idx1);
     entry_a = tc_table_entry(p, bi, idx_a);
-    row_cur = pair_row(p, idx0, e0);
+    row_cur = tc_row_from_entry(p, idx0, e0);
     issue_loads(row_cur);
     if (kBf) prefetch_row(row_cur);
-    row_n = pair_row(p, idx1, e1);
+    row_n = tc_row_from_entry(p, idx1, e1);
     prefetch_row(row_n);
   }
   for (int j = 0; j < ntiles; ++j) {
@@ -717,7 +705,7 @@ __device__ __forceinline__ void pair_role_kproducer(const SfaParams& p, const Pa
     if (lane == 0) mbar_arrive(smem_u32(&ctl->kfull[half]));
     if (j + 1 < ntiles) issue_loads(row_n);  // the half rows of tile j+1 (in L2: prefetched a tile ago)
     row_cur = row_n;
-    row_n = pair_row(p, idx_a, entry_a);     // tile j+2: into L2
+    row_n = tc_row_from_entry(p, idx_a, entry_a);     // tile j+2: into L2
     prefetch_row(row_n);
     idx_a = idx_b;
     entry_a = tc_table_entry(p, bi, idx_a);  // block-table entries of tile j+3
@@ -777,9 +765,9 @@ __device__ __forceinline__ void pair_role_vproducer(const SfaParams& p, const Pa
     const int e0 = tc_table_entry(p, c.bi, idx0);
     const int e1 = tc_table_entry(p, c.bi, idx1);
     entry_a = tc_table_entry(p, c.bi, idx_a);
-    row_cur = pair_row(p, idx0, e0);
+    row_cur = tc_row_from_entry(p, idx0, e0);
     issue_loads(row_cur);
-    row_n = pair_row(p, idx1, e1);
+    row_n = tc_row_from_entry(p, idx1, e1);
   }
   for (int j = 0; j < ntiles; ++j) {
     if (j > 0) {  // the P.V MMAs of the previous tile that read this key quarter are complete
@@ -813,7 +801,7 @@ __device__ __forceinline__ void pair_role_vproducer(const SfaParams& p, const Pa
     if (lane == 0) mbar_arrive(smem_u32(&ctl->vfull[q]));
     if (j + 1 < ntiles) issue_loads(row_n);
     row_cur = row_n;
-    row_n = pair_row(p, idx_a, entry_a);
+    row_n = tc_row_from_entry(p, idx_a, entry_a);
     idx_a = idx_b;
     entry_a = tc_table_entry(p, c.bi, idx_a);
     idx_b = load_idx(j + 4);

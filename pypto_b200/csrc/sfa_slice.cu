@@ -22,7 +22,7 @@
 //                   groups of four warps, half of the heads each
 //   warps 12..      producers, four rows of a tile each: gather, int8 -> bf16, swizzled stores
 // What bounds it: the chain gather -> conversion -> scores -> softmax -> products over two tile buffers. 4096 tokens x 2048 rows
-// x 16 heads take 2.00 ms, i.e. 5.3 k cycles per tile of 80 rows (2.11 ms with all heads in four softmax warps), of which the MMAs' issue is 2184 (one with N = 16 takes 39
+// x 16 heads take 1.98 ms, i.e. 5.2 k cycles per tile of 80 rows (2.11 ms with all heads in four softmax warps), of which the MMAs' issue is 2184 (one with N = 16 takes 39
 // cycles, measured in isolation, and there are 36 + 4 kTK/16 of them); the counters show no unit more than half busy (issue slots
 // 46 %, tensor pipe 7 %, L2 16 %).
 // Why bf16: a form that multiplied the rows as int8, queries and probabilities as fixed-point limbs, took 1.24 ms, but a
@@ -170,9 +170,6 @@ __device__ __forceinline__ void slice_role_producer(const SfaParams& p, SliceCtl
     ++cur_j;
     return true;
   };
-  auto row_of = [&](int idx, int entry) -> int {  // 32 bits: the host side refuses caches of 2^31 rows or more
-    return static_cast<int>(tc_row_from_entry(p, idx, entry));
-  };
   uint4 d[2][2];  // [row pair][half]: this lane's 16 bytes of row 2 pair + rsel
   uint4 rope;     // unit lane % 8 of row lane / 8
   float4 sc;      // the four scales of row r
@@ -216,9 +213,9 @@ __device__ __forceinline__ void slice_role_producer(const SfaParams& p, SliceCtl
     const int e0 = has ? tc_table_entry(p, bi0, idx0) : kTableSkip;
     const int e1 = has_n ? tc_table_entry(p, bi_n, idx_n) : kTableSkip;
     if (has_a) entry_a = tc_table_entry(p, bi_a, idx_a);
-    if (has) issue_loads(row_of(idx0, e0));
+    if (has) issue_loads(tc_row_from_entry(p, idx0, e0));
     if (has_n) {
-      row_n = row_of(idx_n, e1);
+      row_n = tc_row_from_entry(p, idx_n, e1);
       prefetch_row(row_n);
     }
   }
@@ -261,7 +258,7 @@ __device__ __forceinline__ void slice_role_producer(const SfaParams& p, SliceCtl
     has = has_n;
     has_n = has_a;
     if (has_a) {
-      row_n = row_of(idx_a, entry_a);
+      row_n = tc_row_from_entry(p, idx_a, entry_a);
       prefetch_row(row_n);
     }
     has_a = has_b;

@@ -173,6 +173,28 @@ def test_merge_of_splits(tokens):
     _check(_run(d), want)
 
 
+@pytest.mark.parametrize("nq", [128, 16])
+@pytest.mark.parametrize("block_size", [1, 2, 3, 100, 4096])  # the kernels divide a position by it through a reciprocal
+def test_block_sizes_address_the_same_rows(block_size, nq):
+    n = 1201
+    d = gen.make_inputs([n], s1=1, seed=5, with_indexer=False, with_topk=True, attn_heads=nq)
+    rows = d.block_table[0].long()[torch.arange(n) // 128] * 128 + torch.arange(n) % 128  # row of each position
+    pages = -(-n // block_size)
+    order = torch.randperm(pages, generator=torch.Generator().manual_seed(block_size))    # where each page of the new cache lies
+    place = order[torch.arange(n) // block_size] * block_size + torch.arange(n) % block_size
+    total = pages * block_size
+    kn, kr, ks = (torch.zeros(total, x.shape[1], dtype=x.dtype) for x in (d.key_nope_2d, d.key_rope_2d, d.k_nope_scales))
+    for dst, src in ((kn, d.key_nope_2d), (kr, d.key_rope_2d), (ks, d.k_nope_scales)):
+        dst[place] = src[rows]
+    out = torch.zeros((1, 1, nq, 512), dtype=torch.bfloat16, device=DEV)
+    pto.sparse_flash_attention_quant_d(d.query_nope.to(DEV), d.query_rope.to(DEV), kn.to(DEV), kr.to(DEV), ks.to(DEV),
+                                       d.topk_indices.to(DEV), order.to(torch.int32)[None].contiguous().to(DEV),
+                                       d.act_seq_key.to(DEV), out, nq, 1, SCALE, 2048, block_size, pages)
+    torch.cuda.synchronize()
+    assert pto.workspace_status()[0] == 0
+    assert torch.equal(out.cpu(), _run(d, nq=nq))
+
+
 def test_order_of_indices_does_not_matter_beyond_rounding():
     d = gen.make_inputs([5000], s1=1, seed=2, with_indexer=False, with_topk=True)
     a = _run(d)
