@@ -13,10 +13,14 @@
 //   q.K^T  (M = 128 heads, N = 128 keys of a tile, K = 576): A = this CTA's 64 query rows, B = the tile's keys,
 //          of which CTA c gathers and dequantises keys [64c, 64c+64) in full width (9 chunks of 64 dims).
 //   P.V    (M = 128 heads, N = 256 of the 512 values per MMA, K = 128 keys): A = this CTA's P, B = V, of which
-//          CTA c supplies the value columns [256c, 256c+256) of ALL 128 keys. Shared memory between the SMs
-//          moves about 7 bytes per clock (measured: a 32 KB bulk copy to the peer takes 4-5 k cycles), far too
-//          slow to ship the other CTA's keys over, so a second group of producers gathers that half of all
-//          128 rows again (an L2 hit: the other CTA has just fetched the row) and dequantises it.
+//          CTA c supplies the value columns [256c, 256c+256) of ALL 128 keys. Those of its own 64 keys are the chunks 4c ..
+//          4c+3 of its K tile, the same bytes (K-major there, MN-major here). Those of the peer's keys it gathers (an L2
+//          hit: the other CTA has just fetched the row) and dequantises itself, since shared memory between the SMs moves
+//          about 7 bytes per clock (measured: a 32 KB bulk copy to the peer takes 4-5 k cycles); they go into the other
+//          four chunks of the K tile once q.K^T has read those, while the softmax works.
+//          So a tile needs 64 + 8 KB of shared memory, two tiles are in flight, and a row is dequantised one and a half
+//          times. (With regions of their own for K and V, one tile each, every row was dequantised twice: 4096 tokens x
+//          2048 rows 3.75 -> 3.35 ms, 64 tokens 79 -> 74 us behind a selection, 2 tokens 18.5 -> 16.6 us with the merge.)
 // Tensor memory of a 2-SM MMA with 64 rows per CTA: lanes 0-63 hold the first half of the N columns, lanes
 // 64-127 the second half (row = lane % 64). So of a score tile lane l holds (head l % 64, keys 64 (l / 64) ..+63),
 // and of O lane l holds (head l % 64, values 256 (l / 64) ..+255).
@@ -26,7 +30,7 @@
 //   warps 0, 1, 2   CTA 1: forward the "ready" events of their CTA to CTA 0 (tcgen05.commit arrivals on CTA 0's barriers)
 //   warps 4..11     softmax: four threads per head (two TMEM lanes x two column halves), P goes to shared memory
 //   warps 12..19    K producers: 16-byte gathers of the CTA's 64 rows, int8 -> bf16 in registers, swizzled stores
-//   warps 20..27    V producers: this CTA's half of the value columns of all 128 rows
+//   warps 20..27    V producers: this CTA's half of the value columns of the peer's 64 rows; rope parts of the CTA's own
 // Cache formats: int8 latent + bf16 rope + fp32 scales in three arrays, the same as packed 656-byte rows, or bf16
 // latent + rope arrays (the non-quantised cache): there the producers dequantise nothing, they copy the rows' bytes
 // from L2 to the same swizzled places with cp.async once their part of the buffer is free. The MMAs, the softmax and the
@@ -47,11 +51,12 @@ constexpr int kPRows = 64;               // rows a CTA gathers in full width per
 constexpr int kChunk = kPRows * 128;     // 64 rows x 64 bf16 (128-byte rows, 128-byte swizzle): 8 KB
 constexpr int kQChunks = 9;              // 8 latent chunks + 1 rope chunk
 constexpr int kSmemQ = 0;
-constexpr int kSmemK = kSmemQ + kQChunks * kChunk;        // 73,728
-constexpr int kSmemV = kSmemK + kQChunks * kChunk;        // 147,456: two regions (keys 0-63, keys 64-127) of 4 chunks
-constexpr int kSmemP = kSmemV + 8 * kChunk;               // 212,992: two chunks (keys 0-63, keys 64-127)
+constexpr int kSmemT = kSmemQ + kQChunks * kChunk;        // 73,728: two tile buffers of eight latent chunks
+constexpr int kTileBytes = 8 * kChunk;
+constexpr int kVHalfBytes = 4 * kChunk;                   // 64 keys x 256 values: half of a tile buffer
+constexpr int kSmemRope = kSmemT + 2 * kTileBytes;        // 204,800: rope chunk of a tile
+constexpr int kSmemP = kSmemRope + kChunk;                // 212,992: two chunks (keys 0-63, keys 64-127)
 constexpr int kSmemCtl = kSmemP + 2 * kChunk;             // 229,376
-constexpr int kVHalfBytes = 4 * kChunk;                   // 32 KB: 64 keys x 256 values
 constexpr int kPairSoftmaxWarp0 = 4, kPairSoftmaxWarps = 8;
 constexpr int kPairKWarp0 = 12, kPairKWarps = 8;
 constexpr int kPairVWarp0 = 20, kPairVWarps = 8;
@@ -60,21 +65,23 @@ constexpr uint32_t kPairTmemCols = 512;
 constexpr uint32_t kPairColO = 0, kPairColS = 256;        // S buffer b at kPairColS + 64 b
 constexpr float kPairRescale = 8.0f;
 
+// Tile buffer b = j % 2 of tile j; half h of it = chunks 4h .. 4h+3. In CTA c a half goes through
+//   half c:      K of the CTA's own 64 keys (chunks 4c .. 4c+3) for q.K^T, then, the same bytes, V of those keys
+//   half 1 - c:  K of its own keys (the other four chunks), then V (columns 256c ..) of the peer's keys
+// so that half h holds, in both CTAs, V of the keys 64h .. 64h+63 when P.V reads it. The rope chunk of tile j+1 is copied when
+// q.K^T of tile j has read its predecessor, by the V producers along with V of tile j: event j+1 of `vfull` (event 0: rope of
+// tile 0). Barriers that may complete for tile j+1 before everybody has waited for tile j exist once per buffer.
 struct PairCtl {
-  // The K chunks are handed over in halves, the V regions in quarters, so that the refill of one runs behind the MMAs
-  // that read the others: K half h = chunks 4h .. 4h+3 (h = 1: and the rope chunk); V quarter q = keys 32q .. +31.
-  // The loop convert -> notice of the other CTA -> MMAs -> hand-back -> convert is a chain of latencies of about 3 k
-  // cycles beside the work itself; in halves a tile could not take less than that chain plus half its conversion.
-  uint64_t kfull[2];   // K producers filled half h of this CTA's K chunks of tile j     (4 warps)
-  uint64_t kfree[2];   // the q.K^T MMAs that read half h are complete                   (tcgen05.commit, both CTAs)
-  uint64_t vfull[4];   // V producers filled this CTA's V rows of key quarter q          (2 warps)
-  uint64_t vfree[4];   // the P.V MMAs that read key quarter q are complete              (tcgen05.commit, both CTAs)
-  uint64_t sfull[2];   // q.K^T of a tile complete (score buffer b)                      (tcgen05.commit, both CTAs)
-  uint64_t pvdone;     // P.V of a tile complete                                        (tcgen05.commit, both CTAs)
-  uint64_t pfull;      // this CTA's P of tile j written                                (8 warps)
-  uint64_t sread[2];   // this CTA's softmax warps have the scores in registers         (8 warps)
+  uint64_t kfull[2][2];  // [b][h] K producers filled half h of buffer b               (4 warps)
+  uint64_t kread[2];     // the q.K^T MMAs that read half 0 of buffer b are complete   (tcgen05.commit, both CTAs)
+  uint64_t vfull[2];     // [event % 2] V of tile event - 1, rope of tile event        (8 warps)
+  uint64_t bfree[2][2];  // [b][h] the P.V MMAs that read half h are complete          (tcgen05.commit, both CTAs)
+  uint64_t sfull[2];     // q.K^T of a tile complete (score buffer b)                  (tcgen05.commit, both CTAs)
+  uint64_t pvdone;       // P.V of a tile complete                                    (tcgen05.commit, both CTAs)
+  uint64_t pfull;        // this CTA's P of tile j written                            (8 warps)
+  uint64_t sread[2];     // this CTA's softmax warps have the scores in registers     (8 warps)
   // in CTA 0 only: the same events of CTA 1, forwarded (one arrival each)
-  uint64_t kpeer[2], vpeer[4], ppeer, speer[2];
+  uint64_t kpeer[2][2], vpeer[2], ppeer, speer[2];
   uint32_t tmem_base;
   int abort;
   int go[2];           // outcome of the softmax role's latest waits
@@ -211,9 +218,10 @@ __device__ __forceinline__ uint32_t pair_setup_sync(PairCtl* ctl) {
 
 // ================================ MMA issuers (CTA 0) ===========================================
 // Two threads on two different schedulers: warp 0 issues the score products, warp 2 the value products.
-//   q.K^T first half  (chunks 0-3: 16 MMAs)  needs K half 0 of the tile and the score buffer it overwrites read
-//   q.K^T second half (chunks 4-8: 20 MMAs)  needs K half 1; completes the tile's scores
-//   P.V quarter q     (keys 32q .. +31: 4 MMAs)  needs P of the tile and V key quarter q; the last completes the tile's P.V
+//   q.K^T half 0  (chunks 0-3: 16 MMAs)  needs K half 0 of the tile and the score buffer it overwrites read
+//   q.K^T half 1  (chunks 4-7: 16 MMAs)  needs K half 1
+//   q.K^T rope    (chunk 8: 4 MMAs)      needs the rope chunk; completes the tile's scores
+//   P.V half h    (keys 64h .. +63: 8 MMAs)  needs P of the tile and V of the keys; the second completes the tile's P.V
 // After each action a commit hands the part it read back to its producers, so that the refill for the next tile
 // runs behind the MMAs that read the others. One thread issuing everything was what a tile waited for: 36 + 16 MMAs kept it
 // busy for 8.7 k cycles per tile (two threads: 80.1 -> 77.7 us on 64 tokens x 2048 rows). The products of the two threads
@@ -238,15 +246,17 @@ __device__ __forceinline__ bool pair_poll(uint32_t bar, uint32_t parity) {  // w
   }
 }
 
-// half kH of the score product into score buffer `d`: four latent chunks, with the second half the rope chunk too
-template <int kH>
-__device__ __forceinline__ void pair_issue_qk_half(uint32_t d, uint64_t a_desc, uint64_t b_desc) {
+// part kPart of the score product of buffer kB into score buffer kB: four latent chunks, or (2) the rope chunk
+template <int kB, int kPart>
+__device__ __forceinline__ void pair_issue_qk(uint32_t tmem_base, uint64_t a_desc, uint64_t b_desc) {
   constexpr uint32_t idesc_qk = umma_idesc(kCFmtF32, kABFmtBF16, kABFmtBF16, 0, 0, 128, kPT);
 #pragma unroll
-  for (int ch = 4 * kH; ch < (kH == 0 ? 4 : kQChunks); ++ch) {
+  for (int ch = 4 * kPart; ch < (kPart == 2 ? kQChunks : 4 * kPart + 4); ++ch) {
+    const int kch = kPart == 2 ? (kSmemRope - kSmemT) / kChunk : kB * 8 + ch;  // chunks from the first tile buffer on
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      mma2_f16_ss(d, a_desc + ch * (kChunk >> 4) + 2 * k, b_desc + ch * (kChunk >> 4) + 2 * k, idesc_qk, (ch | k) != 0 ? 1u : 0u);
+      mma2_f16_ss(tmem_base + kPairColS + 64 * kB, a_desc + ch * (kChunk >> 4) + 2 * k, b_desc + kch * (kChunk >> 4) + 2 * k, idesc_qk,
+                  (ch | k) != 0 ? 1u : 0u);
     }
   }
 }
@@ -257,28 +267,27 @@ __device__ __forceinline__ void pair_role_issue_qk(const SfaParams& p, PairCtx c
   PairCtl* ctl = c.ctl;
   const int ntiles = c.ntiles;
   const uint32_t tmem_base = pair_setup_sync(ctl);
-  const uint64_t a_desc = umma_desc_kmajor_sw128(c.base + kSmemQ), b_desc = umma_desc_kmajor_sw128(c.base + kSmemK);
+  const uint64_t a_desc = umma_desc_kmajor_sw128(c.base + kSmemQ), b_desc = umma_desc_kmajor_sw128(c.base + kSmemT);
   bool ok = true;
   for (int j = 0; j < ntiles && ok; ++j) {
-    const uint32_t ph = j & 1;
+    const uint32_t b = j & 1, ph = (j >> 1) & 1;
     if (j >= 2) {  // the score buffer it overwrites has been read in both CTAs
-      const uint32_t sp = ((j - 2) >> 1) & 1;
-      ok = pair_poll(smem_u32(&ctl->sread[j & 1]), sp) && pair_poll(smem_u32(&ctl->speer[j & 1]), sp);
+      ok = pair_poll(smem_u32(&ctl->sread[b]), ph ^ 1) && pair_poll(smem_u32(&ctl->speer[b]), ph ^ 1);
     }
-    const uint32_t d = tmem_base + kPairColS + 64 * (j & 1);
-#define PAIR_QK_HALF(q)                                                                                      \
-  ok = ok && pair_poll(smem_u32(&ctl->kfull[q]), ph) && pair_poll(smem_u32(&ctl->kpeer[q]), ph);                \
+#define PAIR_QK_PART(part, mine, peer, done)                                                                    \
+  ok = ok && pair_poll(smem_u32(&(mine)), ph) && pair_poll(smem_u32(&(peer)), ph);                              \
   if (!ok) break;                                                                                               \
   tc_fence_after();                                                                                             \
   if (elect_one()) {                                                                                            \
-    pair_issue_qk_half<q>(d, a_desc, b_desc);                                                                \
-    tc2_commit(smem_u32(&ctl->kfree[q]));                                                                       \
-    if ((q) == 1) tc2_commit(smem_u32(&ctl->sfull[j & 1]));                                                     \
+    if (b == 0) pair_issue_qk<0, part>(tmem_base, a_desc, b_desc);                                              \
+    else pair_issue_qk<1, part>(tmem_base, a_desc, b_desc);                                                     \
+    if ((part) != 1) tc2_commit(smem_u32(&(done)));                                                             \
   }                                                                                                             \
   __syncwarp();
-    PAIR_QK_HALF(0)
-    PAIR_QK_HALF(1)
-#undef PAIR_QK_HALF
+    PAIR_QK_PART(0, ctl->kfull[b][0], ctl->kpeer[b][0], ctl->kread[b])
+    PAIR_QK_PART(1, ctl->kfull[b][1], ctl->kpeer[b][1], ctl->kread[b])
+    PAIR_QK_PART(2, ctl->vfull[b], ctl->vpeer[b], ctl->sfull[b])
+#undef PAIR_QK_PART
   }
   if (!ok && (threadIdx.x & 31) == 0) {
     ctl->abort = 1;
@@ -287,19 +296,17 @@ __device__ __forceinline__ void pair_role_issue_qk(const SfaParams& p, PairCtx c
   __syncwarp();
 }
 
-// keys 32 kQ .. +31 of a tile into both pairs of value columns
-template <int kQ>
-__device__ __forceinline__ void pair_issue_pv_quarter(uint32_t d, uint64_t a_desc, uint64_t b_desc, uint32_t accumulate) {
+// keys 64 kH .. +63 of the tile in buffer kB into both pairs of value columns
+template <int kB, int kH>
+__device__ __forceinline__ void pair_issue_pv(uint32_t d, uint64_t a_desc, uint64_t b_desc, uint32_t accumulate) {
   constexpr uint32_t idesc_pv = umma_idesc(kCFmtF32, kABFmtBF16, kABFmtBF16, 0, 1, 128, 256);
 #pragma unroll
   for (int dp = 0; dp < 2; ++dp) {
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      constexpr int kh = kQ >> 1;
-      const int k = 2 * (kQ & 1) + e;
-      mma2_f16_ss(d + 128 * dp, a_desc + kh * (kChunk >> 4) + 2 * k,
-                  b_desc + ((kh * kVHalfBytes + dp * 2 * kChunk + k * 16 * 128) >> 4), idesc_pv,
-                  (kQ > 0 || e > 0) ? 1u : accumulate);
+    for (int k = 0; k < 4; ++k) {
+      mma2_f16_ss(d + 128 * dp, a_desc + kH * (kChunk >> 4) + 2 * k,
+                  b_desc + ((kB * kTileBytes + kH * kVHalfBytes + dp * 2 * kChunk + k * 16 * 128) >> 4), idesc_pv,
+                  (kH > 0 || k > 0) ? 1u : accumulate);
     }
   }
 }
@@ -310,26 +317,26 @@ __device__ __forceinline__ void pair_role_issue_pv(const SfaParams& p, PairCtx c
   PairCtl* ctl = c.ctl;
   const int ntiles = c.ntiles;
   const uint32_t tmem_base = pair_setup_sync(ctl);
-  const uint64_t a_desc = umma_desc_kmajor_sw128(c.base + kSmemP), b_desc = desc_mnmajor_sw128(c.base + kSmemV, kChunk, 1024);
+  const uint64_t a_desc = umma_desc_kmajor_sw128(c.base + kSmemP), b_desc = desc_mnmajor_sw128(c.base + kSmemT, kChunk, 1024);
   bool ok = true;
   for (int j = 0; j < ntiles && ok; ++j) {
-    const uint32_t ph = j & 1;
-    ok = pair_poll(smem_u32(&ctl->pfull), ph) && pair_poll(smem_u32(&ctl->ppeer), ph);
-#define PAIR_PV_QUARTER(q)                                                                                      \
-  ok = ok && pair_poll(smem_u32(&ctl->vfull[q]), ph) && pair_poll(smem_u32(&ctl->vpeer[q]), ph);                \
+    const uint32_t b = j & 1, pp = j & 1, ev = (j + 1) & 1, eph = ((j + 1) >> 1) & 1;
+    ok = pair_poll(smem_u32(&ctl->pfull), pp) && pair_poll(smem_u32(&ctl->ppeer), pp);
+    // V of the keys that are not a CTA's own: keys 0-63 in CTA 1, 64-127 in CTA 0
+#define PAIR_PV_HALF(h, bar)                                                                                    \
+  ok = ok && pair_poll(smem_u32(&(bar)), eph);                                                                  \
   if (!ok) break;                                                                                               \
   tc_fence_after();                                                                                             \
   if (elect_one()) {                                                                                            \
-    pair_issue_pv_quarter<q>(tmem_base + kPairColO, a_desc, b_desc, j > 0 ? 1u : 0u);                           \
-    tc2_commit(smem_u32(&ctl->vfree[q]));                                                                       \
-    if ((q) == 3) tc2_commit(smem_u32(&ctl->pvdone));                                                           \
+    if (b == 0) pair_issue_pv<0, h>(tmem_base + kPairColO, a_desc, b_desc, j > 0 ? 1u : 0u);                    \
+    else pair_issue_pv<1, h>(tmem_base + kPairColO, a_desc, b_desc, j > 0 ? 1u : 0u);                           \
+    tc2_commit(smem_u32(&ctl->bfree[b][h]));                                                                    \
+    if ((h) == 1) tc2_commit(smem_u32(&ctl->pvdone));                                                           \
   }                                                                                                             \
   __syncwarp();
-    PAIR_PV_QUARTER(0)
-    PAIR_PV_QUARTER(1)
-    PAIR_PV_QUARTER(2)
-    PAIR_PV_QUARTER(3)
-#undef PAIR_PV_QUARTER
+    PAIR_PV_HALF(0, ctl->vpeer[ev])
+    PAIR_PV_HALF(1, ctl->vfull[ev])
+#undef PAIR_PV_HALF
   }
   if (!ok && (threadIdx.x & 31) == 0) {
     ctl->abort = 1;
@@ -349,24 +356,26 @@ __device__ __forceinline__ void pair_role_relay(const SfaParams& p, PairCtx c) {
   const int ntiles = c.ntiles;
   pair_setup_sync(ctl);
   bool ok = true;
-  for (int j = 0; j < ntiles && ok; ++j) {
-    const uint32_t ph = j & 1;
+  for (int j = 0; j < (kWhat == kRelayV ? ntiles + 1 : ntiles) && ok; ++j) {  // (V: events)
+    const uint32_t b = j & 1, ph = (j >> 1) & 1;
     if (kWhat == kRelayP) {
       if (j < ntiles - 2) {  // scores of tile j read: only tiles that have a successor two on
-        ok = pair_poll(smem_u32(&ctl->sread[j & 1]), (j >> 1) & 1);
-        if (ok && elect_one()) pair_signal(smem_u32(&ctl->speer[j & 1]));
+        ok = pair_poll(smem_u32(&ctl->sread[b]), ph);
+        if (ok && elect_one()) pair_signal(smem_u32(&ctl->speer[b]));
         __syncwarp();
       }
-      ok = ok && pair_poll(smem_u32(&ctl->pfull), ph);
+      ok = ok && pair_poll(smem_u32(&ctl->pfull), j & 1);
       if (ok && elect_one()) pair_signal(smem_u32(&ctl->ppeer));
       __syncwarp();
+    } else if (kWhat == kRelayV) {
+      ok = pair_poll(smem_u32(&ctl->vfull[b]), ph);
+      if (ok && elect_one()) pair_signal(smem_u32(&ctl->vpeer[b]));
+      __syncwarp();
     } else {
-      uint64_t* full = kWhat == kRelayK ? ctl->kfull : ctl->vfull;
-      uint64_t* peer = kWhat == kRelayK ? ctl->kpeer : ctl->vpeer;
 #pragma unroll
-      for (int q = 0; q < (kWhat == kRelayK ? 2 : 4); ++q) {
-        ok = ok && pair_poll(smem_u32(&full[q]), ph);
-        if (ok && elect_one()) pair_signal(smem_u32(&peer[q]));
+      for (int h = 0; h < 2; ++h) {
+        ok = ok && pair_poll(smem_u32(&ctl->kfull[b][h]), ph);
+        if (ok && elect_one()) pair_signal(smem_u32(&ctl->kpeer[b][h]));
         __syncwarp();
       }
     }
@@ -499,13 +508,13 @@ __device__ __forceinline__ void pair_role_softmax(const SfaParams& p, PairCtx c)
   }
   // The rows go out through shared memory: a thread holds 128 values of ONE row, so direct stores put every lane of
   // a warp on its own 128-byte line (4096 lines per CTA, about 4 k cycles); staged, a warp writes 512 contiguous
-  // bytes. Staging area: the K chunks (all q.K^T of this cluster are complete once the last P.V is), rows of
+  // bytes. Staging area: the tile buffers (all products of this cluster are complete once the last P.V is), rows of
   // 1 KB + 16 B (the pad keeps the lanes of a warp, which write different rows, on different banks); a row holds
   // the 256-byte pieces of the head's four threads. bf16 rows take one pass, fp32 partial rows two.
   {
-    const uint32_t stage = c.base + kSmemK;
+    const uint32_t stage = c.base + kSmemT;
     constexpr uint32_t kStageRow = 1024 + 16;
-    static_assert(64 * kStageRow <= kQChunks * kChunk, "output staging exceeds the K chunks");
+    static_assert(64 * kStageRow <= 2 * kTileBytes, "output staging exceeds the tile buffers");
     const int stid = threadIdx.x - 32 * kPairSoftmaxWarp0;       // 0..255
     const uint32_t my_piece = stage + head * kStageRow + slot * 256;
     const bool direct = p.n_split == 1;
@@ -575,7 +584,7 @@ __device__ __forceinline__ void pair_role_softmax(const SfaParams& p, PairCtx c)
 
 // ================================ K producers ===================================================
 // Eight warps, four per half of the K chunks: warp (half, g) converts the half (256 bytes of latent: two lines of 128
-// dims, each with its scale) of the CTA's rows 16g .. 16g+15; the warps of half 1 also copy the rope part. Every warp
+// dims, each with its scale) of the CTA's rows 16g .. 16g+15. Every warp
 // waits for its own half, so the load of a half, its conversion, the notice and the MMAs that read it overlap those of
 // the other, and each warp pays the hand-over (wait, fence, arrive) once per tile. (All eight warps walking through
 // quarters together paid it four times: 7.9 k cycles per tile instead of 6.5 k. Two warps per quarter, each one line of 32
@@ -592,7 +601,7 @@ __device__ __forceinline__ void pair_role_softmax(const SfaParams& p, PairCtx c)
 // rope arrays (the non-quantised cache). With a bf16 cache nothing passes through registers: when the half is free
 // every lane issues its 16-byte `cp.async` copies from L2 (the rows were prefetched there two tiles ago) straight to
 // the swizzled places the dequantised units would go, waits for them, fences and arrives.
-// A padding or rejected row reads row 0 with scale 0, which dequantises to zeros (its rope part is zero-filled).
+// A padding or rejected row reads row 0 with scale 0, which dequantises to zeros.
 template <int kFmt>
 __device__ __forceinline__ void pair_role_kproducer(const SfaParams& p, const PairCtx c) {
   constexpr bool kPacked = kFmt == 1, kBf = kFmt == 2;
@@ -606,7 +615,7 @@ __device__ __forceinline__ void pair_role_kproducer(const SfaParams& p, const Pa
   const int my_row = 64 * static_cast<int>(c.crank) + 16 * g + (lane & 15);  // key of the tile this lane looks ahead for
   const int32_t* idx_ptr = c.idx_row + c.begin + my_row;
   const int n_mine = c.end - (c.begin + my_row);  // entry j * 128 of idx_ptr is valid iff j * 128 < n_mine
-  constexpr int stride_n = kPacked ? 656 : (kBf ? 1024 : 512), stride_r = kPacked ? 656 : 128, stride_s = kPacked ? 656 : 16;
+  constexpr int stride_n = kPacked ? 656 : (kBf ? 1024 : 512), stride_s = kPacked ? 656 : 16;
   // (the base pointers are read from the parameter block where they are used: they would otherwise occupy six
   // registers across the whole tile loop)
 #define PAIR_KN reinterpret_cast<const uint8_t*>(p.kn)
@@ -628,22 +637,22 @@ __device__ __forceinline__ void pair_role_kproducer(const SfaParams& p, const Pa
     sc = 0.f;
     if (phys >= 0) asm volatile("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(sc) : "l"(PAIR_SCL + static_cast<int64_t>(phys) * stride_s + half * 8 + (lane >> 4) * 4));
   };
-  auto prefetch_row = [&](int phys) {  // lanes r and r + 16: a line each of the half row; half 1 also the rest of the row
+  auto prefetch_row = [&](int phys) {  // lanes r and r + 16: a line each of the half row; half 0 also the rope part, half 1 the scales
     if (phys < 0) return;
     const int l = lane >> 4;
     if (kBf) {
       const uint8_t* a = PAIR_KN + static_cast<int64_t>(phys) * 1024 + half * 512 + l * 256;
       asm volatile("prefetch.global.L2 [%0];" ::"l"(a));
       asm volatile("prefetch.global.L2 [%0];" ::"l"(a + 128));
-      if (half == 1 && l == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(PAIR_ROPE + static_cast<int64_t>(phys) * 128));
+      if (half == 0 && l == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(PAIR_ROPE + static_cast<int64_t>(phys) * 128));
     } else if (kPacked) {
       if (half == 0 && lane < 16) bulk_prefetch_l2(PAIR_KN + static_cast<int64_t>(phys) * 656, 656);
     } else {
       asm volatile("prefetch.global.L2 [%0];" ::"l"(PAIR_KN + static_cast<int64_t>(phys) * 512 + half * 256 + l * 128));
-      if (half == 1) asm volatile("prefetch.global.L2 [%0];" ::"l"(l == 0 ? PAIR_ROPE + static_cast<int64_t>(phys) * 128 : PAIR_SCL + static_cast<int64_t>(phys) * 16));
+      if (l == half) asm volatile("prefetch.global.L2 [%0];" ::"l"(half == 0 ? PAIR_ROPE + static_cast<int64_t>(phys) * 128 : PAIR_SCL + static_cast<int64_t>(phys) * 16));
     }
   };
-  const uint32_t k_rows = c.base + kSmemK + (4 * half + cp) * kChunk + (16 * g + r4) * 128;  // row r4 of this lane's chunk of line 0
+  const uint32_t k_rows0 = c.base + kSmemT + (4 * half + cp) * kChunk + (16 * g + r4) * 128;  // row r4 of this lane's chunk of line 0
   bool ok = true;
   pair_setup_arrive();
   pdl_wait();          // the selected indices come from the kernel before this one, which may still be running
@@ -665,19 +674,12 @@ __device__ __forceinline__ void pair_role_kproducer(const SfaParams& p, const Pa
     prefetch_row(row_n);
   }
   for (int j = 0; j < ntiles; ++j) {
-    if (j > 0) {  // the q.K^T MMAs of the previous tile that read this half of the chunks are complete
-      ok = pair_wait(smem_u32(&ctl->kfree[half]), (j - 1) & 1);
+    const uint32_t b2 = j & 1;
+    if (j >= 2) {  // the P.V MMAs that read this half of the buffer are complete
+      ok = pair_wait(smem_u32(&ctl->bfree[b2][half]), ((j >> 1) - 1) & 1);
       if (!ok) break;
     }
-    if (half == 1) {  // the rope part goes straight from L2 to shared memory behind the conversion below
-#pragma unroll
-      for (int m = 0; m < 4; ++m) {  // rows 4m + lane / 8 of the warp's 16
-        const int r = 4 * m + (lane >> 3);
-        const int pr = __shfl_sync(0xffffffffu, row_cur, r);
-        cp_async_16(c.base + kSmemK + 8 * kChunk + (16 * g + r) * 128 + (((lane & 7) ^ (r & 7)) << 4),
-                    PAIR_ROPE + (pr >= 0 ? static_cast<int64_t>(pr) * stride_r + (lane & 7) * 16 : 0), pr >= 0 ? 16u : 0u);
-      }
-    }
+    const uint32_t k_rows = k_rows0 + b2 * kTileBytes;
 #pragma unroll
     for (int m = 0; m < 4; ++m) {  // row 4m + r4: swizzle term 4 (m % 2) + r4
       const int x = 4 * (m & 1) + r4;
@@ -698,11 +700,11 @@ __device__ __forceinline__ void pair_role_kproducer(const SfaParams& p, const Pa
         }
       }
     }
-    if (kBf || half == 1) asm volatile("cp.async.wait_all;" ::: "memory");
+    if (kBf) asm volatile("cp.async.wait_all;" ::: "memory");
     fence_proxy_async();
     if (j == 0) pair_setup_wait();
     __syncwarp();
-    if (lane == 0) mbar_arrive(smem_u32(&ctl->kfull[half]));
+    if (lane == 0) mbar_arrive(smem_u32(&ctl->kfull[b2][half]));
     if (j + 1 < ntiles) issue_loads(row_n);  // the half rows of tile j+1 (in L2: prefetched a tile ago)
     row_cur = row_n;
     row_n = tc_row_from_entry(p, idx_a, entry_a);     // tile j+2: into L2
@@ -718,65 +720,87 @@ __device__ __forceinline__ void pair_role_kproducer(const SfaParams& p, const Pa
 }
 
 // ================================ V producers ===================================================
-// Eight warps, two per key quarter: warp (q, h) converts this CTA's half of the value columns (256 of the 512 latent
-// bytes: two lines) of the 16 rows with keys 32q + 16h .. +15, lanes arranged as in the K producers (the other CTA's K
-// producers have fetched or are fetching the same lines: L2 hits). Lane r % 16 walks the look-ahead chain of row r (no
-// L2 prefetch: the row's owner issues it).
+// Eight warps; warp v converts this CTA's half of the value columns (256 of the 512 latent bytes: two lines) of the peer's
+// rows 8v .. 8v+7, lanes arranged as in the K producers (the other CTA's K producers have fetched or are fetching the same
+// lines: L2 hits), and copies the rope parts of the CTA's own rows 8v .. 8v+7 of the next tile. Lane r < 8 walks the look-ahead
+// chain of the peer's row 8v + r, lane 8 + r that of its own row 8v + r one tile later (no L2 prefetch: the row's owner issues it).
+// What it may overwrite: V goes where q.K^T of the same tile has read K (CTA 1: half 0, early; CTA 0: half 1), the rope part
+// where q.K^T has read the tile's own.
 template <int kFmt>
 __device__ __forceinline__ void pair_role_vproducer(const SfaParams& p, const PairCtx c) {
   constexpr bool kPacked = kFmt == 1, kBf = kFmt == 2;
   PairCtl* ctl = c.ctl;
   const int ntiles = c.ntiles;
   const int lane = threadIdx.x & 31;
-  const int vtid = threadIdx.x - kPairVWarp0 * 32;
-  const int q = vtid >> 6, h = (vtid >> 5) & 1;
+  const int v = (threadIdx.x >> 5) - kPairVWarp0;
+  const int crank = static_cast<int>(c.crank);
   const int u = lane & 3, r4 = (lane >> 2) & 3, cp = lane >> 4;
   const int line_off = cp * 64 + u * 16;  // this lane's 16 bytes of a line
-  const int my_row = 32 * q + 16 * h + (lane & 15);  // key of the tile this lane looks ahead for
+  const bool for_rope = (lane & 8) != 0;
+  const int my_row = 8 * v + (lane & 7) + (for_rope ? 64 * crank + kPT : 64 * (1 - crank));  // key this lane looks ahead for, from tile j's first on
   const int32_t* idx_ptr = c.idx_row + c.begin + my_row;
   const int n_mine = c.end - (c.begin + my_row);
-  const int col0 = 256 * static_cast<int>(c.crank);  // first latent byte of this CTA's value columns
-  constexpr int stride_n = kPacked ? 656 : (kBf ? 1024 : 512), stride_s = kPacked ? 656 : 16;
-  uint4 d[4][2];   // [m][line]: this lane's 16 bytes of the line of row 4m + r4
-  float sc = 0.f;  // scale lane / 16 (of this CTA's two) of row lane % 16
+  const int col0 = 256 * crank;  // first latent byte of this CTA's value columns
+  constexpr int stride_n = kPacked ? 656 : (kBf ? 1024 : 512), stride_r = kPacked ? 656 : 128, stride_s = kPacked ? 656 : 16;
+  uint4 d[2][2];   // [m][line]: this lane's 16 bytes of the line of row 4m + r4
+  float sc = 0.f;  // scale lane / 16 (of this CTA's two) of row lane % 8
   auto load_idx = [&](int j) -> int { return (j < ntiles && j * kPT < n_mine) ? ldg_pinned_i32(idx_ptr + j * kPT) : -1; };
   auto issue_loads = [&](int phys) {
     if (kBf) return;
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
+    for (int m = 0; m < 2; ++m) {
       const int pm = max(__shfl_sync(0xffffffffu, phys, 4 * m + r4), 0);
       const uint8_t* src = PAIR_KN + static_cast<int64_t>(pm) * stride_n + col0 + line_off;
       d[m][0] = ldg_pinned_v4(src);
       d[m][1] = ldg_pinned_v4(src + 128);
     }
+    const int ps = __shfl_sync(0xffffffffu, phys, lane & 7);
     sc = 0.f;
-    if (phys >= 0) asm volatile("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(sc) : "l"(PAIR_SCL + static_cast<int64_t>(phys) * stride_s + (col0 >> 5) + (lane >> 4) * 4));
+    if (ps >= 0) asm volatile("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(sc) : "l"(PAIR_SCL + static_cast<int64_t>(ps) * stride_s + (col0 >> 5) + (lane >> 4) * 4));
   };
-  // row r4 of this warp's 16 in this lane's chunk of line 0; line 1 lies two chunks further
-  const uint32_t v_rows = c.base + kSmemV + (q >> 1) * kVHalfBytes + cp * kChunk + (32 * (q & 1) + 16 * h + r4) * 128;
+  auto copy_rope = [&](int phys) {  // rows in lanes 8 .. 15; a padding or rejected row becomes zeros
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      const int r = 4 * m + (lane >> 3);
+      const int pr = __shfl_sync(0xffffffffu, phys, 8 + r);
+      cp_async_16(c.base + kSmemRope + (8 * v + r) * 128 + (((lane & 7) ^ r) << 4),
+                  PAIR_ROPE + (pr >= 0 ? static_cast<int64_t>(pr) * stride_r + (lane & 7) * 16 : 0), pr >= 0 ? 16u : 0u);
+    }
+  };
+  // row r4 of this warp's 8 in this lane's chunk of line 0; line 1 lies two chunks further
+  const uint32_t v_rows0 = c.base + kSmemT + (1 - crank) * kVHalfBytes + cp * kChunk + (8 * v + r4) * 128;
   bool ok = true;
   pair_setup_arrive();
   pdl_wait();
   int row_cur, row_n, idx_a, entry_a, idx_b;  // this lane's row of tiles j, j+1; index and block-table entry of j+2; index of j+3
   {
+    const int first = for_rope && n_mine > -kPT ? ldg_pinned_i32(idx_ptr - kPT) : -1;  // rope of tile 0
     const int idx0 = load_idx(0), idx1 = load_idx(1);
     idx_a = load_idx(2);
     idx_b = load_idx(3);
+    const int ef = tc_table_entry(p, c.bi, first);
     const int e0 = tc_table_entry(p, c.bi, idx0);
     const int e1 = tc_table_entry(p, c.bi, idx1);
     entry_a = tc_table_entry(p, c.bi, idx_a);
+    copy_rope(tc_row_from_entry(p, first, ef));
     row_cur = tc_row_from_entry(p, idx0, e0);
     issue_loads(row_cur);
     row_n = tc_row_from_entry(p, idx1, e1);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    fence_proxy_async();
+    pair_setup_wait();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(smem_u32(&ctl->vfull[0]));
   }
   for (int j = 0; j < ntiles; ++j) {
-    if (j > 0) {  // the P.V MMAs of the previous tile that read this key quarter are complete
-      ok = pair_wait(smem_u32(&ctl->vfree[q]), (j - 1) & 1);
-      if (!ok) break;
-    }
+    const uint32_t b2 = j & 1, ph = (j >> 1) & 1;
+    ok = pair_wait(smem_u32(crank == 0 ? &ctl->sfull[b2] : &ctl->kread[b2]), ph);
+    if (!ok) break;
+    if (crank == 0 && j + 1 < ntiles) copy_rope(row_cur);
+    const uint32_t v_rows = v_rows0 + b2 * kTileBytes;
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {  // row 4m + r4
-      const int x = 4 * (m & 1) + r4;
+    for (int m = 0; m < 2; ++m) {  // row 4m + r4
+      const int x = 4 * m + r4;
       const uint32_t a = ((2 * u) ^ x) << 4, b = ((2 * u + 1) ^ x) << 4;
 #pragma unroll
       for (int l = 0; l < 2; ++l) {
@@ -788,17 +812,21 @@ __device__ __forceinline__ void pair_role_vproducer(const SfaParams& p, const Pa
           cp_async_16(row_addr + b, src + (pm >= 0 ? 16 : 0), pm >= 0 ? 16u : 0u);
         } else {
           const float scale = __shfl_sync(0xffffffffu, sc, 16 * l + 4 * m + r4);
-          const uint4 v = d[m][l];
-          sts_v4u(row_addr + a, pair_dequant8(v.x, v.y, scale));
-          sts_v4u(row_addr + b, pair_dequant8(v.z, v.w, scale));
+          const uint4 w = d[m][l];
+          sts_v4u(row_addr + a, pair_dequant8(w.x, w.y, scale));
+          sts_v4u(row_addr + b, pair_dequant8(w.z, w.w, scale));
         }
       }
     }
-    if (kBf) asm volatile("cp.async.wait_all;" ::: "memory");
+    if (crank == 1 && j + 1 < ntiles) {
+      ok = pair_wait(smem_u32(&ctl->sfull[b2]), ph);
+      if (!ok) break;
+      copy_rope(row_cur);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     fence_proxy_async();
-    if (j == 0) pair_setup_wait();
     __syncwarp();
-    if (lane == 0) mbar_arrive(smem_u32(&ctl->vfull[q]));
+    if (lane == 0) mbar_arrive(smem_u32(&ctl->vfull[b2 ^ 1]));  // event j + 1
     if (j + 1 < ntiles) issue_loads(row_n);
     row_cur = row_n;
     row_n = tc_row_from_entry(p, idx_a, entry_a);
@@ -885,14 +913,14 @@ sfa_pair_kernel(const __grid_constant__ SfaParams p) {
       mbar_init(smem_u32(&ctl->sfull[b]), 1);
       mbar_init(smem_u32(&ctl->sread[b]), kPairSoftmaxWarps);
       mbar_init(smem_u32(&ctl->speer[b]), 1);
-      mbar_init(smem_u32(&ctl->kfull[b]), kPairKWarps / 2);
-      mbar_init(smem_u32(&ctl->kfree[b]), 1);
-      mbar_init(smem_u32(&ctl->kpeer[b]), 1);
-    }
-    for (int q = 0; q < 4; ++q) {
-      mbar_init(smem_u32(&ctl->vfull[q]), kPairVWarps / 4);
-      mbar_init(smem_u32(&ctl->vfree[q]), 1);
-      mbar_init(smem_u32(&ctl->vpeer[q]), 1);
+      mbar_init(smem_u32(&ctl->kread[b]), 1);
+      mbar_init(smem_u32(&ctl->vfull[b]), kPairVWarps);
+      mbar_init(smem_u32(&ctl->vpeer[b]), 1);
+      for (int h = 0; h < 2; ++h) {
+        mbar_init(smem_u32(&ctl->kfull[b][h]), kPairKWarps / 2);
+        mbar_init(smem_u32(&ctl->kpeer[b][h]), 1);
+        mbar_init(smem_u32(&ctl->bfree[b][h]), 1);
+      }
     }
     ctl->abort = 0;
     fence_mbar_init();
