@@ -22,7 +22,7 @@
 //                   groups of four warps, half of the heads each
 //   warps 12..      producers, four rows of a tile each: gather, int8 -> bf16, swizzled stores
 // What bounds it: the chain gather -> conversion -> scores -> softmax -> products over two tile buffers. 4096 tokens x 2048 rows
-// x 16 heads take 1.98 ms, i.e. 5.2 k cycles per tile of 80 rows (2.11 ms with all heads in four softmax warps), of which the MMAs' issue is 2184 (one with N = 16 takes 39
+// x 16 heads take 1.90 ms, i.e. 5.0 k cycles per tile of 80 rows (2.11 ms with all heads in four softmax warps), of which the MMAs' issue is 2184 (one with N = 16 takes 39
 // cycles, measured in isolation, and there are 36 + 4 kTK/16 of them); the counters show no unit more than half busy (issue slots
 // 46 %, tensor pipe 7 %, L2 16 %).
 // Why bf16: a form that multiplied the rows as int8, queries and probabilities as fixed-point limbs, took 1.24 ms, but a
@@ -254,8 +254,10 @@ __device__ __forceinline__ void slice_role_producer(const SfaParams& p, SliceCtl
     fence_proxy_async();
     __syncwarp();
     if (lane == 0) mbar_arrive(smem_u32(&ctl->full[b]));
-    if (has_n) issue_loads(row_n);
+    // The look-ahead comes before the row loads: what it waits for was requested a tile ago, but a wait behind the row loads
+    // is a wait for these too (loads share the few scoreboards of a warp).
     has = has_n;
+    const int row_next = row_n;
     has_n = has_a;
     if (has_a) {
       row_n = tc_row_from_entry(p, idx_a, entry_a);
@@ -264,6 +266,7 @@ __device__ __forceinline__ void slice_role_producer(const SfaParams& p, SliceCtl
     has_a = has_b;
     idx_a = idx_b;
     if (has_b) entry_a = tc_table_entry(p, bi_b, idx_b);
+    if (has) issue_loads(row_next);
   }
   if (!ok && lane == 0) {
     ctl->abort = 1;
