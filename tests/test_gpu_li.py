@@ -394,6 +394,33 @@ def test_topk_stage_over_row_lengths_and_distributions(rows, n, k, kind, sort):
 
 
 @pytest.mark.parametrize("sort", [True, False], ids=["ordered", "unordered"])
+@pytest.mark.parametrize("n", [6148, 8193, 30001, 100003])  # chunks of a row: fewer than, as many as and more than are in flight
+@pytest.mark.parametrize("kind", ["normal", "ties", "last"])
+def test_many_rows_two_to_an_sm(kind, n, sort):
+    """More rows than two per SM, in several rounds; every third row is short."""
+    rows, k = 700, 2048
+    g = torch.Generator(device=DEV).manual_seed(n)
+    sc = torch.randn(rows, (n + 127) // 128 * 128, generator=g, device=DEV)
+    if kind == "ties":
+        sc = (sc * 3).round() / 3 + 0.0
+    elif kind == "last":
+        sc[:, n - 3000:n] += 20.0
+    act = torch.full((rows,), n, dtype=torch.int32, device=DEV)
+    act[::3] = torch.randint(1, n, (len(act[::3]),), generator=g, device=DEV, dtype=torch.int32)
+    out = torch.full((rows, 1, k), -7, dtype=torch.int32, device=DEV)
+    pto.lightning_indexer_topk(sc, act, out, 1, k, sort=sort)
+    torch.cuda.synchronize()
+    assert pto.workspace_status()[0] == 0
+    inside = torch.arange(sc.shape[1], device=DEV)[None] < act[:, None]
+    order = torch.where(inside, sc, -torch.inf).sort(dim=1, descending=True, stable=True).indices[:, :k]
+    want = torch.where(torch.arange(k, device=DEV)[None] < act[:, None], order, -1)
+    got = out[:, 0].long()
+    if not sort:
+        got, want = got.sort(dim=1).values, want.sort(dim=1).values
+    assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("sort", [True, False], ids=["ordered", "unordered"])
 @pytest.mark.parametrize("rows,n", [(8, 32768), (40, 65536), (160, 20000), (3, 131072),  # clusters of 4, 2, 1 and 8 CTAs
                                     (1, 5000000)])  # a sample of its own size
 @pytest.mark.parametrize("where", ["last", "runs", "aligned", "scattered"])
