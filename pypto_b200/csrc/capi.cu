@@ -4,6 +4,7 @@
 #include <cuda.h>
 #include <dlfcn.h>
 
+#include <algorithm>
 #include <climits>
 #include <cstdarg>
 #include <cstdlib>
@@ -138,21 +139,22 @@ size_t li_scores_bytes(int t, int max_blocks, int block_size) {
   return align_up(static_cast<size_t>(t) * max_blocks * block_size * sizeof(float), 256);
 }
 
-int sfa_split(int t, int nq) {
+constexpr int kSfaSplitLastRoundRows = 1024;
+pto::SfaSplit sfa_split(int t, int nq) {
   if (nq == 128) return pto::sfa_pair_split(t, 148);  // one cluster of two CTAs per (token, split)
   const int n_hb = nq / pto::sfa_slice_heads(nq);
   const long long ctas = static_cast<long long>(t) * n_hb;
-  if (ctas >= 148) return 1;
+  if (ctas >= 148) return {0, 1};
   long long s = 148 / (ctas > 0 ? ctas : 1);
   if (s > 32) s = 32;
   if (s < 1) s = 1;
-  return static_cast<int>(s);
+  return {0, static_cast<int>(s)};
 }
 
 size_t sfa_part_bytes(int t, int nq) {
-  const int ns = sfa_split(t, nq);
-  if (ns == 1) return 0;
-  const size_t rows = static_cast<size_t>(t) * ns * nq;
+  const pto::SfaSplit sp = sfa_split(t, nq);
+  if (sp.n == 1) return 0;
+  const size_t rows = static_cast<size_t>(t - sp.begin) * sp.n * nq;
   return align_up(rows * 2 * sizeof(float), 256) + align_up(rows * 512 * sizeof(float), 256);
 }
 
@@ -305,8 +307,10 @@ int run_sfa(const void* qn, const void* qr, const void* kn, const void* kr, cons
   int rc = get_device_info(&di);
   if (rc != PTO_OK) return rc;
   const int t = b * s1;
-  const int ns = sfa_split(t, nq);
-  if (ns > 1 && part_bytes < sfa_part_bytes(t, nq)) return fail(PTO_ERR_WORKSPACE, "attention workspace too small");
+  pto::SfaSplit sp = sfa_split(t, nq);
+  // a split costs the merge's launch, 2.5 us: where a round of pairs has gone before and a token's rows are few tiles, more than it gains
+  if (sp.begin > 0 && std::min<long long>(topk, static_cast<long long>(max_blocks) * block_size) < kSfaSplitLastRoundRows) sp = {0, 1};
+  if (sp.n > 1 && part_bytes < sfa_part_bytes(t, nq)) return fail(PTO_ERR_WORKSPACE, "attention workspace too small");
   pto::SfaParams p{};
   p.q_nope = reinterpret_cast<const __nv_bfloat16*>(qn);
   p.q_rope = reinterpret_cast<const __nv_bfloat16*>(qr);
@@ -317,8 +321,8 @@ int run_sfa(const void* qn, const void* qr, const void* kn, const void* kr, cons
   p.block_table = bt;
   p.act_seq = act;
   p.out = reinterpret_cast<__nv_bfloat16*>(out);
-  if (ns > 1) {
-    const size_t rows = static_cast<size_t>(t) * ns * nq;
+  if (sp.n > 1) {
+    const size_t rows = static_cast<size_t>(t - sp.begin) * sp.n * nq;
     p.part_ml = reinterpret_cast<float*>(part_base);
     p.part_o = reinterpret_cast<float*>(part_base + align_up(rows * 2 * sizeof(float), 256));
   }
@@ -334,7 +338,8 @@ int run_sfa(const void* qn, const void* qr, const void* kn, const void* kr, cons
   p.page_shift = 31 + l;
   p.page_mul = static_cast<uint32_t>((1ull << p.page_shift) / static_cast<uint32_t>(block_size) + 1);
   p.max_blocks = max_blocks;
-  p.n_split = ns;
+  p.n_split = sp.n;
+  p.split_begin = sp.begin;
   p.packed = packed ? 1 : 0;
   p.kn_bf16 = bf16 ? 1 : 0;
   p.pdl = behind_topk;

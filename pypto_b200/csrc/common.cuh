@@ -337,9 +337,10 @@ struct SfaParams {
   const int32_t* block_table;   // [b, max_blocks]
   const int32_t* act_seq;       // [b]
   __nv_bfloat16* out;           // [t, nq_total, 512]
-  float* part_o;                // [t, n_split, nq, 512]
-  float* part_ml;               // [t, n_split, nq, 2]
+  float* part_o;                // [t - split_begin, n_split, nq, 512]
+  float* part_ml;               // [t - split_begin, n_split, nq, 2]
   int b, s1, nq, nq_total, head_begin, topk_k, block_size, max_blocks, n_split, packed, kn_bf16;
+  int split_begin;  // first token whose rows are split (n_split > 1); the ones before it are one piece each
   uint32_t page_mul;  // position / block_size = position * page_mul >> page_shift, for every position below 2^31: a division by an
   int page_shift;     // integer that the kernel does not know is about 35 instructions (Granlund and Montgomery 1994)
   int pdl;  // launched behind the top-k kernel with programmatic serialization: setup overlaps the selection
@@ -354,7 +355,10 @@ cudaError_t launch_li_score_simt(const LiParams& p, cudaStream_t stream);
 cudaError_t launch_li_topk(const TopkParams& p, int num_sms, cudaStream_t stream, bool pdl);  // pdl: behind its score kernel
 cudaError_t launch_sfa(const SfaParams& p, int num_sms, cudaStream_t stream);
 cudaError_t launch_sfa_pair(const SfaParams& p, cudaStream_t stream);     // nq == 128, any cache format: 2-SM MMAs, heads split over the pair
-int sfa_pair_split(int t, int num_sms);
+struct SfaSplit {
+  int begin, n;  // tokens from `begin` on are split n ways
+};
+SfaSplit sfa_pair_split(int t, int num_sms);
 cudaError_t launch_sfa_slice(const SfaParams& p, int num_sms, cudaStream_t stream);  // other head counts, int8 caches
 int sfa_slice_heads(int nq);  // heads per work item of that kernel
 

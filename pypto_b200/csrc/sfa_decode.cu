@@ -31,11 +31,11 @@ sfa_combine_kernel(SfaParams p, int rows) {
   constexpr int kVec = 4 / kWarps;                 // float4 per lane and split
   constexpr int kGroup = kWarps == 1 ? 4 : 16;     // splits asked for together
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int th = blockIdx.x * (4 / kWarps) + warp / kWarps;  // token * nq + head
+  const int th = blockIdx.x * (4 / kWarps) + warp / kWarps;  // (token - split_begin) * nq + head
   pdl_wait();  // launched with programmatic serialization behind the kernel that writes the partials
   if (th >= rows) return;
-  const int ti = th / p.nq, head = th % p.nq;
-  const int64_t prow0 = static_cast<int64_t>(ti) * p.n_split * p.nq + head;  // row of split 0; splits are nq rows apart
+  const int pt = th / p.nq, ti = p.split_begin + pt, head = th % p.nq;
+  const int64_t prow0 = static_cast<int64_t>(pt) * p.n_split * p.nq + head;  // row of split 0; splits are nq rows apart
   const int col = (warp % kWarps) * 128 + lane * 4;                          // first value of this lane; the next float4 128 on
   float mi = -INFINITY, li = 0.f;
   if (lane < p.n_split) {
@@ -102,7 +102,7 @@ cudaError_t launch_sfa(const SfaParams& p, int num_sms, cudaStream_t stream) {
     if (p.n_split > kMaxSplit) return cudaErrorInvalidValue;
     count_launch();
     // may be scheduled while the attention kernel drains; its first instruction waits for that grid
-    const int rows = t * p.nq;
+    const int rows = (t - p.split_begin) * p.nq;
     e = p.n_split > 4 ? launch_maybe_pdl(sfa_combine_kernel<4>, dim3(rows), dim3(128), 0, stream, true, p, rows)
                       : launch_maybe_pdl(sfa_combine_kernel<1>, dim3((rows + 3) / 4), dim3(128), 0, stream, true, p, rows);
   }

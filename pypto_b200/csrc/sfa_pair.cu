@@ -188,7 +188,8 @@ struct PairCtx {
   const int32_t* idx_row;  // this token's selected positions
   int64_t q_row0;          // first query/output row of the token
   uint32_t base, tmem_base, crank;
-  int ntiles, begin, end, ti, sp, bi;
+  int ntiles, begin, end, sp, bi;
+  int pt;  // token among those that are split, or -1: the rows are one piece, the output is written as it is
 };
 
 // The one meeting of all threads of the pair before the tile loop (barriers initialised, tensor memory allocated, both Q
@@ -517,7 +518,7 @@ __device__ __forceinline__ void pair_role_softmax(const SfaParams& p, PairCtx c)
     static_assert(64 * kStageRow <= 2 * kTileBytes, "output staging exceeds the tile buffers");
     const int stid = threadIdx.x - 32 * kPairSoftmaxWarp0;       // 0..255
     const uint32_t my_piece = stage + head * kStageRow + slot * 256;
-    const bool direct = p.n_split == 1;
+    const bool direct = c.pt < 0;
     const float inv = l_tot > 0.f ? 1.f / l_tot : 0.f;
     const int npass = direct ? 1 : 2;
     if (ok) tc_fence_after();
@@ -554,7 +555,7 @@ __device__ __forceinline__ void pair_role_softmax(const SfaParams& p, PairCtx c)
           gbase = reinterpret_cast<uint8_t*>(p.out + (c.q_row0 + 64 * static_cast<int>(c.crank)) * 512);
           grow_bytes = 1024;
         } else {
-          const int64_t prow0 = (static_cast<int64_t>(c.ti) * p.n_split + c.sp) * p.nq + 64 * static_cast<int>(c.crank);
+          const int64_t prow0 = (static_cast<int64_t>(c.pt) * p.n_split + c.sp) * p.nq + 64 * static_cast<int>(c.crank);
           gbase = reinterpret_cast<uint8_t*>(p.part_o + prow0 * 512);
           grow_bytes = 2048;
         }
@@ -571,7 +572,7 @@ __device__ __forceinline__ void pair_role_softmax(const SfaParams& p, PairCtx c)
       if (ps + 1 < npass) asm volatile("bar.sync 1, 256;" ::: "memory");  // staging area reused by the next pass
     }
     if (ok && !direct && slot == 0) {
-      const int64_t prow = (static_cast<int64_t>(c.ti) * p.n_split + c.sp) * p.nq + 64 * static_cast<int>(c.crank) + head;
+      const int64_t prow = (static_cast<int64_t>(c.pt) * p.n_split + c.sp) * p.nq + 64 * static_cast<int>(c.crank) + head;
       p.part_ml[prow * 2] = m_seen;
       p.part_ml[prow * 2 + 1] = l_tot;
     }
@@ -859,11 +860,18 @@ sfa_pair_kernel(const __grid_constant__ SfaParams p) {
   c.crank = pair_ctarank();
   const uint32_t crank = c.crank;
   const int bid = blockIdx.x >> 1;  // cluster index
-  c.sp = bid % p.n_split;
-  c.ti = bid / p.n_split;
-  c.bi = c.ti / p.s1;
-  const int si = c.ti % p.s1;
-  c.q_row0 = static_cast<int64_t>(c.ti) * p.nq_total + p.head_begin;
+  c.sp = 0;
+  c.pt = -1;
+  int ti = bid, n_split = 1;
+  if (p.n_split > 1 && bid >= p.split_begin) {
+    n_split = p.n_split;
+    c.sp = (bid - p.split_begin) % n_split;
+    c.pt = (bid - p.split_begin) / n_split;
+    ti = p.split_begin + c.pt;
+  }
+  c.bi = ti / p.s1;
+  const int si = ti % p.s1;
+  c.q_row0 = static_cast<int64_t>(ti) * p.nq_total + p.head_begin;
 
   // This CTA's 64 query rows for shared memory, nine swizzled chunks of 64 dims (A operand of q.K^T): 64 x 72 16-byte
   // units, twelve per thread of the twelve warps that are not producers. Requested before the sequence length is there (it
@@ -884,21 +892,21 @@ sfa_pair_kernel(const __grid_constant__ SfaParams p) {
   int n = p.act_seq[c.bi] - p.s1 + 1 + si;
   n = max(0, min(n, p.topk_k));
   const int tiles_total = (n + kPT - 1) / kPT;
-  const int tiles_per_split = (tiles_total + p.n_split - 1) / p.n_split;
+  const int tiles_per_split = (tiles_total + n_split - 1) / n_split;
   c.begin = min(n, c.sp * tiles_per_split * kPT);
   c.end = min(n, (c.sp + 1) * tiles_per_split * kPT);
   c.ntiles = (c.end - c.begin + kPT - 1) / kPT;
-  c.idx_row = p.topk + static_cast<int64_t>(c.ti) * p.topk_k;
+  c.idx_row = p.topk + static_cast<int64_t>(ti) * p.topk_k;
 
   if (c.ntiles == 0) {  // same decision in both CTAs of the pair
-    if (p.n_split == 1) {
+    if (c.pt < 0) {
       for (int e = tid; e < 64 * 64; e += kPairThreads) {
         const int r = e >> 6, cc = e & 63;
         *reinterpret_cast<uint4*>(p.out + (c.q_row0 + 64 * crank + r) * 512 + cc * 8) = make_uint4(0, 0, 0, 0);
       }
     } else {
       for (int r = tid; r < 64; r += kPairThreads) {
-        float* ml = p.part_ml + ((static_cast<int64_t>(c.ti) * p.n_split + c.sp) * p.nq + 64 * crank + r) * 2;
+        float* ml = p.part_ml + ((static_cast<int64_t>(c.pt) * p.n_split + c.sp) * p.nq + 64 * crank + r) * 2;
         ml[0] = -INFINITY;
         ml[1] = 0.f;
       }
@@ -986,13 +994,14 @@ sfa_pair_kernel(const __grid_constant__ SfaParams p) {
 
 }  // namespace
 
-// split of a token's selected rows over clusters so that the grid fills the SM pairs once
-int sfa_pair_split(int t, int num_sms) {
-  const int pairs = num_sms / 2;
-  if (t >= pairs) return 1;
-  int s = pairs / (t > 0 ? t : 1);
-  if (s > 16) s = 16;
-  return s < 1 ? 1 : s;
+// Split of the tokens' selected rows over clusters: fewer tokens than SM pairs fill the pairs once; of more tokens, those that are
+// left over by whole rounds of pairs share the last round, if they leave half of it or more idle (256 tokens x 2048 rows, three
+// rounds and 34 tokens: 318 -> 300 us). Behind many rounds half a round is no gain that could be measured.
+constexpr int kPairSplitRounds = 8;
+SfaSplit sfa_pair_split(int t, int num_sms) {
+  const int pairs = num_sms / 2, rest = t % pairs;
+  const int begin = t - rest, n = rest > 0 && begin <= kPairSplitRounds * pairs ? pairs / rest : 1;
+  return n >= 2 ? SfaSplit{begin, n < 16 ? n : 16} : SfaSplit{0, 1};
 }
 
 cudaError_t launch_sfa_pair(const SfaParams& p, cudaStream_t stream) {
@@ -1001,7 +1010,7 @@ cudaError_t launch_sfa_pair(const SfaParams& p, cudaStream_t stream) {
   if (e != cudaSuccess) return e;
   const int t = p.b * p.s1;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(t) * p.n_split * 2, 1, 1);
+  cfg.gridDim = dim3((static_cast<unsigned>(p.split_begin) + static_cast<unsigned>(t - p.split_begin) * p.n_split) * 2, 1, 1);
   cfg.blockDim = dim3(kPairThreads, 1, 1);
   cfg.dynamicSmemBytes = kPairSmemBytes;
   cfg.stream = stream;

@@ -173,6 +173,18 @@ def test_merge_of_splits(tokens):
     _check(_run(d), want)
 
 
+@pytest.mark.parametrize("tokens", [74, 75, 111, 112, 149], ids=lambda t: f"{t}_tokens")  # rests of 0, 1, 37, 38 and 1: 1, 16, 2, 1 and 16 splits
+@pytest.mark.parametrize("longest", [700, 1500])  # rows of few tiles are not split behind a whole round
+def test_split_of_the_last_round(tokens, longest):
+    act = [(1, 130, 300, 5)[i % 4] for i in range(tokens)]
+    act[0] = act[73] = act[-1] = longest
+    d = gen.make_inputs(act, s1=1, seed=tokens, with_indexer=False, with_topk=True)
+    want = oracle.sparse_attention(d.query_nope, d.query_rope, d.key_nope_2d, d.key_rope_2d, d.k_nope_scales,
+                                   d.topk_indices, d.block_table, d.act_seq, d.s1)
+    _check(_run(d), want)
+    assert torch.equal(_run(d, bf16_cache=True), _run(d))
+
+
 @pytest.mark.parametrize("nq", [128, 16])
 @pytest.mark.parametrize("block_size", [1, 2, 3, 100, 4096])  # the kernels divide a position by it through a reciprocal
 def test_block_sizes_address_the_same_rows(block_size, nq):
