@@ -22,9 +22,11 @@
 //                   groups of four warps, half of the heads each
 //   warps 12..      producers, four rows of a tile each: gather, int8 -> bf16, swizzled stores
 // What bounds it: the chain gather -> conversion -> scores -> softmax -> products over two tile buffers. 4096 tokens x 2048 rows
-// x 16 heads take 1.90 ms, i.e. 5.0 k cycles per tile of 80 rows (2.11 ms with all heads in four softmax warps), of which the MMAs' issue is 2184 (one with N = 16 takes 39
-// cycles, measured in isolation, and there are 36 + 4 kTK/16 of them); the counters show no unit more than half busy (issue slots
-// 46 %, tensor pipe 7 %, L2 16 %).
+// x 16 heads take 1.84 ms, i.e. 4.8 k cycles per tile of 80 rows, of which the MMAs' issue is 2184 (one with N = 16 takes 39
+// cycles, measured in isolation, 32 of them for the 128 lanes of its A operand at the shared memory's 128 bytes a clock; there are
+// 36 + 4 kTK/16 of them). No unit is more than half busy: with all MMAs left out it takes 1.35, with all work of the producers left out
+// 1.5. All heads in four softmax warps 2.11 ms, two groups of them 2.00; look-ahead before the row loads 1.90; tiles handed over and
+// given back in halves, and 48 registers for the issuing warps, which spilled with 40, 1.84.
 // Why bf16: a form that multiplied the rows as int8, queries and probabilities as fixed-point limbs, took 1.24 ms, but a
 // fixed-point probability has an absolute error: beside a row with 0.96 of the weight the others rounded to zero (rel-L2
 // against 64 bits 0.22, 16 heads; this form 0.0020, the mma.sync kernel before it 0.0024).
@@ -56,9 +58,9 @@ struct SliceCfg {
   static constexpr uint32_t kColO = 2 * 5 * kHB;            // O block c at kColO + c * kHB
   static constexpr uint32_t kTmemCols = kHB == 16 ? 256 : 512;
   static_assert(kColO + 4 * kHB <= kTmemCols, "tensor memory");
-  // registers per thread: at launch, issuers / loaders, softmax, producers
+  // registers per thread: at launch, issuers / loaders, softmax, producers (nothing spills: a spilled register costs a trip to L2)
   static constexpr int kRegLaunch = kHB == 16 ? 64 : 72;
-  static constexpr int kRegIssue = 40, kRegSoftmax = kHB == 16 ? 72 : 104, kRegProd = 64;
+  static constexpr int kRegIssue = kHB == 16 ? 48 : 56, kRegSoftmax = kHB == 16 ? 72 : 96, kRegProd = 64;
   static_assert(128 * kRegIssue + 256 * kRegSoftmax + 32 * kProdWarps * kRegProd <= kThreads * kRegLaunch, "register split");
 };
 
@@ -69,8 +71,10 @@ struct SliceCtl {
   __align__(16) float mref[kHB];          // reference maximum of a head (log2 units)
   __align__(16) float alpha[kHB];
   float red[4][kHB];
-  uint64_t full[2];   // producers filled the tile buffer            (producer warps)
-  uint64_t done[2];   // P.V of the tile complete: tile buffer and P buffer free, O at rest (commit)
+  // Halves of a tile: chunks 0-3, then chunks 4-7, rope part and scales. Each is handed over as it is filled and given back as it is
+  // read, so that the scores of the first run beside the conversion of the second.
+  uint64_t full[2][2];  // [buffer][half] filled                      (producer warps)
+  uint64_t done[2][2];  // P.V of the half complete (commit); of the second: P buffer free, O at rest
   uint64_t sfull[2];  // scores of the tile complete                 (commit)
   uint64_t sfree[2];  // scores read                                 (8 softmax warps)
   uint64_t pfull[2];  // P^T of the tile written                     (8 softmax warps)
@@ -149,9 +153,10 @@ __device__ __forceinline__ void slice_role_producer(const SfaParams& p, SliceCtl
   const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) - 12;
   const int r = lane & 3, rsel = (lane >> 2) & 1;
   const int src_off = (((lane & 3) | ((lane >> 3) << 2)) << 4);  // this lane's 16 bytes of a half row
-  const uint8_t* const kn = reinterpret_cast<const uint8_t*>(p.kn);
-  const uint8_t* const kr = kPacked ? kn + 512 : reinterpret_cast<const uint8_t*>(p.kr);
-  const uint8_t* const ks = kPacked ? kn + 640 : reinterpret_cast<const uint8_t*>(p.kn_scales);
+  // (the base pointers are read from the parameter block where they are used: they would otherwise occupy six registers)
+#define SLICE_KN reinterpret_cast<const uint8_t*>(p.kn)
+#define SLICE_KR (kPacked ? SLICE_KN + 512 : reinterpret_cast<const uint8_t*>(p.kr))
+#define SLICE_KS (kPacked ? SLICE_KN + 640 : reinterpret_cast<const uint8_t*>(p.kn_scales))
   constexpr int stride_n = kPacked ? 656 : 512, stride_r = kPacked ? 656 : 128, stride_s = kPacked ? 656 : 16;
 
   int cur_item = blockIdx.x, cur_j = 0;
@@ -180,26 +185,26 @@ __device__ __forceinline__ void slice_role_producer(const SfaParams& p, SliceCtl
 #pragma unroll
     for (int pr = 0; pr < 2; ++pr) {
       const int pm = max(__shfl_sync(0xffffffffu, phys, 2 * pr + rsel), 0);
-      const uint8_t* src = kn + static_cast<int64_t>(pm) * stride_n + src_off;
+      const uint8_t* src = SLICE_KN + static_cast<int64_t>(pm) * stride_n + src_off;
       d[pr][0] = ldg_pinned_v4(src);
       d[pr][1] = ldg_pinned_v4(src + 256);
     }
     const int px = __shfl_sync(0xffffffffu, phys, lane >> 3);
     rope = make_uint4(0, 0, 0, 0);
-    if (px >= 0) rope = ldg_pinned_v4(kr + static_cast<int64_t>(px) * stride_r + (lane & 7) * 16);
+    if (px >= 0) rope = ldg_pinned_v4(SLICE_KR + static_cast<int64_t>(px) * stride_r + (lane & 7) * 16);
     uint4 s4 = make_uint4(0, 0, 0, 0);
-    if (phys >= 0) s4 = ldg_pinned_v4(ks + static_cast<int64_t>(phys) * stride_s);
+    if (phys >= 0) s4 = ldg_pinned_v4(SLICE_KS + static_cast<int64_t>(phys) * stride_s);
     sc = make_float4(__uint_as_float(s4.x), __uint_as_float(s4.y), __uint_as_float(s4.z), __uint_as_float(s4.w));
   };
   auto prefetch_row = [&](int phys) {  // lanes r, r+4, ...: one line of the row each
     if (phys < 0) return;
     const int l = lane >> 2;
     if (kPacked) {
-      if (l < 6) asm volatile("prefetch.global.L2 [%0];" ::"l"(kn + static_cast<int64_t>(phys) * 656 + min(l * 128, 640)));
+      if (l < 6) asm volatile("prefetch.global.L2 [%0];" ::"l"(SLICE_KN + static_cast<int64_t>(phys) * 656 + min(l * 128, 640)));
     } else {
-      if (l < 4) asm volatile("prefetch.global.L2 [%0];" ::"l"(kn + static_cast<int64_t>(phys) * 512 + l * 128));
-      else if (l == 4) asm volatile("prefetch.global.L2 [%0];" ::"l"(kr + static_cast<int64_t>(phys) * 128));
-      else if (l == 5) asm volatile("prefetch.global.L2 [%0];" ::"l"(ks + static_cast<int64_t>(phys) * 16));
+      if (l < 4) asm volatile("prefetch.global.L2 [%0];" ::"l"(SLICE_KN + static_cast<int64_t>(phys) * 512 + l * 128));
+      else if (l == 4) asm volatile("prefetch.global.L2 [%0];" ::"l"(SLICE_KR + static_cast<int64_t>(phys) * 128));
+      else if (l == 5) asm volatile("prefetch.global.L2 [%0];" ::"l"(SLICE_KS + static_cast<int64_t>(phys) * 16));
     }
   };
 
@@ -225,35 +230,36 @@ __device__ __forceinline__ void slice_role_producer(const SfaParams& p, SliceCtl
     // the tile after the next: index (requested now, used at the end of this step) and block-table entry
     int idx_b = -1, bi_b = 0;
     const bool has_b = has_a && fetch(idx_b, bi_b);
-    if (t >= 2) {
-      ok = slice_wait(smem_u32(&ctl->done[b]), ((t >> 1) - 1) & 1);
-      if (!ok) break;
-    }
     const uint32_t tile = base + Cfg::kSmemTile + b * Cfg::kTile;
 #pragma unroll
-    for (int pr = 0; pr < 2; ++pr) {
-      const int row = 4 * w + 2 * pr + rsel, x = row & 7;
-      const uint32_t dst = tile + (lane >> 3) * Cfg::kChunk + row * 128;
-      const uint32_t a = ((2 * (lane & 3)) ^ x) << 4, c = ((2 * (lane & 3) + 1) ^ x) << 4;
+    for (int hf = 0; hf < 2; ++hf) {
+      if (t >= 2) {
+        ok = slice_wait(smem_u32(&ctl->done[b][hf]), ((t >> 1) - 1) & 1);
+        if (!ok) break;
+      }
 #pragma unroll
-      for (int hf = 0; hf < 2; ++hf) {
+      for (int pr = 0; pr < 2; ++pr) {
+        const int row = 4 * w + 2 * pr + rsel, x = row & 7;
+        const uint32_t dst = tile + (4 * hf + (lane >> 3)) * Cfg::kChunk + row * 128;
+        const uint32_t a = ((2 * (lane & 3)) ^ x) << 4, c = ((2 * (lane & 3) + 1) ^ x) << 4;
         const uint4 v = d[pr][hf];
         const uint2 v0 = slice_cvt4(v.x), v1 = slice_cvt4(v.y), v2 = slice_cvt4(v.z), v3 = slice_cvt4(v.w);
-        sts_v4u(dst + hf * 4 * Cfg::kChunk + a, make_uint4(v0.x, v0.y, v1.x, v1.y));
-        sts_v4u(dst + hf * 4 * Cfg::kChunk + c, make_uint4(v2.x, v2.y, v3.x, v3.y));
+        sts_v4u(dst + a, make_uint4(v0.x, v0.y, v1.x, v1.y));
+        sts_v4u(dst + c, make_uint4(v2.x, v2.y, v3.x, v3.y));
       }
-    }
-    {
-      const int row = 4 * w + (lane >> 3);
-      sts_v4u(tile + 8 * Cfg::kChunk + row * 128 + (((lane & 7) ^ (row & 7)) << 4), rope);
-      if (lane < 4) {
-        *reinterpret_cast<float4*>(&ctl->scales[b][4 * w + lane][0]) = sc;
-        ctl->live[b][4 * w + lane] = row_loaded >= 0 ? 1.f : 0.f;
+      if (hf == 1) {
+        const int row = 4 * w + (lane >> 3);
+        sts_v4u(tile + 8 * Cfg::kChunk + row * 128 + (((lane & 7) ^ (row & 7)) << 4), rope);
+        if (lane < 4) {
+          *reinterpret_cast<float4*>(&ctl->scales[b][4 * w + lane][0]) = sc;
+          ctl->live[b][4 * w + lane] = row_loaded >= 0 ? 1.f : 0.f;
+        }
       }
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&ctl->full[b][hf]));
     }
-    fence_proxy_async();
-    __syncwarp();
-    if (lane == 0) mbar_arrive(smem_u32(&ctl->full[b]));
+    if (!ok) break;
     // The look-ahead comes before the row loads: what it waits for was requested a tile ago, but a wait behind the row loads
     // is a wait for these too (loads share the few scoreboards of a warp).
     has = has_n;
@@ -281,12 +287,12 @@ __device__ __forceinline__ void slice_role_producer(const SfaParams& p, SliceCtl
 // constants of the code for that (kBase, the address where a kernel without static shared memory finds its dynamic
 // part; kBase = 0 is the same code with the address in a register): 2.25 -> 2.05 ms for 4096 tokens of 16 heads.
 constexpr uint32_t kSliceUsualBase = 1024;
-template <int kHB, int kTK>
+template <int kHB, int kTK, int kHalf>
 __device__ __forceinline__ void slice_issue_scores(uint32_t d, uint64_t a_desc, uint64_t b_desc) {
   using Cfg = SliceCfg<kHB, kTK>;
   constexpr uint32_t idesc = umma_idesc(kCFmtF32, kABFmtBF16, kABFmtBF16, 0, 0, 128, kHB);
 #pragma unroll
-  for (int ch = 0; ch < kSliceChunks; ++ch) {  // accumulator ch / 2: one per scale tile, the rope part the fifth
+  for (int ch = 4 * kHalf; ch < (kHalf == 0 ? 4 : kSliceChunks); ++ch) {  // accumulator ch / 2: one per scale tile, the rope part the fifth
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       mma_f16_ss(d + (ch >> 1) * kHB, a_desc + ch * (Cfg::kChunk >> 4) + 2 * k, b_desc + ch * (Cfg::kQChunk >> 4) + 2 * k,
@@ -294,12 +300,12 @@ __device__ __forceinline__ void slice_issue_scores(uint32_t d, uint64_t a_desc, 
     }
   }
 }
-template <int kHB, int kTK>
+template <int kHB, int kTK, int kHalf>
 __device__ __forceinline__ void slice_issue_values(uint32_t d, uint64_t a_desc, uint64_t b_desc, uint32_t accumulate) {
   using Cfg = SliceCfg<kHB, kTK>;
   constexpr uint32_t idesc = umma_idesc(kCFmtF32, kABFmtBF16, kABFmtBF16, 1, 1, 128, kHB);
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
+  for (int c = 2 * kHalf; c < 2 * kHalf + 2; ++c) {
 #pragma unroll
     for (int k = 0; k < kTK / 16; ++k) {  // 16 rows per step: 2 KB of a chunk, 16 rows of the tile's copy of P^T
       mma_f16_ss(d + c * kHB, a_desc + c * (2 * Cfg::kChunk >> 4) + k * (2048 >> 4),
@@ -323,11 +329,17 @@ __device__ __forceinline__ void slice_role_scores(const SfaParams& p, SliceCtl<k
     for (int j = 0; j < ntiles && ok; ++j, ++t) {
       const uint32_t b = t & 1;
       if (t >= 2) ok = slice_wait(smem_u32(&ctl->sfree[b]), ((t >> 1) - 1) & 1);
-      ok = ok && slice_wait(smem_u32(&ctl->full[b]), (t >> 1) & 1);
+      ok = ok && slice_wait(smem_u32(&ctl->full[b][0]), (t >> 1) & 1);
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t d = tmem + Cfg::kColS + b * 5 * kHB;
+      if (elect_one()) slice_issue_scores<kHB, kTK, 0>(d, a_desc + b * (Cfg::kTile >> 4), b_desc);
+      __syncwarp();
+      ok = slice_wait(smem_u32(&ctl->full[b][1]), (t >> 1) & 1);
       if (!ok) break;
       tc_fence_after();
       if (elect_one()) {
-        slice_issue_scores<kHB, kTK>(tmem + Cfg::kColS + b * 5 * kHB, a_desc + b * (Cfg::kTile >> 4), b_desc);
+        slice_issue_scores<kHB, kTK, 1>(d, a_desc + b * (Cfg::kTile >> 4), b_desc);
         tc_commit(smem_u32(&ctl->sfull[b]));
         if (j + 1 == ntiles) tc_commit(smem_u32(&ctl->qfree));
       }
@@ -357,13 +369,15 @@ __device__ __forceinline__ void slice_role_values(const SfaParams& p, SliceCtl<k
     if (n > 0) ok = slice_wait(smem_u32(&ctl->ofree), (n - 1) & 1);
     for (int j = 0; j < ntiles && ok; ++j, ++t) {
       const uint32_t b = t & 1;
-      ok = slice_wait(smem_u32(&ctl->pfull[b]), (t >> 1) & 1) && slice_wait(smem_u32(&ctl->full[b]), (t >> 1) & 1);
+      ok = slice_wait(smem_u32(&ctl->pfull[b]), (t >> 1) & 1) && slice_wait(smem_u32(&ctl->full[b][1]), (t >> 1) & 1);
       if (!ok) break;
       tc_fence_after();
       if (elect_one()) {
-        slice_issue_values<kHB, kTK>(tmem + Cfg::kColO, a_desc + b * (Cfg::kTile >> 4), b_desc + b * (4 * Cfg::kPBytes >> 4),
-                                     j > 0 ? 1u : 0u);
-        tc_commit(smem_u32(&ctl->done[b]));
+        const uint64_t a = a_desc + b * (Cfg::kTile >> 4), pb = b_desc + b * (4 * Cfg::kPBytes >> 4);
+        slice_issue_values<kHB, kTK, 0>(tmem + Cfg::kColO, a, pb, j > 0 ? 1u : 0u);
+        tc_commit(smem_u32(&ctl->done[b][0]));
+        slice_issue_values<kHB, kTK, 1>(tmem + Cfg::kColO, a, pb, j > 0 ? 1u : 0u);
+        tc_commit(smem_u32(&ctl->done[b][1]));
       }
       __syncwarp();
     }
@@ -475,7 +489,7 @@ __device__ __forceinline__ void slice_role_softmax(const SfaParams& p, SliceCtl<
       const uint32_t b = t & 1;
       // (a wait that expired is voted on below, so that the group's four warps leave together: one that left alone would leave the
       // others at a barrier)
-      ok = ok && slice_wait(smem_u32(&ctl->sfull[b]), (t >> 1) & 1) && slice_wait(smem_u32(&ctl->full[b]), (t >> 1) & 1);
+      ok = ok && slice_wait(smem_u32(&ctl->sfull[b]), (t >> 1) & 1) && slice_wait(smem_u32(&ctl->full[b][1]), (t >> 1) & 1);
       tc_fence_after();
       float s[kH];
       float4 sc = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -527,7 +541,7 @@ __device__ __forceinline__ void slice_role_softmax(const SfaParams& p, SliceCtl<
         }
         slice_meet(group);
         if (j > 0) {
-          ok = slice_wait(smem_u32(&ctl->done[b ^ 1]), ((t - 1) >> 1) & 1);  // the output so far is at rest
+          ok = slice_wait(smem_u32(&ctl->done[b ^ 1][1]), ((t - 1) >> 1) & 1);  // the output so far is at rest
           if (ok) tc_fence_after();
 #pragma unroll
           for (int h = 0; h < kH; ++h) l[h] *= alpha[h];
@@ -559,7 +573,7 @@ __device__ __forceinline__ void slice_role_softmax(const SfaParams& p, SliceCtl<
         l[h] += s[h];
       }
       if (t >= 2) {  // the products that read this P buffer are complete
-        ok = slice_wait(smem_u32(&ctl->done[b]), ((t >> 1) - 1) & 1) && ok;
+        ok = slice_wait(smem_u32(&ctl->done[b][1]), ((t >> 1) - 1) & 1) && ok;
       }
       if (ok && key < kTK) {
         const float scv[4] = {sc.x, sc.y, sc.z, sc.w};
@@ -609,7 +623,7 @@ __device__ __forceinline__ void slice_role_softmax(const SfaParams& p, SliceCtl<
       }
     }
     slice_meet(group);
-    ok = slice_wait(smem_u32(&ctl->done[(t - 1) & 1]), ((t - 1) >> 1) & 1);
+    ok = slice_wait(smem_u32(&ctl->done[(t - 1) & 1][1]), ((t - 1) >> 1) & 1);
     tc_fence_after();
 #pragma unroll
     for (int c = 0; c < 4 && ok; ++c) {  // dim 128 c + key of every head: 32 lanes write consecutive dims of a head's row
@@ -649,8 +663,10 @@ sfa_slice_kernel(const __grid_constant__ SfaParams p, int n_items) {
   const int tid = threadIdx.x, warp = tid >> 5;
   if (tid == 0) {
     for (int b = 0; b < 2; ++b) {
-      mbar_init(smem_u32(&ctl->full[b]), Cfg::kProdWarps);
-      mbar_init(smem_u32(&ctl->done[b]), 1);
+      for (int hf = 0; hf < 2; ++hf) {
+        mbar_init(smem_u32(&ctl->full[b][hf]), Cfg::kProdWarps);
+        mbar_init(smem_u32(&ctl->done[b][hf]), 1);
+      }
       mbar_init(smem_u32(&ctl->sfull[b]), 1);
       mbar_init(smem_u32(&ctl->sfree[b]), 8);
       mbar_init(smem_u32(&ctl->pfull[b]), 8);
