@@ -183,6 +183,14 @@ __device__ __forceinline__ uint4 pair_dequant8(const uint32_t w0, const uint32_t
   return o;
 }
 
+// this lane's 32 bytes of a row: 32 values, half `part` of the chunk's 64
+__device__ __forceinline__ void pair_store_wide(uint32_t row_addr, int part, int x, const uint4 lo, const uint4 hi, float scale) {
+  sts_v4u(row_addr + (((4 * part) ^ x) << 4), pair_dequant8(lo.x, lo.y, scale));
+  sts_v4u(row_addr + (((4 * part + 1) ^ x) << 4), pair_dequant8(lo.z, lo.w, scale));
+  sts_v4u(row_addr + (((4 * part + 2) ^ x) << 4), pair_dequant8(hi.x, hi.y, scale));
+  sts_v4u(row_addr + (((4 * part + 3) ^ x) << 4), pair_dequant8(hi.z, hi.w, scale));
+}
+
 struct PairCtx {
   PairCtl* ctl;
   const int32_t* idx_row;  // this token's selected positions
@@ -599,13 +607,14 @@ __device__ __forceinline__ void pair_role_softmax(const SfaParams& p, PairCtx c)
 // Lane r % 16 also walks the look-ahead chain of row 16g + r: the selected index four tiles ahead, its block-table entry three
 // tiles ahead, an L2 prefetch of the half row two tiles ahead, the half row itself (by all lanes) one tile ahead.
 // kFmt: 0 = int8 latent, bf16 rope and fp32 scales in three arrays, 1 = packed 656-byte rows, 2 = bf16 latent and
-// rope arrays (the non-quantised cache). With a bf16 cache nothing passes through registers: when the half is free
+// rope arrays (the non-quantised cache), 3 = as 0 on a 32-byte boundary: 32 bytes a lane, half as many loads (kWide; a chunk of 4096
+// tokens over 131072 keys 10.03 -> 9.84 ms. Eight lanes of a store instruction are then both halves of four rows: eight different bank groups again). With a bf16 cache nothing passes through registers: when the half is free
 // every lane issues its 16-byte `cp.async` copies from L2 (the rows were prefetched there two tiles ago) straight to
 // the swizzled places the dequantised units would go, waits for them, fences and arrives.
 // A padding or rejected row reads row 0 with scale 0, which dequantises to zeros.
 template <int kFmt>
 __device__ __forceinline__ void pair_role_kproducer(const SfaParams& p, const PairCtx c) {
-  constexpr bool kPacked = kFmt == 1, kBf = kFmt == 2;
+  constexpr bool kPacked = kFmt == 1, kBf = kFmt == 2, kWide = kFmt == 3;
   PairCtl* ctl = c.ctl;
   const int ntiles = c.ntiles, bi = c.bi;
   const int lane = threadIdx.x & 31;
@@ -622,18 +631,29 @@ __device__ __forceinline__ void pair_role_kproducer(const SfaParams& p, const Pa
 #define PAIR_KN reinterpret_cast<const uint8_t*>(p.kn)
 #define PAIR_ROPE (kPacked ? PAIR_KN + 512 : reinterpret_cast<const uint8_t*>(p.kr))
 #define PAIR_SCL (kPacked ? PAIR_KN + 640 : reinterpret_cast<const uint8_t*>(p.kn_scales))
-  uint4 d[4][2];   // [m][line]: this lane's 16 bytes of the line of row 4m + r4
+  uint4 d[4][2];   // [m][line]: this lane's 16 bytes of the line of row 4m + r4 (kWide: [2m, 2m + 1][line]: its 32 bytes of row 8m + r8)
+  const int part = lane & 1, r8 = 4 * (lane >> 4) + ((lane >> 1) & 3), cpw = (lane >> 3) & 1;  // kWide
   float sc = 0.f;  // scale lane / 16 (of the half's two) of row lane % 16
   auto load_idx = [&](int j) -> int { return (j < ntiles && j * kPT < n_mine) ? ldg_pinned_i32(idx_ptr + j * kPT) : -1; };
   // `phys`: this lane's look-ahead row of the tile
   auto issue_loads = [&](int phys) {
     if (kBf) return;  // (copied from L2 when the buffer is free)
+    if constexpr (kWide) {
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        const int pm = max(__shfl_sync(0xffffffffu, phys, 8 * m + r8), 0);
+        const uint8_t* src = PAIR_KN + static_cast<int64_t>(pm) * stride_n + half * 256 + (2 * cpw + part) * 32;
+        ldg_pinned_v8(src, d[2 * m][0], d[2 * m + 1][0]);
+        ldg_pinned_v8(src + 128, d[2 * m][1], d[2 * m + 1][1]);
+      }
+    } else {
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
       const int pm = max(__shfl_sync(0xffffffffu, phys, 4 * m + r4), 0);
       const uint8_t* src = PAIR_KN + static_cast<int64_t>(pm) * stride_n + half * 256 + line_off;
       d[m][0] = ldg_pinned_v4(src);
       d[m][1] = ldg_pinned_v4(src + 128);
+    }
     }
     sc = 0.f;
     if (phys >= 0) asm volatile("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(sc) : "l"(PAIR_SCL + static_cast<int64_t>(phys) * stride_s + half * 8 + (lane >> 4) * 4));
@@ -681,6 +701,17 @@ __device__ __forceinline__ void pair_role_kproducer(const SfaParams& p, const Pa
       if (!ok) break;
     }
     const uint32_t k_rows = k_rows0 + b2 * kTileBytes;
+    if constexpr (kWide) {
+      const uint32_t rows = c.base + kSmemT + b2 * kTileBytes + (4 * half + cpw) * kChunk + (16 * g + r8) * 128;
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+#pragma unroll
+        for (int l = 0; l < 2; ++l) {
+          const float scale = __shfl_sync(0xffffffffu, sc, 16 * l + 8 * m + r8);
+          pair_store_wide(rows + 8 * m * 128 + l * 2 * kChunk, part, r8, d[2 * m][l], d[2 * m + 1][l], scale);
+        }
+      }
+    } else {
 #pragma unroll
     for (int m = 0; m < 4; ++m) {  // row 4m + r4: swizzle term 4 (m % 2) + r4
       const int x = 4 * (m & 1) + r4;
@@ -700,6 +731,7 @@ __device__ __forceinline__ void pair_role_kproducer(const SfaParams& p, const Pa
           sts_v4u(row_addr + b, pair_dequant8(v.z, v.w, scale));
         }
       }
+    }
     }
     if (kBf) asm volatile("cp.async.wait_all;" ::: "memory");
     fence_proxy_async();
@@ -731,7 +763,7 @@ __device__ __forceinline__ void pair_role_kproducer(const SfaParams& p, const Pa
 // where q.K^T has read the tile's own.
 template <int kFmt>
 __device__ __forceinline__ void pair_role_vproducer(const SfaParams& p, const PairCtx c) {
-  constexpr bool kPacked = kFmt == 1, kBf = kFmt == 2;
+  constexpr bool kPacked = kFmt == 1, kBf = kFmt == 2, kWide = kFmt == 3;
   PairCtl* ctl = c.ctl;
   const int ntiles = c.ntiles;
   const int lane = threadIdx.x & 31;
@@ -745,17 +777,25 @@ __device__ __forceinline__ void pair_role_vproducer(const SfaParams& p, const Pa
   const int n_mine = c.end - (c.begin + my_row);
   const int col0 = 256 * crank;  // first latent byte of this CTA's value columns
   constexpr int stride_n = kPacked ? 656 : (kBf ? 1024 : 512), stride_r = kPacked ? 656 : 128, stride_s = kPacked ? 656 : 16;
-  uint4 d[2][2];   // [m][line]: this lane's 16 bytes of the line of row 4m + r4
+  uint4 d[2][2];   // [m][line]: this lane's 16 bytes of the line of row 4m + r4 (kWide: [0, 1][line]: its 32 bytes of row r8)
+  const int part = lane & 1, r8 = 4 * (lane >> 4) + ((lane >> 1) & 3), cpw = (lane >> 3) & 1;  // kWide
   float sc = 0.f;  // scale lane / 16 (of this CTA's two) of row lane % 8
   auto load_idx = [&](int j) -> int { return (j < ntiles && j * kPT < n_mine) ? ldg_pinned_i32(idx_ptr + j * kPT) : -1; };
   auto issue_loads = [&](int phys) {
     if (kBf) return;
+    if constexpr (kWide) {
+      const int pm = max(__shfl_sync(0xffffffffu, phys, r8), 0);
+      const uint8_t* src = PAIR_KN + static_cast<int64_t>(pm) * stride_n + col0 + (2 * cpw + part) * 32;
+      ldg_pinned_v8(src, d[0][0], d[1][0]);
+      ldg_pinned_v8(src + 128, d[0][1], d[1][1]);
+    } else {
 #pragma unroll
-    for (int m = 0; m < 2; ++m) {
-      const int pm = max(__shfl_sync(0xffffffffu, phys, 4 * m + r4), 0);
-      const uint8_t* src = PAIR_KN + static_cast<int64_t>(pm) * stride_n + col0 + line_off;
-      d[m][0] = ldg_pinned_v4(src);
-      d[m][1] = ldg_pinned_v4(src + 128);
+      for (int m = 0; m < 2; ++m) {
+        const int pm = max(__shfl_sync(0xffffffffu, phys, 4 * m + r4), 0);
+        const uint8_t* src = PAIR_KN + static_cast<int64_t>(pm) * stride_n + col0 + line_off;
+        d[m][0] = ldg_pinned_v4(src);
+        d[m][1] = ldg_pinned_v4(src + 128);
+      }
     }
     const int ps = __shfl_sync(0xffffffffu, phys, lane & 7);
     sc = 0.f;
@@ -801,6 +841,14 @@ __device__ __forceinline__ void pair_role_vproducer(const SfaParams& p, const Pa
     if (!ok) break;
     if (crank == 0 && j + 1 < ntiles) copy_rope(row_cur);
     const uint32_t v_rows = v_rows0 + b2 * kTileBytes;
+    if constexpr (kWide) {
+      const uint32_t rows = c.base + kSmemT + b2 * kTileBytes + (1 - crank) * kVHalfBytes + cpw * kChunk + (8 * v + r8) * 128;
+#pragma unroll
+      for (int l = 0; l < 2; ++l) {
+        const float scale = __shfl_sync(0xffffffffu, sc, 16 * l + r8);
+        pair_store_wide(rows + l * 2 * kChunk, part, r8, d[0][l], d[1][l], scale);
+      }
+    } else {
 #pragma unroll
     for (int m = 0; m < 2; ++m) {  // row 4m + r4
       const int x = 4 * m + r4;
@@ -820,6 +868,7 @@ __device__ __forceinline__ void pair_role_vproducer(const SfaParams& p, const Pa
           sts_v4u(row_addr + b, pair_dequant8(w.z, w.w, scale));
         }
       }
+    }
     }
     if (crank == 1 && j + 1 < ntiles) {
       ok = pair_wait(smem_u32(&ctl->sfull[b2]), ph);
@@ -972,11 +1021,13 @@ sfa_pair_kernel(const __grid_constant__ SfaParams p) {
     PAIR_SETREG("setmaxnreg.inc.sync.aligned.u32 72;");  // (no change of the count; without it ptxas spills in this role)
     if (p.kn_bf16) pair_role_kproducer<2>(p, c);
     else if (p.packed) pair_role_kproducer<1>(p, c);
+    else if (p.kn_aligned32) pair_role_kproducer<3>(p, c);
     else pair_role_kproducer<0>(p, c);
   } else {
     PAIR_SETREG("setmaxnreg.dec.sync.aligned.u32 64;");
     if (p.kn_bf16) pair_role_vproducer<2>(p, c);
     else if (p.packed) pair_role_vproducer<1>(p, c);
+    else if (p.kn_aligned32) pair_role_vproducer<3>(p, c);
     else pair_role_vproducer<0>(p, c);
   }
 
