@@ -22,11 +22,11 @@
 //                   groups of four warps, half of the heads each
 //   warps 12..      producers, four rows of a tile each: gather, int8 -> bf16, swizzled stores
 // What bounds it: the chain gather -> conversion -> scores -> softmax -> products over two tile buffers. 4096 tokens x 2048 rows
-// x 16 heads take 1.84 ms, i.e. 4.8 k cycles per tile of 80 rows, of which the MMAs' issue is 2184 (one with N = 16 takes 39
+// x 16 heads take 1.82 ms, i.e. 4.8 k cycles per tile of 80 rows, of which the MMAs' issue is 2184 (one with N = 16 takes 39
 // cycles, measured in isolation, 32 of them for the 128 lanes of its A operand at the shared memory's 128 bytes a clock; there are
 // 36 + 4 kTK/16 of them). No unit is more than half busy: with all MMAs left out it takes 1.35, with all work of the producers left out
 // 1.5. All heads in four softmax warps 2.11 ms, two groups of them 2.00; look-ahead before the row loads 1.90; tiles handed over and
-// given back in halves, and 48 registers for the issuing warps, which spilled with 40, 1.84.
+// given back in halves, and 48 registers for the issuing warps, which spilled with 40, 1.84; 32-byte loads 1.82.
 // Why bf16: a form that multiplied the rows as int8, queries and probabilities as fixed-point limbs, took 1.24 ms, but a
 // fixed-point probability has an absolute error: beside a row with 0.96 of the weight the others rounded to zero (rel-L2
 // against 64 bits 0.22, 16 heads; this form 0.0020, the mma.sync kernel before it 0.0024).
@@ -144,10 +144,12 @@ __device__ __forceinline__ uint2 slice_cvt4(uint32_t w) {
 // ================================ producers =====================================================
 // Warp w owns rows 4w .. 4w+3 of every tile. A gather instruction reads half the latent bytes of two rows (four whole
 // 128-byte lines); the eight lanes of a quarter-warp hold four 16-byte units of two neighbouring rows, whose swizzle
-// terms differ in the lowest bit, so their stores hit eight different bank groups. Lane r % 4 walks the look-ahead chain
+// terms differ in the lowest bit, so their stores hit eight different bank groups. (kWide, latent rows on
+// 32-byte boundaries: half the latent bytes of all four rows, 32 bytes a lane; eight lanes hold both halves of a 64-dim chunk of
+// four rows.) Lane r % 4 walks the look-ahead chain
 // of row 4w + r: selected index three tiles ahead, block-table entry two, L2 prefetch of the row two, the row itself
 // one tile ahead (into registers, as soon as the tile before it is converted). The chain runs on across items.
-template <int kHB, int kTK, bool kPacked>
+template <int kHB, int kTK, bool kPacked, bool kWide>
 __device__ __forceinline__ void slice_role_producer(const SfaParams& p, SliceCtl<kHB, kTK>* ctl, uint32_t base, int n_items) {
   using Cfg = SliceCfg<kHB, kTK>;
   const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) - 12;
@@ -175,19 +177,27 @@ __device__ __forceinline__ void slice_role_producer(const SfaParams& p, SliceCtl
     ++cur_j;
     return true;
   };
-  uint4 d[2][2];  // [row pair][half]: this lane's 16 bytes of row 2 pair + rsel
+  uint4 d[2][2];  // [row pair][half]: this lane's 16 bytes of row 2 pair + rsel (kWide: [0, 1][half]: its 32 bytes of row r4)
+  const int part = lane & 1, r4 = (lane >> 1) & 3;  // kWide
   uint4 rope;     // unit lane % 8 of row lane / 8
   float4 sc;      // the four scales of row r
   int row_loaded = -1;
   // a padding or rejected row reads row 0; it is masked out of the softmax (`live`), its rope part is zeroed
   auto issue_loads = [&](int phys) {
     row_loaded = phys;
+    if constexpr (kWide) {
+      const int pm = max(__shfl_sync(0xffffffffu, phys, r4), 0);
+      const uint8_t* src = SLICE_KN + static_cast<int64_t>(pm) * stride_n + (2 * (lane >> 3) + part) * 32;
+      ldg_pinned_v8(src, d[0][0], d[1][0]);
+      ldg_pinned_v8(src + 256, d[0][1], d[1][1]);
+    } else {
 #pragma unroll
-    for (int pr = 0; pr < 2; ++pr) {
-      const int pm = max(__shfl_sync(0xffffffffu, phys, 2 * pr + rsel), 0);
-      const uint8_t* src = SLICE_KN + static_cast<int64_t>(pm) * stride_n + src_off;
-      d[pr][0] = ldg_pinned_v4(src);
-      d[pr][1] = ldg_pinned_v4(src + 256);
+      for (int pr = 0; pr < 2; ++pr) {
+        const int pm = max(__shfl_sync(0xffffffffu, phys, 2 * pr + rsel), 0);
+        const uint8_t* src = SLICE_KN + static_cast<int64_t>(pm) * stride_n + src_off;
+        d[pr][0] = ldg_pinned_v4(src);
+        d[pr][1] = ldg_pinned_v4(src + 256);
+      }
     }
     const int px = __shfl_sync(0xffffffffu, phys, lane >> 3);
     rope = make_uint4(0, 0, 0, 0);
@@ -239,9 +249,10 @@ __device__ __forceinline__ void slice_role_producer(const SfaParams& p, SliceCtl
       }
 #pragma unroll
       for (int pr = 0; pr < 2; ++pr) {
-        const int row = 4 * w + 2 * pr + rsel, x = row & 7;
+        const int row = 4 * w + (kWide ? r4 : 2 * pr + rsel), x = row & 7;
         const uint32_t dst = tile + (4 * hf + (lane >> 3)) * Cfg::kChunk + row * 128;
-        const uint32_t a = ((2 * (lane & 3)) ^ x) << 4, c = ((2 * (lane & 3) + 1) ^ x) << 4;
+        const int unit = kWide ? 4 * part + 2 * pr : 2 * (lane & 3);  // first of the two 16-byte units of the chunk's 128 bytes
+        const uint32_t a = (unit ^ x) << 4, c = ((unit + 1) ^ x) << 4;
         const uint4 v = d[pr][hf];
         const uint2 v0 = slice_cvt4(v.x), v1 = slice_cvt4(v.y), v2 = slice_cvt4(v.z), v3 = slice_cvt4(v.w);
         sts_v4u(dst + a, make_uint4(v0.x, v0.y, v1.x, v1.y));
@@ -700,8 +711,9 @@ sfa_slice_kernel(const __grid_constant__ SfaParams p, int n_items) {
     slice_role_softmax<kHB, kTK>(p, ctl, base, tmem, n_items);
   } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::kRegProd));
-    if (p.packed) slice_role_producer<kHB, kTK, true>(p, ctl, base, n_items);
-    else slice_role_producer<kHB, kTK, false>(p, ctl, base, n_items);
+    if (p.packed) slice_role_producer<kHB, kTK, true, false>(p, ctl, base, n_items);
+    else if (p.kn_aligned32) slice_role_producer<kHB, kTK, false, true>(p, ctl, base, n_items);
+    else slice_role_producer<kHB, kTK, false, false>(p, ctl, base, n_items);
   }
   tc_fence_before();
   __syncthreads();

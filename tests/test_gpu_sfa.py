@@ -207,19 +207,20 @@ def test_block_sizes_address_the_same_rows(block_size, nq):
     assert torch.equal(out.cpu(), _run(d, nq=nq))
 
 
-def test_latent_cache_on_a_16_byte_boundary():
+@pytest.mark.parametrize("nq", [128, 16, 32])
+def test_latent_cache_on_a_16_byte_boundary(nq):
     """32-byte loads take caches on a 32-byte boundary, 16-byte ones any other: the same values either way."""
-    d = gen.make_inputs([3000, 700], s1=1, seed=8, with_indexer=False, with_topk=True)
-    want = _run(d)
+    d = gen.make_inputs([3000, 700], s1=1, seed=8, with_indexer=False, with_topk=True, attn_heads=nq)
+    want = _run(d, nq=nq)
     g = d.to(DEV)
     raw = torch.zeros(g.key_nope_2d.numel() + 48, dtype=torch.int8, device=DEV)
     at = -raw.data_ptr() % 32 + 16
     kn = raw[at:at + g.key_nope_2d.numel()].view(-1, 512)
     kn.copy_(g.key_nope_2d)
     assert kn.data_ptr() % 32 == 16
-    out = torch.zeros((d.b, 1, 128, 512), dtype=torch.bfloat16, device=DEV)
+    out = torch.zeros((d.b, 1, nq, 512), dtype=torch.bfloat16, device=DEV)
     pto.sparse_flash_attention_quant_d(g.query_nope, g.query_rope, kn, g.key_rope_2d, g.k_nope_scales, g.topk_indices, g.block_table,
-                                       g.act_seq_key, out, 128, 1, SCALE, 2048, 128, d.max_blocks)
+                                       g.act_seq_key, out, nq, 1, SCALE, 2048, 128, d.max_blocks)
     torch.cuda.synchronize()
     assert pto.workspace_status()[0] == 0
     assert torch.equal(out.cpu(), want)
