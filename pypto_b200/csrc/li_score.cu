@@ -218,7 +218,7 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
   // this kernel is launched the ordinary way (everything before it has completed); the top-k kernel behind it
   // may be scheduled as soon as SMs drain and waits there for this grid to complete
   if (tid == 0) pdl_trigger();
-  const int s1 = p.s1;
+  const int s1 = kMode == kLiQuant ? 1 : p.s1;  // (that formulation is launched for one token)
   const int items_per_page = s1 > 2 ? 2 : 1;                     // an item: one or two query tokens of a page
   const uint32_t unit_cols = s1 > 1 ? 2 * kHeads : kHeads;       // columns of an accumulator
   const uint32_t n_accs = kTmemCols / unit_cols;                 // 8 or 4
@@ -595,38 +595,40 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
             }
           } else {
 #pragma unroll
-          for (int i = 0; i < 2; ++i) {
+          for (int i = 0; i < (kMode == kLiQuant ? 1 : 2); ++i) {
             if (i < cnt) {
-              uint32_t v0[32], v1[32];
-              tmem_ld_32x32b_x32(taddr + i * kHeads, v0);
-              tmem_ld_32x32b_x32(taddr + i * kHeads + 32, v1);
-              tc_wait_ld();
-              if (i == cnt - 1) {
-                // TMEM and the scale row are read: hand the accumulator back before the arithmetic
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&ctl->accempty[acc]));
+              // One half of the heads after the other: with both in registers, and the code of several tokens in the formulation that
+              // is launched for one, these modes spilled (64 sequences of up to 65536 keys 54.6 -> 53.4 us, 8 x 32768 10.9 -> 10.3,
+              // bf16 16 x 8192 11.0 -> 10.6).
+              float part[2];
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                uint32_t v[32];
+                tmem_ld_32x32b_x32(taddr + i * kHeads + 32 * h, v);
+                tc_wait_ld();
+                if (h == 1 && i == cnt - 1) {
+                  // TMEM and the scale row are read: hand the accumulator back before the arithmetic
+                  tc_fence_before();
+                  __syncwarp();
+                  if (lane == 0) mbar_arrive(smem_u32(&ctl->accempty[acc]));
+                }
+                const float* w = ws + i * kHeads + 32 * h;
+                part[h] = kBf16 ? weighted_relu_sum_32(v, w) : (kMode == kLiQuant ? weighted_sum_32(v, w) : chain_sum_32(v, w, ks2));
               }
-              if (kBf16) {
-                res[i] = weighted_relu_sum_32(v0, ws + i * kHeads) + weighted_relu_sum_32(v1, ws + i * kHeads + 32);
-              } else if (kMode == kLiQuant) {
-                res[i] = (weighted_sum_32(v0, ws + i * kHeads) + weighted_sum_32(v1, ws + i * kHeads + 32)) * ks;
-              } else {
-                res[i] = __fadd_rn(chain_sum_32(v0, ws + i * kHeads, ks2), chain_sum_32(v1, ws + i * kHeads + 32, ks2));
-              }
+              res[i] = kChain ? __fadd_rn(part[0], part[1]) : (part[0] + part[1]) * (kBf16 ? 1.f : ks);
             }
           }
           }
           if (pos < seq_len) {
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
+            for (int i = 0; i < (kMode == kLiQuant ? 1 : 2); ++i) {
               if (i < cnt) p.scores[(tok0 + 2 * half + i) * p.row_stride + pos] = res[i];
             }
           }
           if (with_hist) {
             // counts for the top-k kernel: positions below the token's causal end
 #pragma unroll
-            for (int i = 0; i < kLiHistMaxS1; ++i) {
+            for (int i = 0; i < (kMode == kLiQuant ? 1 : kLiHistMaxS1); ++i) {
               if (i < s1) {
                 const int eff = seq_len - (p.s1_total - 1 - (tok_first + i));
                 if (pos < eff) atomicAdd(&hist_sm[i * kLiHistBins + (li_float_order(res[i]) >> kLiHistShift)], 1u);
