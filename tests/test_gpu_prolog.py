@@ -189,6 +189,12 @@ def test_row_counts_at_tile_edges(t, odd):
     check_against(run_prolog(p, odd_outputs=odd), po.mla_indexer_prolog(p, eps_cq=1e-5, eps_ckv=1e-5), p["cache_index"])
 
 
+@pytest.mark.parametrize("t,odd", [(256, True), (520, False)])  # two whole tiles of rows with single-element accesses; four and 8 rows
+def test_row_counts_of_several_tiles(t, odd):
+    p = gen.make_prolog_inputs([130] * t, s1=1, seed=t)
+    check_against(run_prolog(p, odd_outputs=odd), po.mla_indexer_prolog(p, eps_cq=1e-5, eps_ckv=1e-5), p["cache_index"])
+
+
 def test_bad_cache_index_is_reported_not_written():
     p = gen.make_prolog_inputs([200, 300], s1=1, seed=4)
     p["cache_index"][1] = p["kv_cache"].shape[0] + 5
