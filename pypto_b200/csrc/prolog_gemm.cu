@@ -186,10 +186,9 @@ prolog_i8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_
       if (!ok || ctl->abort) break;
       tc_fence_after();
       const bool second = tile >= p.tiles[0];
-      const int which = second ? 1 : 0;
       const int n = (second ? tile - p.tiles[0] : tile) * kGTileN + q * 32 + lane;
-      int32_t* dst = p.out[which] + n;
-      const int64_t ld = p.ld[which];
+      int32_t* dst = (second ? p.out[1] : p.out[0]) + n;  // (indexed by a variable, the parameters are copied to local memory)
+      const int64_t ld = second ? p.ld[1] : p.ld[0];
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * 64u;
       for (int c0 = 0; c0 < p.t_pad; c0 += 16) {
         uint32_t v[16];
