@@ -186,10 +186,12 @@ int check_li_bf16(const void* q, const void* kc, const void* w, const void* act,
                          max_blocks);
 }
 
-// Score stage for tokens-per-sequence s1 (any s1 >= 1: groups of up to 4 tokens per launch).
+// Score stage for tokens-per-sequence s1 (any s1 >= 1: groups of up to 4 tokens per launch). `for_selection`: nobody but the
+// selection behind it reads the scores, so that those behind a token's causal end may be left out.
 int run_li_scores(const int8_t* q, const void* qs, const int8_t* kc, const void* ks, const void* w, int scale_dtype,
                   const int32_t* act, const int32_t* bt, float* scores, void* first_mm, int b, int s1, int block_num,
-                  int max_blocks, int flags, int32_t* status, cudaStream_t stream, unsigned int* hist = nullptr) {
+                  int max_blocks, int flags, int32_t* status, cudaStream_t stream, unsigned int* hist = nullptr,
+                  bool for_selection = false) {
   pto::LiParams p{};
   p.q = q;
   p.q_scale = qs;
@@ -206,6 +208,7 @@ int run_li_scores(const int8_t* q, const void* qs, const int8_t* kc, const void*
   p.block_num = block_num;
   p.max_blocks = max_blocks;
   p.status = status;
+  p.causal = for_selection ? 1 : 0;
   const bool simt = (flags & PTO_LI_SCORE_SIMT) != 0;
   PTO_REQUIRE(simt || first_mm == nullptr, "first_mm is only produced with PTO_LI_SCORE_SIMT");
   if (hist != nullptr) {  // li_hist_usable() said yes: every launch below takes all s1 tokens of a sequence
@@ -649,7 +652,7 @@ int pto_li_decode(const int8_t* idx_query, const void* idx_query_scale, const in
                                            li_scores_bytes(b * s1, max_blocks, block_size));
   }
   rc = run_li_scores(idx_query, idx_query_scale, idx_key_cache, idx_key_scale, idx_weight, scale_dtype, act_seq_key,
-                     block_table, scores, nullptr, b, s1, block_num, max_blocks, flags, status, stream, hist);
+                     block_table, scores, nullptr, b, s1, block_num, max_blocks, flags, status, stream, hist, /*for_selection=*/true);
   if (rc != PTO_OK) return rc;
   return run_li_topk(scores, static_cast<int64_t>(max_blocks) * block_size, act_seq_key, topk_res, b, s1,
                      selected_count, flags, status, stream, hist);
@@ -689,7 +692,7 @@ int pto_li_decode_bf16(const void* idx_query, const void* idx_key_cache, const v
   }
   rc = run_li_scores(reinterpret_cast<const int8_t*>(idx_query), nullptr, reinterpret_cast<const int8_t*>(idx_key_cache),
                      nullptr, idx_weight, PTO_DT_F16, act_seq_key, block_table, scores, nullptr, b, s1, block_num,
-                     max_blocks, kLiFlagBf16, status, stream, hist);
+                     max_blocks, kLiFlagBf16, status, stream, hist, /*for_selection=*/true);
   if (rc != PTO_OK) return rc;
   return run_li_topk(scores, static_cast<int64_t>(max_blocks) * block_size, act_seq_key, topk_res, b, s1,
                      selected_count, flags, status, stream, hist);
@@ -725,7 +728,7 @@ int pto_li_decode_static(const int8_t* idx_query, const void* idx_query_scale, c
   int32_t* status = reinterpret_cast<int32_t*>(scratch);
   float* scores = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(scratch) + kStatusBytes);
   rc = run_li_scores(idx_query, idx_query_scale, idx_key_cache, idx_key_scale, idx_weight, scale_dtype, act_seq_key,
-                     block_table, scores, nullptr, b, s1, block_num, max_blocks, flags, status, stream);
+                     block_table, scores, nullptr, b, s1, block_num, max_blocks, flags, status, stream, nullptr, /*for_selection=*/true);
   if (rc != PTO_OK) return rc;
   rc = run_li_topk(scores, static_cast<int64_t>(max_blocks) * block_size, act_seq_key, topk_res, b, s1,
                    selected_count, flags, status, stream);
@@ -1072,7 +1075,7 @@ int pto_decode_fused(const int8_t* idx_query, const void* idx_query_scale, const
   unsigned int* hist =  // behind the attention partials
       li_hist_usable(s1, flags) ? reinterpret_cast<unsigned int*>(part + sfa_part_bytes(b * s1, nq)) : nullptr;
   rc = run_li_scores(idx_query, idx_query_scale, idx_key_cache, idx_key_scale, idx_weight, scale_dtype, act_seq,
-                     block_table, scores, nullptr, b, s1, block_num, max_blocks, flags, status, stream, hist);
+                     block_table, scores, nullptr, b, s1, block_num, max_blocks, flags, status, stream, hist, /*for_selection=*/true);
   if (rc != PTO_OK) return rc;
   rc = run_li_topk(scores, static_cast<int64_t>(max_blocks) * 128, act_seq, topk_res, b, s1, selected_count, flags,
                    status, stream, hist);
@@ -1102,7 +1105,7 @@ int pto_decode_fused_bf16(const void* idx_query, const void* idx_key_cache, cons
       li_hist_usable(s1, flags) ? reinterpret_cast<unsigned int*>(part + sfa_part_bytes(b * s1, nq)) : nullptr;
   rc = run_li_scores(reinterpret_cast<const int8_t*>(idx_query), nullptr, reinterpret_cast<const int8_t*>(idx_key_cache),
                      nullptr, idx_weight, PTO_DT_F16, act_seq, block_table, scores, nullptr, b, s1, block_num, max_blocks,
-                     kLiFlagBf16, status, stream, hist);
+                     kLiFlagBf16, status, stream, hist, /*for_selection=*/true);
   if (rc != PTO_OK) return rc;
   rc = run_li_topk(scores, static_cast<int64_t>(max_blocks) * 128, act_seq, topk_res, b, s1, selected_count, flags,
                    status, stream, hist);

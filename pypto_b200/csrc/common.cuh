@@ -300,6 +300,7 @@ struct LiParams {
   int bf16;        // non-quantised formulation: q, k_cache and weight are bf16, the scales are not read
   int s1_total;    // query tokens per sequence in memory (>= s1)
   int tok_offset;  // first token of each sequence handled by this launch
+  int causal;      // only scores below each token's causal end are wanted (tensor-core kernel, one sequence: pages behind it are left out)
   int groups;      // token groups of s1 tokens taken by one launch (tensor-core kernel), >= 1
   // optional, tensor-core kernel with s1 <= 2 per launch: per query token a histogram [t, kLiHistBins] (zeroed by the
   // caller) of the scores at positions below the token's causal end, binned by the top 12 bits of the

@@ -252,15 +252,26 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
     tmem_alloc(smem_u32(&ctl->tmem_base), kTmemCols);
     tmem_relinquish();
   }
+  // A chunk of one prompt whose scores only the selection reads: a token group needs the pages up to its last token's causal end, and
+  // the list below is one of groups instead of sequences. (All pages for every group: twice the work where the chunk is the prompt.)
+  // The CTAs share it by cost: a group's queries and weights take as long as `kGroupCost` of its pages, and the first groups have
+  // few of these (by pages alone the first CTA got seventy groups of a chunk of 4096). 4096 tokens that are the prompt 208 -> 137 us,
+  // behind 12288 keys 756 -> 642, 512 tokens 12.4 -> 11.0; with few tokens behind many keys there is nothing to leave out.
+  const bool by_group = p.causal != 0 && p.b == 1 && p.groups > 1 && p.groups <= kMaxSeqPerLaunch;
+  const int n_lists = by_group ? p.groups : p.b;
+  constexpr int kGroupCost = 2;
+  const int head = by_group ? kGroupCost : 0;  // units of cost before a list's first page
   if (warp == kLiEpilogueWarp0) {
-    // exclusive prefix of pages per sequence
+    // exclusive prefix of pages per sequence (or token group)
     int carry = 0;
-    for (int b0 = 0; b0 < p.b; b0 += 32) {
+    const int first_end = by_group ? p.act_seq[0] - p.s1_total + p.tok_offset + s1 : 0;  // causal end of the first group
+    for (int b0 = 0; b0 < n_lists; b0 += 32) {
       int v = 0;
-      if (b0 + lane < p.b) {
-        int s = p.act_seq[b0 + lane];
+      if (b0 + lane < n_lists) {
+        int s = by_group ? first_end + (b0 + lane) * s1 : p.act_seq[b0 + lane];
         s = max(s, 0);
         v = min((s + kPageKeys - 1) / kPageKeys, p.max_blocks);
+        if (v > 0) v += head;
       }
       int incl = v;
 #pragma unroll
@@ -268,10 +279,10 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
         int n = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += n;
       }
-      if (b0 + lane < p.b) ctl->prefix[b0 + lane] = carry + incl - v;
+      if (b0 + lane < n_lists) ctl->prefix[b0 + lane] = carry + incl - v;
       carry += __shfl_sync(0xffffffffu, incl, 31);
     }
-    if (lane == 0) ctl->prefix[p.b] = carry;
+    if (lane == 0) ctl->prefix[n_lists] = carry;
   }
   tc_fence_before();
   __syncthreads();
@@ -279,8 +290,8 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
   const uint32_t tmem_base = ctl->tmem_base;
 
   // pages of all sequences, once per token group
-  const int total = ctl->prefix[p.b];
-  const long long all = static_cast<long long>(total) * p.groups;
+  const int total = ctl->prefix[n_lists];
+  const long long all = static_cast<long long>(total) * (by_group ? 1 : p.groups);
   const long long it0 = all * blockIdx.x / gridDim.x, it1 = all * (blockIdx.x + 1) / gridDim.x;
 
   const uint32_t idesc1 = kBf16 ? umma_idesc(kCFmtF32, kABFmtBF16, kABFmtBF16, 0, 0, 128, kHeads)
@@ -291,16 +302,16 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
   const uint32_t q_half_bytes = static_cast<uint32_t>(s1 * kHeads) * 128u;  // bf16: one 64-dim half of the query tile
 
   long long cur = it0;
-  int bi = 0, group = 0;
+  int li = 0, group = 0;  // list (sequence or token group)
   if (cur < it1) {
     group = static_cast<int>(cur / total);
     const int lc = static_cast<int>(cur - static_cast<long long>(group) * total);
-    int lo = 0, hi = p.b;  // largest bi with prefix[bi] <= lc
+    int lo = 0, hi = n_lists;  // largest list with prefix[lo] <= lc
     while (hi - lo > 1) {
       int mid = (lo + hi) >> 1;
       if (ctl->prefix[mid] <= lc) lo = mid; else hi = mid;
     }
-    bi = lo;
+    li = lo;
   }
   uint32_t n_page = 0;  // pages and items of the segments before
   uint32_t n_item = 0;
@@ -322,14 +333,20 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
     int lc = static_cast<int>(cur - static_cast<long long>(group) * total);
     if (lc >= total) {  // next token group, from the first sequence
       ++group;
-      bi = 0;
+      li = 0;
       lc = 0;
     }
-    while (ctl->prefix[bi + 1] <= lc) ++bi;
-    const int page0 = lc - ctl->prefix[bi];
-    const int npages = static_cast<int>(min(it1 - cur, static_cast<long long>(ctl->prefix[bi + 1] - lc)));
+    while (ctl->prefix[li + 1] <= lc) ++li;
+    const int cost = static_cast<int>(min(it1 - cur, static_cast<long long>(ctl->prefix[li + 1] - lc)));
+    const int page0 = max(0, lc - ctl->prefix[li] - head);
+    const int npages = max(0, lc - ctl->prefix[li] - head + cost) - page0;
+    if (npages == 0) {  // (the same in every thread)
+      cur += cost;
+      continue;
+    }
+    const int bi = by_group ? 0 : li;
     const int seq_len = p.act_seq[bi];
-    const int tok_first = p.tok_offset + group * s1;  // first query token of the segment within its sequence
+    const int tok_first = p.tok_offset + (by_group ? li : group) * s1;  // first query token of the segment within its sequence
     const int64_t tok0 = static_cast<int64_t>(bi) * p.s1_total + tok_first;
 
     // The producer warp takes no part in the two barriers of a segment: the ring's own barriers order its loads, so
@@ -640,7 +657,7 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
     }
     n_page += npages;
     n_item += npages * items_per_page;
-    cur += npages;
+    cur += cost;
     ++seg;
   }
 

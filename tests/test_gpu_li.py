@@ -301,6 +301,23 @@ def test_prefill_chunk_groups_share_a_launch():
             torch.testing.assert_close(b[bi * 22 + i, :s], a[bi * 22 + i, :s], rtol=3e-6, atol=1e-9)
 
 
+@pytest.mark.parametrize("kind", ["float32", "float16", "fp16_chain"])
+@pytest.mark.parametrize("n,s1", [(40, 40), (1030, 1030), (2300, 131), (5000, 9), (20, 50), (1200, 1024)])
+def test_pages_behind_the_causal_end_are_left_out(n, s1, kind):
+    """A chunk of one prompt: the selection of the chained call equals the selection alone over whole score rows. Groups of four
+    tokens that begin before, at and behind the ends of pages, tokens that see no key, a last group of its own."""
+    d = gen.make_inputs([n], s1=s1, seed=n + s1, with_attention=False,
+                        scale_dtype=torch.float32 if kind == "float32" else torch.float16)
+    g = d.to(DEV)
+    sc = torch.full((d.t, d.max_blocks * 128), float("nan"), dtype=torch.float32, device=DEV)
+    pto.lightning_indexer_scores(g.idx_query, g.idx_query_scale, g.idx_key_cache, g.idx_key_scale, g.idx_weight, g.act_seq_key,
+                                 g.block_table, sc, fp16_chain=kind == "fp16_chain")
+    assert torch.isfinite(sc[:, :n]).all()
+    want = torch.zeros((d.t, 1, 2048), dtype=torch.int32, device=DEV)
+    pto.lightning_indexer_topk(sc, g.act_seq_key, want, s1, 2048)
+    assert torch.equal(_decode(d, fp16_chain=kind == "fp16_chain").cpu(), want.cpu())
+
+
 @pytest.mark.parametrize("s1", [1, 2, 3])
 def test_chained_selection_from_the_score_kernels_histogram_equals_the_two_stages(s1):
     """Asked to (`histogram=True`), with at most two query tokens per sequence, the score kernel leaves a 4096-bin
@@ -394,7 +411,7 @@ def test_topk_stage_over_row_lengths_and_distributions(rows, n, k, kind, sort):
 
 
 @pytest.mark.parametrize("sort", [True, False], ids=["ordered", "unordered"])
-@pytest.mark.parametrize("n", [6148, 8193, 30001, 100003])  # chunks of a row: fewer than, as many as and more than are in flight
+@pytest.mark.parametrize("n", [3001, 5120, 5121, 6148, 8193, 30001, 100003])  # rows that are lists, that are in one form only, longer ones
 @pytest.mark.parametrize("kind", ["normal", "ties", "last"])
 def test_many_rows_two_to_an_sm(kind, n, sort):
     """More rows than two per SM, in several rounds; every third row is short."""

@@ -47,6 +47,16 @@ def _check_sets(idx, want_idx, rows, d):
         assert torch.all(idx[ti, 0, nvalid:] == -1)
 
 
+@pytest.mark.parametrize("n,s1", [(40, 40), (1030, 515)])
+def test_pages_behind_the_causal_end_are_left_out(n, s1):
+    d = gen.make_nonquant_inputs([n], s1=s1, seed=n)
+    g = d.to(DEV)
+    sc = _scores(g, d).to(DEV)
+    want = torch.zeros((d.t, 1, 2048), dtype=torch.int32, device=DEV)
+    pto.lightning_indexer_topk(sc, g.act_seq_key, want, s1, 2048)
+    assert torch.equal(_topk(g, d), want.cpu())
+
+
 @pytest.mark.parametrize("name", NONQUANT_CASES)
 def test_scores_and_sets_match_reference_fixture(name):
     d, z = load_case(name)
