@@ -460,13 +460,14 @@ li_topk_kernel(TopkParams p) {
   int eff = p.act_seq[bi] - (p.s1 - 1 - i);
   if (eff > p.row_stride) eff = static_cast<int>(p.row_stride);
   const int k = min(p.k, eff);  // entries of the result
-  if (tid == 0) {
-    for (int c = 0; c < kRing; ++c) {
-      mbar_init(smem_u32(&sm->full[c]), 1);
-      mbar_init(smem_u32(&sm->empty[c]), kGroupWarps);
-    }
+  if (tid < kRing) {  // (a thread each: one that set them all took a thousand cycles)
+    mbar_init(smem_u32(&sm->full[tid]), 1);
+    mbar_init(smem_u32(&sm->empty[tid]), kGroupWarps);
     fence_mbar_init();
     fence_proxy_async();
+  }
+  __syncwarp();
+  if (tid == 0) {
     sm->n_mine = 0;
     sm->n_list = 0;
     sm->n_sel = 0;
@@ -789,9 +790,11 @@ cudaError_t launch_li_topk(const TopkParams& p, int num_sms, cudaStream_t stream
   const int rows = p.b * p.s1;
   int csize = 1;
   while (csize < 8 && rows * csize * 2 <= num_sms && p.row_stride > static_cast<int64_t>(csize) * 8192) csize *= 2;
-  // More rows than SMs, too long to be lists: two to an SM, so that one streams while the other finds its bound or orders its list
-  // (behind their score kernel, with the scan by groups of warps: 4096 rows of 131072 990 -> 780 us, 256 rows 88 -> 78)
-  const bool many = rows > num_sms && p.hist == nullptr && p.row_stride > TopkSmem<false>::kListCap;
+  // More rows than SMs: two to an SM, so that one streams while the other finds its bound or orders its list (behind their score
+  // kernel, with the scan by groups of warps: 4096 rows of 131072 990 -> 780 us, 256 rows 88 -> 78; 4096 rows of 4096, which are lists,
+  // 106 -> 79, 1000 rows of 3000 42 -> 27). Not where only the longer list of a CTA alone takes whole rows.
+  const bool many = rows > num_sms && p.hist == nullptr &&
+                    (p.row_stride <= TopkSmem<true>::kListCap || p.row_stride > TopkSmem<false>::kListCap);
   auto kernel = many ? li_topk_kernel<true> : li_topk_kernel<false>;
   static_assert(sizeof(TopkSmem<true>) <= 113 * 1024, "two CTAs to an SM");
   const size_t smem = many ? sizeof(TopkSmem<true>) : sizeof(TopkSmem<false>);
