@@ -36,6 +36,7 @@ SIGNATURES = {
     "pto_li_scores_bf16": (_i, [_vp] * 6 + [_i] * 8 + [_vp, _sz, _vp]),
     "pto_li_topk": (_i, [_vp, _i64, _vp, _vp, _i, _i, _i, _i, _vp, _sz, _vp]),
     "pto_sfa_workspace_bytes": (_sz, [_i, _i]),
+    "pto_sfa_extra_bytes": (_sz, [_i, _i]),
     "pto_sfa_quant": (_i, [_vp] * 9 + [_i, _i, _i, _i, _f, _i, _i, _i64, _i, _i, _i, _vp, _sz, _vp]),
     "pto_sfa_bf16": (_i, [_vp] * 8 + [_i, _i, _i, _i, _f, _i, _i, _i64, _i, _i, _i, _vp, _sz, _vp]),
     "pto_sfa_packed": (_i, [_vp] * 7 + [_i, _i, _i, _i, _f, _i, _i, _i64, _i, _i, _i, _vp, _sz, _vp]),

@@ -151,11 +151,19 @@ pto::SfaSplit sfa_split(int t, int nq) {
   return {0, static_cast<int>(s)};
 }
 
-size_t sfa_part_bytes(int t, int nq) {
-  const pto::SfaSplit sp = sfa_split(t, nq);
+size_t sfa_split_bytes(int t, int nq, const pto::SfaSplit& sp) {
   if (sp.n == 1) return 0;
   const size_t rows = static_cast<size_t>(t - sp.begin) * sp.n * nq;
   return align_up(rows * 2 * sizeof(float), 256) + align_up(rows * 512 * sizeof(float), 256);
+}
+// partials that a call needs room for; those of the last round, without which it runs unsplit
+size_t sfa_part_bytes(int t, int nq) {
+  const pto::SfaSplit sp = sfa_split(t, nq);
+  return sp.begin == 0 ? sfa_split_bytes(t, nq, sp) : 0;
+}
+size_t sfa_extra_bytes(int t, int nq) {
+  const pto::SfaSplit sp = sfa_split(t, nq);
+  return sp.begin > 0 ? sfa_split_bytes(t, nq, sp) : 0;
 }
 
 int check_li_common(const void* q, const void* qs, const void* kc, const void* ks, const void* w, int scale_dtype,
@@ -313,7 +321,8 @@ int run_sfa(const void* qn, const void* qr, const void* kn, const void* kr, cons
   pto::SfaSplit sp = sfa_split(t, nq);
   // a split costs the merge's launch, 2.5 us: where a round of pairs has gone before and a token's rows are few tiles, more than it gains
   if (sp.begin > 0 && std::min<long long>(topk, static_cast<long long>(max_blocks) * block_size) < kSfaSplitLastRoundRows) sp = {0, 1};
-  if (sp.n > 1 && part_bytes < sfa_part_bytes(t, nq)) return fail(PTO_ERR_WORKSPACE, "attention workspace too small");
+  if (sp.begin > 0 && part_bytes < sfa_extra_bytes(t, nq)) sp = {0, 1};  // (a workspace of the size the call needs, no more)
+  if (sp.n > 1 && sp.begin == 0 && part_bytes < sfa_part_bytes(t, nq)) return fail(PTO_ERR_WORKSPACE, "attention workspace too small");
   pto::SfaParams p{};
   p.q_nope = reinterpret_cast<const __nv_bfloat16*>(qn);
   p.q_rope = reinterpret_cast<const __nv_bfloat16*>(qr);
@@ -754,6 +763,7 @@ size_t pto_sfa_workspace_bytes(int t, int nq) {
   if (t < 1 || nq < 1) return 0;
   return kStatusBytes + sfa_part_bytes(t, nq);
 }
+size_t pto_sfa_extra_bytes(int t, int nq) { return t < 1 || nq < 1 ? 0 : sfa_extra_bytes(t, nq); }
 
 int pto_sfa_quant(const void* query_nope, const void* query_rope, const int8_t* key_nope_2d, const void* key_rope_2d,
                   const float* k_nope_scales, const int32_t* topk_indices, const int32_t* block_table,
@@ -1055,6 +1065,24 @@ size_t pto_decode_workspace_bytes(int t, int max_blocks, int block_size, int nq)
   return kStatusBytes + li_scores_bytes(t, max_blocks, block_size) + sfa_part_bytes(t, nq) + li_hist_bytes(t);
 }
 
+}  // extern "C"
+
+namespace {
+// Where a chained call's partials lie: in front of the histogram rows, or, if they are those of the last round only, in what the
+// caller gave beyond the size the call needs.
+struct FusedParts {
+  uint8_t* base;
+  size_t bytes;
+};
+FusedParts fused_parts(uint8_t* workspace, size_t workspace_bytes, uint8_t* part, int t, int nq, int max_blocks) {
+  const size_t need = pto_decode_workspace_bytes(t, max_blocks, 128, nq);
+  if (sfa_extra_bytes(t, nq) > 0) return {workspace + need, workspace_bytes - need};
+  return {part, sfa_part_bytes(t, nq)};
+}
+}  // namespace
+
+extern "C" {
+
 int pto_decode_fused(const int8_t* idx_query, const void* idx_query_scale, const int8_t* idx_key_cache,
                      const void* idx_key_scale, const void* idx_weight, int scale_dtype, const void* query_nope,
                      const void* query_rope, const int8_t* key_nope_2d, const void* key_rope_2d,
@@ -1072,6 +1100,7 @@ int pto_decode_fused(const int8_t* idx_query, const void* idx_query_scale, const
   int32_t* status = reinterpret_cast<int32_t*>(base);
   float* scores = reinterpret_cast<float*>(base + kStatusBytes);
   uint8_t* part = base + kStatusBytes + li_scores_bytes(b * s1, max_blocks, 128);
+  const FusedParts parts = fused_parts(base, workspace_bytes, part, b * s1, nq, max_blocks);
   unsigned int* hist =  // behind the attention partials
       li_hist_usable(s1, flags) ? reinterpret_cast<unsigned int*>(part + sfa_part_bytes(b * s1, nq)) : nullptr;
   rc = run_li_scores(idx_query, idx_query_scale, idx_key_cache, idx_key_scale, idx_weight, scale_dtype, act_seq,
@@ -1082,7 +1111,7 @@ int pto_decode_fused(const int8_t* idx_query, const void* idx_query_scale, const
   if (rc != PTO_OK) return rc;
   return run_sfa(query_nope, query_rope, key_nope_2d, key_rope_2d, k_nope_scales, 0, topk_res, block_table, act_seq,
                  attention_out, b, s1, nq, 1, softmax_scale, selected_count, 128, static_cast<int64_t>(block_num) * 128,
-                 max_blocks, nq, 0, part, sfa_part_bytes(b * s1, nq), status, stream, /*behind_topk=*/1);
+                 max_blocks, nq, 0, parts.base, parts.bytes, status, stream, /*behind_topk=*/1);
 }
 
 int pto_decode_fused_bf16(const void* idx_query, const void* idx_key_cache, const void* idx_weight,
@@ -1101,6 +1130,7 @@ int pto_decode_fused_bf16(const void* idx_query, const void* idx_key_cache, cons
   int32_t* status = reinterpret_cast<int32_t*>(base);
   float* scores = reinterpret_cast<float*>(base + kStatusBytes);
   uint8_t* part = base + kStatusBytes + li_scores_bytes(b * s1, max_blocks, 128);
+  const FusedParts parts = fused_parts(base, workspace_bytes, part, b * s1, nq, max_blocks);
   unsigned int* hist =  // behind the attention partials
       li_hist_usable(s1, flags) ? reinterpret_cast<unsigned int*>(part + sfa_part_bytes(b * s1, nq)) : nullptr;
   rc = run_li_scores(reinterpret_cast<const int8_t*>(idx_query), nullptr, reinterpret_cast<const int8_t*>(idx_key_cache),
@@ -1112,7 +1142,7 @@ int pto_decode_fused_bf16(const void* idx_query, const void* idx_key_cache, cons
   if (rc != PTO_OK) return rc;
   return run_sfa(query_nope, query_rope, key_nope_2d, key_rope_2d, nullptr, kSfaSplitBf16, topk_res, block_table,
                  act_seq, attention_out, b, s1, nq, 1, softmax_scale, selected_count, 128,
-                 static_cast<int64_t>(block_num) * 128, max_blocks, nq, 0, part, sfa_part_bytes(b * s1, nq), status, stream,
+                 static_cast<int64_t>(block_num) * 128, max_blocks, nq, 0, parts.base, parts.bytes, status, stream,
                  /*behind_topk=*/1);
 }
 

@@ -302,7 +302,7 @@ PyObject* sfa(PyObject*, PyObject* const* a, Py_ssize_t n) {
   }
   if (!c.ok()) Py_RETURN_FALSE;
   const void *knp = kn->data_ptr(), *krp = kr->data_ptr();
-  return launch(c, pto_sfa_workspace_bytes(x.t, static_cast<int>(nq)), [&](void* ws, size_t have, pto_stream_t s) {
+  return launch(c, pto_sfa_workspace_bytes(x.t, static_cast<int>(nq)) + pto_sfa_extra_bytes(x.t, static_cast<int>(nq)), [&](void* ws, size_t have, pto_stream_t s) {
     const auto *ti = static_cast<const int32_t*>(x.ti), *bt = static_cast<const int32_t*>(x.bt), *act = static_cast<const int32_t*>(x.act);
     const int s1 = x.t / x.b, inq = static_cast<int>(nq), ik = static_cast<int>(topk), ibs = static_cast<int>(bs),
               int_ = static_cast<int>(nt), ih = static_cast<int>(h0);
@@ -335,7 +335,7 @@ PyObject* sfa_packed(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (!c.ok()) Py_RETURN_FALSE;
   const int64_t rows = cache->size(0);
   const auto* p = static_cast<const int8_t*>(cache->data_ptr());
-  return launch(c, pto_sfa_workspace_bytes(x.t, static_cast<int>(nq)), [&](void* ws, size_t have, pto_stream_t s) {
+  return launch(c, pto_sfa_workspace_bytes(x.t, static_cast<int>(nq)) + pto_sfa_extra_bytes(x.t, static_cast<int>(nq)), [&](void* ws, size_t have, pto_stream_t s) {
     return pto_sfa_packed(x.qn, x.qr, p, static_cast<const int32_t*>(x.ti), static_cast<const int32_t*>(x.bt),
                           static_cast<const int32_t*>(x.act), x.out, x.b, x.t / x.b, static_cast<int>(nq), 1,
                           static_cast<float>(scale), static_cast<int>(topk), static_cast<int>(bs), rows, x.max_blocks,
@@ -367,7 +367,7 @@ PyObject* fused(PyObject*, PyObject* const* a, Py_ssize_t n) {
   c.need(sc->scalar_type() == kF32 && sc->dim() == 2 && sc->size(0) == rows && sc->size(1) == 4);
   if (!c.ok()) Py_RETURN_FALSE;
   const void *knp = kn->data_ptr(), *krp = kr->data_ptr(), *scp = sc->data_ptr();
-  return launch(c, pto_decode_workspace_bytes(x.t, x.max_blocks, 128, static_cast<int>(nq)), [&](void* ws, size_t have, pto_stream_t s) {
+  return launch(c, pto_decode_workspace_bytes(x.t, x.max_blocks, 128, static_cast<int>(nq)) + pto_sfa_extra_bytes(x.t, static_cast<int>(nq)), [&](void* ws, size_t have, pto_stream_t s) {
     return pto_decode_fused(static_cast<const int8_t*>(x.q), x.qs, static_cast<const int8_t*>(x.kc), x.ks, x.w, x.scale_dtype,
                             y.qn, y.qr, static_cast<const int8_t*>(knp), krp, static_cast<const float*>(scp),
                             static_cast<const int32_t*>(x.act), static_cast<const int32_t*>(x.bt), static_cast<int32_t*>(y.ti),
@@ -399,7 +399,7 @@ PyObject* fused_bf16(PyObject*, PyObject* const* a, Py_ssize_t n) {
   c.need(kr->scalar_type() == kBf16 && kr->dim() == 2 && kr->size(0) == rows && kr->size(1) == 64);
   if (!c.ok()) Py_RETURN_FALSE;
   const void *knp = kn->data_ptr(), *krp = kr->data_ptr();
-  return launch(c, pto_decode_workspace_bytes(x.t, x.max_blocks, 128, static_cast<int>(nq)), [&](void* ws, size_t have, pto_stream_t s) {
+  return launch(c, pto_decode_workspace_bytes(x.t, x.max_blocks, 128, static_cast<int>(nq)) + pto_sfa_extra_bytes(x.t, static_cast<int>(nq)), [&](void* ws, size_t have, pto_stream_t s) {
     return pto_decode_fused_bf16(x.q, x.kc, x.w, y.qn, y.qr, knp, krp, static_cast<const int32_t*>(x.act),
                                  static_cast<const int32_t*>(x.bt), static_cast<int32_t*>(y.ti), y.out, x.b, x.t / x.b, x.block_num,
                                  x.max_blocks, static_cast<int>(k), static_cast<int>(nq), static_cast<float>(scale),

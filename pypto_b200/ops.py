@@ -321,7 +321,7 @@ def _sparse_flash_attention_quant(query_nope, query_rope, key_nope_2d, key_rope_
     _need(bt.shape[1] >= int(max_blocknum_perbatch), "block_table narrower than max_blocknum_perbatch")
     _need(int(nq) % 16 == 0, "nq must be a multiple of 16")
     lib = _lib.load()
-    nbytes = lib.pto_sfa_workspace_bytes(t, int(nq))
+    nbytes = lib.pto_sfa_workspace_bytes(t, int(nq)) + lib.pto_sfa_extra_bytes(t, int(nq))
     tail = (b, t // b, int(nq), int(n_kv), float(softmax_scale), int(topk), int(block_size), n_rows, bt.shape[1],
             int(nq if nq_total is None else nq_total), int(head_begin))
     if kn.dtype == torch.bfloat16:
@@ -383,7 +383,7 @@ def _sparse_attention_antiquant(query_nope, query_rope, nope_cache, topk_indices
           "nope_cache: int8 [rows, 656] = 512 int8 | 64 bf16 | 4 fp32")
     dev = _same_device([qn, qr, cache, ti, bt, act, out])
     lib = _lib.load()
-    nbytes = lib.pto_sfa_workspace_bytes(t, int(nq))
+    nbytes = lib.pto_sfa_workspace_bytes(t, int(nq)) + lib.pto_sfa_extra_bytes(t, int(nq))
     with torch.cuda.device(dev):
         ws = _workspace(dev, nbytes)
         _lib.check(lib.pto_sfa_packed(qn.data_ptr(), qr.data_ptr(), cache.data_ptr(), ti.data_ptr(), bt.data_ptr(),
@@ -567,7 +567,7 @@ def decode_indexer_attention_quant(idx_query, idx_query_scale, idx_key_cache, id
     _need(sc.dtype == torch.float32 and tuple(sc.shape) == (n_rows, 4), "k_nope_scales: float32 [block_num*128, 4]")
     dev = _same_device([q, qs, kc, ks, w, act, bt, qn, qr, kn, kr, sc, out_idx, out])
     lib = _lib.load()
-    nbytes = lib.pto_decode_workspace_bytes(t, m["max_blocks"], 128, int(nq))
+    nbytes = lib.pto_decode_workspace_bytes(t, m["max_blocks"], 128, int(nq)) + lib.pto_sfa_extra_bytes(t, int(nq))
     with torch.cuda.device(dev):
         ws = _workspace(dev, nbytes)
         _lib.check(lib.pto_decode_fused(q.data_ptr(), qs.data_ptr(), kc.data_ptr(), ks.data_ptr(), w.data_ptr(),
@@ -604,7 +604,7 @@ def decode_indexer_attention(idx_query, idx_key_cache, idx_weight, query_nope, q
     _need(kr.dtype == torch.bfloat16 and tuple(kr.shape) == (n_rows, 64), "key_rope_2d: bfloat16 [block_num*128, 64]")
     dev = _same_device([q, kc, w, act, bt, qn, qr, kn, kr, out_idx, out])
     lib = _lib.load()
-    nbytes = lib.pto_decode_workspace_bytes(t, m["max_blocks"], 128, int(nq))
+    nbytes = lib.pto_decode_workspace_bytes(t, m["max_blocks"], 128, int(nq)) + lib.pto_sfa_extra_bytes(t, int(nq))
     with torch.cuda.device(dev):
         ws = _workspace(dev, nbytes)
         _lib.check(lib.pto_decode_fused_bf16(q.data_ptr(), kc.data_ptr(), w.data_ptr(), qn.data_ptr(), qr.data_ptr(),

@@ -54,6 +54,13 @@ def test_host_only_calls(lib):
                                                                  - 256 + 64 * 4096 * 4)
 
 
+def test_extra_bytes_of_the_last_round(lib):
+    """Tokens left over by whole rounds of 74 SM pairs, at least half of which they would leave idle, up to eight rounds."""
+    for t, rest, n in ((1, 0, 0), (74, 0, 0), (75, 1, 16), (80, 6, 12), (111, 37, 2), (112, 38, 0), (256, 34, 2), (593, 1, 16), (667, 1, 0)):
+        assert lib.pto_sfa_extra_bytes(t, 128) == rest * n * 128 * (512 + 2) * 4 if n else lib.pto_sfa_extra_bytes(t, 128) == 0, t
+    assert lib.pto_sfa_extra_bytes(80, 16) == 0
+
+
 def test_argument_errors_are_reported_before_any_cuda_call(lib):
     # null pointers: rejected on the host, no launch, no GPU needed
     rc = lib.pto_li_decode(None, None, None, None, None, 1, None, None, None, 1, 1, 64, 128, 128, 1, 1, 2048, 0,

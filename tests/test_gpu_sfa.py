@@ -5,6 +5,7 @@ import torch
 
 import oracle
 import pypto_b200 as pto
+from pypto_b200 import _lib
 from pypto_b200 import inputs as gen
 from golden_util import SFA_CASES, from_np_bf16, load_case, mask_empty_rows
 
@@ -183,6 +184,24 @@ def test_split_of_the_last_round(tokens, longest):
                                    d.topk_indices, d.block_table, d.act_seq, d.s1)
     _check(_run(d), want)
     assert torch.equal(_run(d, bf16_cache=True), _run(d))
+
+
+def test_a_workspace_without_room_for_the_last_round():
+    """A C caller's workspace of the size that the call needs and no more: the same call, unsplit."""
+    d = gen.make_inputs([1500] + [130] * 73 + [1500], s1=1, seed=6, with_indexer=False, with_topk=True)
+    want = _run(d)
+    g, lib = d.to(DEV), _lib.load()
+    assert lib.pto_sfa_extra_bytes(75, 128) > 0
+    ws = torch.zeros(lib.pto_sfa_workspace_bytes(75, 128), dtype=torch.uint8, device=DEV)
+    out = torch.zeros((75, 1, 128, 512), dtype=torch.bfloat16, device=DEV)
+    rc = lib.pto_sfa_quant(*(x.data_ptr() for x in (g.query_nope, g.query_rope, g.key_nope_2d, g.key_rope_2d, g.k_nope_scales,
+                                                    g.topk_indices, g.block_table, g.act_seq_key, out)),
+                           75, 1, 128, 1, SCALE, 2048, 128, g.key_nope_2d.shape[0], d.max_blocks, 128, 0, ws.data_ptr(), ws.numel(),
+                           torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert rc == 0 and int(ws[:4].view(torch.int32)) == 0
+    _check(out.cpu(), want)
+    assert torch.equal(out.cpu()[1:74], want[1:74])
 
 
 @pytest.mark.parametrize("nq", [128, 16])
