@@ -106,49 +106,98 @@ __device__ __forceinline__ WideItem wide_item(const WideParams& p, int item) {
 
 __device__ __forceinline__ float wide_bf16_round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 
-// This warp's rows: lane l holds 128 bytes of row l. They go to `dst` + l * `pitch` through the warp's staging area, four
-// whole lines per store instruction. `n_rows`: rows that exist; `n_bytes`: bytes that exist of each (a multiple of 16).
-template <bool kAligned>
-__device__ __forceinline__ void store_rows(uint32_t stage, const uint32_t (&w)[32], uint8_t* dst, int64_t pitch, int n_rows,
-                                           int n_bytes) {
+__device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
+__device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
+
+// This warp's rows: lane l holds 128 bytes of row l, which go to its staging area. 16-byte unit u of row r comes back from there.
+__device__ __forceinline__ void stage_rows(uint32_t stage, const uint32_t (&w)[32]) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     sts_v4u(stage + lane * 128 + ((i ^ (lane & 7)) << 4), make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]));
   }
   __syncwarp();
+}
+__device__ __forceinline__ uint4 staged_unit(uint32_t stage, int r, int u) { return lds_v4u(stage + r * 128 + ((u ^ (r & 7)) << 4)); }
+template <bool kAligned>
+__device__ __forceinline__ void store_unit(uint8_t* at, const uint4& v) {
+  if constexpr (kAligned) {
+    *reinterpret_cast<uint4*>(at) = v;
+  } else {
+    const uint32_t x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int e = 0; e < 16; ++e) at[e] = static_cast<uint8_t>(x[e >> 2] >> (8 * (e & 3)));
+  }
+}
+// The rows go to `dst` + l * `pitch` through the staging area, four whole lines per store instruction. `n_rows`: rows that
+// exist; `n_bytes`: bytes that exist of each (a multiple of 16).
+template <bool kAligned>
+__device__ __forceinline__ void store_rows(uint32_t stage, const uint32_t (&w)[32], uint8_t* dst, int64_t pitch, int n_rows,
+                                           int n_bytes) {
+  const int lane = threadIdx.x & 31;
+  stage_rows(stage, w);
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int r = 4 * i + (lane >> 3), u = lane & 7;
-    const uint4 v = lds_v4u(stage + r * 128 + ((u ^ (r & 7)) << 4));
-    if (r < n_rows && u * 16 < n_bytes) {
-      uint8_t* at = dst + r * pitch + u * 16;
-      if constexpr (kAligned) {
-        *reinterpret_cast<uint4*>(at) = v;
-      } else {
-        const uint32_t x[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int e = 0; e < 16; ++e) at[e] = static_cast<uint8_t>(x[e >> 2] >> (8 * (e & 3)));
-      }
-    }
+    const uint4 v = staged_unit(stage, r, u);
+    if (r < n_rows && u * 16 < n_bytes) store_unit<kAligned>(dst + r * pitch + u * 16, v);
   }
   __syncwarp();
 }
-// a token's 64 cosines or sines, eight at a time
+// eight of a token's 64 cosines or sines, two to a word
 template <bool kAligned>
-__device__ __forceinline__ void load_bf16_8(const __nv_bfloat16* p, float (&v)[8]) {
-  if constexpr (!kAligned) {
+__device__ __forceinline__ uint4 load_bf16_8(const __nv_bfloat16* p) {
+  if constexpr (kAligned) return ldg_pinned_v4(p);
+  const unsigned short* q = reinterpret_cast<const unsigned short*>(p);
+  uint32_t w[4];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) v[e] = __bfloat162float(p[e]);
-    return;
-  }
-  const uint4 w = __ldg(reinterpret_cast<const uint4*>(p));
-  const uint32_t x[4] = {w.x, w.y, w.z, w.w};
+  for (int e = 0; e < 4; ++e) w[e] = q[2 * e] | static_cast<uint32_t>(q[2 * e + 1]) << 16;
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+// The same for rows of 64 bf16 that are rotated on the way: out[j] = a[j] cos[j] - b[j] sin[j], out[32 + j] = b[j] cos[32 + j] +
+// a[j] sin[32 + j]. kPairs: a and b are the even and the odd dims (the outputs are de-interleaved), else the halves. The lane that
+// stores eight outputs computes them, so a load of cosines touches the four lines that its store does; with a row to a lane every
+// load touched 32 (1000 tokens: both up-projections 57.8 -> 53.7 us).
+template <bool kAligned, bool kPairs>
+__device__ __forceinline__ void store_rows_rotated(const WideParams& p, uint32_t stage, const uint32_t (&w)[32], int row0, uint8_t* dst,
+                                                   int64_t pitch, int n_rows) {
+  const int lane = threadIdx.x & 31, u = lane & 7;
+  const bool first = u < 4;
+  stage_rows(stage, w);
+  uint4 cs[8], sn[8];
 #pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    v[2 * e] = __uint_as_float(x[e] << 16);
-    v[2 * e + 1] = __uint_as_float(x[e] & 0xffff0000u);
+  for (int i = 0; i < 8; ++i) {
+    const int64_t at = static_cast<int64_t>(min(row0 + 4 * i + (lane >> 3), p.t - 1)) * 64 + 8 * u;
+    cs[i] = load_bf16_8<kAligned>(p.cos + at);
+    sn[i] = load_bf16_8<kAligned>(p.sin + at);
   }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = 4 * i + (lane >> 3);
+    const uint4 v0 = staged_unit(stage, r, kPairs ? 2 * (u & 3) : u), v1 = staged_unit(stage, r, kPairs ? 2 * (u & 3) + 1 : u ^ 4);
+    float x[8], y[8];  // the dim that meets the cosine, and the one that meets the sine
+    const uint32_t a[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      if constexpr (kPairs) {
+        x[e] = first ? bf16_lo(a[e]) : bf16_hi(a[e]);
+        y[e] = first ? -bf16_hi(a[e]) : bf16_lo(a[e]);
+      } else {
+        x[e] = (e & 1) != 0 ? bf16_hi(a[e >> 1]) : bf16_lo(a[e >> 1]);
+        const float o = (e & 1) != 0 ? bf16_hi(a[4 + (e >> 1)]) : bf16_lo(a[4 + (e >> 1)]);
+        y[e] = first ? -o : o;
+      }
+    }
+    const uint32_t c[4] = {cs[i].x, cs[i].y, cs[i].z, cs[i].w}, s[4] = {sn[i].x, sn[i].y, sn[i].z, sn[i].w};
+    uint32_t o[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      o[e] = pack_bf16x2(__fadd_rn(__fmul_rn(x[2 * e], bf16_lo(c[e])), __fmul_rn(y[2 * e], bf16_lo(s[e]))),
+                         __fadd_rn(__fmul_rn(x[2 * e + 1], bf16_hi(c[e])), __fmul_rn(y[2 * e + 1], bf16_hi(s[e]))));
+    }
+    if (r < n_rows) store_unit<kAligned>(dst + r * pitch + u * 16, make_uint4(o[0], o[1], o[2], o[3]));
+  }
+  __syncwarp();
 }
 
 // int32 accumulators of 64 columns -> bf16 products with the row and column scales, two to a word
@@ -176,28 +225,6 @@ __device__ __forceinline__ void wide_dequant_64(uint32_t taddr, float rs, const 
     }
   }
 }
-__device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
-__device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
-// outputs 8i .. 8i+7 and 32 + 8i .. 32 + 8i+7 of a row's rope: out[j] = a[j] cos[j] - b[j] sin[j], out[32 + j] = b[j] cos[32 + j] +
-// a[j] sin[32 + j], where a and b are the halves that turn into each other
-template <bool kAligned>
-__device__ __forceinline__ void wide_rope_8(const WideParams& p, int row, int i, const float (&a)[8], const float (&b)[8], uint32_t (&lo)[4],
-                                            uint32_t (&hi)[4]) {
-  float cs[8], sn[8], x[8];
-  load_bf16_8<kAligned>(p.cos + static_cast<int64_t>(row) * 64 + 8 * i, cs);
-  load_bf16_8<kAligned>(p.sin + static_cast<int64_t>(row) * 64 + 8 * i, sn);
-#pragma unroll
-  for (int e = 0; e < 8; ++e) x[e] = __fadd_rn(__fmul_rn(a[e], cs[e]), __fmul_rn(-b[e], sn[e]));
-#pragma unroll
-  for (int e = 0; e < 4; ++e) lo[e] = pack_bf16x2(x[2 * e], x[2 * e + 1]);
-  load_bf16_8<kAligned>(p.cos + static_cast<int64_t>(row) * 64 + 32 + 8 * i, cs);
-  load_bf16_8<kAligned>(p.sin + static_cast<int64_t>(row) * 64 + 32 + 8 * i, sn);
-#pragma unroll
-  for (int e = 0; e < 8; ++e) x[e] = __fadd_rn(__fmul_rn(b[e], cs[e]), __fmul_rn(a[e], sn[e]));
-#pragma unroll
-  for (int e = 0; e < 4; ++e) hi[e] = pack_bf16x2(x[2 * e], x[2 * e + 1]);
-}
-
 // One tile's rows out of tensor memory: this warp's 32 rows start at `row0`, `taddr` is its lanes of the tile's accumulator. The
 // alignment is a template parameter: with a branch at each of the scales' and cosines' loads they came one after the other, a trip to
 // L2 each (1000 tokens: both up-projections 70 -> 57 us, absorbed query 47.5 -> 43.3, the whole prolog 174 -> 158).
@@ -244,27 +271,9 @@ __device__ __forceinline__ void wide_epilogue(const WideParams& p, const WideIte
         store_rows<kAligned>(stage, v, reinterpret_cast<uint8_t*>(p.out) + ((static_cast<int64_t>(row0) * 128 + head) * kHeadNope + 64 * part) * 2,
                    128 * kHeadNope * 2, n_rows, 128);
       } else {
-        // de-interleaved layout: outputs 0-31 from the even dims, 32-63 from the odd ones; rotate_half = (-second, first). Eight
-        // words of dims become four words of either half of the outputs
-        uint32_t o[32];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          float even[8], odd[8];
-          uint32_t lo[4], hi[4];
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            even[e] = bf16_lo(v[8 * i + e]);
-            odd[e] = bf16_hi(v[8 * i + e]);
-          }
-          wide_rope_8<kAligned>(p, row, i, even, odd, lo, hi);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            o[4 * i + e] = lo[e];
-            o[16 + 4 * i + e] = hi[e];
-          }
-        }
-        store_rows<kAligned>(stage, o, reinterpret_cast<uint8_t*>(p.out2) + (static_cast<int64_t>(row0) * 128 + head) * 128, 128 * 128, n_rows,
-                   128);
+        // de-interleaved layout: outputs 0-31 from the even dims, 32-63 from the odd ones; rotate_half = (-second, first)
+        store_rows_rotated<kAligned, true>(p, stage, v, row0, reinterpret_cast<uint8_t*>(p.out2) + (static_cast<int64_t>(row0) * 128 + head) * 128,
+                                           128 * 128, n_rows);
       }
     }
   } else if (kEpi == kWideUp) {
@@ -273,28 +282,10 @@ __device__ __forceinline__ void wide_epilogue(const WideParams& p, const WideIte
     for (int c = 0; c < kN; c += 64) {
       uint32_t v[32];
       wide_dequant_64<kAligned>(taddr + c, rs, p.col_scale_idx + n0 + c, v);
-      if ((c & 64) == 0) {  // rope on the head's first 64 dims: halves, no de-interleave
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          float first[8], second[8];
-          uint32_t lo[4], hi[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            first[2 * e] = bf16_lo(v[4 * i + e]);
-            first[2 * e + 1] = bf16_hi(v[4 * i + e]);
-            second[2 * e] = bf16_lo(v[16 + 4 * i + e]);
-            second[2 * e + 1] = bf16_hi(v[16 + 4 * i + e]);
-          }
-          wide_rope_8<kAligned>(p, row, i, first, second, lo, hi);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            v[4 * i + e] = lo[e];
-            v[16 + 4 * i + e] = hi[e];
-          }
-        }
-      }
-      store_rows<kAligned>(stage, v, reinterpret_cast<uint8_t*>(p.out_idx) + (static_cast<int64_t>(row0) * 64 * 128 + n0 + c) * 2, 64 * 128 * 2,
-                 n_rows, 128);
+      uint8_t* dst = reinterpret_cast<uint8_t*>(p.out_idx) + (static_cast<int64_t>(row0) * 64 * 128 + n0 + c) * 2;
+      // rope on the head's first 64 dims: halves, no de-interleave
+      if ((c & 64) == 0) store_rows_rotated<kAligned, false>(p, stage, v, row0, dst, 64 * 128 * 2, n_rows);
+      else store_rows<kAligned>(stage, v, dst, 64 * 128 * 2, n_rows, 128);
     }
   } else {  // kWideHad: two readings of the row's 128 accumulators, one for the maximum, one to quantise
     static_assert(kEpi != kWideHad || kN == 128, "a Hadamard row is 128 wide");
