@@ -23,6 +23,9 @@
 // columns outside the tensors read as zeros. Two accumulators of kN columns, one per epilogue group of four warps, so
 // that one tile is stored while the next is multiplied. Items run over token blocks first: the CTAs that are at work at
 // the same time read the same weight columns from L2.
+// Of many rows two CTAs on neighbouring SMs take 256 rows x 256 columns together (tcgen05.mma.cta_group::2): each loads its own rows and
+// half of the columns, so a stage is 32 KB instead of 48, six fit, and a third less of the operands passes from L2. CTA 0 issues the
+// MMAs; each CTA stores its rows (1000 tokens: projections 32.4 -> 28.9 us, 1.14 PFLOP/s; the line is drawn at the launch).
 // Roles: warp 0 TMA, warp 1 MMA, warps 2-5 / 6-9 epilogue. All waits are bounded.
 #include <cuda.h>
 
@@ -36,16 +39,16 @@ namespace {
 
 constexpr int kWRows = 128;                  // token rows per tile (MMA M)
 constexpr int kWXBytes = kWRows * 128;
-constexpr int kWStages = 4;
 constexpr int kWThreads = 320;
 constexpr int kWStaging = 8 * 4096;           // per epilogue warp: 128 bytes of 32 rows
 constexpr int kHeadQ = 192, kHeadNope = 128;  // widths of an attention head of the up-projection
 
 enum { kWideF32 = 0, kWideBf16 = 1, kWideUp = 2, kWideHad = 3 };
 
+constexpr int kWMaxStages = 6;
 struct WideCtl {
-  uint64_t full[kWStages];
-  uint64_t empty[kWStages];
+  uint64_t full[kWMaxStages];   // (of a pair: in CTA 0, for both CTAs' bytes)
+  uint64_t empty[kWMaxStages];
   uint64_t acc_full[2];
   uint64_t acc_empty[2];
   uint32_t tmem_base;
@@ -58,7 +61,7 @@ struct WideParams {
   int n_tiles;            // kN-column tiles per problem
   int chunks, per_split, splits;
   int batch;              // problems (heads)
-  int row_blocks;
+  int row_blocks;         // (of a pair: two blocks of 128 rows)
   int w_batch_rows;       // rows of W between problems
   int x_batch_bytes;      // bytes along a row of x between problems
   long long out_batch;    // output elements between problems
@@ -78,14 +81,16 @@ struct WideParams {
   int32_t* status;
 };
 
-template <bool kI8, int kN>
+template <bool kI8, int kN, bool kPair>
 struct WideCfg {
+  static constexpr int kStages = kPair ? 6 : 4;
   static constexpr int kChunkK = kI8 ? 128 : 64;     // k per stage: 128 bytes of a row of x
   static constexpr int kGroup = kI8 ? 128 : 64;      // columns per 128-byte box of W
   static constexpr int kBoxBytes = kChunkK * 128;
-  static constexpr int kWBytes = kN / kGroup * kBoxBytes;
+  static constexpr int kBoxes = kN / kGroup / (kPair ? 2 : 1);  // of a pair, each CTA holds half of the columns
+  static constexpr int kWBytes = kBoxes * kBoxBytes;
   static constexpr int kStage = kWXBytes + kWBytes;
-  static constexpr int kSmem = kWStages * kStage + kWStaging + sizeof(WideCtl) + 1024;
+  static constexpr int kSmem = kStages * kStage + kWStaging + sizeof(WideCtl) + 1024;
   static_assert(kSmem <= 232448, "exceeds the 227 KB of shared memory a CTA may use");
   static constexpr uint32_t kTmemCols = 2 * kN;
 };
@@ -102,6 +107,68 @@ __device__ __forceinline__ WideItem wide_item(const WideParams& p, int item) {
   it.tile = r % p.n_tiles;
   it.b = r / p.n_tiles;
   return it;
+}
+
+// --- a pair of SMs on one tile (tcgen05.mma.cta_group::2) ---
+__device__ __forceinline__ uint32_t wide_cta_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t wide_in_cta0(uint32_t local) {  // the same place in the pair's first CTA
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(local));
+  return r;
+}
+__device__ __forceinline__ void wide_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// into this CTA's shared memory, completion on a barrier of either CTA of the pair
+__device__ __forceinline__ void wide_load_pair(uint32_t dst_smem, const void* tmap, int x, int y, uint32_t cluster_bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3}], [%4];"
+      ::"r"(dst_smem), "l"(tmap), "r"(x), "r"(y), "r"(cluster_bar)
+      : "memory");
+}
+template <bool kI8>
+__device__ __forceinline__ void wide_mma_pair(uint32_t d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  if constexpr (kI8) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+  } else {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+  }
+}
+// arrives on the barrier at this place in both CTAs once all MMAs issued so far have completed
+__device__ __forceinline__ void wide_commit_pair(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(bar), "h"(static_cast<uint16_t>(3))
+               : "memory");
+}
+__device__ __forceinline__ void wide_arrive_cluster(uint32_t cluster_bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+__device__ __forceinline__ bool wide_wait_cluster(uint32_t bar, uint32_t parity) {  // bounded; arrivals from both CTAs
+  const long long t0 = clock64();
+  while (true) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (ok != 0) return true;
+    if (clock64() - t0 > kWaitBudgetCycles) return false;
+  }
 }
 
 __device__ __forceinline__ float wide_bf16_round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
@@ -321,17 +388,20 @@ __device__ __forceinline__ void wide_epilogue(const WideParams& p, const WideIte
   }
 }
 
-template <bool kI8, int kEpi, int kN>
+template <bool kI8, int kEpi, int kN, bool kPair>
 __global__ void __launch_bounds__(kWThreads, 1)
 prolog_wide_kernel(const __grid_constant__ PrologWMaps maps_w,  // int8: map 0 attention, map 1 indexer
                    const __grid_constant__ CUtensorMap tmap_x, const WideParams p) {
-  using Cfg = WideCfg<kI8, kN>;
+  using Cfg = WideCfg<kI8, kN, kPair>;
+  constexpr int kWStages = Cfg::kStages;
   extern __shared__ uint8_t wide_smem_raw[];
   const uint32_t raw = smem_u32(wide_smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   WideCtl* ctl = reinterpret_cast<WideCtl*>(wide_smem_raw + (base - raw) + kWStages * Cfg::kStage + kWStaging);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n_items = p.row_blocks * p.batch * p.n_tiles * p.splits;
+  const uint32_t rank = kPair ? wide_cta_rank() : 0u;
+  constexpr int kShift = kPair ? 1 : 0;  // CTAs per worker
 
   if (tid == 0) {
     for (int i = 0; i < kWStages; ++i) {
@@ -340,7 +410,7 @@ prolog_wide_kernel(const __grid_constant__ PrologWMaps maps_w,  // int8: map 0 a
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&ctl->acc_full[i]), 1);
-      mbar_init(smem_u32(&ctl->acc_empty[i]), 4);
+      mbar_init(smem_u32(&ctl->acc_empty[i]), kPair ? 8 : 4);
     }
     ctl->abort = 0;
     fence_mbar_init();
@@ -349,11 +419,18 @@ prolog_wide_kernel(const __grid_constant__ PrologWMaps maps_w,  // int8: map 0 a
     tma_prefetch_desc(&tmap_x);
   }
   if (warp == 1) {
-    tmem_alloc(smem_u32(&ctl->tmem_base), Cfg::kTmemCols);
-    tmem_relinquish();
+    if constexpr (kPair) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctl->tmem_base)), "r"(Cfg::kTmemCols)
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      tmem_alloc(smem_u32(&ctl->tmem_base), Cfg::kTmemCols);
+      tmem_relinquish();
+    }
   }
   tc_fence_before();
   __syncthreads();
+  if constexpr (kPair) wide_cluster_sync();  // both CTAs' barriers are there
   tc_fence_after();
   const uint32_t tmem_base = ctl->tmem_base;
   pdl_wait();  // the set-up above overlaps the tail of the kernel before this one
@@ -363,21 +440,22 @@ prolog_wide_kernel(const __grid_constant__ PrologWMaps maps_w,  // int8: map 0 a
     // ---------------- producer ----------------
     bool ok = true;
     uint32_t it = 0;
-    for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+    for (int item = blockIdx.x >> kShift; item < n_items && ok; item += gridDim.x >> kShift) {
       const WideItem w = wide_item(p, item);
       const int k0 = w.split * p.per_split;
       const int kn = min(p.per_split, p.chunks - k0);
       const bool idx = kEpi == kWideUp && w.tile < p.idx_tiles;
-      constexpr int kBoxes = kN / Cfg::kGroup;
+      constexpr int kBoxes = Cfg::kBoxes;
+      const int box0 = static_cast<int>(rank) * kBoxes;  // first of this CTA's boxes of the tile
       const CUtensorMap* tm[kBoxes];
       int col[kBoxes];  // bytes
 #pragma unroll
       for (int g = 0; g < kBoxes; ++g) {
         if (kI8) {
           tm[g] = &maps_w.map[idx ? 1 : 0];
-          col[g] = (idx ? w.tile : w.tile - p.idx_tiles) * kN + g * 128;
+          col[g] = (idx ? w.tile : w.tile - p.idx_tiles) * kN + (box0 + g) * 128;
         } else {
-          tm[g] = prolog_w_box(maps_w, p.boxes, w.tile * kBoxes + g, &col[g]);
+          tm[g] = prolog_w_box(maps_w, p.boxes, w.tile * (kN / Cfg::kGroup) + box0 + g, &col[g]);
         }
       }
       for (int c = 0; c < kn; ++c, ++it) {
@@ -388,11 +466,17 @@ prolog_wide_kernel(const __grid_constant__ PrologWMaps maps_w,  // int8: map 0 a
           const uint32_t bar = smem_u32(&ctl->full[s]);
           const uint32_t dst = base + s * Cfg::kStage;
           const int krow = w.b * p.w_batch_rows + (k0 + c) * Cfg::kChunkK;
-          mbar_arrive_expect_tx(bar, Cfg::kStage);
-          tma_load_2d(dst, &tmap_x, w.b * p.x_batch_bytes + (k0 + c) * 128, w.rb * kWRows, bar);
+          if constexpr (kPair) {
+            if (rank == 0) mbar_arrive_expect_tx(bar, 2 * Cfg::kStage);
+            const uint32_t bar0 = wide_in_cta0(bar);
+            wide_load_pair(dst, &tmap_x, w.b * p.x_batch_bytes + (k0 + c) * 128, (2 * w.rb + static_cast<int>(rank)) * kWRows, bar0);
 #pragma unroll
-          for (int g = 0; g < kBoxes; ++g) {
-            tma_load_2d(dst + kWXBytes + g * Cfg::kBoxBytes, tm[g], col[g], krow, bar);
+            for (int g = 0; g < kBoxes; ++g) wide_load_pair(dst + kWXBytes + g * Cfg::kBoxBytes, tm[g], col[g], krow, bar0);
+          } else {
+            mbar_arrive_expect_tx(bar, Cfg::kStage);
+            tma_load_2d(dst, &tmap_x, w.b * p.x_batch_bytes + (k0 + c) * 128, w.rb * kWRows, bar);
+#pragma unroll
+            for (int g = 0; g < kBoxes; ++g) tma_load_2d(dst + kWXBytes + g * Cfg::kBoxBytes, tm[g], col[g], krow, bar);
           }
         }
         __syncwarp();
@@ -404,15 +488,19 @@ prolog_wide_kernel(const __grid_constant__ PrologWMaps maps_w,  // int8: map 0 a
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    constexpr uint32_t idesc = kI8 ? umma_idesc(kCFmtS32, kABFmtS8, kABFmtS8, 0, 1, kWRows, kN)
-                                   : umma_idesc(kCFmtF32, kABFmtBF16, kABFmtBF16, 0, 1, kWRows, kN);
+    constexpr int kM = kPair ? 2 * kWRows : kWRows;
+    constexpr uint32_t idesc = kI8 ? umma_idesc(kCFmtS32, kABFmtS8, kABFmtS8, 0, 1, kM, kN)
+                                   : umma_idesc(kCFmtF32, kABFmtBF16, kABFmtBF16, 0, 1, kM, kN);
     bool ok = true;
     uint32_t it = 0, ti = 0;
-    for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++ti) {
+    for (int item = rank == 0 ? blockIdx.x >> kShift : n_items; item < n_items && ok; item += gridDim.x >> kShift, ++ti) {  // (of a pair: CTA 0 for both)
       const WideItem w = wide_item(p, item);
       const int kn = min(p.per_split, p.chunks - w.split * p.per_split);
       const uint32_t acc = ti & 1;
-      if (ti >= 2) ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->acc_empty[acc]), ((ti >> 1) - 1) & 1));
+      if (ti >= 2) {
+        const uint32_t bar = smem_u32(&ctl->acc_empty[acc]), ph = ((ti >> 1) - 1) & 1;
+        ok = __all_sync(0xffffffffu, kPair ? wide_wait_cluster(bar, ph) : mbar_wait(bar, ph));
+      }
       if (!ok) break;
       tc_fence_after();
       const uint32_t d = tmem_base + acc * kN;
@@ -427,11 +515,17 @@ prolog_wide_kernel(const __grid_constant__ PrologWMaps maps_w,  // int8: map 0 a
           const uint64_t b_desc = desc_mnmajor_sw128(a + kWXBytes, Cfg::kBoxBytes, 1024);
 #pragma unroll
           for (int j = 0; j < 4; ++j) {  // 32 bytes along x's rows; 32 (int8) or 16 (bf16) rows of W
-            if (kI8) mma_i8_ss(d, a_desc + 2 * j, b_desc + j * (4096 >> 4), idesc, (c | j) != 0 ? 1u : 0u);
+            if (kPair) wide_mma_pair<kI8>(d, a_desc + 2 * j, b_desc + j * ((kI8 ? 4096 : 2048) >> 4), idesc, (c | j) != 0 ? 1u : 0u);
+            else if (kI8) mma_i8_ss(d, a_desc + 2 * j, b_desc + j * (4096 >> 4), idesc, (c | j) != 0 ? 1u : 0u);
             else mma_f16_ss(d, a_desc + 2 * j, b_desc + j * (2048 >> 4), idesc, (c | j) != 0 ? 1u : 0u);
           }
-          tc_commit(smem_u32(&ctl->empty[s]));
-          if (c + 1 == kn) tc_commit(smem_u32(&ctl->acc_full[acc]));
+          if constexpr (kPair) {
+            wide_commit_pair(smem_u32(&ctl->empty[s]));
+            if (c + 1 == kn) wide_commit_pair(smem_u32(&ctl->acc_full[acc]));
+          } else {
+            tc_commit(smem_u32(&ctl->empty[s]));
+            if (c + 1 == kn) tc_commit(smem_u32(&ctl->acc_full[acc]));
+          }
         }
         __syncwarp();
       }
@@ -446,7 +540,7 @@ prolog_wide_kernel(const __grid_constant__ PrologWMaps maps_w,  // int8: map 0 a
     const uint32_t g = static_cast<uint32_t>(warp - 2) >> 2;
     bool ok = true;
     uint32_t ti = 0;
-    for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++ti) {
+    for (int item = blockIdx.x >> kShift; item < n_items; item += gridDim.x >> kShift, ++ti) {
       if ((ti & 1) != g) continue;
       ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->acc_full[g]), (ti >> 1) & 1));
       if (!ok) break;
@@ -454,11 +548,15 @@ prolog_wide_kernel(const __grid_constant__ PrologWMaps maps_w,  // int8: map 0 a
       const WideItem w = wide_item(p, item);
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + g * kN;
       const uint32_t stage = base + kWStages * Cfg::kStage + static_cast<uint32_t>(warp - 2) * 4096u;
-      if (p.aligned) wide_epilogue<kEpi, kN, true>(p, w, taddr, w.rb * kWRows + q * 32, stage);
-      else wide_epilogue<kEpi, kN, false>(p, w, taddr, w.rb * kWRows + q * 32, stage);
+      const int row0 = (kPair ? 2 * w.rb + static_cast<int>(rank) : w.rb) * kWRows + q * 32;
+      if (p.aligned) wide_epilogue<kEpi, kN, true>(p, w, taddr, row0, stage);
+      else wide_epilogue<kEpi, kN, false>(p, w, taddr, row0, stage);
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&ctl->acc_empty[g]));
+      if (lane == 0) {
+        if (!kPair || rank == 0) mbar_arrive(smem_u32(&ctl->acc_empty[g]));
+        else wide_arrive_cluster(wide_in_cta0(smem_u32(&ctl->acc_empty[g])));
+      }
     }
     if (!ok && lane == 0) {
       ctl->abort = 1;
@@ -473,9 +571,11 @@ prolog_wide_kernel(const __grid_constant__ PrologWMaps maps_w,  // int8: map 0 a
     for (int i = 0; i < 1000; ++i) __nanosleep(1000);
     __syncthreads();
   }
+  if constexpr (kPair) wide_cluster_sync();  // neither CTA leaves while the other's loads, MMAs or arrivals may still reach it
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, Cfg::kTmemCols);
+    if constexpr (kPair) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(Cfg::kTmemCols) : "memory");
+    else tmem_dealloc(tmem_base, Cfg::kTmemCols);
   }
 }
 
@@ -486,23 +586,48 @@ int wide_aligned(std::initializer_list<const void*> ptrs) {
   return 1;
 }
 
-template <bool kI8, int kEpi, int kN>
-cudaError_t wide_launch(const PrologWMaps& maps_w, const void* tmap_x, WideParams& p, int k, int num_sms, cudaStream_t stream, bool pdl) {
-  using Cfg = WideCfg<kI8, kN>;
+template <bool kI8, int kEpi, int kN, bool kPair>
+cudaError_t wide_launch_as(const PrologWMaps& maps_w, const void* tmap_x, WideParams& p, int k, int num_sms, cudaStream_t stream, bool pdl) {
+  using Cfg = WideCfg<kI8, kN, kPair>;
   p.n_tiles = (p.n + kN - 1) / kN;
   p.chunks = (k + Cfg::kChunkK - 1) / Cfg::kChunkK;
   p.per_split = (p.chunks + p.splits - 1) / p.splits;
   if ((p.chunks + p.per_split - 1) / p.per_split != p.splits) return cudaErrorInvalidValue;  // a split without work
-  p.row_blocks = (p.t + kWRows - 1) / kWRows;
-  auto kernel = prolog_wide_kernel<kI8, kEpi, kN>;
+  constexpr int kRows = kPair ? 2 * kWRows : kWRows, kCtas = kPair ? 2 : 1;
+  p.row_blocks = (p.t + kRows - 1) / kRows;
+  auto kernel = prolog_wide_kernel<kI8, kEpi, kN, kPair>;
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem);
   if (e != cudaSuccess) return e;
   const long long items = static_cast<long long>(p.row_blocks) * p.batch * p.n_tiles * p.splits;
   if (items > 0x7fffffffLL) return cudaErrorInvalidValue;
-  const int grid = static_cast<int>(items < num_sms ? items : num_sms);
+  const int units = num_sms / kCtas;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(kCtas * (items < units ? static_cast<int>(items) : units)), 1, 1);
+  cfg.blockDim = dim3(kWThreads, 1, 1);
+  cfg.dynamicSmemBytes = Cfg::kSmem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kCtas;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 2 : 1;
   count_launch();
-  return launch_maybe_pdl(kernel, dim3(grid), dim3(kWThreads), Cfg::kSmem, stream, pdl,
-                          maps_w, *reinterpret_cast<const CUtensorMap*>(tmap_x), p);
+  return cudaLaunchKernelEx(&cfg, kernel, maps_w, *reinterpret_cast<const CUtensorMap*>(tmap_x), static_cast<const WideParams&>(p));
+}
+
+// Pairs of SMs from four blocks of 128 rows on. Whole prolog, a CTA per tile -> a pair, us: 200 rows 63.4 -> 63.7, 256 67.0 -> 68.3, 300
+// 81.1 -> 85.7, 512 95.8 -> 94.3, 600 115.1 -> 113.9, 1000 153.4 -> 148.8, 1100 180.0 -> 173.3, 2048 279.3 -> 267.7, 4096 561 -> 526. The
+// absorbed query has two chunks of K per tile and is bound by its stores (pairs 47 -> 51), the Hadamard matrix fits one CTA's tile.
+template <bool kI8, int kEpi, int kN>
+cudaError_t wide_launch(const PrologWMaps& maps_w, const void* tmap_x, WideParams& p, int k, int num_sms, cudaStream_t stream, bool pdl) {
+  if constexpr (kEpi == kWideUp || kEpi == kWideF32) {
+    if (p.t > 3 * kWRows) return wide_launch_as<kI8, kEpi, kN, true>(maps_w, tmap_x, p, k, num_sms, stream, pdl);
+  }
+  return wide_launch_as<kI8, kEpi, kN, false>(maps_w, tmap_x, p, k, num_sms, stream, pdl);
 }
 
 }  // namespace
