@@ -644,11 +644,15 @@ cudaError_t wide_launch_as(const PrologWMaps& maps_w, const void* tmap_x, WidePa
 
 // Pairs of SMs from four blocks of 128 rows on. Whole prolog, a CTA per tile -> a pair, us: 200 rows 63.4 -> 63.7, 256 67.0 -> 68.3, 300
 // 81.1 -> 85.7, 512 95.8 -> 94.3, 600 115.1 -> 113.9, 1000 153.4 -> 148.8, 1100 180.0 -> 173.3, 2048 279.3 -> 267.7, 4096 561 -> 526. The
-// absorbed query has two chunks of K per tile and is bound by its stores (pairs 47 -> 51), the Hadamard matrix fits one CTA's tile.
+// bf16 up-projections of the non-quantised prolog: 385 109.0 -> 105.5, 1000 180.2 -> 170.7, 2048 335.8 -> 313.8, but not five blocks, with
+// a sixth of the work empty (513 127.8 -> 129.2). The absorbed query has two chunks of K per tile and is bound by its stores (pairs
+// 47 -> 51), the Hadamard matrix fits one CTA's tile.
 template <bool kI8, int kEpi, int kN>
 cudaError_t wide_launch(const PrologWMaps& maps_w, const void* tmap_x, WideParams& p, int k, int num_sms, cudaStream_t stream, bool pdl) {
-  if constexpr (kEpi == kWideUp || kEpi == kWideF32) {
-    if (p.t > 3 * kWRows) return wide_launch_as<kI8, kEpi, kN, true>(maps_w, tmap_x, p, k, num_sms, stream, pdl);
+  if constexpr (kEpi != kWideHad) {
+    const int blocks = (p.t + kWRows - 1) / kWRows;
+    const bool pairs = blocks >= 4 && (kEpi != kWideBf16 || (blocks != 5 && k > 128));
+    if (pairs) return wide_launch_as<kI8, kEpi, kN, true>(maps_w, tmap_x, p, k, num_sms, stream, pdl);
   }
   return wide_launch_as<kI8, kEpi, kN, false>(maps_w, tmap_x, p, k, num_sms, stream, pdl);
 }

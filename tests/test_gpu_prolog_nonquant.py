@@ -92,6 +92,18 @@ def test_against_oracle(act_seq, s1):
     check_untouched(o, p)
 
 
+@pytest.mark.parametrize("t", [385, 513])  # the first counts of two SMs to a tile of the projections, and of the norm that keeps its row in registers
+def test_many_rows_against_oracle(t):
+    p = gen.make_prolog_nonquant_inputs([130] * t, s1=1, seed=t)
+    o, _ = run_prolog(p, with_q_norm=True)
+    want = po.mla_indexer_prolog_nonquant(p, 1e-5, 1e-5)
+    for key in ("q_norm", "q_nope", "q_rope", "idx_query", "weights"):
+        close(o[key], want[key], key)
+    for key in ("kv_cache", "kr_cache", "idx_k_cache"):
+        close(o[key][p["cache_index"]], want[key][p["cache_index"]], key)
+    check_untouched(o, p)
+
+
 def test_whole_layer_against_oracle_chain():
     """`decode_indexer_attention_layer` (arguments in the reference's order, sin before cos): its selection against
     the oracle indexer run on the oracle prolog's outputs, its attention against the oracle attention on the kernel's
