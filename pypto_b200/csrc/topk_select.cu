@@ -366,7 +366,8 @@ __device__ __noinline__ float sample_bound_fine(Smem* sm, const float* row, int 
 }
 
 // Lower bound of the k largest of row[0, eff) from a sample: 1024 groups of four, or a multiple of that: long rows need a larger
-// sample for a list of the same length (beyond 2^20 positions one that meets 32 or more of 2048 selected ones). -inf: no useful bound.
+// sample for a list of the same length (beyond 2^20 positions one that meets 32 or more of 2048 selected ones, which is enough for a
+// list of 6144; rows as long as that do not come here with the list of 5120). -inf: no useful bound.
 template <typename Smem>
 __device__ float sample_bound(Smem* sm, const float* row, int eff, int k) {
   const int tid = threadIdx.x;
@@ -792,8 +793,13 @@ cudaError_t launch_li_topk(const TopkParams& p, int num_sms, cudaStream_t stream
   while (csize < 8 && rows * csize * 2 <= num_sms && p.row_stride > static_cast<int64_t>(csize) * 8192) csize *= 2;
   // More rows than SMs: two to an SM, so that one streams while the other finds its bound or orders its list (behind their score
   // kernel, with the scan by groups of warps: 4096 rows of 131072 990 -> 780 us, 256 rows 88 -> 78; 4096 rows of 4096, which are lists,
-  // 106 -> 79, 1000 rows of 3000 42 -> 27). Not where only the longer list of a CTA alone takes whole rows.
-  const bool many = rows > num_sms && p.hist == nullptr &&
+  // 106 -> 79, 1000 rows of 3000 42 -> 27). Not where only the longer list of a CTA alone takes whole rows, and not rows so long that
+  // the sample's bound leaves the shorter list no room: what it collects, about 2048 (1 + 4.5 / sqrt(m) + 4 / m) keys where the sample
+  // meets m of 2048 selected ones, is 4.4 standard deviations below 5120 at m = 51, i.e. 655360 positions, and from 960 thousand on too
+  // many to be expected at all, so that such rows went to the radix select (200 rows, us, one to an SM / two: 600000 positions 153 / 132,
+  // 983040 226 / 481, 2^20 223 / 1286; two with twice the sample 326, 342).
+  constexpr int64_t kManyMaxRow = 5 << 17;
+  const bool many = rows > num_sms && p.hist == nullptr && p.row_stride <= kManyMaxRow &&
                     (p.row_stride <= TopkSmem<true>::kListCap || p.row_stride > TopkSmem<false>::kListCap);
   auto kernel = many ? li_topk_kernel<true> : li_topk_kernel<false>;
   static_assert(sizeof(TopkSmem<true>) <= 113 * 1024, "two CTAs to an SM");

@@ -462,6 +462,23 @@ def test_neighbouring_positions_need_no_radix_select(where, rows, n, sort):
     assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("n", [640000, 655361, 900000, 983040, 1048576, 1500000])
+def test_many_long_rows_need_no_radix_select(n):
+    """More rows than SMs, around and beyond the length up to which two of them share an SM."""
+    rows, k = 150, 2048
+    g = torch.Generator(device=DEV).manual_seed(n)
+    sc = torch.randn(rows, (n + 127) // 128 * 128, generator=g, device=DEV)
+    act = torch.full((rows,), n, dtype=torch.int32, device=DEV)
+    out = torch.zeros((rows, 1, k), dtype=torch.int32, device=DEV)
+    pto.reset_workspace_status()
+    pto.lightning_indexer_topk(sc, act, out, 1, k)
+    status = pto.workspace_status()
+    assert status[0] == 0 and status[_lib.PTO_STATUS_RADIX_ROWS] == 0
+    got = out[:, 0].long()
+    assert torch.equal(sc.gather(1, got), sc[:, :n].topk(k, dim=1).values)
+    assert torch.all(got.sort(dim=1).values.diff(dim=1) > 0) and int(got.max()) < n
+
+
 @pytest.mark.parametrize("sort", [True, False], ids=["ordered", "unordered"])
 @pytest.mark.parametrize("rows,n", [(3, 5000), (8, 32768), (40, 65536), (160, 20000), (2, 1200000)])
 @pytest.mark.parametrize("kind", ["outlier", "far_outliers", "tail", "masked", "infinite", "offset", "small"])
