@@ -39,19 +39,19 @@ constexpr int kBins = 2048;
 constexpr int kMaxK = 2048;
 constexpr int kBinCap = 512;               // keys of a bin that are still ranked by counting
 
-// A chunk of the row is one bulk copy, read by four of the sixteen warps, sixteen values a thread; the four groups take the chunks in
-// turn, each through places of its own. (What a warp spends per chunk besides the comparisons, about 100 instructions and a chain
-// of shared-memory round trips, is what the scan costs; with all warps in each chunk and eight values a thread a row of
-// 131072 took 64 k cycles beside another, 2 k per chunk.)
-constexpr int kGroups = 4, kGroupWarps = kTopkWarps / kGroups;
-constexpr int kVals = 16;
-constexpr int kChunk = 32 * kGroupWarps * kVals;  // positions
-// kMany: two CTAs share an SM, each with a whole row (see launch_li_topk): fewer copies in flight, a shorter list, and none besides the
-// row's own
+constexpr int kVals = 16;                  // of a chunk per thread
+// A chunk of the row is one bulk copy. kMany: two CTAs share an SM, each with a whole row (see launch_li_topk): fewer copies in flight, a
+// shorter list, and none besides the row's own. A chunk is read by four of the sixteen warps; the four groups take the chunks in turn,
+// each through places of its own. (What a warp spends per chunk besides the comparisons, about 100 instructions and a chain of
+// shared-memory round trips, is what the scan costs there; with all warps in each chunk and eight values a thread a row of 131072 took
+// 64 k cycles beside another, 2 k per chunk.) A CTA alone on its SM waits for the copies: all warps take each chunk, larger ones and
+// fewer (one row to a CTA or cluster, four groups / one, us: 128 x 131072 23.7 / 23.0, 64 x 131072 18.4 / 17.8, 1 x 5000000 95.1 / 91.0).
 template <bool kMany>
 struct TopkSmem {
-  static constexpr int kPlaces = kMany ? 2 : 3;        // chunks of a group in flight
-  static constexpr int kRing = kGroups * kPlaces;      // 64 / 96 KB
+  static constexpr int kGroups = kMany ? 4 : 1, kGroupWarps = kTopkWarps / kGroups;
+  static constexpr int kChunk = 32 * kGroupWarps * kVals;  // positions
+  static constexpr int kPlaces = kMany ? 2 : 3;            // chunks of a group in flight
+  static constexpr int kRing = kGroups * kPlaces;          // 64 / 96 KB
   static constexpr int kListCap = kMany ? 5120 : 6144;
   static_assert(kMaxK <= kListCap, "a row of at most k positions is handled as a list");
   union {
@@ -444,6 +444,7 @@ __global__ void __launch_bounds__(kTopkThreads, kMany ? 2 : 1)
 li_topk_kernel(TopkParams p) {
   using Smem = TopkSmem<kMany>;
   constexpr int kRing = Smem::kRing, kPlaces = Smem::kPlaces, kListCap = Smem::kListCap;
+  constexpr int kGroups = Smem::kGroups, kGroupWarps = Smem::kGroupWarps, kChunk = Smem::kChunk;
   extern __shared__ __align__(16) uint8_t topk_smem_raw[];
   Smem* sm = reinterpret_cast<Smem*>(topk_smem_raw);
   // with programmatic serialization the score kernel before it may still be running
@@ -568,8 +569,13 @@ li_topk_kernel(TopkParams p) {
 #pragma unroll
       for (int u = 0; u < kVals / 4; ++u) {
         const float4 v = *reinterpret_cast<const float4*>(chunk + offset(4 * u));
-        mask |= (at_least(v.x, bound) & (1u << (4 * u))) | (at_least(v.y, bound) & (2u << (4 * u)));
-        mask |= (at_least(v.z, bound) & (4u << (4 * u))) | (at_least(v.w, bound) & (8u << (4 * u)));
+        if constexpr (kMany) {
+          mask |= (at_least(v.x, bound) & (1u << (4 * u))) | (at_least(v.y, bound) & (2u << (4 * u)));
+          mask |= (at_least(v.z, bound) & (4u << (4 * u))) | (at_least(v.w, bound) & (8u << (4 * u)));
+        } else {  // (the masks of the other form, us: 1 x 5000000 91.0 -> 91.9, 200 x 2^20 222.7 -> 225.6)
+          mask |= (v.x >= bound ? 1u << (4 * u) : 0u) | (v.y >= bound ? 2u << (4 * u) : 0u) | (v.z >= bound ? 4u << (4 * u) : 0u) |
+                  (v.w >= bound ? 8u << (4 * u) : 0u);
+        }
       }
       if (p0 + kChunk > end) {  // the last chunk: what lies behind the end is not part of the row
 #pragma unroll
