@@ -642,16 +642,19 @@ cudaError_t wide_launch_as(const PrologWMaps& maps_w, const void* tmap_x, WidePa
   return cudaLaunchKernelEx(&cfg, kernel, maps_w, *reinterpret_cast<const CUtensorMap*>(tmap_x), static_cast<const WideParams&>(p));
 }
 
-// Pairs of SMs from four blocks of 128 rows on. Whole prolog, a CTA per tile -> a pair, us: 200 rows 63.4 -> 63.7, 256 67.0 -> 68.3, 300
-// 81.1 -> 85.7, 512 95.8 -> 94.3, 600 115.1 -> 113.9, 1000 153.4 -> 148.8, 1100 180.0 -> 173.3, 2048 279.3 -> 267.7, 4096 561 -> 526. The
-// bf16 up-projections of the non-quantised prolog: 385 109.0 -> 105.5, 1000 180.2 -> 170.7, 2048 335.8 -> 313.8, but not five blocks, with
-// a sixth of the work empty (513 127.8 -> 129.2). The absorbed query has two chunks of K per tile and is bound by its stores (pairs
-// 47 -> 51), the Hadamard matrix fits one CTA's tile.
+// Pairs of SMs from four blocks of 128 rows on; with fewer, whole prologs lost (two blocks up to 1.4 us, three up to 4.9). What a pair saves
+// of a tile has to outweigh the work of the last pair's missing block, if the number of blocks is odd. The projections and the bf16
+// up-projections save enough at any count: whole prolog by blocks, a CTA per tile -> pairs, us: projections 5 112.2 -> 109.4, 8 145.7 -> 139.8,
+// 16 261.5 -> 252.3; bf16 up-projections 4 115.5 -> 110.7, 5 138.0 -> 137.2, 7 168.2 -> 165.2, 8 185.2 -> 174.5, 16 343 -> 322. Those of
+// int8 save about a sixteenth, so pairs where the empty share is no more: 4 94.4 -> 92.8, 8 145.7 -> 144.4, 16 261.5 -> 256.8, but 5 112.2 ->
+// 114.7, 7 136.5 -> 138.7, 9 173.7 -> 175.4, 13 228.0 -> 230.3; 15 249.8 -> 248.9, 21 363.5 -> 359.7. The absorbed query has two chunks of K per tile
+// and is bound by its stores (pairs 47 -> 51), the Hadamard matrix fits one CTA's tile.
 template <bool kI8, int kEpi, int kN>
 cudaError_t wide_launch(const PrologWMaps& maps_w, const void* tmap_x, WideParams& p, int k, int num_sms, cudaStream_t stream, bool pdl) {
   if constexpr (kEpi != kWideHad) {
     const int blocks = (p.t + kWRows - 1) / kWRows;
-    const bool pairs = blocks >= 4 && (kEpi != kWideBf16 || (blocks != 5 && k > 128));
+    const int empty = blocks & 1;
+    const bool pairs = blocks >= 4 && (kEpi != kWideBf16 || k > 128) && (kEpi != kWideUp || 16 * empty <= blocks + empty);
     if (pairs) return wide_launch_as<kI8, kEpi, kN, true>(maps_w, tmap_x, p, k, num_sms, stream, pdl);
   }
   return wide_launch_as<kI8, kEpi, kN, false>(maps_w, tmap_x, p, k, num_sms, stream, pdl);
