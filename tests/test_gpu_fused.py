@@ -4,6 +4,7 @@ import torch
 
 import oracle
 import pypto_b200 as pto
+from pypto_b200 import _lib
 from pypto_b200 import inputs as gen
 
 pytestmark = pytest.mark.gpu
@@ -140,7 +141,7 @@ def test_empty_and_tiny_sequences():
     assert e["max_abs"] <= 2e-2 and e["rel_l2"] <= 5e-3, e
 
 
-@pytest.mark.parametrize("b,s1", [(3, 2), (64, 1), (70, 1)])
+@pytest.mark.parametrize("b,s1", [(3, 2), (64, 1), (70, 1), (75, 1), (40, 2)])  # the last two: tokens left over by a round of SM pairs are split
 def test_back_to_back_fused_calls_equal_the_stages_run_one_by_one(b, s1):
     """Inside the fused call the top-k and attention kernels are launched with programmatic serialization (they
     may start while their predecessor drains). Six calls without any synchronisation in between, a fill kernel
@@ -173,6 +174,47 @@ def test_back_to_back_fused_calls_equal_the_stages_run_one_by_one(b, s1):
                                            576 ** -0.5, 2048, 128, d.max_blocks)
         torch.cuda.synchronize()
         assert torch.equal(out2, outs[r])
+
+
+def test_a_chain_of_two_rounds_with_a_bf16_cache_equals_its_stages():
+    """76 tokens, the last two of which are split: the chain's partials lie behind what its other stages use."""
+    d = gen.make_nonquant_inputs([130, 3000] * 19, s1=2, seed=4, device=DEV)
+    idx = torch.full((d.t, 1, 2048), -7, dtype=torch.int32, device=DEV)
+    out, alone = (torch.full((d.b, 2, 128, 512), f, dtype=torch.bfloat16, device=DEV) for f in (7.0, 5.0))
+    args = (d.query_nope, d.query_rope, d.key_nope_2d, d.key_rope_2d)
+    pto.decode_indexer_attention(d.idx_query, d.idx_key_cache, d.idx_weight, *args, d.act_seq_key, d.block_table, idx, out)
+    pto.sparse_flash_attention_quant_d(*args, None, idx.reshape(d.t, 2048), d.block_table, d.act_seq_key, alone, 128, 1, 576 ** -0.5, 2048,
+                                       128, d.max_blocks)
+    torch.cuda.synchronize()
+    assert pto.workspace_status()[0] == 0
+    assert torch.equal(out, alone)
+
+
+def test_a_chain_keeps_to_a_workspace_of_the_size_it_needs():
+    """A C caller's workspace without room for the last round's partials: the call runs unsplit and touches nothing behind it."""
+    d = gen.make_inputs([1500] + [130] * 73 + [1500], s1=1, seed=6, device=DEV)
+    lib = _lib.load()
+    need, extra = lib.pto_decode_workspace_bytes(75, d.max_blocks, 128, 128), lib.pto_sfa_extra_bytes(75, 128)
+    assert extra > 0
+    tensors = (d.query_nope, d.query_rope, d.key_nope_2d, d.key_rope_2d, d.k_nope_scales, d.act_seq_key, d.block_table)
+    li = (d.idx_query, d.idx_query_scale, d.idx_key_cache, d.idx_key_scale, d.idx_weight)
+    results = []
+    for size in (need, need + extra - 1, need + extra):
+        ws = torch.full((need + extra + 4096,), 0x5a, dtype=torch.uint8, device=DEV)
+        ws[:need] = 0
+        idx = torch.full((75, 1, 2048), -7, dtype=torch.int32, device=DEV)
+        out = torch.full((75, 1, 128, 512), 7.0, dtype=torch.bfloat16, device=DEV)
+        rc = lib.pto_decode_fused(*(x.data_ptr() for x in li), _lib.PTO_DT_F32, *(x.data_ptr() for x in tensors), idx.data_ptr(), out.data_ptr(),
+                                  75, 1, d.idx_key_cache.shape[0], d.max_blocks, 2048, 128, 576 ** -0.5, _lib.PTO_LI_UNSORTED, ws.data_ptr(),
+                                  size, torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        assert rc == 0 and int(ws[:4].view(torch.int32)) == 0
+        assert torch.all(ws[size if size == need + extra else need:] == 0x5a)
+        results.append(out)
+    assert torch.equal(results[0], results[1])
+    assert torch.equal(results[0][:74], results[2][:74])  # (the last one is split)
+    e = oracle.attention_errors(results[2].cpu(), results[0].cpu())
+    assert e["max_abs"] <= 2e-2 and e["rel_l2"] <= 5e-3, e
 
 
 def test_random_shapes_against_oracle_chain():

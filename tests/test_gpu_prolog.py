@@ -195,6 +195,14 @@ def test_row_counts_of_several_tiles(t, odd):
     check_against(run_prolog(p, odd_outputs=odd), po.mla_indexer_prolog(p, eps_cq=1e-5, eps_ckv=1e-5), p["cache_index"])
 
 
+@pytest.mark.parametrize("t", [385, 520, 1000])  # pairs of SMs for projections and up-projections, for projections only, for both again
+def test_unaligned_outputs_equal_aligned_ones(t):
+    p = gen.make_prolog_inputs([130] * t, s1=1, seed=t)
+    want, got = run_prolog(p), run_prolog(p, odd_outputs=True)
+    for key in want:
+        assert torch.equal(got[key], want[key]), key
+
+
 def test_bad_cache_index_is_reported_not_written():
     p = gen.make_prolog_inputs([200, 300], s1=1, seed=4)
     p["cache_index"][1] = p["kv_cache"].shape[0] + 5
