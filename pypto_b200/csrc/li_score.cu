@@ -194,7 +194,7 @@ __device__ __forceinline__ float weighted_relu_sum_32(const uint32_t (&v)[32], c
   return (a01.x + a01.y) + (a23.x + a23.y);
 }
 
-template <int kMode>
+template <int kMode, bool kByGroup>
 __global__ void __launch_bounds__(kLiThreads, 1)
 li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_q, LiParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -257,21 +257,22 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
   // The CTAs share it by cost: a group's queries and weights take as long as `kGroupCost` of its pages, and the first groups have
   // few of these (by pages alone the first CTA got seventy groups of a chunk of 4096). 4096 tokens that are the prompt 208 -> 137 us,
   // behind 12288 keys 756 -> 642, 512 tokens 12.4 -> 11.0; with few tokens behind many keys there is nothing to leave out.
-  const bool by_group = p.causal != 0 && p.b == 1 && p.groups > 1 && p.groups <= kMaxSeqPerLaunch;
-  const int n_lists = by_group ? p.groups : p.b;
+  // kByGroup: kernels of their own, since calls that have nothing to leave out lose by the code for it (whole steps with inputs that are not
+  // in L2: 10 sequences of three tokens 79.3 / 77.9 us, 40 of one 109.5 / 108.2; a bf16 layer of 16 95.0 / 93.7).
+  const int n_lists = kByGroup ? p.groups : p.b;
   constexpr int kGroupCost = 2;
-  const int head = by_group ? kGroupCost : 0;  // units of cost before a list's first page
+  constexpr int head = kByGroup ? kGroupCost : 0;  // units of cost before a list's first page
   if (warp == kLiEpilogueWarp0) {
     // exclusive prefix of pages per sequence (or token group)
     int carry = 0;
-    const int first_end = by_group ? p.act_seq[0] - p.s1_total + p.tok_offset + s1 : 0;  // causal end of the first group
+    const int first_end = kByGroup ? p.act_seq[0] - p.s1_total + p.tok_offset + s1 : 0;  // causal end of the first group
     for (int b0 = 0; b0 < n_lists; b0 += 32) {
       int v = 0;
       if (b0 + lane < n_lists) {
-        int s = by_group ? first_end + (b0 + lane) * s1 : p.act_seq[b0 + lane];
+        int s = kByGroup ? first_end + (b0 + lane) * s1 : p.act_seq[b0 + lane];
         s = max(s, 0);
         v = min((s + kPageKeys - 1) / kPageKeys, p.max_blocks);
-        if (v > 0) v += head;
+        if (kByGroup && v > 0) v += head;
       }
       int incl = v;
 #pragma unroll
@@ -291,7 +292,7 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
 
   // pages of all sequences, once per token group
   const int total = ctl->prefix[n_lists];
-  const long long all = static_cast<long long>(total) * (by_group ? 1 : p.groups);
+  const long long all = static_cast<long long>(total) * (kByGroup ? 1 : p.groups);
   const long long it0 = all * blockIdx.x / gridDim.x, it1 = all * (blockIdx.x + 1) / gridDim.x;
 
   const uint32_t idesc1 = kBf16 ? umma_idesc(kCFmtF32, kABFmtBF16, kABFmtBF16, 0, 0, 128, kHeads)
@@ -338,15 +339,15 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
     }
     while (ctl->prefix[li + 1] <= lc) ++li;
     const int cost = static_cast<int>(min(it1 - cur, static_cast<long long>(ctl->prefix[li + 1] - lc)));
-    const int page0 = max(0, lc - ctl->prefix[li] - head);
-    const int npages = max(0, lc - ctl->prefix[li] - head + cost) - page0;
-    if (npages == 0) {  // (the same in every thread)
+    const int page0 = kByGroup ? max(0, lc - ctl->prefix[li] - head) : lc - ctl->prefix[li];
+    const int npages = kByGroup ? max(0, lc - ctl->prefix[li] - head + cost) - page0 : cost;
+    if (kByGroup && npages == 0) {  // (the same in every thread)
       cur += cost;
       continue;
     }
-    const int bi = by_group ? 0 : li;
+    const int bi = kByGroup ? 0 : li;
     const int seq_len = p.act_seq[bi];
-    const int tok_first = p.tok_offset + (by_group ? li : group) * s1;  // first query token of the segment within its sequence
+    const int tok_first = p.tok_offset + (kByGroup ? li : group) * s1;  // first query token of the segment within its sequence
     const int64_t tok0 = static_cast<int64_t>(bi) * p.s1_total + tok_first;
 
     // The producer warp takes no part in the two barriers of a segment: the ring's own barriers order its loads, so
@@ -760,8 +761,12 @@ li_score_simt_kernel(LiParams p) {
 
 cudaError_t launch_li_score_tc(const LiParams& p, const void* tmap_k, const void* tmap_q, int num_sms,
                                cudaStream_t stream) {
-  auto kernel = p.bf16 ? li_score_tc_kernel<kLiBf16>
-                       : (p.fp16_chain ? li_score_tc_kernel<kLiChain> : (p.s1 > 1 ? li_score_tc_kernel<kLiQuantTc> : li_score_tc_kernel<kLiQuant>));
+  auto kernel = p.bf16 ? li_score_tc_kernel<kLiBf16, false>
+                       : (p.fp16_chain ? li_score_tc_kernel<kLiChain, false>
+                                       : (p.s1 > 1 ? li_score_tc_kernel<kLiQuantTc, false> : li_score_tc_kernel<kLiQuant, false>));
+  if (p.causal != 0 && p.b == 1 && p.groups > 1 && p.groups <= kMaxSeqPerLaunch) {  // (a launch of one token has one group)
+    kernel = p.bf16 ? li_score_tc_kernel<kLiBf16, true> : (p.fp16_chain ? li_score_tc_kernel<kLiChain, true> : li_score_tc_kernel<kLiQuantTc, true>);
+  }
   if (p.hist != nullptr && p.s1 > kLiHistMaxS1) return cudaErrorInvalidValue;
   const size_t smem_bytes = kLiSmemBytes + (p.hist != nullptr ? kLiHistSmemBytes : 0);
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
