@@ -341,7 +341,7 @@ struct SfaParams {
   float* part_o;                // [t - split_begin, n_split, nq, 512]
   float* part_ml;               // [t - split_begin, n_split, nq, 2]
   int b, s1, nq, nq_total, head_begin, topk_k, block_size, max_blocks, n_split, packed, kn_bf16;
-  int kn_aligned32; // kn lies on a 32-byte boundary
+  int kn_wide;     // 32-byte loads of int8 latent rows (kn lies on a 32-byte boundary)
   int split_begin;  // first token whose rows are split (n_split > 1); the ones before it are one piece each
   uint32_t page_mul;  // position / block_size = position * page_mul >> page_shift, for every position below 2^31: a division by an
   int page_shift;     // integer that the kernel does not know is about 35 instructions (Granlund and Montgomery 1994)
@@ -361,6 +361,7 @@ struct SfaSplit {
   int begin, n;  // tokens from `begin` on are split n ways
 };
 SfaSplit sfa_pair_split(int t, int num_sms);
+bool sfa_pair_wide_loads(int t, int num_sms);  // whether it gains by 32-byte loads
 cudaError_t launch_sfa_slice(const SfaParams& p, int num_sms, cudaStream_t stream);  // other head counts, int8 caches
 int sfa_slice_heads(int nq);  // heads per work item of that kernel
 

@@ -607,8 +607,8 @@ __device__ __forceinline__ void pair_role_softmax(const SfaParams& p, PairCtx c)
 // Lane r % 16 also walks the look-ahead chain of row 16g + r: the selected index four tiles ahead, its block-table entry three
 // tiles ahead, an L2 prefetch of the half row two tiles ahead, the half row itself (by all lanes) one tile ahead.
 // kFmt: 0 = int8 latent, bf16 rope and fp32 scales in three arrays, 1 = packed 656-byte rows, 2 = bf16 latent and
-// rope arrays (the non-quantised cache), 3 = as 0 on a 32-byte boundary: 32 bytes a lane, half as many loads (kWide; a chunk of 4096
-// tokens over 131072 keys 10.03 -> 9.84 ms. Eight lanes of a store instruction are then both halves of four rows: eight different bank groups again). With a bf16 cache nothing passes through registers: when the half is free
+// rope arrays (the non-quantised cache), 3 = as 0 in 32-byte loads, half as many (kWide, see sfa_pair_wide_loads. Eight lanes of a store
+// instruction are then both halves of four rows: eight different bank groups again). With a bf16 cache nothing passes through registers: when the half is free
 // every lane issues its 16-byte `cp.async` copies from L2 (the rows were prefetched there two tiles ago) straight to
 // the swizzled places the dequantised units would go, waits for them, fences and arrives.
 // A padding or rejected row reads row 0 with scale 0, which dequantises to zeros.
@@ -1021,13 +1021,13 @@ sfa_pair_kernel(const __grid_constant__ SfaParams p) {
     PAIR_SETREG("setmaxnreg.inc.sync.aligned.u32 72;");  // (no change of the count; without it ptxas spills in this role)
     if (p.kn_bf16) pair_role_kproducer<2>(p, c);
     else if (p.packed) pair_role_kproducer<1>(p, c);
-    else if (p.kn_aligned32) pair_role_kproducer<3>(p, c);
+    else if (p.kn_wide) pair_role_kproducer<3>(p, c);
     else pair_role_kproducer<0>(p, c);
   } else {
     PAIR_SETREG("setmaxnreg.dec.sync.aligned.u32 64;");
     if (p.kn_bf16) pair_role_vproducer<2>(p, c);
     else if (p.packed) pair_role_vproducer<1>(p, c);
-    else if (p.kn_aligned32) pair_role_vproducer<3>(p, c);
+    else if (p.kn_wide) pair_role_vproducer<3>(p, c);
     else pair_role_vproducer<0>(p, c);
   }
 
@@ -1054,6 +1054,12 @@ SfaSplit sfa_pair_split(int t, int num_sms) {
   const int begin = t - rest, n = rest > 0 && begin <= kPairSplitRounds * pairs ? pairs / rest : 1;
   return n >= 2 ? SfaSplit{begin, n < 16 ? n : 16} : SfaSplit{0, 1};
 }
+
+// 32-byte row loads where the tokens are more than one round of pairs, 16-byte ones in a single round, in which all pairs go through their
+// tiles in step. Attention alone, tokens x 2048 rows in L2, 16 -> 32 bytes, us: 256 217.8 -> 210.6, 1024 879 -> 829, 4096 3314 -> 3130; 64
+// 59.6 -> 62.9. Steps of up to 30000 keys called one by one, inputs not in L2: 22 tokens 63.2 -> 66.5, 31 74.5 -> 81.1, 44 93.1 -> 100.1, 64 110.5 ->
+// 115.8, 74 116.0 -> 120.3, but 76 130.5 -> 130.9, 111 184.4 -> 181.5, 148 200.7 -> 194.4, 256 295 -> 289; 19 and fewer equal.
+bool sfa_pair_wide_loads(int t, int num_sms) { return t > num_sms / 2; }
 
 cudaError_t launch_sfa_pair(const SfaParams& p, cudaStream_t stream) {
   cudaError_t e = cudaFuncSetAttribute(sfa_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -712,7 +712,7 @@ sfa_slice_kernel(const __grid_constant__ SfaParams p, int n_items) {
   } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::kRegProd));
     if (p.packed) slice_role_producer<kHB, kTK, true, false>(p, ctl, base, n_items);
-    else if (p.kn_aligned32) slice_role_producer<kHB, kTK, false, true>(p, ctl, base, n_items);
+    else if (p.kn_wide) slice_role_producer<kHB, kTK, false, true>(p, ctl, base, n_items);
     else slice_role_producer<kHB, kTK, false, false>(p, ctl, base, n_items);
   }
   tc_fence_before();

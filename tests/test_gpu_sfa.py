@@ -245,6 +245,26 @@ def test_latent_cache_on_a_16_byte_boundary(nq):
     assert torch.equal(out.cpu(), want)
 
 
+@pytest.mark.parametrize("tokens", [74, 75])  # the last count that is read in 16-byte loads wherever the cache lies, the first that is not
+def test_latent_cache_on_a_16_byte_boundary_and_a_second_round(tokens):
+    act = [(700, 130, 1, 5)[i % 4] for i in range(tokens)]
+    d = gen.make_inputs(act, s1=1, seed=tokens, with_indexer=False, with_topk=True)
+    want = _run(d)
+    _check(want, oracle.sparse_attention(d.query_nope, d.query_rope, d.key_nope_2d, d.key_rope_2d, d.k_nope_scales, d.topk_indices,
+                                         d.block_table, d.act_seq, d.s1))
+    g = d.to(DEV)
+    raw = torch.zeros(g.key_nope_2d.numel() + 48, dtype=torch.int8, device=DEV)
+    at = -raw.data_ptr() % 32 + 16
+    kn = raw[at:at + g.key_nope_2d.numel()].view(-1, 512)
+    kn.copy_(g.key_nope_2d)
+    out = torch.zeros((tokens, 1, 128, 512), dtype=torch.bfloat16, device=DEV)
+    pto.sparse_flash_attention_quant_d(g.query_nope, g.query_rope, kn, g.key_rope_2d, g.k_nope_scales, g.topk_indices, g.block_table,
+                                       g.act_seq_key, out, 128, 1, SCALE, 2048, 128, d.max_blocks)
+    torch.cuda.synchronize()
+    assert pto.workspace_status()[0] == 0
+    assert torch.equal(out.cpu(), want)
+
+
 def test_order_of_indices_does_not_matter_beyond_rounding():
     d = gen.make_inputs([5000], s1=1, seed=2, with_indexer=False, with_topk=True)
     a = _run(d)
