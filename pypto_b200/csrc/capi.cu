@@ -319,7 +319,9 @@ int run_sfa(const void* qn, const void* qr, const void* kn, const void* kr, cons
   if (rc != PTO_OK) return rc;
   const int t = b * s1;
   pto::SfaSplit sp = sfa_split(t, nq);
-  // a split costs the merge's launch, 2.5 us: where a round of pairs has gone before and a token's rows are few tiles, more than it gains
+  // A split costs the merge's launch, 2.5 us, and fp32 partials: where a round of pairs has gone before and a token's rows are few tiles, more
+  // than it gains. One piece -> split, us: 1024 rows 75 tokens 59.3 -> 45.1, 100 63.5 -> 61.5, 111 65.6 -> 65.6, 256 134.0 -> 131.2; 768 rows 48.0 ->
+  // 39.2, 51.2 -> 51.1, 51.9 -> 54.9, 109.2 -> 109.7; 2048 rows 110.3 -> 73.7, 113.9 -> 98.3, 116.3 -> 103.0, 253.6 -> 233.5.
   if (sp.begin > 0 && std::min<long long>(topk, static_cast<long long>(max_blocks) * block_size) < kSfaSplitLastRoundRows) sp = {0, 1};
   if (sp.begin > 0 && part_bytes < sfa_extra_bytes(t, nq)) sp = {0, 1};  // (a workspace of the size the call needs, no more)
   if (sp.n > 1 && sp.begin == 0 && part_bytes < sfa_part_bytes(t, nq)) return fail(PTO_ERR_WORKSPACE, "attention workspace too small");

@@ -255,12 +255,15 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
   // A chunk of one prompt whose scores only the selection reads: a token group needs the pages up to its last token's causal end, and
   // the list below is one of groups instead of sequences. (All pages for every group: twice the work where the chunk is the prompt.)
   // The CTAs share it by cost: a group's queries and weights take as long as `kGroupCost` of its pages, and the first groups have
-  // few of these (by pages alone the first CTA got seventy groups of a chunk of 4096). 4096 tokens that are the prompt 208 -> 137 us,
+  // few of these (by pages alone the first CTA got seventy groups of a chunk of 4096). 4096 tokens that are the prompt 208 -> 119 us,
   // behind 12288 keys 756 -> 642, 512 tokens 12.4 -> 11.0; with few tokens behind many keys there is nothing to leave out.
+  // The cost in pages, 0 / 1 / 2 / 3 / 4 / 6 / 8, selection included, us: int8, 4096 tokens that are the prompt 305 / 228 / 186 / 171 / 172 / 177 /
+  // 181, 3000 176 / 129 / 103 / 101 / 102 / 105 / 109; bf16, whose groups are two tokens, 4000 414 / 305 / 245 / 210 / 192 / 180 / 183, 2000 121 / 76 /
+  // 62 / 56 / 53 / 54 / 56; behind other keys and up to 1000 tokens the same within a percent from 1 to 4.
   // kByGroup: kernels of their own, since calls that have nothing to leave out lose by the code for it (whole steps with inputs that are not
   // in L2: 10 sequences of three tokens 79.3 / 77.9 us, 40 of one 109.5 / 108.2; a bf16 layer of 16 95.0 / 93.7).
   const int n_lists = kByGroup ? p.groups : p.b;
-  constexpr int kGroupCost = 2;
+  constexpr int kGroupCost = kBf16 ? 6 : 3;
   constexpr int head = kByGroup ? kGroupCost : 0;  // units of cost before a list's first page
   if (warp == kLiEpilogueWarp0) {
     // exclusive prefix of pages per sequence (or token group)
