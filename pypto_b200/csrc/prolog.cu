@@ -448,7 +448,7 @@ prolog_idxq_kernel(const int32_t* __restrict__ qi_i32, const float* __restrict__
 // ---- per token: latent KV row, rope key, indexer key, indexer weights; scatter into the caches ---------
 // grid = tokens, block = 128 (thread i owns latent dims 4i..4i+3: warp w = 128-wide quantisation tile w). kMany: 64 registers, so
 // that eight blocks share an SM and 1184 tokens are one round (the up-projections' CTAs need whole SMs and wait for the last block:
-// whole prolog 770 tokens 131.7 -> 129.2 us, 1000 142.0 -> 140.1, 1100 168.7 -> 165.5; 600 109.9 -> 109.5)
+// whole prolog 770 tokens 131.7 -> 129.2 us, 1000 142.0 -> 140.1, 1100 168.7 -> 165.5; 600 109.9 -> 109.5; 32 bytes of a thread spill for it)
 template <bool kMany>
 __global__ void __launch_bounds__(128, kMany ? 8 : 0)
 prolog_kv_kernel(const float* __restrict__ kv, const float* __restrict__ ki, const float* __restrict__ wp, int ld,

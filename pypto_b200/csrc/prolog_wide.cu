@@ -310,7 +310,8 @@ __device__ __forceinline__ void wide_dequant_64(uint32_t taddr, float rs, const 
 
 // One tile's rows out of tensor memory: this warp's 32 rows start at `row0`, `taddr` is its lanes of the tile's accumulator. The
 // alignment is a template parameter: with a branch at each of the scales' and cosines' loads they came one after the other, a trip to
-// L2 each (1000 tokens: both up-projections 70 -> 57 us, absorbed query 47.5 -> 43.3, the whole prolog 174 -> 158).
+// L2 each (1000 tokens: both up-projections 70 -> 57 us, absorbed query 47.5 -> 43.3, the whole prolog 174 -> 158). Of the int8
+// up-projections' 168 registers two words of a thread spill.
 template <int kEpi, int kN, bool kAligned>
 __device__ __forceinline__ void wide_epilogue(const WideParams& p, const WideItem& w, const float (&sc)[8], uint32_t taddr, int row0,
                                               uint32_t stage) {

@@ -56,25 +56,6 @@ __device__ __forceinline__ void tmem_st_32x32b_x8(uint32_t taddr, const uint32_t
                : "memory");
 }
 
-// 16 int8 -> 16 bf16 of (value * scale): byte b^0x80 placed in the mantissa of 2^23 gives
-// 2^23 + 128 + x exactly; subtracting 8388736 leaves x; one fp32 multiply and one rounding to bf16,
-// i.e. bf16(fp32(x) * scale) as the golden computes it.
-__device__ __forceinline__ void dequant16(const uint4 v, const float scale, uint4& o0, uint4& o1) {
-  const uint32_t w[4] = {v.x ^ 0x80808080u, v.y ^ 0x80808080u, v.z ^ 0x80808080u, v.w ^ 0x80808080u};
-  uint32_t o[8];
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const float f0 = (__uint_as_float(__byte_perm(w[e], 0x4B000000u, 0x7540)) - 8388736.0f) * scale;
-    const float f1 = (__uint_as_float(__byte_perm(w[e], 0x4B000000u, 0x7541)) - 8388736.0f) * scale;
-    const float f2 = (__uint_as_float(__byte_perm(w[e], 0x4B000000u, 0x7542)) - 8388736.0f) * scale;
-    const float f3 = (__uint_as_float(__byte_perm(w[e], 0x4B000000u, 0x7543)) - 8388736.0f) * scale;
-    o[2 * e] = pack_bf16x2(f0, f1);
-    o[2 * e + 1] = pack_bf16x2(f2, f3);
-  }
-  o0 = make_uint4(o[0], o[1], o[2], o[3]);
-  o1 = make_uint4(o[4], o[5], o[6], o[7]);
-}
-
 // tcgen05.mma with the A operand in tensor memory (row m of A = TMEM lane m, 32-bit column c holds the
 // K elements 2c and 2c+1 of a 16-bit type), B in shared memory.
 __device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
@@ -126,11 +107,6 @@ __device__ __forceinline__ void ldg_pinned_v8(const void* p, uint4& lo, uint4& h
   asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(lo.x), "=r"(lo.y), "=r"(lo.z), "=r"(lo.w), "=r"(hi.x), "=r"(hi.y), "=r"(hi.z), "=r"(hi.w)
                : "l"(p));
-}
-__device__ __forceinline__ float2 ldg_pinned_v2f(const void* p) {
-  float2 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
-  return v;
 }
 __device__ __forceinline__ int ldg_pinned_i32(const void* p) {
   int v;

@@ -8,8 +8,8 @@
 // Why a pair: the fp32 output of 128 heads x 512 values is 256 KB, all of one SM's tensor memory. With the
 // heads split, CTA c keeps O for its 64 heads (256 columns) and two score buffers (2 x 64 columns), and the
 // whole 576-wide contraction is local to the pair's MMA: no score ever crosses between the CTAs, and nothing
-// else does either except the "ready" notices of a tile (two for K, four for V, P, scores read). A 2-SM MMA reads half of its B operand from
-// each CTA's shared memory:
+// else does either except the "ready" notices of a tile (two for K; V with the next tile's rope part; P; scores read). A 2-SM MMA reads half
+// of its B operand from each CTA's shared memory:
 //   q.K^T  (M = 128 heads, N = 128 keys of a tile, K = 576): A = this CTA's 64 query rows, B = the tile's keys,
 //          of which CTA c gathers and dequantises keys [64c, 64c+64) in full width (9 chunks of 64 dims).
 //   P.V    (M = 128 heads, N = 256 of the 512 values per MMA, K = 128 keys): A = this CTA's P, B = V, of which
@@ -156,8 +156,8 @@ __device__ __forceinline__ bool pair_group_wait(PairCtl* ctl, uint32_t& nwait, u
   return *go != 0;
 }
 
-// 8 int8 (two words) -> 8 bf16 of (value * scale), as `dequant16` but with the subtraction and the multiplication on pairs
-// (fp32x2 instructions): the byte placed in the mantissa of 2^23 gives 2^23 + 128 + x exactly, subtracting 8388736
+// 8 int8 (two words) -> 8 bf16 of (value * scale), with the subtraction and the multiplication on pairs (fp32x2 instructions):
+// byte^0x80 placed in the mantissa of 2^23 gives 2^23 + 128 + x exactly, subtracting 8388736
 // leaves x, one fp32 multiply and one rounding to bf16: bf16(fp32(x) * scale) as the golden computes it.
 __device__ __forceinline__ uint4 pair_dequant8(const uint32_t w0, const uint32_t w1, const float scale) {
   const float2 off = make_float2(-8388736.0f, -8388736.0f), sc = make_float2(scale, scale);
