@@ -194,7 +194,7 @@ __device__ __forceinline__ float weighted_relu_sum_32(const uint32_t (&v)[32], c
   return (a01.x + a01.y) + (a23.x + a23.y);
 }
 
-template <int kMode, bool kByGroup>
+template <int kMode, bool kGroups>  // kGroups: launched for more than one token group
 __global__ void __launch_bounds__(kLiThreads, 1)
 li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_q, LiParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -260,22 +260,23 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
   // The cost in pages, 0 / 1 / 2 / 3 / 4 / 6 / 8, selection included, us: int8, 4096 tokens that are the prompt 305 / 228 / 186 / 171 / 172 / 177 /
   // 181, 3000 176 / 129 / 103 / 101 / 102 / 105 / 109; bf16, whose groups are two tokens, 4000 414 / 305 / 245 / 210 / 192 / 180 / 183, 2000 121 / 76 /
   // 62 / 56 / 53 / 54 / 56; behind other keys and up to 1000 tokens the same within a percent from 1 to 4.
-  // kByGroup: kernels of their own, since calls that have nothing to leave out lose by the code for it (whole steps with inputs that are not
-  // in L2: 10 sequences of three tokens 79.3 / 77.9 us, 40 of one 109.5 / 108.2; a bf16 layer of 16 95.0 / 93.7).
-  const int n_lists = kByGroup ? p.groups : p.b;
+  // (kGroups: kernels of their own, since calls that have nothing to leave out lose by the code for it; whole steps with inputs that are not
+  // in L2: 10 sequences of three tokens 79.3 / 77.9 us, 40 of one 109.5 / 108.2; a bf16 layer of 16 95.0 / 93.7.)
+  const bool by_group = kGroups && p.causal != 0 && p.b == 1 && p.groups > 1 && p.groups <= kMaxSeqPerLaunch;
+  const int n_lists = by_group ? p.groups : p.b;
   constexpr int kGroupCost = kBf16 ? 6 : 3;
-  constexpr int head = kByGroup ? kGroupCost : 0;  // units of cost before a list's first page
+  const int head = by_group ? kGroupCost : 0;  // units of cost before a list's first page
   if (warp == kLiEpilogueWarp0) {
     // exclusive prefix of pages per sequence (or token group)
     int carry = 0;
-    const int first_end = kByGroup ? p.act_seq[0] - p.s1_total + p.tok_offset + s1 : 0;  // causal end of the first group
+    const int first_end = by_group ? p.act_seq[0] - p.s1_total + p.tok_offset + s1 : 0;  // causal end of the first group
     for (int b0 = 0; b0 < n_lists; b0 += 32) {
       int v = 0;
       if (b0 + lane < n_lists) {
-        int s = kByGroup ? first_end + (b0 + lane) * s1 : p.act_seq[b0 + lane];
+        int s = by_group ? first_end + (b0 + lane) * s1 : p.act_seq[b0 + lane];
         s = max(s, 0);
         v = min((s + kPageKeys - 1) / kPageKeys, p.max_blocks);
-        if (kByGroup && v > 0) v += head;
+        if (kGroups && v > 0) v += head;
       }
       int incl = v;
 #pragma unroll
@@ -295,7 +296,7 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
 
   // pages of all sequences, once per token group
   const int total = ctl->prefix[n_lists];
-  const long long all = static_cast<long long>(total) * (kByGroup ? 1 : p.groups);
+  const long long all = static_cast<long long>(total) * (by_group ? 1 : p.groups);
   const long long it0 = all * blockIdx.x / gridDim.x, it1 = all * (blockIdx.x + 1) / gridDim.x;
 
   const uint32_t idesc1 = kBf16 ? umma_idesc(kCFmtF32, kABFmtBF16, kABFmtBF16, 0, 0, 128, kHeads)
@@ -342,15 +343,15 @@ li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
     }
     while (ctl->prefix[li + 1] <= lc) ++li;
     const int cost = static_cast<int>(min(it1 - cur, static_cast<long long>(ctl->prefix[li + 1] - lc)));
-    const int page0 = kByGroup ? max(0, lc - ctl->prefix[li] - head) : lc - ctl->prefix[li];
-    const int npages = kByGroup ? max(0, lc - ctl->prefix[li] - head + cost) - page0 : cost;
-    if (kByGroup && npages == 0) {  // (the same in every thread)
+    const int page0 = kGroups ? max(0, lc - ctl->prefix[li] - head) : lc - ctl->prefix[li];
+    const int npages = kGroups ? max(0, lc - ctl->prefix[li] - head + cost) - page0 : cost;
+    if (kGroups && npages == 0) {  // (the same in every thread)
       cur += cost;
       continue;
     }
-    const int bi = kByGroup ? 0 : li;
+    const int bi = by_group ? 0 : li;
     const int seq_len = p.act_seq[bi];
-    const int tok_first = p.tok_offset + (kByGroup ? li : group) * s1;  // first query token of the segment within its sequence
+    const int tok_first = p.tok_offset + (by_group ? li : group) * s1;  // first query token of the segment within its sequence
     const int64_t tok0 = static_cast<int64_t>(bi) * p.s1_total + tok_first;
 
     // The producer warp takes no part in the two barriers of a segment: the ring's own barriers order its loads, so
@@ -767,7 +768,7 @@ cudaError_t launch_li_score_tc(const LiParams& p, const void* tmap_k, const void
   auto kernel = p.bf16 ? li_score_tc_kernel<kLiBf16, false>
                        : (p.fp16_chain ? li_score_tc_kernel<kLiChain, false>
                                        : (p.s1 > 1 ? li_score_tc_kernel<kLiQuantTc, false> : li_score_tc_kernel<kLiQuant, false>));
-  if (p.causal != 0 && p.b == 1 && p.groups > 1 && p.groups <= kMaxSeqPerLaunch) {  // (a launch of one token has one group)
+  if (p.groups > 1) {  // (a launch of one token has one group)
     kernel = p.bf16 ? li_score_tc_kernel<kLiBf16, true> : (p.fp16_chain ? li_score_tc_kernel<kLiChain, true> : li_score_tc_kernel<kLiQuantTc, true>);
   }
   if (p.hist != nullptr && p.s1 > kLiHistMaxS1) return cudaErrorInvalidValue;
