@@ -356,7 +356,10 @@ int run_sfa(const void* qn, const void* qr, const void* kn, const void* kr, cons
   p.split_begin = sp.begin;
   p.packed = packed ? 1 : 0;
   p.kn_bf16 = bf16 ? 1 : 0;
-  p.kn_wide = (reinterpret_cast<uintptr_t>(kn) & 31u) == 0 && (nq != 128 || pto::sfa_pair_wide_loads(t, 148)) ? 1 : 0;
+  p.kn_wide = (reinterpret_cast<uintptr_t>(kn) & 31u) == 0 &&
+                      (nq != 128 || pto::sfa_pair_wide_loads(t, topk, static_cast<int64_t>(max_blocks) * block_size, 148))
+                  ? 1
+                  : 0;
   p.pdl = behind_topk;
   p.n_rows = n_rows;
   p.scale_log2 = softmax_scale * 1.4426950408889634f;

@@ -361,7 +361,7 @@ struct SfaSplit {
   int begin, n;  // tokens from `begin` on are split n ways
 };
 SfaSplit sfa_pair_split(int t, int num_sms);
-bool sfa_pair_wide_loads(int t, int num_sms);  // whether it gains by 32-byte loads
+bool sfa_pair_wide_loads(int t, int topk, int64_t positions, int num_sms);  // whether it gains by 32-byte loads
 cudaError_t launch_sfa_slice(const SfaParams& p, int num_sms, cudaStream_t stream);  // other head counts, int8 caches
 int sfa_slice_heads(int nq);  // heads per work item of that kernel
 

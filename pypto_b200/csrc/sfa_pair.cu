@@ -1055,11 +1055,17 @@ SfaSplit sfa_pair_split(int t, int num_sms) {
   return n >= 2 ? SfaSplit{begin, n < 16 ? n : 16} : SfaSplit{0, 1};
 }
 
-// 32-byte row loads where the tokens are more than one round of pairs, 16-byte ones in a single round, in which all pairs go through their
-// tiles in step. Attention alone, tokens x 2048 rows in L2, 16 -> 32 bytes, us: 256 217.8 -> 210.6, 1024 879 -> 829, 4096 3314 -> 3130; 64
-// 59.6 -> 62.9. Steps of up to 30000 keys called one by one, inputs not in L2: 22 tokens 63.2 -> 66.5, 31 74.5 -> 81.1, 44 93.1 -> 100.1, 64 110.5 ->
-// 115.8, 74 116.0 -> 120.3, but 76 130.5 -> 130.9, 111 184.4 -> 181.5, 148 200.7 -> 194.4, 256 295 -> 289; 19 and fewer equal.
-bool sfa_pair_wide_loads(int t, int num_sms) { return t > num_sms / 2; }
+// 32-byte row loads, but 16-byte ones in a single round of pairs, in which all of them go through their tiles in step, if the selected rows
+// may lie apart (more than two positions for every one selected) and a pair has more than four tiles. Attention alone, tokens x 2048 rows
+// in L2, 16 -> 32 bytes, us: 256 217.8 -> 210.6, 1024 879 -> 829, 4096 3314 -> 3130; 64 59.6 -> 62.9. Whole steps, called one by one with inputs
+// that are not in L2: of up to 30000 keys 17 tokens 55.4 -> 56.9, 24 66.4 -> 69.3, 31 74.5 -> 81.1, 44 93.1 -> 100.1, 64 110.5 -> 115.8, 74 116.0 ->
+// 120.3, but 76 130.5 -> 130.9, 111 184.4 -> 181.5, 148 200.7 -> 194.4, 256 295 -> 289; 5 42.3 -> 41.3, 12 50.4 -> 51.0, 16 51.7 -> 51.8. 64 tokens of 8200
+// keys 91.9 -> 97.0, 5000 82.1 -> 84.8, 1200 51.8 -> 50.8, 900 44.9 -> 43.7 (60 tokens); 40 of 8200 82.3 -> 86.1, 5000 74.0 -> 75.0, 4000 72.9 -> 74.1,
+// 2500 70.6 -> 70.9, 1700 59.7 -> 58.5, 900 41.0 -> 40.9; 20 of 6500 55.2 -> 57.3, 4000 49.0 -> 48.9, 900 32.7 -> 31.7.
+constexpr int kPairWideFew = 16;
+bool sfa_pair_wide_loads(int t, int topk, int64_t positions, int num_sms) {
+  return t > num_sms / 2 || t <= kPairWideFew || positions <= 2 * static_cast<int64_t>(topk);
+}
 
 cudaError_t launch_sfa_pair(const SfaParams& p, cudaStream_t stream) {
   cudaError_t e = cudaFuncSetAttribute(sfa_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

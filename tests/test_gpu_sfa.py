@@ -245,9 +245,11 @@ def test_latent_cache_on_a_16_byte_boundary(nq):
     assert torch.equal(out.cpu(), want)
 
 
-@pytest.mark.parametrize("tokens", [74, 75])  # the last count that is read in 16-byte loads wherever the cache lies, the first that is not
-def test_latent_cache_on_a_16_byte_boundary_and_a_second_round(tokens):
+@pytest.mark.parametrize("tokens", [16, 17, 74, 75])  # from 17 to 74 read in 16-byte loads wherever the cache lies, if the longest has
+@pytest.mark.parametrize("longest", [700, 4224])       # more than 4096 keys
+def test_latent_cache_on_a_16_byte_boundary_over_token_counts(tokens, longest):
     act = [(700, 130, 1, 5)[i % 4] for i in range(tokens)]
+    act[1] = longest
     d = gen.make_inputs(act, s1=1, seed=tokens, with_indexer=False, with_topk=True)
     want = _run(d)
     _check(want, oracle.sparse_attention(d.query_nope, d.query_rope, d.key_nope_2d, d.key_rope_2d, d.k_nope_scales, d.topk_indices,
