@@ -196,7 +196,9 @@ int pto_li_topk(const float* scores, int64_t row_stride, const int32_t* act_seq_
  * ------------------------------------------------------------------------------------------ */
 size_t pto_sfa_workspace_bytes(int t, int nq);
 /* Bytes beyond that (and beyond pto_decode_workspace_bytes) with which a call of more tokens than SM pairs splits the tokens left over
- * by whole rounds of pairs; without them it leaves the last round partly idle. 0 where nothing is to be gained. */
+ * by whole rounds of pairs; without them it leaves the last round partly idle. 0 where nothing is to be gained. With them those
+ * tokens, the last t % 74, are sums of several partial rows where the others are one: of equal tokens the results agree to their
+ * rounding, not bit for bit. */
 size_t pto_sfa_extra_bytes(int t, int nq);
 
 int pto_sfa_quant(const void* query_nope, const void* query_rope, const int8_t* key_nope_2d,

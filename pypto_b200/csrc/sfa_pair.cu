@@ -20,7 +20,7 @@
 //          four chunks of the K tile once q.K^T has read those, while the softmax works.
 //          So a tile needs 64 + 8 KB of shared memory, two tiles are in flight, and a row is dequantised one and a half
 //          times. (With regions of their own for K and V, one tile each, every row was dequantised twice: 4096 tokens x
-//          2048 rows 3.75 -> 3.35 ms, 64 tokens 79 -> 74 us behind a selection, 2 tokens 18.5 -> 16.6 us with the merge.)
+//          2048 rows 3.75 -> 3.35 ms; of rows in L2, 64 tokens 79 -> 74 us behind a selection, 2 tokens 18.5 -> 16.6 us with the merge.)
 // Tensor memory of a 2-SM MMA with 64 rows per CTA: lanes 0-63 hold the first half of the N columns, lanes
 // 64-127 the second half (row = lane % 64). So of a score tile lane l holds (head l % 64, keys 64 (l / 64) ..+63),
 // and of O lane l holds (head l % 64, values 256 (l / 64) ..+255).

@@ -22,8 +22,8 @@
 // an MSB-first radix select over the 64-bit keys on rank 0.
 // What bounds it: one trip of the row from L2 (the first version scanned it three times, for its extremes, a histogram
 // and the collection, with a cluster barrier behind each, and ordered its result with a bitonic sort) and about a dozen
-// block barriers. Before -> after, alone: one row of 4096 12.4 -> 6.3 us (in order 18.5 -> 8.3), 8 x 32768 in order
-// 26.7 -> 12.4, 64 x 65536 16.5 -> 14.4, 256 x 131072 86 -> 52, 1024 x 131072 295 -> 160 us.
+// block barriers. Before -> after, alone: one row of 4096 12.4 -> 6.4 us (in order 18.5 -> 7.2), 8 x 32768 in order
+// 26.7 -> 11.9, 64 x 65536 16.5 -> 13.9, 256 x 131072 86 -> 43, 1024 x 131072 295 -> 152 us.
 // When the score kernel has left a histogram of the row (4096 bins over the top 12 bits of the order-preserving
 // image of the float, counted over the positions below the row's causal end), the bound comes from it instead of the sample,
 // if its total equals the row's length and the list it leads to is not too long.
