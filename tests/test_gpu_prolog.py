@@ -195,6 +195,21 @@ def test_row_counts_of_several_tiles(t, odd):
     check_against(run_prolog(p, odd_outputs=odd), po.mla_indexer_prolog(p, eps_cq=1e-5, eps_ckv=1e-5), p["cache_index"])
 
 
+def test_fifteen_tiles_in_pairs_equal_thirteen_that_are_not():
+    """1793 tokens are the first odd number of tiles that the int8 up-projections take in pairs of SMs (the last one a single row);
+    the last 1600 of them alone take a CTA to a tile. Same order of every sum, so the same bits."""
+    t, first = 1793, 193
+    p = gen.make_prolog_inputs([2000], s1=t, seed=t)
+    whole = run_prolog(p, prefill=True)
+    part = {k: (v[first:].contiguous() if k in ("token_x", "cos", "sin", "cache_index") else v) for k, v in p.items()}
+    alone = run_prolog(part, prefill=True)
+    for key in ("q_nope", "q_rope", "q_int8", "q_scale", "weights"):
+        assert torch.equal(whole[key][first:], alone[key]), key
+    for key in ("kv_cache", "kr_cache", "kv_scale_cache", "idx_k_cache", "idx_k_scale_cache"):
+        assert torch.equal(whole[key].reshape(p["kv_cache"].shape[0], -1)[part["cache_index"]],
+                           alone[key].reshape(p["kv_cache"].shape[0], -1)[part["cache_index"]]), key
+
+
 @pytest.mark.parametrize("t", [385, 520, 1000])  # pairs of SMs for projections and up-projections, for projections only, for both again
 def test_unaligned_outputs_equal_aligned_ones(t):
     p = gen.make_prolog_inputs([130] * t, s1=1, seed=t)
