@@ -194,7 +194,7 @@ __device__ __forceinline__ float weighted_relu_sum_32(const uint32_t (&v)[32], c
   return (a01.x + a01.y) + (a23.x + a23.y);
 }
 
-template <int kMode, bool kGroups>  // kGroups: launched for more than one token group
+template <int kMode, bool kGroups>  // kGroups: takes launches of more than one token group
 __global__ void __launch_bounds__(kLiThreads, 1)
 li_score_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_q, LiParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -768,7 +768,12 @@ cudaError_t launch_li_score_tc(const LiParams& p, const void* tmap_k, const void
   auto kernel = p.bf16 ? li_score_tc_kernel<kLiBf16, false>
                        : (p.fp16_chain ? li_score_tc_kernel<kLiChain, false>
                                        : (p.s1 > 1 ? li_score_tc_kernel<kLiQuantTc, false> : li_score_tc_kernel<kLiQuant, false>));
-  if (p.groups > 1) {  // (a launch of one token has one group)
+  // Of one token group, the int8 kernel of several tokens runs faster with the code for groups in it, which it does not use, where pages are
+  // many (registers lie otherwise; whole steps, without -> with, us: 128 x 131072 keys, two tokens 815 -> 804, 32 x 131072 218.5 -> 215.2, 64 x 65536,
+  // three 398.7 -> 395.8, 16 x 65536, four 133.0 -> 132.3; from 13 to 33 pages a CTA the same; 2 x 8000, two 36.3 -> 37.0). The others gain without.
+  constexpr long long kManyPages = 32;  // per CTA
+  const bool many_pages = !p.bf16 && !p.fp16_chain && p.s1 > 1 && static_cast<long long>(p.b) * p.max_blocks > kManyPages * num_sms;
+  if (p.groups > 1 || many_pages) {  // (a launch of one token has one group)
     kernel = p.bf16 ? li_score_tc_kernel<kLiBf16, true> : (p.fp16_chain ? li_score_tc_kernel<kLiChain, true> : li_score_tc_kernel<kLiQuantTc, true>);
   }
   if (p.hist != nullptr && p.s1 > kLiHistMaxS1) return cudaErrorInvalidValue;
